@@ -7,8 +7,8 @@
 // of the loads (tokens pushed into this GPU's buffer by its peers) and an epilogue that stores
 // output rows through a per-row destination table into peer memory and signals the peers.
 //
-// Roles per CTA (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
-// warps 2..5 = epilogue (TMEM -> registers -> global). All waits are bounded (common.cuh).
+// Roles per CTA (320 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
+// warps 2..9 = epilogue (TMEM -> registers -> global). All waits are bounded (common.cuh).
 //
 // Replaces the cuBLAS calls behind nn.Linear / torch.bmm in the reference
 // (model/attention.py:141-143,189; model/feed_forward.py:75; model/moe.py:1520-1538).
@@ -68,7 +68,7 @@ struct GemmParams {
   const uint4* push_src; long long push_vecs;
   uint4* push_dst[8]; int* push_flag[8]; int push_n;
   int* push_ctr;
-  bool st32;                  // output rows and column chunks are 32-byte aligned: use 32-byte stores
+  bool st32, st32_c2;         // rows and column chunks of C / C2 are 32-byte aligned: use 32-byte stores
   const float* bias;          // optional [N] fp32 added to every output row (plain epilogue)
 };
 
@@ -122,23 +122,192 @@ struct Tile {
   int g, m_blk, n_blk;
 };
 
-// MT = 1: one 128 x BN accumulator per tile, double-buffered in tensor memory (the epilogue of a tile runs under the
-// MMAs of the next). MT = 2: a 256 x BN tile as two 128-row halves that share every B tile; per FLOP a third fewer
-// operand bytes cross from L2 into shared memory, which is what bounds the 128 x 256 tile (the L2 -> SM fabric
-// delivers about 16 TB/s, the 128 x 256 tile asks for 11.4 bytes per kFLOP). The two accumulators fill all 512
-// tensor-memory columns, so they are single-buffered: MMA issue pauses while a tile drains.
-template <int BN, int STAGES, int MT>
-__global__ void __launch_bounds__(192, 1)
+// Tile order: bands of BAND M blocks, so that one wave of CTAs touches a band of A row blocks and a few B row blocks
+// instead of all of A, and both operands are re-read from L2 rather than from DRAM.
+template <int BAND>
+__device__ __forceinline__ Tile decode_tile(int t, int m_blocks, int n_blocks) {
+  Tile tl;
+  const int per_group = m_blocks * n_blocks;
+  tl.g = t / per_group;
+  const int r = t - tl.g * per_group;
+  const int per_band = BAND * n_blocks;
+  const int band = r / per_band;
+  const int first_m = band * BAND;
+  const int gsize = (m_blocks - first_m) < BAND ? (m_blocks - first_m) : BAND;
+  const int within = r - band * per_band;
+  tl.m_blk = first_m + within % gsize;
+  tl.n_blk = within / gsize;
+  return tl;
+}
+
+// Where a thread's output row goes. Row-table launches: into the peer named by the table; rows and columns outside the
+// output are not stored.
+struct OutRow {
+  char* c;
+  const char* cin;   // accumulate source or nullptr
+  bool ok;
+};
+__device__ __forceinline__ OutRow out_row(const GemmParams& p, int g, int row) {
+  OutRow o;
+  const int es = p.out_f32 ? 4 : 2;
+  o.ok = row < p.M;
+  if (p.row_dst) {
+    const long long d = o.ok ? p.row_dst[row] : -1;
+    o.ok = o.ok && d >= 0;
+    const long long peer = o.ok ? (d >> 40) : 0;
+    const long long drow = d & ((1ll << 40) - 1);
+    o.c = (char*)p.peer_base[peer] + (size_t)drow * p.ldc * es;
+  } else {
+    o.c = (char*)p.C + ((size_t)g * p.group_stride_c + (size_t)row * p.ldc) * es;
+  }
+  o.cin = p.Cin ? (const char*)p.Cin + ((size_t)g * p.group_stride_c + (size_t)row * p.ldcin) * es : nullptr;
+  return o;
+}
+
+// Plain epilogue of 32 accumulator columns starting at output column `col`: alpha, bias, accumulate source, output type.
+__device__ __forceinline__ void store_chunk(const GemmParams& p, const OutRow& o, uint32_t* r, int col) {
+  if (!o.ok || col >= p.N) return;
+  const bool full = col + 32 <= p.N;
+  if (p.bias) {  // the same 32 values for every row of the warp: broadcast loads
+    const float inv_alpha = 1.f / p.alpha;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const float b = (col + i < p.N) ? __ldg(p.bias + col + i) : 0.f;
+      r[i] = __float_as_uint(fmaf(b, inv_alpha, __uint_as_float(r[i])));
+    }
+  }
+  if (p.out_f32) {
+    float* dst = (float*)o.c + col;
+    if (full) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float4 v = make_float4(__uint_as_float(r[4 * i]) * p.alpha, __uint_as_float(r[4 * i + 1]) * p.alpha,
+                               __uint_as_float(r[4 * i + 2]) * p.alpha, __uint_as_float(r[4 * i + 3]) * p.alpha);
+        if (o.cin) {
+          const float4 c = reinterpret_cast<const float4*>((const float*)o.cin + col)[i];
+          v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
+        }
+        reinterpret_cast<float4*>(dst)[i] = v;
+      }
+    } else {
+      _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
+        float v = __uint_as_float(r[i]) * p.alpha;
+        if (o.cin) v += ((const float*)o.cin + col)[i];
+        dst[i] = v;
+      }
+    }
+  } else {
+    __nv_bfloat16* dst = (__nv_bfloat16*)o.c + col;
+    if (full) {
+      uint32_t pk[16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float f[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[8 * i + j]) * p.alpha;
+        if (o.cin) {
+          const uint4 c = reinterpret_cast<const uint4*>((const __nv_bfloat16*)o.cin + col)[i];
+          const float2 c0 = np::unpack_bf16(c.x), c1 = np::unpack_bf16(c.y), c2 = np::unpack_bf16(c.z), c3 = np::unpack_bf16(c.w);
+          f[0] += c0.x; f[1] += c0.y; f[2] += c1.x; f[3] += c1.y;
+          f[4] += c2.x; f[5] += c2.y; f[6] += c3.x; f[7] += c3.y;
+        }
+        pk[4 * i] = np::pack_bf16(f[0], f[1]); pk[4 * i + 1] = np::pack_bf16(f[2], f[3]);
+        pk[4 * i + 2] = np::pack_bf16(f[4], f[5]); pk[4 * i + 3] = np::pack_bf16(f[6], f[7]);
+      }
+      store64(dst, pk, p.st32);
+    } else {
+      _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
+        float v = __uint_as_float(r[i]) * p.alpha;
+        if (o.cin) v += __bfloat162float(((const __nv_bfloat16*)o.cin + col)[i]);
+        dst[i] = __float2bfloat16(v);
+      }
+    }
+  }
+}
+
+// SwiGLU epilogue of 32 gate and 32 up columns: silu(gate) * up, and the pre-activations side by side when asked for.
+__device__ __forceinline__ void store_swiglu_chunk(const GemmParams& p, const OutRow& o, const uint32_t* g, const uint32_t* u,
+                                                   int row, int col) {
+  if (!o.ok || col >= p.N) return;
+  const bool full = col + 32 <= p.N;
+  uint32_t h[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
+    const float u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
+    h[i] = np::pack_bf16(np::silu_f(g0) * u0, np::silu_f(g1) * u1);
+  }
+  __nv_bfloat16* dst = (__nv_bfloat16*)o.c + col;
+  if (full) {
+    store64(dst, h, p.st32);
+  } else {
+    _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) dst[i] = reinterpret_cast<__nv_bfloat16*>(h)[i];
+  }
+  if (!p.C2) return;
+  __nv_bfloat16* d2 = (__nv_bfloat16*)p.C2 + (size_t)row * p.ldc2 + col;
+  if (full) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = np::pack_bf16(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1]));
+    store64(d2, h, p.st32_c2);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = np::pack_bf16(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
+    store64(d2 + p.N, h, p.st32_c2);
+  } else {
+    _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
+      d2[i] = __float2bfloat16(__uint_as_float(g[i]));
+      d2[p.N + i] = __float2bfloat16(__uint_as_float(u[i]));
+    }
+  }
+}
+
+// Two warps share the 32 tensor-memory lanes of a quarter and take half of a tile's columns each: the drain of a tile
+// that no MMA of a next tile covers (the only, or the last one of a CTA) takes half as long as with one.
+constexpr int EPI_WARPS = 8;
+constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
+
+// Half `half` of the BN accumulator columns of one 128-row tile: tensor memory (`taddr`: this warp's lanes, first column)
+// through the epilogue of the launch to output row `row`, columns from `n0`. Executed by whole warps (the tensor-memory
+// loads are .sync.aligned).
+template <int BN>
+__device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t taddr, int g_idx, int row, int n0, int half,
+                                           bool have_acc) {
+  const OutRow o = out_row(p, g_idx, row);
+  if (p.epilogue == 1) {
+    // gate = columns [0, BN/2), up = columns [BN/2, BN)
+#pragma unroll 1
+    for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
+      uint32_t g[32], u[32];
+      np::tmem_ld32(taddr + c * 32, g);
+      np::tmem_ld32(taddr + BN / 2 + c * 32, u);
+      np::tmem_ld_wait();
+      store_swiglu_chunk(p, o, g, u, row, n0 + c * 32);
+    }
+  } else {
+#pragma unroll 1
+    for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+      uint32_t r[32];
+      if (have_acc) {
+        np::tmem_ld32(taddr + c * 32, r);
+        np::tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = 0u;
+      }
+      store_chunk(p, o, r, n0 + c * 32);
+    }
+  }
+}
+
+// One CTA per tile: a 128 x BN accumulator, double-buffered in tensor memory (the epilogue of a tile runs under the
+// MMAs of the next).
+template <int BN, int STAGES>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmAloc,
                  const __grid_constant__ CUtensorMap tmBloc, const GemmParams p) {
-  constexpr int TM = BM * MT;                 // rows of a tile
-  constexpr int A_HALF = BM * BK * 2;         // one 128-row half of the A tile
-  constexpr int A_BYTES = TM * BK * 2;
+  constexpr int A_BYTES = BM * BK * 2;
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr int NACC = MT == 1 ? 2 : 1;       // accumulator buffers in tensor memory
-  static_assert(MT * BN * NACC <= 512, "tensor memory holds 512 columns");
   constexpr int TMEM_COLS = (2 * BN <= 32) ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));
 
   extern __shared__ uint8_t smem_raw[];
@@ -157,7 +326,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int lane = threadIdx.x & 31;
   const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
 
-  const int m_blocks = (p.M + TM - 1) / TM;
+  const int m_blocks = (p.M + BM - 1) / BM;
   const int bn_out = (p.epilogue == 1) ? BN / 2 : BN;  // output columns per tile
   const int n_blocks = (p.N + bn_out - 1) / bn_out;
   const int groups = (p.mode == 2) ? p.num_groups : 1;
@@ -171,7 +340,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       np::mbar_init(tfull_bar(a), 1);
-      np::mbar_init(tempty_bar(a), 4);
+      np::mbar_init(tempty_bar(a), EPI_WARPS);
     }
     *abort_flag = 0;
     np::mbar_fence_init();
@@ -203,26 +372,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 
   auto decode = [&](int t) {
-    Tile tl;
-    tl.g = t / tiles_per_group;
-    const int r = t - tl.g * tiles_per_group;
-    // bands of 16 M blocks: one wave of CTAs touches ~16 A row-blocks and ~9 B row-blocks instead of all
-    // of A, so both operands are re-read from L2 rather than from DRAM
-    constexpr int BAND = 16;
-    const int per_band = BAND * n_blocks;
-    const int band = r / per_band;
-    const int first_m = band * BAND;
-    const int gsize = (m_blocks - first_m) < BAND ? (m_blocks - first_m) : BAND;
-    const int within = r - band * per_band;
-    tl.m_blk = first_m + within % gsize;
-    tl.n_blk = within / gsize;
+    Tile tl = decode_tile<16>(t, m_blocks, n_blocks);
     if (p.m_rot) tl.m_blk = (tl.m_blk + p.m_rot) % m_blocks;
     if (p.n_rot) tl.n_blk = (tl.n_blk + p.n_rot) % n_blocks;
     return tl;
   };
   // rows of this M block that carry data (0 = nothing to do); waits for the arrival flag first.
   auto tile_rows = [&](const Tile& tl, int role) -> int {
-    if (p.mode != 1 || MT != 1) return TM;   // the row-grouped form (per-128-row-block tables) runs with MT = 1
+    if (p.mode != 1) return BM;
     if (p.ready_flags) {
       const int fi = p.mblk_flag ? p.mblk_flag[tl.m_blk] : 0;
       if (fi >= 0 && !np::wait_flag_ge(p.ready_flags + fi, epoch, p.flag_limit_ns, KID_GEMM, 100 + role)) {
@@ -243,7 +400,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int rows = tile_rows(tl, 0);
         if (rows < 0) break;
         if (rows == 0) continue;
-        const int m0 = tl.m_blk * TM;
+        const int m0 = tl.m_blk * BM;
         const int n0 = tl.n_blk * bn_out;
         long long goff = 0;  // row offset of this tile's group inside the stacked B tensor
         if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[tl.m_blk] * p.group_stride_b;
@@ -275,15 +432,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint32_t sB = sA + A_BYTES;
           np::mbar_expect_tx(full_bar(stage), STAGE_BYTES);
           if (!p.a_mn) {
-            if (MT == 1 && m0 >= p.a_loc_lo && m0 < p.a_loc_hi) {
-              np::tma_load_2d(sA, &tmAloc, full_bar(stage), k0, m0 - p.a_loc_lo);
-            } else {
-#pragma unroll
-              for (int h = 0; h < MT; ++h) np::tma_load_2d(sA + h * A_HALF, &tmA, full_bar(stage), k0, m0 + h * BM);
-            }
+            if (m0 >= p.a_loc_lo && m0 < p.a_loc_hi) np::tma_load_2d(sA, &tmAloc, full_bar(stage), k0, m0 - p.a_loc_lo);
+            else np::tma_load_2d(sA, &tmA, full_bar(stage), k0, m0);
           } else {
 #pragma unroll
-            for (int c = 0; c < TM / 64; ++c)
+            for (int c = 0; c < BM / 64; ++c)
               np::tma_load_2d(sA + c * (64 * BK * 2), &tmA, full_bar(stage), m0 + c * 64, k0);
           }
           if (!p.b_mn) {
@@ -322,7 +475,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (count_k(p, tl.g) == 0) continue;
         if (!np::mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 2)) break;
         np::tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * MT * BN);
+        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
         uint32_t accum = 0;
         for_each_k(p, tl.g, [&](int) -> bool {
           if (!np::mbar_wait(full_bar(stage), phase, abort_flag, KID_GEMM, 3)) return false;
@@ -333,13 +486,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int kk = 0; kk < BK / 16; ++kk) {
             const uint64_t bd = p.b_mn ? np::make_smem_desc(sB + kk * 2048, 64 * BK * 2, 1024)
                                        : np::make_smem_desc(sB + kk * 32, 16, 1024);
-#pragma unroll
-            for (int h = 0; h < MT; ++h) {   // both halves read the same B tile
-              const uint32_t sAh = sA + h * A_HALF;
-              const uint64_t ad = p.a_mn ? np::make_smem_desc(sAh + kk * 2048, 64 * BK * 2, 1024)
-                                         : np::make_smem_desc(sAh + kk * 32, 16, 1024);
-              np::tc_mma_f16(tmem_d + (uint32_t)(h * BN), ad, bd, idesc, accum);
-            }
+            const uint64_t ad = p.a_mn ? np::make_smem_desc(sA + kk * 2048, 64 * BK * 2, 1024)
+                                       : np::make_smem_desc(sA + kk * 32, 16, 1024);
+            np::tc_mma_f16(tmem_d, ad, bd, idesc, accum);
             accum = 1;
           }
           np::tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
@@ -347,13 +496,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           return true;
         });
         np::tc_commit(tfull_bar(acc));
-        if (++acc == NACC) { acc = 0; acc_phase ^= 1u; }
+        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
       if (*abort_flag) __nanosleep(1000000);
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
-    const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32)
+    // ------------------------------------------------------------ epilogue
+    const int quarter = warp & 3, half = (warp - 2) >> 2;  // TMEM lanes [32*quarter, 32*quarter+32), column half
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
@@ -368,151 +517,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 4)) break;
         np::tc_fence_after();
       }
-#pragma unroll 1
-      for (int h = 0; h < MT; ++h) {   // the 128-row halves of the tile, one accumulator each
-      const int row = tl.m_blk * TM + h * BM + quarter * 32 + lane;
-      bool row_ok = row < p.M;
-      char* crow;
-      if (p.row_dst) {
-        const long long d = row_ok ? p.row_dst[row] : -1;
-        row_ok = row_ok && d >= 0;
-        const long long peer = row_ok ? (d >> 40) : 0;
-        const long long drow = d & ((1ll << 40) - 1);
-        crow = (char*)p.peer_base[peer] + (size_t)drow * p.ldc * (p.out_f32 ? 4 : 2);
-      } else {
-        crow = (char*)p.C + ((size_t)tl.g * p.group_stride_c + (size_t)row * p.ldc) * (p.out_f32 ? 4 : 2);
-      }
-      const char* cin_row = p.Cin ? (const char*)p.Cin + ((size_t)tl.g * p.group_stride_c + (size_t)row * p.ldcin) * (p.out_f32 ? 4 : 2)
-                                  : nullptr;
-      const uint32_t taddr = tmem_base + (uint32_t)((acc * MT + h) * BN) + ((uint32_t)(quarter * 32) << 16);
-      if (p.epilogue == 1) {
-        // gate = columns [0, BN/2), up = columns [BN/2, BN); out = silu(gate) * up
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t g[32], u[32];
-          np::tmem_ld32(taddr + c * 32, g);
-          np::tmem_ld32(taddr + BN / 2 + c * 32, u);
-          np::tmem_ld_wait();
-          const int col = n0 + c * 32;
-          if (row_ok && col < p.N) {
-            uint32_t o[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
-              const float u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
-              o[i] = np::pack_bf16(np::silu_f(g0) * u0, np::silu_f(g1) * u1);
-            }
-            __nv_bfloat16* dst = (__nv_bfloat16*)crow + col;
-            if (col + 32 <= p.N) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                reinterpret_cast<uint4*>(dst)[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-            } else {
-              _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N)
-                dst[i] = reinterpret_cast<__nv_bfloat16*>(o)[i];
-            }
-            if (p.C2) {
-              __nv_bfloat16* d2 = (__nv_bfloat16*)p.C2 + (size_t)row * p.ldc2 + col;
-              if (col + 32 <= p.N) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  reinterpret_cast<uint4*>(d2)[i] =
-                      make_uint4(np::pack_bf16(__uint_as_float(g[8 * i]), __uint_as_float(g[8 * i + 1])),
-                                 np::pack_bf16(__uint_as_float(g[8 * i + 2]), __uint_as_float(g[8 * i + 3])),
-                                 np::pack_bf16(__uint_as_float(g[8 * i + 4]), __uint_as_float(g[8 * i + 5])),
-                                 np::pack_bf16(__uint_as_float(g[8 * i + 6]), __uint_as_float(g[8 * i + 7])));
-                  reinterpret_cast<uint4*>(d2 + p.N)[i] =
-                      make_uint4(np::pack_bf16(__uint_as_float(u[8 * i]), __uint_as_float(u[8 * i + 1])),
-                                 np::pack_bf16(__uint_as_float(u[8 * i + 2]), __uint_as_float(u[8 * i + 3])),
-                                 np::pack_bf16(__uint_as_float(u[8 * i + 4]), __uint_as_float(u[8 * i + 5])),
-                                 np::pack_bf16(__uint_as_float(u[8 * i + 6]), __uint_as_float(u[8 * i + 7])));
-                }
-              } else {
-                _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
-                  d2[i] = __float2bfloat16(__uint_as_float(g[i]));
-                  d2[p.N + i] = __float2bfloat16(__uint_as_float(u[i]));
-                }
-              }
-            }
-          }
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          if (have_acc) {
-            np::tmem_ld32(taddr + c * 32, r);
-            np::tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = 0u;
-          }
-          const int col = n0 + c * 32;
-          if (!row_ok || col >= p.N) continue;
-          const bool full = col + 32 <= p.N;
-          if (p.bias) {  // the same 32 values for every row of the warp: broadcast loads
-            const float inv_alpha = 1.f / p.alpha;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float b = (col + i < p.N) ? __ldg(p.bias + col + i) : 0.f;
-              r[i] = __float_as_uint(fmaf(b, inv_alpha, __uint_as_float(r[i])));
-            }
-          }
-          if (p.out_f32) {
-            float* dst = (float*)crow + col;
-            if (full) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                float4 v = make_float4(__uint_as_float(r[4 * i]) * p.alpha, __uint_as_float(r[4 * i + 1]) * p.alpha,
-                                       __uint_as_float(r[4 * i + 2]) * p.alpha, __uint_as_float(r[4 * i + 3]) * p.alpha);
-                if (cin_row) {
-                  const float4 o = reinterpret_cast<const float4*>((const float*)cin_row + col)[i];
-                  v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                reinterpret_cast<float4*>(dst)[i] = v;
-              }
-            } else {
-              _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
-                float v = __uint_as_float(r[i]) * p.alpha;
-                if (cin_row) v += ((const float*)cin_row + col)[i];
-                dst[i] = v;
-              }
-            }
-          } else {
-            __nv_bfloat16* dst = (__nv_bfloat16*)crow + col;
-            if (full) {
-              uint32_t pk[16];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                float f[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[8 * i + j]) * p.alpha;
-                if (cin_row) {
-                  const uint4 o = reinterpret_cast<const uint4*>((const __nv_bfloat16*)cin_row + col)[i];
-                  const float2 o0 = np::unpack_bf16(o.x), o1 = np::unpack_bf16(o.y), o2 = np::unpack_bf16(o.z), o3 = np::unpack_bf16(o.w);
-                  f[0] += o0.x; f[1] += o0.y; f[2] += o1.x; f[3] += o1.y;
-                  f[4] += o2.x; f[5] += o2.y; f[6] += o3.x; f[7] += o3.y;
-                }
-                pk[4 * i] = np::pack_bf16(f[0], f[1]); pk[4 * i + 1] = np::pack_bf16(f[2], f[3]);
-                pk[4 * i + 2] = np::pack_bf16(f[4], f[5]); pk[4 * i + 3] = np::pack_bf16(f[6], f[7]);
-              }
-              store64(dst, pk, p.st32);
-            } else {
-              _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
-                float v = __uint_as_float(r[i]) * p.alpha;
-                if (cin_row) v += __bfloat162float(((const __nv_bfloat16*)cin_row + col)[i]);
-                dst[i] = __float2bfloat16(v);
-              }
-            }
-          }
-        }
-      }
-      }   // halves
+      store_tile<BN>(p, tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
+                     tl.m_blk * BM + quarter * 32 + lane, n0, half, have_acc);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
         if (lane == 0) np::mbar_arrive(tempty_bar(acc));
-        if (++acc == NACC) { acc = 0; acc_phase ^= 1u; }
+        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
       if (p.done_counters) {
         // all rows of this tile are stored (possibly into peer memory): publish, then count the
@@ -520,10 +531,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __threadfence_system();
         __syncwarp();
         if (lane == 0) {
-          // each of the four epilogue warps counts once per tile: expected is in tiles
+          // each epilogue warp counts once per tile: expected is in tiles
           const int fi = p.mblk_flag ? p.mblk_flag[tl.m_blk] : 0;
           const int done = atomicAdd(&p.done_counters[fi], 1) + 1;
-          if (done == 4 * n_blocks * p.done_expected[fi]) {  // done_expected counts M blocks
+          if (done == EPI_WARPS * n_blocks * p.done_expected[fi]) {  // done_expected counts M blocks
             __threadfence_system();
             np::st_release_sys(p.done_flag_ptr[fi], epoch);
           }
@@ -540,7 +551,261 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// ------------------------------------------------------------------------------------------- two CTAs per tile
+// A 256 x 256 tile computed by a cluster of two CTAs (tcgen05 cta_group::2): each CTA stages 128 rows of A and 128 of
+// the 256 rows of B, the leader issues one 256 x 256 x 16 MMA that reads both CTAs' shared memory, and each CTA's tensor
+// memory receives its own 128 rows of the result. Against the one-CTA 128 x 256 tile, which asks the L2 -> SM fabric for
+// 48 KB per 64-wide K step and SM, this needs 32 KB for the same FLOPs, and unlike a 256 x 256 tile on one SM the
+// 128 x 256 accumulator still fits tensor memory twice, so a tile drains under the MMAs of the next. The freed shared
+// memory deepens the pipeline to PAIR_STAGES K steps. No load is multicast.
+//
+// Barriers: full[s] lives in the leader and counts the bytes of both CTAs' loads; empty[s] and tfull[a] exist in both
+// CTAs and are signalled by one multicast commit of the leader; tempty[a] lives in the leader and takes the arrivals of
+// the epilogue warps of both CTAs. The cluster barrier at the end keeps a CTA's shared memory alive until its peer's last
+// remote arrival; both CTAs reach it on every path because every wait before it is bounded.
+constexpr int PAIR_BN = 256, PAIR_STAGES = 6;
+constexpr int PAIR_STAGE_BYTES = BM * BK * 2 + (PAIR_BN / 2) * BK * 2;   // per CTA
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t leader_addr(uint32_t smem_addr) {   // the same shared-memory offset in CTA 0
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_addr));
+  return r;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// load into this CTA's shared memory, bytes counted on a barrier of either CTA of the pair (not a multicast)
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {   // arrives on the barrier at this offset in both CTAs
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      ::"r"(bar), "h"((uint16_t)3)
+      : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmB2, const GemmParams p) {
+  constexpr int BN = PAIR_BN, STAGES = PAIR_STAGES, TM = 2 * BM, HN = BN / 2;
+  constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = PAIR_STAGE_BYTES;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (np::smem_u32(smem_raw) + 1023u) & ~1023u;   // the same offset in both CTAs
+  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
+  auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
+  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
+  uint8_t* tail = smem_raw + (bar_base - np::smem_u32(smem_raw)) + 8 * (2 * STAGES + 4);
+  volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(tail);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
+  const int m_blocks = (p.M + TM - 1) / TM, m_blocks128 = (p.M + BM - 1) / BM;
+  const int bn_out = (p.epilogue == 1) ? HN : BN;
+  const int n_blocks = (p.N + bn_out - 1) / bn_out;
+  const int num_tiles = m_blocks * n_blocks * ((p.mode == 2) ? p.num_groups : 1);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      np::mbar_init(full_bar(s), 1);
+      np::mbar_init(empty_bar(s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      np::mbar_init(tfull_bar(a), 1);
+      np::mbar_init(tempty_bar(a), 2 * EPI_WARPS);
+    }
+    *abort_flag = 0;
+    np::mbar_fence_init();
+    np::tma_prefetch_desc(&tmA);
+    np::tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     np::smem_u32((const void*)tmem_ptr_smem)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  np::tc_fence_before();
+  __syncthreads();
+  cluster_sync();        // the peer's barriers are initialised before anything arrives on them
+  np::tc_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+
+  // rows of the two 128-row blocks of an M block that carry data, as a mask (0: nothing to do, -1: gave up). Row-grouped
+  // form: both blocks belong to the same group and arrive under the same flag (the caller's tables are made of pairs).
+  auto tile_rows = [&](const Tile& tl, int role) -> int {
+    if (p.mode != 1) return 3;
+    const int b0 = 2 * tl.m_blk;
+    if (p.ready_flags) {
+      const int fi = p.mblk_flag ? p.mblk_flag[b0] : 0;
+      if (fi >= 0 && !np::wait_flag_ge(p.ready_flags + fi, epoch, p.flag_limit_ns, KID_GEMM, 120 + role)) {
+        *abort_flag = 1;
+        return -1;
+      }
+    }
+    if (!p.mblk_rows) return 3;
+    return (p.mblk_rows[b0] > 0 ? 1 : 0) | (b0 + 1 < m_blocks128 && p.mblk_rows[b0 + 1] > 0 ? 2 : 0);
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer (one in each CTA)
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
+        const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
+        const int rows = tile_rows(tl, 0);
+        if (rows < 0) break;
+        if (rows == 0) continue;
+        const int m0 = tl.m_blk * TM + rank * BM;
+        const int n0 = tl.n_blk * bn_out;
+        long long goff = 0;
+        if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[2 * tl.m_blk] * p.group_stride_b;
+        // SwiGLU: the leader's half of B is the gate tile, the peer's the up tile (another tensor, the same rows)
+        const CUtensorMap* bm = (p.epilogue == 1 && rank) ? &tmB2 : &tmB;
+        const int nrow = n0 + (p.epilogue == 1 ? 0 : rank * HN);
+        for_each_k(p, tl.g, [&](int k0) -> bool {
+          if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 11)) return false;
+          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
+          const uint32_t fb = leader_addr(full_bar(stage));
+          if (rank == 0) np::mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
+          if (!p.a_mn) {
+            tma_load_2d_pair(sA, &tmA, fb, k0, m0);
+          } else {
+#pragma unroll
+            for (int c = 0; c < BM / 64; ++c) tma_load_2d_pair(sA + c * (64 * BK * 2), &tmA, fb, m0 + c * 64, k0);
+          }
+          if (!p.b_mn) {
+            tma_load_2d_pair(sB, bm, fb, k0, (int)(nrow + goff));
+          } else {
+#pragma unroll
+            for (int c = 0; c < HN / 64; ++c)
+              tma_load_2d_pair(sB + c * (64 * BK * 2), bm, fb, nrow + c * 64, k0 + (int)goff);
+          }
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          return true;
+        });
+      }
+      // the leader's last commits have arrived here before this CTA may exit (a stage never used passes at once)
+      for (int s = 0; s < STAGES; ++s) {
+        if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 15)) break;
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (*abort_flag) __nanosleep(1000000);   // let copies already issued land before exit
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer (the leader's)
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc = np::make_idesc(TM, BN, 1, 1, p.a_mn, p.b_mn);
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
+        const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
+        const int rows = tile_rows(tl, 1);
+        if (rows < 0) break;
+        if (rows == 0) continue;
+        if (count_k(p, tl.g) == 0) continue;
+        if (!np::mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 12)) break;
+        np::tc_fence_after();
+        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+        uint32_t accum = 0;
+        for_each_k(p, tl.g, [&](int) -> bool {
+          if (!np::mbar_wait(full_bar(stage), phase, abort_flag, KID_GEMM, 13)) return false;
+          np::tc_fence_after();
+          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk) {
+            const uint64_t ad = p.a_mn ? np::make_smem_desc(sA + kk * 2048, 64 * BK * 2, 1024)
+                                       : np::make_smem_desc(sA + kk * 32, 16, 1024);
+            const uint64_t bd = p.b_mn ? np::make_smem_desc(sB + kk * 2048, 64 * BK * 2, 1024)
+                                       : np::make_smem_desc(sB + kk * 32, 16, 1024);
+            tc_mma_f16_pair(tmem_d, ad, bd, idesc, accum);
+            accum = 1;
+          }
+          tc_commit_pair(empty_bar(stage));
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          return true;
+        });
+        tc_commit_pair(tfull_bar(acc));
+        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+      }
+      if (*abort_flag) __nanosleep(1000000);
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue (both CTAs)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
+      const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
+      const int rows = tile_rows(tl, 2);
+      if (rows < 0) break;
+      if (rows == 0) continue;
+      const bool have_acc = count_k(p, tl.g) > 0;
+      const bool mine = (rows >> rank) & 1;   // this CTA's 128-row block carries data
+      if (have_acc) {
+        if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 14)) break;
+        np::tc_fence_after();
+      }
+      if (mine)
+        store_tile<BN>(p, tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
+                       tl.m_blk * TM + rank * BM + quarter * 32 + lane, tl.n_blk * bn_out, half, have_acc);
+      if (have_acc) {
+        np::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_cluster(leader_addr(tempty_bar(acc)));
+        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+      }
+      if (p.done_counters && mine) {
+        __threadfence_system();
+        __syncwarp();
+        if (lane == 0) {
+          const int fi = p.mblk_flag ? p.mblk_flag[2 * tl.m_blk] : 0;
+          const int done = atomicAdd(&p.done_counters[fi], 1) + 1;
+          if (done == EPI_WARPS * n_blocks * p.done_expected[fi]) {   // done_expected counts 128-row blocks
+            __threadfence_system();
+            np::st_release_sys(p.done_flag_ptr[fi], epoch);
+          }
+        }
+      }
+    }
+  }
+  np::tc_fence_before();
+  __syncthreads();
+  cluster_sync();        // nothing of the peer reads or arrives here any more
+  if (warp == 1) {
+    np::tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  }
+}
+
 int g_num_sms = 0;
+// Cost of one tile in units of the pair kernel's 256 x 256 tile on two SMs (see np_gemm_bf16).
+constexpr double COST_PAIR = 1.0, COST_256 = 1.15, COST_128 = 0.65;
 
 }  // namespace
 
@@ -604,18 +869,27 @@ struct NpGemmArgs {
   // push_ctr: a zeroed local int
   const void* push_src; long long push_bytes; void* const* push_dst; int* const* push_flag; int push_n; int* push_ctr;
   const float* bias;  // optional [N] fp32 bias added in the plain epilogue (alpha != 0)
-  int mt;             // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles, dense and K-grouped forms)
+  int mt;             // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles on a pair of CTAs)
+  int paired;         // row-grouped form: blocks 2 i and 2 i + 1 share their group and their arrival flag
 };
 
-template <int BN, int STAGES, int MT>
+static int num_sms() {
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return g_num_sms > 0 ? g_num_sms : 148;
+}
+
+template <int BN, int STAGES, bool PAIR>
 static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
-  constexpr int TM = BM * MT;
   CUtensorMap tmA, tmB, tmB2, tmAloc, tmBloc;
   int rc;
   if (!a.a_mn) rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.K, (uint64_t)a.lda, BK, BM);
   else rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.M, (uint64_t)a.lda, 64, BK);
   if (rc) return 100 + rc;
-  const uint32_t b_box_rows = a.epilogue == 1 ? BN / 2 : BN;
+  const uint32_t b_box_rows = (PAIR || a.epilogue == 1) ? BN / 2 : BN;
   if (!a.b_mn) rc = np_make_tmap_2d(&tmB, a.B, 2, (uint64_t)a.b_rows, (uint64_t)a.K, (uint64_t)a.ldb, BK, b_box_rows);
   else rc = np_make_tmap_2d(&tmB, a.B, 2, (uint64_t)a.b_rows, (uint64_t)a.N, (uint64_t)a.ldb, 64, BK);
   if (rc) return 200 + rc;
@@ -631,8 +905,9 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
   // 32-byte stores need every (row, 32-column chunk) address 32-byte aligned; destinations behind peer_base are
   // allocations of the symmetric heap (256-byte aligned)
   static const bool st32_on = !(getenv("NPB200_ST32") != nullptr && getenv("NPB200_ST32")[0] == '0');
-  p.st32 = st32_on && !a.out_f32 && a.epilogue != 1 && (a.ldc % 16 == 0) && (a.group_stride_c % 16 == 0) &&
+  p.st32 = st32_on && !a.out_f32 && (a.ldc % 16 == 0) && (a.group_stride_c % 16 == 0) &&
            (a.row_dst || (((uintptr_t)a.C) % 32 == 0));
+  p.st32_c2 = st32_on && a.ldc2 % 16 == 0 && a.N % 16 == 0 && ((uintptr_t)a.C2) % 32 == 0;
   if (a.push_src && a.push_n > 0) {
     if (a.push_n > 8 || (a.push_bytes & 15) || (((uintptr_t)a.push_src) & 15)) return 1;
     p.push_src = (const uint4*)a.push_src; p.push_vecs = a.push_bytes >> 4; p.push_n = a.push_n;
@@ -667,27 +942,29 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
   p.epoch_base = a.epoch_base;
   p.b_ready_flags = a.b_ready_flags; p.b_rows_per_flag = a.b_rows_per_flag;
 
-  constexpr int SMEM = STAGES * (TM * BK * 2 + BN * BK * 2) + 1024 + 256;
+  constexpr int SMEM = STAGES * (PAIR ? PAIR_STAGE_BYTES : BM * BK * 2 + BN * BK * 2) + 1024 + 256;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t e;
+    if constexpr (PAIR) e = cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    else e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
   }
-  if (g_num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  const int cap = a.max_ctas > 0 ? a.max_ctas : num_sms();
+  const int bn_out = a.epilogue == 1 ? BN / 2 : BN, tm = PAIR ? 2 * BM : BM;
+  const long long tiles = (long long)((a.M + tm - 1) / tm) * ((a.N + bn_out - 1) / bn_out) * (a.mode == 2 ? a.num_groups : 1);
+  if constexpr (PAIR) {
+    const long long pairs = tiles < cap / 2 ? tiles : cap / 2;
+    if (pairs <= 0) return 0;
+    gemm_bf16_pair_kernel<<<(int)(2 * pairs), GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmB2, p);
+  } else {
+    const int grid = (int)(tiles < cap ? tiles : cap);
+    if (grid <= 0) return 0;
+    gemm_bf16_kernel<BN, STAGES><<<grid, GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmB2, tmAloc, tmBloc, p);
   }
-  const int bn_out = a.epilogue == 1 ? BN / 2 : BN;
-  const int m_blocks = (a.M + TM - 1) / TM, n_blocks = (a.N + bn_out - 1) / bn_out;
-  const long long tiles = (long long)m_blocks * n_blocks * (a.mode == 2 ? a.num_groups : 1);
-  int cap = a.max_ctas > 0 ? a.max_ctas : g_num_sms;
-  int grid = (int)(tiles < cap ? tiles : cap);
-  if (grid <= 0) return 0;
-  gemm_bf16_kernel<BN, STAGES, MT><<<grid, 192, SMEM, stream>>>(tmA, tmB, tmB2, tmAloc, tmBloc, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
@@ -707,37 +984,29 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
     ctx_bound = true;
   }
   if ((a.lda % 8) || (a.ldb % 8) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15)) return 1;
-  int bn = a.bn;
+  // Which kernel. The pair kernel takes the forms without peer-arrival flags on B, pushes or split operands; row-grouped
+  // launches only when their tables come in pairs of 128-row blocks (`paired`).
+  const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
+                     (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
+  int bn = a.bn, mt = a.mt;
   if (a.epilogue == 1) bn = 256;
-  if (bn == 0) bn = (a.N >= 256 && (a.N % 256 == 0 || a.N >= 2048)) ? 256 : 128;
-  if (bn == 256) {
-    // 256 x 256 tiles where the form allows (no per-128-row-block tables, flags or pushes) and the problem has
-    // enough of them to occupy the SMs; NPB200_GEMM_MT=1 keeps the 128-row tiles
-    static const int mt_env = getenv("NPB200_GEMM_MT") ? atoi(getenv("NPB200_GEMM_MT")) : 0;
-    int mt = a.mt ? a.mt : mt_env;
-    const bool plain = a.mode != 1 && !a.row_dst && !a.ready_flags && !a.b_ready_flags && !a.push_src && !a.A_loc &&
-                       !a.B_loc && !a.done_counters && a.m_rot == 0 && a.n_rot == 0;
-    if (mt == 0) {
-      // A 256-row tile costs about 1.68 tiles of 128 rows (measured on B200: 8192^3 1354 -> 1610 TFLOP/s, 4096 x 32000
-      // x 2048 1282 -> 1444, 4096 x 2048 x 5632 1037 -> 1264), so it wins unless its coarser grain wastes the last wave
-      const int bn_out = a.epilogue == 1 ? 128 : 256;
-      const long long groups = a.mode == 2 ? a.num_groups : 1;
-      const long long nb = (a.N + bn_out - 1) / bn_out;
-      const long long tiles1 = (long long)((a.M + 127) / 128) * nb * groups;
-      const long long tiles2 = (long long)((a.M + 255) / 256) * nb * groups;
-      if (g_num_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-      }
-      const int sms = a.max_ctas > 0 ? a.max_ctas : (g_num_sms > 0 ? g_num_sms : 148);
-      const long long w1 = (tiles1 + sms - 1) / sms, w2 = (tiles2 + sms - 1) / sms;
-      mt = (plain && a.M >= 256 && 1.68 * (double)w2 < (double)w1) ? 2 : 1;
-    }
-    if (mt == 2 && plain) return launch_gemm<256, 3, 2>(a, (cudaStream_t)stream);
-    return launch_gemm<256, 4, 1>(a, (cudaStream_t)stream);
+  if (bn == 0 || (bn == 256 && mt == 0)) {
+    const int sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
+    const long long groups = a.mode == 2 ? a.num_groups : 1;
+    auto waves = [&](int tm, int tn, int units) {
+      const long long t = (long long)((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn) * groups;
+      return (double)((t + units - 1) / units);
+    };
+    const int n256 = a.epilogue == 1 ? 128 : 256;
+    const double c128 = (a.epilogue == 1 || a.bn == 256) ? 1e30 : COST_128 * waves(128, 128, sms);
+    const double c256 = COST_256 * waves(128, n256, sms);
+    const double cpair = (plain && a.M > 128 && sms >= 2 && mt != 1) ? COST_PAIR * waves(256, n256, sms / 2) : 1e30;
+    if (cpair <= c128 && cpair <= c256) { bn = 256; mt = 2; }
+    else bn = c256 <= c128 ? 256 : 128;
   }
-  return launch_gemm<128, 6, 1>(a, (cudaStream_t)stream);
+  if (bn == 256 && mt == 2 && plain) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream);
+  if (bn == 256) return launch_gemm<256, 4, false>(a, (cudaStream_t)stream);
+  return launch_gemm<128, 6, false>(a, (cudaStream_t)stream);
 }
 
 NP_API int np_status_read(int* out8) {

@@ -114,7 +114,9 @@ class FusedMoERuntime:
         self.E_local = num_experts // self.N
         self.capacity = int(capacity_factor * tokens / num_experts) if capacity_factor is not None else -1
         cap_rows = min(self.capacity, tokens) if self.capacity >= 0 else tokens
-        self.R = max(128, (cap_rows + 127) // 128 * 128)
+        # rows of a receive region: whole pairs of 128-row blocks once it holds more than one, so that the expert GEMMs
+        # can run 256-row tiles on pairs of CTAs (``paired`` below)
+        self.R = 128 if cap_rows <= 128 else (cap_rows + 255) // 256 * 256
         self.bpr = self.R // 128
         self.rows_total = self.E_local * self.N * self.R
         self.blocks = self.rows_total // 128
@@ -286,6 +288,7 @@ class FusedMoERuntime:
         g.M, g.N, g.K = M, N, K
         g.a_mn, g.b_mn = 0, int(b_mn)
         g.mode, g.alpha = 1, 1.0
+        g.paired = int(self.bpr % 2 == 0)
         g.mblk_group, g.mblk_rows = self.mblk_group.data_ptr(), self.mblk_rows.data_ptr()
         g.group_stride_b = group_stride_b
         g.mblk_flag = self.mblk_flag.data_ptr()
