@@ -19,9 +19,13 @@
 namespace {
 
 constexpr int KID_ATTN = 30;
-constexpr int BQ = 128, BKV = 128, HD = 128;
-constexpr int TILE_BYTES = 128 * 128 * 2;   // one [128 x 128] bf16 tile = two 64-column swizzled chunks
+constexpr int BQ = 128, BKV = 128;
 constexpr int CHUNK_BYTES = 128 * 64 * 2;
+// Every kernel is built for head dimensions 128 and 64 (template parameter HD): one [128 x HD] bf16 tile is HD / 64
+// 64-column swizzled chunks. With 64 the products over the head dimension take half the K steps, the products that
+// produce it half the columns, and all tiles half the bytes.
+template <int HD>
+constexpr int tile_bytes() { return 128 * HD * 2; }
 constexpr int MAX_SRC = 8;
 
 struct TmapList {
@@ -35,16 +39,17 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tm,
       ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-// [128 rows x 128 cols] tile (cols = hd) of head `h`, rows starting at `s0`, batch `b`: two 64-col chunks
+// [128 rows x HD cols] tile of head `h`, rows starting at `s0`, batch `b`: 64-col chunks
+template <int HD>
 __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int h, int s0, int b) {
-  tma_load_4d(dst, tm, bar, 0, h, s0, b);
-  tma_load_4d(dst + CHUNK_BYTES, tm, bar, 64, h, s0, b);
+#pragma unroll
+  for (int c = 0; c < HD / 64; ++c) tma_load_4d(dst + c * CHUNK_BYTES, tm, bar, c * 64, h, s0, b);
 }
-// K-major operand [rows, 128 k]: k-step kk (16 elements) -> chunk kk/4, +32 B per step inside the chunk
+// K-major operand [rows, HD k]: k-step kk (16 elements) -> chunk kk/4, +32 B per step inside the chunk
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t tile, int kk) {
   return np::make_smem_desc(tile + (kk >> 2) * CHUNK_BYTES + (kk & 3) * 32, 16, 1024);
 }
-// MN-major operand stored as [k rows, 128 mn cols] (two 64-col chunks): k-step = 16 rows = +2048 B,
+// MN-major operand stored as [k rows, HD mn cols] (64-col chunks): k-step = 16 rows = +2048 B,
 // LBO = distance between the two 64-wide chunks
 __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile, int kk) {
   return np::make_smem_desc(tile + kk * 2048, CHUNK_BYTES, 1024);
@@ -216,10 +221,11 @@ constexpr int F_KST = 3, F_VST = 3;   // three-deep K and V rings: a TMA load ha
 // Tensor memory map of the forward kernel (columns): S double buffer, O accumulator, P double buffer (bf16 pairs)
 constexpr uint32_t F_S = 0, F_O = 256, F_P = 384;
 
-template <int NS>
+template <int NS, int HD>
 __global__ void __launch_bounds__(nthreads(NS), 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ TmapList tmK,
                 const __grid_constant__ TmapList tmV, const FwdParams p) {
+  constexpr int TILE_BYTES = tile_bytes<HD>();
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t base = np::smem_u32(smem_al);
   if (base & 1023u) {   // the swizzled tiles need it; nothing has been allocated or started yet
@@ -270,7 +276,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (lane == 0) {
       if (!own_ready(p.fl, KID_ATTN)) *abort_flag = 1;
       np::mbar_expect_tx(B_(FB_Q), TILE_BYTES);
-      load_tile(sQ, &tmQ, B_(FB_Q), h, qb * BQ, b);
+      load_tile<HD>(sQ, &tmQ, B_(FB_Q), h, qb * BQ, b);
       int i = 0, last_src = -1;
       for (int j = next_vis(0); j < total_blocks && !*abort_flag; j = next_vis(j + 1), ++i) {
         const int ks = i % F_KST, vs = i % F_VST;
@@ -281,23 +287,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         if (!np::mbar_wait(B_(FB_KE + ks), ((uint32_t)(i / F_KST) & 1u) ^ 1u, abort_flag, KID_ATTN, 1)) break;
         np::mbar_expect_tx(B_(FB_K + ks), TILE_BYTES);
-        load_tile(sK0 + ks * TILE_BYTES, &tmK.m[src], B_(FB_K + ks), hkv, jb * BKV, b);
+        load_tile<HD>(sK0 + ks * TILE_BYTES, &tmK.m[src], B_(FB_K + ks), hkv, jb * BKV, b);
         if (!np::mbar_wait(B_(FB_VE + vs), ((uint32_t)(i / F_VST) & 1u) ^ 1u, abort_flag, KID_ATTN, 10)) break;
         np::mbar_expect_tx(B_(FB_V + vs), TILE_BYTES);
-        load_tile(sV0 + vs * TILE_BYTES, &tmV.m[src], B_(FB_V + vs), hkv, jb * BKV, b);
+        load_tile<HD>(sV0 + vs * TILE_BYTES, &tmV.m[src], B_(FB_V + vs), hkv, jb * BKV, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc_qk = np::make_idesc(128, 128, 1, 1, 0, 0);   // Q (K-major) x K (K-major)
-      const uint32_t idesc_pv = np::make_idesc(128, 128, 1, 1, 0, 1);   // P (TMEM) x V (MN-major)
+      const uint32_t idesc_pv = np::make_idesc(128, HD, 1, 1, 0, 1);   // P (TMEM) x V (MN-major)
       bool ok = np::mbar_wait(B_(FB_Q), 0, abort_flag, KID_ATTN, 2);
       auto issue_qk = [&](int i) {
         const int st = i & 1, ks = i % F_KST;
         if (!np::mbar_wait(B_(FB_K + ks), (uint32_t)(i / F_KST) & 1u, abort_flag, KID_ATTN, 3)) return false;
         np::tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           np::tc_mma_f16(tmem + F_S + st * 128, desc_kmajor(sQ, kk), desc_kmajor(sK0 + ks * TILE_BYTES, kk), idesc_qk, kk > 0);
         np::tc_commit(B_(FB_S + st));
         np::tc_commit(B_(FB_KE + ks));
@@ -324,7 +330,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else {
-    constexpr int CW = 128 / NS;
+    constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
     const int quarter = warp & 3, hf = (warp - 2) >> 2;     // this thread: row r, columns [CW hf, CW hf + CW)
     const int r = quarter * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
@@ -371,11 +377,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             ok = warp_wait(B_(FB_O), (uint32_t)(i - 1) & 1u, abort_flag, KID_ATTN, 8);   // P V of block i-1 is done
             if (ok) {
               np::tc_fence_after();
-              uint32_t t[CW];
-              tmem_ld_cols<CW>(tO + lane_off + hf * CW, t);
+              uint32_t t[OW];
+              tmem_ld_cols<OW>(tO + lane_off + hf * OW, t);
 #pragma unroll
-              for (int e = 0; e < CW; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * alpha);
-              tmem_st_cols<CW>(tO + lane_off + hf * CW, t);
+              for (int e = 0; e < OW; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * alpha);
+              tmem_st_cols<OW>(tO + lane_off + hf * OW, t);
             }
           }
           l *= alpha;
@@ -414,19 +420,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     ok = __all_sync(0xffffffffu, ok);
     const int row = qb * BQ + r;
     if (ok) {
-      uint32_t t[CW];
+      uint32_t t[OW];
       if (nvis > 0) {
         np::tc_fence_after();
-        tmem_ld_cols<CW>(tO + lane_off + hf * CW, t);
+        tmem_ld_cols<OW>(tO + lane_off + hf * OW, t);
       } else {
 #pragma unroll
-        for (int e = 0; e < CW; ++e) t[e] = 0u;
+        for (int e = 0; e < OW; ++e) t[e] = 0u;
       }
       if (row < p.Sq) {
         const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
-        __nv_bfloat16* dst = p.O + (size_t)b * p.o_sb + (size_t)row * p.o_ss + (size_t)h * p.o_sh + hf * CW;
+        __nv_bfloat16* dst = p.O + (size_t)b * p.o_sb + (size_t)row * p.o_ss + (size_t)h * p.o_sh + hf * OW;
 #pragma unroll
-        for (int g = 0; g < CW / 8; ++g) {
+        for (int g = 0; g < OW / 8; ++g) {
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(t[8 * g + e]) * inv;
@@ -469,9 +475,11 @@ __device__ unsigned long long g_fwd2_prof[8];
 #endif
 constexpr int G_KST = 3, G_VST = 2;   // Q0, Q1, three K stages, two V stages: seven 32 KB tiles
 
+template <int HD>
 __global__ void __launch_bounds__(320, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
+  constexpr int TILE_BYTES = tile_bytes<HD>();
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t base = np::smem_u32(smem_al);
   if (base & 1023u) {
@@ -520,28 +528,28 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 0) {
     if (lane == 0) {
       np::mbar_expect_tx(B_(G_Q), 2 * TILE_BYTES);
-      load_tile(sQ, &tmQ, B_(G_Q), h, row0, b);
-      load_tile(sQ + TILE_BYTES, &tmQ, B_(G_Q), h, row0 + BQ, b);   // rows past the end read as zero
+      load_tile<HD>(sQ, &tmQ, B_(G_Q), h, row0, b);
+      load_tile<HD>(sQ + TILE_BYTES, &tmQ, B_(G_Q), h, row0 + BQ, b);   // rows past the end read as zero
       for (int i = 0; i < nv && !*abort_flag; ++i) {
         const int ks = i % G_KST, vs = i % G_VST;
         if (!np::mbar_wait(B_(G_KE + ks), ((uint32_t)(i / G_KST) & 1u) ^ 1u, abort_flag, KID_ATTN, 21)) break;
         np::mbar_expect_tx(B_(G_K + ks), TILE_BYTES);
-        load_tile(sK0 + ks * TILE_BYTES, &tmK, B_(G_K + ks), hkv, i * BKV, b);
+        load_tile<HD>(sK0 + ks * TILE_BYTES, &tmK, B_(G_K + ks), hkv, i * BKV, b);
         if (!np::mbar_wait(B_(G_VE + vs), ((uint32_t)(i / G_VST) & 1u) ^ 1u, abort_flag, KID_ATTN, 22)) break;
         np::mbar_expect_tx(B_(G_V + vs), TILE_BYTES);
-        load_tile(sV0 + vs * TILE_BYTES, &tmV, B_(G_V + vs), hkv, i * BKV, b);
+        load_tile<HD>(sV0 + vs * TILE_BYTES, &tmV, B_(G_V + vs), hkv, i * BKV, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc_qk = np::make_idesc(128, 128, 1, 1, 0, 0);
-      const uint32_t idesc_pv = np::make_idesc(128, 128, 1, 1, 0, 1);
+      const uint32_t idesc_pv = np::make_idesc(128, HD, 1, 1, 0, 1);
       bool ok = np::mbar_wait(B_(G_Q), 0, abort_flag, KID_ATTN, 23);
       // S of tile t for block i (the K stage must have landed; the caller has waited for it)
       auto issue_s = [&](int t, int i) {
         const int ks = i % G_KST;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           np::tc_mma_f16(tmem + t * 128, desc_kmajor(sQ + t * TILE_BYTES, kk), desc_kmajor(sK0 + ks * TILE_BYTES, kk),
                          idesc_qk, kk > 0);
         np::tc_commit(B_(G_S + t));
@@ -649,7 +657,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (!ok) break;
           np::tc_fence_after();
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < HD / 32; ++c) {
             uint32_t o[32];
             tmem_ld_cols<32>(tO + c * 32, o);
 #pragma unroll
@@ -696,7 +704,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       __nv_bfloat16* dst = p.O + (size_t)b * p.o_sb + (size_t)row * p.o_ss + (size_t)h * p.o_sh;
       if (my_nv > 0) np::tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < HD / 32; ++c) {
         uint32_t o[32];
         if (my_nv > 0) {
           tmem_ld_cols<32>(tO + c * 32, o);
@@ -727,11 +735,11 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
-int make_tmap_4d(CUtensorMap* out, const void* base, long long B, long long S, long long H, long long sb, long long ss,
+int make_tmap_4d(CUtensorMap* out, const void* base, int hd, long long B, long long S, long long H, long long sb, long long ss,
                  long long sh) {
   NpEncodeTiledFn enc = np_get_encode_tiled();
   if (!enc) return -1;
-  cuuint64_t dims[4] = {(cuuint64_t)HD, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
+  cuuint64_t dims[4] = {(cuuint64_t)hd, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)sh * 2, (cuuint64_t)ss * 2, (cuuint64_t)sb * 2};
   cuuint32_t box[4] = {64, 1, 128, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -795,6 +803,7 @@ struct NpAttnFwdArgs {
   // then *push_flag[r] = flag_epoch (+ *epoch_base); push_ctr: two local ints the caller zeroes before the launch
   const void* push_k; const void* push_v; long long push_bytes; void* const* push_dst; int* const* push_flag;
   int push_n; int* push_ctr;
+  int head_dim;    // 128 (also when 0) or 64
 };
 
 #ifdef NP_ATTN_PROF
@@ -805,21 +814,60 @@ NP_API int np_attn_prof_read(unsigned long long* out8, int reset) {
 }
 #endif
 
+template <int HD>
+static int launch_fwd2(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const FwdParams& p,
+                       cudaStream_t stream) {
+  constexpr int SMEM = (2 + G_KST + G_VST) * tile_bytes<HD>() + 8 * G_COUNT + 8 + 16;
+  static_assert(SMEM <= 227 * 1024, "shared memory budget");
+  static NpPerDeviceOnce attr_once;
+  bool& attr_set = *attr_once.slot();
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(attn_fwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return 400 + (int)e;
+    attr_set = true;
+  }
+  dim3 grid(p.Hq * p.B, (p.Sq + 2 * BQ - 1) / (2 * BQ));
+  attn_fwd2_kernel<HD><<<grid, 320, SMEM, stream>>>(tmQ, tmK, tmV, p);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
+template <int HD>
+static int launch_fwd(const CUtensorMap& tmQ, const TmapList& tmK, const TmapList& tmV, const FwdParams& p,
+                      cudaStream_t stream) {
+  constexpr int NS = 2;   // softmax threads per row
+  constexpr int SMEM = (1 + F_KST + F_VST) * tile_bytes<HD>() + 8 * FB_COUNT + 8 + 16 + 2 * NS * 128 * 4 + 16;
+  static_assert(SMEM <= 227 * 1024, "shared memory budget");
+  static NpPerDeviceOnce attr_once;
+  bool& attr_set = *attr_once.slot();
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<NS, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return 400 + (int)e;
+    attr_set = true;
+  }
+  dim3 grid(p.Hq * p.B, (p.Sq + BQ - 1) / BQ);
+  attn_fwd_kernel<NS, HD><<<grid, nthreads(NS), SMEM, stream>>>(tmQ, tmK, tmV, p);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
 NP_API int np_attn_fwd(const NpAttnFwdArgs* a, void* stream) {
   if (a->B <= 0 || a->Sq <= 0 || a->src_len <= 0) return 0;
   if (a->n_src < 1 || a->n_src > MAX_SRC || a->Hq % a->Hkv) return 1;
+  const int hd = a->head_dim ? a->head_dim : 128;
+  if (hd != 128 && hd != 64) return 1;
   if ((a->q_ss | a->q_sh | a->q_sb | a->k_ss | a->k_sh | a->k_sb | a->o_ss | a->o_sh | a->o_sb) % 8 ||
       (((uintptr_t)a->q | (uintptr_t)a->o) & 15))
     return 1;
   if (!bind_ctx()) return 2;
   CUtensorMap tmQ;
   TmapList tmK, tmV;
-  int rc = make_tmap_4d(&tmQ, a->q, a->B, a->Sq, a->Hq, a->q_sb, a->q_ss, a->q_sh);
+  int rc = make_tmap_4d(&tmQ, a->q, hd, a->B, a->Sq, a->Hq, a->q_sb, a->q_ss, a->q_sh);
   if (rc) return 100 + rc;
   for (int s = 0; s < a->n_src; ++s) {
-    rc = make_tmap_4d(&tmK.m[s], a->k_ptrs[s], a->B, a->src_len, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
+    rc = make_tmap_4d(&tmK.m[s], a->k_ptrs[s], hd, a->B, a->src_len, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
     if (rc) return 200 + rc;
-    rc = make_tmap_4d(&tmV.m[s], a->v_ptrs[s], a->B, a->src_len, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
+    rc = make_tmap_4d(&tmV.m[s], a->v_ptrs[s], hd, a->B, a->src_len, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
     if (rc) return 300 + rc;
   }
   for (int s = a->n_src; s < MAX_SRC; ++s) { tmK.m[s] = tmK.m[0]; tmV.m[s] = tmV.m[0]; }
@@ -837,34 +885,11 @@ NP_API int np_attn_fwd(const NpAttnFwdArgs* a, void* stream) {
   static const bool fwd2_on = [] { const char* e = getenv("NPB200_ATTN_FWD2"); return !(e && e[0] == '0'); }();
   if (fwd2_on && a->n_src == 1 && !a->src_flags && !a->push_k && !a->q_blk_pos && !a->k_blk_pos && a->flag_own == 0 &&
       a->Sq > BQ) {
-    constexpr int SMEM2 = (2 + G_KST + G_VST) * TILE_BYTES + 8 * G_COUNT + 8 + 16;
-    static_assert(SMEM2 <= 227 * 1024, "shared memory budget");
-    static NpPerDeviceOnce attr2_once;
-    bool& attr2_set = *attr2_once.slot();
-    if (!attr2_set) {
-      cudaError_t e = cudaFuncSetAttribute(attn_fwd2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2);
-      if (e != cudaSuccess) return 400 + (int)e;
-      attr2_set = true;
-    }
-    dim3 grid2(a->Hq * a->B, (a->Sq + 2 * BQ - 1) / (2 * BQ));
-    attn_fwd2_kernel<<<grid2, 320, SMEM2, (cudaStream_t)stream>>>(tmQ, tmK.m[0], tmV.m[0], p);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? 0 : 500 + (int)e;
+    return hd == 128 ? launch_fwd2<128>(tmQ, tmK.m[0], tmV.m[0], p, (cudaStream_t)stream)
+                     : launch_fwd2<64>(tmQ, tmK.m[0], tmV.m[0], p, (cudaStream_t)stream);
   }
-  constexpr int NS = 2;   // softmax threads per row
-  constexpr int SMEM = (1 + F_KST + F_VST) * TILE_BYTES + 8 * FB_COUNT + 8 + 16 + 2 * NS * 128 * 4 + 16;
-  static_assert(SMEM <= 227 * 1024, "shared memory budget");
-  static NpPerDeviceOnce attr_once;
-  bool& attr_set = *attr_once.slot();
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return 400 + (int)e;
-    attr_set = true;
-  }
-  dim3 grid(a->Hq * a->B, (a->Sq + BQ - 1) / BQ);
-  attn_fwd_kernel<NS><<<grid, nthreads(NS), SMEM, (cudaStream_t)stream>>>(tmQ, tmK, tmV, p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 500 + (int)e;
+  return hd == 128 ? launch_fwd<128>(tmQ, tmK, tmV, p, (cudaStream_t)stream)
+                   : launch_fwd<64>(tmQ, tmK, tmV, p, (cudaStream_t)stream);
 }
 
 // ====================================================================================== backward
@@ -904,18 +929,33 @@ struct BwdParams {
   __nv_bfloat16* dK; __nv_bfloat16* dV; long long dk_sb, dk_ss, dk_sh;
 };
 
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
-                                  const __nv_bfloat16* __restrict__ d_o, long long d_sb, long long d_ss, long long d_sh,
-                                  float* __restrict__ delta, int B, int S, int H) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= B * S * H) return;
-  const int h = w % H, s = (w / H) % S, b = w / (H * S);
-  const uint2 a = *reinterpret_cast<const uint2*>(o + (size_t)b * o_sb + (size_t)s * o_ss + (size_t)h * o_sh + lane * 4);
-  const uint2 g = *reinterpret_cast<const uint2*>(d_o + (size_t)b * d_sb + (size_t)s * d_ss + (size_t)h * d_sh + lane * 4);
-  const float2 a0 = np::unpack_bf16(a.x), a1 = np::unpack_bf16(a.y), g0 = np::unpack_bf16(g.x), g1 = np::unpack_bf16(g.y);
-  float v = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y;
-  v = np::warp_sum(v);
-  if (lane == 0) delta[((size_t)b * H + h) * S + s] = v;
+// delta[b, h, s] = sum over the head dimension of o * d_o: HD / 8 lanes per row, 16 bytes of each tensor per lane
+template <int HD>
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
+                  const __nv_bfloat16* __restrict__ d_o, long long d_sb, long long d_ss, long long d_sh,
+                  float* __restrict__ delta, int B, int S, int H) {
+  constexpr int L = HD / 8;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long n = (long long)B * S * H, w = t / L;
+  const int lane = (int)(t % L);
+  float v = 0.f;
+  int h = 0, sq = 0, b = 0;
+  if (w < n) {
+    h = (int)(w % H); sq = (int)((w / H) % S); b = (int)(w / ((long long)H * S));
+    const uint4 a = *reinterpret_cast<const uint4*>(o + (size_t)b * o_sb + (size_t)sq * o_ss + (size_t)h * o_sh + lane * 8);
+    const uint4 g = *reinterpret_cast<const uint4*>(d_o + (size_t)b * d_sb + (size_t)sq * d_ss + (size_t)h * d_sh + lane * 8);
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = np::unpack_bf16(aw[i]), y = np::unpack_bf16(gw[i]);
+      v = fmaf(x.x, y.x, v);
+      v = fmaf(x.y, y.y, v);
+    }
+  }
+#pragma unroll
+  for (int m = L / 2; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+  if (w < n && lane == 0) delta[((size_t)b * H + h) * S + sq] = v;
 }
 
 enum { QB_QDO = 0, QB_K = 1, QB_KE = 4, QB_V = 7, QB_VE = 9, QB_S = 11, QB_DP = 13, QB_DS = 14, QB_FIN = 15, QB_COUNT = 16 };
@@ -923,10 +963,11 @@ enum { QB_QDO = 0, QB_K = 1, QB_KE = 4, QB_V = 7, QB_VE = 9, QB_S = 11, QB_DP = 
 constexpr int Q_KST = 3, Q_VST = 2;
 constexpr int BWD_TILES = 7;   // seven 32 KB tiles: the dynamic shared memory must itself start on a 1024-byte boundary
 
-template <int NS>
+template <int NS, int HD>
 __global__ void __launch_bounds__(nthreads(NS), 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                    const __grid_constant__ TmapList tmK, const __grid_constant__ TmapList tmV, const BwdParams p) {
+  constexpr int TILE_BYTES = tile_bytes<HD>();
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t base = np::smem_u32(smem_al);
   if (base & 1023u) {   // the swizzled tiles need it; nothing has been allocated or started yet
@@ -973,8 +1014,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (lane == 0) {
       if (!own_ready(p.fl, KID_ATTN_DQ)) *abort_flag = 1;
       np::mbar_expect_tx(B_(QB_QDO), 2 * TILE_BYTES);
-      load_tile(sQ, &tmQ, B_(QB_QDO), h, qb * BQ, b);
-      load_tile(sdO, &tmdO, B_(QB_QDO), h, qb * BQ, b);
+      load_tile<HD>(sQ, &tmQ, B_(QB_QDO), h, qb * BQ, b);
+      load_tile<HD>(sdO, &tmdO, B_(QB_QDO), h, qb * BQ, b);
       int i = 0, last_src = -1;
       for (int j = next_vis(0); j < total_blocks && !*abort_flag; j = next_vis(j + 1), ++i) {
         const int ks = i % Q_KST, vs = i % Q_VST;
@@ -985,23 +1026,23 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
         if (!np::mbar_wait(B_(QB_KE + ks), ((uint32_t)(i / Q_KST) & 1u) ^ 1u, abort_flag, KID_ATTN_DQ, 1)) break;
         np::mbar_expect_tx(B_(QB_K + ks), TILE_BYTES);
-        load_tile(sK0 + ks * TILE_BYTES, &tmK.m[src], B_(QB_K + ks), hkv, jb * BKV, b);
+        load_tile<HD>(sK0 + ks * TILE_BYTES, &tmK.m[src], B_(QB_K + ks), hkv, jb * BKV, b);
         if (!np::mbar_wait(B_(QB_VE + vs), ((uint32_t)(i / Q_VST) & 1u) ^ 1u, abort_flag, KID_ATTN_DQ, 10)) break;
         np::mbar_expect_tx(B_(QB_V + vs), TILE_BYTES);
-        load_tile(sV0 + vs * TILE_BYTES, &tmV.m[src], B_(QB_V + vs), hkv, jb * BKV, b);
+        load_tile<HD>(sV0 + vs * TILE_BYTES, &tmV.m[src], B_(QB_V + vs), hkv, jb * BKV, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);   // both operands K-major (over hd)
-      const uint32_t idesc_mn = np::make_idesc(128, 128, 1, 1, 0, 1);   // A from TMEM, B MN-major
+      const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);   // A from TMEM, B MN-major
       bool ok = np::mbar_wait(B_(QB_QDO), 0, abort_flag, KID_ATTN_DQ, 2);
       auto issue_s = [&](int i) {
         const int st = i & 1, ks = i % Q_KST;
         if (!np::mbar_wait(B_(QB_K + ks), (uint32_t)(i / Q_KST) & 1u, abort_flag, KID_ATTN_DQ, 3)) return false;
         np::tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           np::tc_mma_f16(tmem + st * 128, desc_kmajor(sQ, kk), desc_kmajor(sK0 + ks * TILE_BYTES, kk), idesc_kk, kk > 0);
         np::tc_commit(B_(QB_S + st));
         return true;
@@ -1011,7 +1052,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!np::mbar_wait(B_(QB_V + vs), (uint32_t)(i / Q_VST) & 1u, abort_flag, KID_ATTN_DQ, 4)) return false;
         np::tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           np::tc_mma_f16(tdP, desc_kmajor(sdO, kk), desc_kmajor(sV0 + vs * TILE_BYTES, kk), idesc_kk, kk > 0);
         np::tc_commit(B_(QB_DP));
         np::tc_commit(B_(QB_VE + vs));
@@ -1035,7 +1076,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       np::tc_commit(B_(QB_FIN));
     }
   } else {
-    constexpr int CW = 128 / NS;
+    constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
     const int quarter = warp & 3, hf = (warp - 2) >> 2;     // this thread: row r, KV columns [CW hf, CW hf + CW)
     const int r = quarter * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
@@ -1093,18 +1134,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     ok = __all_sync(0xffffffffu, ok && !*abort_flag) && warp_wait(B_(QB_FIN), 0, abort_flag, KID_ATTN_DQ, 9);
     if (ok) {   // warp-uniform: the tensor-memory loads are executed by whole warps, only the stores are guarded
-      uint32_t t[CW];
+      uint32_t t[OW];
       if (nvis > 0) {
         np::tc_fence_after();
-        tmem_ld_cols<CW>(tdQ + lane_off + hf * CW, t);
+        tmem_ld_cols<OW>(tdQ + lane_off + hf * OW, t);
       } else {
 #pragma unroll
-        for (int e = 0; e < CW; ++e) t[e] = 0u;
+        for (int e = 0; e < OW; ++e) t[e] = 0u;
       }
       if (row < p.Sq) {
-        __nv_bfloat16* dst = p.dQ + (size_t)b * p.dq_sb + (size_t)row * p.dq_ss + (size_t)h * p.dq_sh + hf * CW;
+        __nv_bfloat16* dst = p.dQ + (size_t)b * p.dq_sb + (size_t)row * p.dq_ss + (size_t)h * p.dq_sh + hf * OW;
 #pragma unroll
-        for (int g = 0; g < CW / 8; ++g) {
+        for (int g = 0; g < OW / 8; ++g) {
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(t[8 * g + e]) * p.scale;
@@ -1128,10 +1169,11 @@ enum { KB_KV = 0, KB_Q = 1, KB_QE = 4, KB_DO = 7, KB_DOE = 9, KB_ST = 11, KB_DPT
 // dV += P^T dO: two.
 constexpr int K_QST = 3, K_DOST = 2;
 
-template <int NS>
+template <int NS, int HD>
 __global__ void __launch_bounds__(nthreads(NS), 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const __grid_constant__ TmapList tmQ, const __grid_constant__ TmapList tmdO, const BwdParams p) {
+  constexpr int TILE_BYTES = tile_bytes<HD>();
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t base = np::smem_u32(smem_al);
   if (base & 1023u) {   // the swizzled tiles need it; nothing has been allocated or started yet
@@ -1187,8 +1229,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     if (lane == 0) {
       if (!own_ready(p.fl, KID_ATTN_DKV)) *abort_flag = 1;
       np::mbar_expect_tx(B_(KB_KV), 2 * TILE_BYTES);
-      load_tile(sK, &tmK, B_(KB_KV), hkv, jb * BKV, b);
-      load_tile(sV, &tmV, B_(KB_KV), hkv, jb * BKV, b);
+      load_tile<HD>(sK, &tmK, B_(KB_KV), hkv, jb * BKV, b);
+      load_tile<HD>(sV, &tmV, B_(KB_KV), hkv, jb * BKV, b);
       int i = 0, last_src = -1;
       for (int c = next_vis(0); c < total && !*abort_flag; c = next_vis(c + 1), ++i) {
         const int qs = i % K_QST, ds = i % K_DOST;
@@ -1199,23 +1241,23 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
         if (!np::mbar_wait(B_(KB_QE + qs), ((uint32_t)(i / K_QST) & 1u) ^ 1u, abort_flag, KID_ATTN_DKV, 1)) break;
         np::mbar_expect_tx(B_(KB_Q + qs), TILE_BYTES);
-        load_tile(sQ0 + qs * TILE_BYTES, &tmQ.m[src], B_(KB_Q + qs), h, qi * BQ, b);
+        load_tile<HD>(sQ0 + qs * TILE_BYTES, &tmQ.m[src], B_(KB_Q + qs), h, qi * BQ, b);
         if (!np::mbar_wait(B_(KB_DOE + ds), ((uint32_t)(i / K_DOST) & 1u) ^ 1u, abort_flag, KID_ATTN_DKV, 2)) break;
         np::mbar_expect_tx(B_(KB_DO + ds), TILE_BYTES);
-        load_tile(sdO0 + ds * TILE_BYTES, &tmdO.m[src], B_(KB_DO + ds), h, qi * BQ, b);
+        load_tile<HD>(sdO0 + ds * TILE_BYTES, &tmdO.m[src], B_(KB_DO + ds), h, qi * BQ, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);
-      const uint32_t idesc_mn = np::make_idesc(128, 128, 1, 1, 0, 1);
+      const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);
       bool ok = np::mbar_wait(B_(KB_KV), 0, abort_flag, KID_ATTN_DKV, 3);
       auto issue_st = [&](int i) {
         const int qs = i % K_QST;
         if (!np::mbar_wait(B_(KB_Q + qs), (uint32_t)(i / K_QST) & 1u, abort_flag, KID_ATTN_DKV, 4)) return false;
         np::tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           np::tc_mma_f16(tSt, desc_kmajor(sK, kk), desc_kmajor(sQ0 + qs * TILE_BYTES, kk), idesc_kk, kk > 0);
         np::tc_commit(B_(KB_ST));
         return true;
@@ -1225,7 +1267,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         if (!np::mbar_wait(B_(KB_DO + ds), (uint32_t)(i / K_DOST) & 1u, abort_flag, KID_ATTN_DKV, 5)) return false;
         np::tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           np::tc_mma_f16(tdPt, desc_kmajor(sV, kk), desc_kmajor(sdO0 + ds * TILE_BYTES, kk), idesc_kk, kk > 0);
         np::tc_commit(B_(KB_DPT));
         return true;
@@ -1255,7 +1297,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       np::tc_commit(B_(KB_FIN));
     }
   } else {
-    constexpr int CW = 128 / NS;
+    constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
     const int quarter = warp & 3, hf = (warp - 2) >> 2;   // this thread: KV row r, Q columns [CW hf, CW hf + CW)
     const int r = quarter * 32 + lane;
     const int t256 = threadIdx.x - 64;                    // index among the softmax threads
@@ -1343,21 +1385,21 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     const int row = jb * BKV + r;
     if (ok) {   // warp-uniform; only the stores are guarded by the row bound
       np::tc_fence_after();
-      const size_t off = (size_t)b * p.dk_sb + (size_t)row * p.dk_ss + (size_t)hkv * p.dk_sh + hf * CW;
+      const size_t off = (size_t)b * p.dk_sb + (size_t)row * p.dk_ss + (size_t)hkv * p.dk_sh + hf * OW;
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
         __nv_bfloat16* dst = (which ? p.dK : p.dV) + off;
         const float mul = which ? p.scale : 1.f;
-        uint32_t t[CW];
+        uint32_t t[OW];
         if (nvis > 0) {
-          tmem_ld_cols<CW>((which ? tdK : tdV) + lane_off + hf * CW, t);
+          tmem_ld_cols<OW>((which ? tdK : tdV) + lane_off + hf * OW, t);
         } else {
 #pragma unroll
-          for (int e = 0; e < CW; ++e) t[e] = 0u;
+          for (int e = 0; e < OW; ++e) t[e] = 0u;
         }
         if (row < p.Sk) {
 #pragma unroll
-          for (int g = 0; g < CW / 8; ++g) {
+          for (int g = 0; g < OW / 8; ++g) {
             float f[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(t[8 * g + e]) * mul;
@@ -1409,16 +1451,42 @@ struct NpAttnBwdArgs {
   // K|V shard pushed by the dQ kernel itself (as in NpAttnFwdArgs)
   const void* push_k; const void* push_v; long long push_bytes; void* const* push_dst; int* const* push_flag;
   int push_n; int* push_ctr;
+  int head_dim;    // 128 (also when 0) or 64
 };
+
+template <int NS, int HD>
+static int launch_bwd(dim3 gq, dim3 gk, int skip, const CUtensorMap& tmQ, const CUtensorMap& tmdO, const CUtensorMap& tmK,
+                      const CUtensorMap& tmV, const TmapList& lK, const TmapList& lV, const TmapList& lQ,
+                      const TmapList& ldO, const BwdParams& pq, const BwdParams& pk, cudaStream_t stream) {
+  constexpr int SMEM_DQ = BWD_TILES * tile_bytes<HD>() + 8 * QB_COUNT + 16 + 16;
+  constexpr int SMEM_DKV = BWD_TILES * tile_bytes<HD>() + 8 * KB_COUNT + 16 + 2048 + 16;
+  static_assert(SMEM_DKV <= 227 * 1024, "shared memory budget");
+  static NpPerDeviceOnce attr_once;
+  bool& attr_set = *attr_once.slot();
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(attn_bwd_dq_kernel<NS, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DQ);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<NS, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DKV);
+    if (e != cudaSuccess) return 400 + (int)e;
+    attr_set = true;
+  }
+  if (!(skip & 1)) attn_bwd_dq_kernel<NS, HD><<<gq, nthreads(NS), SMEM_DQ, stream>>>(tmQ, tmdO, lK, lV, pq);
+  if (!(skip & 2)) attn_bwd_dkv_kernel<NS, HD><<<gk, nthreads(NS), SMEM_DKV, stream>>>(tmK, tmV, lQ, ldO, pk);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
 
 NP_API int np_attn_bwd(const NpAttnBwdArgs* a, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   if (a->B <= 0 || a->Sq <= 0 || a->Sk <= 0) return 0;
   if (a->n_src < 1 || a->n_src > MAX_SRC || a->Hq % a->Hkv) return 1;
+  const int hd = a->head_dim ? a->head_dim : 128;
+  if (hd != 128 && hd != 64) return 1;
   if (!bind_ctx()) return 2;
   if (a->phase & 1) {
-    const long long warps = (long long)a->B * a->Sq * a->Hq;
-    attn_delta_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, stream>>>(
+    const long long lanes = (long long)a->B * a->Sq * a->Hq * (hd / 8);
+    auto kern = hd == 128 ? attn_delta_kernel<128> : attn_delta_kernel<64>;
+    kern<<<(unsigned)((lanes + 255) / 256), 256, 0, stream>>>(
         (const __nv_bfloat16*)a->o, a->o_sb, a->o_ss, a->o_sh, (const __nv_bfloat16*)a->d_o, a->do_sb, a->do_ss, a->do_sh,
         a->delta, a->B, a->Sq, a->Hq);
   }
@@ -1426,15 +1494,15 @@ NP_API int np_attn_bwd(const NpAttnBwdArgs* a, void* stream_) {
   const int qblocks = (a->Sq + BQ - 1) / BQ, kblocks = (a->Sk + BKV - 1) / BKV;
   CUtensorMap tmQ, tmdO, tmK, tmV;
   TmapList lK, lV, lQ, ldO;
-  int rc = make_tmap_4d(&tmQ, a->q, a->B, a->Sq, a->Hq, a->q_sb, a->q_ss, a->q_sh);
-  rc = rc ? rc : make_tmap_4d(&tmdO, a->d_o, a->B, a->Sq, a->Hq, a->do_sb, a->do_ss, a->do_sh);
-  rc = rc ? rc : make_tmap_4d(&tmK, a->k, a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
-  rc = rc ? rc : make_tmap_4d(&tmV, a->v, a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
+  int rc = make_tmap_4d(&tmQ, a->q, hd, a->B, a->Sq, a->Hq, a->q_sb, a->q_ss, a->q_sh);
+  rc = rc ? rc : make_tmap_4d(&tmdO, a->d_o, hd, a->B, a->Sq, a->Hq, a->do_sb, a->do_ss, a->do_sh);
+  rc = rc ? rc : make_tmap_4d(&tmK, a->k, hd, a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
+  rc = rc ? rc : make_tmap_4d(&tmV, a->v, hd, a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
   for (int s = 0; s < a->n_src && !rc; ++s) {
-    rc = make_tmap_4d(&lK.m[s], a->k_src[s], a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
-    rc = rc ? rc : make_tmap_4d(&lV.m[s], a->v_src[s], a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
-    rc = rc ? rc : make_tmap_4d(&lQ.m[s], a->q_src[s], a->B, a->Sq, a->Hq, a->q_sb, a->q_ss, a->q_sh);
-    rc = rc ? rc : make_tmap_4d(&ldO.m[s], a->do_src[s], a->B, a->Sq, a->Hq, a->do_sb, a->do_ss, a->do_sh);
+    rc = make_tmap_4d(&lK.m[s], a->k_src[s], hd, a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
+    rc = rc ? rc : make_tmap_4d(&lV.m[s], a->v_src[s], hd, a->B, a->Sk, a->Hkv, a->k_sb, a->k_ss, a->k_sh);
+    rc = rc ? rc : make_tmap_4d(&lQ.m[s], a->q_src[s], hd, a->B, a->Sq, a->Hq, a->q_sb, a->q_ss, a->q_sh);
+    rc = rc ? rc : make_tmap_4d(&ldO.m[s], a->do_src[s], hd, a->B, a->Sq, a->Hq, a->do_sb, a->do_ss, a->do_sh);
   }
   if (rc) return 100 + rc;
   for (int s = a->n_src; s < MAX_SRC; ++s) { lK.m[s] = lK.m[0]; lV.m[s] = lV.m[0]; lQ.m[s] = lQ.m[0]; ldO.m[s] = ldO.m[0]; }
@@ -1451,19 +1519,6 @@ NP_API int np_attn_bwd(const NpAttnBwdArgs* a, void* stream_) {
     p.lse_src.p[s] = a->lse_src[s < a->n_src ? s : 0];
     p.delta_src.p[s] = a->delta_src[s < a->n_src ? s : 0];
   }
-  constexpr int SMEM_DQ = BWD_TILES * TILE_BYTES + 8 * QB_COUNT + 16 + 16;
-  constexpr int SMEM_DKV = BWD_TILES * TILE_BYTES + 8 * KB_COUNT + 16 + 2048 + 16;
-  static_assert(SMEM_DKV <= 227 * 1024, "shared memory budget");
-  static NpPerDeviceOnce attr_once;
-  bool& attr_set = *attr_once.slot();
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_dq_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DQ);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_bwd_dq_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DQ);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DKV);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DKV);
-    if (e != cudaSuccess) return 400 + (int)e;
-    attr_set = true;
-  }
   // dQ: local Q blocks against every source's KV blocks
   BwdParams pq = p;
   pq.src_blocks = kblocks; pq.src_len = a->Sk;
@@ -1478,13 +1533,7 @@ NP_API int np_attn_bwd(const NpAttnBwdArgs* a, void* stream_) {
   fill_flags(&pk.fl, (a->flag_which & 2) ? a->src_flags : nullptr, a->flag_idx, a->n_src, a->flag_epoch, a->epoch_base,
              a->flag_limit_ns, a->flag_own - 1);
   const dim3 gq(a->Hq * a->B, qblocks), gk(a->Hkv * a->B, kblocks);
-  if (a->split == 4) {
-    if (!(a->skip & 1)) attn_bwd_dq_kernel<4><<<gq, nthreads(4), SMEM_DQ, stream>>>(tmQ, tmdO, lK, lV, pq);
-    if (!(a->skip & 2)) attn_bwd_dkv_kernel<4><<<gk, nthreads(4), SMEM_DKV, stream>>>(tmK, tmV, lQ, ldO, pk);
-  } else {
-    if (!(a->skip & 1)) attn_bwd_dq_kernel<2><<<gq, nthreads(2), SMEM_DQ, stream>>>(tmQ, tmdO, lK, lV, pq);
-    if (!(a->skip & 2)) attn_bwd_dkv_kernel<2><<<gk, nthreads(2), SMEM_DKV, stream>>>(tmK, tmV, lQ, ldO, pk);
-  }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 500 + (int)e;
+  if (hd == 64) return launch_bwd<2, 64>(gq, gk, a->skip, tmQ, tmdO, tmK, tmV, lK, lV, lQ, ldO, pq, pk, stream);
+  if (a->split == 4) return launch_bwd<4, 128>(gq, gk, a->skip, tmQ, tmdO, tmK, tmV, lK, lV, lQ, ldO, pq, pk, stream);
+  return launch_bwd<2, 128>(gq, gk, a->skip, tmQ, tmdO, tmK, tmV, lK, lV, lQ, ldO, pq, pk, stream);
 }

@@ -90,11 +90,12 @@ class AttnFwdArgs(C.Structure):
         ("src_len", c_int), ("q_off", c_int),
         ("scale", c_float),
         ("q_blk_pos", c_void_p), ("k_blk_pos", c_void_p),
-        ("split", c_int), ("lse_heads", c_int),
+        ("lse_heads", c_int),
         ("src_flags", c_void_p), ("flag_idx", c_void_p), ("flag_epoch", c_int), ("epoch_base", c_void_p),
         ("flag_limit_ns", c_ull), ("flag_own", c_int),
         ("push_k", c_void_p), ("push_v", c_void_p), ("push_bytes", c_ll), ("push_dst", c_void_p),
         ("push_flag", c_void_p), ("push_n", c_int), ("push_ctr", c_void_p),
+        ("head_dim", c_int),
     ]
 
 
@@ -116,11 +117,12 @@ class AttnBwdArgs(C.Structure):
         ("scale", c_float),
         ("q_blk_pos_local", c_void_p), ("k_blk_pos_all", c_void_p),
         ("k_blk_pos_local", c_void_p), ("q_blk_pos_all", c_void_p),
-        ("split", c_int), ("lse_heads", c_int),
+        ("lse_heads", c_int),
         ("src_flags", c_void_p), ("flag_idx", c_void_p), ("flag_epoch", c_int), ("epoch_base", c_void_p),
         ("flag_limit_ns", c_ull), ("flag_which", c_int), ("skip", c_int), ("flag_own", c_int),
         ("push_k", c_void_p), ("push_v", c_void_p), ("push_bytes", c_ll), ("push_dst", c_void_p),
         ("push_flag", c_void_p), ("push_n", c_int), ("push_ctr", c_void_p),
+        ("head_dim", c_int),
     ]
 
 

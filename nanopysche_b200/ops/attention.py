@@ -6,9 +6,10 @@ Returns the log-sum-exp as well when asked, which the context-parallel ring uses
 results (the reference sums per-chunk softmax outputs with no LSE merge,
 distributed/context_parallel.py:307-317).
 
-On bf16 CUDA tensors with head_dim 128 attention runs on this library's tcgen05 flash kernels
+On bf16 CUDA tensors with head_dim 128 or 64 attention runs on this library's tcgen05 flash kernels
 (csrc/attn_sm100.cu: forward, dQ and dK/dV kernels; scores, probabilities and the output accumulator live
-in tensor memory); other shapes and the CPU use PyTorch SDPA. The explicit-position fp32 form below is the
+in tensor memory), other head dims below 128 on the same kernels with the head dimension zero-padded; other shapes and
+the CPU use PyTorch SDPA. The explicit-position fp32 form below is the
 oracle of the kernels and the CPU path of ring attention.
 """
 from __future__ import annotations
@@ -100,10 +101,15 @@ def _set_flags(a, flags, keep: list):
 
 
 def flash_supported(q: torch.Tensor, k: torch.Tensor) -> bool:
-    """The tcgen05 kernels cover bf16, head_dim 128, 16-byte aligned strided ``[B, S, H, 128]`` views."""
+    """The tcgen05 kernels cover bf16, head_dim 128, 16-byte aligned strided ``[B, S, H, 128]`` views (the
+    context-parallel forms are built for this head dim)."""
     return (_lib.on(q) and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and q.shape[-1] == 128
             and k.shape[-1] == 128 and q.stride(-1) == 1 and k.stride(-1) == 1 and _lib.available()
             and all(s % 8 == 0 for s in q.stride()[:3]) and all(s % 8 == 0 for s in k.stride()[:3]))
+
+
+def _rows_aligned(t: torch.Tensor) -> bool:
+    return t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 and s != 0 for s in t.stride()[:3])
 
 
 def flash_fwd(q, k_list, v_list, *, causal=True, scale=None, q_off=0, q_blk_pos=None, k_blk_pos=None, split=0,
@@ -132,7 +138,7 @@ def flash_fwd(q, k_list, v_list, *, causal=True, scale=None, q_off=0, q_blk_pos=
     a.o_sb, a.o_ss, a.o_sh = _strides3(o)
     a.lse = lse.data_ptr()
     a.B, a.Sq, a.Hq, a.Hkv, a.causal, a.n_src, a.src_len, a.q_off = B, Sq, Hq, Hkv, int(causal), n, Sk, q_off
-    a.scale = scale or 1.0 / math.sqrt(hd)
+    a.scale, a.head_dim = scale or 1.0 / math.sqrt(hd), hd
     a.q_blk_pos = q_blk_pos.data_ptr() if q_blk_pos is not None else None
     a.k_blk_pos = k_blk_pos.data_ptr() if k_blk_pos is not None else None
     a.split = split
@@ -164,8 +170,8 @@ def flash_bwd(q, k, v, o, d_o, lse, *, causal=True, scale=None, q_off=0, delta=N
     Sk, Hkv = k.shape[1], k.shape[2]
     if delta is None:
         delta = torch.empty((B, Hq, Sq), device=q.device, dtype=torch.float32)
-    if d_o.stride(3) != 1 or any(s % 8 for s in d_o.stride()[:3]):
-        d_o = d_o.contiguous()
+    # dO is read through a tensor map, O by 16-byte loads: strided views of 16-byte aligned rows, no broadcast dimension
+    d_o, o = (t if _rows_aligned(t) else t.clone(memory_format=torch.contiguous_format) for t in (d_o, o))
     # ``out``: optional (dq, dk, dv) destinations (tensors or raw device pointers, layouts of q / k); ``skip``:
     # 1 = no dQ kernel, 2 = no dK/dV kernel
     dq = dk = dv = None
@@ -200,7 +206,7 @@ def flash_bwd(q, k, v, o, d_o, lse, *, causal=True, scale=None, q_off=0, delta=N
     a.k_src, a.v_src, a.q_src, a.do_src, a.lse_src, a.delta_src = [x[1] for x in keep]
     a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.causal, a.n_src, a.q_off, a.phase = \
         B, Sq, Sk, Hq, Hkv, int(causal), n_src, q_off, phase
-    a.scale = scale or 1.0 / math.sqrt(hd)
+    a.scale, a.head_dim = scale or 1.0 / math.sqrt(hd), hd
     a.split, a.skip = split, skip
     _set_flags(a, flags, keep)
     for name, t in (("q_blk_pos_local", q_blk_pos_local), ("k_blk_pos_all", k_blk_pos_all),
@@ -228,7 +234,7 @@ def flash_fwd_raw(q_ptr, k_ptrs, v_ptrs, o_ptr, lse_ptr, *, like_q, like_k, head
     a.k_ptrs, a.v_ptrs = kk[1], vv[1]
     a.B, a.Sq, a.Hq, a.Hkv, a.causal, a.n_src, a.src_len, a.q_off = \
         B, Sq, heads[0], heads[1], int(causal), len(k_ptrs), like_k.shape[1], 0
-    a.scale = scale or 1.0 / math.sqrt(hd)
+    a.scale, a.head_dim = scale or 1.0 / math.sqrt(hd), hd
     a.q_blk_pos = q_blk_pos.data_ptr() if q_blk_pos is not None else None
     a.k_blk_pos = k_blk_pos.data_ptr() if k_blk_pos is not None else None
     a.lse_heads = lse_heads
@@ -258,7 +264,7 @@ def flash_bwd_raw(ptr, src, *, lse, delta, like_q, like_k, heads, lse_heads, cau
     a.k_src, a.v_src, a.q_src, a.do_src, a.lse_src, a.delta_src = [x[1] for x in keep]
     a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.causal, a.n_src, a.q_off, a.phase = \
         B, Sq, like_k.shape[1], heads[0], heads[1], int(causal), len(src["k"]), 0, 2
-    a.scale = scale or 1.0 / math.sqrt(hd)
+    a.scale, a.head_dim = scale or 1.0 / math.sqrt(hd), hd
     a.lse_heads = lse_heads
     a.q_blk_pos_local = a.k_blk_pos_local = blk_local.data_ptr() if blk_local is not None else None
     a.k_blk_pos_all = a.q_blk_pos_all = blk_all.data_ptr() if blk_all is not None else None
@@ -300,12 +306,16 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
     hd = q.shape[-1]
     if USE_FLASH and PAD_SMALL_HEADS and attn_mask is None and _lib.on(q) and q.dtype == torch.bfloat16 and \
             k.dtype == torch.bfloat16 and hd < 128 and hd % 8 == 0 and (not causal or q.shape[1] <= k.shape[1]):
-        # head dims below 128 (the 125m / 350m / 1b presets have 64): zero-pad the head dimension so the tcgen05
-        # kernels apply. The padded columns add nothing to q.k and come out of P.V as zeros; the price is the work
-        # of the padding (twice the FLOPs and traffic at 64). ``NPB200_SDPA=1`` picks PyTorch's library kernel instead.
-        pad = (0, 128 - hd)
-        o = flash_attention(F.pad(q, pad), F.pad(k, pad), F.pad(v, pad), causal=causal,
-                            scale=scale if scale is not None else 1.0 / math.sqrt(hd))
+        scale = scale if scale is not None else 1.0 / math.sqrt(hd)
+        if hd == 64:
+            # the head dim of the 125m / 350m / 1b presets: kernels of its own; views they cannot read are copied
+            q, k, v = (t if _rows_aligned(t) else t.clone(memory_format=torch.contiguous_format) for t in (q, k, v))
+            return flash_attention(q, k, v, causal=causal, scale=scale)
+        # other head dims below 128: zero-pad the head dimension to the next one the kernels are built for. The padded
+        # columns add nothing to q.k and come out of P.V as zeros; the price is the work of the padding and three copies.
+        # ``NPB200_SDPA=1`` picks PyTorch's library kernel instead.
+        pad = (0, (64 if hd < 64 else 128) - hd)
+        o = flash_attention(F.pad(q, pad), F.pad(k, pad), F.pad(v, pad), causal=causal, scale=scale)
         return o[..., :hd]
     qt, kt, vt = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
     is_causal = causal and attn_mask is None and q.shape[1] == k.shape[1]
