@@ -68,6 +68,7 @@ struct GemmParams {
   const uint4* push_src; long long push_vecs;
   uint4* push_dst[8]; int* push_flag[8]; int push_n;
   int* push_ctr;
+  int splits;                 // pair kernel: parts of K (cluster of 2 * splits CTAs), 1 = whole
   bool st32, st32_c2;         // rows and column chunks of C / C2 are 32-byte aligned: use 32-byte stores
   const float* bias;          // optional [N] fp32 added to every output row (plain epilogue)
 };
@@ -277,6 +278,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t taddr, 
 #pragma unroll 1
     for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
       uint32_t g[32], u[32];
+      __syncwarp();   // rows that are not stored leave the chunk early
       np::tmem_ld32(taddr + c * 32, g);
       np::tmem_ld32(taddr + BN / 2 + c * 32, u);
       np::tmem_ld_wait();
@@ -286,6 +288,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t taddr, 
 #pragma unroll 1
     for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
       uint32_t r[32];
+      __syncwarp();
       if (have_acc) {
         np::tmem_ld32(taddr + c * 32, r);
         np::tmem_ld_wait();
@@ -574,9 +577,9 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ uint32_t leader_addr(uint32_t smem_addr) {   // the same shared-memory offset in CTA 0
+__device__ __forceinline__ uint32_t peer_addr(uint32_t smem_addr, uint32_t cta) {   // the same offset in another CTA
   uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_addr));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(cta));
   return r;
 }
 __device__ __forceinline__ void arrive_cluster(uint32_t addr) {
@@ -598,14 +601,26 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_d, uint64_t adesc,
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {   // arrives on the barrier at this offset in both CTAs
+// arrives on the barrier at this offset in both CTAs of the pair whose leader has cluster rank `leader`
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint32_t leader) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"((uint16_t)3)
+      ::"r"(bar), "h"((uint16_t)(3u << leader))
       : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+               : "memory");
+}
+
+// SPLIT: a cluster of `splits` pairs computes one tile, each pair a contiguous part of the K steps. When all of them are
+// done, the operand stages are free: every pair sends the others their share of the columns (256 / splits each, fp32,
+// through distributed shared memory), sums its own share in the order of the parts and runs the epilogue on it. No
+// workspace, no atomics, and the same result every time. It is for outputs with too few tiles to occupy the SMs: the time
+// of such a GEMM is its K steps one after the other (about 0.4 us each), not its FLOPs.
+template <bool SPLIT>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmB2, const GemmParams p) {
   constexpr int BN = PAIR_BN, STAGES = PAIR_STAGES, TM = 2 * BM, HN = BN / 2;
@@ -622,13 +637,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)cluster_rank();
-  const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+  const uint32_t crank = cluster_rank(), lead = crank & ~1u;
+  const int rank = (int)(crank & 1u);                              // 0: leader of its pair
+  const int splits = SPLIT ? p.splits : 1, split = SPLIT ? (int)(crank >> 1) : 0;
+  const int pair = (int)blockIdx.x / (2 * splits), pairs = (int)gridDim.x / (2 * splits);
   const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
   const int m_blocks = (p.M + TM - 1) / TM, m_blocks128 = (p.M + BM - 1) / BM;
   const int bn_out = (p.epilogue == 1) ? HN : BN;
   const int n_blocks = (p.N + bn_out - 1) / bn_out;
   const int num_tiles = m_blocks * n_blocks * ((p.mode == 2) ? p.num_groups : 1);
+  // the K steps of this CTA's part
+  auto k_steps = [&](int g, auto&& f) {
+    if constexpr (SPLIT) {
+      const int nkb = (p.K + BK - 1) / BK, hi = (int)((long long)nkb * (split + 1) / splits);
+      for (int kb = (int)((long long)nkb * split / splits); kb < hi; ++kb)
+        if (!f(kb * BK)) return;
+    } else {
+      for_each_k(p, g, f);
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -671,6 +698,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     return (p.mblk_rows[b0] > 0 ? 1 : 0) | (b0 + 1 < m_blocks128 && p.mblk_rows[b0 + 1] > 0 ? 2 : 0);
   };
 
+  bool done = false;   // SPLIT: this epilogue warp's accumulator is complete
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one in each CTA)
     if (lane == 0) {
@@ -688,10 +716,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         // SwiGLU: the leader's half of B is the gate tile, the peer's the up tile (another tensor, the same rows)
         const CUtensorMap* bm = (p.epilogue == 1 && rank) ? &tmB2 : &tmB;
         const int nrow = n0 + (p.epilogue == 1 ? 0 : rank * HN);
-        for_each_k(p, tl.g, [&](int k0) -> bool {
+        k_steps(tl.g, [&](int k0) -> bool {
           if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 11)) return false;
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
-          const uint32_t fb = leader_addr(full_bar(stage));
+          const uint32_t fb = peer_addr(full_bar(stage), lead);
           if (rank == 0) np::mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
           if (!p.a_mn) {
             tma_load_2d_pair(sA, &tmA, fb, k0, m0);
@@ -733,7 +761,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         np::tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
         uint32_t accum = 0;
-        for_each_k(p, tl.g, [&](int) -> bool {
+        k_steps(tl.g, [&](int) -> bool {
           if (!np::mbar_wait(full_bar(stage), phase, abort_flag, KID_GEMM, 13)) return false;
           np::tc_fence_after();
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
@@ -746,11 +774,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             tc_mma_f16_pair(tmem_d, ad, bd, idesc, accum);
             accum = 1;
           }
-          tc_commit_pair(empty_bar(stage));
+          tc_commit_pair(empty_bar(stage), lead);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           return true;
         });
-        tc_commit_pair(tfull_bar(acc));
+        tc_commit_pair(tfull_bar(acc), lead);
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
       if (*abort_flag) __nanosleep(1000000);
@@ -771,13 +799,14 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 14)) break;
         np::tc_fence_after();
       }
+      if constexpr (SPLIT) { done = true; break; }   // one tile per cluster, finished below
       if (mine)
         store_tile<BN>(p, tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
                        tl.m_blk * TM + rank * BM + quarter * 32 + lane, tl.n_blk * bn_out, half, have_acc);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(leader_addr(tempty_bar(acc)));
+        if (lane == 0) arrive_cluster(peer_addr(tempty_bar(acc), lead));
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
       if (p.done_counters && mine) {
@@ -785,14 +814,71 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         __syncwarp();
         if (lane == 0) {
           const int fi = p.mblk_flag ? p.mblk_flag[2 * tl.m_blk] : 0;
-          const int done = atomicAdd(&p.done_counters[fi], 1) + 1;
-          if (done == EPI_WARPS * n_blocks * p.done_expected[fi]) {   // done_expected counts 128-row blocks
+          const int n_done = atomicAdd(&p.done_counters[fi], 1) + 1;
+          if (n_done == EPI_WARPS * n_blocks * p.done_expected[fi]) {   // done_expected counts 128-row blocks
             __threadfence_system();
             np::st_release_sys(p.done_flag_ptr[fi], epoch);
           }
         }
       }
     }
+  }
+  if constexpr (SPLIT) {
+    __syncthreads();
+    cluster_sync();      // every pair of the cluster has consumed its operand stages
+    const int quarter = warp & 3, half = (warp - 2) >> 2, r = quarter * 32 + lane;
+    const int W = BN / splits, per_half = W / 64;   // columns of a share; 32-column chunks of it per warp
+    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    auto slot = [&](int from, int c) {   // chunk c of the share sent by part `from`: [8 vectors][128 rows] of 16 bytes
+      return smem_base + (uint32_t)(from * W * 512 + c * 8 * 2048 + r * 16);
+    };
+    if (done) {
+      np::tc_fence_after();
+      for (int d = 0; d < splits; ++d) {
+        if (d == split) continue;
+        for (int c = half * per_half; c < (half + 1) * per_half; ++c) {
+          uint32_t v[32];
+          np::tmem_ld32(taddr + d * W + c * 32, v);
+          np::tmem_ld_wait();
+          const uint32_t dst = peer_addr(slot(split, c), (uint32_t)(2 * d + rank));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) st_cluster_v4(dst + i * 2048, v + 4 * i);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync();      // all shares have arrived
+    if (done) {
+      const Tile tl = decode_tile<8>(pair, m_blocks, n_blocks);
+      const OutRow o = out_row(p, 0, tl.m_blk * TM + rank * BM + r);
+      for (int c = half * per_half; c < (half + 1) * per_half; ++c) {
+        uint32_t own[32];
+        float sum[32];
+        __syncwarp();
+        np::tmem_ld32(taddr + split * W + c * 32, own);
+        np::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+        for (int d = 0; d < splits; ++d) {
+          if (d == split) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sum[i] += __uint_as_float(own[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              float4 f;
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "r"(slot(d, c) + i * 2048) : "memory");
+              sum[4 * i] += f.x; sum[4 * i + 1] += f.y; sum[4 * i + 2] += f.z; sum[4 * i + 3] += f.w;
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) own[i] = __float_as_uint(sum[i]);
+        store_chunk(p, o, own, tl.n_blk * BN + split * W + c * 32);
+      }
+    }
+    __syncwarp();
   }
   np::tc_fence_before();
   __syncthreads();
@@ -870,6 +956,7 @@ struct NpGemmArgs {
   const void* push_src; long long push_bytes; void* const* push_dst; int* const* push_flag; int push_n; int* push_ctr;
   const float* bias;  // optional [N] fp32 bias added in the plain epilogue (alpha != 0)
   int mt;             // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles on a pair of CTAs)
+  int split;          // parts of K on the pair kernel: 0 = choose, 1, 2 or 4 (dense form, plain epilogue)
   int paired;         // row-grouped form: blocks 2 i and 2 i + 1 share their group and their arrival flag
 };
 
@@ -883,7 +970,7 @@ static int num_sms() {
 }
 
 template <int BN, int STAGES, bool PAIR>
-static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
+static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1) {
   CUtensorMap tmA, tmB, tmB2, tmAloc, tmBloc;
   int rc;
   if (!a.a_mn) rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.K, (uint64_t)a.lda, BK, BM);
@@ -948,8 +1035,11 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
   bool& attr_set = *attr_once.slot();
   if (!attr_set) {
     cudaError_t e;
-    if constexpr (PAIR) e = cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    else e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if constexpr (PAIR) {
+      e = cudaFuncSetAttribute(gemm_bf16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(gemm_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    } else e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
   }
@@ -959,7 +1049,17 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
   if constexpr (PAIR) {
     const long long pairs = tiles < cap / 2 ? tiles : cap / 2;
     if (pairs <= 0) return 0;
-    gemm_bf16_pair_kernel<<<(int)(2 * pairs), GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmB2, p);
+    p.splits = splits;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2 * splits; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = SMEM; cfg.stream = stream; cfg.attrs = &at; cfg.numAttrs = 1;
+    const cudaError_t e = splits > 1 ? cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<true>, tmA, tmB, tmB2, p)
+                                     : cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<false>, tmA, tmB, tmB2, p);
+    if (e != cudaSuccess) return 500 + (int)e;
   } else {
     const int grid = (int)(tiles < cap ? tiles : cap);
     if (grid <= 0) return 0;
@@ -968,6 +1068,9 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream) {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
+
+int np_skinny_linear(const void* x, long long ldx, const void* w, long long ldw, int M, int N, int K, void* out, long long ldo,
+                     int out_f32, float alpha, const float* bias, const void* cin, long long ldcin, cudaStream_t stream);
 
 // C[M,N] (+)= alpha * A * B^T with the operand layouts described in NpGemmArgs.
 // Returns 0 or a launch/setup error; device-side problems are reported via np_status_read.
@@ -984,10 +1087,15 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
     ctx_bound = true;
   }
   if ((a.lda % 8) || (a.ldb % 8) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15)) return 1;
-  // Which kernel. The pair kernel takes the forms without peer-arrival flags on B, pushes or split operands; row-grouped
-  // launches only when their tables come in pairs of 128-row blocks (`paired`).
   const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
                      (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
+  // A few rows: the weight is streamed once through all SMs (skinny.cu). `mt`, `bn` and `split` ask for a tile kernel.
+  if (a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && plain && a.K > 0 && a.K % 8 == 0 && a.bn == 0 && a.mt == 0 &&
+      a.split == 0 && a.max_ctas == 0 && a.alpha != 0.f)
+    return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
+                            a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
+  // Which kernel. The pair kernel takes the forms without peer-arrival flags on B, pushes or split operands; row-grouped
+  // launches only when their tables come in pairs of 128-row blocks (`paired`).
   int bn = a.bn, mt = a.mt;
   if (a.epilogue == 1) bn = 256;
   if (bn == 0 || (bn == 256 && mt == 0)) {
@@ -1004,7 +1112,11 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
     if (cpair <= c128 && cpair <= c256) { bn = 256; mt = 2; }
     else bn = c256 <= c128 ? 256 : 128;
   }
-  if (bn == 256 && mt == 2 && plain) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream);
+  if (bn == 256 && mt == 2 && plain) {
+    const bool can = a.mode == 0 && a.epilogue == 0 && (a.K + BK - 1) / BK >= 8 && a.max_ctas == 0;
+    const int splits = can && (a.split == 2 || a.split == 4) ? a.split : 1;
+    return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
+  }
   if (bn == 256) return launch_gemm<256, 4, false>(a, (cudaStream_t)stream);
   return launch_gemm<128, 6, false>(a, (cudaStream_t)stream);
 }

@@ -132,13 +132,17 @@ class Attention(nn.Module):
                 k = self.k_norm(k.float()).to(x.dtype) if k.dtype != torch.float32 else self.k_norm(k)
             q = rope_ops.apply_rope(q, cos, sin, start_pos, pid)
             k = rope_ops.apply_rope(k, cos, sin, start_pos, pid)
-        if kv_cache is not None:
-            k = torch.cat([kv_cache[0], k], dim=1)
-            v = torch.cat([kv_cache[1], v], dim=1)
-        if self._cp_module is not None:
-            o = self._cp_module(q, k, v, causal=causal)
+        if kv_cache is not None and self._cp_module is None and attn_mask is None and \
+                getattr(self.sdpa, "__func__", None) is Attention.sdpa:   # not replaced by a subclass or on the instance
+            o, k, v = attn_ops.attention_append(q, kv_cache[0], kv_cache[1], k, v, causal=causal)
         else:
-            o = self.sdpa(q, k, v, causal=causal, attn_mask=attn_mask)
+            if kv_cache is not None:
+                k = torch.cat([kv_cache[0], k], dim=1)
+                v = torch.cat([kv_cache[1], v], dim=1)
+            if self._cp_module is not None:
+                o = self._cp_module(q, k, v, causal=causal)
+            else:
+                o = self.sdpa(q, k, v, causal=causal, attn_mask=attn_mask)
         o = o.reshape(B, S, self._local_heads * self.head_dim)
         if self.output_dropout is not None:
             o = self.output_dropout(o)

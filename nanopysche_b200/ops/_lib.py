@@ -47,7 +47,7 @@ class GemmArgs(C.Structure):
         ("push_src", c_void_p), ("push_bytes", c_ll), ("push_dst", c_void_p), ("push_flag", c_void_p),
         ("push_n", c_int), ("push_ctr", c_void_p),
         ("bias", c_void_p),
-        ("mt", c_int), ("paired", c_int),
+        ("mt", c_int), ("split", c_int), ("paired", c_int),
     ]
 
 
@@ -90,7 +90,7 @@ class AttnFwdArgs(C.Structure):
         ("src_len", c_int), ("q_off", c_int),
         ("scale", c_float),
         ("q_blk_pos", c_void_p), ("k_blk_pos", c_void_p),
-        ("lse_heads", c_int),
+        ("split", c_int), ("lse_heads", c_int),
         ("src_flags", c_void_p), ("flag_idx", c_void_p), ("flag_epoch", c_int), ("epoch_base", c_void_p),
         ("flag_limit_ns", c_ull), ("flag_own", c_int),
         ("push_k", c_void_p), ("push_v", c_void_p), ("push_bytes", c_ll), ("push_dst", c_void_p),
@@ -117,12 +117,27 @@ class AttnBwdArgs(C.Structure):
         ("scale", c_float),
         ("q_blk_pos_local", c_void_p), ("k_blk_pos_all", c_void_p),
         ("k_blk_pos_local", c_void_p), ("q_blk_pos_all", c_void_p),
-        ("lse_heads", c_int),
+        ("split", c_int), ("lse_heads", c_int),
         ("src_flags", c_void_p), ("flag_idx", c_void_p), ("flag_epoch", c_int), ("epoch_base", c_void_p),
         ("flag_limit_ns", c_ull), ("flag_which", c_int), ("skip", c_int), ("flag_own", c_int),
         ("push_k", c_void_p), ("push_v", c_void_p), ("push_bytes", c_ll), ("push_dst", c_void_p),
         ("push_flag", c_void_p), ("push_n", c_int), ("push_ctr", c_void_p),
         ("head_dim", c_int),
+    ]
+
+
+class DecodeArgs(C.Structure):
+    """Mirror of ``NpDecodeArgs`` in csrc/skinny.cu."""
+
+    _fields_ = [
+        ("q", c_void_p), ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
+        ("kc", c_void_p), ("vc", c_void_p), ("kc_sb", c_ll), ("kc_ss", c_ll), ("kc_sh", c_ll),
+        ("vc_sb", c_ll), ("vc_ss", c_ll), ("vc_sh", c_ll),
+        ("kn", c_void_p), ("vn", c_void_p), ("kn_sb", c_ll), ("kn_ss", c_ll), ("kn_sh", c_ll),
+        ("vn_sb", c_ll), ("vn_ss", c_ll), ("vn_sh", c_ll),
+        ("ko", c_void_p), ("vo", c_void_p), ("o", c_void_p),
+        ("B", c_int), ("Sq", c_int), ("Hq", c_int), ("Hkv", c_int), ("past", c_int), ("fresh", c_int),
+        ("causal", c_int), ("head_dim", c_int), ("scale", c_float),
     ]
 
 
@@ -201,6 +216,7 @@ def lib():
                                            c_void_p]
     _LIB.np_attn_fwd.argtypes = [C.POINTER(AttnFwdArgs), c_void_p]
     _LIB.np_attn_bwd.argtypes = [C.POINTER(AttnBwdArgs), c_void_p]
+    _LIB.np_decode_attn.argtypes = [C.POINTER(DecodeArgs), c_void_p]
     _LIB.np_status_read.argtypes = [C.POINTER(c_int)]
     return _LIB
 

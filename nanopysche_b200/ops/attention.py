@@ -297,6 +297,61 @@ def flash_attention(q, k, v, causal=True, scale=None):
     return _FlashAttention.apply(q, k, v, causal, scale)
 
 
+def _decode_views(*ts: torch.Tensor) -> bool:
+    """[B, S, H, hd] bf16 tensors that the decode kernel reads with 16-byte loads (broadcast dimensions included)."""
+    return all(t.dtype == torch.bfloat16 and t.stride(3) == 1 and t.data_ptr() % 16 == 0 and
+               t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(2) % 8 == 0 for t in ts)
+
+
+def _decode(q, k, v, k_new, v_new, causal, scale):
+    """Launch of the decode kernel: keys and values ``[k | k_new]``; returns ``(out, k_cat, v_cat)`` (``None`` for the
+    concatenations when nothing is appended)."""
+    import ctypes as C
+
+    B, Sq, Hq, hd = q.shape
+    P, Hkv = k.shape[1], k.shape[2]
+    o = torch.empty((B, Sq, Hq, hd), device=q.device, dtype=torch.bfloat16)
+    a = _lib.DecodeArgs()
+    a.q, a.kc, a.vc, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
+    a.q_sb, a.q_ss, a.q_sh = q.stride()[:3]
+    a.kc_sb, a.kc_ss, a.kc_sh = k.stride()[:3]
+    a.vc_sb, a.vc_ss, a.vc_sh = v.stride()[:3]
+    ko = vo = None
+    if k_new is not None:
+        n = k_new.shape[1]
+        ko = torch.empty((B, P + n, Hkv, hd), device=q.device, dtype=torch.bfloat16)
+        vo = torch.empty_like(ko)
+        a.kn, a.vn, a.ko, a.vo, a.fresh = k_new.data_ptr(), v_new.data_ptr(), ko.data_ptr(), vo.data_ptr(), n
+        a.kn_sb, a.kn_ss, a.kn_sh = k_new.stride()[:3]
+        a.vn_sb, a.vn_ss, a.vn_sh = v_new.stride()[:3]
+    a.B, a.Sq, a.Hq, a.Hkv, a.past, a.causal, a.head_dim = B, Sq, Hq, Hkv, P, int(causal), hd
+    a.scale = scale if scale is not None else 1.0 / math.sqrt(hd)
+    _lib.check(_lib.lib().np_decode_attn(C.byref(a), C.c_void_p(_lib.stream())), "decode_attn")
+    return o, ko, vo
+
+
+# Query rows of one KV head (query heads of its group x new tokens) that the decode kernel holds in registers.
+DECODE_ROWS = 8
+
+
+def attention_append(q, k_cache, v_cache, k_new, v_new, causal: bool = True, scale: float | None = None):
+    """Attention of ``q [B, S, Hq, hd]`` over a KV cache with ``S`` new positions behind it; returns ``(out, k, v)`` with
+    ``k = cat(k_cache, k_new)`` and ``v`` likewise (dim 1). Without gradients and for a few query rows per KV head (token
+    generation) one kernel reads each key and value once, attends and writes the concatenation; else a concatenation
+    followed by ``attention``."""
+    B, S, Hq, hd = q.shape
+    Hkv = k_new.shape[2]
+    ts = (q, k_cache, v_cache, k_new, v_new)
+    if (USE_FLASH and _lib.on(q) and hd in (64, 128) and Hq // Hkv * S <= DECODE_ROWS and k_cache.shape[1] > 0 and
+            not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) and
+            k_new.shape == (B, S, Hkv, hd) == v_new.shape and
+            k_cache.shape == v_cache.shape == (B, k_cache.shape[1], Hkv, hd) and
+            all(t.device == q.device for t in ts) and _decode_views(*ts)):
+        return _decode(q, k_cache, v_cache, k_new, v_new, causal, scale)
+    k, v = torch.cat([k_cache, k_new], dim=1), torch.cat([v_cache, v_new], dim=1)
+    return attention(q, k, v, causal=causal, scale=scale), k, v
+
+
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True,
               attn_mask: torch.Tensor | None = None, scale: float | None = None) -> torch.Tensor:
     """``softmax(q k^T / sqrt(hd)) v`` for ``q [B,S,Hq,hd]``, ``k/v [B,Sk,Hkv,hd]`` -> ``[B,S,Hq,hd]``."""
