@@ -45,15 +45,15 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* tm, u
 #pragma unroll
   for (int c = 0; c < HD / 64; ++c) tma_load_4d(dst + c * CHUNK_BYTES, tm, bar, c * 64, h, s0, b);
 }
-// K-major operand [rows, HD k]: k-step kk (16 elements) -> chunk kk/4, +32 B per step inside the chunk
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t tile, int kk) {
-  return np::make_smem_desc(tile + (kk >> 2) * CHUNK_BYTES + (kk & 3) * 32, 16, 1024);
-}
-// MN-major operand stored as [k rows, HD mn cols] (64-col chunks): k-step = 16 rows = +2048 B,
-// LBO = distance between the two 64-wide chunks
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile, int kk) {
-  return np::make_smem_desc(tile + kk * 2048, CHUNK_BYTES, 1024);
-}
+// Operand descriptors: of a tile's first 16-wide K step, and what K step kk adds to the (16-byte) address field. They are
+// built once per kernel; a stage adds its offset, a K step a constant. (Built anew for every MMA by one lane in a divergent
+// branch, the issue of a 128 x 128 x 128 product took longer than the product.)
+// K-major operand [rows, HD k]: 16 elements -> chunk kk / 4, +32 B per step inside the chunk
+__device__ __forceinline__ uint64_t desc_kmajor(uint32_t tile) { return np::make_smem_desc(tile, 16, 1024); }
+__device__ __forceinline__ constexpr uint32_t koff(int kk) { return ((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) >> 4; }
+// MN-major operand stored as [k rows, HD mn cols] (64-col chunks): 16 rows = +2048 B, LBO = distance between chunks
+__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile) { return np::make_smem_desc(tile, CHUNK_BYTES, 1024); }
+__device__ __forceinline__ constexpr uint32_t mnoff(int kk) { return (kk * 2048) >> 4; }
 // Sources that are still arriving in this GPU's memory (a peer is pushing them): flag[idx[s]] reaches the epoch
 // once source s is complete. The TMA producer checks it before its first load from the source.
 struct SrcFlags {
@@ -294,40 +294,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_qk = np::make_idesc(128, 128, 1, 1, 0, 0);   // Q (K-major) x K (K-major)
-      const uint32_t idesc_pv = np::make_idesc(128, HD, 1, 1, 0, 1);   // P (TMEM) x V (MN-major)
-      bool ok = np::mbar_wait(B_(FB_Q), 0, abort_flag, KID_ATTN, 2);
-      auto issue_qk = [&](int i) {
-        const int st = i & 1, ks = i % F_KST;
-        if (!np::mbar_wait(B_(FB_K + ks), (uint32_t)(i / F_KST) & 1u, abort_flag, KID_ATTN, 3)) return false;
-        np::tc_fence_after();
+    const uint32_t idesc_qk = np::make_idesc(128, 128, 1, 1, 0, 0);   // Q (K-major) x K (K-major)
+    const uint32_t idesc_pv = np::make_idesc(128, HD, 1, 1, 0, 1);    // P (TMEM) x V (MN-major)
+    const uint64_t dQ = desc_kmajor(sQ), dK = desc_kmajor(sK0), dV = desc_mnmajor(sV0);
+    bool ok = np::mbar_wait_warp(B_(FB_Q), 0, abort_flag, KID_ATTN, 2);
+    auto issue_qk = [&](int i) {
+      const int st = i & 1, ks = i % F_KST;
+      if (!np::mbar_wait_warp(B_(FB_K + ks), (uint32_t)(i / F_KST) & 1u, abort_flag, KID_ATTN, 3)) return false;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dK + (uint32_t)(ks * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk)
-          np::tc_mma_f16(tmem + F_S + st * 128, desc_kmajor(sQ, kk), desc_kmajor(sK0 + ks * TILE_BYTES, kk), idesc_qk, kk > 0);
+          np::tc_mma_f16(tmem + F_S + st * 128, dQ + koff(kk), b + koff(kk), idesc_qk, kk > 0);
         np::tc_commit(B_(FB_S + st));
         np::tc_commit(B_(FB_KE + ks));
-        return true;
-      };
-      int j = next_vis(0);
-      if (ok && j < total_blocks) ok = issue_qk(0);
-      for (int i = 0; j < total_blocks && ok && !*abort_flag; ++i) {
-        const int st = i & 1, vs = i % F_VST;
-        // S of the next block is computed while the softmax warps work on this one. Its S and P buffers were
-        // last used for block i-1: S read before P of block i-1 arrived, P consumed by P V of block i-1 (issued).
-        j = next_vis(j + 1);
-        if (j < total_blocks) ok = issue_qk(i + 1);
-        ok = ok && np::mbar_wait(B_(FB_P), (uint32_t)i & 1u, abort_flag, KID_ATTN, 5) &&   // P ready, O rescaled
-             np::mbar_wait(B_(FB_V + vs), (uint32_t)(i / F_VST) & 1u, abort_flag, KID_ATTN, 4);
-        if (!ok) break;
-        np::tc_fence_after();
+      }
+      __syncwarp();
+      return true;
+    };
+    int j = next_vis(0);
+    if (ok && j < total_blocks) ok = issue_qk(0);
+    for (int i = 0; j < total_blocks && ok; ++i) {
+      const int st = i & 1, vs = i % F_VST;
+      // S of the next block is computed while the softmax warps work on this one. Its S and P buffers were
+      // last used for block i-1: S read before P of block i-1 arrived, P consumed by P V of block i-1 (issued).
+      j = next_vis(j + 1);
+      if (j < total_blocks) ok = issue_qk(i + 1);
+      ok = ok && np::mbar_wait_warp(B_(FB_P), (uint32_t)i & 1u, abort_flag, KID_ATTN, 5) &&   // P ready, O rescaled
+           np::mbar_wait_warp(B_(FB_V + vs), (uint32_t)(i / F_VST) & 1u, abort_flag, KID_ATTN, 4);
+      if (!ok) break;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dV + (uint32_t)(vs * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          tc_mma_f16_ts(tO, tmem + F_P + st * 64 + kk * 8, desc_mnmajor(sV0 + vs * TILE_BYTES, kk), idesc_pv,
-                        (i > 0) || (kk > 0));
+          tc_mma_f16_ts(tO, tmem + F_P + st * 64 + kk * 8, b + mnoff(kk), idesc_pv, (i > 0) || (kk > 0));
         np::tc_commit(B_(FB_O));
         np::tc_commit(B_(FB_VE + vs));
       }
+      __syncwarp();
     }
   } else {
     constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
@@ -541,73 +547,75 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_qk = np::make_idesc(128, 128, 1, 1, 0, 0);
-      const uint32_t idesc_pv = np::make_idesc(128, HD, 1, 1, 0, 1);
-      bool ok = np::mbar_wait(B_(G_Q), 0, abort_flag, KID_ATTN, 23);
-      // S of tile t for block i (the K stage must have landed; the caller has waited for it)
-      auto issue_s = [&](int t, int i) {
-        const int ks = i % G_KST;
+    const uint32_t idesc_qk = np::make_idesc(128, 128, 1, 1, 0, 0);
+    const uint32_t idesc_pv = np::make_idesc(128, HD, 1, 1, 0, 1);
+    const uint64_t dQ = desc_kmajor(sQ), dK = desc_kmajor(sK0), dV = desc_mnmajor(sV0);
+    bool ok = np::mbar_wait_warp(B_(G_Q), 0, abort_flag, KID_ATTN, 23);
+    // S of tile t for block i (the K stage must have landed; the caller has waited for it); `last`: no other tile reads
+    // this K stage any more
+    auto issue_s = [&](int t, int i, bool last) {
+      const int ks = i % G_KST;
+      if (np::elect_one()) {
+        const uint64_t a = dQ + (uint32_t)(t * (TILE_BYTES >> 4)), b = dK + (uint32_t)(ks * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          np::tc_mma_f16(tmem + t * 128, desc_kmajor(sQ + t * TILE_BYTES, kk), desc_kmajor(sK0 + ks * TILE_BYTES, kk),
-                         idesc_qk, kk > 0);
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tmem + t * 128, a + koff(kk), b + koff(kk), idesc_qk, kk > 0);
         np::tc_commit(B_(G_S + t));
-      };
-      auto wait_k = [&](int i) {
-        const bool w = np::mbar_wait(B_(G_K + i % G_KST), (uint32_t)(i / G_KST) & 1u, abort_flag, KID_ATTN, 24);
-        np::tc_fence_after();
-        return w;
-      };
-      auto issue_pv = [&](int t, int i) {
-        const int vs = i % G_VST;
+        if (last) np::tc_commit(B_(G_KE + ks));
+      }
+      __syncwarp();
+    };
+    auto wait_k = [&](int i) {
+      const bool w = np::mbar_wait_warp(B_(G_K + i % G_KST), (uint32_t)(i / G_KST) & 1u, abort_flag, KID_ATTN, 24);
+      np::tc_fence_after();
+      return w;
+    };
+    auto issue_pv = [&](int t, int i, bool last) {
+      const int vs = i % G_VST;
+      if (np::elect_one()) {
+        const uint64_t b = dV + (uint32_t)(vs * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          tc_mma_f16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, desc_mnmajor(sV0 + vs * TILE_BYTES, kk), idesc_pv,
-                        (i > 0) || (kk > 0));
+          tc_mma_f16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, b + mnoff(kk), idesc_pv, (i > 0) || (kk > 0));
         np::tc_commit(B_(G_O + t));
-      };
-      if (ok && nv > 0) {
-        ok = wait_k(0);
-        if (ok) {
-          if (nv0 > 0) issue_s(0, 0);
-          if (nv1 > 0) issue_s(1, 0);
-          np::tc_commit(B_(G_KE + 0));
-        }
+        if (last) np::tc_commit(B_(G_VE + vs));
       }
-      for (int i = 0; i < nv && ok && !*abort_flag; ++i) {
-        const int vs = i % G_VST;
-        bool have_k = false;
-        ok = np::mbar_wait(B_(G_V + vs), (uint32_t)(i / G_VST) & 1u, abort_flag, KID_ATTN, 25);
-        if (ok && i < nv0) {
-          ok = np::mbar_wait(B_(G_P + 0), (uint32_t)i & 1u, abort_flag, KID_ATTN, 26);   // P of tile 0 stored, O rescaled
-          if (!ok) break;
-          np::tc_fence_after();
-          issue_pv(0, i);
-          if (i + 1 < nv0) {
-            ok = wait_k(i + 1);
-            if (!ok) break;
-            have_k = true;
-            issue_s(0, i + 1);
-          }
-        }
-        if (ok && i < nv1) {
-          ok = np::mbar_wait(B_(G_P + 1), (uint32_t)i & 1u, abort_flag, KID_ATTN, 27);
-          if (!ok) break;
-          np::tc_fence_after();
-          issue_pv(1, i);
-        }
+      __syncwarp();
+    };
+    if (ok && nv > 0) {
+      ok = wait_k(0);
+      if (ok) {
+        if (nv0 > 0) issue_s(0, 0, nv1 == 0);
+        if (nv1 > 0) issue_s(1, 0, true);
+      }
+    }
+    for (int i = 0; i < nv && ok; ++i) {
+      const int vs = i % G_VST;
+      bool have_k = false;
+      ok = np::mbar_wait_warp(B_(G_V + vs), (uint32_t)(i / G_VST) & 1u, abort_flag, KID_ATTN, 25);
+      if (ok && i < nv0) {
+        ok = np::mbar_wait_warp(B_(G_P + 0), (uint32_t)i & 1u, abort_flag, KID_ATTN, 26);   // P of tile 0 stored, O rescaled
         if (!ok) break;
-        np::tc_commit(B_(G_VE + vs));
-        if (i + 1 < nv) {
-          if (i + 1 < nv1) {
-            if (!have_k) ok = wait_k(i + 1);
-            if (!ok) break;
-            issue_s(1, i + 1);
-          }
-          np::tc_commit(B_(G_KE + (i + 1) % G_KST));
+        np::tc_fence_after();
+        issue_pv(0, i, i >= nv1);
+        if (i + 1 < nv0) {
+          ok = wait_k(i + 1);
+          if (!ok) break;
+          have_k = true;
+          issue_s(0, i + 1, i + 1 >= nv1);
         }
       }
+      if (ok && i < nv1) {
+        ok = np::mbar_wait_warp(B_(G_P + 1), (uint32_t)i & 1u, abort_flag, KID_ATTN, 27);
+        if (!ok) break;
+        np::tc_fence_after();
+        issue_pv(1, i, true);
+        if (i + 1 < nv1) {
+          if (!have_k) ok = wait_k(i + 1);
+          if (!ok) break;
+          issue_s(1, i + 1, true);
+        }
+      }
+      if (!ok) break;
     }
   } else {
     // ---------------------------------------------------------------- softmax groups: one thread per query row
@@ -1033,48 +1041,58 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);   // both operands K-major (over hd)
-      const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);   // A from TMEM, B MN-major
-      bool ok = np::mbar_wait(B_(QB_QDO), 0, abort_flag, KID_ATTN_DQ, 2);
-      auto issue_s = [&](int i) {
-        const int st = i & 1, ks = i % Q_KST;
-        if (!np::mbar_wait(B_(QB_K + ks), (uint32_t)(i / Q_KST) & 1u, abort_flag, KID_ATTN_DQ, 3)) return false;
-        np::tc_fence_after();
+    const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);   // both operands K-major (over hd)
+    const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);    // A from TMEM, B MN-major
+    const uint64_t dQ = desc_kmajor(sQ), ddO = desc_kmajor(sdO), dK = desc_kmajor(sK0), dV = desc_kmajor(sV0),
+                   dKm = desc_mnmajor(sK0);
+    bool ok = np::mbar_wait_warp(B_(QB_QDO), 0, abort_flag, KID_ATTN_DQ, 2);
+    auto issue_s = [&](int i) {
+      const int st = i & 1, ks = i % Q_KST;
+      if (!np::mbar_wait_warp(B_(QB_K + ks), (uint32_t)(i / Q_KST) & 1u, abort_flag, KID_ATTN_DQ, 3)) return false;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dK + (uint32_t)(ks * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          np::tc_mma_f16(tmem + st * 128, desc_kmajor(sQ, kk), desc_kmajor(sK0 + ks * TILE_BYTES, kk), idesc_kk, kk > 0);
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tmem + st * 128, dQ + koff(kk), b + koff(kk), idesc_kk, kk > 0);
         np::tc_commit(B_(QB_S + st));
-        return true;
-      };
-      auto issue_dp = [&](int i) {
-        const int vs = i % Q_VST;
-        if (!np::mbar_wait(B_(QB_V + vs), (uint32_t)(i / Q_VST) & 1u, abort_flag, KID_ATTN_DQ, 4)) return false;
-        np::tc_fence_after();
+      }
+      __syncwarp();
+      return true;
+    };
+    auto issue_dp = [&](int i) {
+      const int vs = i % Q_VST;
+      if (!np::mbar_wait_warp(B_(QB_V + vs), (uint32_t)(i / Q_VST) & 1u, abort_flag, KID_ATTN_DQ, 4)) return false;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dV + (uint32_t)(vs * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          np::tc_mma_f16(tdP, desc_kmajor(sdO, kk), desc_kmajor(sV0 + vs * TILE_BYTES, kk), idesc_kk, kk > 0);
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tdP, ddO + koff(kk), b + koff(kk), idesc_kk, kk > 0);
         np::tc_commit(B_(QB_DP));
         np::tc_commit(B_(QB_VE + vs));
-        return true;
-      };
-      int j = next_vis(0);
-      if (ok && j < total_blocks) ok = issue_s(0) && issue_dp(0);
-      for (int i = 0; j < total_blocks && ok && !*abort_flag; ++i) {
-        const int ks = i % Q_KST;
-        j = next_vis(j + 1);
-        if (j < total_blocks) ok = issue_s(i + 1);   // its buffer was read for block i-1 before dS of block i-1 arrived
-        ok = ok && np::mbar_wait(B_(QB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 5);
-        if (!ok) break;
-        np::tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          tc_mma_f16_ts(tdQ, tdP + kk * 8, desc_mnmajor(sK0 + ks * TILE_BYTES, kk), idesc_mn, (i > 0) || (kk > 0));
-        np::tc_commit(B_(QB_KE + ks));
-        if (j < total_blocks) ok = issue_dp(i + 1);  // overwrites dS after the dQ product above has consumed it
       }
-      np::tc_commit(B_(QB_FIN));
+      __syncwarp();
+      return true;
+    };
+    int j = next_vis(0);
+    if (ok && j < total_blocks) ok = issue_s(0) && issue_dp(0);
+    for (int i = 0; j < total_blocks && ok; ++i) {
+      const int ks = i % Q_KST;
+      j = next_vis(j + 1);
+      if (j < total_blocks) ok = issue_s(i + 1);   // its buffer was read for block i-1 before dS of block i-1 arrived
+      ok = ok && np::mbar_wait_warp(B_(QB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 5);
+      if (!ok) break;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dKm + (uint32_t)(ks * (TILE_BYTES >> 4));
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) tc_mma_f16_ts(tdQ, tdP + kk * 8, b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
+        np::tc_commit(B_(QB_KE + ks));
+      }
+      __syncwarp();
+      if (j < total_blocks) ok = issue_dp(i + 1);  // overwrites dS after the dQ product above has consumed it
     }
+    if (np::elect_one()) np::tc_commit(B_(QB_FIN));
+    __syncwarp();
   } else {
     constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
     const int quarter = warp & 3, hf = (warp - 2) >> 2;     // this thread: row r, KV columns [CW hf, CW hf + CW)
@@ -1248,54 +1266,69 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);
-      const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);
-      bool ok = np::mbar_wait(B_(KB_KV), 0, abort_flag, KID_ATTN_DKV, 3);
-      auto issue_st = [&](int i) {
-        const int qs = i % K_QST;
-        if (!np::mbar_wait(B_(KB_Q + qs), (uint32_t)(i / K_QST) & 1u, abort_flag, KID_ATTN_DKV, 4)) return false;
-        np::tc_fence_after();
+    const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);
+    const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);
+    const uint64_t dK = desc_kmajor(sK), dV = desc_kmajor(sV), dQ = desc_kmajor(sQ0), ddO = desc_kmajor(sdO0),
+                   dQm = desc_mnmajor(sQ0), ddOm = desc_mnmajor(sdO0);
+    bool ok = np::mbar_wait_warp(B_(KB_KV), 0, abort_flag, KID_ATTN_DKV, 3);
+    auto issue_st = [&](int i) {
+      const int qs = i % K_QST;
+      if (!np::mbar_wait_warp(B_(KB_Q + qs), (uint32_t)(i / K_QST) & 1u, abort_flag, KID_ATTN_DKV, 4)) return false;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dQ + (uint32_t)(qs * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          np::tc_mma_f16(tSt, desc_kmajor(sK, kk), desc_kmajor(sQ0 + qs * TILE_BYTES, kk), idesc_kk, kk > 0);
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tSt, dK + koff(kk), b + koff(kk), idesc_kk, kk > 0);
         np::tc_commit(B_(KB_ST));
-        return true;
-      };
-      auto issue_dpt = [&](int i) {
-        const int ds = i % K_DOST;
-        if (!np::mbar_wait(B_(KB_DO + ds), (uint32_t)(i / K_DOST) & 1u, abort_flag, KID_ATTN_DKV, 5)) return false;
-        np::tc_fence_after();
+      }
+      __syncwarp();
+      return true;
+    };
+    auto issue_dpt = [&](int i) {
+      const int ds = i % K_DOST;
+      if (!np::mbar_wait_warp(B_(KB_DO + ds), (uint32_t)(i / K_DOST) & 1u, abort_flag, KID_ATTN_DKV, 5)) return false;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = ddO + (uint32_t)(ds * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          np::tc_mma_f16(tdPt, desc_kmajor(sV, kk), desc_kmajor(sdO0 + ds * TILE_BYTES, kk), idesc_kk, kk > 0);
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tdPt, dV + koff(kk), b + koff(kk), idesc_kk, kk > 0);
         np::tc_commit(B_(KB_DPT));
-        return true;
-      };
-      int c = next_vis(0);
-      if (ok && c < total) ok = issue_st(0) && issue_dpt(0);
-      for (int i = 0; c < total && ok && !*abort_flag; ++i) {
-        const int qs = i % K_QST, ds = i % K_DOST;
-        c = next_vis(c + 1);
-        ok = np::mbar_wait(B_(KB_P), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 6);
-        if (!ok) break;
-        np::tc_fence_after();
+      }
+      __syncwarp();
+      return true;
+    };
+    int c = next_vis(0);
+    if (ok && c < total) ok = issue_st(0) && issue_dpt(0);
+    for (int i = 0; c < total && ok; ++i) {
+      const int qs = i % K_QST, ds = i % K_DOST;
+      c = next_vis(c + 1);
+      ok = np::mbar_wait_warp(B_(KB_P), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 6);
+      if (!ok) break;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = ddOm + (uint32_t)(ds * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // dV += P^T dO
-          tc_mma_f16_ts(tdV, tSt + kk * 8, desc_mnmajor(sdO0 + ds * TILE_BYTES, kk), idesc_mn, (i > 0) || (kk > 0));
+          tc_mma_f16_ts(tdV, tSt + kk * 8, b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
         np::tc_commit(B_(KB_DOE + ds));
-        if (c < total) ok = issue_st(i + 1);        // overwrites P^T after the product above consumed it
-        ok = ok && np::mbar_wait(B_(KB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 7);
-        if (!ok) break;
-        np::tc_fence_after();
+      }
+      __syncwarp();
+      if (c < total) ok = issue_st(i + 1);        // overwrites P^T after the product above consumed it
+      ok = ok && np::mbar_wait_warp(B_(KB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 7);
+      if (!ok) break;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+        const uint64_t b = dQm + (uint32_t)(qs * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // dK += dS^T Q
-          tc_mma_f16_ts(tdK, tdPt + kk * 8, desc_mnmajor(sQ0 + qs * TILE_BYTES, kk), idesc_mn, (i > 0) || (kk > 0));
+          tc_mma_f16_ts(tdK, tdPt + kk * 8, b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
         np::tc_commit(B_(KB_QE + qs));
-        if (c < total) ok = issue_dpt(i + 1);       // overwrites dS^T after the product above consumed it
       }
-      np::tc_commit(B_(KB_FIN));
+      __syncwarp();
+      if (c < total) ok = issue_dpt(i + 1);       // overwrites dS^T after the product above consumed it
     }
+    if (np::elect_one()) np::tc_commit(B_(KB_FIN));
+    __syncwarp();
   } else {
     constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
     const int quarter = warp & 3, hf = (warp - 2) >> 2;   // this thread: KV row r, Q columns [CW hf, CW hf + CW)

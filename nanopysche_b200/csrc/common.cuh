@@ -135,6 +135,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// The same wait made by a whole warp (every lane calls it); the outcome is the same for all lanes. A warp that issues
+// tensor-core work stays converged this way and elects one lane around the issuing instructions only: loop state, barrier
+// addresses and descriptors are then warp-uniform values. With one lane running the whole loop in a divergent branch the
+// issue of a 64-wide K step took about 600 cycles, more than the MMAs themselves.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int kernel_id,
+                                               int detail) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, kernel_id, detail));
+}
+
 }  // namespace np
 // Debug-bounds build: compile with -DNP_DEBUG (NPB200_NVCC_EXTRA=-DNP_DEBUG python -m nanopysche_b200.build --force).
 // compute-sanitizer is not always available; these index predicates record (code 4, kernel id, block, offending

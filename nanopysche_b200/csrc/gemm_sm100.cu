@@ -123,6 +123,13 @@ struct Tile {
   int g, m_blk, n_blk;
 };
 
+// Operand tile in shared memory (64-wide K stage): descriptor of its first 16-wide K step, and what one K step adds to the
+// (16-byte) address field. K-major: 32 bytes along the swizzled row; MN-major: 16 rows of 128 bytes.
+__device__ __forceinline__ uint64_t operand_desc(uint32_t tile, int mn) {
+  return np::make_smem_desc(tile, mn ? 64 * BK * 2 : 16, 1024);
+}
+__device__ __forceinline__ uint32_t k_step(int mn) { return mn ? 2048 >> 4 : 32 >> 4; }
+
 // Tile order: bands of BAND M blocks, so that one wave of CTAs touches a band of A row blocks and a few B row blocks
 // instead of all of A, and both operands are re-read from L2 rather than from DRAM.
 template <int BAND>
@@ -464,45 +471,43 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = np::make_idesc(BM, BN, 1, 1, p.a_mn, p.b_mn);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
-        const Tile tl = decode(t);
-        const int rows = tile_rows(tl, 1);
-        if (rows < 0) break;
-        if (rows == 0) continue;
-        if (count_k(p, tl.g) == 0) continue;
-        if (!np::mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 2)) break;
+    const uint32_t idesc = np::make_idesc(BM, BN, 1, 1, p.a_mn, p.b_mn);
+    const uint64_t a_desc0 = operand_desc(smem_base, p.a_mn), b_desc0 = operand_desc(smem_base + A_BYTES, p.b_mn);
+    const uint32_t a_step = k_step(p.a_mn), b_step = k_step(p.b_mn);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+      const Tile tl = decode(t);
+      const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(tl, 1) : 0, 0);
+      if (rows < 0) break;
+      if (rows == 0) continue;
+      if (count_k(p, tl.g) == 0) continue;
+      if (!np::mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 2)) break;
+      np::tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+      uint32_t accum = 0;
+      for_each_k(p, tl.g, [&](int) -> bool {
+        if (!np::mbar_wait_warp(full_bar(stage), phase, abort_flag, KID_GEMM, 3)) return false;
         np::tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
-        uint32_t accum = 0;
-        for_each_k(p, tl.g, [&](int) -> bool {
-          if (!np::mbar_wait(full_bar(stage), phase, abort_flag, KID_GEMM, 3)) return false;
-          np::tc_fence_after();
-          const uint32_t sA = smem_base + stage * STAGE_BYTES;
-          const uint32_t sB = sA + A_BYTES;
+        if (np::elect_one()) {
+          const uint64_t ad = a_desc0 + (uint32_t)(stage * (STAGE_BYTES >> 4)), bd = b_desc0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t bd = p.b_mn ? np::make_smem_desc(sB + kk * 2048, 64 * BK * 2, 1024)
-                                       : np::make_smem_desc(sB + kk * 32, 16, 1024);
-            const uint64_t ad = p.a_mn ? np::make_smem_desc(sA + kk * 2048, 64 * BK * 2, 1024)
-                                       : np::make_smem_desc(sA + kk * 32, 16, 1024);
-            np::tc_mma_f16(tmem_d, ad, bd, idesc, accum);
-            accum = 1;
-          }
+          for (int kk = 0; kk < BK / 16; ++kk)
+            np::tc_mma_f16(tmem_d, ad + kk * a_step, bd + kk * b_step, idesc, kk ? 1u : accum);
           np::tc_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          return true;
-        });
-        np::tc_commit(tfull_bar(acc));
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
-      }
-      if (*abort_flag) __nanosleep(1000000);
+        }
+        __syncwarp();
+        accum = 1;
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        return true;
+      });
+      if (np::elect_one()) np::tc_commit(tfull_bar(acc));
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
+    if (*abort_flag) __nanosleep(1000000);
   } else {
     // ------------------------------------------------------------ epilogue
     const int quarter = warp & 3, half = (warp - 2) >> 2;  // TMEM lanes [32*quarter, 32*quarter+32), column half
@@ -747,38 +752,39 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader's)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = np::make_idesc(TM, BN, 1, 1, p.a_mn, p.b_mn);
+      const uint64_t a_desc0 = operand_desc(smem_base, p.a_mn), b_desc0 = operand_desc(smem_base + A_BYTES, p.b_mn);
+      const uint32_t a_step = k_step(p.a_mn), b_step = k_step(p.b_mn);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
-      for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
+      for (int t = pair; t < num_tiles; t += pairs) {
         const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
-        const int rows = tile_rows(tl, 1);
+        const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(tl, 1) : 0, 0);
         if (rows < 0) break;
         if (rows == 0) continue;
         if (count_k(p, tl.g) == 0) continue;
-        if (!np::mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 12)) break;
+        if (!np::mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 12)) break;
         np::tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
         uint32_t accum = 0;
         k_steps(tl.g, [&](int) -> bool {
-          if (!np::mbar_wait(full_bar(stage), phase, abort_flag, KID_GEMM, 13)) return false;
+          if (!np::mbar_wait_warp(full_bar(stage), phase, abort_flag, KID_GEMM, 13)) return false;
           np::tc_fence_after();
-          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
+          if (np::elect_one()) {
+            const uint64_t ad = a_desc0 + (uint32_t)(stage * (STAGE_BYTES >> 4)), bd = b_desc0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t ad = p.a_mn ? np::make_smem_desc(sA + kk * 2048, 64 * BK * 2, 1024)
-                                       : np::make_smem_desc(sA + kk * 32, 16, 1024);
-            const uint64_t bd = p.b_mn ? np::make_smem_desc(sB + kk * 2048, 64 * BK * 2, 1024)
-                                       : np::make_smem_desc(sB + kk * 32, 16, 1024);
-            tc_mma_f16_pair(tmem_d, ad, bd, idesc, accum);
-            accum = 1;
+            for (int kk = 0; kk < BK / 16; ++kk)
+              tc_mma_f16_pair(tmem_d, ad + kk * a_step, bd + kk * b_step, idesc, kk ? 1u : accum);
+            tc_commit_pair(empty_bar(stage), lead);
           }
-          tc_commit_pair(empty_bar(stage), lead);
+          __syncwarp();
+          accum = 1;
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           return true;
         });
-        tc_commit_pair(tfull_bar(acc), lead);
+        if (np::elect_one()) tc_commit_pair(tfull_bar(acc), lead);
+        __syncwarp();
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
       if (*abort_flag) __nanosleep(1000000);
