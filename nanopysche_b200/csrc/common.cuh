@@ -120,12 +120,12 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // every later wait in the CTA returns false at once so the CTA drains and exits.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int kernel_id, int detail) {
-  if (mbar_try(bar, parity)) return true;
-  uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;   // started by the first 256 failed polls: the timer stays off the path of ordinary waits
   for (uint32_t it = 1;; ++it) {
     if (mbar_try(bar, parity)) return true;
     if ((it & 255u) == 0u) {
       if (*abort_flag) return false;
+      if (t0 == 0) t0 = globaltimer_ns();
       if (globaltimer_ns() - t0 > NP_WAIT_LIMIT_NS) {
         *abort_flag = 1;
         report(NP_ERR_MBAR_TIMEOUT, kernel_id, detail);

@@ -70,10 +70,11 @@ struct GemmParams {
   int* push_ctr;
   int splits;                 // pair kernel: parts of K (cluster of 2 * splits CTAs), 1 = whole
   bool st32, st32_c2;         // rows and column chunks of C / C2 are 32-byte aligned: use 32-byte stores
+  bool tma_c;                 // outputs leave through shared memory and TMA stores (tmC, tmC2)
   const float* bias;          // optional [N] fp32 added to every output row (plain epilogue)
 };
 
-// 64 bytes (32 bf16 packed in 16 registers) to a row: two 32-byte stores when the address allows it (a full sector
+// 64 bytes (16 registers: 32 bf16 or 16 fp32) to a row: two 32-byte stores when the address allows it (a full sector
 // per request - what a row pushed to a peer over NVLink is made of), else four 16-byte stores.
 __device__ __forceinline__ void store64(void* dst, const uint32_t* o, bool st32) {
   if (st32) {
@@ -132,19 +133,24 @@ __device__ __forceinline__ uint32_t k_step(int mn) { return mn ? 2048 >> 4 : 32 
 
 // Tile order: bands of BAND M blocks, so that one wave of CTAs touches a band of A row blocks and a few B row blocks
 // instead of all of A, and both operands are re-read from L2 rather than from DRAM.
+__device__ __forceinline__ int fast_div(int n, int d) {   // n / d for 0 <= n < 2^24 (every role decodes every tile)
+  int q = (int)((float)n * __frcp_rn((float)d));
+  const int r = n - q * d;
+  if (r < 0) --q;
+  else if (r >= d) ++q;
+  return q;
+}
 template <int BAND>
 __device__ __forceinline__ Tile decode_tile(int t, int m_blocks, int n_blocks) {
   Tile tl;
   const int per_group = m_blocks * n_blocks;
-  tl.g = t / per_group;
+  tl.g = t < per_group ? 0 : fast_div(t, per_group);
   const int r = t - tl.g * per_group;
-  const int per_band = BAND * n_blocks;
-  const int band = r / per_band;
-  const int first_m = band * BAND;
+  const int first_m = fast_div(r, BAND * n_blocks) * BAND;
   const int gsize = (m_blocks - first_m) < BAND ? (m_blocks - first_m) : BAND;
-  const int within = r - band * per_band;
-  tl.m_blk = first_m + within % gsize;
-  tl.n_blk = within / gsize;
+  const int within = r - first_m * n_blocks;
+  tl.n_blk = gsize == BAND ? within / BAND : fast_div(within, gsize);
+  tl.m_blk = first_m + within - tl.n_blk * gsize;
   return tl;
 }
 
@@ -172,63 +178,77 @@ __device__ __forceinline__ OutRow out_row(const GemmParams& p, int g, int row) {
   return o;
 }
 
-// Plain epilogue of 32 accumulator columns starting at output column `col`: alpha, bias, accumulate source, output type.
-__device__ __forceinline__ void store_chunk(const GemmParams& p, const OutRow& o, uint32_t* r, int col) {
-  if (!o.ok || col >= p.N) return;
-  const bool full = col + 32 <= p.N;
-  if (p.bias) {  // the same 32 values for every row of the warp: broadcast loads
-    const float inv_alpha = 1.f / p.alpha;
+// 32 accumulator columns from output column `col`: times alpha, plus bias. The conditions are outside the loops: tested per
+// element they cost more than the rest of the epilogue.
+__device__ __forceinline__ void scale_bias(const GemmParams& p, uint32_t* r, int col) {
+  if (p.alpha != 1.f) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float b = (col + i < p.N) ? __ldg(p.bias + col + i) : 0.f;
-      r[i] = __float_as_uint(fmaf(b, inv_alpha, __uint_as_float(r[i])));
+    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * p.alpha);
+  }
+  if (p.bias) {   // the same 32 values for every row of the warp: broadcast loads
+    if (col + 32 <= p.N) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(p.bias + col + i));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (col + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(p.bias + col + i));
     }
   }
-  if (p.out_f32) {
-    float* dst = (float*)o.c + col;
-    if (full) {
+}
+__device__ __forceinline__ void pack32(const uint32_t* r, uint32_t* w) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float4 v = make_float4(__uint_as_float(r[4 * i]) * p.alpha, __uint_as_float(r[4 * i + 1]) * p.alpha,
-                               __uint_as_float(r[4 * i + 2]) * p.alpha, __uint_as_float(r[4 * i + 3]) * p.alpha);
-        if (o.cin) {
+  for (int i = 0; i < 16; ++i) w[i] = np::pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
+
+// Plain epilogue of 32 accumulator columns, stored from the registers (accumulate sources, peer rows, odd alignments).
+__device__ __forceinline__ void store_chunk(const GemmParams& p, const OutRow& o, uint32_t* r, int col) {
+  if (!o.ok || col >= p.N) return;
+  scale_bias(p, r, col);
+  if (col + 32 <= p.N) {
+    if (o.cin) {
+      if (p.out_f32) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
           const float4 c = reinterpret_cast<const float4*>((const float*)o.cin + col)[i];
-          v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
+          r[4 * i] = __float_as_uint(__uint_as_float(r[4 * i]) + c.x);
+          r[4 * i + 1] = __float_as_uint(__uint_as_float(r[4 * i + 1]) + c.y);
+          r[4 * i + 2] = __float_as_uint(__uint_as_float(r[4 * i + 2]) + c.z);
+          r[4 * i + 3] = __float_as_uint(__uint_as_float(r[4 * i + 3]) + c.w);
         }
-        reinterpret_cast<float4*>(dst)[i] = v;
-      }
-    } else {
-      _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
-        float v = __uint_as_float(r[i]) * p.alpha;
-        if (o.cin) v += ((const float*)o.cin + col)[i];
-        dst[i] = v;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint4 c = reinterpret_cast<const uint4*>((const __nv_bfloat16*)o.cin + col)[i];
+          const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 f = np::unpack_bf16(cw[q]);
+            r[8 * i + 2 * q] = __float_as_uint(__uint_as_float(r[8 * i + 2 * q]) + f.x);
+            r[8 * i + 2 * q + 1] = __float_as_uint(__uint_as_float(r[8 * i + 2 * q + 1]) + f.y);
+          }
+        }
       }
     }
-  } else {
-    __nv_bfloat16* dst = (__nv_bfloat16*)o.c + col;
-    if (full) {
-      uint32_t pk[16];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float f[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[8 * i + j]) * p.alpha;
-        if (o.cin) {
-          const uint4 c = reinterpret_cast<const uint4*>((const __nv_bfloat16*)o.cin + col)[i];
-          const float2 c0 = np::unpack_bf16(c.x), c1 = np::unpack_bf16(c.y), c2 = np::unpack_bf16(c.z), c3 = np::unpack_bf16(c.w);
-          f[0] += c0.x; f[1] += c0.y; f[2] += c1.x; f[3] += c1.y;
-          f[4] += c2.x; f[5] += c2.y; f[6] += c3.x; f[7] += c3.y;
-        }
-        pk[4 * i] = np::pack_bf16(f[0], f[1]); pk[4 * i + 1] = np::pack_bf16(f[2], f[3]);
-        pk[4 * i + 2] = np::pack_bf16(f[4], f[5]); pk[4 * i + 3] = np::pack_bf16(f[6], f[7]);
-      }
-      store64(dst, pk, p.st32);
+    if (p.out_f32) {
+      float* dst = (float*)o.c + col;
+      store64(dst, r, p.st32);
+      store64(dst + 16, r + 16, p.st32);
     } else {
-      _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
-        float v = __uint_as_float(r[i]) * p.alpha;
-        if (o.cin) v += __bfloat162float(((const __nv_bfloat16*)o.cin + col)[i]);
-        dst[i] = __float2bfloat16(v);
-      }
+      uint32_t w[16];
+      pack32(r, w);
+      store64((__nv_bfloat16*)o.c + col, w, p.st32);
+    }
+    return;
+  }
+  _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) {
+    float v = __uint_as_float(r[i]);
+    if (p.out_f32) {
+      if (o.cin) v += ((const float*)o.cin)[col + i];
+      ((float*)o.c)[col + i] = v;
+    } else {
+      if (o.cin) v += __bfloat162float(((const __nv_bfloat16*)o.cin)[col + i]);
+      ((__nv_bfloat16*)o.c)[col + i] = __float2bfloat16(v);
     }
   }
 }
@@ -272,13 +292,111 @@ __device__ __forceinline__ void store_swiglu_chunk(const GemmParams& p, const Ou
 // that no MMA of a next tile covers (the only, or the last one of a CTA) takes half as long as with one.
 constexpr int EPI_WARPS = 8;
 constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
+constexpr int STG_BYTES = 4096;   // staging of one epilogue warp: 32 rows of 128 bytes
+
+// A warp's 32 rows of 128 bytes (w: this lane's row, 32 words) to the output at (col, row0, plane): through the warp's
+// staging buffer, in the 128-byte swizzle of the tensor map, and one TMA store. Stored straight from the registers every
+// instruction touches 32 rows, one sector each: a 128 x 256 fp32 tile took about 10 us that way.
+__device__ __forceinline__ void stage_store(const CUtensorMap* tm, uint32_t stg, int lane, const uint32_t* w, int col, int row0,
+                                            int plane) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the buffer's last store has read it
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * 128 + ((j ^ (lane & 7)) << 4)), "r"(w[4 * j]),
+                 "r"(w[4 * j + 1]), "r"(w[4 * j + 2]), "r"(w[4 * j + 3])
+                 : "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tm), "r"(stg), "r"(col),
+                 "r"(row0), "r"(plane)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+// Before the CTA exits: the staging buffer has been read.
+__device__ __forceinline__ void stage_drain(int lane) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
+// 32 accumulator columns of this lane's row (zeros without an accumulator)
+__device__ __forceinline__ void load_acc(uint32_t taddr, bool have_acc, uint32_t* r) {
+  if (have_acc) {
+    np::tmem_ld32(taddr, r);
+    np::tmem_ld_wait();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = 0u;
+  }
+}
 
 // Half `half` of the BN accumulator columns of one 128-row tile: tensor memory (`taddr`: this warp's lanes, first column)
-// through the epilogue of the launch to output row `row`, columns from `n0`. Executed by whole warps (the tensor-memory
-// loads are .sync.aligned).
+// through the epilogue of the launch to output rows row0 .. row0 + 31, columns from `n0`. Executed by whole warps (the
+// tensor-memory loads are .sync.aligned).
 template <int BN>
-__device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t taddr, int g_idx, int row, int n0, int half,
-                                           bool have_acc) {
+__device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmC2, uint32_t stg,
+                                           uint32_t taddr, int g_idx, int row0, int lane, int n0, int half, bool have_acc) {
+  if (p.tma_c) {
+    if (row0 >= p.M) return;
+    if (p.epilogue == 1) {
+      // BN / 2 output columns: 64 per warp for BN = 256; h, then the gate and the up pre-activations
+#pragma unroll 1
+      for (int c = half * (BN / 256); c < (half + 1) * (BN / 256); ++c) {
+        const int col = n0 + c * 64;
+        if (col >= p.N) break;
+        uint32_t w[32];
+#pragma unroll 1
+        for (int out = 0; out < (p.C2 ? 3 : 1); ++out) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            uint32_t g[32], u[32];
+            const uint32_t tg = taddr + c * 64 + q * 32;
+            if (out == 0) {
+              np::tmem_ld32(tg, g);
+              np::tmem_ld32(tg + BN / 2, u);
+              np::tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                g[i] = __float_as_uint(np::silu_f(__uint_as_float(g[i])) * __uint_as_float(u[i]));
+            } else {
+              np::tmem_ld32(out == 1 ? tg : tg + BN / 2, g);
+              np::tmem_ld_wait();
+            }
+            pack32(g, w + 16 * q);
+          }
+          stage_store(out == 0 ? tmC : tmC2, stg, lane, w, col, row0, out == 2 ? 1 : 0);
+        }
+      }
+    } else if (p.out_f32) {
+#pragma unroll 1
+      for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+        const int col = n0 + c * 32;
+        if (col >= p.N) break;
+        uint32_t r[32];
+        load_acc(taddr + c * 32, have_acc, r);
+        scale_bias(p, r, col);
+        stage_store(tmC, stg, lane, r, col, row0, g_idx);
+      }
+    } else {
+#pragma unroll 1
+      for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
+        const int col = n0 + c * 64;
+        if (col >= p.N) break;
+        uint32_t w[32];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          uint32_t r[32];
+          load_acc(taddr + c * 64 + q * 32, have_acc, r);
+          scale_bias(p, r, col + q * 32);
+          pack32(r, w + 16 * q);
+        }
+        stage_store(tmC, stg, lane, w, col, row0, g_idx);
+      }
+    }
+    return;
+  }
+  const int row = row0 + lane;
   const OutRow o = out_row(p, g_idx, row);
   if (p.epilogue == 1) {
     // gate = columns [0, BN/2), up = columns [BN/2, BN)
@@ -296,13 +414,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t taddr, 
     for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
       uint32_t r[32];
       __syncwarp();
-      if (have_acc) {
-        np::tmem_ld32(taddr + c * 32, r);
-        np::tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) r[i] = 0u;
-      }
+      load_acc(taddr + c * 32, have_acc, r);
       store_chunk(p, o, r, n0 + c * 32);
     }
   }
@@ -314,7 +426,8 @@ template <int BN, int STAGES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmAloc,
-                 const __grid_constant__ CUtensorMap tmBloc, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmBloc, const __grid_constant__ CUtensorMap tmC,
+                 const __grid_constant__ CUtensorMap tmC2, const GemmParams p) {
   constexpr int A_BYTES = BM * BK * 2;
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -322,7 +435,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (np::smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t stg_base = smem_base + STAGES * STAGE_BYTES;   // staging of the epilogue warps
+  const uint32_t bar_base = stg_base + EPI_WARPS * STG_BYTES;
   // barriers: full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2]; then tmem ptr, abort flag
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
@@ -354,8 +468,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     *abort_flag = 0;
     np::mbar_fence_init();
+  }
+  if (threadIdx.x == 64) {   // while another warp sets up the barriers
     np::tma_prefetch_desc(&tmA);
     np::tma_prefetch_desc(&tmB);
+    if (p.tma_c) np::tma_prefetch_desc(&tmC);
+    if (p.tma_c && p.C2) np::tma_prefetch_desc(&tmC2);
   }
   if (warp == 1) {
     np::tmem_alloc(np::smem_u32((const void*)tmem_ptr_smem), TMEM_COLS);
@@ -525,8 +643,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 4)) break;
         np::tc_fence_after();
       }
-      store_tile<BN>(p, tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
-                     tl.m_blk * BM + quarter * 32 + lane, n0, half, have_acc);
+      store_tile<BN>(p, &tmC, &tmC2, stg_base + (warp - 2) * STG_BYTES,
+                     tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g, tl.m_blk * BM + quarter * 32,
+                     lane, n0, half, have_acc);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
@@ -549,6 +668,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
     }
+    if (p.tma_c) stage_drain(lane);
   }
 
   np::tc_fence_before();
@@ -627,12 +747,14 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 template <bool SPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmB2, const GemmParams p) {
+                      const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
+                      const __grid_constant__ CUtensorMap tmC2, const GemmParams p) {
   constexpr int BN = PAIR_BN, STAGES = PAIR_STAGES, TM = 2 * BM, HN = BN / 2;
   constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = PAIR_STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (np::smem_u32(smem_raw) + 1023u) & ~1023u;   // the same offset in both CTAs
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t stg_base = smem_base + STAGES * STAGE_BYTES;   // staging of the epilogue warps
+  const uint32_t bar_base = stg_base + EPI_WARPS * STG_BYTES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
@@ -673,17 +795,21 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     *abort_flag = 0;
     np::mbar_fence_init();
+  }
+  if (threadIdx.x == 64) {   // while another warp sets up the barriers
     np::tma_prefetch_desc(&tmA);
     np::tma_prefetch_desc(&tmB);
+    if (p.tma_c) np::tma_prefetch_desc(&tmC);
+    if (p.tma_c && p.C2) np::tma_prefetch_desc(&tmC2);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      np::smem_u32((const void*)tmem_ptr_smem)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  __syncwarp();
   np::tc_fence_before();
-  __syncthreads();
-  cluster_sync();        // the peer's barriers are initialised before anything arrives on them
+  cluster_sync();        // this CTA's and the peer's barriers and tensor memory are set up
   np::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
@@ -807,8 +933,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       if constexpr (SPLIT) { done = true; break; }   // one tile per cluster, finished below
       if (mine)
-        store_tile<BN>(p, tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
-                       tl.m_blk * TM + rank * BM + quarter * 32 + lane, tl.n_blk * bn_out, half, have_acc);
+        store_tile<BN>(p, &tmC, &tmC2, stg_base + (warp - 2) * STG_BYTES,
+                       tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
+                       tl.m_blk * TM + rank * BM + quarter * 32, lane, tl.n_blk * bn_out, half, have_acc);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
@@ -828,6 +955,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       }
     }
+    if (p.tma_c) stage_drain(lane);
   }
   if constexpr (SPLIT) {
     __syncthreads();
@@ -896,9 +1024,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 }
 
 int g_num_sms = 0;
-// Cost of one tile in units of the pair kernel's 256 x 256 tile on two SMs (see np_gemm_bf16).
-constexpr double COST_PAIR = 1.0, COST_256 = 1.15, COST_128 = 0.65;
 
+// Estimated time in us of a launch: a fixed part (setup, first loads, the drain of the last tile) and, per wave of tiles,
+// the K steps one after the other plus what of the drain no MMA covers. Measured on B200 (launches of one kernel back to
+// back in a graph): 256 x 256 output, K = 64 / 2048 / 4096: one-CTA 128 x 128 tiles 5.0 / 16.2 / 27.6, 128 x 256 tiles
+// 5.8 / 17.0 / 28.4, pair 6.6 / 15.2 / 24.0, pair with K in two parts 13.9 / 18.3 (K = 2048 / 4096), in four 13.1 / 15.3;
+// with all SMs busy a K step is 10 to 20 % longer (4096 x 2304 x 4096: 104 / 58 / 51 with the first three).
+struct TileCost { double fixed, step, drain; };
+constexpr TileCost COST_128{4.4, 0.37, 0.6}, COST_256{5.3, 0.40, 0.3}, COST_PAIR{6.0, 0.30, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3},
+    COST_SPLIT4{10.7, 0.30, 0.3};
+// Clusters of four and of eight CTAs that run at once (an SM pair per two CTAs, whole clusters within a GPC)
+constexpr int CLUSTERS4 = 32, CLUSTERS8 = 14;
 }  // namespace
 
 // ------------------------------------------------------------------ host side
@@ -975,9 +1111,25 @@ static int num_sms() {
   return g_num_sms > 0 ? g_num_sms : 148;
 }
 
+// Output [planes][rows, cols] written in boxes of 32 rows x 128 bytes (128-byte swizzle)
+static int make_tmap_out(CUtensorMap* out, const void* base, int f32, long long cols, long long rows, long long planes,
+                         long long ld, long long plane_stride) {
+  NpEncodeTiledFn enc = np_get_encode_tiled();
+  if (!enc) return -1;
+  const int es = f32 ? 4 : 2;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)planes};
+  cuuint64_t strides[2] = {(cuuint64_t)(ld * es), (cuuint64_t)(plane_stride * es)};
+  cuuint32_t box[3] = {(cuuint32_t)(128 / es), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base),
+                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
 template <int BN, int STAGES, bool PAIR>
 static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1) {
-  CUtensorMap tmA, tmB, tmB2, tmAloc, tmBloc;
+  CUtensorMap tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2;
   int rc;
   if (!a.a_mn) rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.K, (uint64_t)a.lda, BK, BM);
   else rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.M, (uint64_t)a.lda, 64, BK);
@@ -998,8 +1150,8 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   // 32-byte stores need every (row, 32-column chunk) address 32-byte aligned; destinations behind peer_base are
   // allocations of the symmetric heap (256-byte aligned)
   static const bool st32_on = !(getenv("NPB200_ST32") != nullptr && getenv("NPB200_ST32")[0] == '0');
-  p.st32 = st32_on && !a.out_f32 && (a.ldc % 16 == 0) && (a.group_stride_c % 16 == 0) &&
-           (a.row_dst || (((uintptr_t)a.C) % 32 == 0));
+  const int per32 = a.out_f32 ? 8 : 16;   // elements of 32 bytes
+  p.st32 = st32_on && (a.ldc % per32 == 0) && (a.group_stride_c % per32 == 0) && (a.row_dst || (((uintptr_t)a.C) % 32 == 0));
   p.st32_c2 = st32_on && a.ldc2 % 16 == 0 && a.N % 16 == 0 && ((uintptr_t)a.C2) % 32 == 0;
   if (a.push_src && a.push_n > 0) {
     if (a.push_n > 8 || (a.push_bytes & 15) || (((uintptr_t)a.push_src) & 15)) return 1;
@@ -1035,7 +1187,21 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   p.epoch_base = a.epoch_base;
   p.b_ready_flags = a.b_ready_flags; p.b_rows_per_flag = a.b_rows_per_flag;
 
-  constexpr int SMEM = STAGES * (PAIR ? PAIR_STAGE_BYTES : BM * BK * 2 + BN * BK * 2) + 1024 + 256;
+  // Plain outputs (dense rows, nothing added from memory, 16-byte aligned) leave by TMA; peer-row tables, accumulation and
+  // other alignments store from registers. The SwiGLU form needs both of its outputs aligned.
+  const int es = a.out_f32 ? 4 : 2;
+  const long long groups = a.mode == 2 ? a.num_groups : 1;
+  p.tma_c = !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue == 0 || BN == 256) && ((uintptr_t)a.C & 15) == 0 &&
+            (a.ldc * es) % 16 == 0 && (groups <= 1 || (a.group_stride_c * es) % 16 == 0) &&
+            (a.epilogue == 0 || !a.C2 || (((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0));
+  tmC = tmA;
+  tmC2 = tmA;
+  if (p.tma_c) {
+    rc = make_tmap_out(&tmC, a.C, a.out_f32, a.N, a.M, groups, a.ldc, groups > 1 ? a.group_stride_c : a.ldc);
+    if (!rc && a.epilogue == 1 && a.C2) rc = make_tmap_out(&tmC2, a.C2, 0, a.N, a.M, 2, a.ldc2, a.N);
+    if (rc) return 800 + rc;
+  }
+  constexpr int SMEM = STAGES * (PAIR ? PAIR_STAGE_BYTES : BM * BK * 2 + BN * BK * 2) + EPI_WARPS * STG_BYTES + 1024 + 256;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
@@ -1063,13 +1229,13 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     cfg.gridDim = dim3((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = SMEM; cfg.stream = stream; cfg.attrs = &at; cfg.numAttrs = 1;
-    const cudaError_t e = splits > 1 ? cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<true>, tmA, tmB, tmB2, p)
-                                     : cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<false>, tmA, tmB, tmB2, p);
+    const cudaError_t e = splits > 1 ? cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<true>, tmA, tmB, tmB2, tmC, tmC2, p)
+                                     : cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<false>, tmA, tmB, tmB2, tmC, tmC2, p);
     if (e != cudaSuccess) return 500 + (int)e;
   } else {
     const int grid = (int)(tiles < cap ? tiles : cap);
     if (grid <= 0) return 0;
-    gemm_bf16_kernel<BN, STAGES><<<grid, GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmB2, tmAloc, tmBloc, p);
+    gemm_bf16_kernel<BN, STAGES><<<grid, GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2, p);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
@@ -1100,29 +1266,38 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
       a.split == 0 && a.max_ctas == 0 && a.alpha != 0.f)
     return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
                             a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
-  // Which kernel. The pair kernel takes the forms without peer-arrival flags on B, pushes or split operands; row-grouped
-  // launches only when their tables come in pairs of 128-row blocks (`paired`).
-  int bn = a.bn, mt = a.mt;
+  // Which kernel: the lowest estimate (TileCost). The pair kernel takes the forms without peer-arrival flags on B, pushes or
+  // split operands; row-grouped launches only when their tables come in pairs of 128-row blocks (`paired`). K in parts is
+  // for dense plain outputs with too few tiles for the SMs.
+  const int nk = (a.K + BK - 1) / BK, sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
+  const bool can_split = plain && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
+  int bn = a.bn, mt = a.mt, splits = 1;
   if (a.epilogue == 1) bn = 256;
   if (bn == 0 || (bn == 256 && mt == 0)) {
-    const int sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
     const long long groups = a.mode == 2 ? a.num_groups : 1;
-    auto waves = [&](int tm, int tn, int units) {
+    // K steps of a group: its share of the token axis in the K-grouped form
+    const double steps = a.mode == 2 ? 2.0 * a.blocks_per_group : nk;
+    auto cost = [&](const TileCost& c, int tm, int tn, int units, int parts) {
       const long long t = (long long)((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn) * groups;
-      return (double)((t + units - 1) / units);
+      const double waves = (double)((t + units - 1) / units);
+      // tiles of a persistent CTA follow one another; a cluster that splits K starts anew for every tile
+      return parts == 1 ? c.fixed + waves * (steps * c.step + c.drain) : waves * (c.fixed + steps / parts * c.step + c.drain);
     };
     const int n256 = a.epilogue == 1 ? 128 : 256;
-    const double c128 = (a.epilogue == 1 || a.bn == 256) ? 1e30 : COST_128 * waves(128, 128, sms);
-    const double c256 = COST_256 * waves(128, n256, sms);
-    const double cpair = (plain && a.M > 128 && sms >= 2 && mt != 1) ? COST_PAIR * waves(256, n256, sms / 2) : 1e30;
-    if (cpair <= c128 && cpair <= c256) { bn = 256; mt = 2; }
-    else bn = c256 <= c128 ? 256 : 128;
+    double best = (a.epilogue == 1 || a.bn == 256) ? 1e30 : cost(COST_128, 128, 128, sms, 1);
+    bn = 128;
+    auto take = [&](double c, int bn_, int mt_, int splits_) {
+      if (c < best) { best = c; bn = bn_; mt = mt_; splits = splits_; }
+    };
+    take(cost(COST_256, 128, n256, sms, 1), 256, 1, 1);
+    if (plain && a.M > 128 && sms >= 2 && a.mt != 1) take(cost(COST_PAIR, 256, n256, sms / 2, 1), 256, 2, 1);
+    if (can_split && a.mt != 1 && a.split == 0 && sms >= 128) {
+      take(cost(COST_SPLIT2, 256, 256, CLUSTERS4, 2), 256, 2, 2);
+      take(cost(COST_SPLIT4, 256, 256, CLUSTERS8, 4), 256, 2, 4);
+    }
   }
-  if (bn == 256 && mt == 2 && plain) {
-    const bool can = a.mode == 0 && a.epilogue == 0 && (a.K + BK - 1) / BK >= 8 && a.max_ctas == 0;
-    const int splits = can && (a.split == 2 || a.split == 4) ? a.split : 1;
-    return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
-  }
+  if (can_split && (a.split == 2 || a.split == 4)) splits = a.split;
+  if (bn == 256 && mt == 2 && plain) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
   if (bn == 256) return launch_gemm<256, 4, false>(a, (cudaStream_t)stream);
   return launch_gemm<128, 6, false>(a, (cudaStream_t)stream);
 }
