@@ -57,7 +57,7 @@ class FeedForward(nn.Module):
         x = copy_to_tp_region(x, self._tp_group, self._tp_size)
         fused = self._fused_w13
         if fused is not None and _lib.on(x) and x.dtype == fused.dtype and self.w1.bias is None:
-            h = act_ops.glu(gemm_ops.linear(x, fused), act)
+            h = gemm_ops.linear_glu(x, fused, act)
         elif _lib.on(x) and x.dtype == torch.bfloat16 and self.w1.bias is None:
             gu = torch.cat([gemm_ops.linear(x, self.w1.weight), gemm_ops.linear(x, self.w3.weight)], dim=-1)
             h = act_ops.glu(gu, act)
