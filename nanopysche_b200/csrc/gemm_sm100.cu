@@ -68,6 +68,8 @@ struct GemmParams {
   const uint4* push_src; long long push_vecs;
   uint4* push_dst[8]; int* push_flag[8]; int push_n;
   int* push_ctr;
+  int k_split;                // > 0: B rows of K steps from here on come from tmB2 (two weights, one contraction)
+  int m_split;                // > 0: output rows from here on go to C2, counted from 0 (one contraction, two outputs)
   int splits;                 // pair kernel: parts of K (cluster of 2 * splits CTAs), 1 = whole
   bool st32, st32_c2;         // rows and column chunks of C / C2 are 32-byte aligned: use 32-byte stores
   bool tma_c;                 // outputs leave through shared memory and TMA stores (tmC, tmC2)
@@ -165,6 +167,11 @@ __device__ __forceinline__ OutRow out_row(const GemmParams& p, int g, int row) {
   OutRow o;
   const int es = p.out_f32 ? 4 : 2;
   o.ok = row < p.M;
+  if (p.m_split && row >= p.m_split) {
+    o.c = (char*)p.C2 + ((size_t)g * p.group_stride_c + (size_t)(row - p.m_split) * p.ldc) * es;
+    o.cin = p.Cin ? o.c : nullptr;       // the accumulating form adds to its own output
+    return o;
+  }
   if (p.row_dst) {
     const long long d = o.ok ? p.row_dst[row] : -1;
     o.ok = o.ok && d >= 0;
@@ -339,6 +346,10 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
                                            uint32_t taddr, int g_idx, int row0, int lane, int n0, int half, bool have_acc) {
   if (p.tma_c) {
     if (row0 >= p.M) return;
+    if (p.m_split && row0 >= p.m_split) {
+      tmC = tmC2;
+      row0 -= p.m_split;
+    }
     if (p.epilogue == 1) {
       // BN / 2 output columns: 64 per warp for BN = 256; h, then the gate and the up pre-activations
 #pragma unroll 1
@@ -577,9 +588,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               np::tma_load_2d(sB, &tmB, full_bar(stage), k0, (int)brow);
             }
           } else {
+            const bool second = p.k_split && k0 >= p.k_split;
+            const CUtensorMap* bm = second ? &tmB2 : &tmB;
+            const int kb = k0 + bk_off - (second ? p.k_split : 0);
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
-              np::tma_load_2d(sB + c * (64 * BK * 2), &tmB, full_bar(stage), (int)brow + c * 64, k0 + bk_off);
+              np::tma_load_2d(sB + c * (64 * BK * 2), bm, full_bar(stage), (int)brow + c * 64, kb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           return true;
@@ -861,9 +875,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           if (!p.b_mn) {
             tma_load_2d_pair(sB, bm, fb, k0, (int)(nrow + goff));
           } else {
+            const bool second = p.k_split && k0 >= p.k_split;
+            const CUtensorMap* bk = second ? &tmB2 : bm;
+            const int kb = k0 + (int)goff - (second ? p.k_split : 0);
 #pragma unroll
-            for (int c = 0; c < HN / 64; ++c)
-              tma_load_2d_pair(sB + c * (64 * BK * 2), bm, fb, nrow + c * 64, k0 + (int)goff);
+            for (int c = 0; c < HN / 64; ++c) tma_load_2d_pair(sB + c * (64 * BK * 2), bk, fb, nrow + c * 64, kb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           return true;
@@ -1100,6 +1116,8 @@ struct NpGemmArgs {
   int mt;             // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles on a pair of CTAs)
   int split;          // parts of K on the pair kernel: 0 = choose, 1, 2 or 4 (dense form, plain epilogue)
   int paired;         // row-grouped form: blocks 2 i and 2 i + 1 share their group and their arrival flag
+  int k_split;        // > 0 (MN-major B): K rows [0, k_split) of a group come from B, the rest from B2 (multiple of 64)
+  int m_split;        // > 0: output rows [0, m_split) go to C, the rest to C2 (layout of C; multiple of 256)
 };
 
 static int num_sms() {
@@ -1139,8 +1157,9 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   else rc = np_make_tmap_2d(&tmB, a.B, 2, (uint64_t)a.b_rows, (uint64_t)a.N, (uint64_t)a.ldb, 64, BK);
   if (rc) return 200 + rc;
   tmB2 = tmB;
-  if (a.epilogue == 1) {
-    rc = np_make_tmap_2d(&tmB2, a.B2, 2, (uint64_t)a.b_rows, (uint64_t)a.K, (uint64_t)a.ldb, BK, b_box_rows);
+  if (a.epilogue == 1 || a.k_split > 0) {
+    if (!a.b_mn) rc = np_make_tmap_2d(&tmB2, a.B2, 2, (uint64_t)a.b_rows, (uint64_t)a.K, (uint64_t)a.ldb, BK, b_box_rows);
+    else rc = np_make_tmap_2d(&tmB2, a.B2, 2, (uint64_t)a.b_rows, (uint64_t)a.N, (uint64_t)a.ldb, 64, BK);
     if (rc) return 300 + rc;
   }
   tmAloc = tmA;
@@ -1151,7 +1170,8 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   // allocations of the symmetric heap (256-byte aligned)
   static const bool st32_on = !(getenv("NPB200_ST32") != nullptr && getenv("NPB200_ST32")[0] == '0');
   const int per32 = a.out_f32 ? 8 : 16;   // elements of 32 bytes
-  p.st32 = st32_on && (a.ldc % per32 == 0) && (a.group_stride_c % per32 == 0) && (a.row_dst || (((uintptr_t)a.C) % 32 == 0));
+  p.st32 = st32_on && (a.ldc % per32 == 0) && (a.group_stride_c % per32 == 0) &&
+           (a.row_dst || (((uintptr_t)a.C) % 32 == 0 && (a.m_split == 0 || ((uintptr_t)a.C2) % 32 == 0)));
   p.st32_c2 = st32_on && a.ldc2 % 16 == 0 && a.N % 16 == 0 && ((uintptr_t)a.C2) % 32 == 0;
   if (a.push_src && a.push_n > 0) {
     if (a.push_n > 8 || (a.push_bytes & 15) || (((uintptr_t)a.push_src) & 15)) return 1;
@@ -1159,7 +1179,7 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     p.push_ctr = a.push_ctr;
     for (int r = 0; r < a.push_n; ++r) { p.push_dst[r] = (uint4*)a.push_dst[r]; p.push_flag[r] = a.push_flag[r]; }
   }
-  p.m_rot = a.m_rot; p.n_rot = a.n_rot;
+  p.m_rot = a.m_rot; p.n_rot = a.n_rot; p.k_split = a.k_split; p.m_split = a.m_split;
   if (a.A_loc && !a.a_mn && a.a_loc_hi > a.a_loc_lo && a.a_loc_lo % BM == 0) {
     rc = np_make_tmap_2d(&tmAloc, a.A_loc, 2, (uint64_t)(a.a_loc_hi - a.a_loc_lo), (uint64_t)a.K, (uint64_t)a.lda_loc, BK, BM);
     if (rc) return 600 + rc;
@@ -1193,11 +1213,14 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   const long long groups = a.mode == 2 ? a.num_groups : 1;
   p.tma_c = !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue == 0 || BN == 256) && ((uintptr_t)a.C & 15) == 0 &&
             (a.ldc * es) % 16 == 0 && (groups <= 1 || (a.group_stride_c * es) % 16 == 0) &&
-            (a.epilogue == 0 || !a.C2 || (((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0));
+            (a.epilogue == 0 || !a.C2 || (((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0)) &&
+            (a.m_split == 0 || ((uintptr_t)a.C2 & 15) == 0);
   tmC = tmA;
   tmC2 = tmA;
   if (p.tma_c) {
-    rc = make_tmap_out(&tmC, a.C, a.out_f32, a.N, a.M, groups, a.ldc, groups > 1 ? a.group_stride_c : a.ldc);
+    const long long gs = groups > 1 ? a.group_stride_c : a.ldc;
+    rc = make_tmap_out(&tmC, a.C, a.out_f32, a.N, a.m_split > 0 ? a.m_split : a.M, groups, a.ldc, gs);
+    if (!rc && a.m_split > 0) rc = make_tmap_out(&tmC2, a.C2, a.out_f32, a.N, a.M - a.m_split, groups, a.ldc, gs);
     if (!rc && a.epilogue == 1 && a.C2) rc = make_tmap_out(&tmC2, a.C2, 0, a.N, a.M, 2, a.ldc2, a.N);
     if (rc) return 800 + rc;
   }
@@ -1258,6 +1281,9 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
       return 2;
     ctx_bound = true;
   }
+  if (a.k_split < 0 || a.m_split < 0 || (a.k_split > 0 && (!a.b_mn || a.mode == 2 || a.epilogue != 0 || a.k_split % BK)) ||
+      (a.m_split > 0 && (a.row_dst || a.epilogue != 0 || a.m_split % 256 || a.m_split >= a.M || (a.Cin && a.Cin != a.C))))
+    return 1;
   if ((a.lda % 8) || (a.ldb % 8) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15)) return 1;
   const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
                      (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
@@ -1270,7 +1296,7 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
   // split operands; row-grouped launches only when their tables come in pairs of 128-row blocks (`paired`). K in parts is
   // for dense plain outputs with too few tiles for the SMs.
   const int nk = (a.K + BK - 1) / BK, sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
-  const bool can_split = plain && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
+  const bool can_split = plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
   int bn = a.bn, mt = a.mt, splits = 1;
   if (a.epilogue == 1) bn = 256;
   if (bn == 0 || (bn == 256 && mt == 0)) {

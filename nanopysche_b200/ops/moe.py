@@ -276,8 +276,9 @@ class FusedMoERuntime:
         _lib.check(_lib.lib().np_ep_combine(C.byref(a), C.c_void_p(_lib.stream())), "ep_combine")
 
     def grouped_gemm(self, A, B, *, N, K, b_mn, group_stride_b, out=None, B2=None, C2=None, wait_epoch=0,
-                     push_ptrs=None, push_epoch=0, Cin=None, out_dtype=torch.bfloat16):
-        """Row-grouped GEMM over the receive-buffer layout (mode 1)."""
+                     push_ptrs=None, push_epoch=0, out_dtype=torch.bfloat16, k_split=0):
+        """Row-grouped GEMM over the receive-buffer layout (mode 1). ``B2``: the up weight of the SwiGLU form, or with
+        ``k_split`` the weight that the contraction continues with from there on."""
         g = _lib.GemmArgs()
         M = self.rows_total
         if out is None and push_ptrs is None:
@@ -292,7 +293,9 @@ class FusedMoERuntime:
         g.mblk_group, g.mblk_rows = self.mblk_group.data_ptr(), self.mblk_rows.data_ptr()
         g.group_stride_b = group_stride_b
         g.mblk_flag = self.mblk_flag.data_ptr()
-        if B2 is not None:
+        if k_split:
+            g.B2, g.k_split = B2.data_ptr(), k_split
+        elif B2 is not None:
             g.B2, g.epilogue = B2.data_ptr(), 1
             g.C2 = C2.data_ptr() if C2 is not None else None
             g.ldc2 = C2.stride(0) if C2 is not None else 0
@@ -308,8 +311,6 @@ class FusedMoERuntime:
         else:
             g.C, g.ldc = out.data_ptr(), out.stride(0)
             g.out_f32 = int(out.dtype == torch.float32)
-        if Cin is not None:
-            g.Cin, g.ldcin = Cin.data_ptr(), Cin.stride(0)
         g.epoch_base = self.heap.epoch_base.data_ptr()
         _lib.check(_lib.lib().np_gemm_bf16(C.byref(g), C.c_void_p(_lib.stream())), "grouped_gemm")
         return out
@@ -330,17 +331,26 @@ class FusedMoERuntime:
         return gemm_mxfp8(aq, sfa, bq, sfb, out=out, mblk_group=self.mblk_group, mblk_rows=self.mblk_rows,
                           rows_per_group=N, fill=fill)
 
-    def grouped_wgrad(self, A, Bm, w: torch.Tensor, *, M, N):
+    def grouped_wgrad(self, A, Bm, w: torch.Tensor, *, M, N, w_second: torch.Tensor | None = None):
         """dW[g] (+)= A[rows of g]^T @ B[rows of g] for every local expert g (mode 2), into ``main_grad``
-        when the weight has one, else a fresh tensor that is returned."""
+        when the weight has one, else a fresh tensor that is returned. ``w_second``: a weight whose gradient is the next
+        ``M`` columns of ``A`` against the same rows (gate and up): one launch for both, a pair is returned."""
+        ws = (w,) if w_second is None else (w, w_second)
+        if w_second is not None and (M % 256 or len({(getattr(t, "main_grad", None) is None,
+                                                       bool(getattr(t, "_main_grad_dirty", False))) for t in ws}) > 1):
+            return (self.grouped_wgrad(A[:, :M], Bm, w, M=M, N=N), self.grouped_wgrad(A[:, M:], Bm, w_second, M=M, N=N))
         mg = getattr(w, "main_grad", None)
         first = not getattr(w, "_main_grad_dirty", False)
-        out = mg if mg is not None else torch.empty((self.E_local * M, N), device=A.device, dtype=torch.float32)
+        outs = [t.main_grad if mg is not None else
+                torch.empty((self.E_local * M, N), device=A.device, dtype=torch.float32) for t in ws]
+        out = outs[0]
         g = _lib.GemmArgs()
         g.A, g.B, g.C = A.data_ptr(), Bm.data_ptr(), out.data_ptr()
         g.lda, g.ldb, g.ldc = A.stride(0), Bm.stride(0), N
         g.a_rows, g.b_rows = A.shape[0], Bm.shape[0]
-        g.M, g.N, g.K = M, N, self.rows_total
+        g.M, g.N, g.K = M * len(ws), N, self.rows_total
+        if w_second is not None:
+            g.C2, g.m_split = outs[1].data_ptr(), M
         g.a_mn, g.b_mn, g.mode, g.alpha = 1, 1, 2, 1.0
         g.out_f32 = 1
         g.accumulate = int(mg is not None and not first)
@@ -348,9 +358,11 @@ class FusedMoERuntime:
         g.num_groups, g.blocks_per_group, g.group_stride_c = self.E_local, self.N * self.bpr, M * N
         _lib.check(_lib.lib().np_gemm_bf16(C.byref(g), C.c_void_p(_lib.stream())), "grouped_wgrad")
         if mg is not None:
-            w._main_grad_dirty = True
-            return None
-        return out.to(w.dtype)
+            for t in ws:
+                t._main_grad_dirty = True
+            return None if w_second is None else (None, None)
+        res = tuple(o.to(t.dtype) for o, t in zip(outs, ws))
+        return res[0] if w_second is None else res
 
 
 # ------------------------------------------------------------------------------------------------ the layer
@@ -435,18 +447,17 @@ class _FusedMoE(torch.autograd.Function):
         del hh
         dgu = glu_bwd(gu, dh)
         del dh
-        dg, du = dgu[:, :H], dgu[:, H:]
         if rt.fp8:  # the rows arrived as e4m3: dequantise once for the (bf16) weight-gradient GEMMs
             from .gemm_mxfp8 import mx_dequantize_bf16
 
             xr = mx_dequantize_bf16(rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer])
         else:
             xr = rt.recv_x[layer]
-        dw1 = rt.grouped_wgrad(dg, xr, w1, M=H, N=D)
-        dw3 = rt.grouped_wgrad(du, xr, w3, M=H, N=D)
-        # dX = dG @ w1 + dU @ w3, pushed back to the sources
-        part = rt.grouped_gemm(dg, w1, N=D, K=H, b_mn=True, group_stride_b=H)
-        rt.grouped_gemm(du, w3, N=D, K=H, b_mn=True, group_stride_b=H, push_ptrs=rt.p_ret_g, push_epoch=e2, Cin=part)
+        dw1, dw3 = rt.grouped_wgrad(dgu, xr, w1, M=H, N=D, w_second=w3)
+        # dX = [dG | dU] @ [w1; w3], one contraction over both weights (no bf16 partial result in between), pushed back to
+        # the sources. H is a multiple of 256 (MoEBase), the K steps of 64 never straddle the two.
+        rt.grouped_gemm(dgu, w1, N=D, K=2 * H, b_mn=True, group_stride_b=H, B2=w3, k_split=H, push_ptrs=rt.p_ret_g,
+                        push_epoch=e2)
         dx = torch.empty((T, D), device=dev, dtype=torch.bfloat16)
         rt.combine(rt.ret_g, slot_pos, None, dx, sent, e2)
         dshared = None
