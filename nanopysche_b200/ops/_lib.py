@@ -244,7 +244,9 @@ def on(t: torch.Tensor) -> bool:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (``torch.cuda.current_stream()`` builds a Python object for it,
+    which took several times as long as the rest of a launch's argument handling)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
@@ -314,32 +316,42 @@ def wait_stats(reset: bool = False) -> dict | None:
     return {"exposed_ms": sum(vals) / max(len(vals), 1) / 1e6, "max_sm_ms": max(vals) / 1e6 if vals else 0.0}
 
 
-def call(name: str, *args) -> None:
-    """Call ``np_<name>`` with the current stream appended; scalars are wrapped by type."""
+_BOUND: dict = {}   # name -> library function with its argument types declared
+
+
+def _bind(name: str, args):
+    """Declare the argument types of ``np_<name>`` from its first call (every call site passes the same types): ctypes
+    then converts plain Python values itself."""
     fn = getattr(lib(), "np_" + name)
-    conv = []
+    types = []
     for a in args:
-        if isinstance(a, torch.Tensor):
-            conv.append(c_void_p(a.data_ptr()))
-        elif a is None:
-            conv.append(c_void_p(0))
+        if a is None or isinstance(a, torch.Tensor):
+            types.append(c_void_p)
         elif isinstance(a, float):
-            conv.append(c_float(a))
+            types.append(c_float)
         elif isinstance(a, LL):
-            conv.append(c_ll(int(a)))
-        elif isinstance(a, (bool, int)):
-            conv.append(c_int(int(a)))
+            types.append(c_ll)
+        elif isinstance(a, int):
+            types.append(c_int)
         else:
-            conv.append(a)
-    conv.append(c_void_p(stream()))
+            types.append(type(a))
+    fn.argtypes = [*types, c_void_p]
+    _BOUND[name] = fn
+    return fn
+
+
+def call(name: str, *args) -> None:
+    """Call ``np_<name>`` with the current stream appended; scalars are converted by type, tensors to their address."""
+    fn = _BOUND.get(name) or _bind(name, args)
+    vals = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
     if NVTX:
         torch.cuda.nvtx.range_push("np_" + name)
         try:
-            check(fn(*conv), name)
+            check(fn(*vals, stream()), name)
         finally:
             torch.cuda.nvtx.range_pop()
         return
-    check(fn(*conv), name)
+    check(fn(*vals, stream()), name)
 
 
 class LL(int):
