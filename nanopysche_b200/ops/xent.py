@@ -33,7 +33,7 @@ class _Xent(torch.autograd.Function):
     def backward(ctx, g):
         logits, labels, lse, inv = ctx.saved_tensors
         rows, V = logits.shape
-        dlogits = torch.empty_like(logits)
+        dlogits = torch.empty((rows, logits.stride(0)), device=logits.device, dtype=logits.dtype)[:, :V]   # the same row stride
         gs = g.reshape(1).float().contiguous()
         _lib.call("xent_bwd", logits, labels, lse, gs, inv, dlogits, rows, V, _lib.LL(logits.stride(0)),
                   _lib.LL(ctx.ignore_index))
@@ -42,7 +42,8 @@ class _Xent(torch.autograd.Function):
 
 def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
     """Mean token cross-entropy of ``logits [rows, V]`` against ``labels [rows]``."""
-    if _lib.on(logits) and logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and logits.stride(0) % 8 == 0:
+    if _lib.on(logits) and logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and logits.stride(0) % 8 == 0 and \
+            logits.stride(0) >= logits.shape[1]:
         return _Xent.apply(logits, labels.contiguous().long(), ignore_index)
     return F.cross_entropy(logits.float(), labels.long(), ignore_index=ignore_index)
 
@@ -50,7 +51,8 @@ def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int 
 def _rows_fwd(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int):
     """Per-row loss (0 for ignored rows) and log-sum-exp of one chunk of logits."""
     rows, V = logits.shape
-    if _lib.on(logits) and logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and logits.stride(0) % 8 == 0:
+    if _lib.on(logits) and logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and logits.stride(0) % 8 == 0 and \
+            logits.stride(0) >= logits.shape[1]:
         loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
         lse = torch.empty(rows, device=logits.device, dtype=torch.float32)
         _lib.call("xent_fwd", logits, labels, loss, lse, rows, V, _lib.LL(logits.stride(0)), _lib.LL(ignore_index))
@@ -66,8 +68,9 @@ def _rows_bwd(logits: torch.Tensor, labels: torch.Tensor, lse: torch.Tensor, gs:
               ignore_index: int) -> torch.Tensor:
     """``(softmax - onehot) * gs * inv`` for one chunk (zero rows where the label is ignored), in the logits' dtype."""
     rows, V = logits.shape
-    if _lib.on(logits) and logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and logits.stride(0) % 8 == 0:
-        dlogits = torch.empty_like(logits)
+    if _lib.on(logits) and logits.dtype == torch.bfloat16 and logits.stride(1) == 1 and logits.stride(0) % 8 == 0 and \
+            logits.stride(0) >= logits.shape[1]:
+        dlogits = torch.empty((rows, logits.stride(0)), device=logits.device, dtype=logits.dtype)[:, :V]
         _lib.call("xent_bwd", logits, labels, lse, gs, inv, dlogits, rows, V, _lib.LL(logits.stride(0)),
                   _lib.LL(ignore_index))
         return dlogits
