@@ -247,6 +247,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int qb = nqb - 1 - (int)blockIdx.y;
   const int h = blockIdx.x % p.Hq, b = blockIdx.x / p.Hq;
   const int hkv = h / (p.Hq / p.Hkv);
+  if (p.q_blk_pos || p.k_blk_pos) np::pdl_wait();   // position tables are memory
   const int q_pos0 = p.q_blk_pos ? p.q_blk_pos[qb] : qb * BQ + p.q_off;
   const int total_blocks = p.n_src * p.src_blocks;
   auto k_pos0 = [&](int j) { return p.k_blk_pos ? p.k_blk_pos[j] : (j % p.src_blocks) * BKV; };
@@ -269,6 +270,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   np::tc_fence_after();
   const uint32_t tmem = *tmem_ptr_smem;
+  np::pdl_begin();
   const uint32_t tO = tmem + F_O;
   push_kv(p.push, reinterpret_cast<volatile int*>(tail + 8));
 
@@ -530,6 +532,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   np::tc_fence_after();
   const uint32_t tmem = *tmem_ptr_smem;
+  np::pdl_begin();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -822,6 +825,9 @@ NP_API int np_attn_prof_read(unsigned long long* out8, int reset) {
 }
 #endif
 
+// a kernel of 20 us and more
+static bool busy(int B, int H, int Sq, int Sk, int hd) { return 4.0 * B * H * Sq * (double)Sk * hd > 2e10; }
+
 template <int HD>
 static int launch_fwd2(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const FwdParams& p,
                        cudaStream_t stream) {
@@ -835,7 +841,7 @@ static int launch_fwd2(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUt
     attr_set = true;
   }
   dim3 grid(p.Hq * p.B, (p.Sq + 2 * BQ - 1) / (2 * BQ));
-  attn_fwd2_kernel<HD><<<grid, 320, SMEM, stream>>>(tmQ, tmK, tmV, p);
+  np_launch_if(busy(p.B, p.Hq, p.Sq, p.src_len, HD), attn_fwd2_kernel<HD>, grid, 320, SMEM, stream, 1, tmQ, tmK, tmV, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
@@ -854,7 +860,7 @@ static int launch_fwd(const CUtensorMap& tmQ, const TmapList& tmK, const TmapLis
     attr_set = true;
   }
   dim3 grid(p.Hq * p.B, (p.Sq + BQ - 1) / BQ);
-  attn_fwd_kernel<NS, HD><<<grid, nthreads(NS), SMEM, stream>>>(tmQ, tmK, tmV, p);
+  np_launch_if(busy(p.B, p.Hq, p.Sq, p.src_len, HD), attn_fwd_kernel<NS, HD>, grid, nthreads(NS), SMEM, stream, 1, tmQ, tmK, tmV, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
@@ -943,6 +949,7 @@ __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
                   const __nv_bfloat16* __restrict__ d_o, long long d_sb, long long d_ss, long long d_sh,
                   float* __restrict__ delta, int B, int S, int H) {
+  np::pdl_begin();
   constexpr int L = HD / 8;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)B * S * H, w = t / L;
@@ -994,6 +1001,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int qb = nqb - 1 - (int)blockIdx.y;   // heaviest first across the whole grid, as in the forward
   const int h = blockIdx.x % p.Hq, b = blockIdx.x / p.Hq;
   const int hkv = h / (p.Hq / p.Hkv);
+  if (p.q_blk_pos || p.k_blk_pos) np::pdl_wait();   // position tables are memory
   const int q_pos0 = p.q_blk_pos ? p.q_blk_pos[qb] : qb * BQ + p.q_off;
   const int total_blocks = p.n_src * p.src_blocks;
   auto k_pos0 = [&](int j) { return p.k_blk_pos ? p.k_blk_pos[j] : (j % p.src_blocks) * BKV; };
@@ -1015,6 +1023,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   np::tc_fence_after();
   const uint32_t tmem = *tmem_ptr_smem;
+  np::pdl_begin();
   const uint32_t tdP = tmem + 256, tdQ = tmem + 384;   // S buffers at columns 0 and 128
   push_kv(p.push, reinterpret_cast<volatile int*>(tail + 12));
 
@@ -1211,6 +1220,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   // grid.x over (kv head, batch), grid.y over KV blocks: the first KV block is seen by the most Q blocks
   const int jb = blockIdx.y, hkv = blockIdx.x % p.Hkv, b = blockIdx.x / p.Hkv;
   const int n_rep = p.Hq / p.Hkv;
+  if (p.q_blk_pos || p.k_blk_pos) np::pdl_wait();   // position tables are memory
   const int k_pos0 = p.k_blk_pos ? p.k_blk_pos[jb] : jb * BKV;
   auto q_pos0_of = [&](int src, int i) {
     return p.q_blk_pos ? p.q_blk_pos[src * p.src_blocks + i] : i * BQ + p.q_off;
@@ -1241,6 +1251,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   __syncthreads();
   np::tc_fence_after();
   const uint32_t tmem = *tmem_ptr_smem;
+  np::pdl_begin();
   const uint32_t tSt = tmem, tdPt = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
 
   if (warp == 0) {
@@ -1503,8 +1514,8 @@ static int launch_bwd(dim3 gq, dim3 gk, int skip, const CUtensorMap& tmQ, const 
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
   }
-  if (!(skip & 1)) attn_bwd_dq_kernel<NS, HD><<<gq, nthreads(NS), SMEM_DQ, stream>>>(tmQ, tmdO, lK, lV, pq);
-  if (!(skip & 2)) attn_bwd_dkv_kernel<NS, HD><<<gk, nthreads(NS), SMEM_DKV, stream>>>(tmK, tmV, lQ, ldO, pk);
+  if (!(skip & 1)) np_launch_if(busy(pq.B, pq.Hq, pq.Sq, pq.Sk, HD), attn_bwd_dq_kernel<NS, HD>, gq, nthreads(NS), SMEM_DQ, stream, 1, tmQ, tmdO, lK, lV, pq);
+  if (!(skip & 2)) np_launch_if(busy(pq.B, pq.Hq, pq.Sq, pq.Sk, HD), attn_bwd_dkv_kernel<NS, HD>, gk, nthreads(NS), SMEM_DKV, stream, 1, tmK, tmV, lQ, ldO, pk);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
@@ -1519,7 +1530,7 @@ NP_API int np_attn_bwd(const NpAttnBwdArgs* a, void* stream_) {
   if (a->phase & 1) {
     const long long lanes = (long long)a->B * a->Sq * a->Hq * (hd / 8);
     auto kern = hd == 128 ? attn_delta_kernel<128> : attn_delta_kernel<64>;
-    kern<<<(unsigned)((lanes + 255) / 256), 256, 0, stream>>>(
+    np_launch(kern, (unsigned)((lanes + 255) / 256), 256, 0, stream, 1,
         (const __nv_bfloat16*)a->o, a->o_sb, a->o_ss, a->o_sh, (const __nv_bfloat16*)a->d_o, a->do_sb, a->do_ss, a->do_sh,
         a->delta, a->B, a->Sq, a->Hq);
   }

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
                                                          __nv_bfloat16* __restrict__ h_out,
                                                          float* __restrict__ rstd, int rows, int cols,
                                                          float eps) {
+  np::pdl_begin();
   __shared__ float red[32];
   const int nvec = cols >> 3;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_quant_fwd_kernel(const __nv_bfloat
                                                                float* __restrict__ rstd, uint8_t* __restrict__ q,
                                                                float* __restrict__ scales, int rows, int cols,
                                                                float eps) {
+  np::pdl_begin();
   __shared__ float red[32];
   const int nvec = cols >> 3, bpr = cols >> 7;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -199,6 +201,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ dres,
                                                          __nv_bfloat16* __restrict__ dx,
                                                          float* __restrict__ dw_partial, int rows, int cols) {
+  np::pdl_begin();
   __shared__ float red[32];
   const int nvec = cols >> 3;
   float dwacc[MAXV][8];
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __
 // dependent loads.
 __global__ void __launch_bounds__(256) colsum_tall_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                           int parts, int cols, int accumulate) {
+  np::pdl_begin();
   __shared__ float red[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -324,6 +328,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_warp_kernel(const __nv_bfloat1
                                                               const __nv_bfloat16* __restrict__ dres,
                                                               __nv_bfloat16* __restrict__ dx,
                                                               float* __restrict__ dw_partial, int rows, int cols) {
+  np::pdl_begin();
   extern __shared__ float s_dw[];   // [8 warps][cols]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* mine = s_dw + (size_t)warp * cols;
@@ -395,6 +400,7 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
 // gu = [gate | up] rows of 2F; h = act(gate) * up
 __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h,
                                long long rows, int F, int act) {
+  np::pdl_begin();
   const long long nvec = rows * (F >> 3);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
        i += (long long)gridDim.x * blockDim.x) {
@@ -411,6 +417,7 @@ __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat
 
 __global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
                                __nv_bfloat16* __restrict__ dgu, long long rows, int F, int act) {
+  np::pdl_begin();
   const long long nvec = rows * (F >> 3);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
        i += (long long)gridDim.x * blockDim.x) {
@@ -447,6 +454,7 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* 
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             const int* __restrict__ pos_ids, long long T, int S, int pos_off, int H, int hd,
                             int rot, long long ld_in, long long ld_out, float sign) {
+  np::pdl_begin();
   const int half = rot >> 1;
   const int vec_per_head = hd >> 3;
   const long long total = T * H * vec_per_head;
@@ -498,6 +506,7 @@ __global__ void __launch_bounds__(256) qkv_rope_kernel(HeadSrc s0, HeadSrc s1, H
                                                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                        const int* __restrict__ pos_ids, long long T, int S, int pos_off,
                                                        int hd, int rot, int rot_heads, float sign) {
+  np::pdl_begin();
   const int H = s0.heads + s1.heads + s2.heads;
   const int half = rot >> 1;
   const int hv = half >> 3;                    // 8-wide slices in one half of the rotated range
@@ -568,6 +577,7 @@ __global__ void __launch_bounds__(256) qkv_norm_rope_fwd_kernel(
     const float* __restrict__ bq, const float* __restrict__ gk, const float* __restrict__ bk, float eps,
     __nv_bfloat16* __restrict__ out, float2* __restrict__ stats, const float* __restrict__ cos_t,
     const float* __restrict__ sin_t, const int* __restrict__ pos_ids, long long T, int S, int pos_off) {
+  np::pdl_begin();
   constexpr int HD = 128, HALF = 64;
   const int nrot = hq + hkv, H = hq + 2 * hkv;
   const int items = nrot * 8 + hkv * 16;
@@ -624,6 +634,7 @@ __global__ void __launch_bounds__(256) qkv_norm_rope_bwd_kernel(
     const float* __restrict__ gq, const float* __restrict__ gk, const float2* __restrict__ stats,
     __nv_bfloat16* __restrict__ dqkv, float* __restrict__ partial, const float* __restrict__ cos_t,
     const float* __restrict__ sin_t, const int* __restrict__ pos_ids, long long T, int S, int pos_off) {
+  np::pdl_begin();
   constexpr int HD = 128, HALF = 64;
   __shared__ float s_acc[4][HD];
   const int nrot = hq + hkv, H = hq + 2 * hkv;
@@ -718,6 +729,7 @@ __global__ void __launch_bounds__(256) qkv_norm_rope_bwd_kernel(
 __global__ void rope_table_kernel(float* __restrict__ cos_t, float* __restrict__ sin_t, int S, int rot,
                                   float base, int scaling, float factor, float orig_len, float low_f,
                                   float high_f, float mscale) {
+  np::pdl_begin();
   const int half = rot >> 1;
   const long long total = (long long)S * half;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -753,6 +765,7 @@ __global__ void __launch_bounds__(NT) xent_fwd_kernel(const __nv_bfloat16* __res
                                                       const long long* __restrict__ labels,
                                                       float* __restrict__ loss, float* __restrict__ lse,
                                                       int rows, int V, long long ld, long long ignore) {
+  np::pdl_begin();
   __shared__ float red[32];
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const __nv_bfloat16* lr = logits + (size_t)r * ld;
@@ -792,6 +805,7 @@ __global__ void __launch_bounds__(NT) xent_bwd_kernel(const __nv_bfloat16* __res
                                                       const float* __restrict__ inv_count,
                                                       __nv_bfloat16* __restrict__ dlogits, int rows, int V,
                                                       long long ld, long long ignore) {
+  np::pdl_begin();
   const float sc = gscale[0] * inv_count[0];
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const __nv_bfloat16* lr = logits + (size_t)r * ld;
@@ -824,6 +838,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g,
                              float* __restrict__ v, __nv_bfloat16* __restrict__ w16, long long n, float lr,
                              float b1, float b2, float eps, float wd, float bc1, float bc2,
                              const float* __restrict__ gscale, const float* __restrict__ hyper) {
+  np::pdl_begin();
   const float gs = gscale ? gscale[0] : 1.f;
   if (hyper) { lr = hyper[0]; bc1 = hyper[1]; bc2 = hyper[2]; }  // device-resident schedule (graph replay)
   const long long nvec = n >> 2;
@@ -861,6 +876,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g,
 // partial[b] = sum over this CTA's grid-stride slice of x^2 (fp32 input)
 __global__ void __launch_bounds__(NT) sumsq_kernel(const float* __restrict__ x, long long n,
                                                    float* __restrict__ partial) {
+  np::pdl_begin();
   __shared__ float red[32];
   float s = 0.f;
   const long long nvec = n >> 2;
@@ -878,6 +894,7 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const float* __restrict__ x, 
 // out[0] = min(1, max_norm / (sqrt(sum(partial) + extra_sq[0]) + 1e-6)); out[1] = the norm.
 __global__ void clip_coef_kernel(const float* __restrict__ partial, int parts, const float* __restrict__ extra_sq,
                                  float max_norm, float* __restrict__ out) {
+  np::pdl_begin();
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < parts; i += blockDim.x) s += partial[i];
@@ -891,6 +908,7 @@ __global__ void clip_coef_kernel(const float* __restrict__ partial, int parts, c
 }
 
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+  np::pdl_begin();
   const long long nvec = n >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
        i += (long long)gridDim.x * blockDim.x) {
@@ -920,13 +938,13 @@ NP_API int np_rmsnorm_fwd(const void* x, const void* res, const float* w, void* 
   if (grid <= 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   if (cols <= NT * 8)
-    rmsnorm_fwd_kernel<1><<<grid, NT, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w,
+    np_launch(rmsnorm_fwd_kernel<1>, grid, NT, 0, s, 1, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w,
                                               (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, cols, eps);
   else if (cols <= NT * 16)
-    rmsnorm_fwd_kernel<2><<<grid, NT, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w,
+    np_launch(rmsnorm_fwd_kernel<2>, grid, NT, 0, s, 1, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w,
                                               (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, cols, eps);
   else
-    rmsnorm_fwd_kernel<4><<<grid, NT, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w,
+    np_launch(rmsnorm_fwd_kernel<4>, grid, NT, 0, s, 1, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w,
                                               (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, cols, eps);
   CHECK_LAUNCH();
 }
@@ -939,7 +957,7 @@ NP_API int np_rmsnorm_quant_fwd(const void* x, const void* res, const float* w, 
   const int grid = rows < GRID_CAP ? rows : GRID_CAP;
   if (grid <= 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-#define RQ(V) rmsnorm_quant_fwd_kernel<V><<<grid, NT, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w, \
+#define RQ(V) np_launch(rmsnorm_quant_fwd_kernel<V>, grid, NT, 0, s, 1, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w, \
       (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, (uint8_t*)q, scales, rows, cols, eps)
   if (cols <= NT * 8) RQ(1);
   else if (cols <= NT * 16) RQ(2);
@@ -953,9 +971,9 @@ NP_API int np_rmsnorm_quant_fwd(const void* x, const void* res, const float* w, 
 static int launch_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* rstd, const void* dres,
                                void* dx, float* dw, float* scratch, int rows, int cols, int accumulate_dw, int grid,
                                cudaStream_t s) {
-#define RB(V) rmsnorm_bwd_kernel<V><<<grid, NT, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, \
+#define RB(V) np_launch(rmsnorm_bwd_kernel<V>, grid, NT, 0, s, 1, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, \
                                                        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, cols)
-#define RBW(V) rmsnorm_bwd_warp_kernel<V><<<grid, NT, 8 * cols * sizeof(float), s>>>( \
+#define RBW(V) np_launch(rmsnorm_bwd_warp_kernel<V>, grid, NT, 8 * cols * sizeof(float), s, 1, \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, \
       rows, cols)
   static NpPerDeviceOnce attr_once;
@@ -974,7 +992,7 @@ static int launch_rmsnorm_bwd(const void* dy, const void* x, const float* w, con
   else RB(4);
 #undef RB
 #undef RBW
-  colsum_tall_kernel<<<(cols + 31) / 32, 256, 0, s>>>(scratch, dw, grid, cols, accumulate_dw);
+  np_launch(colsum_tall_kernel, (cols + 31) / 32, 256, 0, s, 1, scratch, dw, grid, cols, accumulate_dw);
   return 0;
 }
 
@@ -1000,14 +1018,14 @@ NP_API int np_rmsnorm_bwd(const void* dy, const void* x, const float* w, const f
 NP_API int np_glu_fwd(const void* gu, void* h, long long rows, int F, int act, void* stream) {
   if (F % 8) return 1;
   if (rows <= 0) return 0;
-  glu_fwd_kernel<<<grid_for(rows * (F / 8), 256, GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(glu_fwd_kernel, grid_for(rows * (F / 8), 256, GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, rows, F, act);
   CHECK_LAUNCH();
 }
 NP_API int np_glu_bwd(const void* gu, const void* dh, void* dgu, long long rows, int F, int act, void* stream) {
   if (F % 8) return 1;
   if (rows <= 0) return 0;
-  glu_bwd_kernel<<<grid_for(rows * (F / 8), 256, GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(glu_bwd_kernel, grid_for(rows * (F / 8), 256, GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dh, (__nv_bfloat16*)dgu, rows, F, act);
   CHECK_LAUNCH();
 }
@@ -1017,7 +1035,7 @@ NP_API int np_rope(const void* x, void* out, const float* cos_t, const float* si
                    float sign, void* stream) {
   if (hd % 8 || rot % 16 || rot > hd || ld_in % 8 || ld_out % 8) return 1;
   if (T <= 0) return 0;
-  rope_kernel<<<grid_for(T * H * (hd / 8), 256, GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(rope_kernel, grid_for(T * H * (hd / 8), 256, GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)x, (__nv_bfloat16*)out, cos_t, sin_t, pos_ids, T, S, pos_off, H, hd, rot, ld_in,
       ld_out, sign);
   CHECK_LAUNCH();
@@ -1032,7 +1050,7 @@ NP_API int np_qkv_rope(const void* p0, long long rs0, long long hs0, int h0, con
   if (T <= 0) return 0;
   HeadSrc s0{(const __nv_bfloat16*)p0, rs0, hs0, h0}, s1{(const __nv_bfloat16*)p1, rs1, hs1, h1},
       s2{(const __nv_bfloat16*)p2, rs2, hs2, h2};
-  qkv_rope_kernel<<<(unsigned)(T < GRID_CAP ? T : GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(qkv_rope_kernel, (unsigned)(T < GRID_CAP ? T : GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       s0, s1, s2, (__nv_bfloat16*)out, cos_t, sin_t, pos_ids, T, S, pos_off, hd, rot, rot_heads, sign);
   CHECK_LAUNCH();
 }
@@ -1045,7 +1063,7 @@ NP_API int np_qkv_norm_rope_fwd(const void* qkv, long long row_stride, int hq, i
                                 int pos_off, void* stream) {
   if (row_stride % 8 || (hq + hkv) * 8 > 512 || (hq + hkv) * 8 + hkv * 16 > 768) return 1;
   if (T <= 0) return 0;
-  qkv_norm_rope_fwd_kernel<<<(unsigned)(T < GRID_CAP ? T : GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(qkv_norm_rope_fwd_kernel, (unsigned)(T < GRID_CAP ? T : GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)qkv, row_stride, hq, hkv, gq, bq, gk, bk, eps, (__nv_bfloat16*)out, (float2*)stats, cos_t,
       sin_t, pos_ids, T, S, pos_off);
   CHECK_LAUNCH();
@@ -1065,17 +1083,17 @@ NP_API int np_qkv_norm_rope_bwd(const void* dq, long long rs0, long long hs0, co
       s2{(const __nv_bfloat16*)dv, rs2, hs2, hkv};
   const int grid = np_qkv_norm_rope_parts(T);
   cudaStream_t s = (cudaStream_t)stream;
-  qkv_norm_rope_bwd_kernel<<<grid, 256, 0, s>>>(s0, s1, s2, (const __nv_bfloat16*)qkv, row_stride, hq, hkv, gq, gk,
+  np_launch(qkv_norm_rope_bwd_kernel, grid, 256, 0, s, 1, s0, s1, s2, (const __nv_bfloat16*)qkv, row_stride, hq, hkv, gq, gk,
                                                 (const float2*)stats, (__nv_bfloat16*)dqkv, scratch, cos_t, sin_t,
                                                 pos_ids, T, S, pos_off);
-  colsum_tall_kernel<<<(4 * 128 + 31) / 32, 256, 0, s>>>(scratch, dparams, grid, 4 * 128, accumulate);
+  np_launch(colsum_tall_kernel, (4 * 128 + 31) / 32, 256, 0, s, 1, scratch, dparams, grid, 4 * 128, accumulate);
   CHECK_LAUNCH();
 }
 
 NP_API int np_rope_table(float* cos_t, float* sin_t, int S, int rot, float base, int scaling, float factor,
                          float orig_len, float low_f, float high_f, float mscale, void* stream) {
   if (S <= 0) return 0;
-  rope_table_kernel<<<grid_for((long long)S * (rot / 2), 256, GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(rope_table_kernel, grid_for((long long)S * (rot / 2), 256, GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       cos_t, sin_t, S, rot, base, scaling, factor, orig_len, low_f, high_f, mscale);
   CHECK_LAUNCH();
 }
@@ -1084,7 +1102,7 @@ NP_API int np_xent_fwd(const void* logits, const long long* labels, float* loss,
                        long long ld, long long ignore, void* stream) {
   if (ld % 8) return 1;
   if (rows <= 0) return 0;
-  xent_fwd_kernel<<<rows < GRID_CAP ? rows : GRID_CAP, NT, 0, (cudaStream_t)stream>>>(
+  np_launch(xent_fwd_kernel, rows < GRID_CAP ? rows : GRID_CAP, NT, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)logits, labels, loss, lse, rows, V, ld, ignore);
   CHECK_LAUNCH();
 }
@@ -1093,7 +1111,7 @@ NP_API int np_xent_bwd(const void* logits, const long long* labels, const float*
                        void* stream) {
   if (ld % 8) return 1;
   if (rows <= 0) return 0;
-  xent_bwd_kernel<<<rows < GRID_CAP ? rows : GRID_CAP, NT, 0, (cudaStream_t)stream>>>(
+  np_launch(xent_bwd_kernel, rows < GRID_CAP ? rows : GRID_CAP, NT, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)logits, labels, lse, gscale, inv_count, (__nv_bfloat16*)dlogits, rows, V, ld, ignore);
   CHECK_LAUNCH();
 }
@@ -1102,7 +1120,7 @@ NP_API int np_adamw(float* p, const float* g, float* m, float* v, void* w16, lon
                     float b2, float eps, float wd, int step, const float* gscale, const float* hyper, void* stream) {
   if (n <= 0) return 0;
   const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  adamw_kernel<<<grid_for(n / 4 + 1, 256, GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(adamw_kernel, grid_for(n / 4 + 1, 256, GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       p, g, m, v, (__nv_bfloat16*)w16, n, lr, b1, b2, eps, wd, bc1, bc2, gscale, hyper);
   CHECK_LAUNCH();
 }
@@ -1110,7 +1128,7 @@ NP_API int np_adamw(float* p, const float* g, float* m, float* v, void* w16, lon
 NP_API int np_sumsq_parts() { return 148 * 4; }
 // partial: fp32 [np_sumsq_parts()]
 NP_API int np_sumsq(const float* x, long long n, float* partial, void* stream) {
-  sumsq_kernel<<<np_sumsq_parts(), NT, 0, (cudaStream_t)stream>>>(x, n, partial);
+  np_launch(sumsq_kernel, np_sumsq_parts(), NT, 0, (cudaStream_t)stream, 1, x, n, partial);
   CHECK_LAUNCH();
 }
 // Embedding backward straight into the fp32 gradient arena: grad[ids[t], :] += dy[t, :]. One thread per four
@@ -1119,6 +1137,7 @@ namespace {
 __global__ void __launch_bounds__(256) embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                             const long long* __restrict__ ids, float* __restrict__ grad,
                                                             long long T, int D, long long V) {
+  np::pdl_begin();
   const int vec_per_row = D >> 2;
   const long long total = T * vec_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -1146,18 +1165,18 @@ NP_API int np_embedding_bwd(const void* dy, const long long* ids, float* grad, l
   }
   long long blocks = (T * (D / 4) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  embedding_bwd_kernel<<<(int)blocks, 256, 0, s>>>((const __nv_bfloat16*)dy, ids, grad, T, D, V);
+  np_launch(embedding_bwd_kernel, (int)blocks, 256, 0, s, 1, (const __nv_bfloat16*)dy, ids, grad, T, D, V);
   CHECK_LAUNCH();
 }
 
 NP_API int np_clip_coef(const float* partial, int parts, const float* extra_sq, float max_norm, float* out2,
                         void* stream) {
-  clip_coef_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(partial, parts, extra_sq, max_norm, out2);
+  np_launch(clip_coef_kernel, 1, 256, 0, (cudaStream_t)stream, 1, partial, parts, extra_sq, max_norm, out2);
   CHECK_LAUNCH();
 }
 NP_API int np_cast_f32_bf16(const float* x, void* y, long long n, void* stream) {
   if (n <= 0) return 0;
-  cast_f32_to_bf16_kernel<<<grid_for(n / 4 + 1, 256, GRID_CAP), 256, 0, (cudaStream_t)stream>>>(
+  np_launch(cast_f32_to_bf16_kernel, grid_for(n / 4 + 1, 256, GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
       x, (__nv_bfloat16*)y, n);
   CHECK_LAUNCH();
 }

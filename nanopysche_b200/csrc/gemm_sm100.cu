@@ -459,7 +459,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
 
   const int m_blocks = (p.M + BM - 1) / BM;
   const int bn_out = (p.epilogue == 1) ? BN / 2 : BN;  // output columns per tile
@@ -494,6 +493,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   np::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  np::pdl_begin();
+  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
 
   if (p.push_src) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.push_vecs;
@@ -782,7 +783,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int rank = (int)(crank & 1u);                              // 0: leader of its pair
   const int splits = SPLIT ? p.splits : 1, split = SPLIT ? (int)(crank >> 1) : 0;
   const int pair = (int)blockIdx.x / (2 * splits), pairs = (int)gridDim.x / (2 * splits);
-  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
   const int m_blocks = (p.M + TM - 1) / TM, m_blocks128 = (p.M + BM - 1) / BM;
   const int bn_out = (p.epilogue == 1) ? HN : BN;
   const int n_blocks = (p.N + bn_out - 1) / bn_out;
@@ -826,6 +826,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync();        // this CTA's and the peer's barriers and tensor memory are set up
   np::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  np::pdl_begin();
+  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
 
   // rows of the two 128-row blocks of an M block that carry data, as a mask (0: nothing to do, -1: gave up). Row-grouped
   // form: both blocks belong to the same group and arrive under the same flag (the caller's tables are made of pairs).
@@ -1241,24 +1243,20 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   const int cap = a.max_ctas > 0 ? a.max_ctas : num_sms();
   const int bn_out = a.epilogue == 1 ? BN / 2 : BN, tm = PAIR ? 2 * BM : BM;
   const long long tiles = (long long)((a.M + tm - 1) / tm) * ((a.N + bn_out - 1) / bn_out) * (a.mode == 2 ? a.num_groups : 1);
+  const bool busy = 2.0 * a.M * a.N * a.K > 2e10;   // 15 us and more
   if constexpr (PAIR) {
     const long long pairs = tiles < cap / 2 ? tiles : cap / 2;
     if (pairs <= 0) return 0;
     p.splits = splits;
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 2 * splits; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = SMEM; cfg.stream = stream; cfg.attrs = &at; cfg.numAttrs = 1;
-    const cudaError_t e = splits > 1 ? cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<true>, tmA, tmB, tmB2, tmC, tmC2, p)
-                                     : cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<false>, tmA, tmB, tmB2, tmC, tmC2, p);
+    const dim3 grid((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
+    const cudaError_t e =
+        np_launch_if(busy, splits > 1 ? gemm_bf16_pair_kernel<true> : gemm_bf16_pair_kernel<false>, grid, GEMM_THREADS, SMEM, stream,
+                  2 * splits, tmA, tmB, tmB2, tmC, tmC2, p);
     if (e != cudaSuccess) return 500 + (int)e;
   } else {
     const int grid = (int)(tiles < cap ? tiles : cap);
     if (grid <= 0) return 0;
-    gemm_bf16_kernel<BN, STAGES><<<grid, GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2, p);
+    np_launch_if(busy, gemm_bf16_kernel<BN, STAGES>, grid, GEMM_THREADS, SMEM, stream, 1, tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2, p);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;

@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256, 4) router_logits_kernel(const __nv_bfloat
                                                                const float* __restrict__ wg,
                                                                const float* __restrict__ bias,
                                                                float* __restrict__ logits, int T, int D, int E) {
+  np::pdl_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
                                                           int* __restrict__ counts, float* __restrict__ psum,
                                                           float* __restrict__ zsum, int T, int E, int K,
                                                           int gating) {
+  np::pdl_begin();
   __shared__ int s_cnt[MAX_E];
   __shared__ float s_p[MAX_E];
   __shared__ float s_z;
@@ -188,6 +190,7 @@ __global__ void __launch_bounds__(256) router_bwd_kernel(const float* __restrict
                                                          const float* __restrict__ daux, float coef_lb,
                                                          float coef_z, float* __restrict__ dlogits, int T, int E,
                                                          int K, int gating) {
+  np::pdl_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   float l[MAX_E], dl[MAX_E];
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(256) router_dgate_kernel(const float* __restri
                                                            const __nv_bfloat16* __restrict__ x,
                                                            float* __restrict__ partial, int T, int D, int E,
                                                            int chunk) {
+  np::pdl_begin();
   __shared__ float red[2][64][EB * 8 + 1];
   const int c = blockIdx.y;
   const int t0 = c * chunk, t1 = min(T, t0 + chunk);
@@ -319,6 +323,7 @@ __global__ void __launch_bounds__(256) router_dgate_kernel(const float* __restri
 // [T, E] x [E, D] product with E of 8 to 64: one thread per 8 output columns, the gate rows come from L1).
 __global__ void __launch_bounds__(256) router_dx_kernel(const float* __restrict__ dl, const float* __restrict__ wg,
                                                         __nv_bfloat16* __restrict__ dx, int T, int D, int E) {
+  np::pdl_begin();
   const int vec_per_row = D >> 3;
   const long long total = (long long)T * vec_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -341,6 +346,7 @@ __global__ void __launch_bounds__(256) router_dx_kernel(const float* __restrict_
 template <int TOK>
 __global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* __restrict__ dl, const float* __restrict__ wg,
                                                             __nv_bfloat16* __restrict__ dx, int T, int D, int E) {
+  np::pdl_begin();
   const int d = threadIdx.x * 8;
   float w[8][8];
 #pragma unroll
@@ -371,6 +377,7 @@ __global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* __restr
 
 __global__ void colsum2_kernel(const float* __restrict__ partial, float* __restrict__ out, int parts,
                                long long cols, int accumulate) {
+  np::pdl_begin();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= cols) return;
   float a8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -387,6 +394,7 @@ __global__ void colsum2_kernel(const float* __restrict__ partial, float* __restr
 // out[c] (+)= sum over rows of a[r, c] for a narrow matrix (cols <= 64): 1024 threads, thread -> (row group, col)
 __global__ void __launch_bounds__(1024) colsum_narrow_kernel(const float* __restrict__ a, float* __restrict__ out,
                                                              int rows, int cols, int accumulate) {
+  np::pdl_begin();
   __shared__ float red[1024];
   const int c = threadIdx.x % cols, g = threadIdx.x / cols, ng = 1024 / cols;
   float s = 0.f;
@@ -469,6 +477,7 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* __restri
                                                              int* __restrict__ keep, int* __restrict__ counts_kept,
                                                              int* __restrict__ drops, int* __restrict__ n_dropped,
                                                              int use_smem) {
+  np::pdl_begin();
   constexpr int EPW = 64 / FB;          // experts per 64-bit word
   constexpr int GROUP = 4 * EPW;        // experts per pass
   constexpr unsigned long long FMASK = (FB == 16) ? 0xffffull : 0xffffffffull;
@@ -569,6 +578,7 @@ struct DispatchParams {
 };
 
 __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p) {
+  np::pdl_begin();
   np::CommSpan span(p.n_ranks > 1);
   const int lane = threadIdx.x & 31;
   const int warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -720,6 +730,7 @@ struct CombineParams {
 };
 
 __global__ void __launch_bounds__(256) ep_combine_kernel(const CombineParams p) {
+  np::pdl_begin();
   __shared__ int s_ok;
   if (p.flags) {
     if (threadIdx.x == 0) s_ok = 1;
@@ -777,6 +788,7 @@ __global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* __re
                                                        const __nv_bfloat16* __restrict__ rows,
                                                        const int* __restrict__ slot_pos, float* __restrict__ dots,
                                                        int T, int K, int D) {
+  np::pdl_begin();
   const int lane = threadIdx.x & 31;
   const int warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -805,7 +817,7 @@ NP_API int np_router_logits(const void* x, const float* wg, const float* bias, f
                             void* stream) {
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
   const int grid = (T * 32 + 255) / 256 < 148 * 8 ? (T * 32 + 255) / 256 : 148 * 8;
-  router_logits_kernel<8><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, wg, bias, logits, T, D, E);
+  np_launch(router_logits_kernel<8>, grid, 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias, logits, T, D, E);
   CHECK_LAUNCH();
 }
 
@@ -814,7 +826,7 @@ NP_API int np_router_topk(const float* logits, const float* score_bias, float* w
                           float* psum, float* zsum, int T, int E, int K, int gating, void* stream) {
   if (E > MAX_E || K > MAX_K || K > E) return 1;
   if (T <= 0) return 0;
-#define TOPK(EM) router_topk_kernel<EM><<<(T + 127) / 128, 128, 0, (cudaStream_t)stream>>>( \
+#define TOPK(EM) np_launch(router_topk_kernel<EM>, (T + 127) / 128, 128, 0, (cudaStream_t)stream, 1, \
       logits, score_bias, weights, indices, counts, psum, zsum, T, E, K, gating)
   if (E <= 8) TOPK(8);
   else if (E <= 16) TOPK(16);
@@ -829,7 +841,7 @@ NP_API int np_router_bwd(const float* logits, const float* score_bias, const flo
                          float* dlogits, int T, int E, int K, int gating, void* stream) {
   if (E > MAX_E || K > MAX_K) return 1;
   if (T <= 0) return 0;
-  router_bwd_kernel<<<(T + 255) / 256, 256, 0, (cudaStream_t)stream>>>(logits, score_bias, weights, indices, dweights,
+  np_launch(router_bwd_kernel, (T + 255) / 256, 256, 0, (cudaStream_t)stream, 1, logits, score_bias, weights, indices, dweights,
                                                                        f, daux, coef_lb, coef_z, dlogits, T, E, K,
                                                                        gating);
   CHECK_LAUNCH();
@@ -844,10 +856,10 @@ NP_API int np_router_dgate(const float* dl, const void* x, float* dwg, float* db
   cudaStream_t s = (cudaStream_t)stream;
   const int parts = np_router_dgate_parts(T);
   dim3 grid((D / 8 + 63) / 64, parts);
-  router_dgate_kernel<8><<<grid, 256, 0, s>>>(dl, (const __nv_bfloat16*)x, scratch, T, D, E, 64);
+  np_launch(router_dgate_kernel<8>, grid, 256, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch, T, D, E, 64);
   const long long cols = (long long)E * D;
-  colsum2_kernel<<<(int)((cols + 63) / 64), 64, 0, s>>>(scratch, dwg, parts, cols, accumulate);
-  if (dbias) colsum_narrow_kernel<<<1, 1024, 0, s>>>(dl, dbias, T, E, accumulate);
+  np_launch(colsum2_kernel, (int)((cols + 63) / 64), 64, 0, s, 1, scratch, dwg, parts, cols, accumulate);
+  if (dbias) np_launch(colsum_narrow_kernel, 1, 1024, 0, s, 1, dl, dbias, T, E, accumulate);
   CHECK_LAUNCH();
 }
 
@@ -856,12 +868,12 @@ NP_API int np_router_dx(const float* dl, const float* wg, void* dx, int T, int D
   if (T <= 0) return 0;
   if (E <= 8 && D % 8 == 0 && D / 8 <= 256 && D / 8 >= 32) {
     constexpr int TOK = 8;
-    router_dx_reg_kernel<TOK><<<(unsigned)((T + TOK - 1) / TOK), D / 8, 0, (cudaStream_t)stream>>>(
+    np_launch(router_dx_reg_kernel<TOK>, (unsigned)((T + TOK - 1) / TOK), D / 8, 0, (cudaStream_t)stream, 1,
         dl, wg, (__nv_bfloat16*)dx, T, D, E);
     CHECK_LAUNCH();
   }
   const long long blocks = ((long long)T * (D / 8) + 255) / 256;
-  router_dx_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(dl, wg, (__nv_bfloat16*)dx, T, D, E);
+  np_launch(router_dx_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, 1, dl, wg, (__nv_bfloat16*)dx, T, D, E);
   CHECK_LAUNCH();
 }
 
@@ -881,10 +893,10 @@ NP_API int np_capacity_scan(const int* indices, int T, int E, int K, int capacit
     attr_set = true;
   }
   if (T < 65536)   // a 16-bit counter holds any per-expert count
-    capacity_scan_kernel<16><<<1, 1024, use_smem ? smem : 0, (cudaStream_t)stream>>>(
+    np_launch(capacity_scan_kernel<16>, 1, 1024, use_smem ? smem : 0, (cudaStream_t)stream, 1,
         indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem);
   else
-    capacity_scan_kernel<32><<<1, 1024, use_smem ? smem : 0, (cudaStream_t)stream>>>(
+    np_launch(capacity_scan_kernel<32>, 1, 1024, use_smem ? smem : 0, (cudaStream_t)stream, 1,
         indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem);
   CHECK_LAUNCH();
 }
@@ -911,7 +923,7 @@ NP_API int np_ep_dispatch(const NpDispatchArgs* a, void* stream) {
   const int cap = a->max_ctas > 0 ? a->max_ctas : 148 * 4;
   if (grid > cap) grid = cap;
   if (grid < 1) grid = 1;
-  ep_dispatch_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+  np_launch(ep_dispatch_kernel, grid, 256, 0, (cudaStream_t)stream, 1, p);
   CHECK_LAUNCH();
 }
 
@@ -934,7 +946,7 @@ NP_API int np_ep_combine(const NpCombineArgs* a, void* stream) {
   long long work = (long long)a->T * (a->D / 8);
   int grid = (int)((work + 255) / 256);
   if (grid > 148 * 8) grid = 148 * 8;
-  ep_combine_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(p);
+  np_launch(ep_combine_kernel, grid, 256, 0, (cudaStream_t)stream, 1, p);
   CHECK_LAUNCH();
 }
 
@@ -944,7 +956,7 @@ NP_API int np_slot_dot(const void* a, const void* rows, const int* slot_pos, flo
   if (T <= 0) return 0;
   int grid = (T * K + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
-  slot_dot_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)rows, slot_pos,
+  np_launch(slot_dot_kernel, grid, 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)a, (const __nv_bfloat16*)rows, slot_pos,
                                                           dots, T, K, D);
   CHECK_LAUNCH();
 }

@@ -47,6 +47,7 @@ template <int MT, int U>
 __global__ void __launch_bounds__(SK_WARPS * 32)
 skinny_linear_kernel(const SkinnyParams p) {
   __shared__ float red[SK_WARPS][MT][16][8];
+  np::pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * 16;
   const int r0 = n0 + g < p.N ? n0 + g : p.N - 1, r1 = n0 + 8 + g < p.N ? n0 + 8 + g : p.N - 1;
@@ -153,6 +154,7 @@ decode_attn_kernel(const DecodeParams p) {
   constexpr int L = HD / 8, KPW = 32 / L, U = R >= 8 ? 2 : 4;
   __shared__ float s_m[DC_WARPS][R], s_l[DC_WARPS][R], s_acc[DC_WARPS][R][HD];
   __shared__ float c_m[R], c_l[R], c_acc[R][HD];
+  np::pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / L, d0 = (lane % L) * 8;
   const int part = blockIdx.x, parts = gridDim.x, h = blockIdx.y, b = blockIdx.z;   // a cluster spans grid.x
   const int n_rep = p.Hq / p.Hkv, rows = n_rep * p.Sq, total = p.past + p.fresh;
@@ -289,14 +291,7 @@ decode_attn_kernel(const DecodeParams p) {
 
 template <int HD, int R>
 int launch_decode(const DecodeParams& p, int parts, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = parts; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(parts, p.Hkv, p.B);
-  cfg.blockDim = dim3(DC_WARPS * 32);
-  cfg.stream = stream; cfg.attrs = &at; cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, decode_attn_kernel<HD, R>, p);
+  const cudaError_t e = np_launch(decode_attn_kernel<HD, R>, dim3(parts, p.Hkv, p.B), DC_WARPS * 32, 0, stream, parts, p);
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
@@ -311,10 +306,10 @@ int np_skinny_linear(const void* x, long long ldx, const void* w, long long ldw,
   p.M = M; p.N = N; p.K = K; p.out = out; p.ldo = ldo; p.out_f32 = out_f32; p.alpha = alpha;
   p.bias = bias; p.cin = cin; p.ldcin = ldcin;
   const int grid = (N + 15) / 16;
-  if (M <= 8) skinny_linear_kernel<1, 4><<<grid, SK_WARPS * 32, 0, stream>>>(p);
-  else if (M <= 16) skinny_linear_kernel<2, 4><<<grid, SK_WARPS * 32, 0, stream>>>(p);
-  else if (M <= 32) skinny_linear_kernel<4, 2><<<grid, SK_WARPS * 32, 0, stream>>>(p);
-  else skinny_linear_kernel<8, 2><<<grid, SK_WARPS * 32, 0, stream>>>(p);
+  if (M <= 8) np_launch(skinny_linear_kernel<1, 4>, grid, SK_WARPS * 32, 0, stream, 1, p);
+  else if (M <= 16) np_launch(skinny_linear_kernel<2, 4>, grid, SK_WARPS * 32, 0, stream, 1, p);
+  else if (M <= 32) np_launch(skinny_linear_kernel<4, 2>, grid, SK_WARPS * 32, 0, stream, 1, p);
+  else np_launch(skinny_linear_kernel<8, 2>, grid, SK_WARPS * 32, 0, stream, 1, p);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
