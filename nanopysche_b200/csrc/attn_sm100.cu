@@ -210,6 +210,61 @@ __device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t* r) 
   for (int c = 0; c < NCOLS / 16; ++c) tmem_st16(taddr + c * 16, r + c * 16);
 }
 
+// Walk over the 128-row blocks of the looped operand - source by source, for the dK/dV kernel head by head within a source -
+// that causality leaves visible. Every role of a kernel walks the same list. Counters instead of one running index: its
+// divisions and remainders (four per block and role) stood in front of every iteration (dK/dV: 1500 of 4700 cycles).
+struct BlockWalk {
+  const int* pos;        // positions of all blocks of all sources, or nullptr: block i of a source starts at i * 128 + off
+  int off, blocks, heads, sources;
+  int first, last;       // without a table: visible blocks of a source are [first, last)
+  int need_lo, need_hi;  // with a table: a block is visible when need_lo <= its position <= need_hi
+  int src, head, i;
+  __device__ __forceinline__ int at() const { return pos ? pos[src * blocks + i] : i * 128 + off; }
+  __device__ __forceinline__ bool done() const { return src >= sources; }
+  __device__ __forceinline__ void settle() {   // from (src, head, i) on to the next visible block
+    for (;;) {
+      if (src >= sources) return;
+      if (i >= last) {
+        i = first;
+        if (++head == heads) { head = 0; ++src; }
+        if (first >= last) { src = sources; return; }
+        continue;
+      }
+      if (!pos) return;
+      const int q = pos[src * blocks + i];
+      if (q >= need_lo && q <= need_hi) return;
+      ++i;
+    }
+  }
+  __device__ __forceinline__ void start() { src = head = 0; i = first; settle(); }
+  __device__ __forceinline__ void next() { ++i; settle(); }
+};
+constexpr int POS_MAX = 0x7fffffff;
+// KV blocks that some row of the Q block at q_pos0 sees: those starting at or before its last row
+__device__ __forceinline__ BlockWalk walk_kv(const int* tab, int blocks, int sources, bool causal, int q_pos0) {
+  BlockWalk w;
+  w.pos = tab; w.off = 0; w.blocks = blocks; w.heads = 1; w.sources = sources;
+  w.first = 0; w.last = blocks; w.need_lo = -POS_MAX; w.need_hi = causal ? q_pos0 + BQ - 1 : POS_MAX;
+  if (!tab && causal) {
+    const int n = q_pos0 + BQ - 1 < 0 ? 0 : (q_pos0 + BQ - 1) / BKV + 1;
+    w.last = n < blocks ? n : blocks;
+  }
+  w.start();
+  return w;
+}
+// Q blocks (of `heads` heads) with some row that sees the KV block at k_pos0: those whose last row is at or behind it
+__device__ __forceinline__ BlockWalk walk_q(const int* tab, int off, int blocks, int heads, int sources, bool causal, int k_pos0) {
+  BlockWalk w;
+  w.pos = tab; w.off = off; w.blocks = blocks; w.heads = heads; w.sources = sources;
+  w.first = 0; w.last = blocks; w.need_lo = causal ? k_pos0 - (BQ - 1) : -POS_MAX; w.need_hi = POS_MAX;
+  if (!tab && causal) {
+    const int d = k_pos0 - (BQ - 1) - off;   // first i with i * 128 >= d
+    w.first = d <= 0 ? 0 : (d + BQ - 1) / BQ;
+  }
+  w.start();
+  return w;
+}
+
 // warp 0: TMA, warp 1: MMA issue, then 4*NS softmax warps (NS per TMEM lane quarter)
 constexpr int nthreads(int ns) { return 64 + ns * 128; }
 constexpr float RESCALE_LOG2 = 8.f;
@@ -249,13 +304,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int hkv = h / (p.Hq / p.Hkv);
   if (p.q_blk_pos || p.k_blk_pos) np::pdl_wait();   // position tables are memory
   const int q_pos0 = p.q_blk_pos ? p.q_blk_pos[qb] : qb * BQ + p.q_off;
-  const int total_blocks = p.n_src * p.src_blocks;
-  auto k_pos0 = [&](int j) { return p.k_blk_pos ? p.k_blk_pos[j] : (j % p.src_blocks) * BKV; };
-  // Every role walks the same list: the KV blocks that causality does not hide from all rows of this Q block.
-  auto next_vis = [&](int j) {
-    while (j < total_blocks && p.causal && k_pos0(j) > q_pos0 + BQ - 1) ++j;
-    return j;
-  };
+  const BlockWalk walk0 = walk_kv(p.k_blk_pos, p.src_blocks, p.n_src, p.causal, q_pos0);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < FB_COUNT; ++i) np::mbar_init(B_(i), i == FB_P ? 4 * NS : 1);
@@ -280,9 +329,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       np::mbar_expect_tx(B_(FB_Q), TILE_BYTES);
       load_tile<HD>(sQ, &tmQ, B_(FB_Q), h, qb * BQ, b);
       int i = 0, last_src = -1;
-      for (int j = next_vis(0); j < total_blocks && !*abort_flag; j = next_vis(j + 1), ++i) {
+      for (BlockWalk w = walk0; !w.done() && !*abort_flag; w.next(), ++i) {
         const int ks = i % F_KST, vs = i % F_VST;
-        const int src = j / p.src_blocks, jb = j - src * p.src_blocks;
+        const int src = w.src, jb = w.i;
         if (src != last_src) {
           if (!src_ready(p.fl, src, KID_ATTN)) { *abort_flag = 1; break; }
           last_src = src;
@@ -315,14 +364,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       __syncwarp();
       return true;
     };
-    int j = next_vis(0);
-    if (ok && j < total_blocks) ok = issue_qk(0);
-    for (int i = 0; j < total_blocks && ok; ++i) {
+    BlockWalk w = walk0;
+    if (ok && !w.done()) ok = issue_qk(0);
+    for (int i = 0; !w.done() && ok; ++i) {
       const int st = i & 1, vs = i % F_VST;
       // S of the next block is computed while the softmax warps work on this one. Its S and P buffers were
       // last used for block i-1: S read before P of block i-1 arrived, P consumed by P V of block i-1 (issued).
-      j = next_vis(j + 1);
-      if (j < total_blocks) ok = issue_qk(i + 1);
+      w.next();
+      if (!w.done()) ok = issue_qk(i + 1);
       ok = ok && np::mbar_wait_warp(B_(FB_P), (uint32_t)i & 1u, abort_flag, KID_ATTN, 5) &&   // P ready, O rescaled
            np::mbar_wait_warp(B_(FB_V + vs), (uint32_t)(i / F_VST) & 1u, abort_flag, KID_ATTN, 4);
       if (!ok) break;
@@ -346,10 +395,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float m = -INFINITY, l = 0.f;                            // running maximum (log2 domain) and row sum
     bool ok = true;
     int nvis = 0;
-    for (int j = next_vis(0); j < total_blocks; j = next_vis(j + 1), ++nvis) {
+    for (BlockWalk w = walk0; !w.done(); w.next(), ++nvis) {
       const int i = nvis, st = i & 1;
-      const int jb = j % p.src_blocks;
-      const int kp0 = k_pos0(j);
+      const int jb = w.i;
+      const int kp0 = w.at();
       const int valid_cols = p.src_len - jb * BKV;           // columns beyond the source's length are padding
       const bool need_mask = (p.causal && kp0 + BKV - 1 > q_pos0) || valid_cols < BKV;
       ok = ok && !*abort_flag && warp_wait(B_(FB_S + st), (uint32_t)(i >> 1) & 1u, abort_flag, KID_ATTN, 7);
@@ -1003,12 +1052,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int hkv = h / (p.Hq / p.Hkv);
   if (p.q_blk_pos || p.k_blk_pos) np::pdl_wait();   // position tables are memory
   const int q_pos0 = p.q_blk_pos ? p.q_blk_pos[qb] : qb * BQ + p.q_off;
-  const int total_blocks = p.n_src * p.src_blocks;
-  auto k_pos0 = [&](int j) { return p.k_blk_pos ? p.k_blk_pos[j] : (j % p.src_blocks) * BKV; };
-  auto next_vis = [&](int j) {   // next KV block that causality does not hide from every row of this Q block
-    while (j < total_blocks && p.causal && k_pos0(j) > q_pos0 + BQ - 1) ++j;
-    return j;
-  };
+  const BlockWalk walk0 = walk_kv(p.k_blk_pos, p.src_blocks, p.n_src, p.causal, q_pos0);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < QB_COUNT; ++i) np::mbar_init(B_(i), i == QB_DS ? 4 * NS : 1);
@@ -1034,9 +1078,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       load_tile<HD>(sQ, &tmQ, B_(QB_QDO), h, qb * BQ, b);
       load_tile<HD>(sdO, &tmdO, B_(QB_QDO), h, qb * BQ, b);
       int i = 0, last_src = -1;
-      for (int j = next_vis(0); j < total_blocks && !*abort_flag; j = next_vis(j + 1), ++i) {
+      for (BlockWalk w = walk0; !w.done() && !*abort_flag; w.next(), ++i) {
         const int ks = i % Q_KST, vs = i % Q_VST;
-        const int src = j / p.src_blocks, jb = j - src * p.src_blocks;
+        const int src = w.src, jb = w.i;
         if (src != last_src) {
           if (!src_ready(p.fl, src, KID_ATTN_DQ)) { *abort_flag = 1; break; }
           last_src = src;
@@ -1082,12 +1126,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       __syncwarp();
       return true;
     };
-    int j = next_vis(0);
-    if (ok && j < total_blocks) ok = issue_s(0) && issue_dp(0);
-    for (int i = 0; j < total_blocks && ok; ++i) {
+    BlockWalk w = walk0;
+    if (ok && !w.done()) ok = issue_s(0) && issue_dp(0);
+    for (int i = 0; !w.done() && ok; ++i) {
       const int ks = i % Q_KST;
-      j = next_vis(j + 1);
-      if (j < total_blocks) ok = issue_s(i + 1);   // its buffer was read for block i-1 before dS of block i-1 arrived
+      w.next();
+      if (!w.done()) ok = issue_s(i + 1);   // its buffer was read for block i-1 before dS of block i-1 arrived
       ok = ok && np::mbar_wait_warp(B_(QB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 5);
       if (!ok) break;
       np::tc_fence_after();
@@ -1098,7 +1142,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         np::tc_commit(B_(QB_KE + ks));
       }
       __syncwarp();
-      if (j < total_blocks) ok = issue_dp(i + 1);  // overwrites dS after the dQ product above has consumed it
+      if (!w.done()) ok = issue_dp(i + 1);  // overwrites dS after the dQ product above has consumed it
     }
     if (np::elect_one()) np::tc_commit(B_(QB_FIN));
     __syncwarp();
@@ -1119,10 +1163,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       dlt = p.delta[idx];
     }
     int nvis = 0;
-    for (int j = next_vis(0); j < total_blocks; j = next_vis(j + 1), ++nvis) {
+    for (BlockWalk w = walk0; !w.done(); w.next(), ++nvis) {
       const int i = nvis, st = i & 1;
-      const int jb = j % p.src_blocks;
-      const int kp0 = k_pos0(j);
+      const int jb = w.i;
+      const int kp0 = w.at();
       const int valid_cols = p.src_len - jb * BKV;
       const bool need_mask = (p.causal && kp0 + BKV - 1 > q_pos0) || valid_cols < BKV;
       ok = ok && !*abort_flag && warp_wait(B_(QB_S + st), (uint32_t)(i >> 1) & 1u, abort_flag, KID_ATTN_DQ, 7);
@@ -1222,21 +1266,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const int n_rep = p.Hq / p.Hkv;
   if (p.q_blk_pos || p.k_blk_pos) np::pdl_wait();   // position tables are memory
   const int k_pos0 = p.k_blk_pos ? p.k_blk_pos[jb] : jb * BKV;
-  auto q_pos0_of = [&](int src, int i) {
-    return p.q_blk_pos ? p.q_blk_pos[src * p.src_blocks + i] : i * BQ + p.q_off;
-  };
-
-  // Work list, walked identically by every role: candidate c = (source, head of the group, Q block), kept when
-  // causality lets at least one row of the Q block see this KV block.
-  const int total = p.n_src * n_rep * p.src_blocks;
-  auto next_vis = [&](int c) {
-    while (c < total && p.causal) {
-      const int i = c % p.src_blocks, src = c / (p.src_blocks * n_rep);
-      if (k_pos0 <= q_pos0_of(src, i) + BQ - 1) break;
-      ++c;
-    }
-    return c;
-  };
+  // Work list: (source, head of the group, Q block), kept when causality lets at least one row of the Q block see this KV block
+  const BlockWalk walk0 = walk_q(p.q_blk_pos, p.q_off, p.src_blocks, n_rep, p.n_src, p.causal, k_pos0);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < KB_COUNT; ++i) np::mbar_init(B_(i), (i == KB_P || i == KB_DS) ? 4 * NS : 1);
@@ -1261,9 +1292,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       load_tile<HD>(sK, &tmK, B_(KB_KV), hkv, jb * BKV, b);
       load_tile<HD>(sV, &tmV, B_(KB_KV), hkv, jb * BKV, b);
       int i = 0, last_src = -1;
-      for (int c = next_vis(0); c < total && !*abort_flag; c = next_vis(c + 1), ++i) {
+      for (BlockWalk w = walk0; !w.done() && !*abort_flag; w.next(), ++i) {
         const int qs = i % K_QST, ds = i % K_DOST;
-        const int qi = c % p.src_blocks, h = hkv * n_rep + (c / p.src_blocks) % n_rep, src = c / (p.src_blocks * n_rep);
+        const int qi = w.i, h = hkv * n_rep + w.head, src = w.src;
         if (src != last_src) {
           if (!src_ready(p.fl, src, KID_ATTN_DKV)) { *abort_flag = 1; break; }
           last_src = src;
@@ -1308,11 +1339,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       __syncwarp();
       return true;
     };
-    int c = next_vis(0);
-    if (ok && c < total) ok = issue_st(0) && issue_dpt(0);
-    for (int i = 0; c < total && ok; ++i) {
+    BlockWalk w = walk0;
+    if (ok && !w.done()) ok = issue_st(0) && issue_dpt(0);
+    for (int i = 0; !w.done() && ok; ++i) {
       const int qs = i % K_QST, ds = i % K_DOST;
-      c = next_vis(c + 1);
+      w.next();
       ok = np::mbar_wait_warp(B_(KB_P), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 6);
       if (!ok) break;
       np::tc_fence_after();
@@ -1324,7 +1355,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         np::tc_commit(B_(KB_DOE + ds));
       }
       __syncwarp();
-      if (c < total) ok = issue_st(i + 1);        // overwrites P^T after the product above consumed it
+      if (!w.done()) ok = issue_st(i + 1);        // overwrites P^T after the product above consumed it
       ok = ok && np::mbar_wait_warp(B_(KB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 7);
       if (!ok) break;
       np::tc_fence_after();
@@ -1336,7 +1367,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         np::tc_commit(B_(KB_QE + qs));
       }
       __syncwarp();
-      if (c < total) ok = issue_dpt(i + 1);       // overwrites dS^T after the product above consumed it
+      if (!w.done()) ok = issue_dpt(i + 1);       // overwrites dS^T after the product above consumed it
     }
     if (np::elect_one()) np::tc_commit(B_(KB_FIN));
     __syncwarp();
@@ -1349,30 +1380,32 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     const int k_pos = k_pos0 + r;
     bool ok = true;
     int nvis = 0, last_src = -1;
+    // Log-sum-exp (threads 0-127) and delta (threads 128-255) of a Q block, one column per thread, loaded one block ahead so
+    // that the load does not stand in front of the iteration
+    auto load_stat = [&](const BlockWalk& w) -> float {
+      if (w.src != last_src) {   // it has to be complete
+        if (ok && !src_ready(p.fl, w.src, KID_ATTN_DKV)) { *abort_flag = 1; ok = false; }
+        last_src = w.src;
+      }
+      const int qrow = w.i * BQ + (t256 & 127);
+      if (qrow >= p.src_len || t256 >= 256) return t256 < 128 ? INFINITY : 0.f;
+      const size_t idx = ((size_t)b * p.lse_H + hkv * n_rep + w.head) * p.src_len + qrow;
+      return t256 < 128 ? p.lse_src.p[w.src][idx] : p.delta_src.p[w.src][idx];
+    };
+    auto put_stat = [&](int st, float v) {
+      if (t256 < 128) s_lse[st * 128 + t256] = v == -INFINITY ? INFINITY : v * LOG2E;
+      else if (t256 < 256) s_dlt[st * 128 + (t256 & 127)] = v;
+    };
+    BlockWalk w = walk0;
+    if (!w.done()) put_stat(0, load_stat(w));
     // every thread runs every iteration: the named barriers need all of them
-    for (int c = next_vis(0); c < total; c = next_vis(c + 1), ++nvis) {
+    for (; !w.done(); ++nvis) {
       const int i = nvis, st = i & 1;
-      const int qi = c % p.src_blocks, h = hkv * n_rep + (c / p.src_blocks) % n_rep, src = c / (p.src_blocks * n_rep);
-      const int q_pos0 = q_pos0_of(src, qi);
-      if (src != last_src) {   // lse / delta of a source are read below: it has to be complete
-        if (ok && !src_ready(p.fl, src, KID_ATTN_DKV)) { *abort_flag = 1; ok = false; }
-        last_src = src;
-      }
-      {  // stage this Q block's log-sum-exp (threads 0-127) and delta (threads 128-255), one column each
-        const int qrow = qi * BQ + (t256 & 127);
-        float val = (t256 < 128) ? INFINITY : 0.f;
-        if (qrow < p.src_len && t256 < 256) {
-          const size_t idx = ((size_t)b * p.lse_H + h) * p.src_len + qrow;
-          if (t256 < 128) {
-            const float l = p.lse_src.p[src][idx];
-            val = (l == -INFINITY) ? INFINITY : l * LOG2E;
-          } else {
-            val = p.delta_src.p[src][idx];
-          }
-        }
-        if (t256 < 256) (t256 < 128 ? s_lse : s_dlt)[st * 128 + (t256 & 127)] = val;
-        softmax_sync_all<NS>();
-      }
+      const int q_pos0 = w.at();
+      w.next();
+      const bool more = !w.done();
+      const float stat_next = more ? load_stat(w) : 0.f;
+      softmax_sync_all<NS>();   // this block's statistics are in place, the last block's have been read
       const bool need_mask = p.causal && k_pos0 + BKV - 1 > q_pos0;
       ok = ok && !*abort_flag && warp_wait(B_(KB_ST), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 8);
       float pr[CW];
@@ -1416,6 +1449,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
               np::pack_bf16(pr[e + 2] * (__uint_as_float(t[e + 2]) - d4.z), pr[e + 3] * (__uint_as_float(t[e + 3]) - d4.w));
         }
       }
+      if (more) put_stat(st ^ 1, stat_next);
       row_sync<NS>(quarter);   // same for dP^T -> dS^T
       if (ok) {
         tmem_st_cols<CW / 2>(tdPt + lane_off + hf * (CW / 2), pk);
