@@ -112,6 +112,100 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
   }
 }
 
+// Sums of R values per thread over the block (blockDim.x a multiple of 32, at most 512). `buf`: [2][R][16] floats; callers
+// alternate `par`, so one barrier per call is enough.
+template <int R>
+__device__ __forceinline__ void block_sums(float* v, float* buf, int par) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int q = 0; q < R; ++q) v[q] = np::warp_sum(v[q]);
+  float* b = buf + par * R * 16;
+  if (l == 0) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) b[q * 16 + w] = v[q];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < R; ++q) v[q] = np::warp_sum(l < nw ? b[q * 16 + l] : 0.f);   // the order of block_sum
+}
+
+constexpr int NR = 4;   // rows that the RMSNorm backward takes at a time
+// RMSNorm backward for up to 4096 columns, four rows per CTA at a time: one 8-wide vector of each row per thread, so the
+// loads of four rows are in flight and one barrier serves four sums; the weight gradient of a thread's eight columns stays in
+// registers over all its rows (a warp per row kept it in shared memory, 16 KB of traffic per row). With the column sum,
+// 4096 x 2048: 23.5 -> 21.1 us, 16384 x 2048: 63.8 -> 56.8, 4096 x 768: 22.2 -> 15.7 (DRAM-cold, floors 10, 41 and 4). The same
+// form of the forward pass was slower than a CTA per row (15.1 -> 20.6): it has half the traffic to hide a barrier behind.
+__global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy,
+                                                               const __nv_bfloat16* __restrict__ x,
+                                                               const float* __restrict__ w, const float* __restrict__ rstd,
+                                                               const __nv_bfloat16* __restrict__ dres,
+                                                               __nv_bfloat16* __restrict__ dx,
+                                                               float* __restrict__ dw_partial, int rows, int cols) {
+  np::pdl_begin();
+  __shared__ float buf[2 * NR * 16];
+  const int c = threadIdx.x;
+  const bool in = c < (cols >> 3);
+  float ww[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, dw[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (in) ld8f(w + c * 8, ww);
+  int par = 0;
+  for (int r0 = blockIdx.x * NR; r0 < rows; r0 += gridDim.x * NR, par ^= 1) {
+    uint4 gq[NR], xq[NR], rq[NR];
+    float rs[NR], dot[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      gq[q] = xq[q] = rq[q] = make_uint4(0, 0, 0, 0);
+      rs[q] = 0.f;
+      if (r0 + q < rows) {
+        rs[q] = rstd[r0 + q];
+        if (in) {
+          const size_t at = (size_t)(r0 + q) * cols + c * 8;
+          gq[q] = *reinterpret_cast<const uint4*>(dy + at);
+          xq[q] = *reinterpret_cast<const uint4*>(x + at);
+          if (dres) rq[q] = *reinterpret_cast<const uint4*>(dres + at);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      float g[8], xv[8];
+      unpack8(gq[q], g);
+      unpack8(xq[q], xv);
+      dot[q] = 0.f;
+      if (r0 + q < rows) {   // a row past the end contributes nothing, whatever rstd stands for
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = xv[j] * rs[q];
+          dw[j] += g[j] * xh;
+          dot[q] += g[j] * ww[j] * xh;
+        }
+      }
+    }
+    block_sums<NR>(dot, buf, par);
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      if (!in || r0 + q >= rows) break;
+      float g[8], xv[8], o[8];
+      unpack8(gq[q], g);
+      unpack8(xq[q], xv);
+      const float d = dot[q] / (float)cols;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = rs[q] * (g[j] * ww[j] - xv[j] * rs[q] * d);
+      if (dres) {
+        float t[8];
+        unpack8(rq[q], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += t[j];
+      }
+      store8(dx + (size_t)(r0 + q) * cols + c * 8, o);
+    }
+  }
+  if (in) {
+    float* dst = dw_partial + (size_t)blockIdx.x * cols + c * 8;
+    *reinterpret_cast<float4*>(dst) = make_float4(dw[0], dw[1], dw[2], dw[3]);
+    *reinterpret_cast<float4*>(dst + 4) = make_float4(dw[4], dw[5], dw[6], dw[7]);
+  }
+}
+
 // RMSNorm forward with an e4m3 output for an fp8 GEMM that follows: the normalised row (rounded to bf16 first, so the
 // result equals quantising the bf16 output of the plain kernel) is quantised per 1x128 block with an fp32 scale
 // amax / 448; y (bf16) is optional. cols must be a multiple of 128: a block is the 16 consecutive threads of a
@@ -316,75 +410,6 @@ __global__ void __launch_bounds__(256) colsum_tall_kernel(const float* __restric
   }
 }
 
-// RMSNorm backward with one warp per row (cols == 256 * VPL <= 2048): no block-wide reduction per row, so all rows
-// of the grid are in flight at once. Every warp adds its dw contributions into a private shared-memory row
-// (deterministic: no atomics); the eight rows are summed into one partial per CTA at the end. The row is read
-// twice, the second time from L1, to keep the register count low enough for three CTAs per SM.
-template <int VPL>
-__global__ void __launch_bounds__(NT) rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                              const __nv_bfloat16* __restrict__ x,
-                                                              const float* __restrict__ w,
-                                                              const float* __restrict__ rstd,
-                                                              const __nv_bfloat16* __restrict__ dres,
-                                                              __nv_bfloat16* __restrict__ dx,
-                                                              float* __restrict__ dw_partial, int rows, int cols) {
-  np::pdl_begin();
-  extern __shared__ float s_dw[];   // [8 warps][cols]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* mine = s_dw + (size_t)warp * cols;
-  for (int i = lane; i < cols; i += 32) mine[i] = 0.f;
-  __syncwarp();
-  for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
-    const float rs = rstd[r];
-    const __nv_bfloat16* gy = dy + (size_t)r * cols;
-    const __nv_bfloat16* xr = x + (size_t)r * cols;
-    float dot = 0.f;
-#pragma unroll 2
-    for (int i = 0; i < VPL; ++i) {
-      const int c = (lane + 32 * i) * 8;
-      float g[8], xv[8], ww[8];
-      load8(gy + c, g);
-      load8(xr + c, xv);
-      ld8f(w + c, ww);
-      float4 a0 = *reinterpret_cast<float4*>(mine + c), a1 = *reinterpret_cast<float4*>(mine + c + 4);
-      float acc[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = xv[j] * rs;
-        acc[j] += g[j] * xh;
-        dot += g[j] * ww[j] * xh;
-      }
-      *reinterpret_cast<float4*>(mine + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-      *reinterpret_cast<float4*>(mine + c + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-    }
-    dot = np::warp_sum(dot) / (float)cols;
-#pragma unroll 2
-    for (int i = 0; i < VPL; ++i) {
-      const int c = (lane + 32 * i) * 8;
-      float g[8], xv[8], ww[8], o[8];
-      load8(gy + c, g);
-      load8(xr + c, xv);
-      ld8f(w + c, ww);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = rs * (g[j] * ww[j] - xv[j] * rs * dot);
-      if (dres) {
-        float t[8];
-        load8(dres + (size_t)r * cols + c, t);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += t[j];
-      }
-      store8(dx + (size_t)r * cols + c, o);
-    }
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < cols; c += NT) {
-    float t = 0.f;
-#pragma unroll
-    for (int ww = 0; ww < 8; ++ww) t += s_dw[(size_t)ww * cols + c];
-    dw_partial[(size_t)blockIdx.x * cols + c] = t;
-  }
-}
-
 // ------------------------------------------------------------------ SwiGLU / GeGLU
 __device__ __forceinline__ float gelu_tanh_f(float x) {
   const float k = 0.7978845608028654f;
@@ -498,14 +523,14 @@ struct HeadSrc {
   long long row_stride, head_stride;
   int heads;
 };
-// One CTA per token; a thread takes a (head, 8-wide slice of the lower half) pair and produces both halves of the
-// rotation from two 16-byte loads, so every input element is read once. Slices outside the rotated range and the
-// V heads are copied.
-__global__ void __launch_bounds__(256) qkv_rope_kernel(HeadSrc s0, HeadSrc s1, HeadSrc s2,
-                                                       __nv_bfloat16* __restrict__ out,
-                                                       const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                       const int* __restrict__ pos_ids, long long T, int S, int pos_off,
-                                                       int hd, int rot, int rot_heads, float sign) {
+// A thread takes a (head, 8-wide slice of the lower half) pair and produces both halves of the rotation from two 16-byte
+// loads, so every input element is read once; slices outside the rotated range and the V heads are copied. The pair is the
+// thread's for all tokens of its CTA (one thread per pair where they fit a block), two tokens in flight: the head and
+// stride arithmetic per token cost as much as the copies (4096 tokens x 32 heads of 128: 18.6 us).
+__global__ void __launch_bounds__(1024) qkv_rope_kernel(HeadSrc s0, HeadSrc s1, HeadSrc s2, __nv_bfloat16* __restrict__ out,
+                                                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                                        const int* __restrict__ pos_ids, long long T, int S, int pos_off,
+                                                        int hd, int rot, int rot_heads, float sign) {
   np::pdl_begin();
   const int H = s0.heads + s1.heads + s2.heads;
   const int half = rot >> 1;
@@ -513,48 +538,60 @@ __global__ void __launch_bounds__(256) qkv_rope_kernel(HeadSrc s0, HeadSrc s1, H
   const int cv = (hd - rot) >> 3;              // slices of a rotated head that are only copied
   const int per_rot = hv + cv, per_plain = hd >> 3;
   const int items = rot_heads * per_rot + (H - rot_heads) * per_plain;
-  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
-    const int pos = pos_ids ? pos_ids[t] : (int)(t % S) + pos_off;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      int hh, v;
-      bool rotate;
-      if (it < rot_heads * per_rot) {
-        hh = it / per_rot;
-        v = it - hh * per_rot;
-        rotate = v < hv;
-      } else {
-        const int r = it - rot_heads * per_rot;
-        hh = rot_heads + r / per_plain;
-        v = r % per_plain;
-        rotate = false;
-      }
-      const __nv_bfloat16* src;
-      if (hh < s0.heads) src = s0.p + t * s0.row_stride + (long long)hh * s0.head_stride;
-      else if (hh < s0.heads + s1.heads) src = s1.p + t * s1.row_stride + (long long)(hh - s0.heads) * s1.head_stride;
-      else src = s2.p + t * s2.row_stride + (long long)(hh - s0.heads - s1.heads) * s2.head_stride;
-      __nv_bfloat16* dst = out + (t * H + hh) * (long long)hd;
-      if (rotate) {
-        const int d0 = v * 8;
-        float a[8], b[8], lo[8], hi[8];
-        load8(src + d0, a);
-        load8(src + d0 + half, b);
-        const float4 c0 = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * half + d0);
-        const float4 c1 = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * half + d0 + 4);
-        const float4 n0 = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * half + d0);
-        const float4 n1 = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * half + d0 + 4);
-        const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-        const float sn[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    int hh, v;
+    bool rotate;
+    if (it < rot_heads * per_rot) {
+      hh = it / per_rot;
+      v = it - hh * per_rot;
+      rotate = v < hv;
+    } else {
+      const int r = it - rot_heads * per_rot;
+      hh = rot_heads + r / per_plain;
+      v = r % per_plain;
+      rotate = false;
+    }
+    const int d0 = rotate ? v * 8 : (it < rot_heads * per_rot ? rot + (v - hv) * 8 : v * 8);
+    const __nv_bfloat16* src;
+    long long rs;
+    if (hh < s0.heads) { src = s0.p + (long long)hh * s0.head_stride; rs = s0.row_stride; }
+    else if (hh < s0.heads + s1.heads) { src = s1.p + (long long)(hh - s0.heads) * s1.head_stride; rs = s1.row_stride; }
+    else { src = s2.p + (long long)(hh - s0.heads - s1.heads) * s2.head_stride; rs = s2.row_stride; }
+    src += d0;
+    __nv_bfloat16* dst = out + (long long)hh * hd + d0;
+    const long long ds = (long long)H * hd;
+    for (long long t0 = blockIdx.x; t0 < T; t0 += 2ll * gridDim.x) {
+      uint4 aq[2], bq[2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float sj = sn[j] * sign;
-          lo[j] = a[j] * c[j] - b[j] * sj;
-          hi[j] = b[j] * c[j] + a[j] * sj;
+      for (int k = 0; k < 2; ++k) {
+        const long long t = t0 + (long long)k * gridDim.x;
+        if (t < T) {
+          aq[k] = *reinterpret_cast<const uint4*>(src + t * rs);
+          if (rotate) bq[k] = *reinterpret_cast<const uint4*>(src + t * rs + half);
         }
-        store8(dst + d0, lo);
-        store8(dst + d0 + half, hi);
-      } else {
-        const int d0 = (it < rot_heads * per_rot) ? rot + (v - hv) * 8 : v * 8;
-        *reinterpret_cast<uint4*>(dst + d0) = *reinterpret_cast<const uint4*>(src + d0);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const long long t = t0 + (long long)k * gridDim.x;
+        if (t >= T) break;
+        if (rotate) {
+          const int pos = pos_ids ? pos_ids[t] : (int)(T <= 0x7fffffff ? (unsigned)t % (unsigned)S : t % S) + pos_off;
+          float a[8], b[8], c[8], sn[8], lo[8], hi[8];
+          unpack8(aq[k], a);
+          unpack8(bq[k], b);
+          ld8f(cos_t + (size_t)pos * half + d0, c);
+          ld8f(sin_t + (size_t)pos * half + d0, sn);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float sj = sn[j] * sign;
+            lo[j] = a[j] * c[j] - b[j] * sj;
+            hi[j] = b[j] * c[j] + a[j] * sj;
+          }
+          store8(dst + t * ds, lo);
+          store8(dst + t * ds + half, hi);
+        } else {
+          *reinterpret_cast<uint4*>(dst + t * ds) = aq[k];
+        }
       }
     }
   }
@@ -797,14 +834,15 @@ __global__ void __launch_bounds__(NT) xent_fwd_kernel(const __nv_bfloat16* __res
   }
 }
 
-// dlogits[r, c] = (exp(logits - lse) - [c == label]) * gscale[0] * inv_count[0]; ignored rows -> 0.
-__global__ void __launch_bounds__(NT) xent_bwd_kernel(const __nv_bfloat16* __restrict__ logits,
-                                                      const long long* __restrict__ labels,
-                                                      const float* __restrict__ lse,
-                                                      const float* __restrict__ gscale,
-                                                      const float* __restrict__ inv_count,
-                                                      __nv_bfloat16* __restrict__ dlogits, int rows, int V,
-                                                      long long ld, long long ignore) {
+constexpr int XT = 512;   // threads of the backward
+// dlogits[r, c] = (exp(logits - lse) - [c == label]) * gscale[0] * inv_count[0]; ignored rows -> 0. Four vectors in flight
+// per thread: 4096 x 32000 119 -> 94 us (floor 80). Holding a whole row in registers, so that the forward reads it once, was
+// slower than its two reads with the second from L1 and L2 (70 -> 108 us).
+__global__ void __launch_bounds__(XT) xent_bwd_kernel(const __nv_bfloat16* __restrict__ logits,
+                                                      const long long* __restrict__ labels, const float* __restrict__ lse,
+                                                      const float* __restrict__ gscale, const float* __restrict__ inv_count,
+                                                      __nv_bfloat16* __restrict__ dlogits, int rows, int V, long long ld,
+                                                      long long ignore) {
   np::pdl_begin();
   const float sc = gscale[0] * inv_count[0];
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -812,21 +850,31 @@ __global__ void __launch_bounds__(NT) xent_bwd_kernel(const __nv_bfloat16* __res
     __nv_bfloat16* dr = dlogits + (size_t)r * ld;
     const long long lab = labels[r];
     const bool ign = (lab == ignore || lab < 0 || lab >= V);
+    const int hit = ign ? -1 : (int)lab;
     const float l = lse[r];
     const int nvec = V >> 3;
-    for (int c = threadIdx.x; c < nvec; c += NT) {
-      float f[8], o[8];
-      load8(lr + c * 8, f);
+    for (int c0 = threadIdx.x; c0 < nvec; c0 += 4 * XT) {
+      uint4 q[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float pr = __expf(f[j] - l);
-        o[j] = ign ? 0.f : (pr - ((long long)(c * 8 + j) == lab ? 1.f : 0.f)) * sc;
+      for (int i = 0; i < 4; ++i)
+        if (c0 + i * XT < nvec) q[i] = *reinterpret_cast<const uint4*>(lr + (c0 + i * XT) * 8);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = c0 + i * XT;
+        if (c >= nvec) break;
+        float f[8], o[8];
+        unpack8(q[i], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float pr = __expf(f[j] - l);
+          o[j] = ign ? 0.f : (pr - (c * 8 + j == hit ? 1.f : 0.f)) * sc;
+        }
+        store8(dr + c * 8, o);
       }
-      store8(dr + c * 8, o);
     }
-    for (int c = nvec * 8 + threadIdx.x; c < V; c += NT) {
+    for (int c = nvec * 8 + threadIdx.x; c < V; c += XT) {
       const float pr = __expf(__bfloat162float(lr[c]) - l);
-      dr[c] = __float2bfloat16(ign ? 0.f : (pr - ((long long)c == lab ? 1.f : 0.f)) * sc);
+      dr[c] = __float2bfloat16(ign ? 0.f : (pr - (c == hit ? 1.f : 0.f)) * sc);
     }
   }
 }
@@ -973,25 +1021,17 @@ static int launch_rmsnorm_bwd(const void* dy, const void* x, const float* w, con
                                cudaStream_t s) {
 #define RB(V) np_launch(rmsnorm_bwd_kernel<V>, grid, NT, 0, s, 1, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, \
                                                        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, cols)
-#define RBW(V) np_launch(rmsnorm_bwd_warp_kernel<V>, grid, NT, 8 * cols * sizeof(float), s, 1, \
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, \
-      rows, cols)
-  static NpPerDeviceOnce attr_once;
-  bool& attr_set = *attr_once.slot();
-  if (!attr_set) {   // the warp-per-row kernels keep 8 x cols floats in shared memory (64 KB at 2048 columns)
-    cudaError_t ea = cudaFuncSetAttribute(rmsnorm_bwd_warp_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2048 * 4);
-    if (ea == cudaSuccess)
-      ea = cudaFuncSetAttribute(rmsnorm_bwd_warp_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 1024 * 4);
-    if (ea != cudaSuccess) return 400 + (int)ea;
-    attr_set = true;
+  // up to 4096 columns a thread holds one vector of each of four rows; wider rows take one CTA per row
+  if (cols <= 4096) {
+    // NR rows at a time, every CTA the same number of turns (at most `grid` CTAs: the scratch has a row for each)
+    const int batches = (rows + NR - 1) / NR, turns = (batches + grid - 1) / grid;
+    grid = (batches + turns - 1) / turns;
+    np_launch(rmsnorm_bwd_rows_kernel, grid, (cols / 8 + 31) / 32 * 32, 0, s, 1, (const __nv_bfloat16*)dy,
+              (const __nv_bfloat16*)x, w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, cols);
+  } else {
+    RB(4);
   }
-  if (cols == 2048) RBW(8);
-  else if (cols == 1024) RBW(4);
-  else if (cols <= NT * 8) RB(1);
-  else if (cols <= NT * 16) RB(2);
-  else RB(4);
 #undef RB
-#undef RBW
   np_launch(colsum_tall_kernel, (cols + 31) / 32, 256, 0, s, 1, scratch, dw, grid, cols, accumulate_dw);
   return 0;
 }
@@ -1050,8 +1090,11 @@ NP_API int np_qkv_rope(const void* p0, long long rs0, long long hs0, int h0, con
   if (T <= 0) return 0;
   HeadSrc s0{(const __nv_bfloat16*)p0, rs0, hs0, h0}, s1{(const __nv_bfloat16*)p1, rs1, hs1, h1},
       s2{(const __nv_bfloat16*)p2, rs2, hs2, h2};
-  np_launch(qkv_rope_kernel, (unsigned)(T < GRID_CAP ? T : GRID_CAP), 256, 0, (cudaStream_t)stream, 1,
-      s0, s1, s2, (__nv_bfloat16*)out, cos_t, sin_t, pos_ids, T, S, pos_off, hd, rot, rot_heads, sign);
+  const int items = rot_heads * ((rot >> 4) + ((hd - rot) >> 3)) + (h0 + h1 + h2 - rot_heads) * (hd >> 3);
+  const int block = items >= 1024 ? 1024 : (items + 31) / 32 * 32;
+  const long long per_sm = block > 0 ? 2048 / block : 1, cap = 148 * per_sm, want = (T + 1) / 2;
+  np_launch(qkv_rope_kernel, (unsigned)(want < cap ? want : cap), block, 0, (cudaStream_t)stream, 1,
+            s0, s1, s2, (__nv_bfloat16*)out, cos_t, sin_t, pos_ids, T, S, pos_off, hd, rot, rot_heads, sign);
   CHECK_LAUNCH();
 }
 
@@ -1111,7 +1154,7 @@ NP_API int np_xent_bwd(const void* logits, const long long* labels, const float*
                        void* stream) {
   if (ld % 8) return 1;
   if (rows <= 0) return 0;
-  np_launch(xent_bwd_kernel, rows < GRID_CAP ? rows : GRID_CAP, NT, 0, (cudaStream_t)stream, 1,
+  np_launch(xent_bwd_kernel, rows < GRID_CAP ? rows : GRID_CAP, XT, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)logits, labels, lse, gscale, inv_count, (__nv_bfloat16*)dlogits, rows, V, ld, ignore);
   CHECK_LAUNCH();
 }

@@ -10,6 +10,26 @@ def rel(a, b):
     return ((a.double() - b.double()).norm() / (b.double().norm() + 1e-30)).item()
 
 
+# rows off the four-row batches and fewer than one, columns off a warp's 256
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 768), (5, 2048), (1023, 1032), (1187, 4096), (2600, 768), (9, 6144)])
+@pytest.mark.parametrize("res", [False, True])
+def test_rmsnorm_rows(rows, cols, res):
+    from nanopysche_b200.ops.norm import rms_norm
+
+    torch.manual_seed(rows)
+    x, r, dy, dh = (torch.randn(rows, cols, device="cuda").bfloat16() for _ in range(4))
+    w = (torch.rand(cols, device="cuda") + 0.5).requires_grad_(True)
+    xa, ra = x.clone().requires_grad_(True), r.clone().requires_grad_(True)
+    out = rms_norm(xa, w, 1e-6, ra if res else None)
+    y, h = out if res else (out, None)
+    torch.autograd.backward([y, h] if res else [y], [dy, dh] if res else [dy])
+    x64, w64 = x.double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    h64 = x64 + r.double() if res else x64
+    y64 = h64 * torch.rsqrt(h64.pow(2).mean(-1, keepdim=True) + 1e-6) * w64
+    torch.autograd.backward([y64, h64] if res else [y64], [dy.double(), dh.double()] if res else [dy.double()])
+    assert rel(y, y64) < 4e-3 and rel(xa.grad, x64.grad) < 5e-3 and rel(w.grad, w64.grad) < 5e-3
+
+
 # rows shorter than a vector per thread, a tail off the vectors, a row stride above the row's length
 @pytest.mark.parametrize("rows,V", [(3, 9), (70, 1003), (5, 16384), (33, 32000), (9, 50264), (2, 70003)])
 def test_cross_entropy_rows(rows, V):
@@ -28,3 +48,27 @@ def test_cross_entropy_rows(rows, V):
     ref = torch.nn.functional.cross_entropy(l64, labels, ignore_index=-100)
     ref.backward()
     assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item()) and rel(logits.grad, l64.grad) < 4e-3
+
+
+# one token, an odd number per CTA, more (head, slice) pairs than a block has threads, partial rotation
+@pytest.mark.parametrize("B,S,hq,hkv,hd,rot", [(1, 1, 2, 1, 64, 64), (2, 333, 16, 8, 128, 128), (1, 77, 12, 12, 64, 32),
+                                               (1, 40, 64, 64, 128, 128), (3, 1000, 4, 4, 64, 64)])
+def test_qkv_rope_shapes(B, S, hq, hkv, hd, rot):
+    from nanopysche_b200.ops.rope import apply_rope_ref, qkv_rope, rope_tables
+
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, (hq + 2 * hkv) * hd, device="cuda").bfloat16().requires_grad_(True)
+    cos, sin = rope_tables(S + 5, rot, device="cuda")
+    q, k, v = qkv_rope(qkv, cos, sin, hq, hkv, hd, pos_offset=5)
+    x = qkv.detach().double().requires_grad_(True)
+    h = x.view(B, S, hq + 2 * hkv, hd)
+    c, s = cos.double()[5:5 + S][None, :, None], sin.double()[5:5 + S][None, :, None]
+    a, b, rest = h[..., :rot // 2], h[..., rot // 2:rot], h[..., rot:]
+    r = torch.cat([a * c - b * s, b * c + a * s, rest], -1)
+    for got, want in ((q, r[:, :, :hq]), (k, r[:, :, hq:hq + hkv]), (v, h[:, :, hq + hkv:])):
+        assert rel(got, want) < 4e-3
+    gq, gk, gv = (torch.randn_like(t) for t in (q, k, v))
+    torch.autograd.backward([q, k, v], [gq, gk, gv])
+    torch.autograd.backward([r[:, :, :hq], r[:, :, hq:hq + hkv], h[:, :, hq + hkv:]], [gq.double(), gk.double(), gv.double()])
+    assert rel(qkv.grad, x.grad) < 4e-3
+    assert apply_rope_ref(q, cos, sin, 5).shape == q.shape
