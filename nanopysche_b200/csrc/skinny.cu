@@ -151,7 +151,7 @@ constexpr int DC_WARPS = 8;
 template <int HD, int R>
 __global__ void __launch_bounds__(DC_WARPS * 32, R <= 2 ? 2 : 1)
 decode_attn_kernel(const DecodeParams p) {
-  constexpr int L = HD / 8, KPW = 32 / L, U = R >= 8 ? 2 : 4;
+  constexpr int L = HD / 8, KPW = 32 / L, U = 2, STEP = DC_WARPS * KPW * U;
   __shared__ float s_m[DC_WARPS][R], s_l[DC_WARPS][R], s_acc[DC_WARPS][R][HD];
   __shared__ float c_m[R], c_l[R], c_acc[R][HD];
   np::pdl_begin();
@@ -170,69 +170,93 @@ decode_attn_kernel(const DecodeParams p) {
     m[r] = -INFINITY; l[r] = 0.f;
     last[r] = p.causal ? total - p.Sq + i : total - 1;
   }
-  for (int base = lo + warp * (KPW * U); base < hi; base += DC_WARPS * KPW * U) {   // the same trip count for the warp
-    uint4 kv[U], vv[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int key = base + u * KPW + sub;
-      kv[u] = vv[u] = make_uint4(0, 0, 0, 0);
-      if (key < hi) {
-        const bool old = key < p.past;
-        const long long j = old ? key : key - p.past;
-        const __nv_bfloat16* ks = old ? p.kc + b * p.kc_sb + j * p.kc_ss + h * p.kc_sh : p.kn + b * p.kn_sb + j * p.kn_ss + h * p.kn_sh;
-        const __nv_bfloat16* vs = old ? p.vc + b * p.vc_sb + j * p.vc_ss + h * p.vc_sh : p.vn + b * p.vn_sb + j * p.vn_ss + h * p.vn_sh;
-        kv[u] = *reinterpret_cast<const uint4*>(ks + d0);
-        vv[u] = *reinterpret_cast<const uint4*>(vs + d0);
-      }
-    }
-    float s[U][R];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int key = base + u * KPW + sub;
-      if (p.ko && key < hi) {
-        const long long off = (((long long)b * total + key) * p.Hkv + h) * HD + d0;
-        *reinterpret_cast<uint4*>(p.ko + off) = kv[u];
-        *reinterpret_cast<uint4*>(p.vo + off) = vv[u];
-      }
-      float f[8];
-      unpack8(kv[u], f);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float v = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v = fmaf(q[r][e], f[e], v);
-#pragma unroll
-        for (int x = L / 2; x > 0; x >>= 1) v += __shfl_xor_sync(0xffffffffu, v, x);
-        s[u][r] = (key < hi && key <= last[r]) ? v : -INFINITY;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float mx = m[r];
-#pragma unroll
-      for (int u = 0; u < U; ++u) mx = fmaxf(mx, s[u][r]);
-      const float mu = mx == -INFINITY ? 0.f : mx;
-      const float c = ex2a(m[r] - mu);
-      m[r] = mx;
-      l[r] *= c;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[r][e] *= c;
+  // Keys [k0, k1) of one source (row k0 at kp / vp), the first of them being key `key0` of the sequence. Two keys per lane
+  // group at a time, the next two already on their way.
+  auto attend = [&](const __nv_bfloat16* kp, const __nv_bfloat16* vp, long long kss, long long vss, int n, int key0) {
+    int at = warp * (KPW * U) + sub;                       // this lane group's first key
+    kp += at * kss + d0;
+    vp += at * vss + d0;
+    const long long kstep = STEP * kss, vstep = STEP * vss, ku = KPW * kss, vu = KPW * vss;
+    __nv_bfloat16* ko = p.ko ? p.ko + (((long long)b * total + key0 + at) * p.Hkv + h) * HD + d0 : nullptr;
+    __nv_bfloat16* vo = p.ko ? p.vo + (((long long)b * total + key0 + at) * p.Hkv + h) * HD + d0 : nullptr;
+    const long long ou = (long long)KPW * p.Hkv * HD, ostep = (long long)STEP * p.Hkv * HD;
+    uint4 kn[U], vn[U];
+    auto fetch = [&]() {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        s[u][r] = ex2a(s[u][r] - mu);
-        l[r] += s[u][r];
+        kn[u] = vn[u] = make_uint4(0, 0, 0, 0);
+        if (at + u * KPW < n) {
+          kn[u] = *reinterpret_cast<const uint4*>(kp + u * ku);
+          vn[u] = *reinterpret_cast<const uint4*>(vp + u * vu);
+        }
+      }
+    };
+    fetch();
+    for (int base = warp * (KPW * U); base < n; base += STEP) {   // the same trip count for the warp
+      uint4 kv[U], vv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) { kv[u] = kn[u]; vv[u] = vn[u]; }
+      const int cur = at;
+      at += STEP;
+      kp += kstep;
+      vp += vstep;
+      fetch();
+      float s[U][R];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = cur + u * KPW < n;
+        if (ko && in) {
+          *reinterpret_cast<uint4*>(ko + u * ou) = kv[u];
+          *reinterpret_cast<uint4*>(vo + u * ou) = vv[u];
+        }
+        float f[8];
+        unpack8(kv[u], f);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float v = 0.f;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v = fmaf(q[r][e], f[e], v);
+#pragma unroll
+          for (int x = L / 2; x > 0; x >>= 1) v += __shfl_xor_sync(0xffffffffu, v, x);
+          s[u][r] = (in && key0 + cur + u * KPW <= last[r]) ? v : -INFINITY;
+        }
+      }
+      if (ko) { ko += ostep; vo += ostep; }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float mx = m[r];
+#pragma unroll
+        for (int u = 0; u < U; ++u) mx = fmaxf(mx, s[u][r]);
+        const float mu = mx == -INFINITY ? 0.f : mx;
+        const float c = ex2a(m[r] - mu);
+        m[r] = mx;
+        l[r] *= c;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[r][e] *= c;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          s[u][r] = ex2a(s[u][r] - mu);
+          l[r] += s[u][r];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float f[8];
+        unpack8(vv[u], f);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(s[u][r], f[e], acc[r][e]);
       }
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float f[8];
-      unpack8(vv[u], f);
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(s[u][r], f[e], acc[r][e]);
-    }
-  }
+  };
+  const int c_hi = hi < p.past ? hi : p.past, f_lo = lo > p.past ? lo : p.past;
+  if (lo < c_hi)
+    attend(p.kc + b * p.kc_sb + lo * p.kc_ss + h * p.kc_sh, p.vc + b * p.vc_sb + lo * p.vc_ss + h * p.vc_sh, p.kc_ss, p.vc_ss,
+           c_hi - lo, lo);
+  if (f_lo < hi)
+    attend(p.kn + b * p.kn_sb + (f_lo - p.past) * p.kn_ss + h * p.kn_sh, p.vn + b * p.vn_sb + (f_lo - p.past) * p.vn_ss + h * p.vn_sh,
+           p.kn_ss, p.vn_ss, hi - f_lo, f_lo);
   // the groups of lanes, then the warps, then the CTAs of the cluster
 #pragma unroll
   for (int r = 0; r < R; ++r) {
