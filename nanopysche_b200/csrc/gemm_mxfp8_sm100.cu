@@ -11,7 +11,7 @@
 //
 // CTA roles: warp 0 lane 0 issues the copies (TMA tiles of A and B, bulk copies of the scale chunks) into a
 // 5-stage ring; warp 1 lane 0 copies the scales of a stage into TMEM and issues four K = 32 MMAs whose instruction
-// descriptors select byte 0..3 of the scale words; warps 2-5 drain one of two 192-column accumulators (tcgen05.ld)
+// descriptors select byte 0..3 of the scale words; warps 2-9 drain one of two 192-column accumulators (tcgen05.ld)
 // while the next tile accumulates into the other. The tile is 128 x 192: two 192-column fp32 accumulators plus the
 // scale columns fit the 512 TMEM columns (two 256-column ones would leave none for the scales), and the operand
 // bytes per FLOP that cross from L2 drop by a fifth against a 128 x 128 tile. A 192-row B tile starts at row 0 or
@@ -89,7 +89,26 @@ __host__ __device__ constexpr uint32_t make_idesc_mx(int m, int n, int a_sf, int
          ((uint32_t)a_sf << 29);
 }
 
-__global__ void __launch_bounds__(192, 1)
+// 64 bytes of a row, as two 32-byte stores where the row allows it: a full sector per request (16-byte stores made the drain
+// of a 128 x 192 tile longer than its 16 K steps at K = 2048)
+__device__ __forceinline__ void store64(void* dst, const uint32_t* o, bool st32) {
+  if (st32) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"((char*)dst + 32 * h), "r"(o[8 * h]),
+                   "r"(o[8 * h + 1]), "r"(o[8 * h + 2]), "r"(o[8 * h + 3]), "r"(o[8 * h + 4]), "r"(o[8 * h + 5]),
+                   "r"(o[8 * h + 6]), "r"(o[8 * h + 7])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      reinterpret_cast<uint4*>(dst)[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+  }
+}
+// Epilogue warps: two per tensor-memory lane quarter, half of the columns each
+constexpr int EPI_WARPS = 8, MX_THREADS = 64 + 32 * EPI_WARPS;
+
+__global__ void __launch_bounds__(MX_THREADS, 1)
 gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const MxParams p) {
   constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, STAGE_BYTES = A_BYTES + B_BYTES + SF_SMEM;
   constexpr int TX_BYTES = A_BYTES + B_BYTES + 3 * SF_BYTES;
@@ -112,7 +131,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { np::mbar_init(full_bar(s), 1); np::mbar_init(empty_bar(s), 1); }
-    for (int a = 0; a < 2; ++a) { np::mbar_init(afull_bar(a), 1); np::mbar_init(aempty_bar(a), 4); }
+    for (int a = 0; a < 2; ++a) { np::mbar_init(afull_bar(a), 1); np::mbar_init(aempty_bar(a), EPI_WARPS); }
     *abort_flag = 0;
     np::mbar_fence_init();
     np::tma_prefetch_desc(&tmA);
@@ -179,46 +198,51 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (*abort_flag) __nanosleep(1000000);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
-        const int m_blk = t % m_blocks, n_blk = t / m_blocks;
-        const int trows = tile_rows(m_blk, 1);
-        if (trows < 0) break;
-        if (trows == 0) continue;
-        // B scales of the tile's first row sit in column (row % 128) / 32 of the first chunk's four columns
-        const uint32_t sfb_off = (uint32_t)((b_row0(m_blk, n_blk) % 128) / 32);
-        bool ok = np::mbar_wait(aempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_MX, 2);
+    // the whole warp walks the loop, one elected lane issues; descriptors are built once and advanced by constants
+    const uint64_t a_desc0 = np::make_smem_desc(smem_base, 16, 1024), b_desc0 = np::make_smem_desc(smem_base + A_BYTES, 16, 1024);
+    const uint64_t sf_desc0 = desc_noswizzle(smem_base + A_BYTES + B_BYTES, 16, 128);
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+      const int m_blk = t % m_blocks, n_blk = t / m_blocks;
+      const int trows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(m_blk, 1) : 0, 0);
+      if (trows < 0) break;
+      if (trows == 0) continue;
+      // B scales of the tile's first row sit in column (row % 128) / 32 of the first chunk's four columns
+      const uint32_t sfb_off = (uint32_t)((b_row0(m_blk, n_blk) % 128) / 32);
+      bool ok = np::mbar_wait_warp(aempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_MX, 2);
+      if (!ok) break;
+      const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+      for (int kb = 0; kb < nkb; ++kb) {
+        ok = np::mbar_wait_warp(full_bar(stage), phase, abort_flag, KID_MX, 3);
         if (!ok) break;
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
-        for (int kb = 0; kb < nkb && ok; ++kb) {
-          ok = np::mbar_wait(full_bar(stage), phase, abort_flag, KID_MX, 3);
-          if (!ok) break;
-          np::tc_fence_after();
-          const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES, sSF = sB + B_BYTES;
+        np::tc_fence_after();
+        if (np::elect_one()) {
+          const uint32_t off = (uint32_t)(stage * (STAGE_BYTES >> 4));
+          const uint64_t ad = a_desc0 + off, bd = b_desc0 + off, sd = sf_desc0 + off;
           const uint32_t t_sfa = tmem_base + (uint32_t)(SF_COL0 + stage * SF_COLS), t_sfb = t_sfa + 4;
-          tmem_cp_32x128b_x4(t_sfa, desc_noswizzle(sSF, 16, 128));
-          tmem_cp_32x128b_x4(t_sfb, desc_noswizzle(sSF + SF_BYTES, 16, 128));
-          tmem_cp_32x128b_x4(t_sfb + 4, desc_noswizzle(sSF + 2 * SF_BYTES, 16, 128));
+          tmem_cp_32x128b_x4(t_sfa, sd);
+          tmem_cp_32x128b_x4(t_sfb, sd + (SF_BYTES >> 4));
+          tmem_cp_32x128b_x4(t_sfb + 4, sd + 2 * (SF_BYTES >> 4));
+          np::tc_fence_after();
 #pragma unroll
-          for (int kk = 0; kk < BK / 32; ++kk) {
-            const uint64_t ad = np::make_smem_desc(sA + kk * 32, 16, 1024);
-            const uint64_t bd = np::make_smem_desc(sB + kk * 32, 16, 1024);
-            np::tc_fence_after();
-            tc_mma_mxf8(tmem_d, ad, bd, make_idesc_mx(BM, BN, kk, kk), t_sfa, t_sfb + sfb_off, (kb | kk) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < BK / 32; ++kk)
+            tc_mma_mxf8(tmem_d, ad + kk * 2, bd + kk * 2, make_idesc_mx(BM, BN, kk, kk), t_sfa, t_sfb + sfb_off,
+                        (kb | kk) ? 1u : 0u);
           np::tc_commit(empty_bar(stage));
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (!ok) break;
-        np::tc_commit(afull_bar(acc));
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
-      if (*abort_flag) __nanosleep(1000000);
+      if (!ok) break;
+      if (np::elect_one()) np::tc_commit(afull_bar(acc));
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
+    if (*abort_flag) __nanosleep(1000000);
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const bool st32 = (((uintptr_t)p.C & 31) == 0 || p.row_dst) && p.ldc % (p.out_f32 ? 8 : 16) == 0;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
@@ -242,28 +266,37 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       } else {
         crow = (char*)p.C + (size_t)row * p.ldc * (p.out_f32 ? 4 : 2);
       }
-#pragma unroll
-      for (int c = 0; c < BN / 32; ++c) {
+#pragma unroll 1
+      for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
         uint32_t r[32];
+        __syncwarp();
         np::tmem_ld32(taddr + c * 32, r);        // warp-uniform: every lane loads, only stores are guarded
         np::tmem_ld_wait();
-        if (row_ok) {
-          if (p.out_f32) {
-            float* dst = (float*)crow + n0 + c * 32;
+        const int col = n0 + c * 32;
+        if (!row_ok || col >= p.N) continue;
+        if (p.out_f32) {
+          float* dst = (float*)crow + col;
+          if (col + 32 <= p.N) {
+            store64(dst, r, st32);
+            store64(dst + 16, r + 16, st32);
+          } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-              if (n0 + c * 32 + 4 * i + 4 <= p.N)
+              if (col + 4 * i + 4 <= p.N)
                 reinterpret_cast<uint4*>(dst)[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+          }
+        } else {
+          __nv_bfloat16* dst = (__nv_bfloat16*)crow + col;
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[i] = np::pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          if (col + 32 <= p.N) {
+            store64(dst, w, st32);
           } else {
-            __nv_bfloat16* dst = (__nv_bfloat16*)crow + n0 + c * 32;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              if (n0 + c * 32 + 8 * i + 8 <= p.N)
-                reinterpret_cast<uint4*>(dst)[i] = make_uint4(
-                    np::pack_bf16(__uint_as_float(r[8 * i]), __uint_as_float(r[8 * i + 1])),
-                    np::pack_bf16(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3])),
-                    np::pack_bf16(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5])),
-                    np::pack_bf16(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7])));
+              if (col + 8 * i + 8 <= p.N)
+                reinterpret_cast<uint4*>(dst)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
           }
         }
       }
@@ -277,7 +310,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (lane == 0) {
           const int fi = p.mblk_flag ? p.mblk_flag[m_blk] : 0;
           const int done = atomicAdd(&p.done_counters[fi], 1) + 1;
-          if (done == 4 * n_blocks * p.done_expected[fi]) {
+          if (done == EPI_WARPS * n_blocks * p.done_expected[fi]) {
             __threadfence_system();
             np::st_release_sys(p.done_flag_ptr[fi], epoch);
           }
@@ -573,7 +606,7 @@ NP_API int np_gemm_mxfp8(const NpMxGemmArgs* args, void* stream) {
   const long long tiles = (long long)((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN);
   const int cap = a.max_ctas > 0 ? a.max_ctas : sms;
   const int grid = (int)(tiles < cap ? tiles : cap);
-  gemm_mxfp8_kernel<<<grid, 192, SMEM, (cudaStream_t)stream>>>(tmA, tmB, p);
+  gemm_mxfp8_kernel<<<grid, MX_THREADS, SMEM, (cudaStream_t)stream>>>(tmA, tmB, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
