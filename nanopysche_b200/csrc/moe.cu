@@ -35,49 +35,57 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 // ------------------------------------------------------------------ router
-// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). One warp per token; the register
-// cap keeps four CTAs per SM resident so that enough row loads are in flight; the gate weights come from L1.
-template <int EB>
-__global__ void __launch_bounds__(256, 4) router_logits_kernel(const __nv_bfloat16* __restrict__ x,
-                                                               const float* __restrict__ wg,
-                                                               const float* __restrict__ bias,
-                                                               float* __restrict__ logits, int T, int D, int E) {
+// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). A warp takes TOK tokens at a time, so that a
+// gate vector read from L1 serves all of them: with one token per warp the gate reads (64 KB per token at d 2048, 8 experts)
+// were the kernel's time (4096 tokens: 21 us). Every token's sum is formed in the same order whatever TOK is.
+template <int EB, int TOK>
+__global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wg,
+                                                            const float* __restrict__ bias, float* __restrict__ logits, int T,
+                                                            int D, int E) {
   np::pdl_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int t = warp; t < T; t += nwarps) {
+  for (int t0 = warp * TOK; t0 < T; t0 += nwarps * TOK) {
     for (int e0 = 0; e0 < E; e0 += EB) {
-      float acc[EB];
+      float acc[TOK][EB];
 #pragma unroll
-      for (int e = 0; e < EB; ++e) acc[e] = 0.f;
-      for (int d = lane * 8; d < D; d += 512) {
-        const bool two = d + 256 < D;
-        const uint4 q0 = *reinterpret_cast<const uint4*>(x + (size_t)t * D + d);
-        const uint4 q1 = two ? *reinterpret_cast<const uint4*>(x + (size_t)t * D + d + 256) : make_uint4(0, 0, 0, 0);
+      for (int k = 0; k < TOK; ++k)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && !two) break;
-          float xv[8];
-          const uint4 q = h ? q1 : q0;
-          float2 a = np::unpack_bf16(q.x), b = np::unpack_bf16(q.y), c = np::unpack_bf16(q.z), dd = np::unpack_bf16(q.w);
-          xv[0] = a.x; xv[1] = a.y; xv[2] = b.x; xv[3] = b.y; xv[4] = c.x; xv[5] = c.y; xv[6] = dd.x; xv[7] = dd.y;
+        for (int e = 0; e < EB; ++e) acc[k][e] = 0.f;
+      for (int d = lane * 8; d < D; d += 256) {
+        uint4 q[TOK];
 #pragma unroll
-          for (int e = 0; e < EB; ++e) {
-            if (e0 + e < E) {
-              const float* wp = wg + (size_t)(e0 + e) * D + d + h * 256;
-              const float4 w0 = __ldg(reinterpret_cast<const float4*>(wp));
-              const float4 w1 = __ldg(reinterpret_cast<const float4*>(wp + 4));
-              acc[e] += xv[0] * w0.x + xv[1] * w0.y + xv[2] * w0.z + xv[3] * w0.w + xv[4] * w1.x + xv[5] * w1.y +
-                        xv[6] * w1.z + xv[7] * w1.w;
-            }
+        for (int k = 0; k < TOK; ++k)
+          q[k] = t0 + k < T ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + k) * D + d) : make_uint4(0, 0, 0, 0);
+        float xv[TOK][8];
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) {
+          const float2 a = np::unpack_bf16(q[k].x), b = np::unpack_bf16(q[k].y), c = np::unpack_bf16(q[k].z),
+                       dd = np::unpack_bf16(q[k].w);
+          xv[k][0] = a.x; xv[k][1] = a.y; xv[k][2] = b.x; xv[k][3] = b.y;
+          xv[k][4] = c.x; xv[k][5] = c.y; xv[k][6] = dd.x; xv[k][7] = dd.y;
+        }
+#pragma unroll
+        for (int e = 0; e < EB; ++e) {
+          if (e0 + e < E) {
+            const float* wp = wg + (size_t)(e0 + e) * D + d;
+            const float4 w0 = __ldg(reinterpret_cast<const float4*>(wp));
+            const float4 w1 = __ldg(reinterpret_cast<const float4*>(wp + 4));
+#pragma unroll
+            for (int k = 0; k < TOK; ++k)
+              acc[k][e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
+                           xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
           }
         }
       }
 #pragma unroll
-      for (int e = 0; e < EB; ++e) {
-        const float sm = np::warp_sum(acc[e]);
-        if (lane == 0 && e0 + e < E) logits[(size_t)t * E + e0 + e] = sm + (bias ? bias[e0 + e] : 0.f);
+      for (int k = 0; k < TOK; ++k) {
+#pragma unroll
+        for (int e = 0; e < EB; ++e) {
+          const float sm = np::warp_sum(acc[k][e]);
+          if (lane == 0 && e0 + e < E && t0 + k < T) logits[(size_t)(t0 + k) * E + e0 + e] = sm + (bias ? bias[e0 + e] : 0.f);
+        }
       }
     }
   }
@@ -176,6 +184,21 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
     atomicAdd(&psum[i], s_p[i]);
   }
   if (threadIdx.x == 0) atomicAdd(zsum, s_z);
+}
+
+// f[e] = counts[e] / T and aux = E * sum_e f[e] * psum[e] / T + coef_z * zsum / T (one warp)
+__global__ void __launch_bounds__(32) router_aux_kernel(const int* __restrict__ counts, const float* __restrict__ psum,
+                                                        const float* __restrict__ zsum, float coef_z, float* __restrict__ f,
+                                                        float* __restrict__ aux, int T, int E) {
+  np::pdl_begin();
+  float s = 0.f;
+  for (int e = threadIdx.x; e < E; e += 32) {
+    const float fe = (float)counts[e] / (float)T;
+    f[e] = fe;
+    s += fe * (psum[e] / (float)T);
+  }
+  s = np::warp_sum(s);
+  if (threadIdx.x == 0) aux[0] = (float)E * s + (coef_z != 0.f ? coef_z * zsum[0] / (float)T : 0.f);
 }
 
 // dlogits[t, :] from d(weights) and d(aux): aux = coef_lb * E * sum_i f_i * mean_t p[t,i]
@@ -476,7 +499,8 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* __restri
                                                              int capacity, int* __restrict__ slot_pos,
                                                              int* __restrict__ keep, int* __restrict__ counts_kept,
                                                              int* __restrict__ drops, int* __restrict__ n_dropped,
-                                                             int use_smem) {
+                                                             int use_smem, int* __restrict__ sent, int n_ranks,
+                                                             long long* __restrict__ stats) {
   np::pdl_begin();
   constexpr int EPW = 64 / FB;          // experts per 64-bit word
   constexpr int GROUP = 4 * EPW;        // experts per pass
@@ -487,7 +511,8 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* __restri
   unsigned char* s_keep = reinterpret_cast<unsigned char*>(s_dyn + (use_smem ? T * K : 0));
   const int* idx = indices;
   if (use_smem) {
-    for (int i = threadIdx.x; i < T * K; i += blockDim.x) s_idx[i] = indices[i];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < T * K; i += blockDim.x) s_idx[i] = __ldg(indices + i);   // several loads in flight
     for (int t = threadIdx.x; t < T; t += blockDim.x) s_keep[t] = 1;
     idx = s_idx;
   } else {
@@ -552,7 +577,22 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* __restri
   }
   U64x4 ndv{{(unsigned long long)nd, 0ull, 0ull, 0ull}}, total;
   block_excl_scan4(ndv, 1, s_warp, &total);
-  if (threadIdx.x == 0) n_dropped[0] = (int)total.w[0];
+  if (threadIdx.x == 0) {
+    n_dropped[0] = (int)total.w[0];
+    if (stats) {   // last step's drops, all drops, all tokens
+      stats[0] = (long long)total.w[0];
+      stats[1] += (long long)total.w[0];
+      stats[2] += T;
+    }
+  }
+  if (sent) {      // kept rows per expert-parallel rank (counts_kept was written before the barriers of the scan above)
+    const int per_rank = E / n_ranks;
+    for (int r = threadIdx.x; r < n_ranks; r += blockDim.x) {
+      int n = 0;
+      for (int e = r * per_rank; e < (r + 1) * per_rank; ++e) n += counts_kept[e];
+      sent[r] = n;
+    }
+  }
 }
 
 // ------------------------------------------------------------------ EP dispatch (peer stores)
@@ -613,19 +653,28 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p
     const size_t row = ((size_t)le * p.n_ranks + p.my_rank) * p.region_rows + pos;
     if (!p.quant) {
       uint4* dst = reinterpret_cast<uint4*>((__nv_bfloat16*)p.peer_rows[peer] + row * p.D);
-      for (int v = lane; v < (p.D >> 3); v += 32) {
-        uint4 u = make_uint4(0, 0, 0, 0);
-        if (!is_pad) {
-          u = *reinterpret_cast<const uint4*>(src + v * 8);
+      // four vectors of the row in flight per lane: one load per store had the row's latency eight times over
+      const int nv = p.D >> 3;
+      for (int v0 = lane; v0 < nv; v0 += 128) {
+        uint4 u[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          u[q] = make_uint4(0, 0, 0, 0);
+          if (!is_pad && v0 + 32 * q < nv) u[q] = *reinterpret_cast<const uint4*>(src + (v0 + 32 * q) * 8);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (v0 + 32 * q >= nv) break;
           if (p.slot_scale) {
             float f[8];
-            float2 a = np::unpack_bf16(u.x), b = np::unpack_bf16(u.y), c = np::unpack_bf16(u.z), d = np::unpack_bf16(u.w);
+            const float2 a = np::unpack_bf16(u[q].x), b = np::unpack_bf16(u[q].y), c = np::unpack_bf16(u[q].z),
+                         d = np::unpack_bf16(u[q].w);
             f[0] = a.x * sc; f[1] = a.y * sc; f[2] = b.x * sc; f[3] = b.y * sc;
             f[4] = c.x * sc; f[5] = c.y * sc; f[6] = d.x * sc; f[7] = d.y * sc;
-            u = pack8(f);
+            u[q] = pack8(f);
           }
+          dst[v0 + 32 * q] = u[q];
         }
-        dst[v] = u;
       }
     } else {
       // 16 lanes x 8 elements = one 128-element scale block; two blocks per warp iteration
@@ -746,17 +795,32 @@ __global__ void __launch_bounds__(256) ep_combine_kernel(const CombineParams p) 
   const long long total = (long long)p.T * vec_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(i / vec_per_row);
+    const int t = total <= 0x7fffffff ? (int)((unsigned)i / (unsigned)vec_per_row) : (int)(i / vec_per_row);
     const int d = (int)(i - (long long)t * vec_per_row) * 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < p.K; ++k) {
-      if (p.slot_pos[(size_t)t * p.K + k] < 0) continue;
-      NP_DBG_SKIP_UNLESS(p.slot_pos[(size_t)t * p.K + k] < (1 << 24), KID_COMBINE, p.slot_pos[(size_t)t * p.K + k])
-      float f[8];
-      load8(p.rows + ((size_t)t * p.K + k) * p.D + d, f);
-      const float w = p.weights ? p.weights[(size_t)t * p.K + k] : 1.f;
+    for (int k0 = 0; k0 < p.K; k0 += 2) {   // two rows in flight
+      uint4 q[2];
+      float w[2];
+      bool on[2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += w * f[j];
+      for (int u = 0; u < 2; ++u) {
+        const size_t slot = (size_t)t * p.K + k0 + u;
+        on[u] = k0 + u < p.K && p.slot_pos[slot] >= 0;
+        q[u] = make_uint4(0, 0, 0, 0);
+        w[u] = 0.f;
+        if (on[u]) {
+          q[u] = *reinterpret_cast<const uint4*>(p.rows + slot * p.D + d);
+          w[u] = p.weights ? p.weights[slot] : 1.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (!on[u]) continue;
+        const float2 a = np::unpack_bf16(q[u].x), b = np::unpack_bf16(q[u].y), c = np::unpack_bf16(q[u].z),
+                     e = np::unpack_bf16(q[u].w);
+        acc[0] += w[u] * a.x; acc[1] += w[u] * a.y; acc[2] += w[u] * b.x; acc[3] += w[u] * b.y;
+        acc[4] += w[u] * c.x; acc[5] += w[u] * c.y; acc[6] += w[u] * e.x; acc[7] += w[u] * e.y;
+      }
     }
     if (p.add1) {
       float f[8];
@@ -816,8 +880,12 @@ __global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* __re
 NP_API int np_router_logits(const void* x, const float* wg, const float* bias, float* logits, int T, int D, int E,
                             void* stream) {
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
-  const int grid = (T * 32 + 255) / 256 < 148 * 8 ? (T * 32 + 255) / 256 : 148 * 8;
-  np_launch(router_logits_kernel<8>, grid, 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias, logits, T, D, E);
+  // four tokens per warp once that still leaves eight warps for every SM
+  const int tok = T >= 148 * 8 * 4 / 2 ? 4 : 1;
+  const long long warps = ((long long)T + tok - 1) / tok, blocks = (warps * 32 + 255) / 256;
+  np_launch(tok == 4 ? router_logits_kernel<8, 4> : router_logits_kernel<8, 1>,
+            (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
+            logits, T, D, E);
   CHECK_LAUNCH();
 }
 
@@ -833,6 +901,13 @@ NP_API int np_router_topk(const float* logits, const float* score_bias, float* w
   else if (E <= 32) TOPK(32);
   else TOPK(64);
 #undef TOPK
+  CHECK_LAUNCH();
+}
+
+NP_API int np_router_aux(const int* counts, const float* psum, const float* zsum, float coef_z, float* f, float* aux, int T,
+                         int E, void* stream) {
+  if (T <= 0 || E > MAX_E) return 1;
+  np_launch(router_aux_kernel, 1, 32, 0, (cudaStream_t)stream, 1, counts, psum, zsum, coef_z, f, aux, T, E);
   CHECK_LAUNCH();
 }
 
@@ -877,9 +952,11 @@ NP_API int np_router_dx(const float* dl, const float* wg, void* dx, int T, int D
   CHECK_LAUNCH();
 }
 
-NP_API int np_capacity_scan(const int* indices, int T, int E, int K, int capacity, int* slot_pos, int* keep,
-                            int* counts_kept, int* drops, int* n_dropped, void* stream) {
-  if (K > MAX_K) return 1;
+// np_capacity_scan with the kept rows per rank (sent [n_ranks], may be null) and the running drop statistics (stats [3]:
+// last dropped, total dropped, total tokens; may be null) in the same launch.
+NP_API int np_capacity_plan(const int* indices, int T, int E, int K, int capacity, int* slot_pos, int* keep, int* counts_kept,
+                            int* drops, int* n_dropped, int* sent, int n_ranks, long long* stats, void* stream) {
+  if (K > MAX_K || (sent && (n_ranks <= 0 || E % n_ranks))) return 1;
   if (T <= 0) return 0;
   const size_t smem = (size_t)T * K * 4 + (size_t)((T + 3) / 4) * 4;
   const int use_smem = smem <= 200 * 1024;
@@ -894,11 +971,16 @@ NP_API int np_capacity_scan(const int* indices, int T, int E, int K, int capacit
   }
   if (T < 65536)   // a 16-bit counter holds any per-expert count
     np_launch(capacity_scan_kernel<16>, 1, 1024, use_smem ? smem : 0, (cudaStream_t)stream, 1,
-        indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem);
+        indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem, sent, n_ranks, stats);
   else
     np_launch(capacity_scan_kernel<32>, 1, 1024, use_smem ? smem : 0, (cudaStream_t)stream, 1,
-        indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem);
+        indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem, sent, n_ranks, stats);
   CHECK_LAUNCH();
+}
+
+NP_API int np_capacity_scan(const int* indices, int T, int E, int K, int capacity, int* slot_pos, int* keep, int* counts_kept,
+                            int* drops, int* n_dropped, void* stream) {
+  return np_capacity_plan(indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, nullptr, 0, nullptr, stream);
 }
 
 struct NpDispatchArgs {

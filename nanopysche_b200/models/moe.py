@@ -573,9 +573,13 @@ class MoEBase(nn.Module):
         self._record_drops(dropped, T, x.device)
         return x[keep_mask], weights[keep_mask], indices[keep_mask], dropped, keep_mask
 
-    def _record_drops(self, dropped, T, device):
+    def _drop_stats(self, device) -> torch.Tensor:
         if self._stats is None or self._stats.device != device:
             self._stats = torch.zeros(3, dtype=torch.long, device=device)
+        return self._stats
+
+    def _record_drops(self, dropped, T, device):
+        self._drop_stats(device)
         d = dropped if torch.is_tensor(dropped) else torch.tensor(dropped, device=device)
         self._stats[0] = d
         self._stats[1] += d

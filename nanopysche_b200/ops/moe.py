@@ -44,14 +44,12 @@ class _Router(torch.autograd.Function):
         _lib.call("router_logits", x2, gate_w, gate_b, logits, T, D, E)
         weights = torch.empty((T, K), device=dev, dtype=torch.float32)
         indices = torch.empty((T, K), device=dev, dtype=torch.int32)
-        stats = torch.zeros(2 * E + 1, device=dev, dtype=torch.float32)
-        counts = torch.zeros(E, device=dev, dtype=torch.int32)
-        _lib.call("router_topk", logits, score_bias, weights, indices, counts, stats[:E], stats[E:E + 1], T, E, K,
-                  gating)
-        f = counts.float() / T
-        aux = E * (f * (stats[:E] / T)).sum()
-        if coef_z:
-            aux = aux + coef_z * stats[E] / T
+        zeros = torch.zeros(2 * E + 1, device=dev, dtype=torch.int32)   # token counts, probability sums, sum of lse^2
+        counts, stats = zeros[:E], zeros[E:].view(torch.float32)
+        _lib.call("router_topk", logits, score_bias, weights, indices, counts, stats[:E], stats[E:], T, E, K, gating)
+        fa = torch.empty(E + 1, device=dev, dtype=torch.float32)
+        f, aux = fa[:E], fa[E]
+        _lib.call("router_aux", counts, stats[:E], stats[E:], float(coef_z or 0.0), f, aux, T, E)
         ctx.save_for_backward(x2, gate_w, logits, weights, indices, f, score_bias if score_bias is not None
                               else logits.new_empty(0))
         ctx.cfg = (K, gating, float(coef_z or 0.0), score_bias is not None)
@@ -82,8 +80,9 @@ class _Router(torch.autograd.Function):
         return dx, dgw, dgb, None, None, None, None
 
 
-def route(x: torch.Tensor, router) -> tuple:
-    """Kernel path of ``MoERouter.forward`` for bf16 CUDA input: (weights, indices int64, aux, counts)."""
+def route(x: torch.Tensor, router, int64: bool = True) -> tuple:
+    """Kernel path of ``MoERouter.forward`` for bf16 CUDA input: (weights, indices int64, aux, counts). ``int64=False``
+    leaves the indices in the kernels' int32."""
     cfg = router.config
     D = x.shape[-1]
     x2 = x.reshape(-1, D)
@@ -92,7 +91,7 @@ def route(x: torch.Tensor, router) -> tuple:
     w, idx, aux, counts = _Router.apply(x2, router.gate.weight, router.gate.bias, router.score_bias, router.top_k,
                                         gating, cfg.z_loss_multiplier or 0.0)
     lead = x.shape[:-1]
-    return w.view(*lead, -1), idx.long().view(*lead, -1), aux, counts
+    return w.view(*lead, -1), (idx.long() if int64 else idx).view(*lead, -1), aux, counts
 
 
 # ------------------------------------------------------------------------------------------------ runtime
@@ -378,8 +377,9 @@ class _FusedMoE(torch.autograd.Function):
         counts_kept = torch.empty(rt.E, device=dev, dtype=torch.int32)
         drops = torch.empty(rt.E, device=dev, dtype=torch.int32)
         n_dropped = torch.empty(1, device=dev, dtype=torch.int32)
-        _lib.call("capacity_scan", indices32, T, rt.E, K, rt.capacity, slot_pos, keep, counts_kept, drops, n_dropped)
-        sent = counts_kept.view(rt.N, rt.E_local).sum(1).to(torch.int32)
+        sent = torch.empty(rt.N, device=dev, dtype=torch.int32)
+        _lib.call("capacity_plan", indices32, T, rt.E, K, rt.capacity, slot_pos, keep, counts_kept, drops, n_dropped, sent,
+                  rt.N, None if stats_mod is None else stats_mod._drop_stats(dev))
         e1 = rt.next_epoch()
         gu = torch.empty((rt.rows_total, 2 * H), device=dev, dtype=torch.bfloat16)
         if rt.fp8:
@@ -423,7 +423,6 @@ class _FusedMoE(torch.autograd.Function):
         ctx.x_shape = x.shape
         if stats_mod is not None:
             stats_mod._per_expert_drop_counts = drops
-            stats_mod._record_drops(n_dropped[0].long(), T, dev)
         return out.view(x.shape)
 
     @staticmethod
@@ -507,7 +506,7 @@ def fused_moe_forward(mod, x: torch.Tensor) -> torch.Tensor:
     xr = x
     if cfg.jitter_eps is not None and mod.training:   # routing noise, as in MoERouter.forward
         xr = x + torch.randn_like(x) * cfg.jitter_eps
-    w, idx, aux, counts = route(xr, mod.router)
+    w, idx, aux, counts = route(xr, mod.router, int64=False)
     mod.router.last_counts = counts
     layer = rt.layer_index(mod)
     if mod.router.score_bias is not None:
@@ -518,5 +517,5 @@ def fused_moe_forward(mod, x: torch.Tensor) -> torch.Tensor:
     mod._aux_loss = aux
     shared = mod.shared_expert(x) if mod.shared_expert is not None else None
     with _lib.nvtx_range("fused_moe"):
-        return _FusedMoE.apply(x, w.reshape(B * S, -1), idx.reshape(B * S, -1).to(torch.int32), mod.w1, mod.w3,
-                               mod.w2, rt, layer, mod, shared)
+        return _FusedMoE.apply(x, w.reshape(B * S, -1), idx.reshape(B * S, -1), mod.w1, mod.w3, mod.w2, rt, layer, mod,
+                               shared)

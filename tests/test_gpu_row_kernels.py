@@ -72,3 +72,42 @@ def test_qkv_rope_shapes(B, S, hq, hkv, hd, rot):
     torch.autograd.backward([r[:, :, :hq], r[:, :, hq:hq + hkv], h[:, :, hq + hkv:]], [gq.double(), gk.double(), gv.double()])
     assert rel(qkv.grad, x.grad) < 4e-3
     assert apply_rope_ref(q, cos, sin, 5).shape == q.shape
+
+
+# below and above the four-tokens-per-warp switch, T off it, experts off a block of eight, D off a warp's 256
+@pytest.mark.parametrize("T,D,E,K", [(5, 64, 4, 2), (2367, 256, 8, 2), (2371, 768, 8, 2), (4099, 2048, 12, 3)])
+def test_router_forward_in_one_piece(T, D, E, K):
+    from nanopysche_b200.models.moe import MoERouter, MoERouterConfig
+    from nanopysche_b200.ops.moe import route
+
+    torch.manual_seed(T)
+    router = MoERouter(d_model=D, config=MoERouterConfig(num_experts=E, top_k=K, z_loss_multiplier=1e-2), device="cuda")
+    x = torch.randn(T, D, device="cuda").bfloat16()
+    w, idx, aux, counts = route(x, router)
+    logits = x.double() @ router.gate.weight.double().t() + router.gate.bias.double()
+    top, i64 = logits.topk(K, -1)
+    assert (idx == i64).all(-1).float().mean() > 0.999           # a last-bit tie may go the other way
+    same = (idx == i64).all(-1)
+    assert rel(w[same], top.softmax(-1)[same]) < 1e-5
+    f = torch.bincount(idx.reshape(-1), minlength=E).double() / T
+    assert torch.equal(counts.long(), torch.bincount(idx.reshape(-1), minlength=E))
+    ref = E * (f * logits.softmax(-1).mean(0)).sum() + 1e-2 * logits.logsumexp(-1).square().mean()
+    assert abs(aux.item() - ref.item()) < 1e-5 * abs(ref.item())
+
+
+@pytest.mark.parametrize("T,cap,ranks", [(1, -1, 1), (700, 150, 2), (4096, 1280, 4)])
+def test_capacity_plan_matches_the_scan(T, cap, ranks):
+    from nanopysche_b200.ops import _lib
+
+    E, K = 8, 2
+    torch.manual_seed(T)
+    idx = torch.rand(T, E, device="cuda").topk(K, -1).indices.to(torch.int32)
+    a, b = ([torch.full(s, -7, device="cuda", dtype=torch.int32) for s in ((T, K), (T,), (E,), (E,), (1,))] for _ in range(2))
+    _lib.call("capacity_scan", idx, T, E, K, cap, *a)
+    sent = torch.empty(ranks, device="cuda", dtype=torch.int32)
+    stats = torch.tensor([9, 100, 1000], device="cuda")
+    _lib.call("capacity_plan", idx, T, E, K, cap, *b, sent, ranks, stats)
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+    assert torch.equal(sent, a[2].view(ranks, -1).sum(1).to(torch.int32))
+    d = a[4].item()
+    assert stats.tolist() == [d, 100 + d, 1000 + T]
