@@ -33,7 +33,7 @@ struct GemmParams {
   int a_mn, b_mn;     // 0: operand is K-major ([rows, K]); 1: MN-major ([K, rows])
   int out_f32;        // 0: bf16 output, 1: fp32 output
   int accumulate;     // C += A*B (read-modify-write)
-  int epilogue;       // 0 plain, 1 swiglu (B tile = 128 gate rows + 128 up rows)
+  int epilogue;       // 0 plain, 1 swiglu (B tile = 128 gate rows + 128 up rows), 2 backward of swiglu (tmC2: [gate | up])
   int mode;           // 0 dense, 1 grouped rows (per-M-block B offset), 2 grouped K (wgrad)
   float alpha;
   const int* mblk_group;      // [m blocks] group of each 128-row block (mode 1) or nullptr
@@ -322,6 +322,70 @@ __device__ __forceinline__ void stage_store(const CUtensorMap* tm, uint32_t stg,
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
 }
+// Backward of h = silu(gate) * up, 32 columns of dh at a time: the pre-activations of the same rows and columns arrive by TMA
+// in the warp's staging buffer (gate box, up box: 32 rows of 64 bytes each, 64-byte swizzle), d(gate) and d(up) are written
+// over them and leave the same way. dh itself never reaches memory: as a pass of its own this was 46 us of a 720 us
+// feed-forward (4096 tokens, 2048 x 5632), 92 MB of it dh written and read.
+struct GluBar {   // of one epilogue warp, over all its tiles
+  uint32_t bar, phase;
+};
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+template <int BN>
+__device__ __forceinline__ void store_glu_bwd(const GemmParams& p, const CUtensorMap* tmD, const CUtensorMap* tmGU, uint32_t stg,
+                                              GluBar& gb, volatile int* abort_flag, uint32_t taddr, int row0, int lane, int n0,
+                                              int half) {
+  if (row0 >= p.M) return;
+#pragma unroll 1
+  for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+    const int col = n0 + c * 32;
+    if (col >= p.N) break;
+    if (lane == 0) {
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the last boxes have left
+      np::mbar_expect_tx(gb.bar, 4096);
+      tma_load_3d(stg, tmGU, gb.bar, col, row0, 0);
+      tma_load_3d(stg + 2048, tmGU, gb.bar, col, row0, 1);
+    }
+    __syncwarp();
+    uint32_t r[32];
+    np::tmem_ld32(taddr + c * 32, r);
+    np::tmem_ld_wait();
+    if (!np::mbar_wait_warp(gb.bar, gb.phase, abort_flag, KID_GEMM, 16)) return;
+    gb.phase ^= 1u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {   // 8 columns: 16 bytes of gate and of up
+      const uint32_t at = stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4);
+      uint32_t g[4], u[4], dg[4], du[4];
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(g[0]), "=r"(g[1]), "=r"(g[2]), "=r"(g[3]) : "r"(at) : "memory");
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(at + 2048) : "memory");
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 gf = np::unpack_bf16(g[q]), uf = np::unpack_bf16(u[q]);
+        const float d0 = __uint_as_float(r[8 * j + 2 * q]) * p.alpha, d1 = __uint_as_float(r[8 * j + 2 * q + 1]) * p.alpha;
+        const float s0 = 1.f / (1.f + __expf(-gf.x)), s1 = 1.f / (1.f + __expf(-gf.y));
+        dg[q] = np::pack_bf16(d0 * uf.x * (s0 * (1.f + gf.x * (1.f - s0))), d1 * uf.y * (s1 * (1.f + gf.y * (1.f - s1))));
+        du[q] = np::pack_bf16(d0 * (gf.x * s0), d1 * (gf.y * s1));
+      }
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(dg[0]), "r"(dg[1]), "r"(dg[2]), "r"(dg[3]) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 2048), "r"(du[0]), "r"(du[1]), "r"(du[2]), "r"(du[3]) : "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (int z = 0; z < 2; ++z)
+        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmD),
+                     "r"(stg + z * 2048), "r"(col), "r"(row0), "r"(z)
+                     : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+}
+
 // Before the CTA exits: the staging buffer has been read.
 __device__ __forceinline__ void stage_drain(int lane) {
   if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -453,7 +517,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
-  uint8_t* tail = smem_raw + (bar_base - np::smem_u32(smem_raw)) + 8 * (2 * STAGES + 4);
+  uint8_t* tail = smem_raw + (bar_base - np::smem_u32(smem_raw)) + 8 * (2 * STAGES + 4 + EPI_WARPS);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
 
@@ -476,6 +540,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       np::mbar_init(tfull_bar(a), 1);
       np::mbar_init(tempty_bar(a), EPI_WARPS);
     }
+    for (int w = 0; w < EPI_WARPS; ++w) np::mbar_init(bar_base + 8u * (2 * STAGES + 4 + w), 1);
     *abort_flag = 0;
     np::mbar_fence_init();
   }
@@ -644,6 +709,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------------------------------------ epilogue
     const int quarter = warp & 3, half = (warp - 2) >> 2;  // TMEM lanes [32*quarter, 32*quarter+32), column half
+    GluBar gb{bar_base + 8u * (2 * STAGES + 4 + warp - 2), 0u};
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
@@ -658,9 +724,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 4)) break;
         np::tc_fence_after();
       }
-      store_tile<BN>(p, &tmC, &tmC2, stg_base + (warp - 2) * STG_BYTES,
-                     tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g, tl.m_blk * BM + quarter * 32,
-                     lane, n0, half, have_acc);
+      const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
+      const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
+      const int row0 = tl.m_blk * BM + quarter * 32;
+      if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+      else store_tile<BN>(p, &tmC, &tmC2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
@@ -774,7 +842,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
-  uint8_t* tail = smem_raw + (bar_base - np::smem_u32(smem_raw)) + 8 * (2 * STAGES + 4);
+  uint8_t* tail = smem_raw + (bar_base - np::smem_u32(smem_raw)) + 8 * (2 * STAGES + 4 + EPI_WARPS);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
 
@@ -807,6 +875,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       np::mbar_init(tfull_bar(a), 1);
       np::mbar_init(tempty_bar(a), 2 * EPI_WARPS);
     }
+    for (int w = 0; w < EPI_WARPS; ++w) np::mbar_init(bar_base + 8u * (2 * STAGES + 4 + w), 1);
     *abort_flag = 0;
     np::mbar_fence_init();
   }
@@ -936,6 +1005,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int quarter = warp & 3, half = (warp - 2) >> 2;
+    GluBar gb{bar_base + 8u * (2 * STAGES + 4 + warp - 2), 0u};
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
@@ -950,10 +1020,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         np::tc_fence_after();
       }
       if constexpr (SPLIT) { done = true; break; }   // one tile per cluster, finished below
-      if (mine)
-        store_tile<BN>(p, &tmC, &tmC2, stg_base + (warp - 2) * STG_BYTES,
-                       tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16), tl.g,
-                       tl.m_blk * TM + rank * BM + quarter * 32, lane, tl.n_blk * bn_out, half, have_acc);
+      if (mine) {
+        const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
+        const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
+        const int row0 = tl.m_blk * TM + rank * BM + quarter * 32, n0 = tl.n_blk * bn_out;
+        if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+        else store_tile<BN>(p, &tmC, &tmC2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
+      }
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
@@ -1090,6 +1163,7 @@ struct NpGemmArgs {
   long long lda, ldb, ldc, ldc2;
   long long a_rows, b_rows;  // total rows (K-major) or total K rows (MN-major) of the A / B tensors
   int M, N, K;
+  // epilogue 2: C is [d gate | d up] and C2 the pre-activations [gate | up], each [M, 2 N]; the product is d h
   int a_mn, b_mn, out_f32, accumulate, epilogue, mode;
   float alpha;
   const int* mblk_group; const int* mblk_rows; long long group_stride_b;
@@ -1133,16 +1207,17 @@ static int num_sms() {
 
 // Output [planes][rows, cols] written in boxes of 32 rows x 128 bytes (128-byte swizzle)
 static int make_tmap_out(CUtensorMap* out, const void* base, int f32, long long cols, long long rows, long long planes,
-                         long long ld, long long plane_stride) {
+                         long long ld, long long plane_stride, int box_bytes = 128) {
   NpEncodeTiledFn enc = np_get_encode_tiled();
   if (!enc) return -1;
   const int es = f32 ? 4 : 2;
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)planes};
   cuuint64_t strides[2] = {(cuuint64_t)(ld * es), (cuuint64_t)(plane_stride * es)};
-  cuuint32_t box[3] = {(cuuint32_t)(128 / es), 32, 1};
+  cuuint32_t box[3] = {(cuuint32_t)(box_bytes / es), 32, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base),
-                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
@@ -1213,13 +1288,17 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   // other alignments store from registers. The SwiGLU form needs both of its outputs aligned.
   const int es = a.out_f32 ? 4 : 2;
   const long long groups = a.mode == 2 ? a.num_groups : 1;
-  p.tma_c = !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue == 0 || BN == 256) && ((uintptr_t)a.C & 15) == 0 &&
+  p.tma_c = !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue != 1 || BN == 256) && ((uintptr_t)a.C & 15) == 0 &&
             (a.ldc * es) % 16 == 0 && (groups <= 1 || (a.group_stride_c * es) % 16 == 0) &&
-            (a.epilogue == 0 || !a.C2 || (((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0)) &&
+            (a.epilogue != 1 || !a.C2 || (((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0)) &&
             (a.m_split == 0 || ((uintptr_t)a.C2 & 15) == 0);
   tmC = tmA;
   tmC2 = tmA;
-  if (p.tma_c) {
+  if (a.epilogue == 2) {   // [d gate | d up] out, [gate | up] in: two planes of N columns each
+    rc = make_tmap_out(&tmC, a.C, 0, a.N, a.M, 2, a.ldc, a.N, 64);
+    if (!rc) rc = make_tmap_out(&tmC2, a.C2, 0, a.N, a.M, 2, a.ldc2, a.N, 64);
+    if (rc) return 900 + rc;
+  } else if (p.tma_c) {
     const long long gs = groups > 1 ? a.group_stride_c : a.ldc;
     rc = make_tmap_out(&tmC, a.C, a.out_f32, a.N, a.m_split > 0 ? a.m_split : a.M, groups, a.ldc, gs);
     if (!rc && a.m_split > 0) rc = make_tmap_out(&tmC2, a.C2, a.out_f32, a.N, a.M - a.m_split, groups, a.ldc, gs);
@@ -1281,6 +1360,9 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
   }
   if (a.k_split < 0 || a.m_split < 0 || (a.k_split > 0 && (!a.b_mn || a.mode == 2 || a.epilogue != 0 || a.k_split % BK)) ||
       (a.m_split > 0 && (a.row_dst || a.epilogue != 0 || a.m_split % 256 || a.m_split >= a.M || (a.Cin && a.Cin != a.C))))
+    return 1;
+  if (a.epilogue == 2 && (a.mode == 2 || a.out_f32 || a.accumulate || a.Cin || a.row_dst || a.done_counters || !a.C2 || a.N % 8 ||
+                          a.ldc % 8 || a.ldc2 % 8 || (((uintptr_t)a.C | (uintptr_t)a.C2) & 15)))
     return 1;
   if ((a.lda % 8) || (a.ldb % 8) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15)) return 1;
   const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&

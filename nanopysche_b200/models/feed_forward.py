@@ -57,15 +57,14 @@ class FeedForward(nn.Module):
         x = copy_to_tp_region(x, self._tp_group, self._tp_size)
         fused = self._fused_w13
         if fused is not None and _lib.on(x) and x.dtype == fused.dtype and self.w1.bias is None:
-            h = gemm_ops.linear_glu(x, fused, act)
+            out = gemm_ops.feed_forward_glu(x, fused, self.w2.weight, act)
         elif _lib.on(x) and x.dtype == torch.bfloat16 and self.w1.bias is None:
             gu = torch.cat([gemm_ops.linear(x, self.w1.weight), gemm_ops.linear(x, self.w3.weight)], dim=-1)
-            h = act_ops.glu(gu, act)
+            out = gemm_ops.linear(act_ops.glu(gu, act), self.w2.weight, None)
         else:
             g = gemm_ops.linear(x, self.w1.weight, self.w1.bias)
             a = F.silu(g) if act == "silu" else F.gelu(g, approximate="tanh")
-            h = a * gemm_ops.linear(x, self.w3.weight, self.w3.bias)
-        out = gemm_ops.linear(h, self.w2.weight, None)
+            out = gemm_ops.linear(a * gemm_ops.linear(x, self.w3.weight, self.w3.bias), self.w2.weight, None)
         out = differentiable_all_reduce(out, self._tp_group, self._tp_size)
         if self.w2.bias is not None:
             out = out + self.w2.bias

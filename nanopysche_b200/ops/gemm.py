@@ -121,6 +121,26 @@ def gemm_swiglu(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, sa
     return h, gu
 
 
+def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor) -> torch.Tensor:
+    """``[d gate | d up]`` of ``h = silu(gate) * up`` for ``dh = dy @ w2`` and ``gu = [gate | up]``, without forming ``dh``:
+    the gradient of the activation is the epilogue of the GEMM (``dy [M, D]``, ``w2 [D, F]``, ``gu [M, 2F]``)."""
+    M, F = dy.shape[0], w2.shape[1]
+    if not _use_kernel(dy):
+        from .activation import glu_bwd
+
+        return glu_bwd(gu, gemm_ref(dy, w2, b_mn=True))
+    assert dy.shape[1] == w2.shape[0] and gu.shape == (M, 2 * F) and gu.stride(1) == 1
+    out = torch.empty((M, 2 * F), device=dy.device, dtype=torch.bfloat16)
+    args = _lib.GemmArgs()
+    args.A, args.B, args.C, args.C2 = dy.data_ptr(), w2.data_ptr(), out.data_ptr(), gu.data_ptr()
+    args.lda, args.ldb, args.ldc, args.ldc2 = dy.stride(0), w2.stride(0), 2 * F, gu.stride(0)
+    args.a_rows, args.b_rows = M, w2.shape[0]
+    args.M, args.N, args.K = M, F, dy.shape[1]
+    args.b_mn, args.epilogue, args.alpha = 1, 2, 1.0
+    _lib.check(_lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream())), "gemm_glu_bwd")
+    return out
+
+
 # Zero-bubble pipeline schedules split a backward pass into B (input gradients, on the critical path between
 # stages) and W (weight gradients, moved into what would be bubbles). While ``_DEFER`` is a list, every weight-gradient
 # GEMM is queued there instead of run; ``run_deferred_wgrads`` executes a queue later. ``SPLIT_MODE`` makes ``linear``
@@ -256,40 +276,54 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -
     return torch.nn.functional.linear(x, w, bias)
 
 
-class _LinearSwiGLU(torch.autograd.Function):
-    """``silu(x @ w1.T) * (x @ w3.T)`` for a fused ``[w1; w3]`` weight: the activation in the epilogue of the gate|up
-    GEMM, which also stores the pre-activations when a backward pass will need them."""
+class _SwiGLUFeedForward(torch.autograd.Function):
+    """``(silu(x @ w1.T) * (x @ w3.T)) @ w2.T`` for a fused ``[w1; w3]`` weight: the activation in the epilogue of the
+    gate|up GEMM (which also stores the pre-activations when a backward pass will need them), its gradient in the epilogue
+    of the down projection's input-gradient GEMM."""
 
     @staticmethod
-    def forward(ctx, x, w13, save):
+    def forward(ctx, x, w13, w2, save):
         F = w13.shape[0] // 2
         x2 = x.reshape(-1, x.shape[-1])
         h, gu = gemm_swiglu(x2, w13[:F], w13[F:], save_gu=save)
-        ctx.save_for_backward(x, w13, gu)
-        return h.view(*x.shape[:-1], F)
+        if save:
+            ctx.save_for_backward(x, w13, w2, h, gu)
+        return gemm(h, w2).view(*x.shape[:-1], w2.shape[0])
 
     @staticmethod
-    def backward(ctx, dh):
-        from .activation import glu_bwd
-
-        x, w13, gu = ctx.saved_tensors
-        dgu = glu_bwd(gu, dh.reshape(-1, dh.shape[-1]))
+    def backward(ctx, dy):
+        x, w13, w2, h, gu = ctx.saved_tensors
+        dy2 = dy.reshape(-1, dy.shape[-1])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
         x2 = x.reshape(-1, x.shape[-1])
-        dx = gemm(dgu, w13, b_mn=True).view(x.shape) if ctx.needs_input_grad[0] else None
-        dw = _wgrad_into(w13, dgu, x2) if (ctx.needs_input_grad[1] or hasattr(w13, "main_grad")) else None
-        return dx, dw, None
+        dw2 = _wgrad_into(w2, dy2, h) if (ctx.needs_input_grad[2] or hasattr(w2, "main_grad")) else None
+        dx = dw13 = None
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or hasattr(w13, "main_grad"):
+            dgu = gemm_glu_bwd(dy2, w2, gu)
+            if ctx.needs_input_grad[0]:
+                dx = gemm(dgu, w13, b_mn=True).view(x.shape)
+            if ctx.needs_input_grad[1] or hasattr(w13, "main_grad"):
+                dw13 = _wgrad_into(w13, dgu, x2)
+        return dx, dw13, dw2, None
 
 
-def linear_glu(x: torch.Tensor, w13: torch.Tensor, act: str = "silu") -> torch.Tensor:
-    """``act(x @ w1.T) * (x @ w3.T)`` for a fused ``[w1; w3]`` weight. SwiGLU of more rows than the few-row kernel takes
-    runs in one GEMM (4096 x 5632 x 2048: the separate pass over ``[gate | up]`` took 34 us of the layer's 720); other
-    activations, fp8 or sharded weights take the GEMM and the GLU kernel."""
+def _plain_weight(w: torch.Tensor) -> bool:
+    """A bf16 weight that the GEMMs read in place: not row-sharded, not tagged for fp8, 16-byte aligned rows."""
+    return (w.dtype == torch.bfloat16 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and
+            w.data_ptr() % 16 == 0 and getattr(w, "_fsdp_rt", None) is None and getattr(w, "_fp8_recipe", None) is None)
+
+
+def feed_forward_glu(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, act: str = "silu") -> torch.Tensor:
+    """``(act(x @ w1.T) * (x @ w3.T)) @ w2.T`` for a fused ``[w1; w3]`` weight. SwiGLU of more rows than the few-row kernel
+    takes runs with the activation and its gradient inside the GEMMs (4096 tokens, 2048 x 5632: the separate passes took 34
+    and 46 us of the layer's 753); other activations, fp8 or sharded weights take GEMMs and the GLU kernels."""
     from .activation import glu
 
-    if (act == "silu" and not SPLIT_MODE and _lib.on(x) and x.dtype == torch.bfloat16 and w13.dtype == torch.bfloat16 and
-            x.numel() > 64 * x.shape[-1] and w13.shape[0] % 16 == 0 and w13.stride(1) == 1 and w13.stride(0) % 8 == 0 and
-            x.shape[-1] % 8 == 0 and w13.data_ptr() % 16 == 0 and
-            getattr(w13, "_fsdp_rt", None) is None and getattr(w13, "_fp8_recipe", None) is None):
-        x2 = x if x.is_contiguous() else x.contiguous()
-        return _LinearSwiGLU.apply(x2, w13, torch.is_grad_enabled() and (x2.requires_grad or w13.requires_grad))
-    return glu(linear(x, w13), act)
+    if (act == "silu" and not SPLIT_MODE and _lib.on(x) and x.dtype == torch.bfloat16 and x.numel() > 64 * x.shape[-1] and
+            w13.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and w2.shape[0] % 8 == 0 and _plain_weight(w13) and
+            _plain_weight(w2)):
+        x2 = x if x.is_contiguous() and x.data_ptr() % 16 == 0 else x.clone(memory_format=torch.contiguous_format)
+        save = torch.is_grad_enabled() and (x2.requires_grad or w13.requires_grad or w2.requires_grad)
+        return _SwiGLUFeedForward.apply(x2, w13, w2, save)
+    return linear(glu(linear(x, w13), act), w2)

@@ -25,7 +25,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .activation import glu, glu_bwd
+from .activation import glu
 
 GATING_IDS = {"softmax": 0, "sigmoid": 1}
 WAIT_LIMIT_NS = int(os.environ.get("NPB200_WAIT_LIMIT_MS", "10000")) * 1_000_000
@@ -275,11 +275,15 @@ class FusedMoERuntime:
         _lib.check(_lib.lib().np_ep_combine(C.byref(a), C.c_void_p(_lib.stream())), "ep_combine")
 
     def grouped_gemm(self, A, B, *, N, K, b_mn, group_stride_b, out=None, B2=None, C2=None, wait_epoch=0,
-                     push_ptrs=None, push_epoch=0, out_dtype=torch.bfloat16, k_split=0):
+                     push_ptrs=None, push_epoch=0, out_dtype=torch.bfloat16, k_split=0, glu_of=None):
         """Row-grouped GEMM over the receive-buffer layout (mode 1). ``B2``: the up weight of the SwiGLU form, or with
-        ``k_split`` the weight that the contraction continues with from there on."""
+        ``k_split`` the weight that the contraction continues with from there on. ``glu_of``: pre-activations ``[gate | up]``;
+        the product is the gradient of ``silu(gate) * up`` and ``[d gate | d up]`` is what is returned."""
         g = _lib.GemmArgs()
         M = self.rows_total
+        if glu_of is not None:
+            out = torch.empty_like(glu_of)
+            g.epilogue, g.C2, g.ldc2 = 2, glu_of.data_ptr(), glu_of.stride(0)
         if out is None and push_ptrs is None:
             out = torch.empty((M, N), device=A.device, dtype=out_dtype)
         g.A, g.B = A.data_ptr(), B.data_ptr()
@@ -439,13 +443,11 @@ class _FusedMoE(torch.autograd.Function):
         # send w[t,k] * dout[t] to the experts (same slots as forward)
         e2 = rt.next_epoch()
         rt.dispatch(do2, indices32, slot_pos, counts_kept, weights, rt.p_recv_g, e2)
-        # dH = dY @ w2^T  (w2 [H, D] per expert is K-major for this contraction)
-        dh = rt.grouped_gemm(rt.recv_g, w2, N=H, K=D, b_mn=False, group_stride_b=H, wait_epoch=e2)
+        # dH = dY @ w2^T  (w2 [H, D] per expert is K-major for this contraction), taken to [dG | dU] in the epilogue
+        dgu = rt.grouped_gemm(rt.recv_g, w2, N=H, K=D, b_mn=False, group_stride_b=H, wait_epoch=e2, glu_of=gu)
         hh = ctx.saved_tensors[10] if ctx.has_h else glu(gu)
         dw2 = rt.grouped_wgrad(hh, rt.recv_g, w2, M=H, N=D)
         del hh
-        dgu = glu_bwd(gu, dh)
-        del dh
         if rt.fp8:  # the rows arrived as e4m3: dequantise once for the (bf16) weight-gradient GEMMs
             from .gemm_mxfp8 import mx_dequantize_bf16
 

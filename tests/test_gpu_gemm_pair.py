@@ -68,3 +68,79 @@ def test_chosen_kernel_agrees_with_the_one_cta_tile(M, N, K):
     torch.manual_seed(N)
     a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
     assert rel(gemm(a, b, out_dtype=torch.float32), gemm(a, b, out_dtype=torch.float32, bn=128)) < 1e-6 * K ** 0.5
+
+
+@pytest.mark.parametrize("M,F,D", [(256, 256, 64), (130, 264, 200), (1000, 712, 512), (4096, 768, 768)])
+@pytest.mark.parametrize("kw", [dict(bn=0), dict(bn=256, mt=1), dict(bn=256, mt=2), dict(bn=128)])
+def test_swiglu_backward_epilogue(M, F, D, kw):
+    """``dh = dy @ w2`` taken to ``[d gate | d up]`` inside the GEMM; bf16 results of fp32 values: 3e-3."""
+    import ctypes as C
+
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(F)
+    dy = torch.randn(M, D, device="cuda").bfloat16()
+    w2 = (torch.randn(D, F, device="cuda") * D ** -0.5).bfloat16()
+    gu = torch.randn(M, 2 * F, device="cuda").bfloat16()
+    out = torch.full((M, 2 * F), float("nan"), device="cuda", dtype=torch.bfloat16)
+    a = _lib.GemmArgs()
+    a.A, a.B, a.C, a.C2 = dy.data_ptr(), w2.data_ptr(), out.data_ptr(), gu.data_ptr()
+    a.lda, a.ldb, a.ldc, a.ldc2, a.a_rows, a.b_rows = D, F, 2 * F, 2 * F, M, D
+    a.M, a.N, a.K, a.b_mn, a.epilogue, a.alpha = M, F, D, 1, 2, 1.0
+    a.bn, a.mt = kw["bn"], kw.get("mt", 0)
+    assert _lib.lib().np_gemm_bf16(C.byref(a), C.c_void_p(_lib.stream())) == 0
+    g64 = gu.double().requires_grad_(True)
+    h = torch.nn.functional.silu(g64[:, :F]) * g64[:, F:]
+    h.backward(dy.double() @ w2.double())
+    assert rel(out, g64.grad) < 3e-3
+
+
+@pytest.mark.parametrize("M,N,H", [(256, 256, 64), (300, 264, 192), (1000, 520, 704)])
+@pytest.mark.parametrize("mt", [1, 2])
+def test_contraction_over_two_weights_and_rows_into_two_outputs(M, N, H, mt):
+    import ctypes as C
+
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(H)
+    a2 = torch.randn(M, 2 * H, device="cuda").bfloat16()
+    w1, w3 = (torch.randn(H, N, device="cuda").bfloat16() for _ in range(2))
+    out = torch.empty(M, N, device="cuda")
+    g = _lib.GemmArgs()
+    g.A, g.B, g.B2, g.C = a2.data_ptr(), w1.data_ptr(), w3.data_ptr(), out.data_ptr()
+    g.lda, g.ldb, g.ldc, g.a_rows, g.b_rows = 2 * H, N, N, M, H
+    g.M, g.N, g.K, g.b_mn, g.out_f32, g.alpha, g.k_split, g.bn, g.mt = M, N, 2 * H, 1, 1, 1.0, H, 256, mt
+    assert _lib.lib().np_gemm_bf16(C.byref(g), C.c_void_p(_lib.stream())) == 0
+    assert rel(out, a2[:, :H].double() @ w1.double() + a2[:, H:].double() @ w3.double()) < 2e-5
+
+    K, rows = M, 256                                # two outputs of 256 rows each from one transposed operand
+    x = torch.randn(K, N, device="cuda").bfloat16()
+    two = torch.randn(K, 2 * rows, device="cuda").bfloat16()
+    for acc in (0, 1):
+        o1, o2 = torch.ones(rows, N, device="cuda"), torch.ones(rows, N, device="cuda")
+        g = _lib.GemmArgs()
+        g.A, g.B, g.C, g.C2 = two.data_ptr(), x.data_ptr(), o1.data_ptr(), o2.data_ptr()
+        g.lda, g.ldb, g.ldc, g.a_rows, g.b_rows = 2 * rows, N, N, K, K
+        g.M, g.N, g.K, g.a_mn, g.b_mn, g.out_f32, g.alpha = 2 * rows, N, K, 1, 1, 1, 1.0
+        g.accumulate, g.m_split, g.bn, g.mt = acc, rows, 256, mt
+        assert _lib.lib().np_gemm_bf16(C.byref(g), C.c_void_p(_lib.stream())) == 0
+        ref = two.double().t() @ x.double() + acc
+        assert rel(o1, ref[:rows]) < 2e-5 and rel(o2, ref[rows:]) < 2e-5
+
+
+def test_feed_forward_without_gradients_and_of_frozen_weights():
+    from nanopysche_b200.ops.gemm import feed_forward_glu
+
+    torch.manual_seed(2)
+    x = torch.randn(2, 70, 128, device="cuda").bfloat16()
+    w13, w2 = (torch.randn(512, 128, device="cuda") * 0.1).bfloat16(), (torch.randn(128, 256, device="cuda") * 0.1).bfloat16()
+    with torch.no_grad():
+        y = feed_forward_glu(x, w13, w2)
+    xa = x.clone().requires_grad_(True)
+    ya = feed_forward_glu(xa, w13, w2)
+    ya.sum().backward()
+    x64 = x.double().requires_grad_(True)
+    gu = x64 @ w13.double().t()
+    y64 = (torch.nn.functional.silu(gu[..., :256]) * gu[..., 256:]) @ w2.double().t()
+    y64.sum().backward()
+    assert torch.equal(y, ya) and rel(y, y64) < 6e-3 and rel(xa.grad, x64.grad) < 1e-2
