@@ -320,7 +320,26 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   __nv_bfloat162 h = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(h);
 }
-__device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
+// 1 / (1 + exp(-x)) and x / (1 + exp(-x)): the hardware's reciprocal estimate and one Newton step on the reciprocal or the
+// quotient, without a branch. An IEEE division branches to a slow path, which keeps the elements of a thread from overlapping:
+// with it the SwiGLU epilogue of a tile took longer than the tile's 16 K steps at K = 1024 (2048 tokens, 1024 x 5632: forward
+// 34 -> 25 us, backward 42 -> 29; 4096 tokens, 2048 x 11264: 164 -> 140 and 109 -> 90). t is a quarter of the denominator, so
+// that its reciprocal is a normal number up to the largest one. Where the residual is not a number (an infinite denominator
+// or x) the estimate stands. Mean relative error against 64 bits over |x| < 80: 2.455e-7 and 2.46e-7, as with the division.
+__device__ __forceinline__ float sigmoid_f(float x) {
+  const float t = fmaf(__expf(-x), 0.25f, 0.25f);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
+  const float e = fmaf(-t, r, 1.f);
+  return 0.25f * (e == e ? fmaf(r, e, r) : r);
+}
+__device__ __forceinline__ float silu_f(float x) {
+  const float t = fmaf(__expf(-x), 0.25f, 0.25f), q = 0.25f * x;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
+  const float h = q * r, e = fmaf(-t, h, q);
+  return e == e ? fmaf(r, e, h) : h;
+}
 
 }  // namespace np
 

@@ -456,7 +456,7 @@ __global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_
     for (int j = 0; j < 8; ++j) {
       float a, da;
       if (act == 0) {
-        const float s = 1.f / (1.f + __expf(-g[j]));
+        const float s = np::sigmoid_f(g[j]);
         a = g[j] * s;
         da = s * (1.f + g[j] * (1.f - s));
       } else {

@@ -366,7 +366,7 @@ __device__ __forceinline__ void store_glu_bwd(const GemmParams& p, const CUtenso
       for (int q = 0; q < 4; ++q) {
         const float2 gf = np::unpack_bf16(g[q]), uf = np::unpack_bf16(u[q]);
         const float d0 = __uint_as_float(r[8 * j + 2 * q]) * p.alpha, d1 = __uint_as_float(r[8 * j + 2 * q + 1]) * p.alpha;
-        const float s0 = 1.f / (1.f + __expf(-gf.x)), s1 = 1.f / (1.f + __expf(-gf.y));
+        const float s0 = np::sigmoid_f(gf.x), s1 = np::sigmoid_f(gf.y);
         dg[q] = np::pack_bf16(d0 * uf.x * (s0 * (1.f + gf.x * (1.f - s0))), d1 * uf.y * (s1 * (1.f + gf.y * (1.f - s1))));
         du[q] = np::pack_bf16(d0 * (gf.x * s0), d1 * (gf.y * s1));
       }

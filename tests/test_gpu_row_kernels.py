@@ -111,3 +111,37 @@ def test_capacity_plan_matches_the_scan(T, cap, ranks):
     assert torch.equal(sent, a[2].view(ranks, -1).sum(1).to(torch.int32))
     d = a[4].item()
     assert stats.tolist() == [d, 100 + d, 1000 + T]
+
+
+# the ends of the exponent: sigmoid at subnormal numbers, at zero, one and infinity; each of the two reciprocal forms
+def test_swiglu_at_the_ends_of_the_range():
+    from nanopysche_b200.ops.activation import glu
+    from nanopysche_b200.ops.gemm import gemm_glu_bwd, gemm_swiglu
+
+    edge = torch.tensor([-3e38, -1e4, -100., -88.5, -88., -80., -20., -1., -0., 0., 1., 20., 88., 1e4, 3e38, -float("inf"),
+                         float("inf"), float("nan")] + [0.5] * 6, device="cuda").bfloat16()
+    F = edge.numel()
+    gu = torch.cat([edge, torch.full_like(edge, 0.75)])[None].contiguous()
+    h = glu(gu, "silu")
+    g64 = edge.double()[None].requires_grad_(True)
+    ref = torch.nn.functional.silu(g64) * 0.75
+    # one rounding to bf16; the fp32 exponential overflows from 88.7 on, where silu is below 1e-36
+    torch.testing.assert_close(h.double(), ref.detach(), rtol=2 ** -8, atol=1e-36, equal_nan=True)
+    finite = edge.isfinite()
+    x = gu.clone().requires_grad_(True)
+    glu(x, "silu").backward(torch.ones_like(h))
+    ref.sum().backward()
+    torch.testing.assert_close(x.grad[0, :F][finite].double(), g64.grad[0][finite], rtol=2 ** -7, atol=1e-34)
+    # the same pre-activations through the GEMM epilogues (identity weights keep them exactly)
+    M = 256
+    X = torch.zeros(M, F, device="cuda").bfloat16()
+    X[:, :] = torch.where(finite, edge, torch.zeros_like(edge))
+    eye = torch.eye(F, device="cuda").bfloat16()
+    hh, pre = gemm_swiglu(X, eye, eye)
+    x64 = X.double()
+    keep = x64.abs() < 1e18   # the square of the rest leaves the range
+    torch.testing.assert_close(hh.double()[keep], (torch.nn.functional.silu(x64) * x64)[keep], rtol=2 ** -7, atol=1e-34)
+    one = torch.ones(M, F, device="cuda").bfloat16()
+    d = gemm_glu_bwd(one, eye, torch.cat([X, 0.75 * one], 1).contiguous())
+    want = torch.where(finite, g64.grad[0], torch.full_like(g64.grad[0], 0.375))
+    torch.testing.assert_close(d[:, :F].double(), want.expand(M, F), rtol=2 ** -7, atol=1e-34)
