@@ -193,9 +193,9 @@ template <int NS>
 __device__ __forceinline__ void row_sync(int quarter) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(NS * 32) : "memory");
 }
-template <int NS>
-__device__ __forceinline__ void softmax_sync_all() {
-  asm volatile("bar.sync 5, %0;" ::"n"(NS * 128) : "memory");
+// Named barrier of the 128 threads that share a range of score columns (group hf)
+__device__ __forceinline__ void group_sync(int hf) {
+  asm volatile("bar.sync %0, 128;" ::"r"(5 + hf) : "memory");
 }
 // CW consecutive fp32 columns of this thread's lane into registers / CW/2 packed columns back
 template <int CW>
@@ -1022,8 +1022,21 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long
   if (w < n && lane == 0) delta[((size_t)b * H + h) * S + sq] = v;
 }
 
-enum { QB_QDO = 0, QB_K = 1, QB_KE = 4, QB_V = 7, QB_VE = 9, QB_S = 11, QB_DP = 13, QB_DS = 14, QB_FIN = 15, QB_COUNT = 16 };
+// P and dS of a thread group go back, as packed bf16, into the first half of the columns that the group itself reads, so that
+// the groups of a row need not wait for one another. Column of 16-wide K step kk in that layout:
+template <int NS>
+__device__ __forceinline__ constexpr int packed_col(int kk) {
+  constexpr int CW = 128 / NS;
+  return kk * 16 / CW * CW + kk * 16 % CW / 2;
+}
+
+enum { QB_QDO = 0, QB_K = 1, QB_KE = 4, QB_V = 7, QB_VE = 9, QB_S = 11, QB_SR = 12, QB_DP = 13, QB_DS = 15, QB_FIN = 17,
+       QB_COUNT = 18 };
 // K tiles live from S = Q K^T (issued one block ahead) to dQ += dS K: three of them; V tiles only feed dP: two.
+// S is free once it is in registers, so one buffer of it is enough and dP gets two: dP of the next block is formed while dS of
+// this one is, and the two thread groups of a row are held together by nothing but the products. With S in two buffers and dP in
+// one, every block waited for dS, dQ and dP one after the other (16 / 8 heads of 128, causal, 1 x 8192, with the
+// delta kernel: 0.385 -> 0.352 ms).
 constexpr int Q_KST = 3, Q_VST = 2;
 constexpr int BWD_TILES = 7;   // seven 32 KB tiles: the dynamic shared memory must itself start on a 1024-byte boundary
 
@@ -1055,7 +1068,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const BlockWalk walk0 = walk_kv(p.k_blk_pos, p.src_blocks, p.n_src, p.causal, q_pos0);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < QB_COUNT; ++i) np::mbar_init(B_(i), i == QB_DS ? 4 * NS : 1);
+    for (int i = 0; i < QB_COUNT; ++i) np::mbar_init(B_(i), (i == QB_SR || i == QB_DS || i == QB_DS + 1) ? 4 * NS : 1);
     *abort_flag = 0;
     np::mbar_fence_init();
   }
@@ -1068,7 +1081,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   np::tc_fence_after();
   const uint32_t tmem = *tmem_ptr_smem;
   np::pdl_begin();
-  const uint32_t tdP = tmem + 256, tdQ = tmem + 384;   // S buffers at columns 0 and 128
+  const uint32_t tS = tmem, tdP = tmem + 128, tdQ = tmem + 384;   // two dP buffers
   push_kv(p.push, reinterpret_cast<volatile int*>(tail + 12));
 
   if (warp == 0) {
@@ -1100,27 +1113,27 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    dKm = desc_mnmajor(sK0);
     bool ok = np::mbar_wait_warp(B_(QB_QDO), 0, abort_flag, KID_ATTN_DQ, 2);
     auto issue_s = [&](int i) {
-      const int st = i & 1, ks = i % Q_KST;
+      const int ks = i % Q_KST;
       if (!np::mbar_wait_warp(B_(QB_K + ks), (uint32_t)(i / Q_KST) & 1u, abort_flag, KID_ATTN_DQ, 3)) return false;
       np::tc_fence_after();
       if (np::elect_one()) {
         const uint64_t b = dK + (uint32_t)(ks * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tmem + st * 128, dQ + koff(kk), b + koff(kk), idesc_kk, kk > 0);
-        np::tc_commit(B_(QB_S + st));
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tS, dQ + koff(kk), b + koff(kk), idesc_kk, kk > 0);
+        np::tc_commit(B_(QB_S));
       }
       __syncwarp();
       return true;
     };
     auto issue_dp = [&](int i) {
-      const int vs = i % Q_VST;
+      const int vs = i % Q_VST, st = i & 1;
       if (!np::mbar_wait_warp(B_(QB_V + vs), (uint32_t)(i / Q_VST) & 1u, abort_flag, KID_ATTN_DQ, 4)) return false;
       np::tc_fence_after();
       if (np::elect_one()) {
         const uint64_t b = dV + (uint32_t)(vs * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tdP, ddO + koff(kk), b + koff(kk), idesc_kk, kk > 0);
-        np::tc_commit(B_(QB_DP));
+        for (int kk = 0; kk < HD / 16; ++kk) np::tc_mma_f16(tdP + st * 128, ddO + koff(kk), b + koff(kk), idesc_kk, kk > 0);
+        np::tc_commit(B_(QB_DP + st));
         np::tc_commit(B_(QB_VE + vs));
       }
       __syncwarp();
@@ -1129,20 +1142,25 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     BlockWalk w = walk0;
     if (ok && !w.done()) ok = issue_s(0) && issue_dp(0);
     for (int i = 0; !w.done() && ok; ++i) {
-      const int ks = i % Q_KST;
+      const int ks = i % Q_KST, st = i & 1;
       w.next();
-      if (!w.done()) ok = issue_s(i + 1);   // its buffer was read for block i-1 before dS of block i-1 arrived
-      ok = ok && np::mbar_wait_warp(B_(QB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 5);
+      if (!w.done()) {
+        ok = np::mbar_wait_warp(B_(QB_SR), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 6);   // S of block i is in registers
+        if (!ok) break;
+        np::tc_fence_after();
+        ok = issue_s(i + 1) && issue_dp(i + 1);   // overwrites dS of block i-1 after its dQ product
+      }
+      ok = ok && np::mbar_wait_warp(B_(QB_DS + st), (uint32_t)(i >> 1) & 1u, abort_flag, KID_ATTN_DQ, 5);
       if (!ok) break;
       np::tc_fence_after();
       if (np::elect_one()) {
         const uint64_t b = dKm + (uint32_t)(ks * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) tc_mma_f16_ts(tdQ, tdP + kk * 8, b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
+        for (int kk = 0; kk < 8; ++kk)
+          tc_mma_f16_ts(tdQ, tdP + st * 128 + packed_col<NS>(kk), b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
         np::tc_commit(B_(QB_KE + ks));
       }
       __syncwarp();
-      if (!w.done()) ok = issue_dp(i + 1);  // overwrites dS after the dQ product above has consumed it
     }
     if (np::elect_one()) np::tc_commit(B_(QB_FIN));
     __syncwarp();
@@ -1169,39 +1187,37 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int kp0 = w.at();
       const int valid_cols = p.src_len - jb * BKV;
       const bool need_mask = (p.causal && kp0 + BKV - 1 > q_pos0) || valid_cols < BKV;
-      ok = ok && !*abort_flag && warp_wait(B_(QB_S + st), (uint32_t)(i >> 1) & 1u, abort_flag, KID_ATTN_DQ, 7);
+      ok = ok && !*abort_flag && warp_wait(B_(QB_S), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 7);
+      if (!ok) continue;
       float pr[CW];
-      uint32_t t[CW];
-      if (ok) {
-        np::tc_fence_after();
-        tmem_ld_cols<CW>(tmem + st * 128 + lane_off + hf * CW, t);
+      uint32_t t[CW], pk[CW / 2];
+      np::tc_fence_after();
+      tmem_ld_cols<CW>(tS + lane_off + hf * CW, t);
+      np::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) np::mbar_arrive(B_(QB_SR));
 #pragma unroll
-        for (int e = 0; e < CW; ++e) pr[e] = ex2(fmaf(__uint_as_float(t[e]), p.scale_log2, -lse2));
-        if (need_mask) {
+      for (int e = 0; e < CW; ++e) pr[e] = ex2(fmaf(__uint_as_float(t[e]), p.scale_log2, -lse2));
+      if (need_mask) {
 #pragma unroll
-          for (int e = 0; e < CW; ++e) {
-            const int col = hf * CW + e;
-            if (col >= valid_cols || (p.causal && kp0 + col > q_pos)) pr[e] = 0.f;
-          }
+        for (int e = 0; e < CW; ++e) {
+          const int col = hf * CW + e;
+          if (col >= valid_cols || (p.causal && kp0 + col > q_pos)) pr[e] = 0.f;
         }
-        ok = warp_wait(B_(QB_DP), (uint32_t)i & 1u, abort_flag, KID_ATTN_DQ, 8);
       }
-      if (ok) {
-        np::tc_fence_after();
-        tmem_ld_cols<CW>(tdP + lane_off + hf * CW, t);
-      }
-      row_sync<NS>(quarter);   // both threads of the row hold their dP values: dS may now overwrite those columns
-      if (ok) {
-        uint32_t pk[CW / 2];
+      ok = warp_wait(B_(QB_DP + st), (uint32_t)(i >> 1) & 1u, abort_flag, KID_ATTN_DQ, 8);
+      if (!ok) continue;
+      np::tc_fence_after();
+      const uint32_t td = tdP + st * 128 + lane_off + hf * CW;
+      tmem_ld_cols<CW>(td, t);
 #pragma unroll
-        for (int e = 0; e < CW; e += 2)
-          pk[e >> 1] = np::pack_bf16(pr[e] * (__uint_as_float(t[e]) - dlt), pr[e + 1] * (__uint_as_float(t[e + 1]) - dlt));
-        tmem_st_cols<CW / 2>(tdP + lane_off + hf * (CW / 2), pk);
-        tmem_st_wait();
-        np::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) np::mbar_arrive(B_(QB_DS));
-      }
+      for (int e = 0; e < CW; e += 2)
+        pk[e >> 1] = np::pack_bf16(pr[e] * (__uint_as_float(t[e]) - dlt), pr[e + 1] * (__uint_as_float(t[e + 1]) - dlt));
+      tmem_st_cols<CW / 2>(td, pk);
+      tmem_st_wait();
+      np::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) np::mbar_arrive(B_(QB_DS + st));
     }
     ok = __all_sync(0xffffffffu, ok && !*abort_flag) && warp_wait(B_(QB_FIN), 0, abort_flag, KID_ATTN_DQ, 9);
     if (ok) {   // warp-uniform: the tensor-memory loads are executed by whole warps, only the stores are guarded
@@ -1235,16 +1251,22 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 enum { KB_KV = 0, KB_Q = 1, KB_QE = 4, KB_DO = 7, KB_DOE = 9, KB_ST = 11, KB_DPT = 12, KB_P = 13, KB_DS = 14, KB_FIN = 15,
-       KB_COUNT = 16 };
-// Q tiles live from S^T = K Q^T (issued one block ahead) to dK += dS^T Q: three of them; dO tiles are done after
-// dV += P^T dO: two.
-constexpr int K_QST = 3, K_DOST = 2;
+       KB_DPR = 16, KB_DSE = 17, KB_COUNT = 18 };
+// dS^T goes to dK += dS^T Q through shared memory, so that dP^T of the next block can be formed while this one's dS^T is: its
+// tile takes the place of a third Q tile at head dimension 128 (16 / 8 heads of 128, causal, 1 x 8192, with the
+// delta kernel: 0.525 -> 0.478 ms; with four threads per row it takes 15 % longer). Q tiles live from S^T = K Q^T (issued one block ahead) to the
+// dK product, dO tiles are done after dV += P^T dO.
+template <int HD>
+constexpr int k_qst() { return HD == 128 ? 2 : 3; }
+constexpr int K_DOST = 2, DS_BYTES = 128 * 128 * 2;
+template <int HD>
+constexpr int dkv_bytes() { return (2 + k_qst<HD>() + K_DOST) * tile_bytes<HD>() + DS_BYTES; }
 
 template <int NS, int HD>
 __global__ void __launch_bounds__(nthreads(NS), 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const __grid_constant__ TmapList tmQ, const __grid_constant__ TmapList tmdO, const BwdParams p) {
-  constexpr int TILE_BYTES = tile_bytes<HD>();
+  constexpr int TILE_BYTES = tile_bytes<HD>(), K_QST = k_qst<HD>();
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t base = np::smem_u32(smem_al);
   if (base & 1023u) {   // the swizzled tiles need it; nothing has been allocated or started yet
@@ -1252,9 +1274,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     return;
   }
   const uint32_t sK = base, sV = base + TILE_BYTES, sQ0 = sV + TILE_BYTES, sdO0 = sQ0 + K_QST * TILE_BYTES;
-  const uint32_t bar = sdO0 + K_DOST * TILE_BYTES;
+  const uint32_t sdS = sdO0 + K_DOST * TILE_BYTES, bar = sdS + DS_BYTES;
   auto B_ = [&](int i) { return bar + 8u * i; };
-  uint8_t* tail = smem_al + BWD_TILES * TILE_BYTES + 8 * KB_COUNT;
+  uint8_t* tail = smem_al + dkv_bytes<HD>() + 8 * KB_COUNT;
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
   float* s_lse = reinterpret_cast<float*>(tail + 16);          // [2][128]
@@ -1270,7 +1292,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
   const BlockWalk walk0 = walk_q(p.q_blk_pos, p.q_off, p.src_blocks, n_rep, p.n_src, p.causal, k_pos0);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < KB_COUNT; ++i) np::mbar_init(B_(i), (i == KB_P || i == KB_DS) ? 4 * NS : 1);
+    for (int i = 0; i < KB_COUNT; ++i) np::mbar_init(B_(i), (i == KB_P || i == KB_DS || i == KB_DPR) ? 4 * NS : 1);
     *abort_flag = 0;
     np::mbar_fence_init();
   }
@@ -1311,7 +1333,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     const uint32_t idesc_kk = np::make_idesc(128, 128, 1, 1, 0, 0);
     const uint32_t idesc_mn = np::make_idesc(128, HD, 1, 1, 0, 1);
     const uint64_t dK = desc_kmajor(sK), dV = desc_kmajor(sV), dQ = desc_kmajor(sQ0), ddO = desc_kmajor(sdO0),
-                   dQm = desc_mnmajor(sQ0), ddOm = desc_mnmajor(sdO0);
+                   dQm = desc_mnmajor(sQ0), ddOm = desc_mnmajor(sdO0), ddS = desc_kmajor(sdS);
     bool ok = np::mbar_wait_warp(B_(KB_KV), 0, abort_flag, KID_ATTN_DKV, 3);
     auto issue_st = [&](int i) {
       const int qs = i % K_QST;
@@ -1351,11 +1373,17 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         const uint64_t b = ddOm + (uint32_t)(ds * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // dV += P^T dO
-          tc_mma_f16_ts(tdV, tSt + kk * 8, b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
+          tc_mma_f16_ts(tdV, tSt + packed_col<NS>(kk), b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
         np::tc_commit(B_(KB_DOE + ds));
       }
       __syncwarp();
-      if (!w.done()) ok = issue_st(i + 1);        // overwrites P^T after the product above consumed it
+      if (!w.done()) {
+        ok = issue_st(i + 1);        // overwrites P^T after the product above consumed it
+        ok = ok && np::mbar_wait_warp(B_(KB_DPR), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 11);   // dP^T is in registers
+        if (!ok) break;
+        np::tc_fence_after();
+        ok = issue_dpt(i + 1);
+      }
       ok = ok && np::mbar_wait_warp(B_(KB_DS), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 7);
       if (!ok) break;
       np::tc_fence_after();
@@ -1363,11 +1391,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         const uint64_t b = dQm + (uint32_t)(qs * (TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // dK += dS^T Q
-          tc_mma_f16_ts(tdK, tdPt + kk * 8, b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
+          np::tc_mma_f16(tdK, ddS + koff(kk), b + mnoff(kk), idesc_mn, (i > 0) || (kk > 0));
         np::tc_commit(B_(KB_QE + qs));
+        np::tc_commit(B_(KB_DSE));
       }
       __syncwarp();
-      if (!w.done()) ok = issue_dpt(i + 1);       // overwrites dS^T after the product above consumed it
     }
     if (np::elect_one()) np::tc_commit(B_(KB_FIN));
     __syncwarp();
@@ -1375,26 +1403,27 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     constexpr int CW = 128 / NS, OW = HD / NS;              // score columns / output columns of a thread
     const int quarter = warp & 3, hf = (warp - 2) >> 2;   // this thread: KV row r, Q columns [CW hf, CW hf + CW)
     const int r = quarter * 32 + lane;
-    const int t256 = threadIdx.x - 64;                    // index among the softmax threads
+    const int tg = threadIdx.x - 64 - hf * 128;           // index among the threads of these columns
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const int k_pos = k_pos0 + r;
     bool ok = true;
     int nvis = 0, last_src = -1;
-    // Log-sum-exp (threads 0-127) and delta (threads 128-255) of a Q block, one column per thread, loaded one block ahead so
-    // that the load does not stand in front of the iteration
+    // Log-sum-exp (threads 0 to CW - 1 of a group) and delta (the CW after them) of a Q block's columns of the group, loaded one
+    // block ahead so that the load does not stand in front of the iteration
     auto load_stat = [&](const BlockWalk& w) -> float {
       if (w.src != last_src) {   // it has to be complete
         if (ok && !src_ready(p.fl, w.src, KID_ATTN_DKV)) { *abort_flag = 1; ok = false; }
         last_src = w.src;
       }
-      const int qrow = w.i * BQ + (t256 & 127);
-      if (qrow >= p.src_len || t256 >= 256) return t256 < 128 ? INFINITY : 0.f;
+      const int qrow = w.i * BQ + hf * CW + (tg & (CW - 1));
+      if (qrow >= p.src_len || tg >= 2 * CW) return tg < CW ? INFINITY : 0.f;
       const size_t idx = ((size_t)b * p.lse_H + hkv * n_rep + w.head) * p.src_len + qrow;
-      return t256 < 128 ? p.lse_src.p[w.src][idx] : p.delta_src.p[w.src][idx];
+      return tg < CW ? p.lse_src.p[w.src][idx] : p.delta_src.p[w.src][idx];
     };
     auto put_stat = [&](int st, float v) {
-      if (t256 < 128) s_lse[st * 128 + t256] = v == -INFINITY ? INFINITY : v * LOG2E;
-      else if (t256 < 256) s_dlt[st * 128 + (t256 & 127)] = v;
+      const int at = st * 128 + hf * CW + (tg & (CW - 1));
+      if (tg < CW) s_lse[at] = v == -INFINITY ? INFINITY : v * LOG2E;
+      else if (tg < 2 * CW) s_dlt[at] = v;
     };
     BlockWalk w = walk0;
     if (!w.done()) put_stat(0, load_stat(w));
@@ -1405,59 +1434,63 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
       w.next();
       const bool more = !w.done();
       const float stat_next = more ? load_stat(w) : 0.f;
-      softmax_sync_all<NS>();   // this block's statistics are in place, the last block's have been read
+      group_sync(hf);   // this block's statistics are in place, the last block's have been read
       const bool need_mask = p.causal && k_pos0 + BKV - 1 > q_pos0;
-      ok = ok && !*abort_flag && warp_wait(B_(KB_ST), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 8);
+      ok = ok && !*abort_flag;
+      ok = __all_sync(0xffffffffu, ok) && warp_wait(B_(KB_ST), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 8);
+      if (more) put_stat(st ^ 1, stat_next);
+      if (!ok) continue;
       float pr[CW];
       uint32_t t[CW], pk[CW / 2];
-      if (ok) {
-        np::tc_fence_after();
-        tmem_ld_cols<CW>(tSt + lane_off + hf * CW, t);
+      np::tc_fence_after();
+      tmem_ld_cols<CW>(tSt + lane_off + hf * CW, t);
 #pragma unroll
-        for (int e = 0; e < CW; e += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(&s_lse[st * 128 + hf * CW + e]);
-          pr[e] = ex2(fmaf(__uint_as_float(t[e]), p.scale_log2, -l4.x));
-          pr[e + 1] = ex2(fmaf(__uint_as_float(t[e + 1]), p.scale_log2, -l4.y));
-          pr[e + 2] = ex2(fmaf(__uint_as_float(t[e + 2]), p.scale_log2, -l4.z));
-          pr[e + 3] = ex2(fmaf(__uint_as_float(t[e + 3]), p.scale_log2, -l4.w));
-        }
-        if (need_mask) {
+      for (int e = 0; e < CW; e += 4) {
+        const float4 l4 = *reinterpret_cast<const float4*>(&s_lse[st * 128 + hf * CW + e]);
+        pr[e] = ex2(fmaf(__uint_as_float(t[e]), p.scale_log2, -l4.x));
+        pr[e + 1] = ex2(fmaf(__uint_as_float(t[e + 1]), p.scale_log2, -l4.y));
+        pr[e + 2] = ex2(fmaf(__uint_as_float(t[e + 2]), p.scale_log2, -l4.z));
+        pr[e + 3] = ex2(fmaf(__uint_as_float(t[e + 3]), p.scale_log2, -l4.w));
+      }
+      if (need_mask) {
 #pragma unroll
-          for (int e = 0; e < CW; ++e)
-            if (k_pos > q_pos0 + hf * CW + e) pr[e] = 0.f;
-        }
+        for (int e = 0; e < CW; ++e)
+          if (k_pos > q_pos0 + hf * CW + e) pr[e] = 0.f;
+      }
 #pragma unroll
-        for (int e = 0; e < CW; e += 2) pk[e >> 1] = np::pack_bf16(pr[e], pr[e + 1]);
-      }
-      row_sync<NS>(quarter);   // both threads of the row hold their S^T values: P^T may now overwrite those columns
-      if (ok) {
-        tmem_st_cols<CW / 2>(tSt + lane_off + hf * (CW / 2), pk);
-        tmem_st_wait();
-        np::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) np::mbar_arrive(B_(KB_P));
-        ok = warp_wait(B_(KB_DPT), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 9);
-      }
-      if (ok) {
-        np::tc_fence_after();
-        tmem_ld_cols<CW>(tdPt + lane_off + hf * CW, t);
+      for (int e = 0; e < CW; e += 2) pk[e >> 1] = np::pack_bf16(pr[e], pr[e + 1]);
+      tmem_st_cols<CW / 2>(tSt + lane_off + hf * CW, pk);
+      tmem_st_wait();
+      np::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) np::mbar_arrive(B_(KB_P));
+      ok = warp_wait(B_(KB_DPT), (uint32_t)i & 1u, abort_flag, KID_ATTN_DKV, 9);
+      if (!ok) continue;
+      np::tc_fence_after();
+      tmem_ld_cols<CW>(tdPt + lane_off + hf * CW, t);
+      np::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) np::mbar_arrive(B_(KB_DPR));
 #pragma unroll
-        for (int e = 0; e < CW; e += 4) {
-          const float4 d4 = *reinterpret_cast<const float4*>(&s_dlt[st * 128 + hf * CW + e]);
-          pk[e >> 1] = np::pack_bf16(pr[e] * (__uint_as_float(t[e]) - d4.x), pr[e + 1] * (__uint_as_float(t[e + 1]) - d4.y));
-          pk[(e >> 1) + 1] =
-              np::pack_bf16(pr[e + 2] * (__uint_as_float(t[e + 2]) - d4.z), pr[e + 3] * (__uint_as_float(t[e + 3]) - d4.w));
-        }
+      for (int e = 0; e < CW; e += 4) {
+        const float4 d4 = *reinterpret_cast<const float4*>(&s_dlt[st * 128 + hf * CW + e]);
+        pk[e >> 1] = np::pack_bf16(pr[e] * (__uint_as_float(t[e]) - d4.x), pr[e + 1] * (__uint_as_float(t[e + 1]) - d4.y));
+        pk[(e >> 1) + 1] =
+            np::pack_bf16(pr[e + 2] * (__uint_as_float(t[e + 2]) - d4.z), pr[e + 3] * (__uint_as_float(t[e + 3]) - d4.w));
       }
-      if (more) put_stat(st ^ 1, stat_next);
-      row_sync<NS>(quarter);   // same for dP^T -> dS^T
-      if (ok) {
-        tmem_st_cols<CW / 2>(tdPt + lane_off + hf * (CW / 2), pk);
-        tmem_st_wait();
-        np::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) np::mbar_arrive(B_(KB_DS));
+      if (i > 0) ok = warp_wait(B_(KB_DSE), (uint32_t)(i - 1) & 1u, abort_flag, KID_ATTN_DKV, 12);   // the last dS^T has been read
+      if (!ok) continue;
+      // row r of dS^T, 64 Q columns (128 bytes) side by side, 128-byte swizzle
+#pragma unroll
+      for (int e = 0; e < CW / 8; ++e) {
+        const int v = hf * (CW / 8) + e;   // 16-byte vector of the row
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sdS + (v >> 3) * (128 * 128) + r * 128 + (((v ^ r) & 7) << 4)),
+                     "r"(pk[4 * e]), "r"(pk[4 * e + 1]), "r"(pk[4 * e + 2]), "r"(pk[4 * e + 3])
+                     : "memory");
       }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) np::mbar_arrive(B_(KB_DS));
     }
     ok = __all_sync(0xffffffffu, ok && !*abort_flag) && warp_wait(B_(KB_FIN), 0, abort_flag, KID_ATTN_DKV, 10);
     const int row = jb * BKV + r;
@@ -1537,7 +1570,7 @@ static int launch_bwd(dim3 gq, dim3 gk, int skip, const CUtensorMap& tmQ, const 
                       const CUtensorMap& tmV, const TmapList& lK, const TmapList& lV, const TmapList& lQ,
                       const TmapList& ldO, const BwdParams& pq, const BwdParams& pk, cudaStream_t stream) {
   constexpr int SMEM_DQ = BWD_TILES * tile_bytes<HD>() + 8 * QB_COUNT + 16 + 16;
-  constexpr int SMEM_DKV = BWD_TILES * tile_bytes<HD>() + 8 * KB_COUNT + 16 + 2048 + 16;
+  constexpr int SMEM_DKV = dkv_bytes<HD>() + 8 * KB_COUNT + 16 + 2048 + 16;
   static_assert(SMEM_DKV <= 227 * 1024, "shared memory budget");
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
