@@ -521,7 +521,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // 128 t + 128), O of tile t at [256 + 128 t, ...); P (bf16 pairs, 64 columns) overwrites the S it came from, which
 // is safe because a thread loads its whole row of S before it stores P, and S of the next block is only issued
 // after the P V that read P.
-enum { G_Q = 0, G_K = 1, G_KE = 4, G_V = 7, G_VE = 9, G_S = 11, G_P = 13, G_O = 15, G_COUNT = 17 };
+enum { G_Q = 0, G_K = 1, G_KE = 4, G_V = 7, G_VE = 9, G_S = 11, G_P = 13, G_O = 15, G_P2 = 17, G_COUNT = 19 };
+constexpr int P_FIRST = 3;   // quarters of P that are handed over as soon as they are stored (G_P), the rest follows (G_P2)
 #ifdef NP_ATTN_PROF   // development build only: cycles per softmax phase, summed over (lane 0 of) all warps
 __device__ unsigned long long g_fwd2_prof[8];
 #define PROF_T(v) const long long v = clock64()
@@ -569,7 +570,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int nv = nv0 > nv1 ? nv0 : nv1;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < G_COUNT; ++i) np::mbar_init(B_(i), (i == G_P || i == G_P + 1) ? 4 : 1);
+    for (int i = 0; i < G_COUNT; ++i) np::mbar_init(B_(i), (i == G_P || i == G_P + 1 || i == G_P2 || i == G_P2 + 1) ? 4 : 1);
     *abort_flag = 0;
     np::mbar_fence_init();
   }
@@ -621,17 +622,29 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       np::tc_fence_after();
       return w;
     };
+    // P of tile t arrives in two parts (the first of them also says that O has been rescaled)
     auto issue_pv = [&](int t, int i, bool last) {
       const int vs = i % G_VST;
+      const uint64_t b = dV + (uint32_t)(vs * (TILE_BYTES >> 4));
+      if (!np::mbar_wait_warp(B_(G_P + t), (uint32_t)i & 1u, abort_flag, KID_ATTN, 26)) return false;
+      np::tc_fence_after();
       if (np::elect_one()) {
-        const uint64_t b = dV + (uint32_t)(vs * (TILE_BYTES >> 4));
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < 2 * P_FIRST; ++kk)
           tc_mma_f16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, b + mnoff(kk), idesc_pv, (i > 0) || (kk > 0));
+      }
+      __syncwarp();
+      if (!np::mbar_wait_warp(B_(G_P2 + t), (uint32_t)i & 1u, abort_flag, KID_ATTN, 27)) return false;
+      np::tc_fence_after();
+      if (np::elect_one()) {
+#pragma unroll
+        for (int kk = 2 * P_FIRST; kk < 8; ++kk)
+          tc_mma_f16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, b + mnoff(kk), idesc_pv, true);
         np::tc_commit(B_(G_O + t));
         if (last) np::tc_commit(B_(G_VE + vs));
       }
       __syncwarp();
+      return true;
     };
     if (ok && nv > 0) {
       ok = wait_k(0);
@@ -645,10 +658,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       bool have_k = false;
       ok = np::mbar_wait_warp(B_(G_V + vs), (uint32_t)(i / G_VST) & 1u, abort_flag, KID_ATTN, 25);
       if (ok && i < nv0) {
-        ok = np::mbar_wait_warp(B_(G_P + 0), (uint32_t)i & 1u, abort_flag, KID_ATTN, 26);   // P of tile 0 stored, O rescaled
+        ok = issue_pv(0, i, i >= nv1);
         if (!ok) break;
-        np::tc_fence_after();
-        issue_pv(0, i, i >= nv1);
         if (i + 1 < nv0) {
           ok = wait_k(i + 1);
           if (!ok) break;
@@ -657,10 +668,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       if (ok && i < nv1) {
-        ok = np::mbar_wait_warp(B_(G_P + 1), (uint32_t)i & 1u, abort_flag, KID_ATTN, 27);
+        ok = issue_pv(1, i, true);
         if (!ok) break;
-        np::tc_fence_after();
-        issue_pv(1, i, true);
         if (i + 1 < nv1) {
           if (!have_k) ok = wait_k(i + 1);
           if (!ok) break;
@@ -745,13 +754,19 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           pk[e >> 1] = np::pack_bf16(p0, p1);
         }
         tmem_st16(tS + c * 16, pk);
+        if (c == P_FIRST - 1) {
+          tmem_st_wait();
+          np::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) np::mbar_arrive(B_(G_P + t));
+        }
       }
       l += (rs[0] + rs[1]) + (rs[2] + rs[3]);
       PROF_T(c4);
       tmem_st_wait();
       np::tc_fence_before();
       __syncwarp();
-      if (lane == 0) np::mbar_arrive(B_(G_P + t));
+      if (lane == 0) np::mbar_arrive(B_(G_P2 + t));
       PROF_T(c5);
       PROF_ADD(0, c0, c1); PROF_ADD(1, c1, c2); PROF_ADD(2, c2, c3); PROF_ADD(3, c3, c4); PROF_ADD(4, c4, c5);
       PROF_ADD(5, c0, c0 + 1);
