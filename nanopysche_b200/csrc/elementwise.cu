@@ -834,6 +834,39 @@ __global__ void __launch_bounds__(NT) xent_fwd_kernel(const __nv_bfloat16* __res
   }
 }
 
+// mean[0] = sum(loss) / n and inv[0] = 1 / n, n the number of labels other than `ignore` (at least one). One block, sums in a
+// fixed order, in 64 bits: the eight launches of a few microseconds that count, clamp, convert, invert and add otherwise.
+constexpr int MEAN_THREADS = 1024;
+__global__ void __launch_bounds__(MEAN_THREADS) xent_mean_kernel(const float* __restrict__ loss,
+                                                                 const long long* __restrict__ labels,
+                                                                 float* __restrict__ mean, float* __restrict__ inv, int rows,
+                                                                 long long ignore) {
+  np::pdl_begin();
+  __shared__ double s_sum[32];
+  __shared__ int s_n[32];
+  double sum = 0.;
+  int n = 0;
+#pragma unroll 4
+  for (int r = threadIdx.x; r < rows; r += MEAN_THREADS) {
+    sum += (double)loss[r];
+    n += labels[r] != ignore;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    n += __shfl_xor_sync(0xffffffffu, n, m);
+  }
+  if (lane == 0) { s_sum[warp] = sum; s_n[warp] = n; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < MEAN_THREADS / 32; ++w) { sum += s_sum[w]; n += s_n[w]; }
+    n = n > 0 ? n : 1;
+    mean[0] = (float)(sum / n);
+    inv[0] = 1.f / (float)n;
+  }
+}
+
 constexpr int XT = 512;   // threads of the backward
 // dlogits[r, c] = (exp(logits - lse) - [c == label]) * gscale[0] * inv_count[0]; ignored rows -> 0. Four vectors in flight
 // per thread: 4096 x 32000 119 -> 94 us (floor 80). Holding a whole row in registers, so that the forward reads it once, was
@@ -1147,6 +1180,13 @@ NP_API int np_xent_fwd(const void* logits, const long long* labels, float* loss,
   if (rows <= 0) return 0;
   np_launch(xent_fwd_kernel, rows < GRID_CAP ? rows : GRID_CAP, NT, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)logits, labels, loss, lse, rows, V, ld, ignore);
+  CHECK_LAUNCH();
+}
+// mean, inv: one float each
+NP_API int np_xent_mean(const float* loss, const long long* labels, float* mean, float* inv, int rows, long long ignore,
+                        void* stream) {
+  if (rows <= 0) return 1;
+  np_launch(xent_mean_kernel, 1, MEAN_THREADS, 0, (cudaStream_t)stream, 1, loss, labels, mean, inv, rows, ignore);
   CHECK_LAUNCH();
 }
 NP_API int np_xent_bwd(const void* logits, const long long* labels, const float* lse, const float* gscale,

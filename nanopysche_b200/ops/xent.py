@@ -23,11 +23,14 @@ class _Xent(torch.autograd.Function):
         loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
         lse = torch.empty(rows, device=logits.device, dtype=torch.float32)
         _lib.call("xent_fwd", logits, labels, loss, lse, rows, V, _lib.LL(logits.stride(0)), _lib.LL(ignore_index))
-        count = (labels != ignore_index).sum().clamp_min(1).float()
-        inv = (1.0 / count).reshape(1)
+        if rows > 0:
+            mean, inv = torch.empty((), device=loss.device, dtype=torch.float32), torch.empty_like(loss[:1])
+            _lib.call("xent_mean", loss, labels, mean, inv, rows, _lib.LL(ignore_index))
+        else:
+            mean, inv = loss.sum(), torch.ones(1, device=loss.device, dtype=torch.float32)
         ctx.save_for_backward(logits, labels, lse, inv)
         ctx.ignore_index = ignore_index
-        return loss.sum() * inv[0]
+        return mean
 
     @staticmethod
     def backward(ctx, g):

@@ -50,6 +50,21 @@ def test_cross_entropy_rows(rows, V):
     assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item()) and rel(logits.grad, l64.grad) < 4e-3
 
 
+# fewer rows than a warp, more than a block, none that counts
+@pytest.mark.parametrize("rows", [1, 31, 1025, 5000])
+def test_cross_entropy_mean(rows):
+    from nanopysche_b200.ops.xent import cross_entropy
+
+    torch.manual_seed(rows)
+    logits = torch.randn(rows, 16, device="cuda").bfloat16()
+    labels = torch.randint(0, 16, (rows,), device="cuda")
+    labels[::3] = -100
+    ref = torch.nn.functional.cross_entropy(logits.double(), labels, ignore_index=-100, reduction="sum") / max(
+        1, (labels != -100).sum().item())
+    assert abs(cross_entropy(logits, labels).item() - ref.item()) <= 2e-6 * abs(ref.item())   # rows in fp32, few ulp each
+    assert cross_entropy(logits, torch.full_like(labels, -100)).item() == 0
+
+
 # one token, an odd number per CTA, more (head, slice) pairs than a block has threads, partial rotation
 @pytest.mark.parametrize("B,S,hq,hkv,hd,rot", [(1, 1, 2, 1, 64, 64), (2, 333, 16, 8, 128, 128), (1, 77, 12, 12, 64, 32),
                                                (1, 40, 64, 64, 128, 128), (3, 1000, 4, 4, 64, 64)])
