@@ -41,8 +41,11 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 template <int EB, int TOK>
 __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wg,
                                                             const float* __restrict__ bias, float* __restrict__ logits, int T,
-                                                            int D, int E) {
+                                                            int D, int E, int* __restrict__ zero, int n_zero) {
   np::pdl_begin();
+  // what the kernel behind this one adds to (a fill of its own is a launch)
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -615,10 +618,13 @@ struct DispatchParams {
   int epoch;
   int write_meta;              // 1: also write row_dst / mblk_rows / src_blocks (forward); 0: rows only
   const int* epoch_base;       // optional device counter added to `epoch`
+  int* zero_ctr;               // [n_ranks] tile counters of the pushing GEMM behind this dispatch, set to zero; may be nullptr
 };
 
 __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p) {
   np::pdl_begin();
+  if (p.zero_ctr && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < p.n_ranks; i += blockDim.x) p.zero_ctr[i] = 0;
   np::CommSpan span(p.n_ranks > 1);
   const int lane = threadIdx.x & 31;
   const int warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -877,15 +883,16 @@ __global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* __re
 
 #define CHECK_LAUNCH() do { cudaError_t e_ = cudaGetLastError(); return e_ == cudaSuccess ? 0 : 500 + (int)e_; } while (0)
 
-NP_API int np_router_logits(const void* x, const float* wg, const float* bias, float* logits, int T, int D, int E,
-                            void* stream) {
+// zero [n_zero]: set to zero (n_zero may be 0)
+NP_API int np_router_logits(const void* x, const float* wg, const float* bias, float* logits, int T, int D, int E, int* zero,
+                            int n_zero, void* stream) {
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
   // four tokens per warp once that still leaves eight warps for every SM
   const int tok = T >= 148 * 8 * 4 / 2 ? 4 : 1;
   const long long warps = ((long long)T + tok - 1) / tok, blocks = (warps * 32 + 255) / 256;
   np_launch(tok == 4 ? router_logits_kernel<8, 4> : router_logits_kernel<8, 1>,
             (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
-            logits, T, D, E);
+            logits, T, D, E, zero, n_zero);
   CHECK_LAUNCH();
 }
 
@@ -988,7 +995,7 @@ struct NpDispatchArgs {
   int T, K, D, E, E_local, n_ranks, my_rank, region_rows, quant;
   void* const* peer_rows; float* const* peer_scales; long long* const* peer_row_dst;
   int* const* peer_mblk_rows; int* const* peer_src_blocks; int* const* peer_flags;
-  int* done_ctr; int epoch; int write_meta; int max_ctas; const int* epoch_base;
+  int* done_ctr; int epoch; int write_meta; int max_ctas; const int* epoch_base; int* zero_ctr;
 };
 NP_API int np_ep_dispatch(const NpDispatchArgs* a, void* stream) {
   if (a->D % 128 || a->region_rows % 128 || a->E % a->E_local || (a->quant && a->D % 256)) return 1;
@@ -999,7 +1006,7 @@ NP_API int np_ep_dispatch(const NpDispatchArgs* a, void* stream) {
   p.peer_rows = a->peer_rows; p.peer_scales = a->peer_scales; p.peer_row_dst = a->peer_row_dst;
   p.peer_mblk_rows = a->peer_mblk_rows; p.peer_src_blocks = a->peer_src_blocks; p.peer_flags = a->peer_flags;
   p.done_ctr = a->done_ctr; p.epoch = a->epoch; p.write_meta = a->write_meta;
-  p.epoch_base = a->epoch_base;
+  p.epoch_base = a->epoch_base; p.zero_ctr = a->zero_ctr;
   const int items = a->T * a->K + a->E * 128;
   int grid = (items + 7) / 8;
   const int cap = a->max_ctas > 0 ? a->max_ctas : 148 * 4;

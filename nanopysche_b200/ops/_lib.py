@@ -63,7 +63,7 @@ class DispatchArgs(C.Structure):
         ("peer_rows", c_void_p), ("peer_scales", c_void_p), ("peer_row_dst", c_void_p),
         ("peer_mblk_rows", c_void_p), ("peer_src_blocks", c_void_p), ("peer_flags", c_void_p),
         ("done_ctr", c_void_p), ("epoch", c_int), ("write_meta", c_int), ("max_ctas", c_int),
-        ("epoch_base", c_void_p),
+        ("epoch_base", c_void_p), ("zero_ctr", c_void_p),
     ]
 
 

@@ -41,11 +41,11 @@ class _Router(torch.autograd.Function):
         E = gate_w.shape[0]
         dev = x2.device
         logits = torch.empty((T, E), device=dev, dtype=torch.float32)
-        _lib.call("router_logits", x2, gate_w, gate_b, logits, T, D, E)
+        zeros = (torch.empty if T > 0 else torch.zeros)(2 * E + 1, device=dev, dtype=torch.int32)
+        counts, stats = zeros[:E], zeros[E:].view(torch.float32)    # token counts; probability sums, sum of lse^2
+        _lib.call("router_logits", x2, gate_w, gate_b, logits, T, D, E, zeros, 2 * E + 1)
         weights = torch.empty((T, K), device=dev, dtype=torch.float32)
         indices = torch.empty((T, K), device=dev, dtype=torch.int32)
-        zeros = torch.zeros(2 * E + 1, device=dev, dtype=torch.int32)   # token counts, probability sums, sum of lse^2
-        counts, stats = zeros[:E], zeros[E:].view(torch.float32)
         _lib.call("router_topk", logits, score_bias, weights, indices, counts, stats[:E], stats[E:], T, E, K, gating)
         fa = torch.empty(E + 1, device=dev, dtype=torch.float32)
         f, aux = fa[:E], fa[E]
@@ -257,6 +257,7 @@ class FusedMoERuntime:
         a.peer_src_blocks, a.peer_flags = self.p_src_blocks.data_ptr(), self.p_dispatch_flags.data_ptr()
         a.done_ctr, a.epoch, a.write_meta, a.max_ctas = self.dispatch_ctr.data_ptr(), epoch, 1, self.max_ctas_dispatch
         a.epoch_base = self.heap.epoch_base.data_ptr()
+        a.zero_ctr = self.done_counters.data_ptr()      # one GEMM pushes behind every dispatch
         _lib.check(_lib.lib().np_ep_dispatch(C.byref(a), C.c_void_p(_lib.stream())), "ep_dispatch")
 
     def combine(self, rows, slot_pos, weights, out, sent_to_peer, epoch, dl=None, wg=None, add1=None):
@@ -305,7 +306,6 @@ class FusedMoERuntime:
         if wait_epoch:
             g.ready_flags, g.epoch, g.flag_limit_ns = self.dispatch_flags.data_ptr(), wait_epoch, WAIT_LIMIT_NS
         if push_ptrs is not None:
-            self.done_counters.zero_()
             g.row_dst, g.peer_base = self.row_dst.data_ptr(), push_ptrs.data_ptr()
             g.done_counters, g.done_expected = self.done_counters.data_ptr(), self.src_blocks.data_ptr()
             g.done_flag_ptr, g.epoch = self.p_done_flag.data_ptr(), push_epoch
@@ -327,7 +327,6 @@ class FusedMoERuntime:
         if wait_epoch:
             fill.update(ready_flags=self.dispatch_flags.data_ptr(), epoch=wait_epoch, flag_limit_ns=WAIT_LIMIT_NS)
         if push_ptrs is not None:
-            self.done_counters.zero_()
             fill.update(row_dst=self.row_dst.data_ptr(), peer_base=push_ptrs.data_ptr(),
                         done_counters=self.done_counters.data_ptr(), done_expected=self.src_blocks.data_ptr(),
                         done_flag_ptr=self.p_done_flag.data_ptr(), epoch=push_epoch)
