@@ -569,8 +569,8 @@ NP_API int np_gemm_mxfp8(const NpMxGemmArgs* args, void* stream) {
   const NpMxGemmArgs& a = *args;
   if (a.M <= 0 || a.N <= 0) return 0;
   if (a.K % 128 || a.N % 8 || a.b_rows % 128 || (a.lda % 16) || (a.ldb % 16) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15) ||
-      (((uintptr_t)a.sfa) & 15) || (((uintptr_t)a.sfb) & 15) || (a.group_stride_b % 128))
-    return 1;
+      (((uintptr_t)a.sfa) & 15) || (((uintptr_t)a.sfb) & 15) || (a.group_stride_b % 128) || a.ldc % (a.out_f32 ? 4 : 8) || (!a.row_dst && (((uintptr_t)a.C) & 15)))
+    return 1;   // rows of C are stored as 16-byte vectors
   static thread_local bool ctx_bound = false;
   if (!ctx_bound) {
     int dev = 0;

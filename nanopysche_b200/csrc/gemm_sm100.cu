@@ -72,6 +72,7 @@ struct GemmParams {
   int m_split;                // > 0: output rows from here on go to C2, counted from 0 (one contraction, two outputs)
   int splits;                 // pair kernel: parts of K (cluster of 2 * splits CTAs), 1 = whole
   bool st32, st32_c2;         // rows and column chunks of C / C2 are 32-byte aligned: use 32-byte stores
+  bool v16, v16_c2;           // rows of C and of the accumulate source / of C2 are 16-byte aligned: whole vectors, else elements
   bool tma_c;                 // outputs leave through shared memory and TMA stores (tmC, tmC2)
   const float* bias;          // optional [N] fp32 added to every output row (plain epilogue)
 };
@@ -212,7 +213,7 @@ __device__ __forceinline__ void pack32(const uint32_t* r, uint32_t* w) {
 __device__ __forceinline__ void store_chunk(const GemmParams& p, const OutRow& o, uint32_t* r, int col) {
   if (!o.ok || col >= p.N) return;
   scale_bias(p, r, col);
-  if (col + 32 <= p.N) {
+  if (p.v16 && col + 32 <= p.N) {
     if (o.cin) {
       if (p.out_f32) {
 #pragma unroll
@@ -273,14 +274,14 @@ __device__ __forceinline__ void store_swiglu_chunk(const GemmParams& p, const Ou
     h[i] = np::pack_bf16(np::silu_f(g0) * u0, np::silu_f(g1) * u1);
   }
   __nv_bfloat16* dst = (__nv_bfloat16*)o.c + col;
-  if (full) {
+  if (full && p.v16) {
     store64(dst, h, p.st32);
   } else {
     _Pragma("unroll") for (int i = 0; i < 32; ++i) if (col + i < p.N) dst[i] = reinterpret_cast<__nv_bfloat16*>(h)[i];
   }
   if (!p.C2) return;
   __nv_bfloat16* d2 = (__nv_bfloat16*)p.C2 + (size_t)row * p.ldc2 + col;
-  if (full) {
+  if (full && p.v16_c2) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) h[i] = np::pack_bf16(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1]));
     store64(d2, h, p.st32_c2);
@@ -1284,14 +1285,18 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   p.epoch_base = a.epoch_base;
   p.b_ready_flags = a.b_ready_flags; p.b_rows_per_flag = a.b_rows_per_flag;
 
-  // Plain outputs (dense rows, nothing added from memory, 16-byte aligned) leave by TMA; peer-row tables, accumulation and
-  // other alignments store from registers. The SwiGLU form needs both of its outputs aligned.
+  // Rows that start on 16-byte boundaries are stored (and an accumulate source read) as whole vectors, other rows element by
+  // element: an output of 1003 or 50257 columns has such rows. Destinations behind peer_base are symmetric-heap allocations.
   const int es = a.out_f32 ? 4 : 2;
   const long long groups = a.mode == 2 ? a.num_groups : 1;
-  p.tma_c = !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue != 1 || BN == 256) && ((uintptr_t)a.C & 15) == 0 &&
-            (a.ldc * es) % 16 == 0 && (groups <= 1 || (a.group_stride_c * es) % 16 == 0) &&
-            (a.epilogue != 1 || !a.C2 || (((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0)) &&
-            (a.m_split == 0 || ((uintptr_t)a.C2 & 15) == 0);
+  p.v16 = (a.ldc * es) % 16 == 0 && (groups <= 1 || (a.group_stride_c * es) % 16 == 0) &&
+          (a.row_dst || ((uintptr_t)a.C & 15) == 0) && (a.m_split == 0 || ((uintptr_t)a.C2 & 15) == 0) &&
+          (!p.Cin || (((uintptr_t)p.Cin & 15) == 0 && (p.ldcin * es) % 16 == 0));
+  p.v16_c2 = a.C2 && ((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0;   // the up half starts at column N
+  // Plain outputs (dense rows, nothing added from memory, aligned) leave by TMA; peer-row tables, accumulation and other
+  // alignments store from registers. The SwiGLU form needs both of its outputs aligned.
+  p.tma_c = p.v16 && !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue != 1 || BN == 256) && a.ldc >= a.N &&
+            (a.epilogue != 1 || !a.C2 || p.v16_c2);
   tmC = tmA;
   tmC2 = tmA;
   if (a.epilogue == 2) {   // [d gate | d up] out, [gate | up] in: two planes of N columns each

@@ -144,3 +144,45 @@ def test_feed_forward_without_gradients_and_of_frozen_weights():
     y64 = (torch.nn.functional.silu(gu[..., :256]) * gu[..., 256:]) @ w2.double().t()
     y64.sum().backward()
     assert torch.equal(y, ya) and rel(y, y64) < 6e-3 and rel(xa.grad, x64.grad) < 1e-2
+
+
+# rows that do not start on 16-byte boundaries: odd widths on both sides of the few-row switch (64 rows) and of the 128-row tiles,
+# an aligned width behind an odd base, a row stride below a vector's
+@pytest.mark.parametrize("M", [5, 65, 130, 700])
+@pytest.mark.parametrize("N,off,ld", [(1003, 0, 1003), (129, 0, 129), (2052, 0, 2052), (512, 1, 520), (1001, 3, 1010), (7, 0, 7)])
+@pytest.mark.parametrize("kw", [dict(), dict(bn=128), dict(bn=256, mt=1), dict(bn=256, mt=2), dict(bn=256, mt=2, split=2)])
+def test_outputs_with_unaligned_rows(M, N, off, ld, kw):
+    from nanopysche_b200.ops.gemm import gemm
+
+    torch.manual_seed(M + N)
+    K = 512
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    ref = x.double() @ w.double().t()
+    bias = torch.randn(N, device="cuda")
+    for dt, tol in ((torch.bfloat16, 3e-3), (torch.float32, 2e-5)):
+        def view(fill):
+            buf = torch.full((M * ld + off + 8,), fill, device="cuda", dtype=dt)
+            return buf, buf[off:off + M * ld].view(M, ld)[:, :N]
+
+        buf, out = view(7.0)
+        gemm(x, w, out=out, bias=bias, **kw)
+        assert rel(out, ref + bias.double()) < tol
+        rest = torch.ones_like(buf, dtype=torch.bool)                  # nothing beside the rows is written
+        rest[off:off + M * ld].view(M, ld)[:, :N] = False
+        assert (buf[rest] == 7.0).all()
+        _, acc = view(1.5)
+        gemm(x, w, out=acc, accumulate=True, **kw)
+        assert rel(acc, ref + 1.5) < tol
+        _, res = view(0.25)
+        assert rel(gemm(x, w, residual=res, out_dtype=dt, **kw), ref + 0.25) < tol
+
+
+@pytest.mark.parametrize("M,F", [(65, 100), (300, 1003), (700, 129), (256, 260)])
+def test_swiglu_with_unaligned_rows(M, F):
+    from nanopysche_b200.ops.gemm import gemm_swiglu
+
+    torch.manual_seed(F)
+    x, w = torch.randn(M, 128, device="cuda").bfloat16(), (torch.randn(2 * F, 128, device="cuda") * 0.1).bfloat16()
+    h, gu = gemm_swiglu(x, w[:F], w[F:])
+    g, u = x.double() @ w[:F].double().t(), x.double() @ w[F:].double().t()
+    assert rel(gu, torch.cat([g, u], 1)) < 3e-3 and rel(h, torch.nn.functional.silu(g) * u) < 3e-3
