@@ -1172,7 +1172,7 @@ struct NpGemmArgs {
   const int* ready_flags; const int* mblk_flag; int epoch; unsigned long long flag_limit_ns;
   const long long* row_dst; void* const* peer_base;
   int* done_counters; const int* done_expected; int* const* done_flag_ptr;
-  int bn;        // 0 = choose, else 128 or 256
+  int bn;        // columns of a tile: 0 = choose, else 128 or 256 (128: one CTA per tile, whatever mt and split say)
   int max_ctas;  // 0 = all SMs
   const void* Cin; long long ldcin;  // optional accumulate source (defaults to C when accumulate != 0)
   const int* epoch_base;             // optional device counter added to `epoch`
@@ -1190,8 +1190,10 @@ struct NpGemmArgs {
   // push_ctr: a zeroed local int
   const void* push_src; long long push_bytes; void* const* push_dst; int* const* push_flag; int push_n; int* push_ctr;
   const float* bias;  // optional [N] fp32 bias added in the plain epilogue (alpha != 0)
-  int mt;             // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles on a pair of CTAs)
-  int split;          // parts of K on the pair kernel: 0 = choose, 1, 2 or 4 (dense form, plain epilogue)
+  // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles on a pair of CTAs; forms that the pair kernel does
+  // not take, and launches of one CTA, run one CTA per tile)
+  int mt;
+  int split;          // parts of K: 0 = choose, 1, or 2 or 4 on the pair kernel (dense, plain epilogue, 8 K steps, M above 128)
   int paired;         // row-grouped form: blocks 2 i and 2 i + 1 share their group and their arrival flag
   int k_split;        // > 0 (MN-major B): K rows [0, k_split) of a group come from B, the rest from B2 (multiple of 64)
   int m_split;        // > 0: output rows [0, m_split) go to C, the rest to C2 (layout of C; multiple of 256)
@@ -1327,10 +1329,11 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   const int cap = a.max_ctas > 0 ? a.max_ctas : num_sms();
   const int bn_out = a.epilogue == 1 ? BN / 2 : BN, tm = PAIR ? 2 * BM : BM;
   const long long tiles = (long long)((a.M + tm - 1) / tm) * ((a.N + bn_out - 1) / bn_out) * (a.mode == 2 ? a.num_groups : 1);
+  if (tiles <= 0) return 0;   // K-grouped form without groups
   const bool busy = 2.0 * a.M * a.N * a.K > 2e10;   // 15 us and more
   if constexpr (PAIR) {
     const long long pairs = tiles < cap / 2 ? tiles : cap / 2;
-    if (pairs <= 0) return 0;
+    if (pairs <= 0) return 1;   // the dispatch gives launches of one CTA to the other kernel
     p.splits = splits;
     const dim3 grid((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
     const cudaError_t e =
@@ -1339,7 +1342,6 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     if (e != cudaSuccess) return 500 + (int)e;
   } else {
     const int grid = (int)(tiles < cap ? tiles : cap);
-    if (grid <= 0) return 0;
     np_launch_if(busy, gemm_bf16_kernel<BN, STAGES>, grid, GEMM_THREADS, SMEM, stream, 1, tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2, p);
   }
   cudaError_t e = cudaGetLastError();
@@ -1382,9 +1384,13 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
   // for dense plain outputs with too few tiles for the SMs.
   const int nk = (a.K + BK - 1) / BK, sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
   const bool can_split = plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
+  const bool can_pair = plain && sms >= 2;   // a pair needs two CTAs
   int bn = a.bn, mt = a.mt, splits = 1;
   if (a.epilogue == 1) bn = 256;
-  if (bn == 0 || (bn == 256 && mt == 0)) {
+  if (can_pair && bn != 128 && (mt == 2 || (mt == 0 && can_split && (a.split == 2 || a.split == 4)))) {
+    bn = 256;   // asked for
+    mt = 2;
+  } else if (bn == 0 || (bn == 256 && mt == 0)) {
     const long long groups = a.mode == 2 ? a.num_groups : 1;
     // K steps of a group: its share of the token axis in the K-grouped form
     const double steps = a.mode == 2 ? 2.0 * a.blocks_per_group : nk;
@@ -1401,14 +1407,14 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
       if (c < best) { best = c; bn = bn_; mt = mt_; splits = splits_; }
     };
     take(cost(COST_256, 128, n256, sms, 1), 256, 1, 1);
-    if (plain && a.M > 128 && sms >= 2 && a.mt != 1) take(cost(COST_PAIR, 256, n256, sms / 2, 1), 256, 2, 1);
-    if (can_split && a.mt != 1 && a.split == 0 && sms >= 128) {
+    if (can_pair && a.M > 128 && a.mt == 0) take(cost(COST_PAIR, 256, n256, sms / 2, 1), 256, 2, 1);
+    if (can_split && a.mt == 0 && a.split == 0 && sms >= 128) {
       take(cost(COST_SPLIT2, 256, 256, CLUSTERS4, 2), 256, 2, 2);
       take(cost(COST_SPLIT4, 256, 256, CLUSTERS8, 4), 256, 2, 4);
     }
   }
   if (can_split && (a.split == 2 || a.split == 4)) splits = a.split;
-  if (bn == 256 && mt == 2 && plain) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
+  if (bn == 256 && mt == 2 && can_pair) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
   if (bn == 256) return launch_gemm<256, 4, false>(a, (cudaStream_t)stream);
   return launch_gemm<128, 6, false>(a, (cudaStream_t)stream);
 }

@@ -75,7 +75,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     assert out.dtype in (torch.float32, torch.bfloat16)
     args.accumulate = int(accumulate)
     args.alpha = alpha
-    # mt: 0 = choose; 2 = 256-row tiles on pairs of CTAs; split: parts of K there (0 = choose, 1, 2, 4)
+    # requests; 0 = choose. mt 2: 256 x 256 tiles on pairs of CTAs, split 2 or 4: parts of K there (bn 128: one-CTA tiles)
     args.bn, args.max_ctas, args.mt, args.split = bn, max_ctas, mt, split
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous()

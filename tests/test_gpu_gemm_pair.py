@@ -186,3 +186,25 @@ def test_swiglu_with_unaligned_rows(M, F):
     h, gu = gemm_swiglu(x, w[:F], w[F:])
     g, u = x.double() @ w[:F].double().t(), x.double() @ w[F:].double().t()
     assert rel(gu, torch.cat([g, u], 1)) < 3e-3 and rel(h, torch.nn.functional.silu(g) * u) < 3e-3
+
+
+def _kernels(f):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        f()
+        torch.cuda.synchronize()
+    return " ".join(e.key for e in p.key_averages())
+
+
+# a launch of one CTA has no pair; a request without a tile width still decides the kernel
+@pytest.mark.parametrize("kw,pair", [(dict(bn=256, mt=2, max_ctas=1), False), (dict(bn=256, mt=2, max_ctas=3), True),
+                                     (dict(mt=2), True), (dict(mt=1), False), (dict(split=2), True), (dict(split=4, mt=2), True),
+                                     (dict(bn=256, split=2), True), (dict(bn=128, mt=2), False)])
+def test_the_kernel_asked_for_runs(kw, pair):
+    from nanopysche_b200.ops.gemm import gemm
+
+    torch.manual_seed(1)
+    a, b = torch.randn(300, 512, device="cuda").bfloat16(), torch.randn(520, 512, device="cuda").bfloat16()
+    out = torch.full((300, 520), float("nan"), device="cuda")
+    gemm(a, b, out=out, **kw)
+    assert rel(out, a.double() @ b.double().t()) < 2e-5
+    assert ("pair" in _kernels(lambda: gemm(a, b, out=out, **kw))) == pair
