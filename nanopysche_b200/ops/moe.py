@@ -47,8 +47,10 @@ class _Router(torch.autograd.Function):
         weights = torch.empty((T, K), device=dev, dtype=torch.float32)
         indices = torch.empty((T, K), device=dev, dtype=torch.int32)
         _lib.call("router_topk", logits, score_bias, weights, indices, counts, stats[:E], stats[E:], T, E, K, gating)
-        fa = torch.empty(E + 1, device=dev, dtype=torch.float32)
-        f, aux = fa[:E], fa[E]
+        # tensors of their own: an output that is a view beside another differentiable output may not be changed in place,
+        # and the saved load fractions must not share the loss's version counter
+        f = torch.empty(E, device=dev, dtype=torch.float32)
+        aux = torch.empty((), device=dev, dtype=torch.float32)
         _lib.call("router_aux", counts, stats[:E], stats[E:], float(coef_z or 0.0), f, aux, T, E)
         ctx.save_for_backward(x2, gate_w, logits, weights, indices, f, score_bias if score_bias is not None
                               else logits.new_empty(0))

@@ -110,6 +110,29 @@ def test_router_forward_in_one_piece(T, D, E, K):
     assert abs(aux.item() - ref.item()) < 1e-5 * abs(ref.item())
 
 
+def test_auxiliary_losses_add_up_in_place():
+    """``aux_loss`` is the caller's own tensor: scaling it and adding to it in place leave the gradients right."""
+    from nanopysche_b200.models.moe import MoEBase
+
+    torch.manual_seed(0)
+    a, b = (MoEBase(d_model=128, hidden_size=256, num_experts=4, top_k=2, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    x = torch.randn(1, 200, 128, device="cuda").bfloat16()
+
+    def grads(total):
+        a.zero_grad(), b.zero_grad()
+        total.backward()
+        return [m.router.gate.weight.grad.clone() for m in (a, b)]
+
+    (a(x), b(x))
+    want = grads(2 * a.aux_loss + b.aux_loss)
+    (a(x), b(x))
+    total = a.aux_loss
+    total.mul_(2)
+    total += b.aux_loss
+    for g, w in zip(grads(total), want):
+        assert w.norm() > 0 and rel(g, w) < 1e-6
+
+
 @pytest.mark.parametrize("T,cap,ranks", [(1, -1, 1), (700, 150, 2), (4096, 1280, 4)])
 def test_capacity_plan_matches_the_scan(T, cap, ranks):
     from nanopysche_b200.ops import _lib
