@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
   if (threadIdx.x == 0) atomicAdd(zsum, s_z);
 }
 
-// f[e] = counts[e] / T and aux = E * sum_e f[e] * psum[e] / T + coef_z * zsum / T (one warp)
+// f[e] = counts[e] / T and aux = E * sum_e f[e] * psum[e] / T + coef_z * zsum / T (one warp); NaN without tokens, the mean of
+// nothing
 __global__ void __launch_bounds__(32) router_aux_kernel(const int* __restrict__ counts, const float* __restrict__ psum,
                                                         const float* __restrict__ zsum, float coef_z, float* __restrict__ f,
                                                         float* __restrict__ aux, int T, int E) {
@@ -913,7 +914,7 @@ NP_API int np_router_topk(const float* logits, const float* score_bias, float* w
 
 NP_API int np_router_aux(const int* counts, const float* psum, const float* zsum, float coef_z, float* f, float* aux, int T,
                          int E, void* stream) {
-  if (T <= 0 || E > MAX_E) return 1;
+  if (T < 0 || E > MAX_E) return 1;
   np_launch(router_aux_kernel, 1, 32, 0, (cudaStream_t)stream, 1, counts, psum, zsum, coef_z, f, aux, T, E);
   CHECK_LAUNCH();
 }

@@ -71,8 +71,9 @@ class _Router(torch.autograd.Function):
                   gating)
         parts = _lib.lib().np_router_dgate_parts(T)
         scratch = torch.empty((parts, E, D), device=x2.device, dtype=torch.float32)
-        dgw = torch.empty_like(gate_w)
-        dgb = torch.empty(E, device=x2.device, dtype=torch.float32)
+        new = torch.empty if T > 0 else torch.zeros    # no tokens: the kernels below do nothing
+        dgw = new(gate_w.shape, device=x2.device, dtype=gate_w.dtype)
+        dgb = new(E, device=x2.device, dtype=torch.float32)
         _lib.call("router_dgate", dl, x2, dgw, dgb, scratch, T, D, E, 0)
         if x2.dtype == torch.bfloat16 and gate_w.dtype == torch.float32 and gate_w.is_contiguous():
             dx = torch.empty_like(x2)

@@ -110,6 +110,18 @@ def test_router_forward_in_one_piece(T, D, E, K):
     assert abs(aux.item() - ref.item()) < 1e-5 * abs(ref.item())
 
 
+def test_router_without_tokens():
+    """No tokens: no error, counts and gradients of zero, and NaN as the mean over nothing."""
+    from nanopysche_b200.ops.moe import _Router
+
+    gate = [t.requires_grad_(True) for t in (torch.randn(4, 64, device="cuda"), torch.randn(4, device="cuda"))]
+    x = torch.zeros(0, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    w, idx, aux, counts = _Router.apply(x, *gate, None, 2, 0, 1e-2)
+    assert w.shape == idx.shape == (0, 2) and aux.isnan() and counts.tolist() == [0] * 4
+    w.sum().backward()
+    assert x.grad.shape == (0, 64) and not gate[0].grad.any() and not gate[1].grad.any()
+
+
 def test_auxiliary_losses_add_up_in_place():
     """``aux_loss`` is the caller's own tensor: scaling it and adding to it in place leave the gradients right."""
     from nanopysche_b200.models.moe import MoEBase
