@@ -108,6 +108,12 @@ def flash_supported(q: torch.Tensor, k: torch.Tensor) -> bool:
             and all(s % 8 == 0 for s in q.stride()[:3]) and all(s % 8 == 0 for s in k.stride()[:3]))
 
 
+def _same_rows(k: torch.Tensor, v: torch.Tensor) -> bool:
+    """One set of strides addresses both: a dimension of size 1 is never stepped over, and ``contiguous()`` leaves its
+    stride as it is (batch 1 of a longer buffer)."""
+    return k.shape == v.shape and all(n == 1 or a == b for n, a, b in zip(k.shape, k.stride(), v.stride()))
+
+
 def _rows_aligned(t: torch.Tensor) -> bool:
     return t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 and s != 0 for s in t.stride()[:3])
 
@@ -186,7 +192,7 @@ def flash_bwd(q, k, v, o, d_o, lse, *, causal=True, scale=None, q_off=0, delta=N
     a.q, a.k, a.v, a.o, a.d_o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr()
     a.q_sb, a.q_ss, a.q_sh = _strides3(q)
     a.k_sb, a.k_ss, a.k_sh = _strides3(k)
-    assert _strides3(v) == _strides3(k), "k and v must share their strides"
+    assert _same_rows(k, v), "k and v must share their strides"
     a.o_sb, a.o_ss, a.o_sh = _strides3(o)
     a.do_sb, a.do_ss, a.do_sh = _strides3(d_o)
     a.lse, a.delta = lse.data_ptr(), delta.data_ptr()
@@ -290,9 +296,9 @@ class _FlashAttention(torch.autograd.Function):
 
 def flash_attention(q, k, v, causal=True, scale=None):
     """Differentiable attention on the tcgen05 flash kernels (see ``flash_supported``)."""
-    if k.stride() != v.stride():
+    if not _same_rows(k, v):
         v = v.contiguous() if k.is_contiguous() else v
-        if k.stride() != v.stride():
+        if not _same_rows(k, v):
             k, v = k.contiguous(), v.contiguous()
     return _FlashAttention.apply(q, k, v, causal, scale)
 

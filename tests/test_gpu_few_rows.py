@@ -112,3 +112,28 @@ def test_flash_head_dim_64_views_that_need_a_copy():
     for q, k, v in ((odd, odd, odd), (tr, odd, wide), (odd, wide, wide)):
         o = attention(q, k, v)
         assert torch.equal(o, attention(q.contiguous(), k.contiguous(), v.contiguous()))
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,Hkv", [(1, 2), (2, 1), (1, 1)])
+def test_flash_keys_of_a_longer_buffer(B, Hkv, hd):
+    """k is the start of a longer buffer, v a tensor of its own: with a batch or head count of 1 both count as contiguous
+    although their strides differ. Forward and backward give what copies give."""
+    from nanopysche_b200.ops.attention import attention
+
+    torch.manual_seed(hd)
+    q = torch.randn(B, 40, 4, hd, device="cuda").bfloat16()
+    buf = torch.randn(B, 300, Hkv, hd, device="cuda").bfloat16()
+    v = torch.randn(B, 200, Hkv, hd, device="cuda").bfloat16()
+    wide = torch.randn(B, 200, 3 * Hkv, hd, device="cuda").bfloat16()
+    g = torch.randn_like(q)
+
+    def grads(k, v):
+        leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+        o = attention(*leaves)
+        return [o, *torch.autograd.grad(o, leaves, g)]
+
+    for kk, vv in ((buf[:, :200], v), (v, buf[:, :200]), (wide[:, :, :Hkv], v), (buf[:, 50:250], wide[:, :, Hkv:2 * Hkv])):
+        for a, b in zip(grads(kk, vv), grads(kk.clone(memory_format=torch.contiguous_format),
+                                             vv.clone(memory_format=torch.contiguous_format))):
+            assert torch.equal(a, b)
