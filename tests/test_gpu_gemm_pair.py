@@ -188,6 +188,19 @@ def test_swiglu_with_unaligned_rows(M, F):
     assert rel(gu, torch.cat([g, u], 1)) < 3e-3 and rel(h, torch.nn.functional.silu(g) * u) < 3e-3
 
 
+def test_feed_forward_of_mismatched_widths_is_refused():
+    from nanopysche_b200.ops.gemm import feed_forward_glu, gemm_swiglu
+
+    x = torch.randn(2, 70, 128, device="cuda").bfloat16()
+    w13, w2 = torch.randn(512, 64, device="cuda").bfloat16(), torch.randn(128, 256, device="cuda").bfloat16()
+    with pytest.raises(AssertionError, match="contraction"):
+        feed_forward_glu(x, w13, w2)
+    with pytest.raises(AssertionError, match="contraction"):
+        feed_forward_glu(x, torch.randn(256, 128, device="cuda").bfloat16(), w2)     # w2 of another hidden size
+    with pytest.raises(AssertionError):
+        gemm_swiglu(x[0], w13[:256].t(), w13[256:].t())
+
+
 def _kernels(f):
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
         f()
