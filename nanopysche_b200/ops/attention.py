@@ -20,6 +20,7 @@ import torch
 import os
 
 import torch.nn.functional as F
+from torch.autograd.forward_ad import unpack_dual
 
 from . import _lib
 
@@ -342,7 +343,7 @@ DECODE_ROWS = 8
 
 def attention_append(q, k_cache, v_cache, k_new, v_new, causal: bool = True, scale: float | None = None):
     """Attention of ``q [B, S, Hq, hd]`` over a KV cache with ``S`` new positions behind it; returns ``(out, k, v)`` with
-    ``k = cat(k_cache, k_new)`` and ``v`` likewise (dim 1). Without gradients and for a few query rows per KV head (token
+    ``k = cat(k_cache, k_new)`` and ``v`` likewise (dim 1). Without gradients (of either mode) and for a few query rows per KV head (token
     generation) one kernel reads each key and value once, attends and writes the concatenation; else a concatenation
     followed by ``attention``."""
     B, S, Hq, hd = q.shape
@@ -350,6 +351,7 @@ def attention_append(q, k_cache, v_cache, k_new, v_new, causal: bool = True, sca
     ts = (q, k_cache, v_cache, k_new, v_new)
     if (USE_FLASH and _lib.on(q) and hd in (64, 128) and Hq // Hkv * S <= DECODE_ROWS and k_cache.shape[1] > 0 and
             not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) and
+            not any(unpack_dual(t).tangent is not None for t in ts) and
             k_new.shape == (B, S, Hkv, hd) == v_new.shape and
             k_cache.shape == v_cache.shape == (B, k_cache.shape[1], Hkv, hd) and
             all(t.device == q.device for t in ts) and _decode_views(*ts)):

@@ -79,6 +79,20 @@ def test_append_under_grad_takes_the_differentiable_path():
     assert q.grad is not None and ko.shape[1] == 41
 
 
+def test_append_does_not_drop_tangents():
+    """Forward-mode derivatives of the flash kernels do not exist: a cached step that carries one says so."""
+    from torch.autograd import forward_ad as fwAD
+
+    from nanopysche_b200.ops.attention import attention_append
+
+    ts = [torch.randn(1, n, 4, 64, device="cuda").bfloat16() for n in (1, 40, 40, 1, 1)]
+    for i in range(5):
+        with fwAD.dual_level(), pytest.raises(NotImplementedError):
+            attention_append(*(fwAD.make_dual(t, torch.ones_like(t)) if j == i else t for j, t in enumerate(ts)))
+    with fwAD.dual_level(), torch.no_grad():
+        assert attention_append(*ts)[1].shape[1] == 41
+
+
 @pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,causal", [(1, 128, 128, 2, 2, True), (2, 129, 129, 4, 2, True),
                                                    (1, 100, 300, 4, 2, True), (1, 1, 257, 8, 8, True),
                                                    (3, 777, 777, 6, 3, False), (2, 1000, 1000, 4, 4, True)])
