@@ -161,7 +161,10 @@ class FusedMoERuntime:
         blk = torch.arange(self.blocks, device=self.device)
         self.mblk_group = (blk // (self.N * self.bpr)).to(torch.int32)
         self.mblk_flag = ((blk // self.bpr) % self.N).to(torch.int32)
+        # tiles that the pushing GEMM has stored per destination: set to zero by the dispatch kernel, so a GEMM may push once
+        # behind every dispatch on the same stream (``_push_counters`` holds callers to that)
         self.done_counters = torch.zeros(self.N, device=self.device, dtype=torch.int32)
+        self._may_push = False
         self.dispatch_ctr = torch.zeros(1, device=self.device, dtype=torch.int32)
         self.layer_of: dict[int, int] = {}
         self.max_ctas_dispatch = max_ctas_dispatch
@@ -260,8 +263,17 @@ class FusedMoERuntime:
         a.peer_src_blocks, a.peer_flags = self.p_src_blocks.data_ptr(), self.p_dispatch_flags.data_ptr()
         a.done_ctr, a.epoch, a.write_meta, a.max_ctas = self.dispatch_ctr.data_ptr(), epoch, 1, self.max_ctas_dispatch
         a.epoch_base = self.heap.epoch_base.data_ptr()
-        a.zero_ctr = self.done_counters.data_ptr()      # one GEMM pushes behind every dispatch
+        a.zero_ctr = self.done_counters.data_ptr()
         _lib.check(_lib.lib().np_ep_dispatch(C.byref(a), C.c_void_p(_lib.stream())), "ep_dispatch")
+        self._may_push = True
+
+    def _push_counters(self) -> int:
+        """Address of the counters for a GEMM that pushes its rows. A second push behind one dispatch would start from the
+        first one's counts, never reach the expected number and leave the combine pass waiting."""
+        if not self._may_push:
+            raise _lib.KernelError("a GEMM of the expert-parallel runtime pushes rows once behind every dispatch")
+        self._may_push = False
+        return self.done_counters.data_ptr()
 
     def combine(self, rows, slot_pos, weights, out, sent_to_peer, epoch, dl=None, wg=None, add1=None):
         a = _lib.CombineArgs()
@@ -310,7 +322,7 @@ class FusedMoERuntime:
             g.ready_flags, g.epoch, g.flag_limit_ns = self.dispatch_flags.data_ptr(), wait_epoch, WAIT_LIMIT_NS
         if push_ptrs is not None:
             g.row_dst, g.peer_base = self.row_dst.data_ptr(), push_ptrs.data_ptr()
-            g.done_counters, g.done_expected = self.done_counters.data_ptr(), self.src_blocks.data_ptr()
+            g.done_counters, g.done_expected = self._push_counters(), self.src_blocks.data_ptr()
             g.done_flag_ptr, g.epoch = self.p_done_flag.data_ptr(), push_epoch
             g.C, g.ldc = None, N
             g.out_f32 = 0
@@ -331,7 +343,7 @@ class FusedMoERuntime:
             fill.update(ready_flags=self.dispatch_flags.data_ptr(), epoch=wait_epoch, flag_limit_ns=WAIT_LIMIT_NS)
         if push_ptrs is not None:
             fill.update(row_dst=self.row_dst.data_ptr(), peer_base=push_ptrs.data_ptr(),
-                        done_counters=self.done_counters.data_ptr(), done_expected=self.src_blocks.data_ptr(),
+                        done_counters=self._push_counters(), done_expected=self.src_blocks.data_ptr(),
                         done_flag_ptr=self.p_done_flag.data_ptr(), epoch=push_epoch)
         return gemm_mxfp8(aq, sfa, bq, sfb, out=out, mblk_group=self.mblk_group, mblk_rows=self.mblk_rows,
                           rows_per_group=N, fill=fill)

@@ -145,6 +145,48 @@ def test_auxiliary_losses_add_up_in_place():
         assert w.norm() > 0 and rel(g, w) < 1e-6
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+def test_every_dispatch_starts_the_push_counters_anew(fp8):
+    """Two rounds of dispatch and push (other tokens, other routing) give what a fresh runtime gives for the second one, the
+    counters hold exactly that round's tiles, and a second push behind one dispatch is refused."""
+    from nanopysche_b200.models.moe import MoEBase
+    from nanopysche_b200.ops import _lib
+    from nanopysche_b200.ops.moe import FusedMoERuntime
+
+    T, D, H, E, K = 700, 256, 256, 8, 2
+    torch.manual_seed(0)
+    m = MoEBase(d_model=D, hidden_size=H, num_experts=E, top_k=K, dtype=torch.bfloat16, device="cuda")
+    with torch.no_grad():
+        for w in (m.w1, m.w2, m.w3):
+            w.normal_(0, 0.05)
+        m.router.gate.weight.normal_()
+    xs = [torch.randn(1, T, D, device="cuda").bfloat16() for _ in range(2)]
+
+    def once(rt, x):
+        m._fused_runtime = rt
+        x = x.clone().requires_grad_(True)
+        for p in m.parameters():
+            p.grad = None
+        rt.layer_index(m)
+        y = m(x)
+        fwd = rt.done_counters.clone()
+        y.float().square().sum().backward()
+        return [y.detach(), x.grad, m.w1.grad, m.w2.grad, m.w3.grad, fwd, rt.done_counters.clone(), rt.src_blocks.clone()]
+
+    def runtime():
+        return FusedMoERuntime(tokens=T, d_model=D, hidden=H, num_experts=E, top_k=K, n_layers=1, capacity_factor=None, fp8=fp8)
+
+    rt = runtime()
+    once(rt, xs[0])
+    got, want = once(rt, xs[1]), once(runtime(), xs[1])
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
+    assert got[-1].item() > 0 and got[5].item() % got[-1].item() == 0 and got[6].item() % got[-1].item() == 0
+    with pytest.raises(_lib.KernelError, match="once behind every dispatch"):
+        rt.grouped_gemm(rt.recv_g, m.w1, N=D, K=H, b_mn=True, group_stride_b=H, push_ptrs=rt.p_ret_g, push_epoch=1)
+    _lib.check_status("after test")
+
+
 @pytest.mark.parametrize("T,cap,ranks", [(1, -1, 1), (700, 150, 2), (4096, 1280, 4)])
 def test_capacity_plan_matches_the_scan(T, cap, ranks):
     from nanopysche_b200.ops import _lib
