@@ -1010,8 +1010,8 @@ struct BwdParams {
 // delta[b, h, s] = sum over the head dimension of o * d_o: HD / 8 lanes per row, 16 bytes of each tensor per lane
 template <int HD>
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
-                  const __nv_bfloat16* __restrict__ d_o, long long d_sb, long long d_ss, long long d_sh,
+attn_delta_kernel(const __nv_bfloat16* o, long long o_sb, long long o_ss, long long o_sh,
+                  const __nv_bfloat16* d_o, long long d_sb, long long d_ss, long long d_sh,
                   float* __restrict__ delta, int B, int S, int H) {
   np::pdl_begin();
   constexpr int L = HD / 8;

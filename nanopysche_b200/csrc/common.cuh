@@ -165,6 +165,9 @@ namespace np {
 // block setup, barrier and tensor-memory allocation and the launch itself overlap that tail. `pdl_wait` returns once every
 // preceding kernel has completed and its memory is visible; nothing but kernel parameters is read, and nothing is written,
 // before it. `pdl_trigger` lets the successor start in turn, as soon as all blocks of this kernel have started.
+// What a kernel reads may thus be written during its lifetime. So its inputs are read with plain loads: `__ldg`, `ld.global.nc`
+// and parameters that are both `const` and `__restrict__` promise the compiler that nobody writes them while the kernel
+// lives, and such a load may be moved in front of the wait. `__restrict__` stands on outputs only.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {

@@ -57,9 +57,9 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
 // y = (x [+ res]) * rsqrt(mean((x+res)^2) + eps) * w ; optionally writes h = x + res.
 // cols must be a multiple of 8 and <= NT*8*MAXV.
 template <int MAXV>
-__global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                         const __nv_bfloat16* __restrict__ res,
-                                                         const float* __restrict__ w,
+__global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* x,
+                                                         const __nv_bfloat16* res,
+                                                         const float* w,
                                                          __nv_bfloat16* __restrict__ y,
                                                          __nv_bfloat16* __restrict__ h_out,
                                                          float* __restrict__ rstd, int rows, int cols,
@@ -135,10 +135,10 @@ constexpr int NR = 4;   // rows that the RMSNorm backward takes at a time
 // registers over all its rows (a warp per row kept it in shared memory, 16 KB of traffic per row). With the column sum,
 // 4096 x 2048: 23.5 -> 21.1 us, 16384 x 2048: 63.8 -> 56.8, 4096 x 768: 22.2 -> 15.7 (DRAM-cold, floors 10, 41 and 4). The same
 // form of the forward pass was slower than a CTA per row (15.1 -> 20.6): it has half the traffic to hide a barrier behind.
-__global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                               const __nv_bfloat16* __restrict__ x,
-                                                               const float* __restrict__ w, const float* __restrict__ rstd,
-                                                               const __nv_bfloat16* __restrict__ dres,
+__global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* dy,
+                                                               const __nv_bfloat16* x,
+                                                               const float* w, const float* rstd,
+                                                               const __nv_bfloat16* dres,
                                                                __nv_bfloat16* __restrict__ dx,
                                                                float* __restrict__ dw_partial, int rows, int cols) {
   np::pdl_begin();
@@ -211,9 +211,9 @@ __global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat
 // amax / 448; y (bf16) is optional. cols must be a multiple of 128: a block is the 16 consecutive threads of a
 // half-warp, 8 elements each.
 template <int MAXV>
-__global__ void __launch_bounds__(NT) rmsnorm_quant_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                               const __nv_bfloat16* __restrict__ res,
-                                                               const float* __restrict__ w,
+__global__ void __launch_bounds__(NT) rmsnorm_quant_fwd_kernel(const __nv_bfloat16* x,
+                                                               const __nv_bfloat16* res,
+                                                               const float* w,
                                                                __nv_bfloat16* __restrict__ y,
                                                                __nv_bfloat16* __restrict__ h_out,
                                                                float* __restrict__ rstd, uint8_t* __restrict__ q,
@@ -288,11 +288,11 @@ __global__ void __launch_bounds__(NT) rmsnorm_quant_fwd_kernel(const __nv_bfloat
 
 // dx = rs * (w*dy - xhat * mean(w*dy*xhat)) [+ dres]; per-CTA partial dw into scratch[grid, cols].
 template <int MAXV>
-__global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                         const __nv_bfloat16* __restrict__ x,
-                                                         const float* __restrict__ w,
-                                                         const float* __restrict__ rstd,
-                                                         const __nv_bfloat16* __restrict__ dres,
+__global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* dy,
+                                                         const __nv_bfloat16* x,
+                                                         const float* w,
+                                                         const float* rstd,
+                                                         const __nv_bfloat16* dres,
                                                          __nv_bfloat16* __restrict__ dx,
                                                          float* __restrict__ dw_partial, int rows, int cols) {
   np::pdl_begin();
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __
 // out[c] (+)= sum_p partial[p, c] with 8 row lanes per 32-column strip (block 32 x 8) and four loads in flight per
 // thread: the partial matrix is a few hundred rows tall, so one thread per column would be a serial chain of
 // dependent loads.
-__global__ void __launch_bounds__(256) colsum_tall_kernel(const float* __restrict__ partial, float* __restrict__ out,
+__global__ void __launch_bounds__(256) colsum_tall_kernel(const float* partial, float* __restrict__ out,
                                                           int parts, int cols, int accumulate) {
   np::pdl_begin();
   __shared__ float red[8][33];
@@ -423,7 +423,7 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
 }
 
 // gu = [gate | up] rows of 2F; h = act(gate) * up
-__global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h,
+__global__ void glu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ h,
                                long long rows, int F, int act) {
   np::pdl_begin();
   const long long nvec = rows * (F >> 3);
@@ -440,7 +440,7 @@ __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat
   }
 }
 
-__global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dh,
+__global__ void glu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* dh,
                                __nv_bfloat16* __restrict__ dgu, long long rows, int F, int act) {
   np::pdl_begin();
   const long long nvec = rows * (F >> 3);
@@ -475,9 +475,9 @@ __global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_
 // x: [T, H, hd] viewed with row stride ld (elements) and head stride hd; half-split rotation on
 // the first rot dims: out[i] = x[i]*cos - x[i+rot/2]*sin ; out[i+rot/2] = x[i+rot/2]*cos + x[i]*sin.
 // sign = -1 gives the inverse rotation (the backward pass). pos = pos_ids ? pos_ids[t] : t % S + off.
-__global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out,
-                            const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                            const int* __restrict__ pos_ids, long long T, int S, int pos_off, int H, int hd,
+__global__ void rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ out,
+                            const float* cos_t, const float* sin_t,
+                            const int* pos_ids, long long T, int S, int pos_off, int H, int hd,
                             int rot, long long ld_in, long long ld_out, float sign) {
   np::pdl_begin();
   const int half = rot >> 1;
@@ -528,8 +528,8 @@ struct HeadSrc {
 // thread's for all tokens of its CTA (one thread per pair where they fit a block), two tokens in flight: the head and
 // stride arithmetic per token cost as much as the copies (4096 tokens x 32 heads of 128: 18.6 us).
 __global__ void __launch_bounds__(1024) qkv_rope_kernel(HeadSrc s0, HeadSrc s1, HeadSrc s2, __nv_bfloat16* __restrict__ out,
-                                                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                        const int* __restrict__ pos_ids, long long T, int S, int pos_off,
+                                                        const float* cos_t, const float* sin_t,
+                                                        const int* pos_ids, long long T, int S, int pos_off,
                                                         int hd, int rot, int rot_heads, float sign) {
   np::pdl_begin();
   const int H = s0.heads + s1.heads + s2.heads;
@@ -610,10 +610,10 @@ __device__ __forceinline__ float group8_sum(float v, unsigned mask) {
 }
 
 __global__ void __launch_bounds__(256) qkv_norm_rope_fwd_kernel(
-    const __nv_bfloat16* __restrict__ qkv, long long row_stride, int hq, int hkv, const float* __restrict__ gq,
-    const float* __restrict__ bq, const float* __restrict__ gk, const float* __restrict__ bk, float eps,
-    __nv_bfloat16* __restrict__ out, float2* __restrict__ stats, const float* __restrict__ cos_t,
-    const float* __restrict__ sin_t, const int* __restrict__ pos_ids, long long T, int S, int pos_off) {
+    const __nv_bfloat16* qkv, long long row_stride, int hq, int hkv, const float* gq,
+    const float* bq, const float* gk, const float* bk, float eps,
+    __nv_bfloat16* __restrict__ out, float2* __restrict__ stats, const float* cos_t,
+    const float* sin_t, const int* pos_ids, long long T, int S, int pos_off) {
   np::pdl_begin();
   constexpr int HD = 128, HALF = 64;
   const int nrot = hq + hkv, H = hq + 2 * hkv;
@@ -667,10 +667,10 @@ __global__ void __launch_bounds__(256) qkv_norm_rope_fwd_kernel(
 // (a thread keeps its (head, slice) across tokens), summed over the heads of a kind in shared memory and written as
 // one partial row [4 x 128] per CTA (dgamma_q, dbeta_q, dgamma_k, dbeta_k).
 __global__ void __launch_bounds__(256) qkv_norm_rope_bwd_kernel(
-    HeadSrc s0, HeadSrc s1, HeadSrc s2, const __nv_bfloat16* __restrict__ qkv, long long row_stride, int hq, int hkv,
-    const float* __restrict__ gq, const float* __restrict__ gk, const float2* __restrict__ stats,
-    __nv_bfloat16* __restrict__ dqkv, float* __restrict__ partial, const float* __restrict__ cos_t,
-    const float* __restrict__ sin_t, const int* __restrict__ pos_ids, long long T, int S, int pos_off) {
+    HeadSrc s0, HeadSrc s1, HeadSrc s2, const __nv_bfloat16* qkv, long long row_stride, int hq, int hkv,
+    const float* gq, const float* gk, const float2* stats,
+    __nv_bfloat16* __restrict__ dqkv, float* __restrict__ partial, const float* cos_t,
+    const float* sin_t, const int* pos_ids, long long T, int S, int pos_off) {
   np::pdl_begin();
   constexpr int HD = 128, HALF = 64;
   __shared__ float s_acc[4][HD];
@@ -798,8 +798,8 @@ __global__ void rope_table_kernel(float* __restrict__ cos_t, float* __restrict__
 
 // ------------------------------------------------------------------ cross-entropy
 // Row-wise: lse[r] = logsumexp(logits[r]), loss[r] = lse - logits[r, label] (0 if label == ignore).
-__global__ void __launch_bounds__(NT) xent_fwd_kernel(const __nv_bfloat16* __restrict__ logits,
-                                                      const long long* __restrict__ labels,
+__global__ void __launch_bounds__(NT) xent_fwd_kernel(const __nv_bfloat16* logits,
+                                                      const long long* labels,
                                                       float* __restrict__ loss, float* __restrict__ lse,
                                                       int rows, int V, long long ld, long long ignore) {
   np::pdl_begin();
@@ -837,8 +837,8 @@ __global__ void __launch_bounds__(NT) xent_fwd_kernel(const __nv_bfloat16* __res
 // mean[0] = sum(loss) / n and inv[0] = 1 / n, n the number of labels other than `ignore` (at least one). One block, sums in a
 // fixed order, in 64 bits: the eight launches of a few microseconds that count, clamp, convert, invert and add otherwise.
 constexpr int MEAN_THREADS = 1024;
-__global__ void __launch_bounds__(MEAN_THREADS) xent_mean_kernel(const float* __restrict__ loss,
-                                                                 const long long* __restrict__ labels,
+__global__ void __launch_bounds__(MEAN_THREADS) xent_mean_kernel(const float* loss,
+                                                                 const long long* labels,
                                                                  float* __restrict__ mean, float* __restrict__ inv, int rows,
                                                                  long long ignore) {
   np::pdl_begin();
@@ -871,9 +871,9 @@ constexpr int XT = 512;   // threads of the backward
 // dlogits[r, c] = (exp(logits - lse) - [c == label]) * gscale[0] * inv_count[0]; ignored rows -> 0. Four vectors in flight
 // per thread: 4096 x 32000 119 -> 94 us (floor 80). Holding a whole row in registers, so that the forward reads it once, was
 // slower than its two reads with the second from L1 and L2 (70 -> 108 us).
-__global__ void __launch_bounds__(XT) xent_bwd_kernel(const __nv_bfloat16* __restrict__ logits,
-                                                      const long long* __restrict__ labels, const float* __restrict__ lse,
-                                                      const float* __restrict__ gscale, const float* __restrict__ inv_count,
+__global__ void __launch_bounds__(XT) xent_bwd_kernel(const __nv_bfloat16* logits,
+                                                      const long long* labels, const float* lse,
+                                                      const float* gscale, const float* inv_count,
                                                       __nv_bfloat16* __restrict__ dlogits, int rows, int V, long long ld,
                                                       long long ignore) {
   np::pdl_begin();
@@ -915,10 +915,10 @@ __global__ void __launch_bounds__(XT) xent_bwd_kernel(const __nv_bfloat16* __res
 // ------------------------------------------------------------------ AdamW + norms
 // Decoupled weight decay on fp32 masters; writes the bf16 compute copy in the same pass.
 // gscale (device scalar, may be null) multiplies the gradient (gradient clipping coefficient).
-__global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
+__global__ void adamw_kernel(float* __restrict__ p, const float* g, float* __restrict__ m,
                              float* __restrict__ v, __nv_bfloat16* __restrict__ w16, long long n, float lr,
                              float b1, float b2, float eps, float wd, float bc1, float bc2,
-                             const float* __restrict__ gscale, const float* __restrict__ hyper) {
+                             const float* gscale, const float* hyper) {
   np::pdl_begin();
   const float gs = gscale ? gscale[0] : 1.f;
   if (hyper) { lr = hyper[0]; bc1 = hyper[1]; bc2 = hyper[2]; }  // device-resident schedule (graph replay)
@@ -955,7 +955,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g,
 }
 
 // partial[b] = sum over this CTA's grid-stride slice of x^2 (fp32 input)
-__global__ void __launch_bounds__(NT) sumsq_kernel(const float* __restrict__ x, long long n,
+__global__ void __launch_bounds__(NT) sumsq_kernel(const float* x, long long n,
                                                    float* __restrict__ partial) {
   np::pdl_begin();
   __shared__ float red[32];
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const float* __restrict__ x, 
 }
 
 // out[0] = min(1, max_norm / (sqrt(sum(partial) + extra_sq[0]) + 1e-6)); out[1] = the norm.
-__global__ void clip_coef_kernel(const float* __restrict__ partial, int parts, const float* __restrict__ extra_sq,
+__global__ void clip_coef_kernel(const float* partial, int parts, const float* extra_sq,
                                  float max_norm, float* __restrict__ out) {
   np::pdl_begin();
   __shared__ float red[32];
@@ -988,7 +988,7 @@ __global__ void clip_coef_kernel(const float* __restrict__ partial, int parts, c
   }
 }
 
-__global__ void cast_f32_to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+__global__ void cast_f32_to_bf16_kernel(const float* x, __nv_bfloat16* __restrict__ y, long long n) {
   np::pdl_begin();
   const long long nvec = n >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
@@ -1217,8 +1217,8 @@ NP_API int np_sumsq(const float* x, long long n, float* partial, void* stream) {
 // Embedding backward straight into the fp32 gradient arena: grad[ids[t], :] += dy[t, :]. One thread per four
 // columns of a token row, one 16-byte vector reduction each; rows of ids outside [0, V) are skipped.
 namespace {
-__global__ void __launch_bounds__(256) embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                            const long long* __restrict__ ids, float* __restrict__ grad,
+__global__ void __launch_bounds__(256) embedding_bwd_kernel(const __nv_bfloat16* dy,
+                                                            const long long* ids, float* __restrict__ grad,
                                                             long long T, int D, long long V) {
   np::pdl_begin();
   const int vec_per_row = D >> 2;

@@ -196,11 +196,11 @@ __device__ __forceinline__ void scale_bias(const GemmParams& p, uint32_t* r, int
   if (p.bias) {   // the same 32 values for every row of the warp: broadcast loads
     if (col + 32 <= p.N) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(p.bias + col + i));
+      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + p.bias[col + i]);
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (col + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(p.bias + col + i));
+        if (col + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + p.bias[col + i]);
     }
   }
 }

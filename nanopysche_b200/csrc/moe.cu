@@ -39,8 +39,8 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 // gate vector read from L1 serves all of them: with one token per warp the gate reads (64 KB per token at d 2048, 8 experts)
 // were the kernel's time (4096 tokens: 21 us). Every token's sum is formed in the same order whatever TOK is.
 template <int EB, int TOK>
-__global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ wg,
-                                                            const float* __restrict__ bias, float* __restrict__ logits, int T,
+__global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* x, const float* wg,
+                                                            const float* bias, float* __restrict__ logits, int T,
                                                             int D, int E, int* __restrict__ zero, int n_zero) {
   np::pdl_begin();
   // what the kernel behind this one adds to (a fill of its own is a launch)
@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16*
         for (int e = 0; e < EB; ++e) {
           if (e0 + e < E) {
             const float* wp = wg + (size_t)(e0 + e) * D + d;
-            const float4 w0 = __ldg(reinterpret_cast<const float4*>(wp));
-            const float4 w1 = __ldg(reinterpret_cast<const float4*>(wp + 4));
+            const float4 w0 = *reinterpret_cast<const float4*>(wp);
+            const float4 w1 = *reinterpret_cast<const float4*>(wp + 4);
 #pragma unroll
             for (int k = 0; k < TOK; ++k)
               acc[k][e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16*
 // One thread per token. gating: 0 softmax over the selected logits, 1 sigmoid + renormalise.
 // stats: counts[E] (int), psum[E] (sum of full-softmax probabilities), zsum[1] (sum of lse^2).
 template <int EMAX>
-__global__ void __launch_bounds__(256) router_topk_kernel(const float* __restrict__ logits,
-                                                          const float* __restrict__ score_bias,
+__global__ void __launch_bounds__(256) router_topk_kernel(const float* logits,
+                                                          const float* score_bias,
                                                           float* __restrict__ weights, int* __restrict__ indices,
                                                           int* __restrict__ counts, float* __restrict__ psum,
                                                           float* __restrict__ zsum, int T, int E, int K,
@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
 
 // f[e] = counts[e] / T and aux = E * sum_e f[e] * psum[e] / T + coef_z * zsum / T (one warp); NaN without tokens, the mean of
 // nothing
-__global__ void __launch_bounds__(32) router_aux_kernel(const int* __restrict__ counts, const float* __restrict__ psum,
-                                                        const float* __restrict__ zsum, float coef_z, float* __restrict__ f,
+__global__ void __launch_bounds__(32) router_aux_kernel(const int* counts, const float* psum,
+                                                        const float* zsum, float coef_z, float* __restrict__ f,
                                                         float* __restrict__ aux, int T, int E) {
   np::pdl_begin();
   float s = 0.f;
@@ -208,13 +208,13 @@ __global__ void __launch_bounds__(32) router_aux_kernel(const int* __restrict__ 
 // dlogits[t, :] from d(weights) and d(aux): aux = coef_lb * E * sum_i f_i * mean_t p[t,i]
 //                                                + coef_z * mean_t lse_t^2
 // f (fractions, [E]) is treated as a constant, as autograd does for the reference's one_hot count.
-__global__ void __launch_bounds__(256) router_bwd_kernel(const float* __restrict__ logits,
-                                                         const float* __restrict__ score_bias,
-                                                         const float* __restrict__ weights,
-                                                         const int* __restrict__ indices,
-                                                         const float* __restrict__ dweights,
-                                                         const float* __restrict__ f,
-                                                         const float* __restrict__ daux, float coef_lb,
+__global__ void __launch_bounds__(256) router_bwd_kernel(const float* logits,
+                                                         const float* score_bias,
+                                                         const float* weights,
+                                                         const int* indices,
+                                                         const float* dweights,
+                                                         const float* f,
+                                                         const float* daux, float coef_lb,
                                                          float coef_z, float* __restrict__ dlogits, int T, int E,
                                                          int K, int gating) {
   np::pdl_begin();
@@ -268,8 +268,8 @@ __global__ void __launch_bounds__(256) router_bwd_kernel(const float* __restrict
 // token lanes; a lane walks every fourth token of the chunk with four row loads in flight, the lanes are summed
 // through shared memory.
 template <int EB>
-__global__ void __launch_bounds__(256) router_dgate_kernel(const float* __restrict__ dl,
-                                                           const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256) router_dgate_kernel(const float* dl,
+                                                           const __nv_bfloat16* x,
                                                            float* __restrict__ partial, int T, int D, int E,
                                                            int chunk) {
   np::pdl_begin();
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) router_dgate_kernel(const float* __restri
 #pragma unroll
           for (int e = 0; e < EB; ++e) {
             if (e0 + e < E) {
-              const float g = __ldg(dl + (size_t)(tb + 4 * u) * E + e0 + e);
+              const float g = dl[(size_t)(tb + 4 * u) * E + e0 + e];
 #pragma unroll
               for (int j = 0; j < 8; ++j) acc[e][j] += g * xv[j];
             }
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256) router_dgate_kernel(const float* __restri
 
 // dx[t, :] = sum_e dl[t, e] * Wg[e, :] in bf16: the router's contribution to the gradient of its input (a
 // [T, E] x [E, D] product with E of 8 to 64: one thread per 8 output columns, the gate rows come from L1).
-__global__ void __launch_bounds__(256) router_dx_kernel(const float* __restrict__ dl, const float* __restrict__ wg,
+__global__ void __launch_bounds__(256) router_dx_kernel(const float* dl, const float* wg,
                                                         __nv_bfloat16* __restrict__ dx, int T, int D, int E) {
   np::pdl_begin();
   const int vec_per_row = D >> 3;
@@ -358,9 +358,9 @@ __global__ void __launch_bounds__(256) router_dx_kernel(const float* __restrict_
     const int t = (int)(i / vec_per_row), d = (int)(i % vec_per_row) * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int e = 0; e < E; ++e) {
-      const float g = __ldg(dl + (size_t)t * E + e);
-      const float4 w0 = __ldg(reinterpret_cast<const float4*>(wg + (size_t)e * D + d));
-      const float4 w1 = __ldg(reinterpret_cast<const float4*>(wg + (size_t)e * D + d + 4));
+      const float g = dl[(size_t)t * E + e];
+      const float4 w0 = *reinterpret_cast<const float4*>(wg + (size_t)e * D + d);
+      const float4 w1 = *reinterpret_cast<const float4*>(wg + (size_t)e * D + d + 4);
       acc[0] += g * w0.x; acc[1] += g * w0.y; acc[2] += g * w0.z; acc[3] += g * w0.w;
       acc[4] += g * w1.x; acc[5] += g * w1.y; acc[6] += g * w1.z; acc[7] += g * w1.w;
     }
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(256) router_dx_kernel(const float* __restrict_
 // Same product for E <= 8 with D = 8 * blockDim.x: a thread keeps its 8 columns of all gate rows in registers and
 // walks TOK tokens, so the only memory traffic per token is the [E] gradient row (broadcast) and one 16-byte store.
 template <int TOK>
-__global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* __restrict__ dl, const float* __restrict__ wg,
+__global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* dl, const float* wg,
                                                             __nv_bfloat16* __restrict__ dx, int T, int D, int E) {
   np::pdl_begin();
   const int d = threadIdx.x * 8;
@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* __restr
   for (int e = 0; e < 8; ++e) {
     float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f), w1 = w0;
     if (e < E) {
-      w0 = __ldg(reinterpret_cast<const float4*>(wg + (size_t)e * D + d));
-      w1 = __ldg(reinterpret_cast<const float4*>(wg + (size_t)e * D + d + 4));
+      w0 = *reinterpret_cast<const float4*>(wg + (size_t)e * D + d);
+      w1 = *reinterpret_cast<const float4*>(wg + (size_t)e * D + d + 4);
     }
     w[e][0] = w0.x; w[e][1] = w0.y; w[e][2] = w0.z; w[e][3] = w0.w;
     w[e][4] = w1.x; w[e][5] = w1.y; w[e][6] = w1.z; w[e][7] = w1.w;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* __restr
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float g = e < E ? __ldg(dl + (size_t)t * E + e) : 0.f;
+      const float g = e < E ? dl[(size_t)t * E + e] : 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += g * w[e][j];
     }
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* __restr
   }
 }
 
-__global__ void colsum2_kernel(const float* __restrict__ partial, float* __restrict__ out, int parts,
+__global__ void colsum2_kernel(const float* partial, float* __restrict__ out, int parts,
                                long long cols, int accumulate) {
   np::pdl_begin();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -419,7 +419,7 @@ __global__ void colsum2_kernel(const float* __restrict__ partial, float* __restr
 }
 
 // out[c] (+)= sum over rows of a[r, c] for a narrow matrix (cols <= 64): 1024 threads, thread -> (row group, col)
-__global__ void __launch_bounds__(1024) colsum_narrow_kernel(const float* __restrict__ a, float* __restrict__ out,
+__global__ void __launch_bounds__(1024) colsum_narrow_kernel(const float* a, float* __restrict__ out,
                                                              int rows, int cols, int accumulate) {
   np::pdl_begin();
   __shared__ float red[1024];
@@ -499,7 +499,7 @@ __device__ __forceinline__ U64x4 block_excl_scan4(const U64x4& v, int nw_used, U
 }
 
 template <int FB>   // bits per counter: 16 or 32
-__global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* __restrict__ indices, int T, int E, int K,
+__global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* indices, int T, int E, int K,
                                                              int capacity, int* __restrict__ slot_pos,
                                                              int* __restrict__ keep, int* __restrict__ counts_kept,
                                                              int* __restrict__ drops, int* __restrict__ n_dropped,
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* __restri
   const int* idx = indices;
   if (use_smem) {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < T * K; i += blockDim.x) s_idx[i] = __ldg(indices + i);   // several loads in flight
+    for (int i = threadIdx.x; i < T * K; i += blockDim.x) s_idx[i] = indices[i];   // several loads in flight
     for (int t = threadIdx.x; t < T; t += blockDim.x) s_keep[t] = 1;
     idx = s_idx;
   } else {
@@ -855,9 +855,9 @@ __global__ void __launch_bounds__(256) ep_combine_kernel(const CombineParams p) 
 }
 
 // dots[t, k] = <a[t, :], rows[t*K + k, :]>  (0 for dropped slots); one warp per slot.
-__global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* __restrict__ a,
-                                                       const __nv_bfloat16* __restrict__ rows,
-                                                       const int* __restrict__ slot_pos, float* __restrict__ dots,
+__global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* a,
+                                                       const __nv_bfloat16* rows,
+                                                       const int* slot_pos, float* __restrict__ dots,
                                                        int T, int K, int D) {
   np::pdl_begin();
   const int lane = threadIdx.x & 31;

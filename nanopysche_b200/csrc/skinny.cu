@@ -35,7 +35,7 @@ __device__ __forceinline__ uint4 ld16(const __nv_bfloat16* row, int k, int K) {
 __device__ __forceinline__ uint4 ld16_stream(const __nv_bfloat16* row, int k, int K) {   // read once: do not keep in L1
   uint4 v = make_uint4(0, 0, 0, 0);
   if (k < K)
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(row + k));
   return v;
 }
