@@ -816,6 +816,11 @@ __global__ void __launch_bounds__(256) ep_combine_kernel(const CombineParams p) 
         q[u] = make_uint4(0, 0, 0, 0);
         w[u] = 0.f;
         if (on[u]) {
+          on[u] = false;   // debug build: a position out of range is reported and its row left out
+          NP_DBG_SKIP_UNLESS(p.slot_pos[slot] < (1 << 24), KID_COMBINE, p.slot_pos[slot])
+          on[u] = true;
+        }
+        if (on[u]) {
           q[u] = *reinterpret_cast<const uint4*>(p.rows + slot * p.D + d);
           w[u] = p.weights ? p.weights[slot] : 1.f;
         }
