@@ -53,7 +53,7 @@ def _newest_header_mtime() -> float:
 
 
 def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool) -> tuple[str, int, str]:
-    extra = os.environ.get("NPB200_NVCC_EXTRA", "").split()   # e.g. -DNP_ATTN_PROF for a development build
+    extra = os.environ.get("NPB200_NVCC_EXTRA", "").split()   # e.g. -DNP_DEBUG, the bounds-checking build
     cmd = [nvcc, *NVCC_FLAGS, *extra, "-I", str(src.parent), "-I", str(CSRC), "-c", str(src), "-o", str(obj)]
     if verbose:
         cmd[1:1] = ["-Xptxas", "-v"]

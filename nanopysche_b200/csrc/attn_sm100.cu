@@ -160,28 +160,11 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// 2^x on the FMA pipe (degree-4 polynomial on the fraction, exponent patched in with integer adds; relative error
-// about 4e-5, 0 below 2^-125): used for a share of the scores so that the special-function unit is not the only
-// pipe the exp2 phase runs on
-__device__ __forceinline__ float ex2_poly(float x) {
-  const bool tiny = x < -125.f;              // masked scores (-inf) must give exactly 0
-  x = fmaxf(x, -125.f);
-  const float t = x + 12582912.f;            // 1.5 * 2^23: the integer part lands in the low mantissa bits
-  const float f = x - (t - 12582912.f);      // [-0.5, 0.5]
-  float p = fmaf(f, 0.0096181291f, 0.0555041087f);
-  p = fmaf(p, f, 0.2402265070f);
-  p = fmaf(p, f, 0.6931471806f);
-  p = fmaf(p, f, 1.0f);
-  return tiny ? 0.f : __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
-}
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-#ifndef NP_FWD2_POLY
-#define NP_FWD2_POLY 0   // 1: every fourth score of the two-Q-tile forward goes through ex2_poly (measured: 1.4x slower)
-#endif
 // mbarrier wait whose outcome is the same for every lane of the warp, so that the .sync.aligned tensor-memory
 // instructions that follow are never reached by part of a warp
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int kid, int where) {
@@ -523,14 +506,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // after the P V that read P.
 enum { G_Q = 0, G_K = 1, G_KE = 4, G_V = 7, G_VE = 9, G_S = 11, G_P = 13, G_O = 15, G_P2 = 17, G_COUNT = 19 };
 constexpr int P_FIRST = 3;   // quarters of P that are handed over as soon as they are stored (G_P), the rest follows (G_P2)
-#ifdef NP_ATTN_PROF   // development build only: cycles per softmax phase, summed over (lane 0 of) all warps
-__device__ unsigned long long g_fwd2_prof[8];
-#define PROF_T(v) const long long v = clock64()
-#define PROF_ADD(i, a, b) do { if (lane == 0) atomicAdd(&g_fwd2_prof[i], (unsigned long long)((b) - (a))); } while (0)
-#else
-#define PROF_T(v) do {} while (0)
-#define PROF_ADD(i, a, b) do {} while (0)
-#endif
 constexpr int G_KST = 3, G_VST = 2;   // Q0, Q1, three K stages, two V stages: seven 32 KB tiles
 
 template <int HD>
@@ -695,14 +670,11 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int kp0 = i * BKV;
       const int valid_cols = p.src_len - kp0;
       const bool need_mask = (p.causal && kp0 + BKV - 1 > q_pos_first) || valid_cols < BKV;
-      PROF_T(c0);
       ok = ok && !*abort_flag && warp_wait(B_(G_S + t), (uint32_t)i & 1u, abort_flag, KID_ATTN, 28);
       if (!ok) break;
       np::tc_fence_after();
-      PROF_T(c1);
       uint32_t s[128];
       tmem_ld_cols<128>(tS, s);
-      PROF_T(c2);
       if (need_mask) {
 #pragma unroll
         for (int e = 0; e < 128; ++e)
@@ -737,7 +709,6 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         l *= alpha;
         m = m_new;
       }
-      PROF_T(c3);
       const float m_use = (m == -INFINITY) ? 0.f : m;
       float rs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -748,7 +719,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const float x0 = fmaf(__uint_as_float(s[c * 32 + e]), p.scale_log2, -m_use);
           const float x1 = fmaf(__uint_as_float(s[c * 32 + e + 1]), p.scale_log2, -m_use);
           const float p0 = ex2(x0);
-          const float p1 = (NP_FWD2_POLY && (e & 2)) ? ex2_poly(x1) : ex2(x1);
+          const float p1 = ex2(x1);
           rs[e & 2] += p0;
           rs[(e & 2) + 1] += p1;
           pk[e >> 1] = np::pack_bf16(p0, p1);
@@ -762,14 +733,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       l += (rs[0] + rs[1]) + (rs[2] + rs[3]);
-      PROF_T(c4);
       tmem_st_wait();
       np::tc_fence_before();
       __syncwarp();
       if (lane == 0) np::mbar_arrive(B_(G_P2 + t));
-      PROF_T(c5);
-      PROF_ADD(0, c0, c1); PROF_ADD(1, c1, c2); PROF_ADD(2, c2, c3); PROF_ADD(3, c3, c4); PROF_ADD(4, c4, c5);
-      PROF_ADD(5, c0, c0 + 1);
     }
     ok = ok && !*abort_flag;
     if (ok && my_nv > 0) ok = warp_wait(B_(G_O + t), (uint32_t)(my_nv - 1) & 1u, abort_flag, KID_ATTN, 30);
@@ -880,14 +847,6 @@ struct NpAttnFwdArgs {
   int push_n; int* push_ctr;
   int head_dim;    // 128 (also when 0) or 64
 };
-
-#ifdef NP_ATTN_PROF
-NP_API int np_attn_prof_read(unsigned long long* out8, int reset) {
-  cudaMemcpyFromSymbol(out8, g_fwd2_prof, sizeof(unsigned long long) * 8);
-  if (reset) { unsigned long long z[8] = {0}; cudaMemcpyToSymbol(g_fwd2_prof, z, sizeof(z)); }
-  return 0;
-}
-#endif
 
 // a kernel of 20 us and more
 static bool busy(int B, int H, int Sq, int Sk, int hd) { return 4.0 * B * H * Sq * (double)Sk * hd > 2e10; }
