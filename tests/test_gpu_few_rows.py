@@ -71,12 +71,19 @@ def test_attention_with_appended_cache(B, S, P, Hq, Hkv, causal, hd):
 def test_append_under_grad_takes_the_differentiable_path():
     from nanopysche_b200.ops.attention import attention_append
 
-    q = torch.randn(1, 1, 4, 64, device="cuda").bfloat16().requires_grad_(True)
-    k, v = (torch.randn(1, 40, 4, 64, device="cuda").bfloat16() for _ in range(2))
-    kn, vn = (torch.randn(1, 1, 4, 64, device="cuda").bfloat16() for _ in range(2))
-    o, ko, _ = attention_append(q, k, v, kn, vn)
-    o.sum().backward()
-    assert q.grad is not None and ko.shape[1] == 41
+    torch.manual_seed(4)
+    leaves = [torch.randn(2, n, h, 64, device="cuda").bfloat16().requires_grad_(True)
+              for n, h in ((1, 4), (40, 2), (40, 2), (1, 2), (1, 2))]
+    o, ko, vo = attention_append(*leaves)
+    g = torch.randn_like(o)
+    o.backward(g)
+    l64 = [t.detach().double().requires_grad_(True) for t in leaves]
+    q, k, v, kn, vn = l64
+    ref = _sdpa64(q, torch.cat([k, kn], 1), torch.cat([v, vn], 1), True)
+    ref.backward(g.double())
+    assert rel(o, ref) < 6e-3 and torch.equal(ko, torch.cat(leaves[1::2], 1)) and torch.equal(vo, torch.cat(leaves[2::2], 1))
+    for a, b in zip(leaves, l64):
+        assert rel(a.grad, b.grad) < 6e-3
 
 
 def test_append_does_not_drop_tangents():

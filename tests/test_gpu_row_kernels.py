@@ -86,7 +86,9 @@ def test_qkv_rope_shapes(B, S, hq, hkv, hd, rot):
     torch.autograd.backward([q, k, v], [gq, gk, gv])
     torch.autograd.backward([r[:, :, :hq], r[:, :, hq:hq + hkv], h[:, :, hq + hkv:]], [gq.double(), gk.double(), gv.double()])
     assert rel(qkv.grad, x.grad) < 4e-3
-    assert apply_rope_ref(q, cos, sin, 5).shape == q.shape
+    one = torch.cat([qkv.detach()[..., :hq * hd].unflatten(-1, (hq, hd))[:, :, :1]] * 2, 2)     # the framework's reference too
+    ref = apply_rope_ref(one, cos, sin, 5)
+    assert rel(ref[:, :, 0], q[:, :, 0]) < 4e-3 and torch.equal(ref[:, :, 0], ref[:, :, 1])
 
 
 # below and above the four-tokens-per-warp switch, T off it, experts off a block of eight, D off a warp's 256
@@ -187,21 +189,37 @@ def test_every_dispatch_starts_the_push_counters_anew(fp8):
     _lib.check_status("after test")
 
 
-@pytest.mark.parametrize("T,cap,ranks", [(1, -1, 1), (700, 150, 2), (4096, 1280, 4)])
-def test_capacity_plan_matches_the_scan(T, cap, ranks):
+def _plan(idx, E, cap):
+    """The capacity rule on the host: a slot's position is its rank among the kept slots of its expert in token order; a token
+    that any of its experts has no room for is dropped as a whole."""
+    T, K = idx.shape
+    hit = torch.zeros(T, E, dtype=torch.bool).scatter_(1, idx.long(), True)
+    over = hit & (hit.cumsum(0) > cap) if cap >= 0 else torch.zeros_like(hit)
+    keep = ~over.any(1)
+    kept = hit & keep[:, None]
+    pos = (kept.cumsum(0) - 1).gather(1, idx.long())
+    pos[~keep] = -1
+    return pos, keep, kept.sum(0), over.sum(0), (~keep).sum()
+
+
+# the counters of the scan, in shared memory and (above 200 KB of indices) in memory, 16 and 32 bits wide
+@pytest.mark.parametrize("T,cap,ranks", [(1, -1, 1), (1, 0, 1), (700, 150, 2), (4096, 1280, 4), (4096, -1, 8), (30000, 7000, 1),
+                                         (70000, -1, 2), (70000, 20000, 4)])
+def test_capacity_plan(T, cap, ranks):
     from nanopysche_b200.ops import _lib
 
     E, K = 8, 2
     torch.manual_seed(T)
     idx = torch.rand(T, E, device="cuda").topk(K, -1).indices.to(torch.int32)
-    a, b = ([torch.full(s, -7, device="cuda", dtype=torch.int32) for s in ((T, K), (T,), (E,), (E,), (1,))] for _ in range(2))
-    _lib.call("capacity_scan", idx, T, E, K, cap, *a)
+    got = [torch.full(s, -7, device="cuda", dtype=torch.int32) for s in ((T, K), (T,), (E,), (E,), (1,))]
     sent = torch.empty(ranks, device="cuda", dtype=torch.int32)
     stats = torch.tensor([9, 100, 1000], device="cuda")
-    _lib.call("capacity_plan", idx, T, E, K, cap, *b, sent, ranks, stats)
-    assert all(torch.equal(x, y) for x, y in zip(a, b))
-    assert torch.equal(sent, a[2].view(ranks, -1).sum(1).to(torch.int32))
-    d = a[4].item()
+    _lib.call("capacity_plan", idx, T, E, K, cap, *got, sent, ranks, stats)
+    want = _plan(idx.cpu(), E, cap)
+    for g, w in zip(got, want):
+        assert torch.equal(g.cpu().long().reshape(w.shape), w.long())
+    assert torch.equal(sent.cpu().long(), want[2].view(ranks, -1).sum(1))
+    d = want[4].item()
     assert stats.tolist() == [d, 100 + d, 1000 + T]
 
 
