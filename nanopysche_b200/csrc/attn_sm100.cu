@@ -1,10 +1,11 @@
-// Flash attention for sm_100a (head_dim 128, bf16, causal or full, GQA-native), forward and backward,
+// Flash attention for sm_100a (head_dim 128 or 64, bf16, causal or full, GQA-native), forward and backward,
 // on tcgen05 tensor cores: S = Q K^T and O += P V (and the five backward products) are tcgen05.mma with
 // TMEM accumulators, Q/K/V/dO tiles arrive by 4-D TMA straight from the strided [B, S, H, hd] tensors
-// (so the q / k / v slices of the fused QKV GEMM output need no copy), softmax runs in registers on
-// eight warps that read S out of TMEM (two threads per row, 64 columns each), and P / dS go back to tensor
-// memory as bf16 and feed the next MMA as its TMEM A operand. The output accumulator stays in TMEM as well and
-// is only rescaled when a row maximum has grown by more than 2^8. Scores never touch shared or global memory.
+// (so the q / k / v slices of the fused QKV GEMM output need no copy), and softmax runs in registers on
+// eight warps that read S out of TMEM (two threads per row, 64 columns each; one thread per row in the forward
+// with two Q tiles). P (forward), dS (dQ kernel) and P^T (dK/dV kernel) go back to tensor memory as bf16 and feed
+// the next MMA as its TMEM A operand; dS^T of the dK/dV kernel goes through shared memory. The output accumulator
+// stays in TMEM and is only rescaled when a row maximum has grown by more than 2^8. Scores never reach global memory.
 //
 // K/V (forward, dQ) and Q/dO (dK/dV) may come from a *list* of tensor maps - one per context-parallel
 // rank, pointing into that rank's symmetric memory - so a sequence sharded over GPUs is attended to by
@@ -506,7 +507,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // after the P V that read P.
 enum { G_Q = 0, G_K = 1, G_KE = 4, G_V = 7, G_VE = 9, G_S = 11, G_P = 13, G_O = 15, G_P2 = 17, G_COUNT = 19 };
 constexpr int P_FIRST = 3;   // quarters of P that are handed over as soon as they are stored (G_P), the rest follows (G_P2)
-constexpr int G_KST = 3, G_VST = 2;   // Q0, Q1, three K stages, two V stages: seven 32 KB tiles
+constexpr int G_KST = 3, G_VST = 2;   // Q0, Q1, three K stages, two V stages: seven tiles of tile_bytes<HD>()
 
 template <int HD>
 __global__ void __launch_bounds__(320, 1)
@@ -938,8 +939,10 @@ NP_API int np_attn_fwd(const NpAttnFwdArgs* a, void* stream) {
 //               and every visible Q block of every source, on the transposed problem so that the
 //               operands land in TMEM lanes the way the next MMA wants them:
 //               S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q  (dV, dK stay in TMEM).
-// P and dS never leave tensor memory: they are written as bf16 over the S / dP columns they were
-// computed from and consumed as TMEM A operands.
+// dQ: dS is written as bf16 over the dP columns it was computed from and consumed as a TMEM A operand. dKV: P^T is
+// written over S^T the same way; dS^T goes to a swizzled tile in shared memory and is read there by the dK product as
+// its A operand (a proxy fence before it is handed over; KB_DSE says that the product has read it), so that its dP^T
+// columns are free for the next block.
 namespace {
 
 constexpr int KID_ATTN_DQ = 31, KID_ATTN_DKV = 32;
@@ -1012,7 +1015,7 @@ enum { QB_QDO = 0, QB_K = 1, QB_KE = 4, QB_V = 7, QB_VE = 9, QB_S = 11, QB_SR = 
 // one, every block waited for dS, dQ and dP one after the other (16 / 8 heads of 128, causal, 1 x 8192, with the
 // delta kernel: 0.385 -> 0.352 ms).
 constexpr int Q_KST = 3, Q_VST = 2;
-constexpr int BWD_TILES = 7;   // seven 32 KB tiles: the dynamic shared memory must itself start on a 1024-byte boundary
+constexpr int BWD_TILES = 2 + Q_KST + Q_VST;   // Q, dO, K and V stages; the swizzled tiles start on 1024-byte boundaries
 
 template <int NS, int HD>
 __global__ void __launch_bounds__(nthreads(NS), 1)

@@ -10,8 +10,8 @@
 // lane quarters) into tensor memory.
 //
 // CTA roles: warp 0 lane 0 issues the copies (TMA tiles of A and B, bulk copies of the scale chunks) into a
-// 5-stage ring; warp 1 lane 0 copies the scales of a stage into TMEM and issues four K = 32 MMAs whose instruction
-// descriptors select byte 0..3 of the scale words; warps 2-9 drain one of two 192-column accumulators (tcgen05.ld)
+// 5-stage ring; warp 1 walks the K steps as a whole and one elected lane of it copies the scales of a stage into TMEM
+// and issues four K = 32 MMAs whose instruction descriptors select byte 0..3 of the scale words; warps 2-9 drain one of two 192-column accumulators (tcgen05.ld)
 // while the next tile accumulates into the other. The tile is 128 x 192: two 192-column fp32 accumulators plus the
 // scale columns fit the 512 TMEM columns (two 256-column ones would leave none for the scales), and the operand
 // bytes per FLOP that cross from L2 drop by a fifth against a 128 x 128 tile. A 192-row B tile starts at row 0 or

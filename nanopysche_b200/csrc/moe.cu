@@ -893,8 +893,8 @@ __global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* a,
 NP_API int np_router_logits(const void* x, const float* wg, const float* bias, float* logits, int T, int D, int E, int* zero,
                             int n_zero, void* stream) {
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
-  // four tokens per warp once that still leaves eight warps for every SM
-  const int tok = T >= 148 * 8 * 4 / 2 ? 4 : 1;
+  // four tokens per warp once that leaves four warps for every SM (2368 tokens)
+  const int tok = T >= 148 * 4 * 4 ? 4 : 1;
   const long long warps = ((long long)T + tok - 1) / tok, blocks = (warps * 32 + 255) / 256;
   np_launch(tok == 4 ? router_logits_kernel<8, 4> : router_logits_kernel<8, 1>,
             (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
