@@ -1125,6 +1125,23 @@ int g_num_sms = 0;
 struct TileCost { double fixed, step, drain; };
 constexpr TileCost COST_128{4.4, 0.37, 0.6}, COST_256{5.3, 0.40, 0.3}, COST_PAIR{6.0, 0.30, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3},
     COST_SPLIT4{10.7, 0.30, 0.3};
+// Products of at most 64 rows. The few-row kernel: CTAs of 16 weight rows, each of which reads all of x again from the L2, so its
+// time per CTA grows with the rows it is built for (8, 16, 32, 64) and, by the loads in flight, with K. The tile kernels pad to
+// 128 rows but read x once per tile: with many columns they are bound by reading the weight. Fitted to 15 weights of 768 x 768 to
+// 128256 x 2048 at 1 to 64 rows, DRAM-cold (us, few-row / best tile): 32000 x 2048: 8 rows 27.6 / 39.9, 16 39.9 / 39.9, 32 56 / 40,
+// 64 92 / 40; 50264 x 768: 8 rows 27.6 / 29.7, 16 46 / 30; 6144 x 4096: 32 rows 27.7 / 32.9, 64 37.8 / 33.8; 4096 x 4096 and
+// narrower outputs: few-row at every count (64 rows 27.6 / 31.8, 2048 x 5632 21.5 / 41.7).
+inline double few_rows_cost(int M, int N, int K) {
+  const double ctas = (N + 15) / 16;
+  if (M <= 8) return 2.0 + ctas * (2.5e-3 + 4.0e-6 * K);
+  if (M <= 16) return 2.0 + ctas * (8.0e-3 + 5.0e-6 * K);
+  if (M <= 32) return 2.0 + ctas * (4.5e-3 + 10.5e-6 * K);
+  return 2.0 + ctas * (9.0e-3 + 15.0e-6 * K);
+}
+inline double few_tiles_cost(double tiles, int N, int K) {   // tiles: estimate without the traffic; 5.0 TB/s of weight beside 5 us
+  const double traffic = 5.0 + 2.0 * N * K / 5.0e6;
+  return tiles > traffic ? tiles : traffic;
+}
 // Clusters of four and of eight CTAs that run at once (an SM pair per two CTAs, whole clusters within a GPC)
 constexpr int CLUSTERS4 = 32, CLUSTERS8 = 14;
 }  // namespace
@@ -1374,18 +1391,14 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
   if ((a.lda % 8) || (a.ldb % 8) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15)) return 1;
   const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
                      (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
-  // A few rows: the weight is streamed once through all SMs (skinny.cu). `mt`, `bn` and `split` ask for a tile kernel.
-  if (a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && plain && a.K > 0 && a.K % 8 == 0 && a.bn == 0 && a.mt == 0 &&
-      a.split == 0 && a.max_ctas == 0 && a.alpha != 0.f)
-    return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
-                            a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
-  // Which kernel: the lowest estimate (TileCost). The pair kernel takes the forms without peer-arrival flags on B, pushes or
+  // Which tile kernel: the lowest estimate (TileCost). The pair kernel takes the forms without peer-arrival flags on B, pushes or
   // split operands; row-grouped launches only when their tables come in pairs of 128-row blocks (`paired`). K in parts is
   // for dense plain outputs with too few tiles for the SMs.
   const int nk = (a.K + BK - 1) / BK, sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
   const bool can_split = plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
   const bool can_pair = plain && sms >= 2;   // a pair needs two CTAs
   int bn = a.bn, mt = a.mt, splits = 1;
+  double best = 1e30;
   if (a.epilogue == 1) bn = 256;
   if (can_pair && bn != 128 && (mt == 2 || (mt == 0 && can_split && (a.split == 2 || a.split == 4)))) {
     bn = 256;   // asked for
@@ -1401,7 +1414,7 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
       return parts == 1 ? c.fixed + waves * (steps * c.step + c.drain) : waves * (c.fixed + steps / parts * c.step + c.drain);
     };
     const int n256 = a.epilogue == 1 ? 128 : 256;
-    double best = (a.epilogue == 1 || a.bn == 256) ? 1e30 : cost(COST_128, 128, 128, sms, 1);
+    if (a.epilogue != 1 && a.bn != 256) best = cost(COST_128, 128, 128, sms, 1);
     bn = 128;
     auto take = [&](double c, int bn_, int mt_, int splits_) {
       if (c < best) { best = c; bn = bn_; mt = mt_; splits = splits_; }
@@ -1413,6 +1426,12 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
       take(cost(COST_SPLIT4, 256, 256, CLUSTERS8, 4), 256, 2, 4);
     }
   }
+  // A few rows of a K-major product: the kernel that streams the weight once through all SMs (skinny.cu), unless a tile kernel
+  // is expected to be faster. `mt`, `bn` and `split` ask for a tile kernel.
+  if (a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && plain && a.K > 0 && a.K % 8 == 0 && a.bn == 0 &&
+      a.mt == 0 && a.split == 0 && a.max_ctas == 0 && a.alpha != 0.f && few_rows_cost(a.M, a.N, a.K) <= few_tiles_cost(best, a.N, a.K))
+    return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
+                            a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
   if (can_split && (a.split == 2 || a.split == 4)) splits = a.split;
   if (bn == 256 && mt == 2 && can_pair) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
   if (bn == 256) return launch_gemm<256, 4, false>(a, (cudaStream_t)stream);

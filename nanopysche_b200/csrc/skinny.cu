@@ -321,7 +321,8 @@ int launch_decode(const DecodeParams& p, int parts, cudaStream_t stream) {
 
 }  // namespace
 
-// Called by np_gemm_bf16 for dense forward products of at most 64 rows (gemm_sm100.cu); K must be a multiple of 8 and the
+// Called by np_gemm_bf16 for dense forward products of at most 64 rows where it is the faster one (few_rows_cost in
+// gemm_sm100.cu); K must be a multiple of 8 and the
 // rows of x and w 16-byte aligned.
 int np_skinny_linear(const void* x, long long ldx, const void* w, long long ldw, int M, int N, int K, void* out, long long ldo,
                      int out_f32, float alpha, const float* bias, const void* cin, long long ldcin, cudaStream_t stream) {

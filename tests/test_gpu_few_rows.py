@@ -158,3 +158,19 @@ def test_flash_keys_of_a_longer_buffer(B, Hkv, hd):
         for a, b in zip(grads(kk, vv), grads(kk.clone(memory_format=torch.contiguous_format),
                                              vv.clone(memory_format=torch.contiguous_format))):
             assert torch.equal(a, b)
+
+
+# the few-row kernel reads all of x again for every 16 columns: with many columns the tile kernels take over as rows are added
+@pytest.mark.parametrize("M,N,K,few", [(1, 32000, 1024, True), (8, 32000, 1024, True), (16, 32000, 1024, False),
+                                       (64, 32000, 1024, False), (64, 2048, 2048, True), (65, 2048, 2048, False)])
+def test_few_row_kernel_where_it_is_the_faster_one(M, N, K, few):
+    from nanopysche_b200.ops.gemm import gemm
+
+    torch.manual_seed(M)
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    out = gemm(x, w)
+    assert rel(out, x.double() @ w.double().t()) < 3e-3
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        gemm(x, w, out=out)
+        torch.cuda.synchronize()
+    assert any("skinny" in e.key for e in p.key_averages()) == few
