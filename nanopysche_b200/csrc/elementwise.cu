@@ -129,16 +129,15 @@ __device__ __forceinline__ void block_sums(float* v, float* buf, int par) {
   for (int q = 0; q < R; ++q) v[q] = np::warp_sum(l < nw ? b[q * 16 + l] : 0.f);   // the order of block_sum
 }
 
-constexpr int NR = 4;   // rows that the RMSNorm backward takes at a time
-// RMSNorm backward for up to 4096 columns, four rows per CTA at a time: one 8-wide vector of each row per thread, so the
-// loads of four rows are in flight and one barrier serves four sums; the weight gradient of a thread's eight columns stays in
-// registers over all its rows (a warp per row kept it in shared memory, 16 KB of traffic per row). With the column sum,
-// 4096 x 2048: 23.5 -> 21.1 us, 16384 x 2048: 63.8 -> 56.8, 4096 x 768: 22.2 -> 15.7 (DRAM-cold, floors 10, 41 and 4). The same
+// RMSNorm backward for up to 2048 columns, NR rows per CTA at a time: one 8-wide vector of each row per thread, so the loads of
+// NR rows are in flight and one barrier serves NR sums; the weight gradient of a thread's eight columns stays in registers over
+// all its rows (a warp per row kept it in shared memory, 16 KB of traffic per row). Two rows at a time as long as every CTA then
+// takes one turn, four above. With the column sum, DRAM-cold, against a CTA per row (768 columns) or a warp per row (2048):
+// 4096 x 2048 21.4 -> 20.2 us, 1184 x 2048 13.3 -> 10.0, 64 x 2048 9.2 -> 5.1, 4096 x 768 20.6 -> 14.6, 300 x 768 6.8 -> 6.3. The same
 // form of the forward pass was slower than a CTA per row (15.1 -> 20.6): it has half the traffic to hide a barrier behind.
-__global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* dy,
-                                                               const __nv_bfloat16* x,
-                                                               const float* w, const float* rstd,
-                                                               const __nv_bfloat16* dres,
+template <int NR>
+__global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w,
+                                                               const float* rstd, const __nv_bfloat16* dres,
                                                                __nv_bfloat16* __restrict__ dx,
                                                                float* __restrict__ dw_partial, int rows, int cols) {
   np::pdl_begin();
@@ -1054,13 +1053,18 @@ static int launch_rmsnorm_bwd(const void* dy, const void* x, const float* w, con
                                cudaStream_t s) {
 #define RB(V) np_launch(rmsnorm_bwd_kernel<V>, grid, NT, 0, s, 1, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, \
                                                        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, cols)
-  // up to 4096 columns a thread holds one vector of each of four rows; wider rows take one CTA per row
-  if (cols <= 4096) {
-    // NR rows at a time, every CTA the same number of turns (at most `grid` CTAs: the scratch has a row for each)
-    const int batches = (rows + NR - 1) / NR, turns = (batches + grid - 1) / grid;
+  // up to 2048 columns a thread holds one vector of each of NR rows; wider rows take one CTA per row (4096 columns with the column
+  // sum: 17.9 us a CTA per row, 21.3 four rows at a time at 1500 rows; 35.5 and 36.8 at 4096)
+  if (cols <= 2048) {
+    // every CTA the same number of turns, at most `grid` CTAs: the scratch has a row for each
+    const int nr = rows <= 2 * grid ? 2 : 4;
+    const int batches = (rows + nr - 1) / nr, turns = (batches + grid - 1) / grid;
     grid = (batches + turns - 1) / turns;
-    np_launch(rmsnorm_bwd_rows_kernel, grid, (cols / 8 + 31) / 32 * 32, 0, s, 1, (const __nv_bfloat16*)dy,
-              (const __nv_bfloat16*)x, w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, cols);
+    np_launch(nr == 2 ? rmsnorm_bwd_rows_kernel<2> : rmsnorm_bwd_rows_kernel<4>, grid, (cols / 8 + 31) / 32 * 32, 0, s, 1,
+              (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch,
+              rows, cols);
+  } else if (cols <= NT * 16) {
+    RB(2);
   } else {
     RB(4);
   }

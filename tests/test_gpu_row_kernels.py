@@ -10,8 +10,10 @@ def rel(a, b):
     return ((a.double() - b.double()).norm() / (b.double().norm() + 1e-30)).item()
 
 
-# rows off the four-row batches and fewer than one, columns off a warp's 256
-@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 768), (5, 2048), (1023, 1032), (1187, 4096), (2600, 768), (9, 6144)])
+# rows off the two- and four-row batches and fewer than one, both sides of the switch between them (592 rows) and of the one
+# to a CTA per row (2048 columns), columns off a warp's 256
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 768), (5, 2048), (1023, 1032), (1187, 4096), (2600, 768), (9, 6144),
+                                       (297, 2048), (591, 264), (593, 2040), (300, 2056), (700, 4104)])
 @pytest.mark.parametrize("res", [False, True])
 def test_rmsnorm_rows(rows, cols, res):
     from nanopysche_b200.ops.norm import rms_norm
