@@ -35,13 +35,13 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 // ------------------------------------------------------------------ router
-// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). A warp takes TOK tokens at a time, so that a
-// gate vector read from L1 serves all of them: with one token per warp the gate reads (64 KB per token at d 2048, 8 experts)
-// were the kernel's time (4096 tokens: 21 us). Every token's sum is formed in the same order whatever TOK is.
-template <int EB, int TOK>
-__global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16* x, const float* wg,
-                                                            const float* bias, float* __restrict__ logits, int T,
-                                                            int D, int E, int* __restrict__ zero, int n_zero) {
+// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). A warp takes TOK tokens at a time and has V
+// vectors of each row in flight; MINB: CTAs per SM that the register count is held to. Every token's sum is formed in the same
+// order in all forms (np_router_logits chooses). The gate rows are 64 KB per token at d 2048 and 8 experts, read through L1.
+template <int EB, int TOK, int V, int MINB>
+__global__ void __launch_bounds__(256, MINB) router_logits_kernel(const __nv_bfloat16* x, const float* wg, const float* bias,
+                                                                  float* __restrict__ logits, int T, int D, int E,
+                                                                  int* __restrict__ zero, int n_zero) {
   np::pdl_begin();
   // what the kernel behind this one adds to (a fill of its own is a launch)
   if (blockIdx.x == 0)
@@ -56,29 +56,37 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16*
       for (int k = 0; k < TOK; ++k)
 #pragma unroll
         for (int e = 0; e < EB; ++e) acc[k][e] = 0.f;
-      for (int d = lane * 8; d < D; d += 256) {
-        uint4 q[TOK];
+      for (int d0 = lane * 8; d0 < D; d0 += 256 * V) {
+        uint4 q[V][TOK];
 #pragma unroll
-        for (int k = 0; k < TOK; ++k)
-          q[k] = t0 + k < T ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + k) * D + d) : make_uint4(0, 0, 0, 0);
-        float xv[TOK][8];
+        for (int h = 0; h < V; ++h)
 #pragma unroll
-        for (int k = 0; k < TOK; ++k) {
-          const float2 a = np::unpack_bf16(q[k].x), b = np::unpack_bf16(q[k].y), c = np::unpack_bf16(q[k].z),
-                       dd = np::unpack_bf16(q[k].w);
-          xv[k][0] = a.x; xv[k][1] = a.y; xv[k][2] = b.x; xv[k][3] = b.y;
-          xv[k][4] = c.x; xv[k][5] = c.y; xv[k][6] = dd.x; xv[k][7] = dd.y;
-        }
+          for (int k = 0; k < TOK; ++k)
+            q[h][k] = t0 + k < T && d0 + h * 256 < D ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + k) * D + d0 + h * 256)
+                                                     : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int e = 0; e < EB; ++e) {
-          if (e0 + e < E) {
-            const float* wp = wg + (size_t)(e0 + e) * D + d;
-            const float4 w0 = *reinterpret_cast<const float4*>(wp);
-            const float4 w1 = *reinterpret_cast<const float4*>(wp + 4);
+        for (int h = 0; h < V; ++h) {
+          const int d = d0 + h * 256;
+          if (h > 0 && d >= D) break;
+          float xv[TOK][8];
 #pragma unroll
-            for (int k = 0; k < TOK; ++k)
-              acc[k][e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
-                           xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
+          for (int k = 0; k < TOK; ++k) {
+            const float2 a = np::unpack_bf16(q[h][k].x), b = np::unpack_bf16(q[h][k].y), c = np::unpack_bf16(q[h][k].z),
+                         dd = np::unpack_bf16(q[h][k].w);
+            xv[k][0] = a.x; xv[k][1] = a.y; xv[k][2] = b.x; xv[k][3] = b.y;
+            xv[k][4] = c.x; xv[k][5] = c.y; xv[k][6] = dd.x; xv[k][7] = dd.y;
+          }
+#pragma unroll
+          for (int e = 0; e < EB; ++e) {
+            if (e0 + e < E) {
+              const float* wp = wg + (size_t)(e0 + e) * D + d;
+              const float4 w0 = *reinterpret_cast<const float4*>(wp);
+              const float4 w1 = *reinterpret_cast<const float4*>(wp + 4);
+#pragma unroll
+              for (int k = 0; k < TOK; ++k)
+                acc[k][e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
+                             xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
+            }
           }
         }
       }
@@ -369,13 +377,26 @@ __global__ void __launch_bounds__(256) router_dx_kernel(const float* dl, const f
 }
 
 // Same product for E <= 8 with D = 8 * blockDim.x: a thread keeps its 8 columns of all gate rows in registers and
-// walks TOK tokens, so the only memory traffic per token is the [E] gradient row (broadcast) and one 16-byte store.
+// walks TOK tokens, so the only memory traffic per token is the [E] gradient row (broadcast) and one 16-byte store. The gradient
+// rows of two tokens are loaded ahead: the first ones before the gate rows, the next ones before the last ones are used.
 template <int TOK>
-__global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* dl, const float* wg,
+__global__ void __launch_bounds__(256, 2) router_dx_reg_kernel(const float* dl, const float* wg,
                                                             __nv_bfloat16* __restrict__ dx, int T, int D, int E) {
   np::pdl_begin();
-  const int d = threadIdx.x * 8;
-  float w[8][8];
+  constexpr int G = 2;
+  static_assert(TOK % G == 0, "whole groups");
+  const int d = threadIdx.x * 8, t0 = blockIdx.x * TOK;
+  float g[2][G][8], w[8][8];
+  auto load_g = [&](int c) {
+#pragma unroll
+    for (int u = 0; u < G; ++u)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int t = t0 + c * G + u;
+        g[c & 1][u][e] = t < T && e < E ? dl[(size_t)t * E + e] : 0.f;
+      }
+  };
+  load_g(0);
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f), w1 = w0;
@@ -386,19 +407,20 @@ __global__ void __launch_bounds__(256) router_dx_reg_kernel(const float* dl, con
     w[e][0] = w0.x; w[e][1] = w0.y; w[e][2] = w0.z; w[e][3] = w0.w;
     w[e][4] = w1.x; w[e][5] = w1.y; w[e][6] = w1.z; w[e][7] = w1.w;
   }
-  const int t0 = blockIdx.x * TOK;
-#pragma unroll 4
-  for (int i = 0; i < TOK; ++i) {
-    const int t = t0 + i;
-    if (t >= T) break;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float g = e < E ? dl[(size_t)t * E + e] : 0.f;
+  for (int c = 0; c < TOK / G; ++c) {
+    if (c + 1 < TOK / G) load_g(c + 1);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += g * w[e][j];
+    for (int u = 0; u < G; ++u) {
+      const int t = t0 + c * G + u;
+      if (t >= T) break;
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += g[c & 1][u][e] * w[e][j];
+      *reinterpret_cast<uint4*>(dx + (size_t)t * D + d) = pack8(acc);
     }
-    *reinterpret_cast<uint4*>(dx + (size_t)t * D + d) = pack8(acc);
   }
 }
 
@@ -893,10 +915,13 @@ __global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* a,
 NP_API int np_router_logits(const void* x, const float* wg, const float* bias, float* logits, int T, int D, int E, int* zero,
                             int n_zero, void* stream) {
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
-  // four tokens per warp once that leaves four warps for every SM (2368 tokens)
-  const int tok = T >= 148 * 4 * 4 ? 4 : 1;
-  const long long warps = ((long long)T + tok - 1) / tok, blocks = (warps * 32 + 255) / 256;
-  np_launch(tok == 4 ? router_logits_kernel<8, 4> : router_logits_kernel<8, 1>,
+  // Gate rows in L2 / in DRAM, us, one token with its gate vectors in registers as they come (127 registers, two CTAs per SM) -
+  // one token, two vectors, four CTAs per SM - four tokens (128 registers): 1024 x 2048, 8 experts 7.8 / 12.6 - 11.8 / 22.7 -
+  // 20.9 / 40.6; 3000 x 1024 12.7 / 14.3 - 10.0 / 14.8 - 13.0 / 23.1; 4096 x 2048 22.0 / 24.5 - 21.6 / 27.0 - 21.7 / 42.1;
+  // 8192 x 2048 41.2 / 44.6 - 41.6 / 47.6 - 22.2 / 44.1. The first as long as it is one wave of CTAs.
+  const bool one_wave = T <= 148 * 2 * 8, many = T >= 8192;
+  const long long warps = many ? ((long long)T + 3) / 4 : T, blocks = (warps * 32 + 255) / 256;
+  np_launch(one_wave ? router_logits_kernel<8, 1, 1, 1> : many ? router_logits_kernel<8, 4, 1, 2> : router_logits_kernel<8, 1, 2, 4>,
             (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
             logits, T, D, E, zero, n_zero);
   CHECK_LAUNCH();

@@ -93,8 +93,10 @@ def test_qkv_rope_shapes(B, S, hq, hkv, hd, rot):
     assert rel(ref[:, :, 0], q[:, :, 0]) < 4e-3 and torch.equal(ref[:, :, 0], ref[:, :, 1])
 
 
-# below and above the four-tokens-per-warp switch, T off it, experts off a block of eight, D off a warp's 256
-@pytest.mark.parametrize("T,D,E,K", [(5, 64, 4, 2), (2367, 256, 8, 2), (2371, 768, 8, 2), (4099, 2048, 12, 3)])
+# both sides of the switches between the forms (2368 and 8192 tokens), T off whole groups of tokens, experts off a block of
+# eight, D off a warp's 256 and off two of them
+@pytest.mark.parametrize("T,D,E,K", [(5, 64, 4, 2), (2367, 256, 8, 2), (2371, 768, 8, 2), (4099, 2048, 12, 3), (2368, 1032, 8, 2),
+                                     (8191, 264, 8, 2), (8193, 776, 9, 2)])
 def test_router_forward_in_one_piece(T, D, E, K):
     from nanopysche_b200.models.moe import MoERouter, MoERouterConfig
     from nanopysche_b200.ops.moe import route
