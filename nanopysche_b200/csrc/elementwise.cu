@@ -112,11 +112,12 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* x,
   }
 }
 
-// Sums of R values per thread over the block (blockDim.x a multiple of 32, at most 512). `buf`: [2][R][16] floats; callers
-// alternate `par`, so one barrier per call is enough.
+// Sums of R values per thread over groups of `width` threads (a multiple of 32; at most 16 warps in the block). `buf`:
+// [2][R][16] floats; callers alternate `par`, so one barrier per call is enough.
 template <int R>
-__device__ __forceinline__ void block_sums(float* v, float* buf, int par) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+__device__ __forceinline__ void group_sums(float* v, float* buf, int par, int width) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = width >> 5;
+  const int w0 = width == (int)blockDim.x ? 0 : threadIdx.x / width * nw;
 #pragma unroll
   for (int q = 0; q < R; ++q) v[q] = np::warp_sum(v[q]);
   float* b = buf + par * R * 16;
@@ -126,28 +127,35 @@ __device__ __forceinline__ void block_sums(float* v, float* buf, int par) {
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < R; ++q) v[q] = np::warp_sum(l < nw ? b[q * 16 + l] : 0.f);   // the order of block_sum
+  for (int q = 0; q < R; ++q) v[q] = np::warp_sum(l < nw ? b[q * 16 + w0 + l] : 0.f);   // the order of block_sum
 }
 
 // RMSNorm backward for up to 2048 columns, NR rows per CTA at a time: one 8-wide vector of each row per thread, so the loads of
 // NR rows are in flight and one barrier serves NR sums; the weight gradient of a thread's eight columns stays in registers over
 // all its rows (a warp per row kept it in shared memory, 16 KB of traffic per row). Two rows at a time as long as every CTA then
-// takes one turn, four above. With the column sum, DRAM-cold, against a CTA per row (768 columns) or a warp per row (2048):
-// 4096 x 2048 21.4 -> 20.2 us, 1184 x 2048 13.3 -> 10.0, 64 x 2048 9.2 -> 5.1, 4096 x 768 20.6 -> 14.6, 300 x 768 6.8 -> 6.3. The same
-// form of the forward pass was slower than a CTA per row (15.1 -> 20.6): it has half the traffic to hide a barrier behind.
-template <int NR>
-__global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w,
-                                                               const float* rstd, const __nv_bfloat16* dres,
-                                                               __nv_bfloat16* __restrict__ dx,
-                                                               float* __restrict__ dw_partial, int rows, int cols) {
+// takes one turn, four above; with many rows a CTA of narrow ones has several groups of threads, each with rows of its own, whose
+// weight gradients meet in shared memory (a group of 128 threads is half of what two CTAs per SM can hold: 16384 x 1024 45.1 ->
+// 33.8 us, a warp per row 33.1; 16384 x 768 41.9 -> 30.5; 16384 x 512 36.0 -> 21.3). Two CTAs per SM: with 168 registers and one,
+// 16384 x 1024 takes 46.9. With the column sum, DRAM-cold, against a CTA per row (768 columns) or a warp per row (2048):
+// 4096 x 2048 21.4 -> 20.2 us, 1184 x 2048 13.3 -> 10.0, 64 x 2048 9.2 -> 5.1, 4096 x 768 21.0 -> 12.1, 300 x 768 6.8 -> 6.3. The
+// same form of the forward pass was slower than a CTA per row (15.1 -> 20.6): it has half the traffic to hide a barrier behind.
+template <int NR, bool GROUPS>
+__global__ void __launch_bounds__(256, 2) rmsnorm_bwd_rows_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* w,
+                                                                  const float* rstd, const __nv_bfloat16* dres,
+                                                                  __nv_bfloat16* __restrict__ dx,
+                                                                  float* __restrict__ dw_partial, int rows, int cols) {
   np::pdl_begin();
   __shared__ float buf[2 * NR * 16];
-  const int c = threadIdx.x;
+  __shared__ float s_dw[GROUPS ? 2048 : 1];    // weight gradients of the groups but the first, at the end
+  const int width = GROUPS ? ((cols >> 3) + 31) / 32 * 32 : blockDim.x, groups = GROUPS ? blockDim.x / width : 1;
+  const int grp = GROUPS ? threadIdx.x / width : 0, c = threadIdx.x - grp * width;
   const bool in = c < (cols >> 3);
   float ww[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, dw[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (in) ld8f(w + c * 8, ww);
   int par = 0;
-  for (int r0 = blockIdx.x * NR; r0 < rows; r0 += gridDim.x * NR, par ^= 1) {
+  // every group takes every turn: the barrier of the sums needs all threads
+  for (int rb = blockIdx.x * groups * NR; rb < rows; rb += gridDim.x * groups * NR, par ^= 1) {
+    const int r0 = rb + grp * NR;
     uint4 gq[NR], xq[NR], rq[NR];
     float rs[NR], dot[NR];
 #pragma unroll
@@ -179,7 +187,7 @@ __global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat
         }
       }
     }
-    block_sums<NR>(dot, buf, par);
+    group_sums<NR>(dot, buf, par, width);
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
       if (!in || r0 + q >= rows) break;
@@ -198,7 +206,19 @@ __global__ void __launch_bounds__(512) rmsnorm_bwd_rows_kernel(const __nv_bfloat
       store8(dx + (size_t)(r0 + q) * cols + c * 8, o);
     }
   }
-  if (in) {
+  if constexpr (GROUPS) {
+    if (in && grp > 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s_dw[(grp - 1) * cols + c * 8 + j] = dw[j];
+    }
+    __syncthreads();
+    if (in && grp == 0)
+      for (int g = 0; g < groups - 1; ++g) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dw[j] += s_dw[g * cols + c * 8 + j];
+      }
+  }
+  if (in && grp == 0) {
     float* dst = dw_partial + (size_t)blockIdx.x * cols + c * 8;
     *reinterpret_cast<float4*>(dst) = make_float4(dw[0], dw[1], dw[2], dw[3]);
     *reinterpret_cast<float4*>(dst + 4) = make_float4(dw[4], dw[5], dw[6], dw[7]);
@@ -1057,10 +1077,13 @@ static int launch_rmsnorm_bwd(const void* dy, const void* x, const float* w, con
   // sum: 17.9 us a CTA per row, 21.3 four rows at a time at 1500 rows; 35.5 and 36.8 at 4096)
   if (cols <= 2048) {
     // every CTA the same number of turns, at most `grid` CTAs: the scratch has a row for each
-    const int nr = rows <= 2 * grid ? 2 : 4;
-    const int batches = (rows + nr - 1) / nr, turns = (batches + grid - 1) / grid;
+    const int nr = rows <= 2 * grid ? 2 : 4, width = (cols / 8 + 31) / 32 * 32;
+    const int groups = rows <= 4 * grid ? 1 : 256 / width;   // as soon as one turn of one group per CTA does not do
+    const int per = nr * groups, batches = (rows + per - 1) / per, turns = (batches + grid - 1) / grid;
     grid = (batches + turns - 1) / turns;
-    np_launch(nr == 2 ? rmsnorm_bwd_rows_kernel<2> : rmsnorm_bwd_rows_kernel<4>, grid, (cols / 8 + 31) / 32 * 32, 0, s, 1,
+    auto kern = groups > 1 ? rmsnorm_bwd_rows_kernel<4, true>
+                           : nr == 4 ? rmsnorm_bwd_rows_kernel<4, false> : rmsnorm_bwd_rows_kernel<2, false>;
+    np_launch(kern, grid, groups * width, 0, s, 1,
               (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch,
               rows, cols);
   } else if (cols <= NT * 16) {

@@ -11,9 +11,10 @@ def rel(a, b):
 
 
 # rows off the two- and four-row batches and fewer than one, both sides of the switch between them (592 rows) and of the one
-# to a CTA per row (2048 columns), columns off a warp's 256
+# to a CTA per row (2048 columns), several groups per CTA (above 1184 rows of at most 1024 columns), columns off a warp's 256
 @pytest.mark.parametrize("rows,cols", [(1, 8), (3, 768), (5, 2048), (1023, 1032), (1187, 4096), (2600, 768), (9, 6144),
-                                       (297, 2048), (591, 264), (593, 2040), (300, 2056), (700, 4104)])
+                                       (297, 2048), (591, 264), (593, 2040), (300, 2056), (700, 4104),
+                                       (1184, 1024), (1185, 1024), (2403, 264), (3001, 8), (2371, 520), (9601, 768)])
 @pytest.mark.parametrize("res", [False, True])
 def test_rmsnorm_rows(rows, cols, res):
     from nanopysche_b200.ops.norm import rms_norm
