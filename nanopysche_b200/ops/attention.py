@@ -349,7 +349,8 @@ def attention_append(q, k_cache, v_cache, k_new, v_new, causal: bool = True, sca
     B, S, Hq, hd = q.shape
     Hkv = k_new.shape[2]
     ts = (q, k_cache, v_cache, k_new, v_new)
-    if (USE_FLASH and _lib.on(q) and hd in (64, 128) and Hq // Hkv * S <= DECODE_ROWS and k_cache.shape[1] > 0 and
+    if (USE_FLASH and _lib.on(q) and hd in (64, 128) and 0 < S and Hq // Hkv * S <= DECODE_ROWS and k_cache.shape[1] > 0 and
+            B <= 65535 and Hkv <= 65535 and       # the kernel's grid
             not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) and
             not any(unpack_dual(t).tangent is not None for t in ts) and
             k_new.shape == (B, S, Hkv, hd) == v_new.shape and

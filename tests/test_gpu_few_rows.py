@@ -86,6 +86,20 @@ def test_append_under_grad_takes_the_differentiable_path():
         assert rel(a.grad, b.grad) < 6e-3
 
 
+def test_append_of_nothing_and_of_more_batches_than_the_grid_takes():
+    from nanopysche_b200.ops.attention import attention_append
+
+    torch.manual_seed(5)
+    for B, S in ((2, 0), (65536, 1)):
+        q, kn, vn = (torch.randn(B, S, 1, 64, device="cuda").bfloat16() for _ in range(3))
+        k, v = (torch.randn(B, 3, 1, 64, device="cuda").bfloat16() for _ in range(2))
+        with torch.no_grad():
+            o, ko, vo = attention_append(q, k, v, kn, vn)
+        assert torch.equal(ko, torch.cat([k, kn], 1)) and torch.equal(vo, torch.cat([v, vn], 1)) and o.shape == q.shape
+        if S:
+            assert rel(o[-64:], _sdpa64(q[-64:], ko[-64:], vo[-64:], True)) < 6e-3
+
+
 def test_append_does_not_drop_tangents():
     """Forward-mode derivatives of the flash kernels do not exist: a cached step that carries one says so."""
     from torch.autograd import forward_ad as fwAD
