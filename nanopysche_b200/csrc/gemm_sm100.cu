@@ -1313,8 +1313,9 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
           (!p.Cin || (((uintptr_t)p.Cin & 15) == 0 && (p.ldcin * es) % 16 == 0));
   p.v16_c2 = a.C2 && ((uintptr_t)a.C2 & 15) == 0 && a.ldc2 % 8 == 0 && a.N % 8 == 0;   // the up half starts at column N
   // Plain outputs (dense rows, nothing added from memory, aligned) leave by TMA; peer-row tables, accumulation and other
-  // alignments store from registers. The SwiGLU form needs both of its outputs aligned.
-  p.tma_c = p.v16 && !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue != 1 || BN == 256) && a.ldc >= a.N &&
+  // alignments store from registers. The SwiGLU form needs both of its outputs aligned. So do rows whose length is no whole number
+  // of 16 bytes: a tensor store rounds it up and fills with zeros, up to seven elements beside the output of a wider buffer.
+  p.tma_c = p.v16 && (a.N * (long long)es) % 16 == 0 && !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue != 1 || BN == 256) && a.ldc >= a.N &&
             (a.epilogue != 1 || !a.C2 || p.v16_c2);
   tmC = tmA;
   tmC2 = tmA;

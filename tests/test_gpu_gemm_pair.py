@@ -147,9 +147,10 @@ def test_feed_forward_without_gradients_and_of_frozen_weights():
 
 
 # rows that do not start on 16-byte boundaries: odd widths on both sides of the few-row switch (64 rows) and of the 128-row tiles,
-# an aligned width behind an odd base, a row stride below a vector's
+# an aligned width behind an odd base, a row stride below a vector's, aligned rows of a length that is no whole number of vectors
 @pytest.mark.parametrize("M", [5, 65, 130, 700])
-@pytest.mark.parametrize("N,off,ld", [(1003, 0, 1003), (129, 0, 129), (2052, 0, 2052), (512, 1, 520), (1001, 3, 1010), (7, 0, 7)])
+@pytest.mark.parametrize("N,off,ld", [(1003, 0, 1003), (129, 0, 129), (2052, 0, 2052), (512, 1, 520), (1001, 3, 1010), (7, 0, 7),
+                                      (13, 0, 16), (207, 8, 208), (100, 0, 112), (1030, 0, 1048)])
 @pytest.mark.parametrize("kw", [dict(), dict(bn=128), dict(bn=256, mt=1), dict(bn=256, mt=2), dict(bn=256, mt=2, split=2)])
 def test_outputs_with_unaligned_rows(M, N, off, ld, kw):
     from nanopysche_b200.ops.gemm import gemm
