@@ -20,7 +20,7 @@ import torch
 import os
 
 import torch.nn.functional as F
-from torch.autograd.forward_ad import unpack_dual
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -112,7 +112,8 @@ def flash_supported(q: torch.Tensor, k: torch.Tensor) -> bool:
 def _same_rows(k: torch.Tensor, v: torch.Tensor) -> bool:
     """One set of strides addresses both: a dimension of size 1 is never stepped over, and ``contiguous()`` leaves its
     stride as it is (batch 1 of a longer buffer)."""
-    return k.shape == v.shape and all(n == 1 or a == b for n, a, b in zip(k.shape, k.stride(), v.stride()))
+    return k.shape == v.shape and (k.stride() == v.stride() or
+                                   all(n == 1 or a == b for n, a, b in zip(k.shape, k.stride(), v.stride())))
 
 
 def _rows_aligned(t: torch.Tensor) -> bool:
@@ -310,6 +311,11 @@ def _decode_views(*ts: torch.Tensor) -> bool:
                t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(2) % 8 == 0 for t in ts)
 
 
+def _has_tangent(ts) -> bool:
+    # outside a dual level nothing carries a tangent (asking all five takes 2 us of a 190 us generation step)
+    return getattr(forward_ad, "_current_level", 0) >= 0 and any(forward_ad.unpack_dual(t).tangent is not None for t in ts)
+
+
 def _decode(q, k, v, k_new, v_new, causal, scale):
     """Launch of the decode kernel: keys and values ``[k | k_new]``; returns ``(out, k_cat, v_cat)`` (``None`` for the
     concatenations when nothing is appended)."""
@@ -352,7 +358,7 @@ def attention_append(q, k_cache, v_cache, k_new, v_new, causal: bool = True, sca
     if (USE_FLASH and _lib.on(q) and hd in (64, 128) and 0 < S and Hq // Hkv * S <= DECODE_ROWS and k_cache.shape[1] > 0 and
             B <= 65535 and Hkv <= 65535 and       # the kernel's grid
             not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) and
-            not any(unpack_dual(t).tangent is not None for t in ts) and
+            not _has_tangent(ts) and
             k_new.shape == (B, S, Hkv, hd) == v_new.shape and
             k_cache.shape == v_cache.shape == (B, k_cache.shape[1], Hkv, hd) and
             all(t.device == q.device for t in ts) and _decode_views(*ts)):

@@ -106,9 +106,9 @@ def gemm_swiglu(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, sa
         u = x.float() @ w_up.float().t()
         h = (torch.nn.functional.silu(g) * u).to(x.dtype)
         return h, (torch.cat([g, u], dim=1).to(x.dtype) if save_gu else None)
-    assert all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 for t in (x, w_gate, w_up)), "kernel path is bf16"
-    assert w_gate.stride(0) == w_up.stride(0) and w_gate.shape == w_up.shape
-    assert w_gate.shape[1] == K, f"contraction mismatch {K} vs {w_gate.shape[1]}"
+    assert x.dtype == w_gate.dtype == w_up.dtype == torch.bfloat16, "kernel path is bf16"
+    assert x.stride(1) == 1 and w_gate.stride(1) == 1 and w_gate.stride() == w_up.stride() and w_gate.shape == w_up.shape
+    assert w_gate.shape == (F, K), f"contraction mismatch {K} vs {w_gate.shape[1]}"
     h = torch.empty((M, F), device=x.device, dtype=torch.bfloat16)
     gu = torch.empty((M, 2 * F), device=x.device, dtype=torch.bfloat16) if save_gu else None
     args = _lib.GemmArgs()
@@ -131,8 +131,8 @@ def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor) -> torch.
         from .activation import glu_bwd
 
         return glu_bwd(gu, gemm_ref(dy, w2, b_mn=True))
-    assert all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 for t in (dy, w2, gu)), "kernel path is bf16"
-    assert dy.shape[1] == w2.shape[0] and gu.shape == (M, 2 * F)
+    assert dy.dtype == w2.dtype == gu.dtype == torch.bfloat16, "kernel path is bf16"
+    assert dy.shape[1] == w2.shape[0] and gu.shape == (M, 2 * F) and dy.stride(1) == w2.stride(1) == gu.stride(1) == 1
     out = torch.empty((M, 2 * F), device=dy.device, dtype=torch.bfloat16)
     args = _lib.GemmArgs()
     args.A, args.B, args.C, args.C2 = dy.data_ptr(), w2.data_ptr(), out.data_ptr(), gu.data_ptr()
