@@ -53,6 +53,31 @@ def test_cross_entropy_rows(rows, V):
     assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item()) and rel(logits.grad, l64.grad) < 4e-3
 
 
+# masked vocabulary entries (-inf): single ones, a thread's whole share, all but one; +inf, NaN and a row of -inf give NaN
+@pytest.mark.parametrize("V", [7, 264, 8200, 32000])
+def test_cross_entropy_infinities(V):
+    from nanopysche_b200.ops.xent import _rows_fwd
+
+    torch.manual_seed(V)
+    ld = (V + 7) // 8 * 8
+    logits = (torch.randn(7, ld, device="cuda") * 3).bfloat16()[:, :V]
+    labels = torch.full((7,), V - 1, device="cuda")
+    logits[0, ::3] = float("-inf")
+    logits[1, :V - 1] = float("-inf")
+    logits[2, : V // 2] = -3.3895e38   # the type's lowest value
+    logits[3, V // 2] = float("inf")
+    logits[4, V // 3] = float("nan")
+    logits[5] = float("-inf")
+    labels[0], labels[6] = 1, 0
+    loss, lse = _rows_fwd(logits, labels, -100)
+    ref = torch.logsumexp(logits.double(), -1)
+    want = ref - logits.double().gather(1, labels[:, None])[:, 0]
+    for r in (0, 1, 2, 6):
+        assert abs(lse[r].item() - ref[r].item()) <= 2e-6 * max(1.0, abs(ref[r].item()))
+        assert abs(loss[r].item() - want[r].item()) <= 1e-5 * max(1.0, abs(want[r].item()))
+    assert lse[3:6].isnan().all()
+
+
 # fewer rows than a warp, more than a block, none that counts
 @pytest.mark.parametrize("rows", [1, 31, 1025, 5000])
 def test_cross_entropy_mean(rows):
