@@ -456,7 +456,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
       }
     } else {
 #pragma unroll 1
-      for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
+      for (int c = half; c < BN / 64; c += 2) {   // 192 columns: two chunks for one warp of a quarter, one for the other
         const int col = n0 + c * 64;
         if (col >= p.N) break;
         uint32_t w[32];
@@ -775,8 +775,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // CTAs and are signalled by one multicast commit of the leader; tempty[a] lives in the leader and takes the arrivals of
 // the epilogue warps of both CTAs. The cluster barrier at the end keeps a CTA's shared memory alive until its peer's last
 // remote arrival; both CTAs reach it on every path because every wait before it is bounded.
-constexpr int PAIR_BN = 256, PAIR_STAGES = 6;
-constexpr int PAIR_STAGE_BYTES = BM * BK * 2 + (PAIR_BN / 2) * BK * 2;   // per CTA
+//
+// Tiles of 256 x 192 and 256 x 128 run the same way, for outputs that 256 x 256 tiles leave SMs without work on or whose last
+// wave they leave nearly empty (us, 256 / 192 / 128 columns: 2048 x 3072 x 1024 16.6 / 15.6 / 18.8, 2331 x 2048 x 2048 25.5 /
+// 23.0 / 30.4, 2048 x 1024 x 2816 19.1 / 17.8 / 17.2).
+template <int BN>
+constexpr int pair_stages() { return BN == 128 ? 8 : 6; }
+// per CTA: its rows of A and half of the rows of B, in whole 64-column chunks when B is MN-major
+template <int BN>
+constexpr int pair_stage_bytes() { return BM * BK * 2 + (BN / 2 + 63) / 64 * 64 * BK * 2; }
 
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -828,13 +835,15 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 // through distributed shared memory), sums its own share in the order of the parts and runs the epilogue on it. No
 // workspace, no atomics, and the same result every time. It is for outputs with too few tiles to occupy the SMs: the time
 // of such a GEMM is its K steps one after the other (about 0.4 us each), not its FLOPs.
-template <bool SPLIT>
+template <bool SPLIT, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                       const __grid_constant__ CUtensorMap tmC2, const GemmParams p) {
-  constexpr int BN = PAIR_BN, STAGES = PAIR_STAGES, TM = 2 * BM, HN = BN / 2;
-  constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = PAIR_STAGE_BYTES;
+  constexpr int STAGES = pair_stages<BN>(), TM = 2 * BM, HN = BN / 2;
+  constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = pair_stage_bytes<BN>();
+  constexpr uint32_t TMEM_COLS = 2 * BN <= 256 ? 256 : 512;
+  static_assert(!SPLIT || BN == 256, "K in parts: 256 columns");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (np::smem_u32(smem_raw) + 1023u) & ~1023u;   // the same offset in both CTAs
   const uint32_t stg_base = smem_base + STAGES * STAGE_BYTES;   // staging of the epilogue warps
@@ -888,7 +897,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     np::smem_u32((const void*)tmem_ptr_smem)), "r"(512) : "memory");
+                     np::smem_u32((const void*)tmem_ptr_smem)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   __syncwarp();
@@ -921,6 +930,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
+      const uint32_t step_bytes = 2 * (A_BYTES + (p.b_mn ? (HN + 63) / 64 * 64 : HN) * BK * 2);   // of both CTAs
       for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
         const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
         const int rows = tile_rows(tl, 0);
@@ -937,7 +947,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 11)) return false;
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
           const uint32_t fb = peer_addr(full_bar(stage), lead);
-          if (rank == 0) np::mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
+          if (rank == 0) np::mbar_expect_tx(full_bar(stage), step_bytes);
           if (!p.a_mn) {
             tma_load_2d_pair(sA, &tmA, fb, k0, m0);
           } else {
@@ -951,7 +961,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             const CUtensorMap* bk = second ? &tmB2 : bm;
             const int kb = k0 + (int)goff - (second ? p.k_split : 0);
 #pragma unroll
-            for (int c = 0; c < HN / 64; ++c) tma_load_2d_pair(sB + c * (64 * BK * 2), bk, fb, nrow + c * 64, kb);
+            for (int c = 0; c < (HN + 63) / 64; ++c) tma_load_2d_pair(sB + c * (64 * BK * 2), bk, fb, nrow + c * 64, kb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           return true;
@@ -1111,7 +1121,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync();        // nothing of the peer reads or arrives here any more
   if (warp == 1) {
     np::tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
 
@@ -1120,10 +1130,11 @@ int g_num_sms = 0;
 // Estimated time in us of a launch: a fixed part (setup, first loads, the drain of the last tile) and, per wave of tiles,
 // the K steps one after the other plus what of the drain no MMA covers. Measured on B200 (launches of one kernel back to
 // back in a graph): 256 x 256 output, K = 64 / 2048 / 4096: one-CTA 128 x 128 tiles 5.0 / 16.2 / 27.6, 128 x 256 tiles
-// 5.8 / 17.0 / 28.4, pair 6.6 / 15.2 / 24.0, pair with K in two parts 13.9 / 18.3 (K = 2048 / 4096), in four 13.1 / 15.3;
+// 5.8 / 17.0 / 28.4, pair 6.6 / 15.2 / 24.0 (K = 64 / 1024 / 4096 with 192 columns 5.2 / 8.8 / 21.0, 128 columns 4.8 / 8.4 /
+// 20.6), pair with K in two parts 13.9 / 18.3 (K = 2048 / 4096), in four 13.1 / 15.3;
 // with all SMs busy a K step is 10 to 20 % longer (4096 x 2304 x 4096: 104 / 58 / 51 with the first three).
 struct TileCost { double fixed, step, drain; };
-constexpr TileCost COST_128{4.4, 0.37, 0.6}, COST_256{5.3, 0.40, 0.3}, COST_PAIR{6.0, 0.30, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3},
+constexpr TileCost COST_128{4.4, 0.37, 0.6}, COST_256{5.3, 0.40, 0.3}, COST_PAIR{6.0, 0.30, 0.3}, COST_PAIR_192{5.7, 0.255, 0.3}, COST_PAIR_128{5.5, 0.25, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3},
     COST_SPLIT4{10.7, 0.30, 0.3};
 // Products of at most 64 rows. The few-row kernel: CTAs of 16 weight rows, each of which reads all of x again from the L2, so its
 // time per CTA grows with the rows it is built for (8, 16, 32, 64) and, by the loads in flight, with K. The tile kernels pad to
@@ -1214,6 +1225,7 @@ struct NpGemmArgs {
   int paired;         // row-grouped form: blocks 2 i and 2 i + 1 share their group and their arrival flag
   int k_split;        // > 0 (MN-major B): K rows [0, k_split) of a group come from B, the rest from B2 (multiple of 64)
   int m_split;        // > 0: output rows [0, m_split) go to C, the rest to C2 (layout of C; multiple of 256)
+  int pair_bn;        // columns of a pair's tile: 0 = choose, 128, 192 or 256
 };
 
 static int num_sms() {
@@ -1242,7 +1254,7 @@ static int make_tmap_out(CUtensorMap* out, const void* base, int f32, long long 
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
-template <int BN, int STAGES, bool PAIR>
+template <int BN, bool PAIR>
 static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1) {
   CUtensorMap tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2;
   int rc;
@@ -1330,16 +1342,18 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     if (!rc && a.epilogue == 1 && a.C2) rc = make_tmap_out(&tmC2, a.C2, 0, a.N, a.M, 2, a.ldc2, a.N);
     if (rc) return 800 + rc;
   }
-  constexpr int SMEM = STAGES * (PAIR ? PAIR_STAGE_BYTES : BM * BK * 2 + BN * BK * 2) + EPI_WARPS * STG_BYTES + 1024 + 256;
+  constexpr int STAGES = PAIR ? pair_stages<BN>() : BN == 256 ? 4 : 6;
+  constexpr int SMEM = STAGES * (PAIR ? pair_stage_bytes<BN>() : BM * BK * 2 + BN * BK * 2) + EPI_WARPS * STG_BYTES + 1024 + 256;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
   if (!attr_set) {
     cudaError_t e;
     if constexpr (PAIR) {
-      e = cudaFuncSetAttribute(gemm_bf16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+      e = cudaFuncSetAttribute(gemm_bf16_pair_kernel<false, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+      if constexpr (BN == 256)
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(gemm_bf16_pair_kernel<true, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     } else e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
@@ -1354,9 +1368,11 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     if (pairs <= 0) return 1;   // the dispatch gives launches of one CTA to the other kernel
     p.splits = splits;
     const dim3 grid((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
+    auto kern = gemm_bf16_pair_kernel<false, BN>;
+    if constexpr (BN == 256)
+      if (splits > 1) kern = gemm_bf16_pair_kernel<true, BN>;
     const cudaError_t e =
-        np_launch_if(busy, splits > 1 ? gemm_bf16_pair_kernel<true> : gemm_bf16_pair_kernel<false>, grid, GEMM_THREADS, SMEM, stream,
-                  2 * splits, tmA, tmB, tmB2, tmC, tmC2, p);
+        np_launch_if(busy, kern, grid, GEMM_THREADS, SMEM, stream, 2 * splits, tmA, tmB, tmB2, tmC, tmC2, p);
     if (e != cudaSuccess) return 500 + (int)e;
   } else {
     const int grid = (int)(tiles < cap ? tiles : cap);
@@ -1401,9 +1417,12 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
   int bn = a.bn, mt = a.mt, splits = 1;
   double best = 1e30;
   if (a.epilogue == 1) bn = 256;
-  if (can_pair && bn != 128 && (mt == 2 || (mt == 0 && can_split && (a.split == 2 || a.split == 4)))) {
+  int pbn = a.epilogue == 1 ? 256 : a.pair_bn;
+  if (pbn != 0 && pbn != 128 && pbn != 192 && pbn != 256) return 1;
+  if (can_pair && bn != 128 && (mt == 2 || (pbn != 0 && a.epilogue != 1) || (mt == 0 && can_split && (a.split == 2 || a.split == 4)))) {
     bn = 256;   // asked for
     mt = 2;
+    if (pbn == 0 || a.split == 2 || a.split == 4) pbn = 256;
   } else if (bn == 0 || (bn == 256 && mt == 0)) {
     const long long groups = a.mode == 2 ? a.num_groups : 1;
     // K steps of a group: its share of the token axis in the K-grouped form
@@ -1417,11 +1436,17 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
     const int n256 = a.epilogue == 1 ? 128 : 256;
     if (a.epilogue != 1 && a.bn != 256) best = cost(COST_128, 128, 128, sms, 1);
     bn = 128;
-    auto take = [&](double c, int bn_, int mt_, int splits_) {
-      if (c < best) { best = c; bn = bn_; mt = mt_; splits = splits_; }
+    auto take = [&](double c, int bn_, int mt_, int splits_, int pbn_ = 256) {
+      if (c < best) { best = c; bn = bn_; mt = mt_; splits = splits_; pbn = pbn_; }
     };
     take(cost(COST_256, 128, n256, sms, 1), 256, 1, 1);
-    if (can_pair && a.M > 128 && a.mt == 0) take(cost(COST_PAIR, 256, n256, sms / 2, 1), 256, 2, 1);
+    if (can_pair && a.M > 128 && a.mt == 0) {
+      take(cost(COST_PAIR, 256, n256, sms / 2, 1), 256, 2, 1);
+      if (a.epilogue != 1 && a.bn == 0) {
+        take(cost(COST_PAIR_192, 256, 192, sms / 2, 1), 256, 2, 1, 192);
+        take(cost(COST_PAIR_128, 256, 128, sms / 2, 1), 256, 2, 1, 128);
+      }
+    }
     if (can_split && a.mt == 0 && a.split == 0 && sms >= 128) {
       take(cost(COST_SPLIT2, 256, 256, CLUSTERS4, 2), 256, 2, 2);
       take(cost(COST_SPLIT4, 256, 256, CLUSTERS8, 4), 256, 2, 4);
@@ -1434,9 +1459,12 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
     return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
                             a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
   if (can_split && (a.split == 2 || a.split == 4)) splits = a.split;
-  if (bn == 256 && mt == 2 && can_pair) return launch_gemm<256, PAIR_STAGES, true>(a, (cudaStream_t)stream, splits);
-  if (bn == 256) return launch_gemm<256, 4, false>(a, (cudaStream_t)stream);
-  return launch_gemm<128, 6, false>(a, (cudaStream_t)stream);
+  if (bn == 256 && mt == 2 && can_pair)
+    return pbn == 128 && splits == 1   ? launch_gemm<128, true>(a, (cudaStream_t)stream)
+           : pbn == 192 && splits == 1 ? launch_gemm<192, true>(a, (cudaStream_t)stream)
+                                       : launch_gemm<256, true>(a, (cudaStream_t)stream, splits);
+  if (bn == 256) return launch_gemm<256, false>(a, (cudaStream_t)stream);
+  return launch_gemm<128, false>(a, (cudaStream_t)stream);
 }
 
 NP_API int np_status_read(int* out8) {

@@ -41,7 +41,7 @@ def gemm_ref(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, accumula
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None, accumulate: bool = False,
          alpha: float = 1.0, bn: int = 0, max_ctas: int = 0, bias: torch.Tensor | None = None,
-         residual: torch.Tensor | None = None, mt: int = 0, split: int = 0) -> torch.Tensor:
+         residual: torch.Tensor | None = None, mt: int = 0, split: int = 0, pair_bn: int = 0) -> torch.Tensor:
     """``out[M, N] (+)= alpha * A @ B^T (+ bias) (+ residual)`` in the operand layouts described in the module
     docstring. ``bias [N]`` (fp32) and ``residual [M, N]`` (dtype of ``out``) are added in the GEMM's epilogue."""
     if not _use_kernel(a):
@@ -75,8 +75,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     assert out.dtype in (torch.float32, torch.bfloat16)
     args.accumulate = int(accumulate)
     args.alpha = alpha
-    # requests; 0 = choose. mt 2: 256 x 256 tiles on pairs of CTAs, split 2 or 4: parts of K there (bn 128: one-CTA tiles)
-    args.bn, args.max_ctas, args.mt, args.split = bn, max_ctas, mt, split
+    # requests; 0 = choose. mt 2: 256 x 256 tiles on pairs of CTAs, split 2 or 4: parts of K there (bn 128: one-CTA tiles),
+    # pair_bn 128, 192 or 256: tiles of that many columns on pairs
+    args.bn, args.max_ctas, args.mt, args.split, args.pair_bn = bn, max_ctas, mt, split, pair_bn
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous()
         args.bias = bias.data_ptr()
@@ -123,7 +124,7 @@ def gemm_swiglu(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, sa
     return h, gu
 
 
-def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor) -> torch.Tensor:
+def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor, pair_bn: int = 0) -> torch.Tensor:
     """``[d gate | d up]`` of ``h = silu(gate) * up`` for ``dh = dy @ w2`` and ``gu = [gate | up]``, without forming ``dh``:
     the gradient of the activation is the epilogue of the GEMM (``dy [M, D]``, ``w2 [D, F]``, ``gu [M, 2F]``)."""
     M, F = dy.shape[0], w2.shape[1]
@@ -139,7 +140,7 @@ def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor) -> torch.
     args.lda, args.ldb, args.ldc, args.ldc2 = dy.stride(0), w2.stride(0), 2 * F, gu.stride(0)
     args.a_rows, args.b_rows = M, w2.shape[0]
     args.M, args.N, args.K = M, F, dy.shape[1]
-    args.b_mn, args.epilogue, args.alpha = 1, 2, 1.0
+    args.b_mn, args.epilogue, args.alpha, args.pair_bn = 1, 2, 1.0, pair_bn
     _lib.check(_lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream())), "gemm_glu_bwd")
     return out
 

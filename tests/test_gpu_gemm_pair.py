@@ -48,6 +48,45 @@ def test_pair_gemm(M, N, K, split, layout):
     assert rel(gemm(A, B, bias=bias, out_dtype=torch.float32, **kw), ref + bias) < 2e-5
 
 
+# tiles of 128 and 192 columns: half of 192 is one and a half of the 64-column chunks that an MN-major B is loaded in
+@pytest.mark.parametrize("M,N,K", [(256, 192, 64), (264, 264, 520), (520, 136, 1000), (129, 40, 4096), (776, 2312, 512)])
+@pytest.mark.parametrize("layout", ["fwd", "dgrad", "wgrad"])
+@pytest.mark.parametrize("pair_bn", [128, 192])
+def test_pair_gemm_narrow_tiles(M, N, K, layout, pair_bn):
+    from nanopysche_b200.ops.gemm import gemm
+
+    torch.manual_seed(M + N + K)
+    a_mn, b_mn = layout == "wgrad", layout != "fwd"
+    M += -M % 8 if a_mn else 0
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    ref = a.float() @ b.float().t()
+    A, B = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
+    kw = dict(a_mn=a_mn, b_mn=b_mn, pair_bn=pair_bn)
+    assert rel(gemm(A, B, **kw), ref) < 3e-3
+    acc = torch.randn(M, N, device="cuda")
+    want = acc.double() + 0.5 * ref.double()
+    gemm(A, B, out=acc, accumulate=True, alpha=0.5, **kw)
+    assert rel(acc, want) < 2e-5
+    wide = torch.full((M, N + 24), 7.0, device="cuda").bfloat16()      # rows of a wider buffer: nothing beside them is written
+    gemm(A, B, out=wide[:, :N], **kw)
+    assert rel(wide[:, :N], ref) < 3e-3 and (wide[:, N:] == 7).all()
+    y = gemm(A, B, out_dtype=torch.float32, **kw)
+    assert rel(y, ref) < 2e-5 and torch.equal(y, gemm(A, B, out_dtype=torch.float32, **kw))
+
+
+@pytest.mark.parametrize("M,F,K", [(256, 192, 64), (300, 264, 200), (1000, 704, 512)])
+@pytest.mark.parametrize("pair_bn", [128, 192, 256])
+def test_pair_glu_bwd_tiles(M, F, K, pair_bn):
+    from nanopysche_b200.ops.gemm import gemm_glu_bwd
+
+    torch.manual_seed(F)
+    dy, w2 = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(K, F, device="cuda") * K ** -0.5).bfloat16()
+    gu = torch.randn(M, 2 * F, device="cuda").bfloat16()
+    g, u = (t.float().requires_grad_(True) for t in gu.chunk(2, 1))
+    (torch.nn.functional.silu(g) * u).backward(dy.float() @ w2.float())
+    assert rel(gemm_glu_bwd(dy, w2, gu, pair_bn=pair_bn), torch.cat([g.grad, u.grad], 1)) < 3e-3
+
+
 @pytest.mark.parametrize("M,F,K", [(256, 128, 64), (300, 264, 200), (1000, 704, 512)])
 def test_pair_swiglu(M, F, K):
     from nanopysche_b200.ops.gemm import gemm_swiglu
