@@ -598,47 +598,54 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x) {
-        const Tile tl = decode(t);
-        const int rows = tile_rows(tl, 0);
-        if (rows < 0) break;
-        if (rows == 0) continue;
-        const int m0 = tl.m_blk * BM;
-        const int n0 = tl.n_blk * bn_out;
-        long long goff = 0;  // row offset of this tile's group inside the stacked B tensor
-        if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[tl.m_blk] * p.group_stride_b;
-        const long long brow = n0 + (p.b_mn ? 0 : goff);
-        const int bk_off = p.b_mn ? (int)goff : 0;
-        int b_flag_hi = -1;   // highest B shard this tile has already waited for (its row ranges only move up)
-        auto wait_b_rows = [&](long long r0, long long r1) -> bool {   // rows [r0, r1] of B are about to be loaded
-          if (!p.b_ready_flags) return true;
+    // The whole warp runs the loop and elects the lane that issues, as the MMA warp does: issued by one lane of a divergent
+    // branch, the loads of a K step took 230 ns whatever their size (24 to 32 KB, 4 to 128 CTAs), more than its MMAs.
+    int stage = 0;
+    uint32_t phase = 0;
+    bool live = true;
+    for (int t = blockIdx.x; t < num_tiles && live; t += gridDim.x) {
+      const Tile tl = decode(t);
+      const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(tl, 0) : 0, 0);
+      if (rows < 0) break;
+      if (rows == 0) continue;
+      const int m0 = tl.m_blk * BM;
+      const int n0 = tl.n_blk * bn_out;
+      long long goff = 0;  // row offset of this tile's group inside the stacked B tensor
+      if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[tl.m_blk] * p.group_stride_b;
+      const long long brow = n0 + (p.b_mn ? 0 : goff);
+      const int bk_off = p.b_mn ? (int)goff : 0;
+      int b_flag_hi = -1;   // highest B shard this tile has already waited for (its row ranges only move up)
+      auto wait_b_rows = [&](long long r0, long long r1) -> bool {   // rows [r0, r1] of B are about to be loaded
+        if (!p.b_ready_flags) return true;
+        bool ok = true;
+        if (lane == 0) {
           const int f0 = (int)(r0 / p.b_rows_per_flag), f1 = (int)(r1 / p.b_rows_per_flag);
-          for (int f = f0 > b_flag_hi ? f0 : b_flag_hi + 1; f <= f1; ++f)
-            if (f != p.b_local_flag && !np::wait_flag_ge(p.b_ready_flags + f, epoch, p.flag_limit_ns, KID_GEMM, 110)) {
-              *abort_flag = 1;
-              return false;
-            }
+          for (int f = f0 > b_flag_hi ? f0 : b_flag_hi + 1; f <= f1 && ok; ++f)
+            if (f != p.b_local_flag) ok = np::wait_flag_ge(p.b_ready_flags + f, epoch, p.flag_limit_ns, KID_GEMM, 110);
+          if (!ok) *abort_flag = 1;
           if (f1 > b_flag_hi) b_flag_hi = f1;
-          return true;
-        };
-        if (!p.b_mn) {
-          const long long last = brow + bn_out - 1 < p.N + goff - 1 ? brow + bn_out - 1 : p.N + goff - 1;
-          if (!wait_b_rows(brow, last)) break;
         }
-        for_each_k(p, tl.g, [&](int k0) -> bool {
-          if (p.b_mn && p.b_ready_flags) {
-            const long long last = k0 + bk_off + BK - 1 < p.K + bk_off - 1 ? k0 + bk_off + BK - 1 : p.K + bk_off - 1;
-            if (!wait_b_rows(k0 + bk_off, last)) return false;
-          }
-          if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 1)) return false;
+        live = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        return live;
+      };
+      if (!p.b_mn) {
+        const long long last = brow + bn_out - 1 < p.N + goff - 1 ? brow + bn_out - 1 : p.N + goff - 1;
+        if (!wait_b_rows(brow, last)) break;
+      }
+      const bool a_loc = m0 >= p.a_loc_lo && m0 < p.a_loc_hi, b_loc = brow >= p.b_loc_lo && brow < p.b_loc_hi;
+      for_each_k(p, tl.g, [&](int k0) -> bool {
+        if (p.b_mn && p.b_ready_flags) {
+          const long long last = k0 + bk_off + BK - 1 < p.K + bk_off - 1 ? k0 + bk_off + BK - 1 : p.K + bk_off - 1;
+          if (!wait_b_rows(k0 + bk_off, last)) return false;
+        }
+        live = np::mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 1);
+        if (!live) return false;
+        if (np::elect_one()) {
           const uint32_t sA = smem_base + stage * STAGE_BYTES;
           const uint32_t sB = sA + A_BYTES;
           np::mbar_expect_tx(full_bar(stage), STAGE_BYTES);
           if (!p.a_mn) {
-            if (m0 >= p.a_loc_lo && m0 < p.a_loc_hi) np::tma_load_2d(sA, &tmAloc, full_bar(stage), k0, m0 - p.a_loc_lo);
+            if (a_loc) np::tma_load_2d(sA, &tmAloc, full_bar(stage), k0, m0 - p.a_loc_lo);
             else np::tma_load_2d(sA, &tmA, full_bar(stage), k0, m0);
           } else {
 #pragma unroll
@@ -649,7 +656,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if (p.epilogue == 1) {
               np::tma_load_2d(sB, &tmB, full_bar(stage), k0, (int)brow);
               np::tma_load_2d(sB + (BN / 2) * BK * 2, &tmB2, full_bar(stage), k0, (int)brow);
-            } else if (brow >= p.b_loc_lo && brow < p.b_loc_hi) {
+            } else if (b_loc) {
               np::tma_load_2d(sB, &tmBloc, full_bar(stage), k0, (int)brow - p.b_loc_lo);
             } else {
               np::tma_load_2d(sB, &tmB, full_bar(stage), k0, (int)brow);
@@ -662,12 +669,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int c = 0; c < BN / 64; ++c)
               np::tma_load_2d(sB + c * (64 * BK * 2), bm, full_bar(stage), (int)brow + c * 64, kb);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          return true;
-        });
-      }
-      if (*abort_flag) __nanosleep(1000000);  // let copies already issued land before exit
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        return true;
+      });
     }
+    if (*abort_flag) __nanosleep(1000000);  // let copies already issued land before exit
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     const uint32_t idesc = np::make_idesc(BM, BN, 1, 1, p.a_mn, p.b_mn);
@@ -777,8 +785,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // remote arrival; both CTAs reach it on every path because every wait before it is bounded.
 //
 // Tiles of 256 x 192 and 256 x 128 run the same way, for outputs that 256 x 256 tiles leave SMs without work on or whose last
-// wave they leave nearly empty (us, 256 / 192 / 128 columns: 2048 x 3072 x 1024 16.6 / 15.6 / 18.8, 2331 x 2048 x 2048 25.5 /
-// 23.0 / 30.4, 2048 x 1024 x 2816 19.1 / 17.8 / 17.2).
+// wave they leave nearly empty (us, 256 / 192 / 128 columns: 2048 x 3072 x 1024 16.2 / 14.9 / 17.1, 2331 x 2048 x 2048 25.2 /
+// 21.4 / 26.1, 2048 x 1024 x 2816 19.0 / 16.5 / 15.3).
 template <int BN>
 constexpr int pair_stages() { return BN == 128 ? 8 : 6; }
 // per CTA: its rows of A and half of the rows of B, in whole 64-column chunks when B is MN-major
@@ -834,7 +842,7 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 // done, the operand stages are free: every pair sends the others their share of the columns (256 / splits each, fp32,
 // through distributed shared memory), sums its own share in the order of the parts and runs the epilogue on it. No
 // workspace, no atomics, and the same result every time. It is for outputs with too few tiles to occupy the SMs: the time
-// of such a GEMM is its K steps one after the other (about 0.4 us each), not its FLOPs.
+// of such a GEMM is its K steps one after the other (about 0.3 us each), not its FLOPs.
 template <bool SPLIT, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -926,25 +934,27 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   bool done = false;   // SPLIT: this epilogue warp's accumulator is complete
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (one in each CTA)
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      const uint32_t step_bytes = 2 * (A_BYTES + (p.b_mn ? (HN + 63) / 64 * 64 : HN) * BK * 2);   // of both CTAs
-      for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
-        const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
-        const int rows = tile_rows(tl, 0);
-        if (rows < 0) break;
-        if (rows == 0) continue;
-        const int m0 = tl.m_blk * TM + rank * BM;
-        const int n0 = tl.n_blk * bn_out;
-        long long goff = 0;
-        if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[2 * tl.m_blk] * p.group_stride_b;
-        // SwiGLU: the leader's half of B is the gate tile, the peer's the up tile (another tensor, the same rows)
-        const CUtensorMap* bm = (p.epilogue == 1 && rank) ? &tmB2 : &tmB;
-        const int nrow = n0 + (p.epilogue == 1 ? 0 : rank * HN);
-        k_steps(tl.g, [&](int k0) -> bool {
-          if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 11)) return false;
+    // ------------------------------------------------------------ TMA producer (one warp in each CTA, converged as above)
+    int stage = 0;
+    uint32_t phase = 0;
+    bool live = true;
+    const uint32_t step_bytes = 2 * (A_BYTES + (p.b_mn ? (HN + 63) / 64 * 64 : HN) * BK * 2);   // of both CTAs
+    for (int t = pair; t < num_tiles && live; t += pairs) {
+      const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
+      const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(tl, 0) : 0, 0);
+      if (rows < 0) break;
+      if (rows == 0) continue;
+      const int m0 = tl.m_blk * TM + rank * BM;
+      const int n0 = tl.n_blk * bn_out;
+      long long goff = 0;
+      if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[2 * tl.m_blk] * p.group_stride_b;
+      // SwiGLU: the leader's half of B is the gate tile, the peer's the up tile (another tensor, the same rows)
+      const CUtensorMap* bm = (p.epilogue == 1 && rank) ? &tmB2 : &tmB;
+      const int nrow = n0 + (p.epilogue == 1 ? 0 : rank * HN);
+      k_steps(tl.g, [&](int k0) -> bool {
+        live = np::mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 11);
+        if (!live) return false;
+        if (np::elect_one()) {
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
           const uint32_t fb = peer_addr(full_bar(stage), lead);
           if (rank == 0) np::mbar_expect_tx(full_bar(stage), step_bytes);
@@ -963,17 +973,18 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 #pragma unroll
             for (int c = 0; c < (HN + 63) / 64; ++c) tma_load_2d_pair(sB + c * (64 * BK * 2), bk, fb, nrow + c * 64, kb);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          return true;
-        });
-      }
-      // the leader's last commits have arrived here before this CTA may exit (a stage never used passes at once)
-      for (int s = 0; s < STAGES; ++s) {
-        if (!np::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 15)) break;
+        }
+        __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-      }
-      if (*abort_flag) __nanosleep(1000000);   // let copies already issued land before exit
+        return true;
+      });
     }
+    // the leader's last commits have arrived here before this CTA may exit (a stage never used passes at once)
+    for (int s = 0; s < STAGES; ++s) {
+      if (!np::mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 15)) break;
+      if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    }
+    if (*abort_flag) __nanosleep(1000000);   // let copies already issued land before exit
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader's)
     if (rank == 0) {
@@ -1129,13 +1140,13 @@ int g_num_sms = 0;
 
 // Estimated time in us of a launch: a fixed part (setup, first loads, the drain of the last tile) and, per wave of tiles,
 // the K steps one after the other plus what of the drain no MMA covers. Measured on B200 (launches of one kernel back to
-// back in a graph): 256 x 256 output, K = 64 / 2048 / 4096: one-CTA 128 x 128 tiles 5.0 / 16.2 / 27.6, 128 x 256 tiles
-// 5.8 / 17.0 / 28.4, pair 6.6 / 15.2 / 24.0 (K = 64 / 1024 / 4096 with 192 columns 5.2 / 8.8 / 21.0, 128 columns 4.8 / 8.4 /
-// 20.6), pair with K in two parts 13.9 / 18.3 (K = 2048 / 4096), in four 13.1 / 15.3;
-// with all SMs busy a K step is 10 to 20 % longer (4096 x 2304 x 4096: 104 / 58 / 51 with the first three).
+// back in a graph): 256 x 256 output, K = 64 / 1024 / 4096: one-CTA 128 x 128 tiles 4.4 / 8.2 / 20.7, 128 x 256 tiles
+// 5.2 / 9.4 / 22.8, pair with 256 columns 5.5 / 9.8 / 23.2, 192 columns 5.1 / 8.3 / 18.4, 128 columns 4.8 / 7.7 / 17.3, 256 with
+// K in two parts 10.4 / 17.1 (K = 1024 / 4096), in four 10.6 / 14.0; with many SMs busy a K step is longer (2048 x 1024, K = 1024
+// / 4096: 8.9 / 22.6, 10.1 / 27.8, 10.3 / 24.7, 9.4 / 21.4, 8.9 / 19.1).
 struct TileCost { double fixed, step, drain; };
-constexpr TileCost COST_128{4.4, 0.37, 0.6}, COST_256{5.3, 0.40, 0.3}, COST_PAIR{6.0, 0.30, 0.3}, COST_PAIR_192{5.7, 0.255, 0.3}, COST_PAIR_128{5.5, 0.25, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3},
-    COST_SPLIT4{10.7, 0.30, 0.3};
+constexpr TileCost COST_128{4.3, 0.28, 0.4}, COST_256{5.0, 0.35, 0.3}, COST_PAIR{5.6, 0.30, 0.3}, COST_PAIR_192{5.3, 0.25, 0.3},
+    COST_PAIR_128{5.2, 0.21, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3}, COST_SPLIT4{10.0, 0.28, 0.3};
 // Products of at most 64 rows. The few-row kernel: CTAs of 16 weight rows, each of which reads all of x again from the L2, so its
 // time per CTA grows with the rows it is built for (8, 16, 32, 64) and, by the loads in flight, with K. The tile kernels pad to
 // 128 rows but read x once per tile: with many columns they are bound by reading the weight. Fitted to 15 weights of 768 x 768 to
