@@ -843,11 +843,48 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 // through distributed shared memory), sums its own share in the order of the parts and runs the epilogue on it. No
 // workspace, no atomics, and the same result every time. It is for outputs with too few tiles to occupy the SMs: the time
 // of such a GEMM is its K steps one after the other (about 0.3 us each), not its FLOPs.
-template <bool SPLIT, int BN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
-                      const __grid_constant__ CUtensorMap tmC2, const GemmParams p) {
+//
+// DUAL: two products in one launch. A backward pass asks for the gradients of a layer's input and of its weight at the same
+// time; alone, each leaves SMs without work in its only or last wave and pays for a launch, first loads and a last drain of its
+// own. A pair takes its tiles of the product with the longer contraction first, then those of the other. us, two launches /
+// one, in a graph, gradients of a layer of T tokens, N outputs, K inputs: T N K = 2048 1024 1024 22.8 / 14.9, 2048 3072 1024 34.1 /
+// 29.5, 2048 5632 1024 51.5 / 40.7, 2331 2048 2048 45.7 / 31.3, 4096 2048 5632 with the SwiGLU gradient 178.7 / 155.9.
+struct PairMaps {
+  CUtensorMap A, B, B2, C, C2;
+};
+struct PairSecond {
+  PairMaps m;
+  GemmParams p;
+  int extra;   // tiles of the second product that a pair with one tile less of the first takes before the rest is dealt to all
+};
+struct PairWork {
+  int which, t;   // product and its tile; t < 0: no more
+};
+// Piece k of a pair's work: n0 tiles of the first product dealt in turn, then n1 of the second. Where the first do not come
+// out even, the pairs from r on have one less and take up to `extra` of the second each; the rest goes to all, those pairs first.
+__host__ __device__ __forceinline__ PairWork pair_work(int k, int pair, int pairs, int n0, int n1, int extra) {
+  const int own = n0 > pair ? (n0 - pair - 1) / pairs + 1 : 0;
+  if (k < own) return {0, pair + k * pairs};
+  k -= own;
+  const int r = n0 % pairs;
+  int base = 0;
+  if (r > 0) {
+    const int slack = pairs - r;
+    if (pair >= r) {
+      if (k < extra) {
+        const int j = pair - r + k * slack;
+        return {1, j < n1 ? j : -1};
+      }
+      k -= extra;
+    }
+    base = extra < (n1 + slack - 1) / slack ? extra * slack : n1;
+  }
+  const int j = base + (pair >= r ? pair - r : pair - r + pairs) + k * pairs;
+  return {1, j < n1 ? j : -1};
+}
+
+template <bool SPLIT, int BN, bool DUAL>
+__device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams& p, const PairSecond* second) {
   constexpr int STAGES = pair_stages<BN>(), TM = 2 * BM, HN = BN / 2;
   constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = pair_stage_bytes<BN>();
   constexpr uint32_t TMEM_COLS = 2 * BN <= 256 ? 256 : 512;
@@ -869,18 +906,33 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int rank = (int)(crank & 1u);                              // 0: leader of its pair
   const int splits = SPLIT ? p.splits : 1, split = SPLIT ? (int)(crank >> 1) : 0;
   const int pair = (int)blockIdx.x / (2 * splits), pairs = (int)gridDim.x / (2 * splits);
-  const int m_blocks = (p.M + TM - 1) / TM, m_blocks128 = (p.M + BM - 1) / BM;
-  const int bn_out = (p.epilogue == 1) ? HN : BN;
-  const int n_blocks = (p.N + bn_out - 1) / bn_out;
-  const int num_tiles = m_blocks * n_blocks * ((p.mode == 2) ? p.num_groups : 1);
+  const int bn_out = (!DUAL && p.epilogue == 1) ? HN : BN;
+  auto m_blocks = [&](const GemmParams& q) { return (q.M + TM - 1) / TM; };
+  auto n_blocks = [&](const GemmParams& q) { return (q.N + bn_out - 1) / bn_out; };
+  auto num_tiles = [&](const GemmParams& q) { return m_blocks(q) * n_blocks(q) * ((q.mode == 2) ? q.num_groups : 1); };
+  const int tiles0 = num_tiles(p), tiles1 = DUAL ? num_tiles(second->p) : 0;
+  auto work = [&](int k) -> PairWork {
+    if constexpr (DUAL) return pair_work(k, pair, pairs, tiles0, tiles1, second->extra);
+    const int t = pair + k * pairs;
+    return {0, t < tiles0 ? t : -1};
+  };
+  // parameters and tensor maps of the product that a piece of work belongs to
+  auto params = [&](const PairWork& w) -> const GemmParams& {
+    if constexpr (DUAL) return w.which ? second->p : p;
+    else return p;
+  };
+  auto tensor_maps = [&](const PairWork& w) -> const PairMaps& {
+    if constexpr (DUAL) return w.which ? second->m : maps;
+    else return maps;
+  };
   // the K steps of this CTA's part
-  auto k_steps = [&](int g, auto&& f) {
+  auto k_steps = [&](const GemmParams& q, int g, auto&& f) {
     if constexpr (SPLIT) {
-      const int nkb = (p.K + BK - 1) / BK, hi = (int)((long long)nkb * (split + 1) / splits);
+      const int nkb = (q.K + BK - 1) / BK, hi = (int)((long long)nkb * (split + 1) / splits);
       for (int kb = (int)((long long)nkb * split / splits); kb < hi; ++kb)
         if (!f(kb * BK)) return;
     } else {
-      for_each_k(p, g, f);
+      for_each_k(q, g, f);
     }
   };
 
@@ -898,10 +950,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     np::mbar_fence_init();
   }
   if (threadIdx.x == 64) {   // while another warp sets up the barriers
-    np::tma_prefetch_desc(&tmA);
-    np::tma_prefetch_desc(&tmB);
-    if (p.tma_c) np::tma_prefetch_desc(&tmC);
-    if (p.tma_c && p.C2) np::tma_prefetch_desc(&tmC2);
+    np::tma_prefetch_desc(&maps.A);
+    np::tma_prefetch_desc(&maps.B);
+    if (p.tma_c) np::tma_prefetch_desc(&maps.C);
+    if (p.tma_c && p.C2) np::tma_prefetch_desc(&maps.C2);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -914,22 +966,22 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   np::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   np::pdl_begin();
-  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
+  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);   // a launch of two products: the first one's
 
   // rows of the two 128-row blocks of an M block that carry data, as a mask (0: nothing to do, -1: gave up). Row-grouped
   // form: both blocks belong to the same group and arrive under the same flag (the caller's tables are made of pairs).
-  auto tile_rows = [&](const Tile& tl, int role) -> int {
-    if (p.mode != 1) return 3;
+  auto tile_rows = [&](const GemmParams& q, const Tile& tl, int role) -> int {
+    if (q.mode != 1) return 3;
     const int b0 = 2 * tl.m_blk;
-    if (p.ready_flags) {
-      const int fi = p.mblk_flag ? p.mblk_flag[b0] : 0;
-      if (fi >= 0 && !np::wait_flag_ge(p.ready_flags + fi, epoch, p.flag_limit_ns, KID_GEMM, 120 + role)) {
+    if (q.ready_flags) {
+      const int fi = q.mblk_flag ? q.mblk_flag[b0] : 0;
+      if (fi >= 0 && !np::wait_flag_ge(q.ready_flags + fi, epoch, q.flag_limit_ns, KID_GEMM, 120 + role)) {
         *abort_flag = 1;
         return -1;
       }
     }
-    if (!p.mblk_rows) return 3;
-    return (p.mblk_rows[b0] > 0 ? 1 : 0) | (b0 + 1 < m_blocks128 && p.mblk_rows[b0 + 1] > 0 ? 2 : 0);
+    if (!q.mblk_rows) return 3;
+    return (q.mblk_rows[b0] > 0 ? 1 : 0) | (b0 + 1 < (q.M + BM - 1) / BM && q.mblk_rows[b0 + 1] > 0 ? 2 : 0);
   };
 
   bool done = false;   // SPLIT: this epilogue warp's accumulator is complete
@@ -938,38 +990,44 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     int stage = 0;
     uint32_t phase = 0;
     bool live = true;
-    const uint32_t step_bytes = 2 * (A_BYTES + (p.b_mn ? (HN + 63) / 64 * 64 : HN) * BK * 2);   // of both CTAs
-    for (int t = pair; t < num_tiles && live; t += pairs) {
-      const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
-      const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(tl, 0) : 0, 0);
+    for (int k = 0; live; ++k) {
+      const PairWork wk = work(k);
+      if (wk.t < 0) break;
+      const GemmParams& q = params(wk);
+      const PairMaps& tm = tensor_maps(wk);
+      const uint32_t step_bytes = 2 * (A_BYTES + (q.b_mn ? (HN + 63) / 64 * 64 : HN) * BK * 2);   // of both CTAs
+      const Tile tl = decode_tile<8>(wk.t, m_blocks(q), n_blocks(q));
+      const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(q, tl, 0) : 0, 0);
       if (rows < 0) break;
       if (rows == 0) continue;
       const int m0 = tl.m_blk * TM + rank * BM;
       const int n0 = tl.n_blk * bn_out;
       long long goff = 0;
-      if (p.mode == 1 && p.mblk_group) goff = (long long)p.mblk_group[2 * tl.m_blk] * p.group_stride_b;
+      if (q.mode == 1 && q.mblk_group) goff = (long long)q.mblk_group[2 * tl.m_blk] * q.group_stride_b;
       // SwiGLU: the leader's half of B is the gate tile, the peer's the up tile (another tensor, the same rows)
-      const CUtensorMap* bm = (p.epilogue == 1 && rank) ? &tmB2 : &tmB;
-      const int nrow = n0 + (p.epilogue == 1 ? 0 : rank * HN);
-      k_steps(tl.g, [&](int k0) -> bool {
+      const bool up = !DUAL && q.epilogue == 1 && rank;
+      const CUtensorMap* bm = up ? &tm.B2 : &tm.B;
+      const int nrow = n0 + (!DUAL && q.epilogue == 1 ? 0 : rank * HN);
+      const int a_mn = q.a_mn, b_mn = q.b_mn, k_split = q.k_split;
+      k_steps(q, tl.g, [&](int k0) -> bool {
         live = np::mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag, KID_GEMM, 11);
         if (!live) return false;
         if (np::elect_one()) {
           const uint32_t sA = smem_base + stage * STAGE_BYTES, sB = sA + A_BYTES;
           const uint32_t fb = peer_addr(full_bar(stage), lead);
           if (rank == 0) np::mbar_expect_tx(full_bar(stage), step_bytes);
-          if (!p.a_mn) {
-            tma_load_2d_pair(sA, &tmA, fb, k0, m0);
+          if (!a_mn) {
+            tma_load_2d_pair(sA, &tm.A, fb, k0, m0);
           } else {
 #pragma unroll
-            for (int c = 0; c < BM / 64; ++c) tma_load_2d_pair(sA + c * (64 * BK * 2), &tmA, fb, m0 + c * 64, k0);
+            for (int c = 0; c < BM / 64; ++c) tma_load_2d_pair(sA + c * (64 * BK * 2), &tm.A, fb, m0 + c * 64, k0);
           }
-          if (!p.b_mn) {
+          if (!b_mn) {
             tma_load_2d_pair(sB, bm, fb, k0, (int)(nrow + goff));
           } else {
-            const bool second = p.k_split && k0 >= p.k_split;
-            const CUtensorMap* bk = second ? &tmB2 : bm;
-            const int kb = k0 + (int)goff - (second ? p.k_split : 0);
+            const bool part2 = k_split && k0 >= k_split;
+            const CUtensorMap* bk = part2 ? &tm.B2 : bm;
+            const int kb = k0 + (int)goff - (part2 ? k_split : 0);
 #pragma unroll
             for (int c = 0; c < (HN + 63) / 64; ++c) tma_load_2d_pair(sB + c * (64 * BK * 2), bk, fb, nrow + c * 64, kb);
           }
@@ -988,22 +1046,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader's)
     if (rank == 0) {
-      const uint32_t idesc = np::make_idesc(TM, BN, 1, 1, p.a_mn, p.b_mn);
-      const uint64_t a_desc0 = operand_desc(smem_base, p.a_mn), b_desc0 = operand_desc(smem_base + A_BYTES, p.b_mn);
-      const uint32_t a_step = k_step(p.a_mn), b_step = k_step(p.b_mn);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
-      for (int t = pair; t < num_tiles; t += pairs) {
-        const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
-        const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(tl, 1) : 0, 0);
+      for (int k = 0;; ++k) {
+        const PairWork wk = work(k);
+        if (wk.t < 0) break;
+        const GemmParams& q = params(wk);
+        const uint32_t idesc = np::make_idesc(TM, BN, 1, 1, q.a_mn, q.b_mn);
+        const uint64_t a_desc0 = operand_desc(smem_base, q.a_mn), b_desc0 = operand_desc(smem_base + A_BYTES, q.b_mn);
+        const uint32_t a_step = k_step(q.a_mn), b_step = k_step(q.b_mn);
+        const Tile tl = decode_tile<8>(wk.t, m_blocks(q), n_blocks(q));
+        const int rows = __shfl_sync(0xffffffffu, lane == 0 ? tile_rows(q, tl, 1) : 0, 0);
         if (rows < 0) break;
         if (rows == 0) continue;
-        if (count_k(p, tl.g) == 0) continue;
+        if (count_k(q, tl.g) == 0) continue;
         if (!np::mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 12)) break;
         np::tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
         uint32_t accum = 0;
-        k_steps(tl.g, [&](int) -> bool {
+        k_steps(q, tl.g, [&](int) -> bool {
           if (!np::mbar_wait_warp(full_bar(stage), phase, abort_flag, KID_GEMM, 13)) return false;
           np::tc_fence_after();
           if (np::elect_one()) {
@@ -1030,12 +1091,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     GluBar gb{bar_base + 8u * (2 * STAGES + 4 + warp - 2), 0u};
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int t = pair; t < num_tiles && !*abort_flag; t += pairs) {
-      const Tile tl = decode_tile<8>(t, m_blocks, n_blocks);
-      const int rows = tile_rows(tl, 2);
+    for (int k = 0; !*abort_flag; ++k) {
+      const PairWork wk = work(k);
+      if (wk.t < 0) break;
+      const GemmParams& q = params(wk);
+      const PairMaps& tm = tensor_maps(wk);
+      const Tile tl = decode_tile<8>(wk.t, m_blocks(q), n_blocks(q));
+      const int rows = tile_rows(q, tl, 2);
       if (rows < 0) break;
       if (rows == 0) continue;
-      const bool have_acc = count_k(p, tl.g) > 0;
+      const bool have_acc = count_k(q, tl.g) > 0;
       const bool mine = (rows >> rank) & 1;   // this CTA's 128-row block carries data
       if (have_acc) {
         if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 14)) break;
@@ -1046,8 +1111,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
         const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
         const int row0 = tl.m_blk * TM + rank * BM + quarter * 32, n0 = tl.n_blk * bn_out;
-        if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
-        else store_tile<BN>(p, &tmC, &tmC2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
+        if (q.epilogue == 2) store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+        else store_tile<BN>(q, &tm.C, &tm.C2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
       }
       if (have_acc) {
         np::tc_fence_before();
@@ -1055,20 +1120,20 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (lane == 0) arrive_cluster(peer_addr(tempty_bar(acc), lead));
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
-      if (p.done_counters && mine) {
+      if (q.done_counters && mine) {
         __threadfence_system();
         __syncwarp();
         if (lane == 0) {
-          const int fi = p.mblk_flag ? p.mblk_flag[2 * tl.m_blk] : 0;
-          const int n_done = atomicAdd(&p.done_counters[fi], 1) + 1;
-          if (n_done == EPI_WARPS * n_blocks * p.done_expected[fi]) {   // done_expected counts 128-row blocks
+          const int fi = q.mblk_flag ? q.mblk_flag[2 * tl.m_blk] : 0;
+          const int n_done = atomicAdd(&q.done_counters[fi], 1) + 1;
+          if (n_done == EPI_WARPS * n_blocks(q) * q.done_expected[fi]) {   // done_expected counts 128-row blocks
             __threadfence_system();
-            np::st_release_sys(p.done_flag_ptr[fi], epoch);
+            np::st_release_sys(q.done_flag_ptr[fi], epoch);
           }
         }
       }
     }
-    if (p.tma_c) stage_drain(lane);
+    stage_drain(lane);
   }
   if constexpr (SPLIT) {
     __syncthreads();
@@ -1096,7 +1161,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     __syncwarp();
     cluster_sync();      // all shares have arrived
     if (done) {
-      const Tile tl = decode_tile<8>(pair, m_blocks, n_blocks);
+      const Tile tl = decode_tile<8>(pair, m_blocks(p), n_blocks(p));
       const OutRow o = out_row(p, 0, tl.m_blk * TM + rank * BM + r);
       for (int c = half * per_half; c < (half + 1) * per_half; ++c) {
         uint32_t own[32];
@@ -1134,6 +1199,18 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     np::tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
+}
+
+template <bool SPLIT, int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ GemmParams p) {
+  pair_body<SPLIT, BN, false>(maps, p, nullptr);
+}
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_pair2_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ GemmParams p,
+                       const __grid_constant__ PairSecond second) {
+  pair_body<false, BN, true>(maps, p, &second);
 }
 
 int g_num_sms = 0;
@@ -1265,9 +1342,10 @@ static int make_tmap_out(CUtensorMap* out, const void* base, int f32, long long 
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
+// Tensor maps and kernel parameters of a launch with tiles of BN columns
 template <int BN, bool PAIR>
-static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1) {
-  CUtensorMap tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2;
+static int prepare_gemm(const NpGemmArgs& a, int splits, PairMaps& m, CUtensorMap& tmAloc, CUtensorMap& tmBloc, GemmParams& p) {
+  CUtensorMap &tmA = m.A, &tmB = m.B, &tmB2 = m.B2, &tmC = m.C, &tmC2 = m.C2;
   int rc;
   if (!a.a_mn) rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.K, (uint64_t)a.lda, BK, BM);
   else rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.M, (uint64_t)a.lda, 64, BK);
@@ -1282,9 +1360,11 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     else rc = np_make_tmap_2d(&tmB2, a.B2, 2, (uint64_t)a.b_rows, (uint64_t)a.N, (uint64_t)a.ldb, 64, BK);
     if (rc) return 300 + rc;
   }
-  tmAloc = tmA;
-  tmBloc = tmB;
-  GemmParams p{};
+  if constexpr (!PAIR) {
+    tmAloc = tmA;
+    tmBloc = tmB;
+  }
+  p = GemmParams{};
   p.b_local_flag = a.b_local_flag - 1;
   // 32-byte stores need every (row, 32-column chunk) address 32-byte aligned; destinations behind peer_base are
   // allocations of the symmetric heap (256-byte aligned)
@@ -1353,8 +1433,24 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
     if (!rc && a.epilogue == 1 && a.C2) rc = make_tmap_out(&tmC2, a.C2, 0, a.N, a.M, 2, a.ldc2, a.N);
     if (rc) return 800 + rc;
   }
+  p.splits = splits;
+  return 0;
+}
+
+template <int BN, bool PAIR>
+constexpr int gemm_smem() {
   constexpr int STAGES = PAIR ? pair_stages<BN>() : BN == 256 ? 4 : 6;
-  constexpr int SMEM = STAGES * (PAIR ? pair_stage_bytes<BN>() : BM * BK * 2 + BN * BK * 2) + EPI_WARPS * STG_BYTES + 1024 + 256;
+  return STAGES * (PAIR ? pair_stage_bytes<BN>() : BM * BK * 2 + BN * BK * 2) + EPI_WARPS * STG_BYTES + 1024 + 256;
+}
+
+template <int BN, bool PAIR>
+static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1) {
+  PairMaps m;
+  CUtensorMap tmAloc, tmBloc;
+  GemmParams p;
+  const int rc = prepare_gemm<BN, PAIR>(a, splits, m, tmAloc, tmBloc, p);
+  if (rc) return rc;
+  constexpr int SMEM = gemm_smem<BN, PAIR>(), STAGES = BN == 256 ? 4 : 6;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
@@ -1377,17 +1473,16 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
   if constexpr (PAIR) {
     const long long pairs = tiles < cap / 2 ? tiles : cap / 2;
     if (pairs <= 0) return 1;   // the dispatch gives launches of one CTA to the other kernel
-    p.splits = splits;
     const dim3 grid((unsigned)(splits > 1 ? tiles * 2 * splits : 2 * pairs));
     auto kern = gemm_bf16_pair_kernel<false, BN>;
     if constexpr (BN == 256)
       if (splits > 1) kern = gemm_bf16_pair_kernel<true, BN>;
     const cudaError_t e =
-        np_launch_if(busy, kern, grid, GEMM_THREADS, SMEM, stream, 2 * splits, tmA, tmB, tmB2, tmC, tmC2, p);
+        np_launch_if(busy, kern, grid, GEMM_THREADS, SMEM, stream, 2 * splits, m, p);
     if (e != cudaSuccess) return 500 + (int)e;
   } else {
     const int grid = (int)(tiles < cap ? tiles : cap);
-    np_launch_if(busy, gemm_bf16_kernel<BN, STAGES>, grid, GEMM_THREADS, SMEM, stream, 1, tmA, tmB, tmB2, tmAloc, tmBloc, tmC, tmC2, p);
+    np_launch_if(busy, gemm_bf16_kernel<BN, STAGES>, grid, GEMM_THREADS, SMEM, stream, 1, m.A, m.B, m.B2, tmAloc, tmBloc, m.C, m.C2, p);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
@@ -1396,20 +1491,18 @@ static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1)
 int np_skinny_linear(const void* x, long long ldx, const void* w, long long ldw, int M, int N, int K, void* out, long long ldo,
                      int out_f32, float alpha, const float* bias, const void* cin, long long ldcin, cudaStream_t stream);
 
-// C[M,N] (+)= alpha * A * B^T with the operand layouts described in NpGemmArgs.
-// Returns 0 or a launch/setup error; device-side problems are reported via np_status_read.
-NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
-  const NpGemmArgs& a = *args;
-  if (a.M <= 0 || a.N <= 0) return 0;
-  // The tensor-map encode below is a driver call: make sure this host thread (e.g. an autograd
-  // worker that has not touched the runtime yet) has the device's primary context bound.
-  static thread_local bool ctx_bound = false;
-  if (!ctx_bound) {
+// The tensor-map encode is a driver call: make sure this host thread (e.g. an autograd worker that has not touched the runtime
+// yet) has the device's primary context bound.
+static bool bind_context() {
+  static thread_local bool bound = false;
+  if (!bound) {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || cudaFree(nullptr) != cudaSuccess)
-      return 2;
-    ctx_bound = true;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || cudaFree(nullptr) != cudaSuccess) return false;
+    bound = true;
   }
+  return true;
+}
+static int check_gemm(const NpGemmArgs& a) {
   if (a.k_split < 0 || a.m_split < 0 || (a.k_split > 0 && (!a.b_mn || a.mode == 2 || a.epilogue != 0 || a.k_split % BK)) ||
       (a.m_split > 0 && (a.row_dst || a.epilogue != 0 || a.m_split % 256 || a.m_split >= a.M || (a.Cin && a.Cin != a.C))))
     return 1;
@@ -1417,6 +1510,18 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
                           a.ldc % 8 || a.ldc2 % 8 || (((uintptr_t)a.C | (uintptr_t)a.C2) & 15)))
     return 1;
   if ((a.lda % 8) || (a.ldb % 8) || (((uintptr_t)a.A) & 15) || (((uintptr_t)a.B) & 15)) return 1;
+  if (a.pair_bn != 0 && a.pair_bn != 128 && a.pair_bn != 192 && a.pair_bn != 256) return 1;
+  return 0;
+}
+
+// Which kernel a product runs on: the few-row kernel, one CTA per tile of `bn` columns, or pairs with tiles of `bn` columns and
+// K in `splits` parts
+struct GemmChoice {
+  bool few, pair;
+  int bn, splits;
+  double cost;   // estimate in us
+};
+static GemmChoice choose_gemm(const NpGemmArgs& a) {
   const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
                      (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
   // Which tile kernel: the lowest estimate (TileCost). The pair kernel takes the forms without peer-arrival flags on B, pushes or
@@ -1425,57 +1530,143 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
   const int nk = (a.K + BK - 1) / BK, sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
   const bool can_split = plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
   const bool can_pair = plain && sms >= 2;   // a pair needs two CTAs
-  int bn = a.bn, mt = a.mt, splits = 1;
-  double best = 1e30;
-  if (a.epilogue == 1) bn = 256;
-  int pbn = a.epilogue == 1 ? 256 : a.pair_bn;
-  if (pbn != 0 && pbn != 128 && pbn != 192 && pbn != 256) return 1;
-  if (can_pair && bn != 128 && (mt == 2 || (pbn != 0 && a.epilogue != 1) || (mt == 0 && can_split && (a.split == 2 || a.split == 4)))) {
-    bn = 256;   // asked for
-    mt = 2;
-    if (pbn == 0 || a.split == 2 || a.split == 4) pbn = 256;
-  } else if (bn == 0 || (bn == 256 && mt == 0)) {
+  const int bn_asked = a.epilogue == 1 ? 256 : a.bn, pbn_asked = a.epilogue == 1 ? 0 : a.pair_bn;
+  const bool split_asked = can_split && (a.split == 2 || a.split == 4);
+  GemmChoice c{false, false, bn_asked == 256 ? 256 : 128, 1, 1e30};
+  if (can_pair && bn_asked != 128 && (a.mt == 2 || pbn_asked != 0 || (a.mt == 0 && split_asked))) {
+    c.pair = true;   // asked for
+    c.bn = split_asked || pbn_asked == 0 ? 256 : pbn_asked;
+  } else if (bn_asked == 0 || (bn_asked == 256 && a.mt == 0)) {
     const long long groups = a.mode == 2 ? a.num_groups : 1;
     // K steps of a group: its share of the token axis in the K-grouped form
     const double steps = a.mode == 2 ? 2.0 * a.blocks_per_group : nk;
-    auto cost = [&](const TileCost& c, int tm, int tn, int units, int parts) {
-      const long long t = (long long)((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn) * groups;
-      const double waves = (double)((t + units - 1) / units);
+    auto take = [&](const TileCost& t, int tm, int tn, int units, int parts, bool pair, int bn) {
+      const long long n = (long long)((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn) * groups;
+      const double waves = (double)((n + units - 1) / units);
       // tiles of a persistent CTA follow one another; a cluster that splits K starts anew for every tile
-      return parts == 1 ? c.fixed + waves * (steps * c.step + c.drain) : waves * (c.fixed + steps / parts * c.step + c.drain);
+      const double cost = parts == 1 ? t.fixed + waves * (steps * t.step + t.drain) : waves * (t.fixed + steps / parts * t.step + t.drain);
+      if (cost < c.cost) c = GemmChoice{false, pair, bn, parts, cost};
     };
     const int n256 = a.epilogue == 1 ? 128 : 256;
-    if (a.epilogue != 1 && a.bn != 256) best = cost(COST_128, 128, 128, sms, 1);
-    bn = 128;
-    auto take = [&](double c, int bn_, int mt_, int splits_, int pbn_ = 256) {
-      if (c < best) { best = c; bn = bn_; mt = mt_; splits = splits_; pbn = pbn_; }
-    };
-    take(cost(COST_256, 128, n256, sms, 1), 256, 1, 1);
+    if (bn_asked == 0) take(COST_128, 128, 128, sms, 1, false, 128);
+    take(COST_256, 128, n256, sms, 1, false, 256);
     if (can_pair && a.M > 128 && a.mt == 0) {
-      take(cost(COST_PAIR, 256, n256, sms / 2, 1), 256, 2, 1);
-      if (a.epilogue != 1 && a.bn == 0) {
-        take(cost(COST_PAIR_192, 256, 192, sms / 2, 1), 256, 2, 1, 192);
-        take(cost(COST_PAIR_128, 256, 128, sms / 2, 1), 256, 2, 1, 128);
+      take(COST_PAIR, 256, n256, sms / 2, 1, true, 256);
+      if (bn_asked == 0) {
+        take(COST_PAIR_192, 256, 192, sms / 2, 1, true, 192);
+        take(COST_PAIR_128, 256, 128, sms / 2, 1, true, 128);
       }
     }
     if (can_split && a.mt == 0 && a.split == 0 && sms >= 128) {
-      take(cost(COST_SPLIT2, 256, 256, CLUSTERS4, 2), 256, 2, 2);
-      take(cost(COST_SPLIT4, 256, 256, CLUSTERS8, 4), 256, 2, 4);
+      take(COST_SPLIT2, 256, 256, CLUSTERS4, 2, true, 256);
+      take(COST_SPLIT4, 256, 256, CLUSTERS8, 4, true, 256);
     }
   }
   // A few rows of a K-major product: the kernel that streams the weight once through all SMs (skinny.cu), unless a tile kernel
-  // is expected to be faster. `mt`, `bn` and `split` ask for a tile kernel.
-  if (a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && plain && a.K > 0 && a.K % 8 == 0 && a.bn == 0 &&
-      a.mt == 0 && a.split == 0 && a.max_ctas == 0 && a.alpha != 0.f && few_rows_cost(a.M, a.N, a.K) <= few_tiles_cost(best, a.N, a.K))
+  // is expected to be faster. `mt`, `bn`, `split` and `pair_bn` ask for a tile kernel.
+  c.few = a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && plain && a.K > 0 && a.K % 8 == 0 && a.bn == 0 &&
+          a.mt == 0 && a.split == 0 && a.pair_bn == 0 && a.max_ctas == 0 && a.alpha != 0.f &&
+          few_rows_cost(a.M, a.N, a.K) <= few_tiles_cost(c.cost, a.N, a.K);
+  if (split_asked) c.splits = a.split;
+  return c;
+}
+
+// C[M,N] (+)= alpha * A * B^T with the operand layouts described in NpGemmArgs.
+// Returns 0 or a launch/setup error; device-side problems are reported via np_status_read.
+NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
+  const NpGemmArgs& a = *args;
+  if (a.M <= 0 || a.N <= 0) return 0;
+  if (!bind_context()) return 2;
+  if (check_gemm(a)) return 1;
+  const GemmChoice c = choose_gemm(a);
+  if (c.few)
     return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
                             a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
-  if (can_split && (a.split == 2 || a.split == 4)) splits = a.split;
-  if (bn == 256 && mt == 2 && can_pair)
-    return pbn == 128 && splits == 1   ? launch_gemm<128, true>(a, (cudaStream_t)stream)
-           : pbn == 192 && splits == 1 ? launch_gemm<192, true>(a, (cudaStream_t)stream)
-                                       : launch_gemm<256, true>(a, (cudaStream_t)stream, splits);
-  if (bn == 256) return launch_gemm<256, false>(a, (cudaStream_t)stream);
+  if (c.pair)
+    return c.bn == 128   ? launch_gemm<128, true>(a, (cudaStream_t)stream)
+           : c.bn == 192 ? launch_gemm<192, true>(a, (cudaStream_t)stream)
+                         : launch_gemm<256, true>(a, (cudaStream_t)stream, c.splits);
+  if (c.bn == 256) return launch_gemm<256, false>(a, (cudaStream_t)stream);
   return launch_gemm<128, false>(a, (cudaStream_t)stream);
+}
+
+template <int BN>
+static int launch_gemm2(const NpGemmArgs& a, const NpGemmArgs& b, int extra, cudaStream_t stream) {
+  PairMaps m;
+  GemmParams p;
+  PairSecond second;
+  CUtensorMap unused;
+  int rc = prepare_gemm<BN, true>(a, 1, m, unused, unused, p);
+  if (!rc) rc = prepare_gemm<BN, true>(b, 1, second.m, unused, unused, second.p);
+  if (rc) return rc;
+  second.extra = extra;
+  constexpr int SMEM = gemm_smem<BN, true>();
+  static NpPerDeviceOnce attr_once;
+  bool& attr_set = *attr_once.slot();
+  if (!attr_set) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_pair2_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return 400 + (int)e;
+    attr_set = true;
+  }
+  auto tiles = [](const NpGemmArgs& g) { return (long long)((g.M + 255) / 256) * ((g.N + BN - 1) / BN); };
+  const long long n = tiles(a) + tiles(b), pairs = n < num_sms() / 2 ? n : num_sms() / 2;
+  const bool busy = 2.0 * a.M * a.N * a.K + 2.0 * b.M * b.N * b.K > 2e10;   // 15 us and more
+  cudaError_t e = np_launch_if(busy, gemm_bf16_pair2_kernel<BN>, dim3((unsigned)(2 * pairs)), GEMM_THREADS, SMEM, stream, 2, m, p, second);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 500 + (int)e;
+}
+
+// Two independent products: in one launch where both are dense, run on pairs of CTAs and are expected to take less time that way,
+// else one after the other. `pair_bn` of the first asks for one launch with tiles of that many columns, `split` 1 or `mt` 2 of
+// the first for two launches.
+NP_API int np_gemm_bf16_two(const NpGemmArgs* first, const NpGemmArgs* second, void* stream) {
+  const NpGemmArgs &a = *first, &b = *second;
+  auto separate = [&] {
+    const int rc = np_gemm_bf16(first, stream);
+    return rc ? rc : np_gemm_bf16(second, stream);
+  };
+  auto dense = [](const NpGemmArgs& g) {
+    return g.M > 128 && g.N > 0 && g.K > 0 && g.mode == 0 && g.epilogue != 1 && !g.b_ready_flags && !g.push_src && !g.A_loc && !g.B_loc &&
+           g.m_rot == 0 && g.n_rot == 0 && !g.row_dst && !g.ready_flags && !g.done_counters && g.bn == 0 && g.mt == 0 && g.split == 0 &&
+           g.max_ctas == 0 && g.m_split == 0;
+  };
+  const int units = num_sms() / 2;
+  // Long products run at the power limit: SMs that idle let the others run faster, so there is nothing to fill (us, two launches /
+  // one: 4096 tokens, 2048 x 11264, 3.8e11 operations 261 / 256; 2048 x 32000, 1.1e12 799 / 846).
+  const bool long_run = 2.0 * a.M * a.N * a.K + 2.0 * b.M * b.N * b.K > 6e11 && a.pair_bn == 0;
+  if (!dense(a) || !dense(b) || b.pair_bn != 0 || units < 1 || long_run) return separate();
+  if (!bind_context()) return 2;
+  if (check_gemm(a) || check_gemm(b)) return 1;
+  // the longer contraction first
+  const bool swap = b.K > a.K;
+  const NpGemmArgs &x = swap ? b : a, &y = swap ? a : b;
+  const double sx = (x.K + BK - 1) / BK, sy = (y.K + BK - 1) / BK;
+  double best = a.pair_bn != 0 ? 1e30 : choose_gemm(a).cost + choose_gemm(b).cost;
+  int bn = 0, extra = 0;
+  auto take = [&](const TileCost& t, int cols) {   // the pair with the most to do
+    if (a.pair_bn != 0 && a.pair_bn != cols) return;
+    const int nx = (int)(((long long)(x.M + 255) / 256) * ((x.N + cols - 1) / cols));
+    const int ny = (int)(((long long)(y.M + 255) / 256) * ((y.N + cols - 1) / cols));
+    const int pairs = nx + ny < units ? nx + ny : units;
+    const double cx = sx * t.step + t.drain, cy = sy * t.step + t.drain;
+    const int ex = (int)(cx / cy);
+    // pair 0 has one of the first product's tiles more than pair r; behind each, the others have as much or less
+    const int r = nx % pairs, slack = pairs - r, rest = ny - (r == 0 ? 0 : ex < (ny + slack - 1) / slack ? ex * slack : ny);
+    auto dealt = [&](int at) { return rest > at ? (rest - at - 1) / pairs + 1 : 0; };
+    const double at_0 = ((nx + pairs - 1) / pairs) * cx + dealt(r == 0 ? 0 : slack) * cy;
+    const int before = ex < (ny + slack - 1) / slack ? ex : (ny + slack - 1) / slack;
+    const double at_r = r == 0 ? 0 : (nx / pairs) * cx + (before + dealt(0)) * cy;
+    const double most = at_0 > at_r ? at_0 : at_r;
+    if (t.fixed + most < best) { best = t.fixed + most; bn = cols; extra = ex; }
+  };
+  take(COST_PAIR, 256);
+  take(COST_PAIR_192, 192);
+  take(COST_PAIR_128, 128);
+  cudaStream_t st = (cudaStream_t)stream;
+  return bn == 256   ? launch_gemm2<256>(x, y, extra, st)
+         : bn == 192 ? launch_gemm2<192>(x, y, extra, st)
+         : bn == 128 ? launch_gemm2<128>(x, y, extra, st)
+                     : separate();
 }
 
 NP_API int np_status_read(int* out8) {

@@ -205,6 +205,7 @@ def lib():
         _LIB_ERR = str(e)
         raise KernelError(f"cannot load {LIB_PATH}: {e}") from e
     _LIB.np_gemm_bf16.argtypes = [C.POINTER(GemmArgs), c_void_p]
+    _LIB.np_gemm_bf16_two.argtypes = [C.POINTER(GemmArgs), C.POINTER(GemmArgs), c_void_p]
     _LIB.np_ep_dispatch.argtypes = [C.POINTER(DispatchArgs), c_void_p]
     _LIB.np_ep_combine.argtypes = [C.POINTER(CombineArgs), c_void_p]
     _LIB.np_gemm_fp8_block.argtypes = [C.POINTER(Fp8GemmArgs), c_void_p]

@@ -57,6 +57,29 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             return y.to(out_dtype or a.dtype)
         out.copy_((y + out.float()) if accumulate else y)
         return out
+    args, out = _gemm_args(a, b, a_mn, b_mn, out, out_dtype, accumulate, alpha)
+    M, N, K = args.M, args.N, args.K
+    # requests; 0 = choose. mt 2: 256 x 256 tiles on pairs of CTAs, split 2 or 4: parts of K there (bn 128: one-CTA tiles),
+    # pair_bn 128, 192 or 256: tiles of that many columns on pairs
+    args.bn, args.max_ctas, args.mt, args.split, args.pair_bn = bn, max_ctas, mt, split, pair_bn
+    if bias is not None:
+        assert bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous()
+        args.bias = bias.data_ptr()
+    if residual is not None:
+        assert not accumulate and residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
+        args.accumulate, args.Cin, args.ldcin = 1, residual.data_ptr(), residual.stride(0)
+    rc = _lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream()))
+    if rc != 0:
+        raise _lib.KernelError(
+            f"gemm_bf16 failed with code {rc}: M={M} N={N} K={K} a_mn={a_mn} b_mn={b_mn} a={tuple(a.shape)}/"
+            f"{a.stride()} b={tuple(b.shape)}/{b.stride()} out={tuple(out.shape)}/{out.stride()} {out.dtype} "
+            f"ptrs={a.data_ptr() % 256},{b.data_ptr() % 256},{out.data_ptr() % 256} bn={bn}")
+    _lib.LAUNCHES += 1
+    return out
+
+
+def _gemm_args(a, b, a_mn, b_mn, out, out_dtype, accumulate, alpha):
+    """Arguments of one product (checked) and its output tensor."""
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "kernel path is bf16"
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
     M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
@@ -75,23 +98,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     assert out.dtype in (torch.float32, torch.bfloat16)
     args.accumulate = int(accumulate)
     args.alpha = alpha
-    # requests; 0 = choose. mt 2: 256 x 256 tiles on pairs of CTAs, split 2 or 4: parts of K there (bn 128: one-CTA tiles),
-    # pair_bn 128, 192 or 256: tiles of that many columns on pairs
-    args.bn, args.max_ctas, args.mt, args.split, args.pair_bn = bn, max_ctas, mt, split, pair_bn
-    if bias is not None:
-        assert bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous()
-        args.bias = bias.data_ptr()
-    if residual is not None:
-        assert not accumulate and residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
-        args.accumulate, args.Cin, args.ldcin = 1, residual.data_ptr(), residual.stride(0)
-    rc = _lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream()))
-    if rc != 0:
-        raise _lib.KernelError(
-            f"gemm_bf16 failed with code {rc}: M={M} N={N} K={K} a_mn={a_mn} b_mn={b_mn} a={tuple(a.shape)}/"
-            f"{a.stride()} b={tuple(b.shape)}/{b.stride()} out={tuple(out.shape)}/{out.stride()} {out.dtype} "
-            f"ptrs={a.data_ptr() % 256},{b.data_ptr() % 256},{out.data_ptr() % 256} bn={bn}")
-    _lib.LAUNCHES += 1
-    return out
+    return args, out
 
 
 def gemm_swiglu(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, save_gu: bool = True):
@@ -124,14 +131,8 @@ def gemm_swiglu(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, sa
     return h, gu
 
 
-def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor, pair_bn: int = 0) -> torch.Tensor:
-    """``[d gate | d up]`` of ``h = silu(gate) * up`` for ``dh = dy @ w2`` and ``gu = [gate | up]``, without forming ``dh``:
-    the gradient of the activation is the epilogue of the GEMM (``dy [M, D]``, ``w2 [D, F]``, ``gu [M, 2F]``)."""
+def _glu_bwd_args(dy, w2, gu):
     M, F = dy.shape[0], w2.shape[1]
-    if not _use_kernel(dy):
-        from .activation import glu_bwd
-
-        return glu_bwd(gu, gemm_ref(dy, w2, b_mn=True))
     assert dy.dtype == w2.dtype == gu.dtype == torch.bfloat16, "kernel path is bf16"
     assert dy.shape[1] == w2.shape[0] and gu.shape == (M, 2 * F) and dy.stride(1) == w2.stride(1) == gu.stride(1) == 1
     out = torch.empty((M, 2 * F), device=dy.device, dtype=torch.bfloat16)
@@ -140,9 +141,42 @@ def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor, pair_bn: 
     args.lda, args.ldb, args.ldc, args.ldc2 = dy.stride(0), w2.stride(0), 2 * F, gu.stride(0)
     args.a_rows, args.b_rows = M, w2.shape[0]
     args.M, args.N, args.K = M, F, dy.shape[1]
-    args.b_mn, args.epilogue, args.alpha, args.pair_bn = 1, 2, 1.0, pair_bn
+    args.b_mn, args.epilogue, args.alpha = 1, 2, 1.0
+    return args, out
+
+
+def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor, pair_bn: int = 0) -> torch.Tensor:
+    """``[d gate | d up]`` of ``h = silu(gate) * up`` for ``dh = dy @ w2`` and ``gu = [gate | up]``, without forming ``dh``:
+    the gradient of the activation is the epilogue of the GEMM (``dy [M, D]``, ``w2 [D, F]``, ``gu [M, 2F]``)."""
+    if not _use_kernel(dy):
+        from .activation import glu_bwd
+
+        return glu_bwd(gu, gemm_ref(dy, w2, b_mn=True))
+    args, out = _glu_bwd_args(dy, w2, gu)
+    args.pair_bn = pair_bn
     _lib.check(_lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream())), "gemm_glu_bwd")
     return out
+
+
+def gemm_dgrad_wgrad(dy: torch.Tensor, w: torch.Tensor, x: torch.Tensor, *, out: torch.Tensor | None = None,
+                     accumulate: bool = False, gu: torch.Tensor | None = None, pair_bn: int = 0, mt: int = 0):
+    """``(dy @ w, dy.T @ x)`` for ``dy [M, N]``, ``w [N, K]``, ``x [M, K]``: the two gradients of a linear layer, in one launch
+    where that is expected to be faster than two. The second goes to ``out`` (added with ``accumulate``), by default a new
+    tensor in the dtype of ``w``. ``gu``: pre-activations ``[gate | up]`` with ``x = silu(gate) * up``; the first result is then
+    ``[d gate | d up]`` (``gemm_glu_bwd``). ``pair_bn`` and ``mt`` ask for one launch with tiles of that many columns, two launches."""
+    if not _use_kernel(dy):
+        dx = gemm(dy, w, b_mn=True) if gu is None else gemm_glu_bwd(dy, w, gu)
+        return dx, gemm(dy, x, a_mn=True, b_mn=True, out=out, out_dtype=w.dtype if out is None else None, accumulate=accumulate)
+    a0, dx = _gemm_args(dy, w, False, True, None, None, False, 1.0) if gu is None else _glu_bwd_args(dy, w, gu)
+    a1, dw = _gemm_args(dy, x, True, True, out, w.dtype, accumulate, 1.0)
+    a0.pair_bn, a0.mt = pair_bn, mt
+    rc = _lib.lib().np_gemm_bf16_two(C.byref(a0), C.byref(a1), C.c_void_p(_lib.stream()))
+    if rc != 0:
+        raise _lib.KernelError(f"gemm_bf16_two failed with code {rc}: dy={tuple(dy.shape)}/{dy.stride()} w={tuple(w.shape)}/"
+                               f"{w.stride()} x={tuple(x.shape)}/{x.stride()} dw={tuple(dw.shape)}/{dw.stride()} {dw.dtype} "
+                               f"ptrs={dy.data_ptr() % 256},{w.data_ptr() % 256},{x.data_ptr() % 256},{dw.data_ptr() % 256}")
+    _lib.LAUNCHES += 1
+    return dx, dw
 
 
 # Zero-bubble pipeline schedules split a backward pass into B (input gradients, on the critical path between
@@ -182,9 +216,23 @@ def run_deferred_wgrads(queue: list) -> None:
                 w.grad = g if w.grad is None else w.grad + g
 
 
+def _deferred(w: torch.Tensor) -> bool:
+    return _DEFER is not None and (w.is_leaf or hasattr(w, "main_grad"))
+
+
+def _main_grad_done(w: torch.Tensor) -> None:
+    """``w.main_grad`` has its gradient: the next one is added, and whoever waits for it is told."""
+    w._main_grad_dirty = True
+    for q in getattr(w, "_covers", None) or (w,):  # a fused view stands for several parameters
+        q._main_grad_dirty = True
+        cb = getattr(q, "_grad_ready_cb", None)      # the arena's overlapped gradient reduction (optim/arena.py)
+        if cb is not None:
+            cb(q)
+
+
 def _wgrad_into(w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
     """dW[N, K] = dy^T x, accumulated into ``w.main_grad`` when present; returns the autograd grad."""
-    if _DEFER is not None and (w.is_leaf or hasattr(w, "main_grad")):
+    if _deferred(w):
         # a weight that is itself computed (two parameters concatenated for one GEMM) has no ``.grad`` to fill later:
         # its gradient has to go back through autograd now, so only leaves and arena views are deferred
         _DEFER.append((w, dy2, x2))
@@ -193,14 +241,30 @@ def _wgrad_into(w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
     if mg is not None:
         first = not getattr(w, "_main_grad_dirty", False)
         gemm(dy2, x2, a_mn=True, b_mn=True, out=mg, accumulate=not first)
-        w._main_grad_dirty = True
-        for q in getattr(w, "_covers", None) or (w,):  # a fused view stands for several parameters
-            q._main_grad_dirty = True
-            cb = getattr(q, "_grad_ready_cb", None)      # the arena's overlapped gradient reduction (optim/arena.py)
-            if cb is not None:
-                cb(q)
+        _main_grad_done(w)
         return None
     return gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=w.dtype if w.is_cuda else None)
+
+
+def _both_grads(w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor, gu: torch.Tensor | None = None):
+    """Input gradient (with ``gu``: the gradient of its pre-activations) and what ``_wgrad_into`` returns for ``w``."""
+    if not _use_kernel(dy2) or _deferred(w):
+        dx = gemm(dy2, w, b_mn=True) if gu is None else gemm_glu_bwd(dy2, w, gu)
+        return dx, _wgrad_into(w, dy2, x2)
+    mg = getattr(w, "main_grad", None)
+    if mg is None:
+        return gemm_dgrad_wgrad(dy2, w, x2, gu=gu)
+    dx, _ = gemm_dgrad_wgrad(dy2, w, x2, out=mg, accumulate=getattr(w, "_main_grad_dirty", False), gu=gu)
+    _main_grad_done(w)
+    return dx, None
+
+
+def _linear_grads(ctx, w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
+    """``(dx, dw)`` of ``x2 @ w.T`` as far as they are asked for (inputs 0 and 1 of the autograd function)."""
+    want_dw = ctx.needs_input_grad[1] or hasattr(w, "main_grad")
+    if ctx.needs_input_grad[0] and want_dw:
+        return _both_grads(w, dy2, x2)
+    return (gemm(dy2, w, b_mn=True) if ctx.needs_input_grad[0] else None), (_wgrad_into(w, dy2, x2) if want_dw else None)
 
 
 class _Linear(torch.autograd.Function):
@@ -217,12 +281,8 @@ class _Linear(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        x2 = x.reshape(-1, x.shape[-1])
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, w, b_mn=True).reshape(x.shape)
-        dw = _wgrad_into(w, dy2, x2) if (ctx.needs_input_grad[1] or hasattr(w, "main_grad")) else None
-        return dx, dw
+        dx, dw = _linear_grads(ctx, w, dy2, x.reshape(-1, x.shape[-1]))
+        return None if dx is None else dx.reshape(x.shape), dw
 
 
 class _LinearBias(torch.autograd.Function):
@@ -242,9 +302,8 @@ class _LinearBias(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        x2 = x.reshape(-1, x.shape[-1])
-        dx = gemm(dy2, w, b_mn=True).reshape(x.shape) if ctx.needs_input_grad[0] else None
-        dw = _wgrad_into(w, dy2, x2) if (ctx.needs_input_grad[1] or hasattr(w, "main_grad")) else None
+        dx, dw = _linear_grads(ctx, w, dy2, x.reshape(-1, x.shape[-1]))
+        dx = None if dx is None else dx.reshape(x.shape)
         db = dy2.float().sum(0).to(ctx.bias_dtype) if ctx.needs_input_grad[2] else None
         return dx, dw, db
 
@@ -301,15 +360,16 @@ class _SwiGLUFeedForward(torch.autograd.Function):
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         x2 = x.reshape(-1, x.shape[-1])
-        dw2 = _wgrad_into(w2, dy2, h) if (ctx.needs_input_grad[2] or hasattr(w2, "main_grad")) else None
-        dx = dw13 = None
-        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or hasattr(w13, "main_grad"):
+        want_dw2 = ctx.needs_input_grad[2] or hasattr(w2, "main_grad")
+        dx = dw13 = dw2 = None
+        if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or hasattr(w13, "main_grad")):
+            return None, None, _wgrad_into(w2, dy2, h) if want_dw2 else None, None
+        if want_dw2:
+            dgu, dw2 = _both_grads(w2, dy2, h, gu)
+        else:
             dgu = gemm_glu_bwd(dy2, w2, gu)
-            if ctx.needs_input_grad[0]:
-                dx = gemm(dgu, w13, b_mn=True).view(x.shape)
-            if ctx.needs_input_grad[1] or hasattr(w13, "main_grad"):
-                dw13 = _wgrad_into(w13, dgu, x2)
-        return dx, dw13, dw2, None
+        dx, dw13 = _linear_grads(ctx, w13, dgu, x2)
+        return None if dx is None else dx.view(x.shape), dw13, dw2, None
 
 
 def _plain_weight(w: torch.Tensor) -> bool:

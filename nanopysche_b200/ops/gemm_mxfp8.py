@@ -221,8 +221,6 @@ class _MXLinear(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w):
-        from .gemm import gemm
-
         x2 = x.reshape(-1, x.shape[-1])
         x2 = x2 if x2.is_contiguous() else x2.contiguous()
         xq, sx = mx_quantize(x2)
@@ -230,19 +228,17 @@ class _MXLinear(torch.autograd.Function):
         y = gemm_mxfp8(xq, sx, wq, sw)
         ctx.save_for_backward(x2, w)
         ctx.x_shape = x.shape
-        ctx.gemm = gemm
         return y.view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        from .gemm import _wgrad_into
+        from .gemm import _linear_grads
 
         x2, w = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
-        dx = ctx.gemm(dy2, w, b_mn=True).view(ctx.x_shape) if ctx.needs_input_grad[0] else None
-        dw = _wgrad_into(w, dy2, x2) if (ctx.needs_input_grad[1] or hasattr(w, "main_grad")) else None
-        return dx, dw
+        dx, dw = _linear_grads(ctx, w, dy2, x2)
+        return None if dx is None else dx.view(ctx.x_shape), dw
 
 
 def mx_linear_supported(x: torch.Tensor, w: torch.Tensor) -> bool:

@@ -87,6 +87,30 @@ def test_pair_glu_bwd_tiles(M, F, K, pair_bn):
     assert rel(gemm_glu_bwd(dy, w2, gu, pair_bn=pair_bn), torch.cat([g.grad, u.grad], 1)) < 3e-3
 
 
+# both gradients of a linear layer in one launch: either contraction the longer one, fewer tiles than pairs of CTAs and several
+# rounds of them that do not come out even, M at which a choice of its own is made, sizes off the tiles
+@pytest.mark.parametrize("T,N,K", [(264, 136, 200), (136, 1032, 264), (2048, 1024, 1024), (2331, 2048, 2048), (4096, 2304, 768), (300, 8200, 1000)])
+@pytest.mark.parametrize("pair_bn", [0, 128, 192, 256])
+def test_two_gradients_in_one_launch(T, N, K, pair_bn):
+    from nanopysche_b200.ops.gemm import gemm_dgrad_wgrad, gemm_glu_bwd
+
+    torch.manual_seed(T + N)
+    dy, x = torch.randn(T, N, device="cuda").bfloat16(), torch.randn(T, K, device="cuda").bfloat16()
+    w = (torch.randn(N, K, device="cuda") * N ** -0.5).bfloat16()
+    acc = torch.randn(N, K, device="cuda")
+    want = dy.float().t() @ x.float()
+    for out, add in ((None, None), (torch.full_like(acc, float("nan")), None), (acc.clone(), acc)):
+        dx, dw = gemm_dgrad_wgrad(dy, w, x, out=out, accumulate=add is not None, pair_bn=pair_bn)
+        assert rel(dx, dy.float() @ w.float()) < 3e-3
+        assert rel(dw, want if add is None else want + add) < (3e-3 if out is None else 2e-5)
+        dx2, dw2 = gemm_dgrad_wgrad(dy, w, x, out=None if out is None else (torch.empty_like(acc) if add is None else add.clone()),
+                                    accumulate=add is not None, mt=2)      # two launches
+        assert rel(dx, dx2) < 2e-3 and rel(dw, dw2) < (2e-3 if out is None else 1e-6)
+    gu = torch.randn(T, 2 * K, device="cuda").bfloat16()
+    dgu, dw = gemm_dgrad_wgrad(dy, w, x, out=torch.empty_like(acc), gu=gu, pair_bn=pair_bn)
+    assert rel(dgu, gemm_glu_bwd(dy, w, gu)) < 2e-3 and rel(dw, want) < 2e-5
+
+
 @pytest.mark.parametrize("M,F,K", [(256, 128, 64), (300, 264, 200), (1000, 704, 512)])
 def test_pair_swiglu(M, F, K):
     from nanopysche_b200.ops.gemm import gemm_swiglu
