@@ -215,8 +215,10 @@ __global__ void __launch_bounds__(32) router_aux_kernel(const int* counts, const
 
 // dlogits[t, :] from d(weights) and d(aux): aux = coef_lb * E * sum_i f_i * mean_t p[t,i]
 //                                                + coef_z * mean_t lse_t^2
-// f (fractions, [E]) is treated as a constant, as autograd does for the reference's one_hot count.
-__global__ void __launch_bounds__(256) router_bwd_kernel(const float* logits,
+// f (fractions, [E]) is treated as a constant, as autograd does for the reference's one_hot count. EMAX bounds E at compile time so
+// that a token's logits and gradients stay in registers (in local memory: 9.4 us at 4096 tokens and 8 experts).
+template <int EMAX>
+__global__ void __launch_bounds__(128) router_bwd_kernel(const float* logits,
                                                          const float* score_bias,
                                                          const float* weights,
                                                          const int* indices,
@@ -228,53 +230,65 @@ __global__ void __launch_bounds__(256) router_bwd_kernel(const float* logits,
   np::pdl_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
-  float l[MAX_E], dl[MAX_E];
+  float l[EMAX], dl[EMAX];
   float mx = -INFINITY;
-#pragma unroll 1
-  for (int e = 0; e < E; ++e) {
-    l[e] = logits[(size_t)t * E + e] + (score_bias ? score_bias[e] : 0.f);
+#pragma unroll
+  for (int e = 0; e < EMAX; ++e) {
+    l[e] = e < E ? logits[(size_t)t * E + e] + (score_bias ? score_bias[e] : 0.f) : -INFINITY;
     mx = fmaxf(mx, l[e]);
     dl[e] = 0.f;
   }
   float se = 0.f;
-#pragma unroll 1
-  for (int e = 0; e < E; ++e) se += __expf(l[e] - mx);
+#pragma unroll
+  for (int e = 0; e < EMAX; ++e) se += e < E ? __expf(l[e] - mx) : 0.f;
   const float lse = mx + logf(se);
   const float da = daux ? daux[0] : 0.f;
   if (da != 0.f) {
     float fp = 0.f;
-#pragma unroll 1
-    for (int e = 0; e < E; ++e) fp += f[e] * __expf(l[e] - lse);
-#pragma unroll 1
-    for (int e = 0; e < E; ++e) {
+#pragma unroll
+    for (int e = 0; e < EMAX; ++e) fp += e < E ? f[e] * __expf(l[e] - lse) : 0.f;
+#pragma unroll
+    for (int e = 0; e < EMAX; ++e) {
+      if (e >= E) break;
       const float p = __expf(l[e] - lse);
       dl[e] += da * (coef_lb * (float)E / (float)T * p * (f[e] - fp) + coef_z * 2.f * lse / (float)T * p);
     }
   }
   if (dweights) {
-    float wsum = 0.f;
-    for (int k = 0; k < K; ++k) wsum += weights[(size_t)t * K + k] * dweights[(size_t)t * K + k];
+    auto logit = [&](int e) {   // by selection: a variable index would put the array into local memory
+      float v = l[0];
+#pragma unroll
+      for (int i = 1; i < EMAX; ++i) v = e == i ? l[i] : v;
+      return v;
+    };
+    float wsum = 0.f, ssum = 1e-8f;
+    for (int k = 0; k < K; ++k) {
+      wsum += weights[(size_t)t * K + k] * dweights[(size_t)t * K + k];
+      if (gating == 1) ssum += 1.f / (1.f + __expf(-logit(indices[(size_t)t * K + k])));
+    }
     for (int k = 0; k < K; ++k) {
       const int e = indices[(size_t)t * K + k];
       const float w = weights[(size_t)t * K + k], dw = dweights[(size_t)t * K + k];
+      float add;
       if (gating == 0) {
-        dl[e] += w * (dw - wsum);
+        add = w * (dw - wsum);
       } else {
         // w_k = s_k / (sum s + eps); ds_k = (dw_k - sum_j w_j dw_j) / (sum s + eps); dl = ds * s(1-s)
-        const float s = 1.f / (1.f + __expf(-l[e]));
-        float ssum = 1e-8f;
-        for (int j = 0; j < K; ++j) ssum += 1.f / (1.f + __expf(-l[indices[(size_t)t * K + j]]));
-        dl[e] += (dw - wsum) / ssum * s * (1.f - s);
+        const float s = 1.f / (1.f + __expf(-logit(e)));
+        add = (dw - wsum) / ssum * s * (1.f - s);
       }
+#pragma unroll
+      for (int i = 0; i < EMAX; ++i) dl[i] += e == i ? add : 0.f;
     }
   }
-#pragma unroll 1
-  for (int e = 0; e < E; ++e) dlogits[(size_t)t * E + e] = dl[e];
+#pragma unroll
+  for (int e = 0; e < EMAX; ++e)
+    if (e < E) dlogits[(size_t)t * E + e] = dl[e];
 }
 
-// partial[c, e, d] = sum over the chunk's tokens of dl[t, e] * x[t, d]. CTA = 64 column threads (8 columns each) x 4
-// token lanes; a lane walks every fourth token of the chunk with four row loads in flight, the lanes are summed
-// through shared memory.
+// partial[c, e, d] = sum over the chunk's tokens of dl[t, e] * x[t, d], and behind them partial[c, E * D + e] = sum of dl[t, e]. CTA =
+// 64 column threads (8 columns each) x 4 token lanes; a lane walks every fourth token of the chunk with four row loads in
+// flight, the lanes are summed through shared memory.
 template <int EB>
 __global__ void __launch_bounds__(256) router_dgate_kernel(const float* dl,
                                                            const __nv_bfloat16* x,
@@ -285,6 +299,18 @@ __global__ void __launch_bounds__(256) router_dgate_kernel(const float* dl,
   const int c = blockIdx.y;
   const int t0 = c * chunk, t1 = min(T, t0 + chunk);
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+  const long long part = (long long)E * D + (E + 3) / 4 * 4;   // floats of a partial: whole vectors
+  if (blockIdx.x == 0) {   // column sums of dl (E <= 64)
+    __shared__ float s_b[4][64];
+    float s = 0.f;
+    if (tx < E) {
+#pragma unroll 4
+      for (int t = t0 + ty; t < t1; t += 4) s += dl[(size_t)t * E + tx];
+    }
+    s_b[ty][tx] = s;
+    __syncthreads();
+    if (ty == 0 && tx < E) partial[c * part + (long long)E * D + tx] = (s_b[0][tx] + s_b[1][tx]) + (s_b[2][tx] + s_b[3][tx]);
+  }
   const int d = (blockIdx.x * 64 + tx) * 8;
   const bool col_ok = d < D;
   for (int e0 = 0; e0 < E; e0 += EB) {
@@ -344,7 +370,7 @@ __global__ void __launch_bounds__(256) router_dgate_kernel(const float* dl,
         if (e0 + e < E) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) acc[e][j] += red[0][tx][e * 8 + j];
-          float* dst = partial + ((size_t)c * E + e0 + e) * D + d;
+          float* dst = partial + c * part + (size_t)(e0 + e) * D + d;
           *reinterpret_cast<float4*>(dst) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
           *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[e][4], acc[e][5], acc[e][6], acc[e][7]);
         }
@@ -424,11 +450,12 @@ __global__ void __launch_bounds__(256, 2) router_dx_reg_kernel(const float* dl, 
   }
 }
 
-__global__ void colsum2_kernel(const float* partial, float* __restrict__ out, int parts,
-                               long long cols, int accumulate) {
+// column sums of `parts` rows (`cols` floats apart): the first n0 columns to out0, n1 behind them to out1 (added with `accumulate`)
+__global__ void colsum2_kernel(const float* partial, float* __restrict__ out0, float* __restrict__ out1, int parts, long long cols,
+                               long long n0, int n1, int accumulate) {
   np::pdl_begin();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+  if (c >= n0 + n1) return;
   float a8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   int p = 0;
   for (; p + 7 < parts; p += 8) {   // eight independent loads in flight
@@ -437,33 +464,8 @@ __global__ void colsum2_kernel(const float* partial, float* __restrict__ out, in
   }
   for (; p < parts; ++p) a8[0] += partial[(size_t)p * cols + c];
   const float s = ((a8[0] + a8[1]) + (a8[2] + a8[3])) + ((a8[4] + a8[5]) + (a8[6] + a8[7]));
-  out[c] = accumulate ? out[c] + s : s;
-}
-
-// out[c] (+)= sum over rows of a[r, c] for a narrow matrix (cols <= 64): 1024 threads, thread -> (row group, col)
-__global__ void __launch_bounds__(1024) colsum_narrow_kernel(const float* a, float* __restrict__ out,
-                                                             int rows, int cols, int accumulate) {
-  np::pdl_begin();
-  __shared__ float red[1024];
-  const int c = threadIdx.x % cols, g = threadIdx.x / cols, ng = 1024 / cols;
-  float s = 0.f;
-  if (g < ng) {
-    float a4[4] = {0.f, 0.f, 0.f, 0.f};
-    int r = g;
-    for (; r + 3 * ng < rows; r += 4 * ng) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a4[u] += a[(size_t)(r + u * ng) * cols + c];
-    }
-    for (; r < rows; r += ng) a4[0] += a[(size_t)r * cols + c];
-    s = (a4[0] + a4[1]) + (a4[2] + a4[3]);
-  }
-  red[threadIdx.x] = (g < ng) ? s : 0.f;
-  __syncthreads();
-  if (threadIdx.x < cols) {
-    float t = 0.f;
-    for (int i = 0; i < ng; ++i) t += red[i * cols + threadIdx.x];
-    out[threadIdx.x] = accumulate ? out[threadIdx.x] + t : t;
-  }
+  float* out = c < n0 ? out0 + c : out1 + (c - n0);
+  *out = accumulate ? *out + s : s;
 }
 
 // ------------------------------------------------------------------ capacity / positions
@@ -476,6 +478,14 @@ __global__ void __launch_bounds__(1024) colsum_narrow_kernel(const float* a, flo
 // counts_kept[E], drops[E] (tokens beyond capacity per expert), n_dropped[1].
 struct U64x4 {
   unsigned long long w[4];
+  // word q, by selection: indexed with a variable, the counters of a thread would live in local memory
+  __device__ __forceinline__ unsigned long long get(int q) const {
+    return q == 0 ? w[0] : q == 1 ? w[1] : q == 2 ? w[2] : w[3];
+  }
+  __device__ __forceinline__ void add(int q, unsigned long long v) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] += q == i ? v : 0ull;
+  }
 };
 __device__ __forceinline__ U64x4 block_excl_scan4(const U64x4& v, int nw_used, U64x4* s_warp, U64x4* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -556,7 +566,7 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* indices,
         if (phase == 1 && !(use_smem ? s_keep[t] : keep[t])) continue;
         for (int k = 0; k < K; ++k) {
           const int e = idx[(size_t)t * K + k] - e0;
-          if (e >= 0 && e < n_e) loc.w[e / EPW] += 1ull << (FB * (e % EPW));
+          if (e >= 0 && e < n_e) loc.add(e / EPW, 1ull << (FB * (e % EPW)));
         }
       }
       U64x4 total;
@@ -571,8 +581,8 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* indices,
             continue;
           }
           const int q = e / EPW, sh = FB * (e % EPW);
-          const int pos = (int)((run.w[q] >> sh) & FMASK);
-          run.w[q] += 1ull << sh;
+          const int pos = (int)((run.get(q) >> sh) & FMASK);
+          run.add(q, 1ull << sh);
           if (phase == 0) {
             if (pos >= capacity) {   // only ever written to 0, by the thread that owns the token
               if (use_smem) s_keep[t] = 0; else keep[t] = 0;
@@ -584,7 +594,7 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* indices,
       }
       if ((int)threadIdx.x < n_e) {
         const int e = threadIdx.x;
-        const int c = (int)((total.w[e / EPW] >> (FB * (e % EPW))) & FMASK);
+        const int c = (int)((total.get(e / EPW) >> (FB * (e % EPW))) & FMASK);
         if (phase == 0) {
           drops[e0 + e] = c > capacity ? c - capacity : 0;
         } else {
@@ -644,6 +654,13 @@ struct DispatchParams {
   int* zero_ctr;               // [n_ranks] tile counters of the pushing GEMM behind this dispatch, set to zero; may be nullptr
 };
 
+// Order what was written before what follows: for peers, or on this GPU when it is the only rank. A system-wide fence takes some
+// 3 us, and there were four of them one after the other.
+__device__ __forceinline__ void rank_fence(int n_ranks) {
+  if (n_ranks > 1) __threadfence_system();
+  else __threadfence();
+}
+
 __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p) {
   np::pdl_begin();
   if (p.zero_ctr && blockIdx.x == 0)
@@ -662,8 +679,8 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p
     long long ret = -1;
     if (!is_pad) {
       pos = p.slot_pos[it];
-      if (pos < 0) continue;
       e = p.indices[it];
+      if (pos < 0) continue;
       NP_DBG_SKIP_UNLESS(e >= 0 && e < p.E, KID_DISPATCH, e)
       src = p.x + (size_t)(it / p.K) * p.D;
       if (p.slot_scale) sc = p.slot_scale[it];
@@ -759,13 +776,13 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p
     if (p.write_meta && lane == 0) p.peer_row_dst[peer][row] = ret;
   }
   // ---- completion: last CTA publishes the block table and releases the epoch flags
-  __threadfence_system();
+  rank_fence(p.n_ranks);
   __syncthreads();
   __shared__ int s_last;
   if (threadIdx.x == 0) s_last = (atomicAdd(p.done_ctr, 1) == (int)gridDim.x - 1);
   __syncthreads();
   if (!s_last) return;
-  __threadfence_system();
+  rank_fence(p.n_ranks);
   const int bpr = p.region_rows >> 7;  // blocks per region
   if (p.write_meta) {
     for (int i = threadIdx.x; i < p.E * bpr; i += blockDim.x) {
@@ -782,10 +799,14 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(const DispatchParams p
       p.peer_src_blocks[peer][p.my_rank] = nb;
     }
   }
-  __threadfence_system();
+  rank_fence(p.n_ranks);
   __syncthreads();
-  for (int peer = threadIdx.x; peer < p.n_ranks; peer += blockDim.x)
-    np::st_release_sys(p.peer_flags[peer] + p.my_rank, p.epoch + (p.epoch_base ? *p.epoch_base : 0));
+  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);
+  if (p.n_ranks == 1) {
+    if (threadIdx.x == 0) np::st_release_gpu(p.peer_flags[0], epoch);
+  } else {
+    for (int peer = threadIdx.x; peer < p.n_ranks; peer += blockDim.x) np::st_release_sys(p.peer_flags[peer] + p.my_rank, epoch);
+  }
   if (threadIdx.x == 0) *p.done_ctr = 0;
 }
 
@@ -954,25 +975,32 @@ NP_API int np_router_bwd(const float* logits, const float* score_bias, const flo
                          float* dlogits, int T, int E, int K, int gating, void* stream) {
   if (E > MAX_E || K > MAX_K) return 1;
   if (T <= 0) return 0;
-  np_launch(router_bwd_kernel, (T + 255) / 256, 256, 0, (cudaStream_t)stream, 1, logits, score_bias, weights, indices, dweights,
-                                                                       f, daux, coef_lb, coef_z, dlogits, T, E, K,
-                                                                       gating);
+#define RBWD(EM) np_launch(router_bwd_kernel<EM>, (T + 127) / 128, 128, 0, (cudaStream_t)stream, 1, logits, score_bias, weights, \
+      indices, dweights, f, daux, coef_lb, coef_z, dlogits, T, E, K, gating)
+  if (E <= 8) RBWD(8);
+  else if (E <= 16) RBWD(16);
+  else if (E <= 32) RBWD(32);
+  else RBWD(64);
+#undef RBWD
   CHECK_LAUNCH();
 }
 
-NP_API int np_router_dgate_parts(int T) { return (T + 63) / 64; }
-// scratch: fp32 [np_router_dgate_parts(T), E, D]; dwg[E, D] (+)= dl^T x ; dbias[E] (+)= column sums of dl.
+// Tokens of a partial sum: few enough that a small batch has CTAs for the chip (512 x 768, 8 experts, with the sum over the parts: 64 tokens 12.3 us, 16 tokens 7.5), many
+// enough that the partials of a large one stay small beside x.
+static int dgate_chunk(int T) { return T <= 1024 ? 16 : 64; }
+NP_API int np_router_dgate_parts(int T) { return (T + dgate_chunk(T) - 1) / dgate_chunk(T); }
+// scratch: fp32 [np_router_dgate_parts(T), E * D + E, the latter in whole fours]; dwg[E, D] (+)= dl^T x ; dbias[E] (+)= column sums of dl.
 NP_API int np_router_dgate(const float* dl, const void* x, float* dwg, float* dbias, float* scratch, int T, int D,
                            int E, int accumulate, void* stream) {
-  if (D % 8) return 1;
+  if (D % 8 || E > MAX_E) return 1;
   if (T <= 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
   const int parts = np_router_dgate_parts(T);
   dim3 grid((D / 8 + 63) / 64, parts);
-  np_launch(router_dgate_kernel<8>, grid, 256, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch, T, D, E, 64);
-  const long long cols = (long long)E * D;
-  np_launch(colsum2_kernel, (int)((cols + 63) / 64), 64, 0, s, 1, scratch, dwg, parts, cols, accumulate);
-  if (dbias) np_launch(colsum_narrow_kernel, 1, 1024, 0, s, 1, dl, dbias, T, E, accumulate);
+  np_launch(router_dgate_kernel<8>, grid, 256, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch, T, D, E, dgate_chunk(T));
+  const long long n = (long long)E * D;
+  np_launch(colsum2_kernel, (int)((n + E + 63) / 64), 64, 0, s, 1, scratch, dwg, dbias, parts, n + (E + 3) / 4 * 4, n,
+            dbias ? E : 0, accumulate);
   CHECK_LAUNCH();
 }
 
@@ -1040,7 +1068,7 @@ NP_API int np_ep_dispatch(const NpDispatchArgs* a, void* stream) {
   p.epoch_base = a->epoch_base; p.zero_ctr = a->zero_ctr;
   const int items = a->T * a->K + a->E * 128;
   int grid = (items + 7) / 8;
-  const int cap = a->max_ctas > 0 ? a->max_ctas : 148 * 4;
+  const int cap = a->max_ctas > 0 ? a->max_ctas : 148 * 8;   // a row per warp as long as they fit the chip at once
   if (grid > cap) grid = cap;
   if (grid < 1) grid = 1;
   np_launch(ep_dispatch_kernel, grid, 256, 0, (cudaStream_t)stream, 1, p);

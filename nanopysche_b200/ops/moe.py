@@ -70,7 +70,7 @@ class _Router(torch.autograd.Function):
         _lib.call("router_bwd", logits, sb if has_sb else None, weights, indices, dw, f, da, 1.0, coef_z, dl, T, E, K,
                   gating)
         parts = _lib.lib().np_router_dgate_parts(T)
-        scratch = torch.empty((parts, E, D), device=x2.device, dtype=torch.float32)
+        scratch = torch.empty((parts, E * D + (E + 3) // 4 * 4), device=x2.device, dtype=torch.float32)
         new = torch.empty if T > 0 else torch.zeros    # no tokens: the kernels below do nothing
         dgw = new(gate_w.shape, device=x2.device, dtype=gate_w.dtype)
         dgb = new(E, device=x2.device, dtype=torch.float32)
