@@ -1,4 +1,5 @@
-"""Build the sm_100a CUDA library in-tree (``nanopysche_b200/lib/libnpb200.so``).
+"""Build the sm_100a CUDA library (``nanopysche_b200/lib/libnpb200.so``) and the native host module that calls it from torch
+(``lib/npb200_host.so``) in-tree.
 
 Every ``csrc/*.cu`` file is compiled with nvcc for ``compute_100a/sm_100a`` (relocatable device
 code, one object per file, in parallel) and linked into one shared library that ``ops/_lib.py``
@@ -21,6 +22,7 @@ CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 OBJ_DIR = LIB_DIR / "obj"
 LIB_PATH = LIB_DIR / "libnpb200.so"
+HOST_PATH = LIB_DIR / "npb200_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -61,6 +63,41 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool) -> tuple[str, i
     return src.name, proc.returncode, proc.stdout + proc.stderr
 
 
+def build_host(force: bool = False) -> Path:
+    """Compile (if stale) the native host module: csrc/host.cpp against this interpreter's torch headers."""
+    import sysconfig
+
+    import torch
+
+    src = CSRC / "host.cpp"
+    newest = max(src.stat().st_mtime, _newest_header_mtime())
+    if not force and HOST_PATH.exists() and HOST_PATH.stat().st_mtime >= newest:
+        return HOST_PATH
+    root = Path(torch.__file__).resolve().parent
+    if not (root / "lib" / "libc10_cuda.so").exists():   # a CPU-only torch never calls it
+        return HOST_PATH
+    nvcc = find_nvcc()
+    cuda = Path(nvcc).resolve().parent.parent if nvcc else Path("/usr/local/cuda")
+    tmp = HOST_PATH.with_suffix(".so.tmp")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=npb200_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", str(root / "include"), "-isystem", str(root / "include/torch/csrc/api/include"),
+           "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"], "-I", str(CSRC), str(src), "-o", str(tmp),
+           "-L", str(root / "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
+           "-L", str(LIB_DIR), "-l:libnpb200.so", "-Wl,-rpath,$ORIGIN"]
+    # the C++ runtime that torch runs on, by its file: a compiler that brings only a static one would put a second copy beside it,
+    # and the two crash on each other's streams and exceptions
+    runtime = next((line.split()[-1] for line in open("/proc/self/maps") if "/libstdc++.so" in line), None)
+    if runtime:
+        cmd += ["-nostdlib++", runtime]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        sys.stderr.write(proc.stdout + proc.stderr)
+        raise RuntimeError("build of npb200_host.so failed")
+    os.replace(tmp, HOST_PATH)
+    return HOST_PATH
+
+
 def build_extension(force: bool = False, verbose: bool = False) -> Path:
     """Compile (if stale) and return the path of the shared library."""
     nvcc = find_nvcc()
@@ -97,6 +134,7 @@ def build_extension(force: bool = False, verbose: bool = False) -> Path:
             sys.stderr.write(proc.stdout + proc.stderr)
             raise RuntimeError("link of libnpb200.so failed")
         os.replace(tmp, LIB_PATH)
+    build_host(force)
     return LIB_PATH
 
 

@@ -16,6 +16,7 @@
 // Replaces F.scaled_dot_product_attention (reference: model/attention.py:121-127) and the dense
 // per-step matmul+softmax of its ring attention (distributed/context_parallel.py:301-317).
 #include "common.cuh"
+#include "args.h"
 
 namespace {
 
@@ -827,27 +828,6 @@ bool bind_ctx() {
 
 }  // namespace
 
-// Tensor layout of q / k / v / o: [B, S, H, 128] bf16 with element strides (sb, ss, sh); the last dim is
-// contiguous. k_ptrs / v_ptrs: one base pointer per KV source (n_src = 1 without context parallelism).
-struct NpAttnFwdArgs {
-  const void* q; long long q_sb, q_ss, q_sh;
-  const void* const* k_ptrs; const void* const* v_ptrs; long long k_sb, k_ss, k_sh;
-  void* o; long long o_sb, o_ss, o_sh;
-  float* lse;
-  int B, Sq, Hq, Hkv, causal, n_src, src_len, q_off;
-  float scale;
-  const int* q_blk_pos; const int* k_blk_pos;
-  int split;       // unused (two softmax threads per row)
-  int lse_heads;   // heads of the lse array when q / o are a head slice of larger tensors (0: Hq)
-  // KV sources that peers are still pushing into this GPU's memory: flags[flag_idx[s]] >= flag_epoch + *epoch_base
-  const int* src_flags; const int* flag_idx; int flag_epoch; const int* epoch_base; unsigned long long flag_limit_ns;
-  int flag_own;    // 1 + flag index that guards q itself (0: none)
-  // this rank's K|V shard pushed by the kernel itself: push_bytes of push_k then push_v to push_dst[r] (r < push_n),
-  // then *push_flag[r] = flag_epoch (+ *epoch_base); push_ctr: two local ints the caller zeroes before the launch
-  const void* push_k; const void* push_v; long long push_bytes; void* const* push_dst; int* const* push_flag;
-  int push_n; int* push_ctr;
-  int head_dim;    // 128 (also when 0) or 64
-};
 
 // a kernel of 20 us and more
 static bool busy(int B, int H, int Sq, int Sk, int hd) { return 4.0 * B * H * Sq * (double)Sk * hd > 2e10; }
@@ -1508,39 +1488,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
 }  // namespace
 
-// Backward of np_attn_fwd. q / o / d_o / dq are local [B, Sq, Hq, 128]; k / v / dk / dv local
-// [B, Sk, Hkv, 128]. kv sources (for dQ) and q / d_o / lse / delta sources (for dK, dV) are lists so a
-// context-parallel rank reads its peers' tensors in place; without context parallelism both lists have
-// one entry, the local tensors. delta = rowsum(dO o O) is computed here into `delta` ([B, Hq, Sq] fp32).
-// phase: 1 = delta only, 2 = dQ + dKV only (delta already published), 3 = all.
-struct NpAttnBwdArgs {
-  const void* q; long long q_sb, q_ss, q_sh;
-  const void* k; const void* v; long long k_sb, k_ss, k_sh;
-  const void* o; long long o_sb, o_ss, o_sh;
-  const void* d_o; long long do_sb, do_ss, do_sh;
-  const float* lse; float* delta;
-  void* dq; long long dq_sb, dq_ss, dq_sh;
-  void* dk; void* dv; long long dk_sb, dk_ss, dk_sh;
-  const void* const* k_src; const void* const* v_src;           // n_src KV sources (layout of k)
-  const void* const* q_src; const void* const* do_src;          // n_src Q / dO sources (layouts of q / d_o)
-  const float* const* lse_src; const float* const* delta_src;   // n_src [B, Hq, Sq] sources
-  int B, Sq, Sk, Hq, Hkv, causal, n_src, q_off, phase;
-  float scale;
-  const int* q_blk_pos_local; const int* k_blk_pos_all;         // for dQ: local Q blocks vs all KV blocks
-  const int* k_blk_pos_local; const int* q_blk_pos_all;         // for dKV: local KV blocks vs all Q blocks
-  int split;                                                    // softmax threads per row: 2 (default) or 4
-  int lse_heads;                                                // heads of the lse / delta arrays (0: Hq)
-  // sources still arriving (as in NpAttnFwdArgs); which = 1: the flags guard the KV sources of the dQ kernel,
-  // 2: the Q / dO / lse / delta sources of the dK/dV kernel, 3: both
-  const int* src_flags; const int* flag_idx; int flag_epoch; const int* epoch_base; unsigned long long flag_limit_ns;
-  int flag_which;
-  int skip;       // 1: no dQ kernel, 2: no dK/dV kernel
-  int flag_own;   // 1 + flag index that guards the resident operands (q, d_o, lse, delta / k, v), 0: none
-  // K|V shard pushed by the dQ kernel itself (as in NpAttnFwdArgs)
-  const void* push_k; const void* push_v; long long push_bytes; void* const* push_dst; int* const* push_flag;
-  int push_n; int* push_ctr;
-  int head_dim;    // 128 (also when 0) or 64
-};
 
 template <int NS, int HD>
 static int launch_bwd(dim3 gq, dim3 gk, int skip, const CUtensorMap& tmQ, const CUtensorMap& tmdO, const CUtensorMap& tmK,

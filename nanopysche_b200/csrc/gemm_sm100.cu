@@ -14,6 +14,7 @@
 // (model/attention.py:141-143,189; model/feed_forward.py:75; model/moe.py:1520-1538).
 #include <cstdlib>
 #include "common.cuh"
+#include "args.h"
 
 __device__ int g_np_status[8];
 __device__ unsigned long long g_np_wait_end[NP_MAX_SMS];
@@ -1274,47 +1275,6 @@ int np_make_tmap_2d(CUtensorMap* out, const void* base, int elt_bytes, uint64_t 
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
-// Arguments of np_gemm_bf16 (mirrored field by field by the ctypes Structure in ops/_lib.py).
-struct NpGemmArgs {
-  const void* A; const void* B; const void* B2; void* C; void* C2;
-  long long lda, ldb, ldc, ldc2;
-  long long a_rows, b_rows;  // total rows (K-major) or total K rows (MN-major) of the A / B tensors
-  int M, N, K;
-  // epilogue 2: C is [d gate | d up] and C2 the pre-activations [gate | up], each [M, 2 N]; the product is d h
-  int a_mn, b_mn, out_f32, accumulate, epilogue, mode;
-  float alpha;
-  const int* mblk_group; const int* mblk_rows; long long group_stride_b;
-  int num_groups, blocks_per_group; long long group_stride_c;
-  const int* ready_flags; const int* mblk_flag; int epoch; unsigned long long flag_limit_ns;
-  const long long* row_dst; void* const* peer_base;
-  int* done_counters; const int* done_expected; int* const* done_flag_ptr;
-  int bn;        // columns of a tile: 0 = choose, else 128 or 256 (128: one CTA per tile, whatever mt and split say)
-  int max_ctas;  // 0 = all SMs
-  const void* Cin; long long ldcin;  // optional accumulate source (defaults to C when accumulate != 0)
-  const int* epoch_base;             // optional device counter added to `epoch`
-  // B arriving in row shards (a sharded weight being all-gathered while the GEMM runs): the producer waits for
-  // the flag of every shard a tile touches before it loads from it
-  const int* b_ready_flags; int b_rows_per_flag;
-  // Local shard read in place (K-major operands only): A rows [a_loc_lo, a_loc_hi) from A_loc (row 0 = a_loc_lo),
-  // B rows [b_loc_lo, b_loc_hi) from B_loc; the block boundaries must be multiples of the tile size. b_local_flag:
-  // 1 + index of the B flag that needs no wait (0: none). m_rot / n_rot: first M / N block of the tile order.
-  const void* A_loc; long long lda_loc; int a_loc_lo, a_loc_hi;
-  const void* B_loc; long long ldb_loc; int b_loc_lo, b_loc_hi;
-  int b_local_flag, m_rot, n_rot;
-  // all-gather pushed by the GEMM's own CTAs before their first tile: push_bytes of push_src to push_dst[r]
-  // (r < push_n <= 8; the destinations already point at this rank's slot), then *push_flag[r] = epoch (+ base);
-  // push_ctr: a zeroed local int
-  const void* push_src; long long push_bytes; void* const* push_dst; int* const* push_flag; int push_n; int* push_ctr;
-  const float* bias;  // optional [N] fp32 bias added in the plain epilogue (alpha != 0)
-  // rows of a tile in units of 128: 0 = choose, 1, or 2 (256 x 256 tiles on a pair of CTAs; forms that the pair kernel does
-  // not take, and launches of one CTA, run one CTA per tile)
-  int mt;
-  int split;          // parts of K: 0 = choose, 1, or 2 or 4 on the pair kernel (dense, plain epilogue, 8 K steps, M above 128)
-  int paired;         // row-grouped form: blocks 2 i and 2 i + 1 share their group and their arrival flag
-  int k_split;        // > 0 (MN-major B): K rows [0, k_split) of a group come from B, the rest from B2 (multiple of 64)
-  int m_split;        // > 0: output rows [0, m_split) go to C, the rest to C2 (layout of C; multiple of 256)
-  int pair_bn;        // columns of a pair's tile: 0 = choose, 128, 192 or 256
-};
 
 static int num_sms() {
   if (g_num_sms == 0) {

@@ -16,6 +16,7 @@
 // Replaces model/moe.py:133-321 (router), :1395-1448 (capacity), :360-498 (NCCL dispatcher: 4
 // collectives + 3 host syncs per layer) and :1386-1390,1691-1714 (scatter-back) of the reference.
 #include "common.cuh"
+#include "args.h"
 
 namespace {
 
@@ -1049,13 +1050,6 @@ NP_API int np_capacity_scan(const int* indices, int T, int E, int K, int capacit
   return np_capacity_plan(indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, nullptr, 0, nullptr, stream);
 }
 
-struct NpDispatchArgs {
-  const void* x; const int* indices; const int* slot_pos; const int* counts_kept; const float* slot_scale;
-  int T, K, D, E, E_local, n_ranks, my_rank, region_rows, quant;
-  void* const* peer_rows; float* const* peer_scales; long long* const* peer_row_dst;
-  int* const* peer_mblk_rows; int* const* peer_src_blocks; int* const* peer_flags;
-  int* done_ctr; int epoch; int write_meta; int max_ctas; const int* epoch_base; int* zero_ctr;
-};
 NP_API int np_ep_dispatch(const NpDispatchArgs* a, void* stream) {
   if (a->D % 128 || a->region_rows % 128 || a->E % a->E_local || (a->quant && a->D % 256)) return 1;
   DispatchParams p;
@@ -1075,12 +1069,6 @@ NP_API int np_ep_dispatch(const NpDispatchArgs* a, void* stream) {
   CHECK_LAUNCH();
 }
 
-struct NpCombineArgs {
-  const void* rows; const int* slot_pos; const float* weights; const void* add1; const void* add2;
-  const float* dl; const float* wg; void* out; int T, K, D, E;
-  const int* flags; const int* sent_to_peer; int n_ranks, epoch; unsigned long long limit_ns;
-  const int* epoch_base;
-};
 NP_API int np_ep_combine(const NpCombineArgs* a, void* stream) {
   if (a->D % 8 || a->n_ranks > 256) return 1;
   if (a->T <= 0) return 0;

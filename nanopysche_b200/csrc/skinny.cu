@@ -3,6 +3,7 @@
 // the cache) through the chip once and are bound by that traffic and by launch latency; tensor-memory tiles of 128 rows
 // would leave most of the chip idle (a 2048 x 2048 weight is 16 tiles).
 #include "common.cuh"
+#include "args.h"
 
 namespace {
 
@@ -339,15 +340,6 @@ int np_skinny_linear(const void* x, long long ldx, const void* w, long long ldw,
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
-// Mirrored by DecodeArgs in ops/_lib.py. All tensors bf16 with 16-byte aligned rows of HD elements (64 or 128).
-struct NpDecodeArgs {
-  const void* q; long long q_sb, q_ss, q_sh;
-  const void* kc; const void* vc; long long kc_sb, kc_ss, kc_sh, vc_sb, vc_ss, vc_sh;
-  const void* kn; const void* vn; long long kn_sb, kn_ss, kn_sh, vn_sb, vn_ss, vn_sh;
-  void* ko; void* vo; void* o;
-  int B, Sq, Hq, Hkv, past, fresh, causal, head_dim;
-  float scale;
-};
 
 NP_API int np_decode_attn(const NpDecodeArgs* a, void* stream) {
   if (a->B <= 0 || a->Sq <= 0 || a->past + a->fresh <= 0) return 0;

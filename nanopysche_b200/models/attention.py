@@ -114,7 +114,13 @@ class Attention(nn.Module):
         pid = None
         if position_ids is not None:
             pid = position_ids if position_ids.dim() == 2 else position_ids[None, :].expand(B, S)
-        if qkv is not None and self.q_norm is None:
+        plain_sdpa = getattr(self.sdpa, "__func__", None) is Attention.sdpa   # not replaced by a subclass or on the instance
+        o = None
+        if qkv is not None and kv_cache is None and not return_kv and self._cp_module is None and attn_mask is None and plain_sdpa:
+            o = attn_ops.qkv_attention(qkv, cos, sin, hq, hkv, hd, start_pos, pid, causal, self.q_norm, self.k_norm)
+        if o is not None:
+            pass   # rotated and attended to in one autograd node
+        elif qkv is not None and self.q_norm is None:
             q, k, v = rope_ops.qkv_rope(qkv, cos, sin, hq, hkv, hd, start_pos, pid)  # split + rotate in one kernel
         elif qkv is not None and self.q_norm.bias is not None and \
                 rope_ops.qkv_norm_rope_supported(qkv, cos, hq, hkv, hd):
@@ -132,8 +138,9 @@ class Attention(nn.Module):
                 k = self.k_norm(k.float()).to(x.dtype) if k.dtype != torch.float32 else self.k_norm(k)
             q = rope_ops.apply_rope(q, cos, sin, start_pos, pid)
             k = rope_ops.apply_rope(k, cos, sin, start_pos, pid)
-        if kv_cache is not None and self._cp_module is None and attn_mask is None and \
-                getattr(self.sdpa, "__func__", None) is Attention.sdpa:   # not replaced by a subclass or on the instance
+        if o is not None:
+            pass
+        elif kv_cache is not None and self._cp_module is None and attn_mask is None and plain_sdpa:
             o, k, v = attn_ops.attention_append(q, kv_cache[0], kv_cache[1], k, v, causal=causal)
         else:
             if kv_cache is not None:
@@ -143,7 +150,7 @@ class Attention(nn.Module):
                 o = self._cp_module(q, k, v, causal=causal)
             else:
                 o = self.sdpa(q, k, v, causal=causal, attn_mask=attn_mask)
-        o = o.reshape(B, S, self._local_heads * self.head_dim)
+        o = o.reshape(B, S, self._local_heads * self.head_dim) if o.dim() == 4 else o
         if self.output_dropout is not None:
             o = self.output_dropout(o)
         if rt is not None:

@@ -18,12 +18,14 @@ import torch
 _LIB = None
 _LIB_ERR: str | None = None
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libnpb200.so"
+HOST_PATH = LIB_PATH.with_name("npb200_host.so")
+_HOST = None
 
 c_void_p, c_int, c_ll, c_ull, c_float = C.c_void_p, C.c_int, C.c_longlong, C.c_ulonglong, C.c_float
 
 
 class GemmArgs(C.Structure):
-    """Mirror of ``NpGemmArgs`` in csrc/gemm_sm100.cu (field order matters)."""
+    """Mirror of ``NpGemmArgs`` in csrc/args.h (field order matters)."""
 
     _fields_ = [
         ("A", c_void_p), ("B", c_void_p), ("B2", c_void_p), ("C", c_void_p), ("C2", c_void_p),
@@ -53,7 +55,7 @@ class GemmArgs(C.Structure):
 
 
 class DispatchArgs(C.Structure):
-    """Mirror of ``NpDispatchArgs`` in csrc/moe.cu."""
+    """Mirror of ``NpDispatchArgs`` in csrc/args.h."""
 
     _fields_ = [
         ("x", c_void_p), ("indices", c_void_p), ("slot_pos", c_void_p), ("counts_kept", c_void_p),
@@ -68,7 +70,7 @@ class DispatchArgs(C.Structure):
 
 
 class CombineArgs(C.Structure):
-    """Mirror of ``NpCombineArgs`` in csrc/moe.cu."""
+    """Mirror of ``NpCombineArgs`` in csrc/args.h."""
 
     _fields_ = [
         ("rows", c_void_p), ("slot_pos", c_void_p), ("weights", c_void_p), ("add1", c_void_p),
@@ -80,7 +82,7 @@ class CombineArgs(C.Structure):
 
 
 class AttnFwdArgs(C.Structure):
-    """Mirror of ``NpAttnFwdArgs`` in csrc/attn_sm100.cu."""
+    """Mirror of ``NpAttnFwdArgs`` in csrc/args.h."""
 
     _fields_ = [
         ("q", c_void_p), ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
@@ -101,7 +103,7 @@ class AttnFwdArgs(C.Structure):
 
 
 class AttnBwdArgs(C.Structure):
-    """Mirror of ``NpAttnBwdArgs`` in csrc/attn_sm100.cu."""
+    """Mirror of ``NpAttnBwdArgs`` in csrc/args.h."""
 
     _fields_ = [
         ("q", c_void_p), ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
@@ -128,7 +130,7 @@ class AttnBwdArgs(C.Structure):
 
 
 class DecodeArgs(C.Structure):
-    """Mirror of ``NpDecodeArgs`` in csrc/skinny.cu."""
+    """Mirror of ``NpDecodeArgs`` in csrc/args.h."""
 
     _fields_ = [
         ("q", c_void_p), ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
@@ -191,7 +193,7 @@ def lib():
     global _LIB, _LIB_ERR
     if _LIB is not None:
         return _LIB
-    if not LIB_PATH.exists():
+    if not (LIB_PATH.exists() and HOST_PATH.exists()):
         try:
             from ..build import build_extension
 
@@ -221,6 +223,26 @@ def lib():
     _LIB.np_decode_attn.argtypes = [C.POINTER(DecodeArgs), c_void_p]
     _LIB.np_status_read.argtypes = [C.POINTER(c_int)]
     return _LIB
+
+
+def host():
+    """The native host module (csrc/host.cpp): the ops of a layer with their launches and autograd nodes."""
+    global _HOST
+    if _HOST is None:
+        import importlib.util
+
+        from . import gemm
+
+        lib()
+        try:
+            spec = importlib.util.spec_from_file_location("npb200_host", str(HOST_PATH))
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+        except (ImportError, OSError) as e:
+            raise KernelError(f"cannot load {HOST_PATH}: {e}") from e
+        mod.setup(KernelError, vars(gemm))
+        _HOST = mod
+    return _HOST
 
 
 def available() -> bool:
@@ -276,14 +298,20 @@ class nvtx_range:
         return False
 
 
-LAUNCHES = 0  # number of successful calls into the kernel library (each launches >= 1 kernel)
+_calls = 0
+
+
+def __getattr__(name: str):
+    if name == "LAUNCHES":   # number of successful calls into the kernel library (each launches >= 1 kernel)
+        return _calls + (_HOST.launches() if _HOST is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def check(rc: int, name: str) -> None:
-    global LAUNCHES
+    global _calls
     if rc != 0:
         raise KernelError(f"{name} failed with code {rc}")
-    LAUNCHES += 1
+    _calls += 1
 
 
 def status() -> tuple[int, ...]:

@@ -317,30 +317,8 @@ def _has_tangent(ts) -> bool:
 
 
 def _decode(q, k, v, k_new, v_new, causal, scale):
-    """Launch of the decode kernel: keys and values ``[k | k_new]``; returns ``(out, k_cat, v_cat)`` (``None`` for the
-    concatenations when nothing is appended)."""
-    import ctypes as C
-
-    B, Sq, Hq, hd = q.shape
-    P, Hkv = k.shape[1], k.shape[2]
-    o = torch.empty((B, Sq, Hq, hd), device=q.device, dtype=torch.bfloat16)
-    a = _lib.DecodeArgs()
-    a.q, a.kc, a.vc, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
-    a.q_sb, a.q_ss, a.q_sh = q.stride()[:3]
-    a.kc_sb, a.kc_ss, a.kc_sh = k.stride()[:3]
-    a.vc_sb, a.vc_ss, a.vc_sh = v.stride()[:3]
-    ko = vo = None
-    if k_new is not None:
-        n = k_new.shape[1]
-        ko = torch.empty((B, P + n, Hkv, hd), device=q.device, dtype=torch.bfloat16)
-        vo = torch.empty_like(ko)
-        a.kn, a.vn, a.ko, a.vo, a.fresh = k_new.data_ptr(), v_new.data_ptr(), ko.data_ptr(), vo.data_ptr(), n
-        a.kn_sb, a.kn_ss, a.kn_sh = k_new.stride()[:3]
-        a.vn_sb, a.vn_ss, a.vn_sh = v_new.stride()[:3]
-    a.B, a.Sq, a.Hq, a.Hkv, a.past, a.causal, a.head_dim = B, Sq, Hq, Hkv, P, int(causal), hd
-    a.scale = scale if scale is not None else 1.0 / math.sqrt(hd)
-    _lib.check(_lib.lib().np_decode_attn(C.byref(a), C.c_void_p(_lib.stream())), "decode_attn")
-    return o, ko, vo
+    """Launch of the decode kernel: keys and values ``[k | k_new]``; returns ``(out, k_cat, v_cat)``."""
+    return _lib.host().decode(q, k, v, k_new, v_new, causal, scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]))
 
 
 # Query rows of one KV head (query heads of its group x new tokens) that the decode kernel holds in registers.
@@ -365,6 +343,27 @@ def attention_append(q, k_cache, v_cache, k_new, v_new, causal: bool = True, sca
         return _decode(q, k_cache, v_cache, k_new, v_new, causal, scale)
     k, v = torch.cat([k_cache, k_new], dim=1), torch.cat([v_cache, v_new], dim=1)
     return attention(q, k, v, causal=causal, scale=scale), k, v
+
+
+def qkv_attention(qkv: torch.Tensor, cos, sin, hq: int, hkv: int, hd: int, pos_offset: int = 0, pos_ids=None, causal: bool = True,
+                  q_norm=None, k_norm=None):
+    """``attention(*qkv_rope(qkv, ...))`` (``qkv_norm_rope`` with norms) as one autograd node whose result is
+    ``[B, S, hq * hd]``, or ``None`` for what the flash kernels or the rotation kernels do not cover."""
+    from . import rope
+
+    if not (USE_FLASH and (hd == 128 or (hd == 64 and PAD_SMALL_HEADS)) and _lib.on(qkv)):
+        return None
+    if q_norm is None:
+        if not rope.qkv_rope_supported(qkv, cos, hd):
+            return None
+        par = (None, None, None, None, 0.0)
+    else:
+        if q_norm.bias is None or not rope.qkv_norm_rope_supported(qkv, cos, hq, hkv, hd):
+            return None
+        par = (q_norm.weight, q_norm.bias, k_norm.weight, k_norm.bias, float(q_norm.eps))
+    if pos_ids is not None:
+        pos_ids = pos_ids.reshape(-1).to(torch.int32)
+    return _lib.host().qkv_attention(qkv, *par, cos, sin, hq, hkv, hd, int(pos_offset), pos_ids, causal, 1.0 / math.sqrt(hd))
 
 
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = True,

@@ -57,25 +57,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             return y.to(out_dtype or a.dtype)
         out.copy_((y + out.float()) if accumulate else y)
         return out
-    args, out = _gemm_args(a, b, a_mn, b_mn, out, out_dtype, accumulate, alpha)
-    M, N, K = args.M, args.N, args.K
     # requests; 0 = choose. mt 2: 256 x 256 tiles on pairs of CTAs, split 2 or 4: parts of K there (bn 128: one-CTA tiles),
     # pair_bn 128, 192 or 256: tiles of that many columns on pairs
-    args.bn, args.max_ctas, args.mt, args.split, args.pair_bn = bn, max_ctas, mt, split, pair_bn
-    if bias is not None:
-        assert bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous()
-        args.bias = bias.data_ptr()
-    if residual is not None:
-        assert not accumulate and residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
-        args.accumulate, args.Cin, args.ldcin = 1, residual.data_ptr(), residual.stride(0)
-    rc = _lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream()))
-    if rc != 0:
-        raise _lib.KernelError(
-            f"gemm_bf16 failed with code {rc}: M={M} N={N} K={K} a_mn={a_mn} b_mn={b_mn} a={tuple(a.shape)}/"
-            f"{a.stride()} b={tuple(b.shape)}/{b.stride()} out={tuple(out.shape)}/{out.stride()} {out.dtype} "
-            f"ptrs={a.data_ptr() % 256},{b.data_ptr() % 256},{out.data_ptr() % 256} bn={bn}")
-    _lib.LAUNCHES += 1
-    return out
+    return _lib.host().gemm(a, b, a_mn, b_mn, out, out_dtype, accumulate, alpha, bn, max_ctas, bias, residual, mt, split, pair_bn)
 
 
 def _gemm_args(a, b, a_mn, b_mn, out, out_dtype, accumulate, alpha):
@@ -175,7 +159,7 @@ def gemm_dgrad_wgrad(dy: torch.Tensor, w: torch.Tensor, x: torch.Tensor, *, out:
         raise _lib.KernelError(f"gemm_bf16_two failed with code {rc}: dy={tuple(dy.shape)}/{dy.stride()} w={tuple(w.shape)}/"
                                f"{w.stride()} x={tuple(x.shape)}/{x.stride()} dw={tuple(dw.shape)}/{dw.stride()} {dw.dtype} "
                                f"ptrs={dy.data_ptr() % 256},{w.data_ptr() % 256},{x.data_ptr() % 256},{dw.data_ptr() % 256}")
-    _lib.LAUNCHES += 1
+    _lib.check(rc, "gemm_bf16_two")
     return dx, dw
 
 
@@ -268,6 +252,8 @@ def _linear_grads(ctx, w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
 
 
 class _Linear(torch.autograd.Function):
+    """``x @ w.T`` off the kernel path with a weight gradient that can be deferred (on it: ``Linear`` in csrc/host.cpp)."""
+
     @staticmethod
     def forward(ctx, x, w):
         ctx.save_for_backward(x, w)
@@ -335,7 +321,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -
                     return fp8_block_linear(x, w, bias)
         if bias is not None:
             return _LinearBias.apply(x, w, bias)
-        return _Linear.apply(x, w)
+        return _lib.host().linear(x, w)
     return torch.nn.functional.linear(x, w, bias)
 
 

@@ -25,62 +25,19 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .activation import glu
 
 GATING_IDS = {"softmax": 0, "sigmoid": 1}
 WAIT_LIMIT_NS = int(os.environ.get("NPB200_WAIT_LIMIT_MS", "10000")) * 1_000_000
 
 
 # ------------------------------------------------------------------------------------------------ router
-class _Router(torch.autograd.Function):
-    """logits -> top-k -> gating weights, with the load-balance / z-loss statistics in the same pass."""
+class _Router:
+    """logits -> top-k -> gating weights, with the load-balance / z-loss statistics in the same pass: ``(weights, indices int32,
+    aux, counts)`` (csrc/host.cpp)."""
 
     @staticmethod
-    def forward(ctx, x2, gate_w, gate_b, score_bias, K, gating, coef_z):
-        T, D = x2.shape
-        E = gate_w.shape[0]
-        dev = x2.device
-        logits = torch.empty((T, E), device=dev, dtype=torch.float32)
-        zeros = (torch.empty if T > 0 else torch.zeros)(2 * E + 1, device=dev, dtype=torch.int32)
-        counts, stats = zeros[:E], zeros[E:].view(torch.float32)    # token counts; probability sums, sum of lse^2
-        _lib.call("router_logits", x2, gate_w, gate_b, logits, T, D, E, zeros, 2 * E + 1)
-        weights = torch.empty((T, K), device=dev, dtype=torch.float32)
-        indices = torch.empty((T, K), device=dev, dtype=torch.int32)
-        _lib.call("router_topk", logits, score_bias, weights, indices, counts, stats[:E], stats[E:], T, E, K, gating)
-        # tensors of their own: an output that is a view beside another differentiable output may not be changed in place,
-        # and the saved load fractions must not share the loss's version counter
-        f = torch.empty(E, device=dev, dtype=torch.float32)
-        aux = torch.empty((), device=dev, dtype=torch.float32)
-        _lib.call("router_aux", counts, stats[:E], stats[E:], float(coef_z or 0.0), f, aux, T, E)
-        ctx.save_for_backward(x2, gate_w, logits, weights, indices, f, score_bias if score_bias is not None
-                              else logits.new_empty(0))
-        ctx.cfg = (K, gating, float(coef_z or 0.0), score_bias is not None)
-        ctx.mark_non_differentiable(indices, counts)
-        return weights, indices, aux, counts
-
-    @staticmethod
-    def backward(ctx, dweights, _di, daux, _dc):
-        x2, gate_w, logits, weights, indices, f, sb = ctx.saved_tensors
-        K, gating, coef_z, has_sb = ctx.cfg
-        T, E = logits.shape
-        D = x2.shape[1]
-        dl = torch.empty_like(logits)
-        dw = dweights.contiguous() if dweights is not None else None
-        da = daux.reshape(1).float().contiguous() if daux is not None else None
-        _lib.call("router_bwd", logits, sb if has_sb else None, weights, indices, dw, f, da, 1.0, coef_z, dl, T, E, K,
-                  gating)
-        parts = _lib.lib().np_router_dgate_parts(T)
-        scratch = torch.empty((parts, E * D + (E + 3) // 4 * 4), device=x2.device, dtype=torch.float32)
-        new = torch.empty if T > 0 else torch.zeros    # no tokens: the kernels below do nothing
-        dgw = new(gate_w.shape, device=x2.device, dtype=gate_w.dtype)
-        dgb = new(E, device=x2.device, dtype=torch.float32)
-        _lib.call("router_dgate", dl, x2, dgw, dgb, scratch, T, D, E, 0)
-        if x2.dtype == torch.bfloat16 and gate_w.dtype == torch.float32 and gate_w.is_contiguous():
-            dx = torch.empty_like(x2)
-            _lib.call("router_dx", dl, gate_w, dx, T, D, E)
-        else:
-            dx = (dl @ gate_w.float()).to(x2.dtype)
-        return dx, dgw, dgb, None, None, None, None
+    def apply(x2, gate_w, gate_b, score_bias, K, gating, coef_z):
+        return _lib.host().router(x2, gate_w, gate_b, score_bias, K, gating, float(coef_z or 0.0))
 
 
 def route(x: torch.Tensor, router, int64: bool = True) -> tuple:
@@ -92,7 +49,7 @@ def route(x: torch.Tensor, router, int64: bool = True) -> tuple:
     x2 = x2 if x2.is_contiguous() else x2.contiguous()
     gating = GATING_IDS[getattr(cfg.gating_function, "value", cfg.gating_function)]
     w, idx, aux, counts = _Router.apply(x2, router.gate.weight, router.gate.bias, router.score_bias, router.top_k,
-                                        gating, cfg.z_loss_multiplier or 0.0)
+                                        gating, cfg.z_loss_multiplier)
     lead = x.shape[:-1]
     return w.view(*lead, -1), (idx.long() if int64 else idx).view(*lead, -1), aux, counts
 
@@ -165,6 +122,7 @@ class FusedMoERuntime:
         # behind every dispatch on the same stream (``_push_counters`` holds callers to that)
         self.done_counters = torch.zeros(self.N, device=self.device, dtype=torch.int32)
         self._may_push = False
+        self._native = None
         self.dispatch_ctr = torch.zeros(1, device=self.device, dtype=torch.int32)
         self.layer_of: dict[int, int] = {}
         self.max_ctas_dispatch = max_ctas_dispatch
@@ -248,6 +206,12 @@ class FusedMoERuntime:
             flow_quantize_weight(w2.detach(), E_l, transpose=True, out=(w2q, s2))
             self._wq_valid.add(layer)
         return w13q, s13, w2q, s2
+
+    def native(self):
+        """The native module's view of this runtime (buffers and tables do not change once they are there)."""
+        if self._native is None:
+            self._native = _lib.host().MoeRuntime(self, WAIT_LIMIT_NS)
+        return self._native
 
     # -- kernels -------------------------------------------------------------------------------------
     def dispatch(self, x2, indices, slot_pos, counts_kept, scale, p_rows, epoch, p_scales=None):
@@ -383,7 +347,9 @@ class FusedMoERuntime:
 
 
 # ------------------------------------------------------------------------------------------------ the layer
-class _FusedMoE(torch.autograd.Function):
+class _FusedMoEFp8(torch.autograd.Function):
+    """The FP8-Flow-MoE form of the layer (the bf16 form: ``FusedMoE`` in csrc/host.cpp)."""
+
     @staticmethod
     def forward(ctx, x, weights, indices32, w1, w3, w2, rt: FusedMoERuntime, layer: int, stats_mod, shared=None):
         T, D, K, H = rt.T, rt.D, rt.K, rt.H
@@ -400,30 +366,20 @@ class _FusedMoE(torch.autograd.Function):
                   rt.N, None if stats_mod is None else stats_mod._drop_stats(dev))
         e1 = rt.next_epoch()
         gu = torch.empty((rt.rows_total, 2 * H), device=dev, dtype=torch.bfloat16)
-        if rt.fp8:
-            # FP8-Flow-MoE forward: rows travel as e4m3 with 1x128 power-of-two scales (quantised inside the dispatch
-            # kernel), the expert weights are e4m3 with 128x128 scales (made once per optimizer step), both expert
-            # GEMMs run on the block-scaled tcgen05 path with the scaling done by the tensor core: one gate|up GEMM,
-            # SwiGLU + re-quantisation in one pass, and the down GEMM pushing rows back to their sources
-            from .gemm_mxfp8 import flow_quantize_act
+        # FP8-Flow-MoE forward: rows travel as e4m3 with 1x128 power-of-two scales (quantised inside the dispatch
+        # kernel), the expert weights are e4m3 with 128x128 scales (made once per optimizer step), both expert
+        # GEMMs run on the block-scaled tcgen05 path with the scaling done by the tensor core: one gate|up GEMM,
+        # SwiGLU + re-quantisation in one pass, and the down GEMM pushing rows back to their sources
+        from .gemm_mxfp8 import flow_quantize_act
 
-            w13q, s13, w2q, s2 = rt.quantised_weights(layer, w1, w3, w2)
-            rt.dispatch(x2, indices32, slot_pos, counts_kept, None, rt.p_recv_xq[layer], e1,
-                        p_scales=rt.p_recv_xs[layer])
-            xq, xs = rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer]
-            rt.grouped_gemm_fp8(xq, xs, w13q, s13, N=2 * H, out=gu, wait_epoch=e1)
-            h = torch.empty((rt.rows_total, H), device=dev, dtype=torch.bfloat16)
-            hq, hs = flow_quantize_act(gu, swiglu=True, h_out=h)
-            rt.grouped_gemm_fp8(hq, hs, w2q, s2, N=D, push_ptrs=rt.p_ret_y[layer], push_epoch=e1)
-        else:
-            rt.dispatch(x2, indices32, slot_pos, counts_kept, None, rt.p_recv_x[layer], e1)
-            # experts: [gate|up] GEMM with SwiGLU epilogue, waits per block on the source's arrival flag
-            h = torch.empty((rt.rows_total, H), device=dev, dtype=torch.bfloat16)
-            rt.grouped_gemm(rt.recv_x[layer], w1, N=H, K=D, b_mn=False, group_stride_b=H, out=h, B2=w3, C2=gu,
-                            wait_epoch=e1)
-            # down projection (w2 is stored [H, D] per expert: MN-major B), rows pushed back to their sources
-            rt.grouped_gemm(h, w2, N=D, K=H, b_mn=True, group_stride_b=H, push_ptrs=rt.p_ret_y[layer],
-                            push_epoch=e1)
+        w13q, s13, w2q, s2 = rt.quantised_weights(layer, w1, w3, w2)
+        rt.dispatch(x2, indices32, slot_pos, counts_kept, None, rt.p_recv_xq[layer], e1,
+                    p_scales=rt.p_recv_xs[layer])
+        xq, xs = rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer]
+        rt.grouped_gemm_fp8(xq, xs, w13q, s13, N=2 * H, out=gu, wait_epoch=e1)
+        h = torch.empty((rt.rows_total, H), device=dev, dtype=torch.bfloat16)
+        hq, hs = flow_quantize_act(gu, swiglu=True, h_out=h)
+        rt.grouped_gemm_fp8(hq, hs, w2q, s2, N=D, push_ptrs=rt.p_ret_y[layer], push_epoch=e1)
         out = torch.empty((T, D), device=dev, dtype=torch.bfloat16)
         add1 = None
         if shared is not None:
@@ -434,9 +390,8 @@ class _FusedMoE(torch.autograd.Function):
         ctx.has_shared = shared is not None
         # the activation h is kept for the w2 weight gradient (57 MB per layer at the 1B shapes: cheap next to
         # re-reading the pre-activations)
-        ctx.has_h = True
-        ctx.save_for_backward(x2, weights, indices32, slot_pos, counts_kept, sent, gu, w1, w3, w2,
-                              *([h] if ctx.has_h else []), *([keep] if ctx.has_shared else []))
+        ctx.save_for_backward(x2, weights, indices32, slot_pos, counts_kept, sent, gu, w1, w3, w2, h,
+                              *([keep] if ctx.has_shared else []))
         ctx.rt, ctx.layer = rt, layer
         ctx.x_shape = x.shape
         if stats_mod is not None:
@@ -459,15 +414,11 @@ class _FusedMoE(torch.autograd.Function):
         rt.dispatch(do2, indices32, slot_pos, counts_kept, weights, rt.p_recv_g, e2)
         # dH = dY @ w2^T  (w2 [H, D] per expert is K-major for this contraction), taken to [dG | dU] in the epilogue
         dgu = rt.grouped_gemm(rt.recv_g, w2, N=H, K=D, b_mn=False, group_stride_b=H, wait_epoch=e2, glu_of=gu)
-        hh = ctx.saved_tensors[10] if ctx.has_h else glu(gu)
-        dw2 = rt.grouped_wgrad(hh, rt.recv_g, w2, M=H, N=D)
-        del hh
-        if rt.fp8:  # the rows arrived as e4m3: dequantise once for the (bf16) weight-gradient GEMMs
-            from .gemm_mxfp8 import mx_dequantize_bf16
+        dw2 = rt.grouped_wgrad(ctx.saved_tensors[10], rt.recv_g, w2, M=H, N=D)
+        # the rows arrived as e4m3: dequantise once for the (bf16) weight-gradient GEMMs
+        from .gemm_mxfp8 import mx_dequantize_bf16
 
-            xr = mx_dequantize_bf16(rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer])
-        else:
-            xr = rt.recv_x[layer]
+        xr = mx_dequantize_bf16(rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer])
         dw1, dw3 = rt.grouped_wgrad(dgu, xr, w1, M=H, N=D, w_second=w3)
         # dX = [dG | dU] @ [w1; w3], one contraction over both weights (no bf16 partial result in between), pushed back to
         # the sources. H is a multiple of 256 (MoEBase), the K steps of 64 never straddle the two.
@@ -533,5 +484,9 @@ def fused_moe_forward(mod, x: torch.Tensor) -> torch.Tensor:
     mod._aux_loss = aux
     shared = mod.shared_expert(x) if mod.shared_expert is not None else None
     with _lib.nvtx_range("fused_moe"):
-        return _FusedMoE.apply(x, w.reshape(B * S, -1), idx.reshape(B * S, -1), mod.w1, mod.w3, mod.w2, rt, layer, mod,
-                               shared)
+        w, idx = w.reshape(B * S, -1), idx.reshape(B * S, -1)
+        if rt.fp8:
+            return _FusedMoEFp8.apply(x, w, idx, mod.w1, mod.w3, mod.w2, rt, layer, mod, shared)
+        out, mod._per_expert_drop_counts = _lib.host().fused_moe(x, w, idx, mod.w1, mod.w3, mod.w2, rt.native(), layer,
+                                                                 mod._drop_stats(x.device), shared)
+        return out

@@ -82,33 +82,6 @@ def apply_rope_ref(x, cos, sin, pos_offset: int = 0, pos_ids=None, sign: float =
     return out.to(x.dtype)
 
 
-class _Rope(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, cos, sin, pos_offset, pos_ids, inplace):
-        B, S, H, hd = x.shape
-        assert x.stride(3) == 1 and x.stride(2) == hd and x.stride(0) == S * x.stride(1)
-        out = x if inplace else torch.empty((B, S, H, hd), device=x.device, dtype=x.dtype)
-        _lib.call("rope", x, out, cos, sin, pos_ids, _lib.LL(B * S), S, int(pos_offset), H, hd, 2 * cos.shape[1],
-                  _lib.LL(x.stride(1)), _lib.LL(out.stride(1)), 1.0)
-        ctx.save_for_backward(cos, sin, pos_ids if pos_ids is not None else cos.new_empty(0))
-        ctx.meta = (pos_offset, pos_ids is not None)
-        if inplace:
-            ctx.mark_dirty(x)
-        return out
-
-    @staticmethod
-    def backward(ctx, dy):
-        cos, sin, pos_ids = ctx.saved_tensors
-        pos_offset, has_ids = ctx.meta
-        B, S, H, hd = dy.shape
-        if not (dy.stride(3) == 1 and dy.stride(2) == hd and dy.stride(0) == S * dy.stride(1)):
-            dy = dy.contiguous()
-        dx = torch.empty((B, S, H, hd), device=dy.device, dtype=dy.dtype)
-        _lib.call("rope", dy, dx, cos, sin, pos_ids if has_ids else None, _lib.LL(B * S), S, int(pos_offset), H, hd,
-                  2 * cos.shape[1], _lib.LL(dy.stride(1)), _lib.LL(dx.stride(1)), -1.0)
-        return dx, None, None, None, None, None
-
-
 def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos_offset: int = 0,
                pos_ids: torch.Tensor | None = None) -> torch.Tensor:
     """Rotate ``x [B, S, H, hd]`` (a possibly strided view with contiguous heads) by its positions."""
@@ -119,7 +92,7 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos_offset
     if ok:
         if pos_ids is not None:
             pos_ids = pos_ids.reshape(-1).to(torch.int32)
-        return _Rope.apply(x, cos, sin, pos_offset, pos_ids, False)
+        return _lib.host().rope(x, cos, sin, int(pos_offset), pos_ids)
     return apply_rope_ref(x, cos, sin, pos_offset, pos_ids)
 
 
@@ -238,14 +211,16 @@ def qkv_norm_rope(qkv, q_norm, k_norm, cos, sin, hq: int, hkv: int, pos_offset: 
                               hq, hkv, pos_offset, pos_ids)
 
 
+def qkv_rope_supported(qkv: torch.Tensor, cos, hd: int) -> bool:
+    return (_lib.on(qkv) and qkv.dtype == torch.bfloat16 and hd % 8 == 0 and (2 * cos.shape[1]) % 16 == 0 and
+            qkv.stride(2) == 1 and qkv.stride(1) % 8 == 0 and qkv.stride(0) == qkv.shape[1] * qkv.stride(1) and
+            cos.dtype == torch.float32)
+
+
 def qkv_rope(qkv: torch.Tensor, cos, sin, hq: int, hkv: int, hd: int, pos_offset: int = 0, pos_ids=None):
     """``qkv [B, S, (hq+2*hkv)*hd]`` -> rotated ``q [B,S,hq,hd]``, ``k [B,S,hkv,hd]`` and ``v`` (strided views of
     one buffer). Falls back to slicing + ``apply_rope`` off the kernel path."""
-    B, S, W = qkv.shape
-    ok = (_lib.on(qkv) and qkv.dtype == torch.bfloat16 and hd % 8 == 0 and (2 * cos.shape[1]) % 16 == 0 and
-          qkv.stride(2) == 1 and qkv.stride(1) % 8 == 0 and qkv.stride(0) == S * qkv.stride(1) and
-          cos.dtype == torch.float32)
-    if ok:
+    if qkv_rope_supported(qkv, cos, hd):
         if pos_ids is not None:
             pos_ids = pos_ids.reshape(-1).to(torch.int32)
         return _QKVRope.apply(qkv, cos, sin, hq, hkv, hd, pos_offset, pos_ids)
