@@ -681,101 +681,138 @@ __global__ void __launch_bounds__(256) qkv_norm_rope_fwd_kernel(
   }
 }
 
+__device__ __forceinline__ float group16_sum(float v, unsigned mask) {
+  v += __shfl_xor_sync(mask, v, 1);
+  v += __shfl_xor_sync(mask, v, 2);
+  v += __shfl_xor_sync(mask, v, 4);
+  v += __shfl_xor_sync(mask, v, 8);
+  return v;
+}
+__device__ __forceinline__ void unpack4(const uint2& u, float* f) {
+  const float2 a = np::unpack_bf16(u.x), b = np::unpack_bf16(u.y);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+__device__ __forceinline__ uint2 pack4(const float* f) { return make_uint2(np::pack_bf16(f[0], f[1]), np::pack_bf16(f[2], f[3])); }
+__device__ __forceinline__ void ld4f(const float* p, float* f) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+}
+// the V heads of a block's tokens: copied by all of its threads, two tokens at a time
+__device__ __forceinline__ void copy_v_heads(const __nv_bfloat16* src, long long rs, long long hs, __nv_bfloat16* dst, long long ds, int hkv,
+                                             long long T) {
+  for (int r = threadIdx.x; r < hkv * 16; r += blockDim.x) {
+    const __nv_bfloat16* v = src + (long long)(r >> 4) * hs + (r & 15) * 8;
+    __nv_bfloat16* o = dst + (r >> 4) * 128 + (r & 15) * 8;
+    for (long long t0 = blockIdx.x; t0 < T; t0 += 2ll * gridDim.x) {
+      const long long t1 = t0 + gridDim.x;
+      const uint4 a = *reinterpret_cast<const uint4*>(v + t0 * rs);
+      uint4 b = a;
+      if (t1 < T) b = *reinterpret_cast<const uint4*>(v + t1 * rs);
+      *reinterpret_cast<uint4*>(o + t0 * ds) = a;
+      if (t1 < T) *reinterpret_cast<uint4*>(o + t1 * ds) = b;
+    }
+  }
+}
+__device__ __forceinline__ int token_pos(const int* pos_ids, long long t, long long T, int S, int pos_off) {
+  return pos_ids ? pos_ids[t] : (int)(T <= 0x7fffffff ? (unsigned)t % (unsigned)S : t % S) + pos_off;
+}
+
 // Backward: inverse rotation of dq / dk, LayerNorm backward against the saved pre-norm values and statistics,
 // dv copied; the three results form one contiguous dqkv. The gamma / beta gradients are accumulated per thread
-// (a thread keeps its (head, slice) across tokens), summed over the heads of a kind in shared memory and written as
-// one partial row [4 x 128] per CTA (dgamma_q, dbeta_q, dgamma_k, dbeta_k).
-__global__ void __launch_bounds__(256) qkv_norm_rope_bwd_kernel(
+// (a thread keeps its (head, slice) across tokens), summed over the heads of a kind through shared memory in their order and written
+// as one partial row [4 x 128] per CTA (dgamma_q, dbeta_q, dgamma_k, dbeta_k). Added up by shared-memory atomics, all heads of a
+// kind on the same words, and with one token in flight the pass took 40 us at 2331 tokens and 16 / 8 heads (15 now) and 95 at 6000
+// (55). A head is handled by 16 neighbouring threads (a 4-wide slice of the lower half and its partner in the upper half); a block
+// has a thread per slice of the rotated heads, which keeps it for all tokens of the block with TOK of them in flight. 8-wide slices
+// need twice the registers: they spilled, or left too few threads on an SM to cover the loads.
+template <int NTH, int MINB, int TOK>
+__global__ void __launch_bounds__(NTH, MINB) qkv_norm_rope_bwd_kernel(
     HeadSrc s0, HeadSrc s1, HeadSrc s2, const __nv_bfloat16* qkv, long long row_stride, int hq, int hkv,
     const float* gq, const float* gk, const float2* stats,
     __nv_bfloat16* __restrict__ dqkv, float* __restrict__ partial, const float* cos_t,
     const float* sin_t, const int* pos_ids, long long T, int S, int pos_off) {
   np::pdl_begin();
-  constexpr int HD = 128, HALF = 64;
-  __shared__ float s_acc[4][HD];
+  constexpr int HD = 128, HALF = 64, ROW = 17;   // floats of a thread's row in shared memory: 8 dgamma, 8 dbeta, off the banks
+  extern __shared__ float s_acc[];               // [nrot * 16][ROW]
   const int nrot = hq + hkv, H = hq + 2 * hkv;
-  const int items = nrot * 8 + hkv * 16;
-  const unsigned mask = 0xffu << (threadIdx.x & 24);
-  for (int i = threadIdx.x; i < 4 * HD; i += blockDim.x) (&s_acc[0][0])[i] = 0.f;
-  float dg[2][16], db[2][16];   // up to two rotated items per thread (nrot * 8 <= 512)
+  const int hh = threadIdx.x >> 4, d0 = (threadIdx.x & 15) * 4;
+  const unsigned mask = 0xffffu << (threadIdx.x & 16);
+  const bool is_q = hh < hq;
+  const __nv_bfloat16* gsrc = is_q ? s0.p + (long long)hh * s0.head_stride + d0 : s1.p + (long long)(hh - hq) * s1.head_stride + d0;
+  const long long grs = is_q ? s0.row_stride : s1.row_stride;
+  const __nv_bfloat16* xsrc = qkv + hh * HD + d0;
+  float gl[4], gh[4], dg[8], db[8];
+  ld4f((is_q ? gq : gk) + d0, gl);
+  ld4f((is_q ? gq : gk) + d0 + HALF, gh);
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+  for (int j = 0; j < 8; ++j) { dg[j] = 0.f; db[j] = 0.f; }
+  for (long long t0 = blockIdx.x; t0 < T; t0 += (long long)TOK * gridDim.x) {
+    uint2 ql[TOK], qh[TOK], qa[TOK], qb[TOK];
+    float2 st[TOK];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) { dg[u][j] = 0.f; db[u][j] = 0.f; }
-  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
-    const int pos = pos_ids ? pos_ids[t] : (int)(t % S) + pos_off;
-    const __nv_bfloat16* row = qkv + t * row_stride;
-    __nv_bfloat16* orow = dqkv + t * (long long)H * HD;
-#pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int it = threadIdx.x + u * 256;
-      if (it >= items) break;
-      if (it < nrot * 8) {
-        const int hh = it >> 3, d0 = (it & 7) * 8;
-        const __nv_bfloat16* gsrc = hh < hq ? s0.p + t * s0.row_stride + (long long)hh * s0.head_stride
-                                            : s1.p + t * s1.row_stride + (long long)(hh - hq) * s1.head_stride;
-        float dl[8], dh[8], a[8], b[8], c[8], sn[8], gl[8], gh[8];
-        load8(gsrc + d0, dl);
-        load8(gsrc + d0 + HALF, dh);
-        load8(row + hh * HD + d0, a);
-        load8(row + hh * HD + d0 + HALF, b);
-        ld8f(cos_t + (size_t)pos * HALF + d0, c);
-        ld8f(sin_t + (size_t)pos * HALF + d0, sn);
-        const float* g = hh < hq ? gq : gk;
-        ld8f(g + d0, gl); ld8f(g + d0 + HALF, gh);
-        const float2 st = stats[t * nrot + hh];
-        float ya[8], yb[8], xa[8], xb[8];
-        float m1 = 0.f, m2 = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          ya[j] = dl[j] * c[j] + dh[j] * sn[j];   // gradient at the LayerNorm output
-          yb[j] = dh[j] * c[j] - dl[j] * sn[j];
-          xa[j] = (a[j] - st.x) * st.y;
-          xb[j] = (b[j] - st.x) * st.y;
-          if (u < 2) {
-            dg[u][j] += ya[j] * xa[j]; dg[u][8 + j] += yb[j] * xb[j];
-            db[u][j] += ya[j]; db[u][8 + j] += yb[j];
-          }
-          ya[j] *= gl[j];
-          yb[j] *= gh[j];
-          m1 += ya[j] + yb[j];
-          m2 += ya[j] * xa[j] + yb[j] * xb[j];
-        }
-        m1 = group8_sum(m1, mask) * (1.f / HD);
-        m2 = group8_sum(m2, mask) * (1.f / HD);
-        float oa[8], ob[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          oa[j] = st.y * (ya[j] - m1 - xa[j] * m2);
-          ob[j] = st.y * (yb[j] - m1 - xb[j] * m2);
-        }
-        store8(orow + hh * HD + d0, oa);
-        store8(orow + hh * HD + d0 + HALF, ob);
-      } else {
-        const int r = it - nrot * 8;
-        const int hv = r >> 4, d0 = (r & 15) * 8;
-        *reinterpret_cast<uint4*>(orow + (nrot + hv) * HD + d0) =
-            *reinterpret_cast<const uint4*>(s2.p + t * s2.row_stride + (long long)hv * s2.head_stride + d0);
+    for (int k = 0; k < TOK; ++k) {
+      const long long t = t0 + (long long)k * gridDim.x;
+      if (t < T) {
+        ql[k] = *reinterpret_cast<const uint2*>(gsrc + t * grs);
+        qh[k] = *reinterpret_cast<const uint2*>(gsrc + t * grs + HALF);
+        qa[k] = *reinterpret_cast<const uint2*>(xsrc + t * row_stride);
+        qb[k] = *reinterpret_cast<const uint2*>(xsrc + t * row_stride + HALF);
+        st[k] = stats[t * nrot + hh];
       }
     }
-  }
-  __syncthreads();
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int it = threadIdx.x + u * 256;
-    if (it < nrot * 8) {
-      const int kind = (it >> 3) < hq ? 0 : 2, d0 = (it & 7) * 8;
+    for (int k = 0; k < TOK; ++k) {
+      const long long t = t0 + (long long)k * gridDim.x;
+      if (t >= T) break;   // the same for the whole block
+      const int pos = token_pos(pos_ids, t, T, S, pos_off);
+      float dl[4], dh[4], xa[4], xb[4], c[4], sn[4], ya[4], yb[4];
+      ld4f(cos_t + (size_t)pos * HALF + d0, c);
+      ld4f(sin_t + (size_t)pos * HALF + d0, sn);
+      unpack4(ql[k], dl);
+      unpack4(qh[k], dh);
+      unpack4(qa[k], xa);
+      unpack4(qb[k], xb);
+      float m1 = 0.f, m2 = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        atomicAdd(&s_acc[kind][d0 + j], dg[u][j]);
-        atomicAdd(&s_acc[kind][d0 + HALF + j], dg[u][8 + j]);
-        atomicAdd(&s_acc[kind + 1][d0 + j], db[u][j]);
-        atomicAdd(&s_acc[kind + 1][d0 + HALF + j], db[u][8 + j]);
+      for (int j = 0; j < 4; ++j) {
+        ya[j] = dl[j] * c[j] + dh[j] * sn[j];   // gradient at the LayerNorm output
+        yb[j] = dh[j] * c[j] - dl[j] * sn[j];
+        xa[j] = (xa[j] - st[k].x) * st[k].y;
+        xb[j] = (xb[j] - st[k].x) * st[k].y;
+        dg[j] += ya[j] * xa[j]; dg[4 + j] += yb[j] * xb[j];
+        db[j] += ya[j]; db[4 + j] += yb[j];
+        ya[j] *= gl[j];
+        yb[j] *= gh[j];
+        m1 += ya[j] + yb[j];
+        m2 += ya[j] * xa[j] + yb[j] * xb[j];
       }
+      m1 = group16_sum(m1, mask) * (1.f / HD);
+      m2 = group16_sum(m2, mask) * (1.f / HD);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        ya[j] = st[k].y * (ya[j] - m1 - xa[j] * m2);
+        yb[j] = st[k].y * (yb[j] - m1 - xb[j] * m2);
+      }
+      __nv_bfloat16* orow = dqkv + t * (long long)H * HD + hh * HD + d0;
+      *reinterpret_cast<uint2*>(orow) = pack4(ya);
+      *reinterpret_cast<uint2*>(orow + HALF) = pack4(yb);
     }
   }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    s_acc[threadIdx.x * ROW + j] = dg[j];
+    s_acc[threadIdx.x * ROW + 8 + j] = db[j];
+  }
+  copy_v_heads(s2.p, s2.row_stride, s2.head_stride, dqkv + nrot * HD, (long long)H * HD, hkv, T);
   __syncthreads();
-  for (int i = threadIdx.x; i < 4 * HD; i += blockDim.x) partial[(size_t)blockIdx.x * 4 * HD + i] = (&s_acc[0][0])[i];
+  for (int i = threadIdx.x; i < 4 * HD; i += blockDim.x) {   // (kind, dgamma or dbeta, column)
+    const int kind = i >> 8, beta = (i >> 7) & 1, d = i & (HD - 1);
+    const int lane = (d & (HALF - 1)) >> 2, slot = beta * 8 + (d >= HALF ? 4 : 0) + (d & 3);
+    const int h0 = kind ? hq : 0, h1 = kind ? nrot : hq;
+    float v = 0.f;
+    for (int h = h0; h < h1; ++h) v += s_acc[(h * 16 + lane) * ROW + slot];
+    partial[(size_t)blockIdx.x * 4 * HD + i] = v;
+  }
 }
 
 // cos/sin tables [S, rot/2] in fp32.
@@ -1193,7 +1230,11 @@ NP_API int np_qkv_norm_rope_fwd(const void* qkv, long long row_stride, int hq, i
       sin_t, pos_ids, T, S, pos_off);
   CHECK_LAUNCH();
 }
-NP_API int np_qkv_norm_rope_parts(long long T) { return (int)(T < 296 ? (T > 0 ? T : 1) : 296); }
+// CTAs of the backward pass: as many as are resident (two per SM up to 24 heads of q and k)
+NP_API int np_qkv_norm_rope_parts(long long T) {
+  const long long grid = (T + 1) / 2;
+  return (int)(grid < 148 * 2 ? (grid > 0 ? grid : 1) : 148 * 2);
+}
 // dparams[4 * 128] (+)= (dgamma_q, dbeta_q, dgamma_k, dbeta_k); scratch: fp32 [np_qkv_norm_rope_parts(T), 4 * 128].
 NP_API int np_qkv_norm_rope_bwd(const void* dq, long long rs0, long long hs0, const void* dk, long long rs1,
                                 long long hs1, const void* dv, long long rs2, long long hs2, const void* qkv,
@@ -1208,9 +1249,18 @@ NP_API int np_qkv_norm_rope_bwd(const void* dq, long long rs0, long long hs0, co
       s2{(const __nv_bfloat16*)dv, rs2, hs2, hkv};
   const int grid = np_qkv_norm_rope_parts(T);
   cudaStream_t s = (cudaStream_t)stream;
-  np_launch(qkv_norm_rope_bwd_kernel, grid, 256, 0, s, 1, s0, s1, s2, (const __nv_bfloat16*)qkv, row_stride, hq, hkv, gq, gk,
-                                                (const float2*)stats, (__nv_bfloat16*)dqkv, scratch, cos_t, sin_t,
-                                                pos_ids, T, S, pos_off);
+  constexpr int ROW_BYTES = 17 * 4;
+  static NpPerDeviceOnce attr_once;
+  bool& attr_set = *attr_once.slot();
+  if (!attr_set) {   // more than 48 KB from 45 heads of q and k on
+    const cudaError_t e = cudaFuncSetAttribute(qkv_norm_rope_bwd_kernel<1024, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 * ROW_BYTES);
+    if (e != cudaSuccess) return 400 + (int)e;
+    attr_set = true;
+  }
+  const int nrot = hq + hkv;   // a thread per 4-wide slice of the lower halves of the q and k heads
+  auto kern = nrot <= 24 ? qkv_norm_rope_bwd_kernel<384, 2, 2> : nrot <= 40 ? qkv_norm_rope_bwd_kernel<640, 1, 2> : qkv_norm_rope_bwd_kernel<1024, 1, 1>;
+  np_launch(kern, grid, nrot * 16, (size_t)nrot * 16 * ROW_BYTES, s, 1, s0, s1, s2, (const __nv_bfloat16*)qkv, row_stride, hq, hkv, gq, gk,
+            (const float2*)stats, (__nv_bfloat16*)dqkv, scratch, cos_t, sin_t, pos_ids, T, S, pos_off);
   np_launch(colsum_tall_kernel, (4 * 128 + 31) / 32, 256, 0, s, 1, scratch, dparams, grid, 4 * 128, accumulate);
   CHECK_LAUNCH();
 }

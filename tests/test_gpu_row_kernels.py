@@ -285,3 +285,30 @@ def test_swiglu_at_the_ends_of_the_range():
     d = gemm_glu_bwd(one, eye, torch.cat([X, 0.75 * one], 1).contiguous())
     want = torch.where(finite, g64.grad[0], torch.full_like(g64.grad[0], 0.375))
     torch.testing.assert_close(d[:, :F].double(), want.expand(M, F), rtol=2 ** -7, atol=1e-34)
+
+
+# fewer heads than a warp holds, each of the three block sizes, one token, an odd number of tokens, more tokens than CTAs take twice
+@pytest.mark.parametrize("B,S,hq,hkv", [(1, 1, 2, 1), (1, 77, 3, 3), (3, 777, 16, 8), (1, 1201, 32, 8), (2, 35, 40, 8), (1, 6, 56, 8)])
+def test_qkv_norm_rope_backward(B, S, hq, hkv):
+    from nanopysche_b200.ops.rope import qkv_norm_rope, rope_tables
+
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, (hq + 2 * hkv) * 128, device="cuda").bfloat16().requires_grad_(True)
+    norms = [torch.nn.LayerNorm(128, device="cuda") for _ in range(2)]
+    for m in norms:
+        torch.nn.init.normal_(m.weight, 1.0, 0.2), torch.nn.init.normal_(m.bias, 0.0, 0.2)
+    par = [p for m in norms for p in m.parameters()]
+    cos, sin = rope_tables(S + 3, 128, device="cuda")
+    out = qkv_norm_rope(qkv, *norms, cos, sin, hq, hkv, 3)
+    g = [torch.randn_like(t) for t in out]
+    got = torch.autograd.grad(out, [qkv, *par], g)
+    x = qkv.detach().double().requires_grad_(True)
+    p64 = [p.detach().double().requires_grad_(True) for p in par]
+    h = x.view(B, S, hq + 2 * hkv, 128)
+    n = [torch.nn.functional.layer_norm(t, (128,), *p64[2 * i:2 * i + 2], norms[i].eps) for i, t in enumerate((h[:, :, :hq], h[:, :, hq:hq + hkv]))]
+    c, s = cos.double()[3:3 + S][None, :, None], sin.double()[3:3 + S][None, :, None]
+    rot = [torch.cat([t[..., :64] * c - t[..., 64:] * s, t[..., 64:] * c + t[..., :64] * s], -1) for t in n]
+    want = torch.autograd.grad([*rot, h[:, :, hq + hkv:]], [x, *p64], [t.double() for t in g])
+    assert rel(got[0], want[0]) < 4e-3
+    for a, b in zip(got[1:], want[1:]):      # fp32 sums over tokens and heads of bf16 terms
+        assert rel(a, b) < 1e-4
