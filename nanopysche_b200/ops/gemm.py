@@ -341,21 +341,25 @@ class _SwiGLUFeedForward(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, w13, w2, h, gu = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        x2 = x.reshape(-1, x.shape[-1])
-        want_dw2 = ctx.needs_input_grad[2] or hasattr(w2, "main_grad")
-        dx = dw13 = dw2 = None
-        if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or hasattr(w13, "main_grad")):
-            return None, None, _wgrad_into(w2, dy2, h) if want_dw2 else None, None
-        if want_dw2:
-            dgu, dw2 = _both_grads(w2, dy2, h, gu)
-        else:
-            dgu = gemm_glu_bwd(dy2, w2, gu)
-        dx, dw13 = _linear_grads(ctx, w13, dgu, x2)
-        return None if dx is None else dx.view(x.shape), dw13, dw2, None
+        dx, dw13, dw2 = _feed_forward_grads(ctx, dy)
+        return None if dx is None else dx.view(dy.shape[:-1] + dx.shape[-1:]), dw13, dw2, None
+
+
+def _feed_forward_grads(ctx, dy: torch.Tensor):
+    """``(dx [rows, D], dw13, dw2)`` as far as they are asked for (inputs 0 to 2 of the autograd function, which saved ``x, w13,
+    w2, h, gu``)."""
+    x, w13, w2, h, gu = ctx.saved_tensors
+    dy2 = dy.reshape(-1, dy.shape[-1])
+    if not dy2.is_contiguous():
+        dy2 = dy2.contiguous()
+    want_dw2 = ctx.needs_input_grad[2] or hasattr(w2, "main_grad")
+    if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or hasattr(w13, "main_grad")):
+        return None, None, _wgrad_into(w2, dy2, h) if want_dw2 else None
+    if want_dw2:
+        dgu, dw2 = _both_grads(w2, dy2, h, gu)
+    else:
+        dgu, dw2 = gemm_glu_bwd(dy2, w2, gu), None
+    return *_linear_grads(ctx, w13, dgu, x.reshape(-1, x.shape[-1])), dw2
 
 
 def _plain_weight(w: torch.Tensor) -> bool:
@@ -376,4 +380,12 @@ def feed_forward_glu(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, act: 
         x2 = x if x.is_contiguous() and x.data_ptr() % 16 == 0 else x.clone(memory_format=torch.contiguous_format)
         save = torch.is_grad_enabled() and (x2.requires_grad or w13.requires_grad or w2.requires_grad)
         return _SwiGLUFeedForward.apply(x2, w13, w2, save)
+    if (act == "silu" and not SPLIT_MODE and _lib.on(x) and x.dtype == torch.bfloat16 and x.numel() > 0 and
+            getattr(w13, "_fp8_recipe", None) == getattr(w2, "_fp8_recipe", None) == "mxfp8" and
+            all(w.is_contiguous() and getattr(w, "_fsdp_rt", None) is None for w in (w13, w2))):
+        from .gemm_mxfp8 import _MXFeedForward, mx_linear_supported
+
+        if mx_linear_supported(x, w13) and mx_linear_supported(x, w2):
+            save = torch.is_grad_enabled() and (x.requires_grad or w13.requires_grad or w2.requires_grad)
+            return _MXFeedForward.apply(x, w13, w2, save)
     return linear(glu(linear(x, w13), act), w2)

@@ -53,13 +53,27 @@ def mx_quantize(x: torch.Tensor):
     """bf16 ``[rows, K]`` (K a multiple of 128, unit column stride) -> ``(e4m3 [rows, K], uint8 scale chunks)``."""
     if not x.is_cuda:
         return mx_quantize_ref(x)
-    rows, K = x.shape
+    return _mx_quant(x, x.shape[1], None)
+
+
+def mx_quantize_glu(gu: torch.Tensor):
+    """``h = silu(gate) * up`` of ``gu = [gate | up]`` in bf16 and quantised, in one pass: ``(e4m3, scale chunks, h)``."""
+    from .activation import glu_ref
+
+    if not gu.is_cuda:
+        h = glu_ref(gu)
+        return (*mx_quantize_ref(h), h)
+    h = torch.empty((gu.shape[0], gu.shape[1] // 2), device=gu.device, dtype=torch.bfloat16)
+    return (*_mx_quant(gu, h.shape[1], h), h)
+
+
+def _mx_quant(x: torch.Tensor, K: int, h: Optional[torch.Tensor]):
+    rows = x.shape[0]
     assert x.dtype == torch.bfloat16 and x.stride(1) == 1 and K % 128 == 0
     q = torch.empty((rows, K), device=x.device, dtype=torch.float8_e4m3fn)
-    sf = torch.full((sf_bytes(rows, K),), 127, dtype=torch.uint8, device=x.device)
-    _lib.check(_lib.lib().np_mx_quant(C.c_void_p(x.data_ptr()), C.c_longlong(x.stride(0)), C.c_void_p(q.data_ptr()),
-                                      C.c_longlong(K), C.c_void_p(sf.data_ptr()), rows, K,
-                                      C.c_void_p(_lib.stream())), "mx_quant")
+    sf = torch.empty((sf_bytes(rows, K),), dtype=torch.uint8, device=x.device)
+    _lib.check(_lib.lib().np_mx_quant(x.data_ptr(), x.stride(0), q.data_ptr(), K, sf.data_ptr(), rows, K,
+                                      h.data_ptr() if h is not None else None, K, _lib.stream()), "mx_quant")
     return q, sf
 
 
@@ -239,6 +253,30 @@ class _MXLinear(torch.autograd.Function):
         dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
         dx, dw = _linear_grads(ctx, w, dy2, x2)
         return None if dx is None else dx.view(ctx.x_shape), dw
+
+
+class _MXFeedForward(torch.autograd.Function):
+    """``(silu(x @ w1.T) * (x @ w3.T)) @ w2.T`` for a fused ``[w1; w3]`` weight with both forward GEMMs in MXFP8: the activation is
+    formed, rounded and quantised in one pass. The backward GEMMs run in bf16 on the unquantised tensors, the gradient of the
+    activation in the epilogue of the down projection's (4096 tokens, 2048 x 5632: quantisers and activation passes 123 -> 68 us)."""
+
+    @staticmethod
+    def forward(ctx, x, w13, w2, save):
+        x2 = x.reshape(-1, x.shape[-1])
+        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        gu = gemm_mxfp8(*mx_quantize(x2), *mx_quantize(w13))
+        hq, sh, h = mx_quantize_glu(gu)
+        if save:
+            ctx.save_for_backward(x2, w13, w2, h, gu)
+        ctx.x_shape = x.shape
+        return gemm_mxfp8(hq, sh, *mx_quantize(w2)).view(*x.shape[:-1], w2.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy):
+        from .gemm import _feed_forward_grads
+
+        dx, dw13, dw2 = _feed_forward_grads(ctx, dy)
+        return None if dx is None else dx.view(ctx.x_shape), dw13, dw2, None
 
 
 def mx_linear_supported(x: torch.Tensor, w: torch.Tensor) -> bool:

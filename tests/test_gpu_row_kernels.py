@@ -312,3 +312,39 @@ def test_qkv_norm_rope_backward(B, S, hq, hkv):
     assert rel(got[0], want[0]) < 4e-3
     for a, b in zip(got[1:], want[1:]):      # fp32 sums over tokens and heads of bf16 terms
         assert rel(a, b) < 1e-4
+
+
+# rows off a scale chunk of 128, one row, several column blocks; a row of zeros and the smallest and largest magnitudes
+@pytest.mark.parametrize("rows,K", [(1, 128), (100, 384), (129, 256), (1000, 2816)])
+def test_mx_quantiser_in_one_pass_with_swiglu(rows, K):
+    from nanopysche_b200.ops.activation import glu
+    from nanopysche_b200.ops.gemm_mxfp8 import mx_quantize, mx_quantize_glu, mx_quantize_ref
+
+    torch.manual_seed(K)
+    gu = (torch.randn(rows, 2 * K, device="cuda") * torch.exp2(torch.randint(-40, 20, (rows, 1), device="cuda").float())).bfloat16()
+    gu[0, :K // 2] = 0
+    x = gu[:, K:]
+    for got, want in ((mx_quantize(x.contiguous()), mx_quantize_ref(x)), (mx_quantize(x), mx_quantize_ref(x))):
+        assert torch.equal(got[0].view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(got[1], want[1])
+    q, sf, h = mx_quantize_glu(gu)
+    two = mx_quantize(glu(gu))
+    assert torch.equal(h, glu(gu)) and torch.equal(q.view(torch.uint8), two[0].view(torch.uint8)) and torch.equal(sf, two[1])
+
+
+@pytest.mark.parametrize("rows,D,F", [(3, 128, 128), (200, 256, 384), (1030, 512, 1408)])
+def test_mx_feed_forward_in_one_node(rows, D, F):
+    """The same forward as the separate layers, bit for bit; gradients without the rounding of dh between them."""
+    from nanopysche_b200.ops.activation import glu
+    from nanopysche_b200.ops.gemm import feed_forward_glu, linear
+
+    torch.manual_seed(F)
+    x = torch.randn(rows, D, device="cuda").bfloat16().requires_grad_(True)
+    w13, w2 = ((torch.randn(n, k, device="cuda") * k ** -0.5).bfloat16().requires_grad_(True) for n, k in ((2 * F, D), (D, F)))
+    w13._fp8_recipe = w2._fp8_recipe = "mxfp8"
+    dy = torch.randn(rows, D, device="cuda").bfloat16()
+    y, z = feed_forward_glu(x, w13, w2), linear(glu(linear(x, w13)), w2)
+    assert type(y.grad_fn).__name__ == "_MXFeedForwardBackward" and torch.equal(y, z)
+    for a, b in zip(torch.autograd.grad(y, [x, w13, w2], dy), torch.autograd.grad(z, [x, w13, w2], dy)):
+        assert rel(a, b) < 6e-3      # bf16 roundings of dh, d gate and d up
+    with torch.no_grad():
+        assert torch.equal(feed_forward_glu(x, w13, w2), z)
