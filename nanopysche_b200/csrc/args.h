@@ -42,6 +42,7 @@ struct NpGemmArgs {
   int k_split;        // > 0 (MN-major B): K rows [0, k_split) of a group come from B, the rest from B2 (multiple of 64)
   int m_split;        // > 0: output rows [0, m_split) go to C, the rest to C2 (layout of C; multiple of 256)
   int pair_bn;        // columns of a pair's tile: 0 = choose, 128, 192 or 256
+  int local_push;     // the destinations behind peer_base and done_flag_ptr are this GPU's: ordered at device scope
 };
 
 // Tensor layout of q / k / v / o: [B, S, H, 128] bf16 with element strides (sb, ss, sh); the last dim is

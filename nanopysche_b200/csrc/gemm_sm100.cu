@@ -52,6 +52,7 @@ struct GemmParams {
   int* done_counters;         // [flags] tiles finished per destination (local)
   const int* done_expected;   // [flags] M blocks expected per destination (x n_blocks tiles each)
   int* const* done_flag_ptr;  // [flags] peer flag word to release when a destination completes
+  bool local_push;            // every destination is this GPU's own memory
   const void* Cin;            // accumulate source (same dtype as C), rows indexed like a dense C
   long long ldcin;
   const int* epoch_base;      // optional device counter added to `epoch` (keeps epochs valid under graph replay)
@@ -127,6 +128,23 @@ __device__ __forceinline__ int count_k(const GemmParams& p, int g) {
 struct Tile {
   int g, m_blk, n_blk;
 };
+
+// One tile's rows are stored by this warp: publish them, count the tile against its destination and release the destination's
+// flag when it is done (`need` arrivals). A system-wide fence takes some 3 us; on one GPU the device scope does.
+__device__ __forceinline__ void count_done(const GemmParams& p, int fi, int need, int epoch, int lane) {
+  if (p.local_push) __threadfence();
+  else __threadfence_system();
+  __syncwarp();
+  if (lane == 0 && atomicAdd(&p.done_counters[fi], 1) + 1 == need) {
+    if (p.local_push) {
+      __threadfence();
+      np::st_release_gpu(p.done_flag_ptr[fi], epoch);
+    } else {
+      __threadfence_system();
+      np::st_release_sys(p.done_flag_ptr[fi], epoch);
+    }
+  }
+}
 
 // Operand tile in shared memory (64-wide K stage): descriptor of its first 16-wide K step, and what one K step adds to the
 // (16-byte) address field. K-major: 32 bytes along the swizzled row; MN-major: 16 rows of 128 bytes.
@@ -745,20 +763,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) np::mbar_arrive(tempty_bar(acc));
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
-      if (p.done_counters) {
-        // all rows of this tile are stored (possibly into peer memory): publish, then count the
-        // tile against its destination and release the peer's flag when the destination is done.
-        __threadfence_system();
-        __syncwarp();
-        if (lane == 0) {
-          // each epilogue warp counts once per tile: expected is in tiles
-          const int fi = p.mblk_flag ? p.mblk_flag[tl.m_blk] : 0;
-          const int done = atomicAdd(&p.done_counters[fi], 1) + 1;
-          if (done == EPI_WARPS * n_blocks * p.done_expected[fi]) {  // done_expected counts M blocks
-            __threadfence_system();
-            np::st_release_sys(p.done_flag_ptr[fi], epoch);
-          }
-        }
+      if (p.done_counters) {   // each epilogue warp counts once per tile; done_expected counts M blocks
+        const int fi = p.mblk_flag ? p.mblk_flag[tl.m_blk] : 0;
+        count_done(p, fi, EPI_WARPS * n_blocks * p.done_expected[fi], epoch, lane);
       }
     }
     if (p.tma_c) stage_drain(lane);
@@ -967,7 +974,7 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
   np::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   np::pdl_begin();
-  const int epoch = p.epoch + (p.epoch_base ? *p.epoch_base : 0);   // a launch of two products: the first one's
+  auto epoch = [](const GemmParams& q) { return q.epoch + (q.epoch_base ? *q.epoch_base : 0); };
 
   // rows of the two 128-row blocks of an M block that carry data, as a mask (0: nothing to do, -1: gave up). Row-grouped
   // form: both blocks belong to the same group and arrive under the same flag (the caller's tables are made of pairs).
@@ -976,7 +983,7 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
     const int b0 = 2 * tl.m_blk;
     if (q.ready_flags) {
       const int fi = q.mblk_flag ? q.mblk_flag[b0] : 0;
-      if (fi >= 0 && !np::wait_flag_ge(q.ready_flags + fi, epoch, q.flag_limit_ns, KID_GEMM, 120 + role)) {
+      if (fi >= 0 && !np::wait_flag_ge(q.ready_flags + fi, epoch(q), q.flag_limit_ns, KID_GEMM, 120 + role)) {
         *abort_flag = 1;
         return -1;
       }
@@ -1121,17 +1128,9 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
         if (lane == 0) arrive_cluster(peer_addr(tempty_bar(acc), lead));
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
-      if (q.done_counters && mine) {
-        __threadfence_system();
-        __syncwarp();
-        if (lane == 0) {
-          const int fi = q.mblk_flag ? q.mblk_flag[2 * tl.m_blk] : 0;
-          const int n_done = atomicAdd(&q.done_counters[fi], 1) + 1;
-          if (n_done == EPI_WARPS * n_blocks(q) * q.done_expected[fi]) {   // done_expected counts 128-row blocks
-            __threadfence_system();
-            np::st_release_sys(q.done_flag_ptr[fi], epoch);
-          }
-        }
+      if (q.done_counters && mine) {   // done_expected counts 128-row blocks
+        const int fi = q.mblk_flag ? q.mblk_flag[2 * tl.m_blk] : 0;
+        count_done(q, fi, EPI_WARPS * n_blocks(q) * q.done_expected[fi], epoch(q), lane);
       }
     }
     stage_drain(lane);
@@ -1362,6 +1361,7 @@ static int prepare_gemm(const NpGemmArgs& a, int splits, PairMaps& m, CUtensorMa
   p.flag_limit_ns = a.flag_limit_ns ? a.flag_limit_ns : NP_WAIT_LIMIT_NS;
   p.row_dst = a.row_dst; p.peer_base = a.peer_base;
   p.done_counters = a.done_counters; p.done_expected = a.done_expected; p.done_flag_ptr = a.done_flag_ptr;
+  p.local_push = a.local_push != 0;
   p.Cin = a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr);
   p.ldcin = a.Cin ? a.ldcin : a.ldc;
   p.epoch_base = a.epoch_base;
@@ -1481,6 +1481,14 @@ struct GemmChoice {
   int bn, splits;
   double cost;   // estimate in us
 };
+// Tiles of tm x tn and K steps of a tile. Grouped forms by the room of their regions, as which rows arrive is not known here; an estimate
+// from the mean rows per expert chose worse (the six GEMMs of an expert layer 525 -> 609 us at 4096 tokens, 174 -> 208 at 512).
+static long long tiles_of(const NpGemmArgs& a, int tm, int tn) {
+  return (long long)((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn) * (a.mode == 2 ? a.num_groups : 1);
+}
+static double tile_steps(const NpGemmArgs& a) { return a.mode == 2 ? 2.0 * a.blocks_per_group : (a.K + BK - 1) / BK; }
+static double operations(const NpGemmArgs& a) { return tiles_of(a, BM, BM) * 2.0 * BM * BM * BK * tile_steps(a); }
+
 static GemmChoice choose_gemm(const NpGemmArgs& a) {
   const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
                      (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
@@ -1497,11 +1505,9 @@ static GemmChoice choose_gemm(const NpGemmArgs& a) {
     c.pair = true;   // asked for
     c.bn = split_asked || pbn_asked == 0 ? 256 : pbn_asked;
   } else if (bn_asked == 0 || (bn_asked == 256 && a.mt == 0)) {
-    const long long groups = a.mode == 2 ? a.num_groups : 1;
-    // K steps of a group: its share of the token axis in the K-grouped form
-    const double steps = a.mode == 2 ? 2.0 * a.blocks_per_group : nk;
+    const double steps = tile_steps(a);
     auto take = [&](const TileCost& t, int tm, int tn, int units, int parts, bool pair, int bn) {
-      const long long n = (long long)((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn) * groups;
+      const long long n = tiles_of(a, tm, tn);
       const double waves = (double)((n + units - 1) / units);
       // tiles of a persistent CTA follow one another; a cluster that splits K starts anew for every tile
       const double cost = parts == 1 ? t.fixed + waves * (steps * t.step + t.drain) : waves * (t.fixed + steps / parts * t.step + t.drain);
@@ -1568,16 +1574,15 @@ static int launch_gemm2(const NpGemmArgs& a, const NpGemmArgs& b, int extra, cud
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
   }
-  auto tiles = [](const NpGemmArgs& g) { return (long long)((g.M + 255) / 256) * ((g.N + BN - 1) / BN); };
-  const long long n = tiles(a) + tiles(b), pairs = n < num_sms() / 2 ? n : num_sms() / 2;
-  const bool busy = 2.0 * a.M * a.N * a.K + 2.0 * b.M * b.N * b.K > 2e10;   // 15 us and more
+  const long long n = tiles_of(a, 256, BN) + tiles_of(b, 256, BN), pairs = n < num_sms() / 2 ? n : num_sms() / 2;
+  const bool busy = operations(a) + operations(b) > 2e10;   // 15 us and more
   cudaError_t e = np_launch_if(busy, gemm_bf16_pair2_kernel<BN>, dim3((unsigned)(2 * pairs)), GEMM_THREADS, SMEM, stream, 2, m, p, second);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
-// Two independent products: in one launch where both are dense, run on pairs of CTAs and are expected to take less time that way,
-// else one after the other. `pair_bn` of the first asks for one launch with tiles of that many columns, `split` 1 or `mt` 2 of
+// Two independent products: in one launch where both run on pairs of CTAs and are expected to take less time that way, else one after
+// the other. A product grouped by rows may wait for arrivals and push; what the other one reads has to be there at launch. `pair_bn` of the first asks for one launch with tiles of that many columns, `split` 1 or `mt` 2 of
 // the first for two launches.
 NP_API int np_gemm_bf16_two(const NpGemmArgs* first, const NpGemmArgs* second, void* stream) {
   const NpGemmArgs &a = *first, &b = *second;
@@ -1585,28 +1590,27 @@ NP_API int np_gemm_bf16_two(const NpGemmArgs* first, const NpGemmArgs* second, v
     const int rc = np_gemm_bf16(first, stream);
     return rc ? rc : np_gemm_bf16(second, stream);
   };
-  auto dense = [](const NpGemmArgs& g) {
-    return g.M > 128 && g.N > 0 && g.K > 0 && g.mode == 0 && g.epilogue != 1 && !g.b_ready_flags && !g.push_src && !g.A_loc && !g.B_loc &&
-           g.m_rot == 0 && g.n_rot == 0 && !g.row_dst && !g.ready_flags && !g.done_counters && g.bn == 0 && g.mt == 0 && g.split == 0 &&
-           g.max_ctas == 0 && g.m_split == 0;
+  auto pairable = [](const NpGemmArgs& g) {
+    return g.M > 128 && g.N > 0 && g.K > 0 && g.epilogue != 1 && !g.b_ready_flags && !g.push_src && !g.A_loc && !g.B_loc &&
+           g.m_rot == 0 && g.n_rot == 0 && g.bn == 0 && g.mt == 0 && g.split == 0 && g.max_ctas == 0 &&
+           (g.mode == 1 ? g.paired != 0 : !g.row_dst && !g.ready_flags && !g.done_counters) && (g.mode != 2 || g.num_groups > 0);
   };
   const int units = num_sms() / 2;
   // Long products run at the power limit: SMs that idle let the others run faster, so there is nothing to fill (us, two launches /
   // one: 4096 tokens, 2048 x 11264, 3.8e11 operations 261 / 256; 2048 x 32000, 1.1e12 799 / 846).
-  const bool long_run = 2.0 * a.M * a.N * a.K + 2.0 * b.M * b.N * b.K > 6e11 && a.pair_bn == 0;
-  if (!dense(a) || !dense(b) || b.pair_bn != 0 || units < 1 || long_run) return separate();
+  const bool long_run = operations(a) + operations(b) > 6e11 && a.pair_bn == 0;
+  if (!pairable(a) || !pairable(b) || b.pair_bn != 0 || units < 1 || long_run) return separate();
   if (!bind_context()) return 2;
   if (check_gemm(a) || check_gemm(b)) return 1;
   // the longer contraction first
-  const bool swap = b.K > a.K;
+  const bool swap = tile_steps(b) > tile_steps(a);
   const NpGemmArgs &x = swap ? b : a, &y = swap ? a : b;
-  const double sx = (x.K + BK - 1) / BK, sy = (y.K + BK - 1) / BK;
+  const double sx = tile_steps(x), sy = tile_steps(y);
   double best = a.pair_bn != 0 ? 1e30 : choose_gemm(a).cost + choose_gemm(b).cost;
   int bn = 0, extra = 0;
   auto take = [&](const TileCost& t, int cols) {   // the pair with the most to do
     if (a.pair_bn != 0 && a.pair_bn != cols) return;
-    const int nx = (int)(((long long)(x.M + 255) / 256) * ((x.N + cols - 1) / cols));
-    const int ny = (int)(((long long)(y.M + 255) / 256) * ((y.N + cols - 1) / cols));
+    const int nx = (int)tiles_of(x, 256, cols), ny = (int)tiles_of(y, 256, cols);
     const int pairs = nx + ny < units ? nx + ny : units;
     const double cx = sx * t.step + t.drain, cy = sy * t.step + t.drain;
     const int ex = (int)(cx / cy);

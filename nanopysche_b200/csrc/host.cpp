@@ -539,7 +539,7 @@ struct MoeRuntime : torch::CustomClassHolder {
   void push_to(NpGemmArgs& g, const Tensor& peers, int epoch) const {   // output rows go back to their sources
     g.row_dst = (const long long*)row_dst.data_ptr(); g.peer_base = (void* const*)peers.data_ptr();
     g.done_counters = ptr<int>(done_counters); g.done_expected = ptr<int>(src_blocks);
-    g.done_flag_ptr = (int* const*)p_done_flag.data_ptr(); g.epoch = epoch; g.ldc = g.N;
+    g.done_flag_ptr = (int* const*)p_done_flag.data_ptr(); g.epoch = epoch; g.ldc = g.N; g.local_push = N == 1;
   }
   // A [rows, M (x outputs)] and B [rows, N] contracted over the rows of every expert, into the fp32 outputs of M rows per expert
   NpGemmArgs by_expert(const Tensor& A, const Tensor& B, int64_t M, int64_t n, const std::vector<Tensor>& outs, bool add) const {
@@ -550,6 +550,17 @@ struct MoeRuntime : torch::CustomClassHolder {
     g.a_mn = g.b_mn = 1; g.mode = 2; g.alpha = 1.f; g.out_f32 = 1; g.accumulate = add; g.mblk_rows = ptr<int>(mblk_rows);
     g.num_groups = (int)E_local; g.blocks_per_group = (int)(N * bpr); g.group_stride_c = M * n;
     return g;
+  }
+  // A product over the dispatched rows and the weight gradient beside it: together when this rank is the only one (the rows are
+  // there when the dispatch kernel has ended; rows of peers are waited for by the first product alone). The six expert GEMMs,
+  // us, apart / paired: 4096 tokens, 8 experts of 2048 x 2816 606 / 525, 512 of 768 x 2048 199 / 174, 2472, 16 of 1024 x 2816 417 / 382.
+  void both(const NpGemmArgs& rows, const NpGemmArgs& experts) const {
+    if (N == 1) {
+      launched(np_gemm_bf16_two(&rows, &experts, stream()), "grouped_gemm and grouped_wgrad");
+    } else {
+      launched(np_gemm_bf16(&rows, stream()), "grouped_gemm");
+      launched(np_gemm_bf16(&experts, stream()), "grouped_wgrad");
+    }
   }
 };
 
@@ -648,35 +659,32 @@ struct FusedMoE : torch::autograd::Function<FusedMoE> {
     NpGemmArgs g = rt->by_rows(rt->recv_g, w2, H, D, false);
     g.epilogue = 2; g.C2 = gu.data_ptr(); g.ldc2 = gu.stride(0); g.C = dgu.data_ptr(); g.ldc = dgu.stride(0);
     rt->wait_for(g, epoch);
-    launched(np_gemm_bf16(&g, stream()), "grouped_gemm");
     ExpertGrads d2 = expert_outputs({w2}, rt->E_local * H, D);
-    g = rt->by_expert(h, rt->recv_g, H, D, d2.outs, d2.add);
-    launched(np_gemm_bf16(&g, stream()), "grouped_wgrad");
+    rt->both(g, rt->by_expert(h, rt->recv_g, H, D, d2.outs, d2.add));
     expert_done(d2, {w2});
     const Tensor& xr = rt->recv_x[layer];
     Tensor dw1, dw3;
-    if (H % 256 == 0 && same_main_grad(w1, w3)) {   // gate and up against the same rows in one launch
-      ExpertGrads d = expert_outputs({w1, w3}, rt->E_local * H, D);
-      g = rt->by_expert(dgu, xr, H, D, d.outs, d.add);
-      launched(np_gemm_bf16(&g, stream()), "grouped_wgrad");
-      expert_done(d, {w1, w3});
-      dw1 = d.grads[0]; dw3 = d.grads[1];
-    } else {
-      for (int i = 0; i < 2; ++i) {
-        const Tensor& w = i ? w3 : w1;
-        ExpertGrads d = expert_outputs({w}, rt->E_local * H, D);
-        g = rt->by_expert(dgu.narrow(1, i * H, H), xr, H, D, d.outs, d.add);
-        launched(np_gemm_bf16(&g, stream()), "grouped_wgrad");
-        expert_done(d, {w});
-        (i ? dw3 : dw1) = d.grads[0];
-      }
-    }
     // dX = [dG | dU] @ [w1; w3], one contraction over both weights (no bf16 partial result in between), pushed back to the
     // sources. H is a multiple of 256 (MoEBase), the K steps of 64 never straddle the two.
     g = rt->by_rows(dgu, w1, D, 2 * H, true);
     g.B2 = w3.data_ptr(); g.k_split = (int)H;
     rt->push_to(g, rt->p_ret_g, epoch);
-    launched(np_gemm_bf16(&g, stream()), "grouped_gemm");
+    if (H % 256 == 0 && same_main_grad(w1, w3)) {   // gate and up against the same rows in one product
+      ExpertGrads d = expert_outputs({w1, w3}, rt->E_local * H, D);
+      rt->both(g, rt->by_expert(dgu, xr, H, D, d.outs, d.add));
+      expert_done(d, {w1, w3});
+      dw1 = d.grads[0]; dw3 = d.grads[1];
+    } else {
+      launched(np_gemm_bf16(&g, stream()), "grouped_gemm");
+      for (int i = 0; i < 2; ++i) {
+        const Tensor& w = i ? w3 : w1;
+        ExpertGrads d = expert_outputs({w}, rt->E_local * H, D);
+        const NpGemmArgs e = rt->by_expert(dgu.narrow(1, i * H, H), xr, H, D, d.outs, d.add);
+        launched(np_gemm_bf16(&e, stream()), "grouped_wgrad");
+        expert_done(d, {w});
+        (i ? dw3 : dw1) = d.grads[0];
+      }
+    }
     rt->pushed();
     Tensor dx = at::empty({T, D}, b16);
     rt->combine(rt->ret_g, slot_pos, Tensor(), Tensor(), dx, sent, epoch);

@@ -50,7 +50,7 @@ class GemmArgs(C.Structure):
         ("push_n", c_int), ("push_ctr", c_void_p),
         ("bias", c_void_p),
         ("mt", c_int), ("split", c_int), ("paired", c_int),
-        ("k_split", c_int), ("m_split", c_int), ("pair_bn", c_int),
+        ("k_split", c_int), ("m_split", c_int), ("pair_bn", c_int), ("local_push", c_int),
     ]
 
 

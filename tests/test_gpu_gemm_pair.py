@@ -285,3 +285,43 @@ def test_the_kernel_asked_for_runs(kw, pair):
     gemm(a, b, out=out, **kw)
     assert rel(out, a.double() @ b.double().t()) < 2e-5
     assert ("pair" in _kernels(lambda: gemm(a, b, out=out, **kw))) == pair
+
+
+# the expert layer's backward with two products per launch: regions of several row blocks, uneven and empty experts, a capacity that
+# drops tokens, gradients into new tensors and added to main_grad
+@pytest.mark.parametrize("T,E,K,capacity", [(1000, 4, 2, None), (1536, 8, 2, 1.25), (2050, 16, 1, None), (520, 4, 4, 2.0)])
+def test_expert_layer_backward_against_64_bits(T, E, K, capacity):
+    from nanopysche_b200.engine import prepare_training
+    from nanopysche_b200.models.moe import MoEBase
+
+    D, H = 256, 512
+    torch.manual_seed(T)
+    m = MoEBase(d_model=D, hidden_size=H, num_experts=E, top_k=K, capacity_factor=capacity, dtype=torch.bfloat16, device="cuda")
+    with torch.no_grad():
+        for w in (m.w1, m.w2, m.w3, m.router.gate.weight):
+            w.normal_(0, 0.05)
+        if K < E:
+            m.router.gate.bias.zero_()[-1] = -30.0      # an expert without tokens
+    _, arena = prepare_training(m, tokens_per_rank=T, lr=1e-3)
+    x = torch.randn(1, T, D, device="cuda").bfloat16().requires_grad_(True)
+    dy = torch.randn(1, T, D, device="cuda").bfloat16() * 0.1
+    for _ in range(2):      # the second pass adds to the gradients of the first
+        x.grad = None
+        m(x).backward(dy)
+    p = {n: w.detach().double().requires_grad_(True) for n, w in m.named_parameters()}
+    x64 = x.detach().double()[0].requires_grad_(True)
+    logits = x64 @ p["router.gate.weight"].t() + p["router.gate.bias"]
+    top, idx = logits.topk(K, -1)
+    gate, hit = top.softmax(-1), torch.zeros(T, E, device="cuda", dtype=torch.double).scatter_(1, idx, 1.0)
+    keep = torch.ones(T, device="cuda", dtype=torch.bool) if capacity is None else ~((hit > 0) & (hit.cumsum(0) > int(capacity * T / E))).any(1)
+    y = torch.zeros_like(x64)
+    for e in range(E):
+        t, k = ((idx == e) & keep[:, None]).nonzero(as_tuple=True)
+        r = slice(e * H, (e + 1) * H)
+        he = torch.nn.functional.silu(x64[t] @ p["w1"][r].t()) * (x64[t] @ p["w3"][r].t())
+        y = y.index_add(0, t, he @ p["w2"][r] * gate[t, k][:, None])
+    want = torch.autograd.grad(y, [x64, *(p[n] for n in ("w1", "w2", "w3"))], dy.double()[0])
+    assert rel(x.grad[0], want[0]) < 1.5e-2          # bf16 activations and gradients between five products
+    main = dict(arena.named_main_grads())
+    for n, g in zip(("w1", "w2", "w3"), want[1:]):
+        assert rel(main[n].view(g.shape), 2 * g) < 1.5e-2
