@@ -36,69 +36,78 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 // ------------------------------------------------------------------ router
-// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). A warp takes TOK tokens at a time and has V
-// vectors of each row in flight; MINB: CTAs per SM that the register count is held to. Every token's sum is formed in the same
-// order in all forms (np_router_logits chooses). The gate rows are 64 KB per token at d 2048 and 8 experts, read through L1.
-template <int EB, int TOK, int V, int MINB>
+// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). Four warps share TOK tokens, each over a quarter of
+// the vectors of a row; MINB: CTAs per SM that the register count is held to, U: steps whose loads are in flight together. The gate
+// rows are 64 KB per TOK tokens at d 2048 and 8 experts, read through L1; a warp to a token (or, above 8192 tokens, to four) had the
+// chain of its eight loads to wait for as well. 8 experts, us, before / now: 64 x 2048 7.1 / 3.9, 1024 10.9 / 4.6, 4096 20.4 / 11.6,
+// 16384 41.2 / 30.4; 64 experts, 4096 x 1024 82 / 48.
+// Every token's sum is formed in the same order in all forms (np_router_logits chooses).
+template <int TOK, int MINB, int U>
 __global__ void __launch_bounds__(256, MINB) router_logits_kernel(const __nv_bfloat16* x, const float* wg, const float* bias,
                                                                   float* __restrict__ logits, int T, int D, int E,
                                                                   int* __restrict__ zero, int n_zero) {
+  constexpr int EB = 8, PARTS = 4, V = TOK * EB;   // V sums per warp, a power of two and at most one per lane
+  __shared__ float s_sum[8][V];
   np::pdl_begin();
   // what the kernel behind this one adds to (a fill of its own is a launch)
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int t0 = warp * TOK; t0 < T; t0 += nwarps * TOK) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = warp % PARTS;
+  for (int tb = blockIdx.x * 2 * TOK; tb < T; tb += gridDim.x * 2 * TOK) {
+    const int t0 = tb + warp / PARTS * TOK;
     for (int e0 = 0; e0 < E; e0 += EB) {
-      float acc[TOK][EB];
+      float acc[V];
 #pragma unroll
-      for (int k = 0; k < TOK; ++k)
+      for (int i = 0; i < V; ++i) acc[i] = 0.f;
+#pragma unroll U
+      for (int d = (part * 32 + lane) * 8; d < D; d += PARTS * 256) {
+        float xv[TOK][8];
 #pragma unroll
-        for (int e = 0; e < EB; ++e) acc[k][e] = 0.f;
-      for (int d0 = lane * 8; d0 < D; d0 += 256 * V) {
-        uint4 q[V][TOK];
+        for (int k = 0; k < TOK; ++k) {
+          if (t0 + k < T) {
+            load8(x + (size_t)(t0 + k) * D + d, xv[k]);
+          } else {
 #pragma unroll
-        for (int h = 0; h < V; ++h)
-#pragma unroll
-          for (int k = 0; k < TOK; ++k)
-            q[h][k] = t0 + k < T && d0 + h * 256 < D ? *reinterpret_cast<const uint4*>(x + (size_t)(t0 + k) * D + d0 + h * 256)
-                                                     : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int h = 0; h < V; ++h) {
-          const int d = d0 + h * 256;
-          if (h > 0 && d >= D) break;
-          float xv[TOK][8];
-#pragma unroll
-          for (int k = 0; k < TOK; ++k) {
-            const float2 a = np::unpack_bf16(q[h][k].x), b = np::unpack_bf16(q[h][k].y), c = np::unpack_bf16(q[h][k].z),
-                         dd = np::unpack_bf16(q[h][k].w);
-            xv[k][0] = a.x; xv[k][1] = a.y; xv[k][2] = b.x; xv[k][3] = b.y;
-            xv[k][4] = c.x; xv[k][5] = c.y; xv[k][6] = dd.x; xv[k][7] = dd.y;
-          }
-#pragma unroll
-          for (int e = 0; e < EB; ++e) {
-            if (e0 + e < E) {
-              const float* wp = wg + (size_t)(e0 + e) * D + d;
-              const float4 w0 = *reinterpret_cast<const float4*>(wp);
-              const float4 w1 = *reinterpret_cast<const float4*>(wp + 4);
-#pragma unroll
-              for (int k = 0; k < TOK; ++k)
-                acc[k][e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
-                             xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
-            }
+            for (int j = 0; j < 8; ++j) xv[k][j] = 0.f;
           }
         }
-      }
-#pragma unroll
-      for (int k = 0; k < TOK; ++k) {
 #pragma unroll
         for (int e = 0; e < EB; ++e) {
-          const float sm = np::warp_sum(acc[k][e]);
-          if (lane == 0 && e0 + e < E && t0 + k < T) logits[(size_t)(t0 + k) * E + e0 + e] = sm + (bias ? bias[e0 + e] : 0.f);
+          if (e0 + e < E) {
+            const float* wp = wg + (size_t)(e0 + e) * D + d;
+            const float4 w0 = *reinterpret_cast<const float4*>(wp);
+            const float4 w1 = *reinterpret_cast<const float4*>(wp + 4);
+#pragma unroll
+            for (int k = 0; k < TOK; ++k)
+              acc[k * EB + e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
+                                 xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
+          }
         }
       }
+      // sums over the lanes: each step hands half of the sums to the partner, until a lane has one of them
+      int left = V;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        if (left > 1) {
+          left /= 2;
+#pragma unroll
+          for (int i = 0; i < V / 2; ++i) {
+            if (i >= left) break;
+            const float mine = lane & o ? acc[i + left] : acc[i], theirs = lane & o ? acc[i] : acc[i + left];
+            acc[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+          }
+        } else {
+          acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        }
+      }
+      if (lane % (32 / V) == 0) s_sum[warp][lane / (32 / V)] = acc[0];
+      __syncthreads();
+      if (part == 0 && lane < V) {
+        const int t = t0 + lane / EB, e = e0 + lane % EB;
+        const float sm = (s_sum[warp][lane] + s_sum[warp + 1][lane]) + (s_sum[warp + 2][lane] + s_sum[warp + 3][lane]);
+        if (t < T && e < E) logits[(size_t)t * E + e] = sm + (bias ? bias[e] : 0.f);
+      }
+      __syncthreads();
     }
   }
 }
@@ -470,132 +479,145 @@ __global__ void colsum2_kernel(const float* partial, float* __restrict__ out0, f
 }
 
 // ------------------------------------------------------------------ capacity / positions
-// One CTA of 1024 threads; thread i owns a contiguous run of tokens, so a block-wide exclusive scan of
-// per-thread pick counts gives positions in token order. The counters of a group of experts are packed into up to
-// four 64-bit words (16-bit fields while T < 65536, else 32-bit) and scanned together. Phase 0 ranks every pick
-// among all tokens that picked the expert and clears keep[t] when any pick of t lies at or beyond `capacity`
-// (capacity < 0: keep all); phase 1 ranks among the kept tokens.
+// One CTA of 32 warps, each over a contiguous run of slots (t, k), 32 at a time, a lane per slot. One ballot per bit of the expert
+// number gives a lane the slots that picked the same expert as its own (its rank among them), and lane e those of expert e (and
+// e + 32), so that the counters of up to 64 experts stand in two registers of a warp; more experts take further passes. Two passes
+// over the slots with the warps' counts exchanged in between give the positions in token order. Phase 0 ranks every pick among all
+// tokens that picked the expert and clears the flag of a token any of whose picks lies at or beyond `capacity` (capacity < 0: keep
+// all); phase 1 ranks among the kept tokens. Up to 8192 slots stay in registers, more are read again (from L1). Bound by its chain
+// of barriers and shuffles, one SM. A thread per run of tokens that
+// scanned packed counters, us, before / now: 512 tokens, 8 experts, top 2 7.5 / 4.9, 4096 18.5 / 10.5, 16384, 64, top 6 977 / 246.
 // Outputs: slot_pos[t,k] (position among kept for expert idx[t,k], -1 if dropped), keep[T],
 // counts_kept[E], drops[E] (tokens beyond capacity per expert), n_dropped[1].
-struct U64x4 {
-  unsigned long long w[4];
-  // word q, by selection: indexed with a variable, the counters of a thread would live in local memory
-  __device__ __forceinline__ unsigned long long get(int q) const {
-    return q == 0 ? w[0] : q == 1 ? w[1] : q == 2 ? w[2] : w[3];
-  }
-  __device__ __forceinline__ void add(int q, unsigned long long v) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] += q == i ? v : 0ull;
-  }
-};
-__device__ __forceinline__ U64x4 block_excl_scan4(const U64x4& v, int nw_used, U64x4* s_warp, U64x4* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  U64x4 inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q < nw_used) {
-        const unsigned long long n = __shfl_up_sync(0xffffffffu, inc.w[q], o);
-        if (lane >= o) inc.w[q] += n;
-      }
-    }
-  }
-  if (lane == 31) s_warp[warp] = inc;
-  __syncthreads();
-  if (warp == 0) {
-    U64x4 wv = lane < nwarps ? s_warp[lane] : U64x4{{0ull, 0ull, 0ull, 0ull}};
-    U64x4 winc = wv;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (q < nw_used) {
-          const unsigned long long n = __shfl_up_sync(0xffffffffu, winc.w[q], o);
-          if (lane >= o) winc.w[q] += n;
-        }
-      }
-    }
-    U64x4 ex;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ex.w[q] = winc.w[q] - wv.w[q];
-    s_warp[lane] = ex;                 // exclusive offset of each warp
-    if (lane == 31) s_warp[32] = winc;  // grand total
-  }
-  __syncthreads();
-  U64x4 res;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) res.w[q] = s_warp[warp].w[q] + inc.w[q] - v.w[q];
-  *total = s_warp[32];
-  __syncthreads();                     // s_warp is reused by the next scan
-  return res;
-}
-
-template <int FB>   // bits per counter: 16 or 32
-__global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* indices, int T, int E, int K,
-                                                             int capacity, int* __restrict__ slot_pos,
-                                                             int* __restrict__ keep, int* __restrict__ counts_kept,
+constexpr int PLAN_CHUNKS = 8;     // runs of 32 slots that a warp holds at once
+template <int EP>                  // experts per pass, 32 or 64
+__global__ void __launch_bounds__(1024) capacity_plan_kernel(const int* indices, int T, int E, int K, int capacity,
+                                                             int* __restrict__ slot_pos, int* keep, int* counts_kept,
                                                              int* __restrict__ drops, int* __restrict__ n_dropped,
-                                                             int use_smem, int* __restrict__ sent, int n_ranks,
+                                                             int smem_flags, int* __restrict__ sent, int n_ranks,
                                                              long long* __restrict__ stats) {
   np::pdl_begin();
-  constexpr int EPW = 64 / FB;          // experts per 64-bit word
-  constexpr int GROUP = 4 * EPW;        // experts per pass
-  constexpr unsigned long long FMASK = (FB == 16) ? 0xffffull : 0xffffffffull;
-  extern __shared__ int s_dyn[];        // routing table staged once, then one keep byte per token
-  __shared__ U64x4 s_warp[33];
-  int* s_idx = s_dyn;
-  unsigned char* s_keep = reinterpret_cast<unsigned char*>(s_dyn + (use_smem ? T * K : 0));
-  const int* idx = indices;
-  if (use_smem) {
-#pragma unroll 4
-    for (int i = threadIdx.x; i < T * K; i += blockDim.x) s_idx[i] = indices[i];   // several loads in flight
-    for (int t = threadIdx.x; t < T; t += blockDim.x) s_keep[t] = 1;
-    idx = s_idx;
-  } else {
-    for (int t = threadIdx.x; t < T; t += blockDim.x) keep[t] = 1;
+  extern __shared__ unsigned char s_keep[];   // a byte per token where they fit, else `keep` itself
+  __shared__ int s_count[32][EP + 1], s_total[EP];
+  __shared__ int s_dropped;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const long long n = (long long)T * K;
+  const int chunks = (int)((n + 1023) / 1024);   // of a warp
+  const bool held = chunks <= PLAN_CHUNKS;
+  const long long s0 = (long long)warp * chunks * 32;
+  const int t0 = (int)(s0 / K);                  // token and pick of the warp's first slot
+  const unsigned k0 = (unsigned)(s0 % K);
+  const int shift = K & (K - 1) ? -1 : __ffs(K) - 1;
+  int ex[PLAN_CHUNKS], pos[PLAN_CHUNKS];
+  auto slot = [&](int c) { return s0 + c * 32 + lane; };
+  auto token = [&](int c) {
+    const unsigned i = k0 + c * 32u + lane;
+    return t0 + (int)(shift >= 0 ? i >> shift : i / (unsigned)K);
+  };
+  auto load = [&](int c0) {
+#pragma unroll
+    for (int u = 0; u < PLAN_CHUNKS; ++u) ex[u] = c0 + u < chunks && slot(c0 + u) < n ? indices[slot(c0 + u)] : -1;
+  };
+  auto is_kept = [&](int t) { return smem_flags ? s_keep[t] != 0 : keep[t] != 0; };
+  load(0);
+  if (threadIdx.x == 0) s_dropped = 0;
+  for (int t = threadIdx.x; t < T; t += 1024) {
+    if (smem_flags) s_keep[t] = 1;
+    else keep[t] = 1;
   }
   __syncthreads();
-  const int per = (T + blockDim.x - 1) / blockDim.x;
-  const int t_lo = min(T, (int)threadIdx.x * per), t_hi = min(T, t_lo + per);
-  for (int phase = (capacity < 0 ? 1 : 0); phase < 2; ++phase) {
-    for (int e0 = 0; e0 < E; e0 += GROUP) {
-      const int n_e = min(GROUP, E - e0);
-      const int nw_used = (n_e + EPW - 1) / EPW;
-      U64x4 loc{{0ull, 0ull, 0ull, 0ull}};
-      for (int t = t_lo; t < t_hi; ++t) {
-        if (phase == 1 && !(use_smem ? s_keep[t] : keep[t])) continue;
-        for (int k = 0; k < K; ++k) {
-          const int e = idx[(size_t)t * K + k] - e0;
-          if (e >= 0 && e < n_e) loc.add(e / EPW, 1ull << (FB * (e % EPW)));
+  for (int phase = capacity < 0 ? 1 : 0; phase < 2; ++phase) {
+    for (int e0 = 0; e0 < E; e0 += EP) {
+      const int n_e = min(EP, E - e0), bits = n_e > 1 ? 32 - __clz(n_e - 1) : 0;
+      int run_lo = 0, run_hi = 0;   // lane e: picks of experts e and e + 32 by the slots so far
+      unsigned valid = 0;           // a bit per chunk: a pick of an expert of this pass by a kept token
+      // counts the picks of a chunk; the position of this lane's slot among those of its expert, given those before it
+      auto visit = [&](int u, int c, bool rank) {
+        const int e = ex[u] - e0;
+        const bool ok = e >= 0 && e < n_e && (phase == 0 || is_kept(token(c)));
+        unsigned same = __ballot_sync(0xffffffffu, ok), lo = same, hi = 0;
+        if (ok) valid |= 1u << u;
+#pragma unroll
+        for (int b = 0; b < 5; ++b) {
+          if (b < bits) {
+            const unsigned bit = (e >> b) & 1, v = __ballot_sync(0xffffffffu, bit);
+            same &= v ^ (bit - 1u);
+            lo &= v ^ (((lane >> b) & 1u) - 1u);
+          }
+        }
+        int before = rank ? __shfl_sync(0xffffffffu, run_lo, e & 31) : 0;
+        if (EP > 32 && bits == 6) {
+          const unsigned bit = (e >> 5) & 1, v = __ballot_sync(0xffffffffu, bit);
+          same &= v ^ (bit - 1u);
+          hi = lo & v;
+          lo &= ~v;
+          const int h = rank ? __shfl_sync(0xffffffffu, run_hi, e & 31) : 0;
+          if (bit) before = h;
+          run_hi += __popc(hi);
+        }
+        run_lo += __popc(lo);
+        return before + __popc(same & below);
+      };
+      for (int c0 = 0; c0 < chunks; c0 += PLAN_CHUNKS) {
+        if (!held) load(c0);
+#pragma unroll
+        for (int u = 0; u < PLAN_CHUNKS; ++u) {
+          if (c0 + u >= chunks) continue;
+          if (held) pos[u] = visit(u, c0 + u, true);
+          else visit(u, c0 + u, false);
         }
       }
-      U64x4 total;
-      U64x4 run = block_excl_scan4(loc, nw_used, s_warp, &total);
-      for (int t = t_lo; t < t_hi; ++t) {
-        const bool kept = phase == 0 || (use_smem ? s_keep[t] : keep[t]);
-        for (int k = 0; k < K; ++k) {
-          const int e = idx[(size_t)t * K + k] - e0;
-          if (e < 0 || e >= n_e) continue;
-          if (!kept) {
-            slot_pos[(size_t)t * K + k] = -1;
-            continue;
-          }
-          const int q = e / EPW, sh = FB * (e % EPW);
-          const int pos = (int)((run.get(q) >> sh) & FMASK);
-          run.add(q, 1ull << sh);
-          if (phase == 0) {
-            if (pos >= capacity) {   // only ever written to 0, by the thread that owns the token
-              if (use_smem) s_keep[t] = 0; else keep[t] = 0;
+      s_count[warp][lane] = run_lo;
+      if (EP > 32) s_count[warp][lane + 32] = run_hi;
+      __syncthreads();
+      for (int e = warp; e < n_e; e += 32) {   // the warps before each one, per expert
+        const int x = s_count[lane][e];
+        int sum = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += y;
+        }
+        s_count[lane][e] = sum - x;
+        if (lane == 31) s_total[e] = sum;
+      }
+      __syncthreads();
+      run_lo = s_count[warp][lane];
+      if (EP > 32) run_hi = s_count[warp][lane + 32];
+      for (int c0 = 0; c0 < chunks; c0 += PLAN_CHUNKS) {
+        if (!held) {
+          valid = 0;
+          load(c0);
+        }
+#pragma unroll
+        for (int u = 0; u < PLAN_CHUNKS; ++u) {
+          if (c0 + u >= chunks) continue;
+          const int e = ex[u] - e0;
+          int at;
+          if (held) {
+            at = __shfl_sync(0xffffffffu, run_lo, e & 31);
+            if (EP > 32) {
+              const int h = __shfl_sync(0xffffffffu, run_hi, e & 31);
+              if (e >= 32) at = h;
             }
+            at += pos[u];
           } else {
-            slot_pos[(size_t)t * K + k] = pos;
+            at = visit(u, c0 + u, true);
+          }
+          const bool ok = (valid >> u) & 1u;
+          if (phase == 0) {
+            if (ok && at >= capacity) {   // only ever written to 0
+              if (smem_flags) s_keep[token(c0 + u)] = 0;
+              else keep[token(c0 + u)] = 0;
+            }
+          } else if (e >= 0 && e < n_e) {
+            slot_pos[slot(c0 + u)] = ok ? at : -1;
           }
         }
       }
       if ((int)threadIdx.x < n_e) {
-        const int e = threadIdx.x;
-        const int c = (int)((total.get(e / EPW) >> (FB * (e % EPW))) & FMASK);
+        const int e = threadIdx.x, c = s_total[e];
         if (phase == 0) {
           drops[e0 + e] = c > capacity ? c - capacity : 0;
         } else {
@@ -604,30 +626,31 @@ __global__ void __launch_bounds__(1024) capacity_scan_kernel(const int* indices,
         }
       }
     }
-    __syncthreads();   // keep flags of phase 0 are complete before phase 1 reads them
+    __syncthreads();   // the flags of phase 0 are complete before phase 1 reads them; counts_kept before `sent` is formed
   }
   int nd = 0;
-  for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    const int kp = use_smem ? (int)s_keep[t] : keep[t];
-    if (use_smem) keep[t] = kp;
-    nd += kp ? 0 : 1;
+  for (int t = threadIdx.x; t < T; t += 1024) {
+    const bool k = is_kept(t);
+    if (smem_flags) keep[t] = k;
+    nd += !k;
   }
-  U64x4 ndv{{(unsigned long long)nd, 0ull, 0ull, 0ull}}, total;
-  block_excl_scan4(ndv, 1, s_warp, &total);
+  nd = __reduce_add_sync(0xffffffffu, nd);
+  if (lane == 0 && nd) atomicAdd(&s_dropped, nd);
+  __syncthreads();
   if (threadIdx.x == 0) {
-    n_dropped[0] = (int)total.w[0];
+    n_dropped[0] = s_dropped;
     if (stats) {   // last step's drops, all drops, all tokens
-      stats[0] = (long long)total.w[0];
-      stats[1] += (long long)total.w[0];
+      stats[0] = s_dropped;
+      stats[1] += s_dropped;
       stats[2] += T;
     }
   }
-  if (sent) {      // kept rows per expert-parallel rank (counts_kept was written before the barriers of the scan above)
+  if (sent) {      // kept rows per expert-parallel rank
     const int per_rank = E / n_ranks;
-    for (int r = threadIdx.x; r < n_ranks; r += blockDim.x) {
-      int n = 0;
-      for (int e = r * per_rank; e < (r + 1) * per_rank; ++e) n += counts_kept[e];
-      sent[r] = n;
+    for (int r = threadIdx.x; r < n_ranks; r += 1024) {
+      int rows = 0;
+      for (int e = r * per_rank; e < (r + 1) * per_rank; ++e) rows += counts_kept[e];
+      sent[r] = rows;
     }
   }
 }
@@ -937,15 +960,15 @@ __global__ void __launch_bounds__(256) slot_dot_kernel(const __nv_bfloat16* a,
 NP_API int np_router_logits(const void* x, const float* wg, const float* bias, float* logits, int T, int D, int E, int* zero,
                             int n_zero, void* stream) {
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
-  // Gate rows in L2 / in DRAM, us, one token with its gate vectors in registers as they come (127 registers, two CTAs per SM) -
-  // one token, two vectors, four CTAs per SM - four tokens (128 registers): 1024 x 2048, 8 experts 7.8 / 12.6 - 11.8 / 22.7 -
-  // 20.9 / 40.6; 3000 x 1024 12.7 / 14.3 - 10.0 / 14.8 - 13.0 / 23.1; 4096 x 2048 22.0 / 24.5 - 21.6 / 27.0 - 21.7 / 42.1;
-  // 8192 x 2048 41.2 / 44.6 - 41.6 / 47.6 - 22.2 / 44.1. The first as long as it is one wave of CTAs.
-  const bool one_wave = T <= 148 * 2 * 8, many = T >= 8192;
-  const long long warps = many ? ((long long)T + 3) / 4 : T, blocks = (warps * 32 + 255) / 256;
-  np_launch(one_wave ? router_logits_kernel<8, 1, 1, 1> : many ? router_logits_kernel<8, 4, 1, 2> : router_logits_kernel<8, 1, 2, 4>,
-            (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
-            logits, T, D, E, zero, n_zero);
+  auto run = [&](auto kernel, int tok) {
+    const int blocks = (T + 2 * tok - 1) / (2 * tok);
+    np_launch(kernel, (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg,
+              bias, logits, T, D, E, zero, n_zero);
+  };
+  // Two tokens per four warps with the vectors of two steps in flight as long as that is one wave of CTAs, then four, which read the
+  // gate rows half as often. us, two / four: 64 x 2048 3.9 / 5.6, 1024 4.6 / 6.1, 2048 8.5 / 6.1, 4096 15.0 / 11.6, 16384 46.8 / 30.4.
+  if (T <= 148 * 2 * 4) run(router_logits_kernel<2, 2, 2>, 2);
+  else run(router_logits_kernel<4, 2, 1>, 4);
   CHECK_LAUNCH();
 }
 
@@ -1025,23 +1048,18 @@ NP_API int np_capacity_plan(const int* indices, int T, int E, int K, int capacit
                             int* drops, int* n_dropped, int* sent, int n_ranks, long long* stats, void* stream) {
   if (K > MAX_K || (sent && (n_ranks <= 0 || E % n_ranks))) return 1;
   if (T <= 0) return 0;
-  const size_t smem = (size_t)T * K * 4 + (size_t)((T + 3) / 4) * 4;
-  const int use_smem = smem <= 200 * 1024;
+  const int flags_fit = T <= 200 * 1024;   // a byte per token beside the counts of the warps
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
-  if (use_smem && !attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(capacity_scan_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  if (flags_fit && !attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(capacity_plan_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(capacity_scan_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      e = cudaFuncSetAttribute(capacity_plan_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
   }
-  if (T < 65536)   // a 16-bit counter holds any per-expert count
-    np_launch(capacity_scan_kernel<16>, 1, 1024, use_smem ? smem : 0, (cudaStream_t)stream, 1,
-        indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem, sent, n_ranks, stats);
-  else
-    np_launch(capacity_scan_kernel<32>, 1, 1024, use_smem ? smem : 0, (cudaStream_t)stream, 1,
-        indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, use_smem, sent, n_ranks, stats);
+  np_launch(E <= 32 ? capacity_plan_kernel<32> : capacity_plan_kernel<64>, 1, 1024, flags_fit ? (size_t)T : 0, (cudaStream_t)stream,
+            1, indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, flags_fit, sent, n_ranks, stats);
   CHECK_LAUNCH();
 }
 

@@ -253,6 +253,42 @@ def test_capacity_plan(T, cap, ranks):
     assert stats.tolist() == [d, 100 + d, 1000 + T]
 
 
+# one, two and more passes over the experts, picks per token that straddle the warps' runs, runs that stay in registers and longer ones
+@pytest.mark.parametrize("T,E,K,cap", [(1, 1, 1, -1), (11, 2, 1, 3), (33, 31, 5, 4), (341, 32, 3, 40), (2731, 33, 3, 250),
+                                       (1024, 64, 8, 128), (1025, 64, 8, 120), (1366, 65, 6, 100), (600, 130, 7, 30), (210000, 5, 1, 50000)])
+def test_capacity_plan_of_many_experts(T, E, K, cap):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(T)
+    idx = torch.rand(T, E, device="cuda").topk(K, -1).indices.to(torch.int32)
+    got = [torch.full(s, -7, device="cuda", dtype=torch.int32) for s in ((T, K), (T,), (E,), (E,), (1,))]
+    _lib.call("capacity_plan", idx, T, E, K, cap, *got, None, 0, None)
+    for g, w in zip(got, _plan(idx.cpu(), E, cap)):
+        assert torch.equal(g.cpu().long().reshape(w.shape), w.long())
+
+
+# widths that are no whole number of steps, more experts than a pass takes, both numbers of tokens per group at their edges
+@pytest.mark.parametrize("T,D,E", [(1, 8, 1), (5, 264, 8), (9, 1032, 9), (1183, 768, 7), (1184, 768, 8), (1185, 768, 8), (1190, 2056, 17),
+                                   (10000, 128, 64)])
+def test_router_logits(T, D, E):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(T)
+    x, w = torch.randn(T, D, device="cuda").bfloat16(), torch.randn(E, D, device="cuda")
+    bias, zero = torch.randn(E, device="cuda"), torch.ones(2 * E + 1, device="cuda", dtype=torch.int32)
+    got = torch.full((T, E), float("nan"), device="cuda")
+    _lib.call("router_logits", x, w, bias, got, T, D, E, zero, 2 * E)
+    want = x.double() @ w.double().t() + bias.double()
+    # fp32: each of the D products meets at most 8 additions a step, 5 + 2 over lanes and warps
+    bound = (x.double().abs() @ w.double().abs().t() + bias.double().abs()) * (8 * -(-D // 1024) + 8) * 2 ** -24
+    assert ((got.double() - want).abs() <= bound).all()
+    assert zero[:-1].eq(0).all() and zero[-1] == 1
+    # a token's sum does not depend on how many come with it
+    few = torch.empty(min(T, 3), E, device="cuda")
+    _lib.call("router_logits", x[-3:].contiguous(), w, bias, few, few.shape[0], D, E, None, 0)
+    assert torch.equal(few, got[-3:])
+
+
 # the ends of the exponent: sigmoid at subnormal numbers, at zero, one and infinity; each of the two reciprocal forms
 def test_swiglu_at_the_ends_of_the_range():
     from nanopysche_b200.ops.activation import glu
