@@ -253,6 +253,30 @@ def test_capacity_plan(T, cap, ranks):
     assert stats.tolist() == [d, 100 + d, 1000 + T]
 
 
+# single elements, vectors and tiles with remainders, more tiles than CTAs
+@pytest.mark.parametrize("n", [1, 3, 4, 1023, 1028, 8191, 8192 * 592 + 8197])
+@pytest.mark.parametrize("copy16", [True, False])
+def test_adamw_and_square_sum(n, copy16):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(n)
+    p, g, m = (torch.randn(n, device="cuda") for _ in range(3))
+    v, w16 = torch.rand(n, device="cuda"), torch.zeros(n, device="cuda", dtype=torch.bfloat16)
+    part = torch.full((_lib.lib().np_sumsq_parts(),), float("nan"), device="cuda")
+    coef, lr, b1, b2, eps, wd, step = torch.tensor([0.5], device="cuda"), 1e-2, 0.9, 0.95, 1e-8, 0.1, 3
+    P, G, M, V = p.double(), g.double() * 0.5, m.double(), v.double()
+    _lib.call("sumsq", g, _lib.LL(n), part)
+    _lib.call("adamw", p, g, m, v, w16 if copy16 else None, _lib.LL(n), lr, b1, b2, eps, wd, step, coef, None)
+    # every square rounded once, then at most 32 additions per tile of a CTA and 13 over threads
+    torch.testing.assert_close(part.double().sum(), g.double().square().sum(), rtol=(32 * (n // (8192 * 592) + 2) + 16) * 2 ** -24, atol=0)
+    M, V = b1 * M + (1 - b1) * G, b2 * V + (1 - b2) * G * G
+    P = P * (1 - lr * wd) - lr * (M / (1 - b1 ** step)) / ((V / (1 - b2 ** step)).sqrt() + eps)
+    tol = dict(rtol=2 ** -20, atol=2 ** -20)      # some ten fp32 roundings of numbers of the size of one; 1 - b2^3 to 2^-21
+    for got, want in ((p, P), (m, M), (v, V)):
+        torch.testing.assert_close(got.double(), want, **tol)
+    assert torch.equal(w16, p.bfloat16() if copy16 else torch.zeros_like(w16))
+
+
 # one, two and more passes over the experts, picks per token that straddle the warps' runs, runs that stay in registers and longer ones
 @pytest.mark.parametrize("T,E,K,cap", [(1, 1, 1, -1), (11, 2, 1, 3), (33, 31, 5, 4), (341, 32, 3, 40), (2731, 33, 3, 250),
                                        (1024, 64, 8, 128), (1025, 64, 8, 120), (1366, 65, 6, 100), (600, 130, 7, 30), (210000, 5, 1, 50000)])
