@@ -131,7 +131,7 @@ class GraphedTrainStep:
                 self._eager(False)
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
-        self.opt.update_hyper(advance=False)   # recording takes no step: the first replay is the next one
+        self.opt.update_hyper()
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self.static_loss = self._eager(True)
