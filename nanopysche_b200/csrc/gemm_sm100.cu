@@ -53,6 +53,7 @@ struct GemmParams {
   const int* done_expected;   // [flags] M blocks expected per destination (x n_blocks tiles each)
   int* const* done_flag_ptr;  // [flags] peer flag word to release when a destination completes
   bool local_push;            // every destination is this GPU's own memory
+  int parts;                  // pair kernel: K in this many parts with an accumulator each, added in the epilogue
   const void* Cin;            // accumulate source (same dtype as C), rows indexed like a dense C
   long long ldcin;
   const int* epoch_base;      // optional device counter added to `epoch` (keeps epochs valid under graph replay)
@@ -411,23 +412,42 @@ __device__ __forceinline__ void stage_drain(int lane) {
   if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// 32 accumulator columns of this lane's row (zeros without an accumulator)
-__device__ __forceinline__ void load_acc(uint32_t taddr, bool have_acc, uint32_t* r) {
-  if (have_acc) {
-    np::tmem_ld32(taddr, r);
+// A tile's accumulator: tensor memory of this warp's lanes, first column. K in parts: PER_BUFFER of them side by side at `t`, the rest
+// likewise at `t2`.
+template <int BN>
+constexpr int PER_BUFFER = BN == 128 ? 2 : 1;
+template <int BN>
+struct Acc {
+  uint32_t t, t2;
+  int parts;   // 0: no K steps, zeros
+};
+// 32 accumulator columns of this lane's row, the parts added in their order
+template <int BN>
+__device__ __forceinline__ void load_acc(const Acc<BN>& acc, int col, uint32_t* r) {
+  if (acc.parts > 0) {
+    np::tmem_ld32(acc.t + col, r);
     np::tmem_ld_wait();
+#pragma unroll 1
+    for (int q = 1; q < acc.parts; ++q) {
+      uint32_t v[32];
+      np::tmem_ld32((q / PER_BUFFER<BN> ? acc.t2 : acc.t) + q % PER_BUFFER<BN> * BN + col, v);
+      np::tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(v[i]));
+    }
   } else {
 #pragma unroll
     for (int i = 0; i < 32; ++i) r[i] = 0u;
   }
 }
 
-// Half `half` of the BN accumulator columns of one 128-row tile: tensor memory (`taddr`: this warp's lanes, first column)
+// Half `half` of the BN accumulator columns of one 128-row tile: tensor memory
 // through the epilogue of the launch to output rows row0 .. row0 + 31, columns from `n0`. Executed by whole warps (the
 // tensor-memory loads are .sync.aligned).
 template <int BN>
 __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmC2, uint32_t stg,
-                                           uint32_t taddr, int g_idx, int row0, int lane, int n0, int half, bool have_acc) {
+                                           const Acc<BN>& acc, int g_idx, int row0, int lane, int n0, int half) {
+  const uint32_t taddr = acc.t;
   if (p.tma_c) {
     if (row0 >= p.M) return;
     if (p.m_split && row0 >= p.m_split) {
@@ -469,7 +489,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
         const int col = n0 + c * 32;
         if (col >= p.N) break;
         uint32_t r[32];
-        load_acc(taddr + c * 32, have_acc, r);
+        load_acc(acc, c * 32, r);
         scale_bias(p, r, col);
         stage_store(tmC, stg, lane, r, col, row0, g_idx);
       }
@@ -482,7 +502,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           uint32_t r[32];
-          load_acc(taddr + c * 64 + q * 32, have_acc, r);
+          load_acc(acc, c * 64 + q * 32, r);
           scale_bias(p, r, col + q * 32);
           pack32(r, w + 16 * q);
         }
@@ -509,7 +529,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
     for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
       uint32_t r[32];
       __syncwarp();
-      load_acc(taddr + c * 32, have_acc, r);
+      load_acc(acc, c * 32, r);
       store_chunk(p, o, r, n0 + c * 32);
     }
   }
@@ -756,7 +776,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
       const int row0 = tl.m_blk * BM + quarter * 32;
       if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
-      else store_tile<BN>(p, &tmC, &tmC2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
+      else store_tile<BN>(p, &tmC, &tmC2, stg, Acc<BN>{taddr, 0u, have_acc ? 1 : 0}, tl.g, row0, lane, n0, half);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
@@ -852,6 +872,12 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 // workspace, no atomics, and the same result every time. It is for outputs with too few tiles to occupy the SMs: the time
 // of such a GEMM is its K steps one after the other (about 0.3 us each), not its FLOPs.
 //
+// p.parts: one pair forms the same parts in turn, each in accumulator columns of its own (128-column tiles: two parts in each of the
+// two buffers; wider ones: one), and the epilogue adds them in their order, so that the result has the bits of the cluster's. It
+// takes a tile as long as a whole sum and a little more: us, whole / two parts / four / cluster of two / of four, 2048 x 1024 x 3072
+// 17.4 / 17.6 / 17.9 / 17.5 / 42.8, 1024 x 768 x 2048 11.9 / 12.1 / 12.5 / 14.6 / 14.0, 768 x 768 x 4096 20.2 / 20.3 / 20.5 / 19.3 / 16.5;
+// 192 columns 18.5 and 256 20.8 with two parts in the first, where no products cover their drain.
+//
 // DUAL: two products in one launch. A backward pass asks for the gradients of a layer's input and of its weight at the same
 // time; alone, each leaves SMs without work in its only or last wave and pays for a launch, first loads and a last drain of its
 // own. A pair takes its tiles of the product with the longer contraction first, then those of the other. us, two launches /
@@ -895,8 +921,7 @@ template <bool SPLIT, int BN, bool DUAL>
 __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams& p, const PairSecond* second) {
   constexpr int STAGES = pair_stages<BN>(), TM = 2 * BM, HN = BN / 2;
   constexpr int A_BYTES = BM * BK * 2, STAGE_BYTES = pair_stage_bytes<BN>();
-  constexpr uint32_t TMEM_COLS = 2 * BN <= 256 ? 256 : 512;
-  static_assert(!SPLIT || BN == 256, "K in parts: 256 columns");
+  static_assert(!SPLIT || BN == 256, "K in parts over a cluster: 256 columns");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (np::smem_u32(smem_raw) + 1023u) & ~1023u;   // the same offset in both CTAs
   const uint32_t stg_base = smem_base + STAGES * STAGE_BYTES;   // staging of the epilogue warps
@@ -919,6 +944,10 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
   auto n_blocks = [&](const GemmParams& q) { return (q.N + bn_out - 1) / bn_out; };
   auto num_tiles = [&](const GemmParams& q) { return m_blocks(q) * n_blocks(q) * ((q.mode == 2) ? q.num_groups : 1); };
   const int tiles0 = num_tiles(p), tiles1 = DUAL ? num_tiles(second->p) : 0;
+  // parts that this pair sums one after the other, and columns of one of the two accumulator buffers
+  auto k_parts = [](const GemmParams& q) { return SPLIT ? 1 : q.parts; };
+  const int acc_cols = k_parts(p) > 1 || (DUAL && k_parts(second->p) > 1) ? PER_BUFFER<BN> * BN : BN;
+  const uint32_t tmem_cols = 2 * acc_cols <= 256 ? 256 : 512;
   auto work = [&](int k) -> PairWork {
     if constexpr (DUAL) return pair_work(k, pair, pairs, tiles0, tiles1, second->extra);
     const int t = pair + k * pairs;
@@ -965,7 +994,7 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     np::smem_u32((const void*)tmem_ptr_smem)), "r"(TMEM_COLS) : "memory");
+                     np::smem_u32((const void*)tmem_ptr_smem)), "r"(tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   __syncwarp();
@@ -1070,9 +1099,26 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
         if (count_k(q, tl.g) == 0) continue;
         if (!np::mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 12)) break;
         np::tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+        uint32_t tmem_d = tmem_base + (uint32_t)(acc * acc_cols);
         uint32_t accum = 0;
-        k_steps(q, tl.g, [&](int) -> bool {
+        const int parts = k_parts(q), nkb = parts > 1 ? count_k(q, tl.g) : 0;
+        // 2 or 4 parts: the first K of the next one (a division per K step made the step half as long again)
+        auto part_end = [&](int part) { return (int)((long long)nkb * (part + 1) >> (parts >> 1)) * BK; };
+        int part = 0, next_k = parts > 1 ? part_end(0) : 0;
+        k_steps(q, tl.g, [&](int k0) -> bool {
+          if (parts > 1 && k0 == next_k) {   // the next part, in its own columns
+            accum = 0;
+            next_k = part_end(++part);
+            tmem_d += BN;
+            if (part == PER_BUFFER<BN>) {   // in the other buffer
+              if (np::elect_one()) tc_commit_pair(tfull_bar(acc), lead);
+              __syncwarp();
+              if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+              if (!np::mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, KID_GEMM, 17)) return false;
+              np::tc_fence_after();
+              tmem_d = tmem_base + (uint32_t)(acc * acc_cols);
+            }
+          }
           if (!np::mbar_wait_warp(full_bar(stage), phase, abort_flag, KID_GEMM, 13)) return false;
           np::tc_fence_after();
           if (np::elect_one()) {
@@ -1110,23 +1156,31 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
       if (rows == 0) continue;
       const bool have_acc = count_k(q, tl.g) > 0;
       const bool mine = (rows >> rank) & 1;   // this CTA's 128-row block carries data
+      const int parts = k_parts(q), buffers = parts > PER_BUFFER<BN> ? 2 : 1;
       if (have_acc) {
         if (!np::mbar_wait(tfull_bar(acc), acc_phase, abort_flag, KID_GEMM, 14)) break;
+        if (buffers == 2 && !np::mbar_wait(tfull_bar(acc ^ 1), acc_phase ^ (uint32_t)acc, abort_flag, KID_GEMM, 18)) break;
         np::tc_fence_after();
       }
       if constexpr (SPLIT) { done = true; break; }   // one tile per cluster, finished below
       if (mine) {
-        const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
+        const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16), taddr = lanes + (uint32_t)(acc * acc_cols);
         const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
         const int row0 = tl.m_blk * TM + rank * BM + quarter * 32, n0 = tl.n_blk * bn_out;
-        if (q.epilogue == 2) store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
-        else store_tile<BN>(q, &tm.C, &tm.C2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
+        if (q.epilogue == 2) {
+          store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+        } else {
+          store_tile<BN>(q, &tm.C, &tm.C2, stg, Acc<BN>{taddr, lanes + (uint32_t)((acc ^ 1) * acc_cols), have_acc ? parts : 0}, tl.g,
+                         row0, lane, n0, half);
+        }
       }
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(peer_addr(tempty_bar(acc), lead));
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        for (int b = 0; b < buffers; ++b) {
+          if (lane == 0) arrive_cluster(peer_addr(tempty_bar(acc), lead));
+          if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+        }
       }
       if (q.done_counters && mine) {   // done_expected counts 128-row blocks
         const int fi = q.mblk_flag ? q.mblk_flag[2 * tl.m_blk] : 0;
@@ -1197,7 +1251,7 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
   cluster_sync();        // nothing of the peer reads or arrives here any more
   if (warp == 1) {
     np::tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
   }
 }
 
@@ -1223,7 +1277,7 @@ int g_num_sms = 0;
 // / 4096: 8.9 / 22.6, 10.1 / 27.8, 10.3 / 24.7, 9.4 / 21.4, 8.9 / 19.1).
 struct TileCost { double fixed, step, drain; };
 constexpr TileCost COST_128{4.3, 0.28, 0.4}, COST_256{5.0, 0.35, 0.3}, COST_PAIR{5.6, 0.30, 0.3}, COST_PAIR_192{5.3, 0.25, 0.3},
-    COST_PAIR_128{5.2, 0.21, 0.3}, COST_SPLIT2{9.3, 0.30, 0.3}, COST_SPLIT4{10.0, 0.28, 0.3};
+    COST_PAIR_128{5.2, 0.21, 0.3}, COST_SPLIT2{9.9, 0.30, 0.3}, COST_SPLIT4{11.7, 0.28, 0.3};
 // Products of at most 64 rows. The few-row kernel: CTAs of 16 weight rows, each of which reads all of x again from the L2, so its
 // time per CTA grows with the rows it is built for (8, 16, 32, 64) and, by the loads in flight, with K. The tile kernels pad to
 // 128 rows but read x once per tile: with many columns they are bound by reading the weight. Fitted to 15 weights of 768 x 768 to
@@ -1243,6 +1297,12 @@ inline double few_tiles_cost(double tiles, int N, int K) {   // tiles: estimate 
 }
 // Clusters of four and of eight CTAs that run at once (an SM pair per two CTAs, whole clusters within a GPC)
 constexpr int CLUSTERS4 = 32, CLUSTERS8 = 14;
+// Where the sum over K is cut (sum_rule): the estimates of the kernels that there were when the cuts were laid down
+constexpr TileCost CUT_128{4.4, 0.37, 0.6}, CUT_256{5.3, 0.40, 0.3}, CUT_PAIR{6.0, 0.30, 0.3}, CUT_SPLIT2{9.3, 0.30, 0.3},
+    CUT_SPLIT4{10.7, 0.30, 0.3};
+// What the drain of a tile with K in parts takes beside that of a whole one: another read of the accumulator, and where the parts take
+// both accumulator buffers, the part of the drain that otherwise runs under the next tile's products
+inline double parts_drain(int parts, int bn) { return parts == 1 ? 0.0 : bn != 128 ? 1.5 : parts == 2 ? 0.2 : 0.8; }
 }  // namespace
 
 // ------------------------------------------------------------------ host side
@@ -1303,7 +1363,7 @@ static int make_tmap_out(CUtensorMap* out, const void* base, int f32, long long 
 
 // Tensor maps and kernel parameters of a launch with tiles of BN columns
 template <int BN, bool PAIR>
-static int prepare_gemm(const NpGemmArgs& a, int splits, PairMaps& m, CUtensorMap& tmAloc, CUtensorMap& tmBloc, GemmParams& p) {
+static int prepare_gemm(const NpGemmArgs& a, int splits, int parts, PairMaps& m, CUtensorMap& tmAloc, CUtensorMap& tmBloc, GemmParams& p) {
   CUtensorMap &tmA = m.A, &tmB = m.B, &tmB2 = m.B2, &tmC = m.C, &tmC2 = m.C2;
   int rc;
   if (!a.a_mn) rc = np_make_tmap_2d(&tmA, a.A, 2, (uint64_t)a.a_rows, (uint64_t)a.K, (uint64_t)a.lda, BK, BM);
@@ -1394,6 +1454,7 @@ static int prepare_gemm(const NpGemmArgs& a, int splits, PairMaps& m, CUtensorMa
     if (rc) return 800 + rc;
   }
   p.splits = splits;
+  p.parts = parts;
   return 0;
 }
 
@@ -1404,11 +1465,11 @@ constexpr int gemm_smem() {
 }
 
 template <int BN, bool PAIR>
-static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1) {
+static int launch_gemm(const NpGemmArgs& a, cudaStream_t stream, int splits = 1, int parts = 1) {
   PairMaps m;
   CUtensorMap tmAloc, tmBloc;
   GemmParams p;
-  const int rc = prepare_gemm<BN, PAIR>(a, splits, m, tmAloc, tmBloc, p);
+  const int rc = prepare_gemm<BN, PAIR>(a, splits, parts, m, tmAloc, tmBloc, p);
   if (rc) return rc;
   constexpr int SMEM = gemm_smem<BN, PAIR>(), STAGES = BN == 256 ? 4 : 6;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
@@ -1474,11 +1535,11 @@ static int check_gemm(const NpGemmArgs& a) {
   return 0;
 }
 
-// Which kernel a product runs on: the few-row kernel, one CTA per tile of `bn` columns, or pairs with tiles of `bn` columns and
-// K in `splits` parts
+// Which kernel a product runs on: the few-row kernel, one CTA per tile of `bn` columns, or pairs with tiles of `bn` columns. K in
+// `splits` parts over a cluster, or in `parts` that one pair sums in turn: the same sums, added in the same order.
 struct GemmChoice {
   bool few, pair;
-  int bn, splits;
+  int bn, splits, parts;
   double cost;   // estimate in us
 };
 // Tiles of tm x tn and K steps of a tile. Grouped forms by the room of their regions, as which rows arrive is not known here; an estimate
@@ -1489,51 +1550,100 @@ static long long tiles_of(const NpGemmArgs& a, int tm, int tn) {
 static double tile_steps(const NpGemmArgs& a) { return a.mode == 2 ? 2.0 * a.blocks_per_group : (a.K + BK - 1) / BK; }
 static double operations(const NpGemmArgs& a) { return tiles_of(a, BM, BM) * 2.0 * BM * BM * BK * tile_steps(a); }
 
-static GemmChoice choose_gemm(const NpGemmArgs& a) {
-  const bool plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
-                     (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
-  // Which tile kernel: the lowest estimate (TileCost). The pair kernel takes the forms without peer-arrival flags on B, pushes or
-  // split operands; row-grouped launches only when their tables come in pairs of 128-row blocks (`paired`). K in parts is
-  // for dense plain outputs with too few tiles for the SMs.
-  const int nk = (a.K + BK - 1) / BK, sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
-  const bool can_split = plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && nk >= 8 && a.max_ctas == 0 && a.M > 128;
-  const bool can_pair = plain && sms >= 2;   // a pair needs two CTAs
-  const int bn_asked = a.epilogue == 1 ? 256 : a.bn, pbn_asked = a.epilogue == 1 ? 0 : a.pair_bn;
-  const bool split_asked = can_split && (a.split == 2 || a.split == 4);
-  GemmChoice c{false, false, bn_asked == 256 ? 256 : 128, 1, 1e30};
-  if (can_pair && bn_asked != 128 && (a.mt == 2 || pbn_asked != 0 || (a.mt == 0 && split_asked))) {
-    c.pair = true;   // asked for
-    c.bn = split_asked || pbn_asked == 0 ? 256 : pbn_asked;
-  } else if (bn_asked == 0 || (bn_asked == 256 && a.mt == 0)) {
-    const double steps = tile_steps(a);
-    auto take = [&](const TileCost& t, int tm, int tn, int units, int parts, bool pair, int bn) {
-      const long long n = tiles_of(a, tm, tn);
-      const double waves = (double)((n + units - 1) / units);
-      // tiles of a persistent CTA follow one another; a cluster that splits K starts anew for every tile
-      const double cost = parts == 1 ? t.fixed + waves * (steps * t.step + t.drain) : waves * (t.fixed + steps / parts * t.step + t.drain);
-      if (cost < c.cost) c = GemmChoice{false, pair, bn, parts, cost};
-    };
-    const int n256 = a.epilogue == 1 ? 128 : 256;
-    if (bn_asked == 0) take(COST_128, 128, 128, sms, 1, false, 128);
-    take(COST_256, 128, n256, sms, 1, false, 256);
-    if (can_pair && a.M > 128 && a.mt == 0) {
-      take(COST_PAIR, 256, n256, sms / 2, 1, true, 256);
-      if (bn_asked == 0) {
-        take(COST_PAIR_192, 256, 192, sms / 2, 1, true, 192);
-        take(COST_PAIR_128, 256, 128, sms / 2, 1, true, 128);
-      }
-    }
-    if (can_split && a.mt == 0 && a.split == 0 && sms >= 128) {
-      take(COST_SPLIT2, 256, 256, CLUSTERS4, 2, true, 256);
-      take(COST_SPLIT4, 256, 256, CLUSTERS8, 4, true, 256);
-    }
+// What a launch allows: forms for the pair kernel, and K in parts (dense plain outputs). The pair kernel takes the forms without
+// peer-arrival flags on B, pushes or split operands; row-grouped launches only when their tables come in pairs of 128-row blocks
+// (`paired`).
+struct GemmForms {
+  bool plain, pair, split;
+  int sms;
+};
+static GemmForms forms_of(const NpGemmArgs& a) {
+  GemmForms f;
+  f.sms = a.max_ctas > 0 ? a.max_ctas : num_sms();
+  f.plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
+            (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
+  f.pair = f.plain && f.sms >= 2;   // a pair needs two CTAs
+  f.split = f.plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && (a.K + BK - 1) / BK >= 8 && a.max_ctas == 0 && a.M > 128;
+  return f;
+}
+static double launch_cost(const NpGemmArgs& a, const TileCost& t, int tm, int tn, int units, int splits) {
+  const long long n = tiles_of(a, tm, tn);
+  const double waves = (double)((n + units - 1) / units), steps = tile_steps(a);
+  // tiles of a persistent CTA follow one another; a cluster that splits K starts anew for every tile
+  return splits == 1 ? t.fixed + waves * (steps * t.step + t.drain) : waves * (t.fixed + steps / splits * t.step + t.drain);
+}
+
+// How a product's sum over K is formed where the caller asks for no tile: by the few-row kernel, whole, or in 2 or 4 parts that are
+// added in order. A rule of the product's own sizes, apart from the choice of the kernel that runs it: a product has the same bits on
+// every tile, alone or beside another one in a launch. Other cuts round differently, and after a layer or two of bf16 results that
+// is more than the last bits: a training step whose gradients were summed whole instead of in parts moved its loss by 2e-3.
+struct SumRule {
+  bool few;
+  int parts;
+};
+static SumRule sum_rule(const NpGemmArgs& a, const GemmForms& f) {
+  double best = 1e30;
+  int parts = 1;
+  auto take = [&](const TileCost& t, int tm, int tn, int units, int n) {
+    const double cost = launch_cost(a, t, tm, tn, units, n);
+    if (cost < best) { best = cost; parts = n; }
+  };
+  const int n256 = a.epilogue == 1 ? 128 : 256;
+  if (a.epilogue != 1 && a.bn != 256) take(CUT_128, 128, 128, f.sms, 1);
+  take(CUT_256, 128, n256, f.sms, 1);
+  if (f.pair && a.M > 128) take(CUT_PAIR, 256, n256, f.sms / 2, 1);
+  if (f.split && a.split == 0 && f.sms >= 128) {
+    take(CUT_SPLIT2, 256, 256, CLUSTERS4, 2);
+    take(CUT_SPLIT4, 256, 256, CLUSTERS8, 4);
   }
   // A few rows of a K-major product: the kernel that streams the weight once through all SMs (skinny.cu), unless a tile kernel
   // is expected to be faster. `mt`, `bn`, `split` and `pair_bn` ask for a tile kernel.
-  c.few = a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && plain && a.K > 0 && a.K % 8 == 0 && a.bn == 0 &&
-          a.mt == 0 && a.split == 0 && a.pair_bn == 0 && a.max_ctas == 0 && a.alpha != 0.f &&
-          few_rows_cost(a.M, a.N, a.K) <= few_tiles_cost(c.cost, a.N, a.K);
-  if (split_asked) c.splits = a.split;
+  const bool few = a.M <= 64 && a.mode == 0 && a.epilogue == 0 && !a.a_mn && !a.b_mn && f.plain && a.K > 0 && a.K % 8 == 0 &&
+                   a.bn == 0 && a.mt == 0 && a.split == 0 && a.pair_bn == 0 && a.max_ctas == 0 && a.alpha != 0.f &&
+                   few_rows_cost(a.M, a.N, a.K) <= few_tiles_cost(best, a.N, a.K);
+  return {few, parts};
+}
+
+// The kernel with the lowest estimate (TileCost) among those that form the sum as the rule says
+static GemmChoice choose_gemm(const NpGemmArgs& a) {
+  const GemmForms f = forms_of(a);
+  const int bn_asked = a.epilogue == 1 ? 256 : a.bn, pbn_asked = a.epilogue == 1 ? 0 : a.pair_bn;
+  const bool split_asked = f.split && (a.split == 2 || a.split == 4);
+  GemmChoice c{false, false, bn_asked == 256 ? 256 : 128, 1, 1, 1e30};
+  if (f.pair && bn_asked != 128 && (a.mt == 2 || pbn_asked != 0 || (a.mt == 0 && split_asked))) {
+    c.pair = true;   // asked for
+    const bool in_pair = split_asked && pbn_asked != 0 && a.split <= (pbn_asked == 128 ? 4 : 2);
+    c.bn = pbn_asked == 0 || (split_asked && !in_pair) ? 256 : pbn_asked;
+    if (split_asked) (in_pair ? c.parts : c.splits) = a.split;
+  } else if (bn_asked == 0 || (bn_asked == 256 && a.mt == 0)) {
+    const SumRule rule = a.mt == 0 ? sum_rule(a, f) : SumRule{false, 1};
+    auto take = [&](TileCost t, int tm, int tn, int units, bool pair, int bn, int splits, int parts) {
+      t.drain += parts_drain(parts, bn);
+      const double cost = launch_cost(a, t, tm, tn, units, splits);
+      if (cost < c.cost) c = GemmChoice{false, pair, bn, splits, parts, cost};
+    };
+    const int n256 = a.epilogue == 1 ? 128 : 256;
+    if (rule.parts == 1) {
+      if (bn_asked == 0) take(COST_128, 128, 128, f.sms, false, 128, 1, 1);
+      take(COST_256, 128, n256, f.sms, false, 256, 1, 1);
+      if (f.pair && a.M > 128 && a.mt == 0) {
+        take(COST_PAIR, 256, n256, f.sms / 2, true, 256, 1, 1);
+        if (bn_asked == 0) {
+          take(COST_PAIR_192, 256, 192, f.sms / 2, true, 192, 1, 1);
+          take(COST_PAIR_128, 256, 128, f.sms / 2, true, 128, 1, 1);
+        }
+      }
+    } else {
+      if (bn_asked == 0) take(COST_PAIR_128, 256, 128, f.sms / 2, true, 128, 1, rule.parts);
+      if (bn_asked == 0 && rule.parts == 2) {
+        take(COST_PAIR_192, 256, 192, f.sms / 2, true, 192, 1, 2);
+        take(COST_PAIR, 256, 256, f.sms / 2, true, 256, 1, 2);
+      }
+      if (rule.parts == 2) take(COST_SPLIT2, 256, 256, CLUSTERS4, true, 256, 2, 1);
+      else take(COST_SPLIT4, 256, 256, CLUSTERS8, true, 256, 4, 1);
+    }
+    c.few = rule.few;
+  }
   return c;
 }
 
@@ -1549,21 +1659,21 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
     return np_skinny_linear(a.A, a.lda, a.B, a.ldb, a.M, a.N, a.K, a.C, a.ldc, a.out_f32, a.alpha, a.bias,
                             a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
   if (c.pair)
-    return c.bn == 128   ? launch_gemm<128, true>(a, (cudaStream_t)stream)
-           : c.bn == 192 ? launch_gemm<192, true>(a, (cudaStream_t)stream)
-                         : launch_gemm<256, true>(a, (cudaStream_t)stream, c.splits);
+    return c.bn == 128   ? launch_gemm<128, true>(a, (cudaStream_t)stream, 1, c.parts)
+           : c.bn == 192 ? launch_gemm<192, true>(a, (cudaStream_t)stream, 1, c.parts)
+                         : launch_gemm<256, true>(a, (cudaStream_t)stream, c.splits, c.parts);
   if (c.bn == 256) return launch_gemm<256, false>(a, (cudaStream_t)stream);
   return launch_gemm<128, false>(a, (cudaStream_t)stream);
 }
 
 template <int BN>
-static int launch_gemm2(const NpGemmArgs& a, const NpGemmArgs& b, int extra, cudaStream_t stream) {
+static int launch_gemm2(const NpGemmArgs& a, int parts_a, const NpGemmArgs& b, int parts_b, int extra, cudaStream_t stream) {
   PairMaps m;
   GemmParams p;
   PairSecond second;
   CUtensorMap unused;
-  int rc = prepare_gemm<BN, true>(a, 1, m, unused, unused, p);
-  if (!rc) rc = prepare_gemm<BN, true>(b, 1, second.m, unused, unused, second.p);
+  int rc = prepare_gemm<BN, true>(a, 1, parts_a, m, unused, unused, p);
+  if (!rc) rc = prepare_gemm<BN, true>(b, 1, parts_b, second.m, unused, unused, second.p);
   if (rc) return rc;
   second.extra = extra;
   constexpr int SMEM = gemm_smem<BN, true>();
@@ -1582,8 +1692,9 @@ static int launch_gemm2(const NpGemmArgs& a, const NpGemmArgs& b, int extra, cud
 }
 
 // Two independent products: in one launch where both run on pairs of CTAs and are expected to take less time that way, else one after
-// the other. A product grouped by rows may wait for arrivals and push; what the other one reads has to be there at launch. `pair_bn` of the first asks for one launch with tiles of that many columns, `split` 1 or `mt` 2 of
-// the first for two launches.
+// the other, with the same bits. A product grouped by rows may wait for arrivals and push; what the other one reads has to be there at
+// launch. `pair_bn` of the first asks for one launch with tiles of that many columns (128 where a sum has four parts), `split` 1 or
+// `mt` 2 of the first for two launches.
 NP_API int np_gemm_bf16_two(const NpGemmArgs* first, const NpGemmArgs* second, void* stream) {
   const NpGemmArgs &a = *first, &b = *second;
   auto separate = [&] {
@@ -1606,13 +1717,16 @@ NP_API int np_gemm_bf16_two(const NpGemmArgs* first, const NpGemmArgs* second, v
   const bool swap = tile_steps(b) > tile_steps(a);
   const NpGemmArgs &x = swap ? b : a, &y = swap ? a : b;
   const double sx = tile_steps(x), sy = tile_steps(y);
+  const int px = sum_rule(x, forms_of(x)).parts, py = sum_rule(y, forms_of(y)).parts;
+  const bool wide = px <= 2 && py <= 2;   // four parts: two accumulators a buffer
+  const int asked = a.pair_bn != 0 && !wide ? 128 : a.pair_bn;
   double best = a.pair_bn != 0 ? 1e30 : choose_gemm(a).cost + choose_gemm(b).cost;
   int bn = 0, extra = 0;
   auto take = [&](const TileCost& t, int cols) {   // the pair with the most to do
-    if (a.pair_bn != 0 && a.pair_bn != cols) return;
+    if (asked != 0 && asked != cols) return;
     const int nx = (int)tiles_of(x, 256, cols), ny = (int)tiles_of(y, 256, cols);
     const int pairs = nx + ny < units ? nx + ny : units;
-    const double cx = sx * t.step + t.drain, cy = sy * t.step + t.drain;
+    const double cx = sx * t.step + t.drain + parts_drain(px, cols), cy = sy * t.step + t.drain + parts_drain(py, cols);
     const int ex = (int)(cx / cy);
     // pair 0 has one of the first product's tiles more than pair r; behind each, the others have as much or less
     const int r = nx % pairs, slack = pairs - r, rest = ny - (r == 0 ? 0 : ex < (ny + slack - 1) / slack ? ex * slack : ny);
@@ -1623,13 +1737,15 @@ NP_API int np_gemm_bf16_two(const NpGemmArgs* first, const NpGemmArgs* second, v
     const double most = at_0 > at_r ? at_0 : at_r;
     if (t.fixed + most < best) { best = t.fixed + most; bn = cols; extra = ex; }
   };
-  take(COST_PAIR, 256);
-  take(COST_PAIR_192, 192);
+  if (wide) {
+    take(COST_PAIR, 256);
+    take(COST_PAIR_192, 192);
+  }
   take(COST_PAIR_128, 128);
   cudaStream_t st = (cudaStream_t)stream;
-  return bn == 256   ? launch_gemm2<256>(x, y, extra, st)
-         : bn == 192 ? launch_gemm2<192>(x, y, extra, st)
-         : bn == 128 ? launch_gemm2<128>(x, y, extra, st)
+  return bn == 256   ? launch_gemm2<256>(x, px, y, py, extra, st)
+         : bn == 192 ? launch_gemm2<192>(x, px, y, py, extra, st)
+         : bn == 128 ? launch_gemm2<128>(x, px, y, py, extra, st)
                      : separate();
 }
 

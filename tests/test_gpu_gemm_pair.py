@@ -325,3 +325,59 @@ def test_expert_layer_backward_against_64_bits(T, E, K, capacity):
     main = dict(arena.named_main_grads())
     for n, g in zip(("w1", "w2", "w3"), want[1:]):
         assert rel(main[n].view(g.shape), 2 * g) < 1.5e-2
+
+
+# outputs whose sum over K is cut into 1, 2 and 4 parts (the cut is a rule of the sizes): every kernel that forms such a sum gives its
+# bits, in one pair of CTAs or over a cluster, stored by TMA and from registers, alone and beside another product in a launch
+@pytest.mark.parametrize("M,N,K", [(1024, 1024, 2048), (768, 768, 4096), (2048, 1024, 3072), (520, 136, 1000), (129, 40, 4096)])
+@pytest.mark.parametrize("pair_bn,split", [(128, 2), (128, 4), (192, 2), (256, 2)])
+@pytest.mark.parametrize("layout", ["fwd", "dgrad", "wgrad"])
+def test_parts_of_a_sum_in_one_pair(M, N, K, pair_bn, split, layout):
+    from nanopysche_b200.ops.gemm import gemm
+
+    torch.manual_seed(M + N + K)
+    a_mn, b_mn = layout == "wgrad", layout != "fwd"
+    M += -M % 8 if a_mn else 0
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    ref = a.float() @ b.float().t()
+    A, B = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
+    acc = torch.randn(M, N, device="cuda")
+    for kw in (dict(), dict(out_dtype=torch.float32), dict(accumulate=True, alpha=0.5)):
+        new = {"out": acc.clone()} if "accumulate" in kw else {}
+        y = gemm(A, B, a_mn=a_mn, b_mn=b_mn, pair_bn=pair_bn, split=split, **kw, **new)
+        new = {"out": acc.clone()} if "accumulate" in kw else {}
+        z = gemm(A, B, a_mn=a_mn, b_mn=b_mn, split=split, **kw, **new)
+        want = acc.double() + 0.5 * ref.double() if "accumulate" in kw else ref
+        assert torch.equal(y, z) and rel(y, want) < (3e-3 if y.dtype == torch.bfloat16 else 2e-5)
+
+
+@pytest.mark.parametrize("T,N,K", [(2048, 1024, 1024), (2048, 5632, 1024), (2048, 3072, 1024), (4096, 768, 768), (4096, 2304, 768),
+                                   (2331, 2048, 4096), (640, 512, 2048), (136, 1032, 264)])
+def test_gradients_do_not_depend_on_what_shares_their_launch(T, N, K):
+    """A frozen weight or a deferred weight gradient leaves the bits of the input gradient as they are, and the other way round."""
+    from nanopysche_b200.ops.gemm import gemm, gemm_dgrad_wgrad
+
+    torch.manual_seed(T + N)
+    dy, x = torch.randn(T, N, device="cuda").bfloat16(), torch.randn(T, K, device="cuda").bfloat16()
+    w, acc = (torch.randn(N, K, device="cuda") * N ** -0.5).bfloat16(), torch.randn(N, K, device="cuda")
+    dx, dw = gemm_dgrad_wgrad(dy, w, x, out=acc.clone(), accumulate=True)
+    assert torch.equal(dx, gemm(dy, w, b_mn=True))
+    assert torch.equal(dw, gemm(dy, x, a_mn=True, b_mn=True, out=acc.clone(), accumulate=True))
+
+
+# Cuts of a sum over K, whatever kernel runs it: by the sizes alone. (M, N, K): parts
+CUTS = {(768, 768, 4096): 4, (2304, 768, 4096): 2, (2048, 1024, 3072): 2, (1024, 1024, 2048): 2, (2048, 1024, 2816): 2, (200, 6144, 4096): 2,
+        (4096, 768, 768): 1, (2048, 3072, 1024): 1, (3072, 1024, 2048): 1, (2331, 2048, 4096): 1}
+
+
+@pytest.mark.parametrize("shape,parts", CUTS.items())
+def test_where_a_sum_is_cut(shape, parts):
+    from nanopysche_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    torch.manual_seed(K)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    y = gemm(a, b, out_dtype=torch.float32)
+    same = {p: torch.equal(y, gemm(a, b, out_dtype=torch.float32, **kw))
+            for p, kw in {1: dict(bn=256, mt=2), 2: dict(split=2), 4: dict(split=4)}.items()}
+    assert same == {p: p == parts for p in same}
