@@ -36,31 +36,31 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 // ------------------------------------------------------------------ router
-// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). Four warps share TOK tokens, each over a quarter of
-// the vectors of a row; MINB: CTAs per SM that the register count is held to, U: steps whose loads are in flight together. The gate
-// rows are 64 KB per TOK tokens at d 2048 and 8 experts, read through L1; a warp to a token (or, above 8192 tokens, to four) had the
-// chain of its eight loads to wait for as well. 8 experts, us, before / now: 64 x 2048 7.1 / 3.9, 1024 10.9 / 4.6, 4096 20.4 / 11.6,
-// 16384 41.2 / 30.4; 64 experts, 4096 x 1024 82 / 48.
-// Every token's sum is formed in the same order in all forms (np_router_logits chooses).
-template <int TOK, int MINB, int U>
+// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). Four warps share TOK tokens, each over the whole rows
+// for EPW experts of a pass; MINB: CTAs per SM that the register count is held to, U: steps whose loads are in flight together. Bound by
+// L1: the gate rows are 64 KB per TOK tokens at d 2048 and 8 experts, and each warp reads the tokens again. A warp to a token had the
+// chain of its loads to wait for. 8 experts, us, before / now: 64 x 2048 7.2 / 3.5, 1024 10.8 / 5.0, 4096 20.7 / 13.3, 16384 41.4 / 40.6; 64
+// experts, 4096 x 1024 82 / 43. A quarter of the row to a warp, added over the warps, takes 11.7 at 4096 and 30.3 at 16384, but forms
+// the sums in another order; gate weights that differ in their last bits move the bf16 rows that they scale.
+// Every token's sum is formed in the same order in all forms: a lane's vectors one after the other, then over the lanes.
+template <int TOK, int EPW, int MINB, int U>
 __global__ void __launch_bounds__(256, MINB) router_logits_kernel(const __nv_bfloat16* x, const float* wg, const float* bias,
                                                                   float* __restrict__ logits, int T, int D, int E,
                                                                   int* __restrict__ zero, int n_zero) {
-  constexpr int EB = 8, PARTS = 4, V = TOK * EB;   // V sums per warp, a power of two and at most one per lane
-  __shared__ float s_sum[8][V];
+  constexpr int PARTS = 4, V = TOK * EPW;   // V sums per warp, a power of two and at most one per lane
   np::pdl_begin();
   // what the kernel behind this one adds to (a fill of its own is a launch)
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n_zero; i += blockDim.x) zero[i] = 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = warp % PARTS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int tb = blockIdx.x * 2 * TOK; tb < T; tb += gridDim.x * 2 * TOK) {
     const int t0 = tb + warp / PARTS * TOK;
-    for (int e0 = 0; e0 < E; e0 += EB) {
+    for (int e0 = warp % PARTS * EPW; e0 < E; e0 += PARTS * EPW) {
       float acc[V];
 #pragma unroll
       for (int i = 0; i < V; ++i) acc[i] = 0.f;
 #pragma unroll U
-      for (int d = (part * 32 + lane) * 8; d < D; d += PARTS * 256) {
+      for (int d = lane * 8; d < D; d += 256) {
         float xv[TOK][8];
 #pragma unroll
         for (int k = 0; k < TOK; ++k) {
@@ -72,15 +72,15 @@ __global__ void __launch_bounds__(256, MINB) router_logits_kernel(const __nv_bfl
           }
         }
 #pragma unroll
-        for (int e = 0; e < EB; ++e) {
+        for (int e = 0; e < EPW; ++e) {
           if (e0 + e < E) {
             const float* wp = wg + (size_t)(e0 + e) * D + d;
             const float4 w0 = *reinterpret_cast<const float4*>(wp);
             const float4 w1 = *reinterpret_cast<const float4*>(wp + 4);
 #pragma unroll
             for (int k = 0; k < TOK; ++k)
-              acc[k * EB + e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
-                                 xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
+              acc[k * EPW + e] += xv[k][0] * w0.x + xv[k][1] * w0.y + xv[k][2] * w0.z + xv[k][3] * w0.w + xv[k][4] * w1.x +
+                                  xv[k][5] * w1.y + xv[k][6] * w1.z + xv[k][7] * w1.w;
           }
         }
       }
@@ -100,14 +100,8 @@ __global__ void __launch_bounds__(256, MINB) router_logits_kernel(const __nv_bfl
           acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
         }
       }
-      if (lane % (32 / V) == 0) s_sum[warp][lane / (32 / V)] = acc[0];
-      __syncthreads();
-      if (part == 0 && lane < V) {
-        const int t = t0 + lane / EB, e = e0 + lane % EB;
-        const float sm = (s_sum[warp][lane] + s_sum[warp + 1][lane]) + (s_sum[warp + 2][lane] + s_sum[warp + 3][lane]);
-        if (t < T && e < E) logits[(size_t)t * E + e] = sm + (bias ? bias[e] : 0.f);
-      }
-      __syncthreads();
+      const int i = lane / (32 / V), t = t0 + i / EPW, e = e0 + i % EPW;
+      if (lane % (32 / V) == 0 && t < T && e < E) logits[(size_t)t * E + e] = acc[0] + (bias ? bias[e] : 0.f);
     }
   }
 }
@@ -962,13 +956,16 @@ NP_API int np_router_logits(const void* x, const float* wg, const float* bias, f
   if (D % 8 || T <= 0) return T <= 0 ? 0 : 1;
   auto run = [&](auto kernel, int tok) {
     const int blocks = (T + 2 * tok - 1) / (2 * tok);
-    np_launch(kernel, (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg,
-              bias, logits, T, D, E, zero, n_zero);
+    np_launch(kernel, (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
+              logits, T, D, E, zero, n_zero);
   };
-  // Two tokens per four warps with the vectors of two steps in flight as long as that is one wave of CTAs, then four, which read the
-  // gate rows half as often. us, two / four: 64 x 2048 3.9 / 5.6, 1024 4.6 / 6.1, 2048 8.5 / 6.1, 4096 15.0 / 11.6, 16384 46.8 / 30.4.
-  if (T <= 148 * 2 * 4) run(router_logits_kernel<2, 2, 2>, 2);
-  else run(router_logits_kernel<4, 2, 1>, 4);
+  // Two tokens per four warps with two experts a warp and the vectors of four steps in flight as long as that is one wave of CTAs, then
+  // four, which read the gate rows half as often: an expert a warp and four steps, from nine experts on four experts a warp, which read the
+  // tokens a quarter as often. us, first / second / third: 64 x 2048, 8 experts 3.5 / 5.2 / 11.5, 1024 5.0 / 5.6 / 11.8, 2048 8.4 / 7.6 / 11.9, 4096
+  // 14.7 / 13.3 / 19.1; 2472 x 1024, 16 experts 10.8 / 11.9 / 11.1; 4096 x 1024, 64 53 / 47 / 43.
+  if (T <= 148 * 2 * 4) run(router_logits_kernel<2, 2, 2, 4>, 2);
+  else if (E <= 8) run(router_logits_kernel<4, 1, 2, 4>, 4);
+  else run(router_logits_kernel<4, 4, 2, 1>, 4);
   CHECK_LAUNCH();
 }
 

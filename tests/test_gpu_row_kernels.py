@@ -313,6 +313,30 @@ def test_router_logits(T, D, E):
     assert torch.equal(few, got[-3:])
 
 
+# the order of a logit's sum: a lane's vectors one after the other, then the lanes in halves. One element per vector, so that the order
+# within a vector does not count; magnitudes so far apart that any other order gives another result
+@pytest.mark.parametrize("T,D,E", [(3, 2048, 8), (1184, 2048, 8), (1185, 2304, 5), (1200, 1024, 17)])
+def test_router_logits_order_of_the_sum(T, D, E):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(D)
+    x, w = torch.zeros(T, D), torch.zeros(E, D)
+    x[:, ::8] = torch.randn(T, D // 8) * 2.0 ** torch.randint(-6, 7, (T, D // 8))
+    x = x.bfloat16()
+    w[:, ::8] = torch.randn(E, D // 8) * 2.0 ** torch.randint(-6, 7, (E, D // 8))
+    bias, got = torch.randn(E), torch.empty(T, E, device="cuda")
+    _lib.call("router_logits", x.cuda(), w.cuda(), bias.cuda(), got, T, D, E, None, 0)
+    t = x.float()[:, None, ::8] * w[None, :, ::8]                    # [T, E, vectors], one rounding each
+    acc = torch.zeros(T, E, 32)
+    for v in range(0, D // 8, 32):
+        part = t[..., v:v + 32]
+        acc[..., :part.shape[-1]] += part
+    lane = torch.arange(32)
+    for o in (16, 8, 4, 2, 1):
+        acc = acc + acc[..., lane ^ o]
+    assert torch.equal(got.cpu(), acc[..., 0] + bias)
+
+
 # the ends of the exponent: sigmoid at subnormal numbers, at zero, one and infinity; each of the two reciprocal forms
 def test_swiglu_at_the_ends_of_the_range():
     from nanopysche_b200.ops.activation import glu
