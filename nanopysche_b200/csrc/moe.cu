@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(128) router_bwd_kernel(const float* logits,
   if (da != 0.f) {
     float fp = 0.f;
 #pragma unroll
-    for (int e = 0; e < EMAX; ++e) fp += e < E ? f[e] * __expf(l[e] - lse) : 0.f;
+    for (int e = 0; e < EMAX; ++e)
+      if (e < E) fp = fmaf(f[e], __expf(l[e] - lse), fp);
 #pragma unroll
     for (int e = 0; e < EMAX; ++e) {
       if (e >= E) break;
@@ -273,16 +274,15 @@ __global__ void __launch_bounds__(128) router_bwd_kernel(const float* logits,
     for (int k = 0; k < K; ++k) {
       const int e = indices[(size_t)t * K + k];
       const float w = weights[(size_t)t * K + k], dw = dweights[(size_t)t * K + k];
-      float add;
-      if (gating == 0) {
-        add = w * (dw - wsum);
-      } else {
+      float u = w, v = dw - wsum;   // u * v is added in one rounding
+      if (gating != 0) {
         // w_k = s_k / (sum s + eps); ds_k = (dw_k - sum_j w_j dw_j) / (sum s + eps); dl = ds * s(1-s)
         const float s = 1.f / (1.f + __expf(-logit(e)));
-        add = (dw - wsum) / ssum * s * (1.f - s);
+        u = (dw - wsum) / ssum * s;
+        v = 1.f - s;
       }
 #pragma unroll
-      for (int i = 0; i < EMAX; ++i) dl[i] += e == i ? add : 0.f;
+      for (int i = 0; i < EMAX; ++i) dl[i] = e == i ? fmaf(u, v, dl[i]) : dl[i];
     }
   }
 #pragma unroll

@@ -432,3 +432,27 @@ def test_mx_feed_forward_in_one_node(rows, D, F):
         assert rel(a, b) < 6e-3      # bf16 roundings of dh, d gate and d up
     with torch.no_grad():
         assert torch.equal(feed_forward_glu(x, w13, w2), z)
+
+
+# a chosen expert's part of the logit gradient is added to that of the auxiliary loss in one rounding
+@pytest.mark.parametrize("T,E,K", [(33, 3, 1), (300, 8, 2), (200, 17, 4), (130, 64, 8)])
+def test_router_logit_gradient_is_added_in_one_rounding(T, E, K):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(E)
+    logits, f, daux = torch.randn(T, E, device="cuda"), torch.rand(E, device="cuda"), torch.randn(1, device="cuda") * T
+    top, idx = logits.topk(K, -1)
+    w, dw, idx = top.softmax(-1).contiguous(), torch.randn(T, K, device="cuda") * 0.1, idx.to(torch.int32)
+    dl = torch.empty(2, T, E, device="cuda")
+    for out, d in zip(dl, (None, dw)):
+        _lib.call("router_bwd", logits, None, w, idx, d, f, daux, 1.0, 0.01, out, T, E, K, 0)
+    aux, got, w, dw = (t.cpu().double() for t in (*dl, w, dw))
+    fma = lambda a, b, c: (a * b + c).float().double()      # the product of two floats is exact in 64 bits  # noqa: E731
+    wsum = torch.zeros(T, dtype=torch.double)
+    for k in range(K):
+        wsum = fma(w[:, k], dw[:, k], wsum)
+    want = aux.clone()
+    for k in range(K):
+        at = (torch.arange(T), idx[:, k].cpu().long())
+        want[at] = fma(w[:, k], (dw[:, k] - wsum).float().double(), want[at])
+    assert torch.equal(got, want)
