@@ -681,8 +681,13 @@ __global__ void __launch_bounds__(256) qkv_norm_rope_fwd_kernel(
   }
 }
 
-__device__ __forceinline__ float group16_sum(float v, unsigned mask) {
-  v += __shfl_xor_sync(mask, v, 1);
+// Sum over the 4 terms of each of 16 neighbouring threads, in the order of a thread per 8: the terms of two threads one after the
+// other, then those groups in halves
+__device__ __forceinline__ float group16_sum(const float* t, unsigned mask) {
+  const float first = ((t[0] + t[1]) + t[2]) + t[3], before = __shfl_xor_sync(mask, first, 1);
+  float v = (((before + t[0]) + t[1]) + t[2]) + t[3];   // of the odd thread
+  const float other = __shfl_xor_sync(mask, v, 1);
+  if (!(threadIdx.x & 1)) v = other;
   v += __shfl_xor_sync(mask, v, 2);
   v += __shfl_xor_sync(mask, v, 4);
   v += __shfl_xor_sync(mask, v, 8);
@@ -721,10 +726,12 @@ __device__ __forceinline__ int token_pos(const int* pos_ids, long long t, long l
 // dv copied; the three results form one contiguous dqkv. The gamma / beta gradients are accumulated per thread
 // (a thread keeps its (head, slice) across tokens), summed over the heads of a kind through shared memory in their order and written
 // as one partial row [4 x 128] per CTA (dgamma_q, dbeta_q, dgamma_k, dbeta_k). Added up by shared-memory atomics, all heads of a
-// kind on the same words, and with one token in flight the pass took 40 us at 2331 tokens and 16 / 8 heads (15 now) and 95 at 6000
+// kind on the same words, and with one token in flight the pass took 39 us at 2331 tokens and 16 / 8 heads (14 now) and 94 at 6000
 // (55). A head is handled by 16 neighbouring threads (a 4-wide slice of the lower half and its partner in the upper half); a block
 // has a thread per slice of the rotated heads, which keeps it for all tokens of the block with TOK of them in flight. 8-wide slices
-// need twice the registers: they spilled, or left too few threads on an SM to cover the loads.
+// need twice the registers and left too few threads on an SM to cover the loads (40 to 60 bytes of these spill as it is: the forms up
+// to 24 and above 40 heads). The two means of a head are summed in the order of 8-wide slices all the same (group16_sum): dq is rounded
+// to bf16, and in another order some of its values, and the projection's gradients behind them, come out differently.
 template <int NTH, int MINB, int TOK>
 __global__ void __launch_bounds__(NTH, MINB) qkv_norm_rope_bwd_kernel(
     HeadSrc s0, HeadSrc s1, HeadSrc s2, const __nv_bfloat16* qkv, long long row_stride, int hq, int hkv,
@@ -772,7 +779,7 @@ __global__ void __launch_bounds__(NTH, MINB) qkv_norm_rope_bwd_kernel(
       unpack4(qh[k], dh);
       unpack4(qa[k], xa);
       unpack4(qb[k], xb);
-      float m1 = 0.f, m2 = 0.f;
+      float t1[4], t2[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         ya[j] = dl[j] * c[j] + dh[j] * sn[j];   // gradient at the LayerNorm output
@@ -783,11 +790,10 @@ __global__ void __launch_bounds__(NTH, MINB) qkv_norm_rope_bwd_kernel(
         db[j] += ya[j]; db[4 + j] += yb[j];
         ya[j] *= gl[j];
         yb[j] *= gh[j];
-        m1 += ya[j] + yb[j];
-        m2 += ya[j] * xa[j] + yb[j] * xb[j];
+        t1[j] = ya[j] + yb[j];
+        t2[j] = ya[j] * xa[j] + yb[j] * xb[j];
       }
-      m1 = group16_sum(m1, mask) * (1.f / HD);
-      m2 = group16_sum(m2, mask) * (1.f / HD);
+      const float m1 = group16_sum(t1, mask) * (1.f / HD), m2 = group16_sum(t2, mask) * (1.f / HD);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         ya[j] = st[k].y * (ya[j] - m1 - xa[j] * m2);

@@ -456,3 +456,33 @@ def test_router_logit_gradient_is_added_in_one_rounding(T, E, K):
         at = (torch.arange(T), idx[:, k].cpu().long())
         want[at] = fma(w[:, k], (dw[:, k] - wsum).float().double(), want[at])
     assert torch.equal(got, want)
+
+
+# the means of a head in the backward of head norms: eight neighbouring columns one after the other, then those groups in halves. Zero
+# inputs leave the first mean alone; pairs of +-2^24 beside small whole numbers make every other order another whole number
+@pytest.mark.parametrize("T,hq,hkv", [(3, 2, 1), (300, 16, 8), (200, 32, 8), (90, 40, 16)])
+def test_head_norm_backward_order_of_the_means(T, hq, hkv):
+    from nanopysche_b200.ops import rope as R
+
+    torch.manual_seed(T)
+    H = hq + hkv
+    d = torch.zeros(T, H, 128)
+    at = torch.rand(T, H, 128).topk(16, -1).indices
+    d.scatter_(2, at, torch.cat([torch.randint(1, 9, (T, H, 10)).float(), torch.tensor([1., -1., 1., -1., 1., -1.]).expand(T, H, 6) * 2 ** 24], -1))
+    qkv = torch.zeros(1, T, (H + hkv) * 128, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    norms = [torch.nn.LayerNorm(128, eps=2.0 ** -16, device="cuda") for _ in range(2)]
+    cos, sin = R.rope_tables(4, 128, device="cuda")
+    ids = torch.zeros(1, T, device="cuda", dtype=torch.int32)      # position 0: no rotation
+    q, k, _ = R.qkv_norm_rope(qkv, *norms, cos, sin, hq, hkv, 0, ids)
+    g = d.cuda().bfloat16()[None]
+    torch.autograd.backward([q, k], [g[:, :, :hq].contiguous(), g[:, :, hq:].contiguous()])
+    t = (d[..., :64] + d[..., 64:]).view(T, H, 8, 8)
+    acc = torch.zeros(T, H, 8)
+    for j in range(8):
+        acc = acc + t[..., j]
+    i = torch.arange(8)
+    for o in (1, 2, 4):
+        acc = acc + acc[..., i ^ o]
+    want = 256.0 * (d - acc[..., :1] / 128)
+    got = qkv.grad[0, :, :H * 128].view(T, H, 128).float().cpu()
+    assert ((got - want).abs() <= want.abs() * 2.0 ** -7).all()
