@@ -43,6 +43,7 @@ struct NpGemmArgs {
   int m_split;        // > 0: output rows [0, m_split) go to C, the rest to C2 (layout of C; multiple of 256)
   int pair_bn;        // columns of a pair's tile: 0 = choose, 128, 192 or 256
   int local_push;     // the destinations behind peer_base and done_flag_ptr are this GPU's: ordered at device scope
+  int round_acc;      // epilogue 2: dh is rounded to bf16 before the gradient of the activation, as a product of its own would store it
 };
 
 // Tensor layout of q / k / v / o: [B, S, H, 128] bf16 with element strides (sb, ss, sh); the last dim is

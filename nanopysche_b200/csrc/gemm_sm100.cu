@@ -53,6 +53,7 @@ struct GemmParams {
   const int* done_expected;   // [flags] M blocks expected per destination (x n_blocks tiles each)
   int* const* done_flag_ptr;  // [flags] peer flag word to release when a destination completes
   bool local_push;            // every destination is this GPU's own memory
+  bool round_acc;             // SwiGLU gradient: of dh rounded to bf16
   int parts;                  // pair kernel: K in this many parts with an accumulator each, added in the epilogue
   const void* Cin;            // accumulate source (same dtype as C), rows indexed like a dense C
   long long ldcin;
@@ -343,75 +344,6 @@ __device__ __forceinline__ void stage_store(const CUtensorMap* tm, uint32_t stg,
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
 }
-// Backward of h = silu(gate) * up, 32 columns of dh at a time: the pre-activations of the same rows and columns arrive by TMA
-// in the warp's staging buffer (gate box, up box: 32 rows of 64 bytes each, 64-byte swizzle), d(gate) and d(up) are written
-// over them and leave the same way. dh itself never reaches memory: as a pass of its own this was 46 us of a 720 us
-// feed-forward (4096 tokens, 2048 x 5632), 92 MB of it dh written and read.
-struct GluBar {   // of one epilogue warp, over all its tiles
-  uint32_t bar, phase;
-};
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
-template <int BN>
-__device__ __forceinline__ void store_glu_bwd(const GemmParams& p, const CUtensorMap* tmD, const CUtensorMap* tmGU, uint32_t stg,
-                                              GluBar& gb, volatile int* abort_flag, uint32_t taddr, int row0, int lane, int n0,
-                                              int half) {
-  if (row0 >= p.M) return;
-#pragma unroll 1
-  for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
-    const int col = n0 + c * 32;
-    if (col >= p.N) break;
-    if (lane == 0) {
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the last boxes have left
-      np::mbar_expect_tx(gb.bar, 4096);
-      tma_load_3d(stg, tmGU, gb.bar, col, row0, 0);
-      tma_load_3d(stg + 2048, tmGU, gb.bar, col, row0, 1);
-    }
-    __syncwarp();
-    uint32_t r[32];
-    np::tmem_ld32(taddr + c * 32, r);
-    np::tmem_ld_wait();
-    if (!np::mbar_wait_warp(gb.bar, gb.phase, abort_flag, KID_GEMM, 16)) return;
-    gb.phase ^= 1u;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {   // 8 columns: 16 bytes of gate and of up
-      const uint32_t at = stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4);
-      uint32_t g[4], u[4], dg[4], du[4];
-      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(g[0]), "=r"(g[1]), "=r"(g[2]), "=r"(g[3]) : "r"(at) : "memory");
-      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(at + 2048) : "memory");
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 gf = np::unpack_bf16(g[q]), uf = np::unpack_bf16(u[q]);
-        const float d0 = __uint_as_float(r[8 * j + 2 * q]) * p.alpha, d1 = __uint_as_float(r[8 * j + 2 * q + 1]) * p.alpha;
-        const float s0 = np::sigmoid_f(gf.x), s1 = np::sigmoid_f(gf.y);
-        dg[q] = np::pack_bf16(d0 * uf.x * (s0 * (1.f + gf.x * (1.f - s0))), d1 * uf.y * (s1 * (1.f + gf.y * (1.f - s1))));
-        du[q] = np::pack_bf16(d0 * (gf.x * s0), d1 * (gf.y * s1));
-      }
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(dg[0]), "r"(dg[1]), "r"(dg[2]), "r"(dg[3]) : "memory");
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 2048), "r"(du[0]), "r"(du[1]), "r"(du[2]), "r"(du[3]) : "memory");
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) {
-#pragma unroll
-      for (int z = 0; z < 2; ++z)
-        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmD),
-                     "r"(stg + z * 2048), "r"(col), "r"(row0), "r"(z)
-                     : "memory");
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    }
-  }
-}
-
-// Before the CTA exits: the staging buffer has been read.
-__device__ __forceinline__ void stage_drain(int lane) {
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-
 // A tile's accumulator: tensor memory of this warp's lanes, first column. K in parts: PER_BUFFER of them side by side at `t`, the rest
 // likewise at `t2`.
 template <int BN>
@@ -439,6 +371,79 @@ __device__ __forceinline__ void load_acc(const Acc<BN>& acc, int col, uint32_t* 
 #pragma unroll
     for (int i = 0; i < 32; ++i) r[i] = 0u;
   }
+}
+
+// Backward of h = silu(gate) * up, 32 columns of dh at a time: the pre-activations of the same rows and columns arrive by TMA
+// in the warp's staging buffer (gate box, up box: 32 rows of 64 bytes each, 64-byte swizzle), d(gate) and d(up) are written
+// over them and leave the same way. dh itself never reaches memory: as a pass of its own this was 46 us of a 720 us
+// feed-forward (4096 tokens, 2048 x 5632), 92 MB of it dh written and read.
+struct GluBar {   // of one epilogue warp, over all its tiles
+  uint32_t bar, phase;
+};
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+template <int BN>
+__device__ __forceinline__ void store_glu_bwd(const GemmParams& p, const CUtensorMap* tmD, const CUtensorMap* tmGU, uint32_t stg,
+                                              GluBar& gb, volatile int* abort_flag, const Acc<BN>& acc, int row0, int lane, int n0,
+                                              int half) {
+  if (row0 >= p.M) return;
+#pragma unroll 1
+  for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+    const int col = n0 + c * 32;
+    if (col >= p.N) break;
+    if (lane == 0) {
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the last boxes have left
+      np::mbar_expect_tx(gb.bar, 4096);
+      tma_load_3d(stg, tmGU, gb.bar, col, row0, 0);
+      tma_load_3d(stg + 2048, tmGU, gb.bar, col, row0, 1);
+    }
+    __syncwarp();
+    uint32_t r[32];
+    load_acc(acc, c * 32, r);
+    if (!np::mbar_wait_warp(gb.bar, gb.phase, abort_flag, KID_GEMM, 16)) return;
+    gb.phase ^= 1u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {   // 8 columns: 16 bytes of gate and of up
+      const uint32_t at = stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4);
+      uint32_t g[4], u[4], dg[4], du[4];
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(g[0]), "=r"(g[1]), "=r"(g[2]), "=r"(g[3]) : "r"(at) : "memory");
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(at + 2048) : "memory");
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 gf = np::unpack_bf16(g[q]), uf = np::unpack_bf16(u[q]);
+        float d0 = __uint_as_float(r[8 * j + 2 * q]) * p.alpha, d1 = __uint_as_float(r[8 * j + 2 * q + 1]) * p.alpha;
+        if (p.round_acc) {
+          const float2 d = np::unpack_bf16(np::pack_bf16(d0, d1));
+          d0 = d.x;
+          d1 = d.y;
+        }
+        const float s0 = np::sigmoid_f(gf.x), s1 = np::sigmoid_f(gf.y);
+        dg[q] = np::pack_bf16(d0 * uf.x * (s0 * (1.f + gf.x * (1.f - s0))), d1 * uf.y * (s1 * (1.f + gf.y * (1.f - s1))));
+        du[q] = np::pack_bf16(d0 * (gf.x * s0), d1 * (gf.y * s1));
+      }
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(dg[0]), "r"(dg[1]), "r"(dg[2]), "r"(dg[3]) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 2048), "r"(du[0]), "r"(du[1]), "r"(du[2]), "r"(du[3]) : "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (int z = 0; z < 2; ++z)
+        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmD),
+                     "r"(stg + z * 2048), "r"(col), "r"(row0), "r"(z)
+                     : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+}
+
+// Before the CTA exits: the staging buffer has been read.
+__device__ __forceinline__ void stage_drain(int lane) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 // Half `half` of the BN accumulator columns of one 128-row tile: tensor memory
@@ -775,7 +780,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
       const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
       const int row0 = tl.m_blk * BM + quarter * 32;
-      if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+      if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, Acc<BN>{taddr, 0u, have_acc ? 1 : 0}, row0, lane, n0, half);
       else store_tile<BN>(p, &tmC, &tmC2, stg, Acc<BN>{taddr, 0u, have_acc ? 1 : 0}, tl.g, row0, lane, n0, half);
       if (have_acc) {
         np::tc_fence_before();
@@ -1167,12 +1172,9 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
         const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16), taddr = lanes + (uint32_t)(acc * acc_cols);
         const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
         const int row0 = tl.m_blk * TM + rank * BM + quarter * 32, n0 = tl.n_blk * bn_out;
-        if (q.epilogue == 2) {
-          store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
-        } else {
-          store_tile<BN>(q, &tm.C, &tm.C2, stg, Acc<BN>{taddr, lanes + (uint32_t)((acc ^ 1) * acc_cols), have_acc ? parts : 0}, tl.g,
-                         row0, lane, n0, half);
-        }
+        const Acc<BN> sum{taddr, lanes + (uint32_t)((acc ^ 1) * acc_cols), have_acc ? parts : 0};
+        if (q.epilogue == 2) store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, sum, row0, lane, n0, half);
+        else store_tile<BN>(q, &tm.C, &tm.C2, stg, sum, tl.g, row0, lane, n0, half);
       }
       if (have_acc) {
         np::tc_fence_before();
@@ -1422,6 +1424,7 @@ static int prepare_gemm(const NpGemmArgs& a, int splits, int parts, PairMaps& m,
   p.row_dst = a.row_dst; p.peer_base = a.peer_base;
   p.done_counters = a.done_counters; p.done_expected = a.done_expected; p.done_flag_ptr = a.done_flag_ptr;
   p.local_push = a.local_push != 0;
+  p.round_acc = a.round_acc != 0;
   p.Cin = a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr);
   p.ldcin = a.Cin ? a.ldcin : a.ldc;
   p.epoch_base = a.epoch_base;
@@ -1563,7 +1566,9 @@ static GemmForms forms_of(const NpGemmArgs& a) {
   f.plain = !a.b_ready_flags && !a.push_src && !a.A_loc && !a.B_loc && a.m_rot == 0 && a.n_rot == 0 &&
             (a.mode == 1 ? a.paired != 0 : !a.row_dst && !a.ready_flags && !a.done_counters);
   f.pair = f.plain && f.sms >= 2;   // a pair needs two CTAs
-  f.split = f.plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && a.epilogue == 0 && (a.K + BK - 1) / BK >= 8 && a.max_ctas == 0 && a.M > 128;
+  // a SwiGLU gradient of a rounded dh: the sum that dh as a product of its own has
+  f.split = f.plain && a.k_split == 0 && a.m_split == 0 && a.mode == 0 && (a.epilogue == 0 || (a.epilogue == 2 && a.round_acc)) &&
+            (a.K + BK - 1) / BK >= 8 && a.max_ctas == 0 && a.M > 128;
   return f;
 }
 static double launch_cost(const NpGemmArgs& a, const TileCost& t, int tm, int tn, int units, int splits) {
@@ -1608,7 +1613,7 @@ static SumRule sum_rule(const NpGemmArgs& a, const GemmForms& f) {
 static GemmChoice choose_gemm(const NpGemmArgs& a) {
   const GemmForms f = forms_of(a);
   const int bn_asked = a.epilogue == 1 ? 256 : a.bn, pbn_asked = a.epilogue == 1 ? 0 : a.pair_bn;
-  const bool split_asked = f.split && (a.split == 2 || a.split == 4);
+  const bool split_asked = f.split && a.epilogue == 0 && (a.split == 2 || a.split == 4);
   GemmChoice c{false, false, bn_asked == 256 ? 256 : 128, 1, 1, 1e30};
   if (f.pair && bn_asked != 128 && (a.mt == 2 || pbn_asked != 0 || (a.mt == 0 && split_asked))) {
     c.pair = true;   // asked for
@@ -1639,8 +1644,10 @@ static GemmChoice choose_gemm(const NpGemmArgs& a) {
         take(COST_PAIR_192, 256, 192, f.sms / 2, true, 192, 1, 2);
         take(COST_PAIR, 256, 256, f.sms / 2, true, 256, 1, 2);
       }
-      if (rule.parts == 2) take(COST_SPLIT2, 256, 256, CLUSTERS4, true, 256, 2, 1);
-      else take(COST_SPLIT4, 256, 256, CLUSTERS8, true, 256, 4, 1);
+      if (a.epilogue == 0) {
+        if (rule.parts == 2) take(COST_SPLIT2, 256, 256, CLUSTERS4, true, 256, 2, 1);
+        else take(COST_SPLIT4, 256, 256, CLUSTERS8, true, 256, 4, 1);
+      }
     }
     c.few = rule.few;
   }

@@ -51,6 +51,7 @@ class GemmArgs(C.Structure):
         ("bias", c_void_p),
         ("mt", c_int), ("split", c_int), ("paired", c_int),
         ("k_split", c_int), ("m_split", c_int), ("pair_bn", c_int), ("local_push", c_int),
+        ("round_acc", c_int),
     ]
 
 

@@ -115,7 +115,7 @@ def gemm_swiglu(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, *, sa
     return h, gu
 
 
-def _glu_bwd_args(dy, w2, gu):
+def _glu_bwd_args(dy, w2, gu, round_dh):
     M, F = dy.shape[0], w2.shape[1]
     assert dy.dtype == w2.dtype == gu.dtype == torch.bfloat16, "kernel path is bf16"
     assert dy.shape[1] == w2.shape[0] and gu.shape == (M, 2 * F) and dy.stride(1) == w2.stride(1) == gu.stride(1) == 1
@@ -125,33 +125,36 @@ def _glu_bwd_args(dy, w2, gu):
     args.lda, args.ldb, args.ldc, args.ldc2 = dy.stride(0), w2.stride(0), 2 * F, gu.stride(0)
     args.a_rows, args.b_rows = M, w2.shape[0]
     args.M, args.N, args.K = M, F, dy.shape[1]
-    args.b_mn, args.epilogue, args.alpha = 1, 2, 1.0
+    args.b_mn, args.epilogue, args.alpha, args.round_acc = 1, 2, 1.0, int(round_dh)
     return args, out
 
 
-def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor, pair_bn: int = 0) -> torch.Tensor:
+def gemm_glu_bwd(dy: torch.Tensor, w2: torch.Tensor, gu: torch.Tensor, pair_bn: int = 0, round_dh: bool = False) -> torch.Tensor:
     """``[d gate | d up]`` of ``h = silu(gate) * up`` for ``dh = dy @ w2`` and ``gu = [gate | up]``, without forming ``dh``:
-    the gradient of the activation is the epilogue of the GEMM (``dy [M, D]``, ``w2 [D, F]``, ``gu [M, 2F]``)."""
+    the gradient of the activation is the epilogue of the GEMM (``dy [M, D]``, ``w2 [D, F]``, ``gu [M, 2F]``). ``round_dh``: the
+    gradient of ``dh`` rounded to bf16, bit for bit what two products and a pass over ``dh`` give."""
     if not _use_kernel(dy):
         from .activation import glu_bwd
 
-        return glu_bwd(gu, gemm_ref(dy, w2, b_mn=True))
-    args, out = _glu_bwd_args(dy, w2, gu)
+        dh = gemm_ref(dy, w2, b_mn=True)
+        return glu_bwd(gu, dh.to(dy.dtype) if round_dh else dh)
+    args, out = _glu_bwd_args(dy, w2, gu, round_dh)
     args.pair_bn = pair_bn
     _lib.check(_lib.lib().np_gemm_bf16(C.byref(args), C.c_void_p(_lib.stream())), "gemm_glu_bwd")
     return out
 
 
 def gemm_dgrad_wgrad(dy: torch.Tensor, w: torch.Tensor, x: torch.Tensor, *, out: torch.Tensor | None = None,
-                     accumulate: bool = False, gu: torch.Tensor | None = None, pair_bn: int = 0, mt: int = 0):
+                     accumulate: bool = False, gu: torch.Tensor | None = None, pair_bn: int = 0, mt: int = 0,
+                     round_dh: bool = False):
     """``(dy @ w, dy.T @ x)`` for ``dy [M, N]``, ``w [N, K]``, ``x [M, K]``: the two gradients of a linear layer, in one launch
     where that is expected to be faster than two. The second goes to ``out`` (added with ``accumulate``), by default a new
     tensor in the dtype of ``w``. ``gu``: pre-activations ``[gate | up]`` with ``x = silu(gate) * up``; the first result is then
-    ``[d gate | d up]`` (``gemm_glu_bwd``). ``pair_bn`` and ``mt`` ask for one launch with tiles of that many columns, two launches."""
+    ``[d gate | d up]`` (``gemm_glu_bwd``, with ``round_dh``). ``pair_bn`` and ``mt`` ask for one launch with tiles of that many columns, two launches."""
     if not _use_kernel(dy):
-        dx = gemm(dy, w, b_mn=True) if gu is None else gemm_glu_bwd(dy, w, gu)
+        dx = gemm(dy, w, b_mn=True) if gu is None else gemm_glu_bwd(dy, w, gu, round_dh=round_dh)
         return dx, gemm(dy, x, a_mn=True, b_mn=True, out=out, out_dtype=w.dtype if out is None else None, accumulate=accumulate)
-    a0, dx = _gemm_args(dy, w, False, True, None, None, False, 1.0) if gu is None else _glu_bwd_args(dy, w, gu)
+    a0, dx = _gemm_args(dy, w, False, True, None, None, False, 1.0) if gu is None else _glu_bwd_args(dy, w, gu, round_dh)
     a1, dw = _gemm_args(dy, x, True, True, out, w.dtype, accumulate, 1.0)
     a0.pair_bn, a0.mt = pair_bn, mt
     rc = _lib.lib().np_gemm_bf16_two(C.byref(a0), C.byref(a1), C.c_void_p(_lib.stream()))
@@ -230,15 +233,15 @@ def _wgrad_into(w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
     return gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=w.dtype if w.is_cuda else None)
 
 
-def _both_grads(w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor, gu: torch.Tensor | None = None):
+def _both_grads(w: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor, gu: torch.Tensor | None = None, round_dh: bool = False):
     """Input gradient (with ``gu``: the gradient of its pre-activations) and what ``_wgrad_into`` returns for ``w``."""
     if not _use_kernel(dy2) or _deferred(w):
-        dx = gemm(dy2, w, b_mn=True) if gu is None else gemm_glu_bwd(dy2, w, gu)
+        dx = gemm(dy2, w, b_mn=True) if gu is None else gemm_glu_bwd(dy2, w, gu, round_dh=round_dh)
         return dx, _wgrad_into(w, dy2, x2)
     mg = getattr(w, "main_grad", None)
     if mg is None:
-        return gemm_dgrad_wgrad(dy2, w, x2, gu=gu)
-    dx, _ = gemm_dgrad_wgrad(dy2, w, x2, out=mg, accumulate=getattr(w, "_main_grad_dirty", False), gu=gu)
+        return gemm_dgrad_wgrad(dy2, w, x2, gu=gu, round_dh=round_dh)
+    dx, _ = gemm_dgrad_wgrad(dy2, w, x2, out=mg, accumulate=getattr(w, "_main_grad_dirty", False), gu=gu, round_dh=round_dh)
     _main_grad_done(w)
     return dx, None
 
@@ -345,9 +348,9 @@ class _SwiGLUFeedForward(torch.autograd.Function):
         return None if dx is None else dx.view(dy.shape[:-1] + dx.shape[-1:]), dw13, dw2, None
 
 
-def _feed_forward_grads(ctx, dy: torch.Tensor):
+def _feed_forward_grads(ctx, dy: torch.Tensor, round_dh: bool = False):
     """``(dx [rows, D], dw13, dw2)`` as far as they are asked for (inputs 0 to 2 of the autograd function, which saved ``x, w13,
-    w2, h, gu``)."""
+    w2, h, gu``). ``round_dh``: as in ``gemm_glu_bwd``."""
     x, w13, w2, h, gu = ctx.saved_tensors
     dy2 = dy.reshape(-1, dy.shape[-1])
     if not dy2.is_contiguous():
@@ -356,9 +359,9 @@ def _feed_forward_grads(ctx, dy: torch.Tensor):
     if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or hasattr(w13, "main_grad")):
         return None, None, _wgrad_into(w2, dy2, h) if want_dw2 else None
     if want_dw2:
-        dgu, dw2 = _both_grads(w2, dy2, h, gu)
+        dgu, dw2 = _both_grads(w2, dy2, h, gu, round_dh)
     else:
-        dgu, dw2 = gemm_glu_bwd(dy2, w2, gu), None
+        dgu, dw2 = gemm_glu_bwd(dy2, w2, gu, round_dh=round_dh), None
     return *_linear_grads(ctx, w13, dgu, x.reshape(-1, x.shape[-1])), dw2
 
 

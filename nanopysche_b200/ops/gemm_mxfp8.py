@@ -258,7 +258,8 @@ class _MXLinear(torch.autograd.Function):
 class _MXFeedForward(torch.autograd.Function):
     """``(silu(x @ w1.T) * (x @ w3.T)) @ w2.T`` for a fused ``[w1; w3]`` weight with both forward GEMMs in MXFP8: the activation is
     formed, rounded and quantised in one pass. The backward GEMMs run in bf16 on the unquantised tensors, the gradient of the
-    activation in the epilogue of the down projection's (4096 tokens, 2048 x 5632: quantisers and activation passes 123 -> 68 us)."""
+    activation in the epilogue of the down projection's (4096 tokens, 2048 x 5632: quantisers and activation passes 123 -> 68 us). Every
+    result has the bits of the two linear layers and the activation between them (``mx_linear``, ``glu``)."""
 
     @staticmethod
     def forward(ctx, x, w13, w2, save):
@@ -275,7 +276,7 @@ class _MXFeedForward(torch.autograd.Function):
     def backward(ctx, dy):
         from .gemm import _feed_forward_grads
 
-        dx, dw13, dw2 = _feed_forward_grads(ctx, dy)
+        dx, dw13, dw2 = _feed_forward_grads(ctx, dy, round_dh=True)
         return None if dx is None else dx.view(ctx.x_shape), dw13, dw2, None
 
 

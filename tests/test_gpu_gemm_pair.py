@@ -381,3 +381,35 @@ def test_where_a_sum_is_cut(shape, parts):
     same = {p: torch.equal(y, gemm(a, b, out_dtype=torch.float32, **kw))
             for p, kw in {1: dict(bn=256, mt=2), 2: dict(split=2), 4: dict(split=4)}.items()}
     assert same == {p: p == parts for p in same}
+
+
+# the MXFP8 feed-forward node against the layers it stands for: the same bits, dh rounded to bf16 before the activation's gradient, its
+# sum whole and in parts; gradients asked for together, with the weights' in main_grad, deferred, and of the input alone
+@pytest.mark.parametrize("T,D,F", [(70, 128, 256), (200, 2048, 5632), (300, 768, 2048), (1030, 256, 640)])
+@pytest.mark.parametrize("form", ["leaf", "main_grad", "deferred", "input"])
+def test_mxfp8_feed_forward_has_the_bits_of_its_layers(T, D, F, form):
+    from nanopysche_b200.ops.activation import glu
+    from nanopysche_b200.ops.gemm import defer_wgrad, feed_forward_glu, linear, run_deferred_wgrads
+
+    torch.manual_seed(T)
+    x0, dy = torch.randn(1, T, D, device="cuda").bfloat16(), torch.randn(1, T, D, device="cuda").bfloat16()
+    ws = [(torch.randn(s, device="cuda") * s[1] ** -0.5).bfloat16() for s in ((2 * F, D), (D, F))]
+
+    def grads(layer):
+        x, w13, w2 = (t.clone().requires_grad_(form != "input" or t is x0) for t in (x0, *ws))
+        for w in (w13, w2):
+            w._fp8_recipe = "mxfp8"
+            if form in ("main_grad", "deferred"):
+                w.main_grad, w._main_grad_dirty = torch.zeros(w.shape, device="cuda"), False
+        y, queue = layer(x, w13, w2), []
+        if form == "deferred":
+            with defer_wgrad(queue):
+                y.backward(dy)
+            run_deferred_wgrads(queue)
+        else:
+            y.backward(dy)
+        return [y, x.grad] + [getattr(w, "main_grad", w.grad) for w in (w13, w2) if form != "input"]
+
+    got = grads(lambda x, w13, w2: feed_forward_glu(x, w13, w2, "silu"))
+    want = grads(lambda x, w13, w2: linear(glu(linear(x, w13), "silu"), w2))
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and len(got) == len(want)
