@@ -53,6 +53,24 @@ def test_cross_entropy_rows(rows, V):
     assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item()) and rel(logits.grad, l64.grad) < 4e-3
 
 
+# The sum of a row is formed in one order against the row's maximum: bits of lse, taken from the two-pass kernel. One large entry per
+# row keeps the logarithm small, so that the last bits of the sum show.
+LSE_BITS = {1003: [1058881404, 1058961473, 1058751203, 1059190132, 1059210456, 1059747382],
+            32000: [1079399911, 1079429039, 1079425302, 1079415901, 1079391680, 1079416142],
+            50264: [1081257709, 1081275162, 1081247448, 1081250681, 1081248575, 1081272020]}
+
+
+@pytest.mark.parametrize("V", LSE_BITS)
+def test_cross_entropy_order_of_the_sum(V):
+    from nanopysche_b200.ops.xent import _rows_fwd
+
+    r, c = torch.arange(6), torch.arange((V + 7) // 8 * 8)
+    x = -5 - ((r[:, None] * 7919 + c * 104729 + c * c % 1543) % 2003).float() / 256
+    x[r, r * 17 + V // 2] = 0.0
+    _, lse = _rows_fwd(x.bfloat16().cuda()[:, :V], torch.zeros(6, dtype=torch.long, device="cuda"), -100)
+    assert lse.view(torch.int32).tolist() == LSE_BITS[V]
+
+
 # masked vocabulary entries (-inf): single ones, a thread's whole share, all but one; +inf, NaN and a row of -inf give NaN
 @pytest.mark.parametrize("V", [7, 264, 8200, 32000])
 def test_cross_entropy_infinities(V):
