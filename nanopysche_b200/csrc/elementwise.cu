@@ -996,7 +996,9 @@ __global__ void __launch_bounds__(XT) xent_bwd_kernel(const __nv_bfloat16* logit
 // Decoupled weight decay on fp32 masters; writes the bf16 compute copy in the same pass.
 // gscale (device scalar, may be null) multiplies the gradient (gradient clipping coefficient). A thread takes one vector of four: the
 // CTAs then sweep the seven arrays together in step, where CTAs that strode over the whole length drifted apart. 100 million
-// parameters (30 bytes each): 499 us with 8 CTAs per SM striding, 441 now, 6.8 TB/s; a vector ahead in registers 552, streaming hints 504.
+// parameters (30 bytes each): 499 us with 8 CTAs per SM striding, 441 now, 6.8 TB/s; a vector ahead in registers 552, streaming hints
+// 504. The last vectors come first: the norm in front of the update has just read them, and they are still in L2 (both together 562 us
+// before, 531 with one vector per thread in ascending order, 513 in this one).
 __global__ void __launch_bounds__(256, 5) adamw_kernel(float* __restrict__ p, const float* g, float* __restrict__ m,
                              float* __restrict__ v, __nv_bfloat16* __restrict__ w16, long long n, float lr,
                              float b1, float b2, float eps, float wd, float bc1, float bc2,
@@ -1004,7 +1006,7 @@ __global__ void __launch_bounds__(256, 5) adamw_kernel(float* __restrict__ p, co
   np::pdl_begin();
   const float gs = gscale ? gscale[0] : 1.f;
   if (hyper) { lr = hyper[0]; bc1 = hyper[1]; bc2 = hyper[2]; }  // device-resident schedule (graph replay)
-  const long long nvec = n >> 2, i = blockIdx.x * 256ll + threadIdx.x;
+  const long long nvec = n >> 2, i = (gridDim.x - 1 - blockIdx.x) * 256ll + threadIdx.x;
   if (i < nvec) {
     float4 pp = reinterpret_cast<float4*>(p)[i];
     const float4 gg = reinterpret_cast<const float4*>(g)[i];
@@ -1035,21 +1037,18 @@ __global__ void __launch_bounds__(256, 5) adamw_kernel(float* __restrict__ p, co
   }
 }
 
-// partial[b] = sum of x^2 over this CTA's tiles (fp32 input), eight loads in flight per thread, the last tiles first: what the
-// optimizer then reads first is still in L2 (sums and update of 100 million parameters 531 us in ascending order, 506 in this one).
+// partial[b] = sum over this CTA's grid-stride slice of x^2 (fp32 input): a thread's vectors one after the other, eight loads in flight.
 __global__ void __launch_bounds__(NT) sumsq_kernel(const float* x, long long n,
                                                    float* __restrict__ partial) {
   np::pdl_begin();
   constexpr int U = 8;
   __shared__ float red[32];
   float s = 0.f;
-  const long long nvec = n >> 2, tiles = (nvec + NT * U - 1) / (NT * U);
-  for (long long t = tiles - 1 - blockIdx.x; t >= 0; t -= gridDim.x) {
-    const long long i = t * (NT * U) + threadIdx.x;
+  const long long nvec = n >> 2, stride = (long long)gridDim.x * NT;
+  for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < nvec; i += U * stride) {
     float4 a[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      a[u] = i + u * NT < nvec ? reinterpret_cast<const float4*>(x)[i + u * NT] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < U; ++u) a[u] = i + u * stride < nvec ? reinterpret_cast<const float4*>(x)[i + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < U; ++u) s += a[u].x * a[u].x + a[u].y * a[u].y + a[u].z * a[u].z + a[u].w * a[u].w;
   }

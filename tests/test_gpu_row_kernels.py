@@ -504,3 +504,30 @@ def test_head_norm_backward_order_of_the_means(T, hq, hkv):
     want = 256.0 * (d - acc[..., :1] / 128)
     got = qkv.grad[0, :, :H * 128].view(T, H, 128).float().cpu()
     assert ((got - want).abs() <= want.abs() * 2.0 ** -7).all()
+
+
+# the order of the gradient norm's sums: a thread's vectors one after the other, lanes in halves, warps in halves. One element per
+# vector, so that the order within a vector does not count
+@pytest.mark.parametrize("n", [3, 40, 151552 * 4, 151552 * 4 * 9 + 4003])
+def test_sum_of_squares_order(n):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(n)
+    parts = _lib.lib().np_sumsq_parts()
+    x = torch.zeros(n)
+    x[::4] = torch.randn(-(-n // 4)) * 2.0 ** torch.randint(-6, 7, (-(-n // 4),))
+    tail = x[n // 4 * 4:]
+    got = torch.zeros(parts, device="cuda")
+    _lib.call("sumsq", x.cuda(), _lib.LL(n), got)
+    t = (x * x)[:n // 4 * 4:4]
+    s = torch.zeros(parts * 256)
+    for k in range(0, t.numel(), parts * 256):
+        s[:t[k:k + parts * 256].numel()] += t[k:k + parts * 256]
+    s[0] += (tail * tail).sum()                      # at most one of them is not zero
+    s, i = s.view(parts, 8, 32), torch.arange(32)
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[..., i ^ o]
+    s = torch.nn.functional.pad(s[..., 0], (0, 24))
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[..., i ^ o]
+    assert torch.equal(got.cpu(), s[:, 0])
