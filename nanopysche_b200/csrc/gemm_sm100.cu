@@ -344,35 +344,6 @@ __device__ __forceinline__ void stage_store(const CUtensorMap* tm, uint32_t stg,
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
 }
-// A tile's accumulator: tensor memory of this warp's lanes, first column. K in parts: PER_BUFFER of them side by side at `t`, the rest
-// likewise at `t2`.
-template <int BN>
-constexpr int PER_BUFFER = BN == 128 ? 2 : 1;
-template <int BN>
-struct Acc {
-  uint32_t t, t2;
-  int parts;   // 0: no K steps, zeros
-};
-// 32 accumulator columns of this lane's row, the parts added in their order
-template <int BN>
-__device__ __forceinline__ void load_acc(const Acc<BN>& acc, int col, uint32_t* r) {
-  if (acc.parts > 0) {
-    np::tmem_ld32(acc.t + col, r);
-    np::tmem_ld_wait();
-#pragma unroll 1
-    for (int q = 1; q < acc.parts; ++q) {
-      uint32_t v[32];
-      np::tmem_ld32((q / PER_BUFFER<BN> ? acc.t2 : acc.t) + q % PER_BUFFER<BN> * BN + col, v);
-      np::tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(v[i]));
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) r[i] = 0u;
-  }
-}
-
 // Backward of h = silu(gate) * up, 32 columns of dh at a time: the pre-activations of the same rows and columns arrive by TMA
 // in the warp's staging buffer (gate box, up box: 32 rows of 64 bytes each, 64-byte swizzle), d(gate) and d(up) are written
 // over them and leave the same way. dh itself never reaches memory: as a pass of its own this was 46 us of a 720 us
@@ -388,7 +359,7 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm,
 }
 template <int BN>
 __device__ __forceinline__ void store_glu_bwd(const GemmParams& p, const CUtensorMap* tmD, const CUtensorMap* tmGU, uint32_t stg,
-                                              GluBar& gb, volatile int* abort_flag, const Acc<BN>& acc, int row0, int lane, int n0,
+                                              GluBar& gb, volatile int* abort_flag, uint32_t taddr, int row0, int lane, int n0,
                                               int half) {
   if (row0 >= p.M) return;
 #pragma unroll 1
@@ -403,7 +374,8 @@ __device__ __forceinline__ void store_glu_bwd(const GemmParams& p, const CUtenso
     }
     __syncwarp();
     uint32_t r[32];
-    load_acc(acc, c * 32, r);
+    np::tmem_ld32(taddr + c * 32, r);
+    np::tmem_ld_wait();
     if (!np::mbar_wait_warp(gb.bar, gb.phase, abort_flag, KID_GEMM, 16)) return;
     gb.phase ^= 1u;
 #pragma unroll
@@ -446,13 +418,23 @@ __device__ __forceinline__ void stage_drain(int lane) {
   if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// Half `half` of the BN accumulator columns of one 128-row tile: tensor memory
+// 32 accumulator columns of this lane's row (zeros without an accumulator)
+__device__ __forceinline__ void load_acc(uint32_t taddr, bool have_acc, uint32_t* r) {
+  if (have_acc) {
+    np::tmem_ld32(taddr, r);
+    np::tmem_ld_wait();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = 0u;
+  }
+}
+
+// Half `half` of the BN accumulator columns of one 128-row tile: tensor memory (`taddr`: this warp's lanes, first column)
 // through the epilogue of the launch to output rows row0 .. row0 + 31, columns from `n0`. Executed by whole warps (the
 // tensor-memory loads are .sync.aligned).
 template <int BN>
 __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmC2, uint32_t stg,
-                                           const Acc<BN>& acc, int g_idx, int row0, int lane, int n0, int half) {
-  const uint32_t taddr = acc.t;
+                                           uint32_t taddr, int g_idx, int row0, int lane, int n0, int half, bool have_acc) {
   if (p.tma_c) {
     if (row0 >= p.M) return;
     if (p.m_split && row0 >= p.m_split) {
@@ -494,7 +476,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
         const int col = n0 + c * 32;
         if (col >= p.N) break;
         uint32_t r[32];
-        load_acc(acc, c * 32, r);
+        load_acc(taddr + c * 32, have_acc, r);
         scale_bias(p, r, col);
         stage_store(tmC, stg, lane, r, col, row0, g_idx);
       }
@@ -507,7 +489,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           uint32_t r[32];
-          load_acc(acc, c * 64 + q * 32, r);
+          load_acc(taddr + c * 64 + q * 32, have_acc, r);
           scale_bias(p, r, col + q * 32);
           pack32(r, w + 16 * q);
         }
@@ -534,7 +516,7 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const CUtensorMa
     for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
       uint32_t r[32];
       __syncwarp();
-      load_acc(acc, c * 32, r);
+      load_acc(taddr + c * 32, have_acc, r);
       store_chunk(p, o, r, n0 + c * 32);
     }
   }
@@ -780,8 +762,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quarter * 32) << 16);
       const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
       const int row0 = tl.m_blk * BM + quarter * 32;
-      if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, Acc<BN>{taddr, 0u, have_acc ? 1 : 0}, row0, lane, n0, half);
-      else store_tile<BN>(p, &tmC, &tmC2, stg, Acc<BN>{taddr, 0u, have_acc ? 1 : 0}, tl.g, row0, lane, n0, half);
+      if (p.epilogue == 2) store_glu_bwd<BN>(p, &tmC, &tmC2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+      else store_tile<BN>(p, &tmC, &tmC2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
       if (have_acc) {
         np::tc_fence_before();
         __syncwarp();
@@ -878,10 +860,10 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 // of such a GEMM is its K steps one after the other (about 0.3 us each), not its FLOPs.
 //
 // p.parts: one pair forms the same parts in turn, each in accumulator columns of its own (128-column tiles: two parts in each of the
-// two buffers; wider ones: one), and the epilogue adds them in their order, so that the result has the bits of the cluster's. It
-// takes a tile as long as a whole sum and a little more: us, whole / two parts / four / cluster of two / of four, 2048 x 1024 x 3072
-// 17.4 / 17.6 / 17.9 / 17.5 / 42.8, 1024 x 768 x 2048 11.9 / 12.1 / 12.5 / 14.6 / 14.0, 768 x 768 x 4096 20.2 / 20.3 / 20.5 / 19.3 / 16.5;
-// 192 columns 18.5 and 256 20.8 with two parts in the first, where no products cover their drain.
+// two buffers; wider ones: one), and the epilogue warps add them in their order, so that the result has the bits of the cluster's. It
+// takes a tile as long as a whole sum and a little more: us, whole / two parts / four / cluster of two / of four, 2048 x 1024 x 3072 17.2 /
+// 17.4 / 17.9 / 17.6 / 42.6, 1024 x 768 x 2048 11.7 / 12.0 / 12.4 / 14.0 / 13.9, 768 x 768 x 4096 20.4 / 20.7 / 21.1 / 19.1 / 16.8. Tiles of 192 and
+// 256 columns sum in parts beside another product only: alone, no products cover their drain (2048 x 1024 x 3072 18.7 and 20.9).
 //
 // DUAL: two products in one launch. A backward pass asks for the gradients of a layer's input and of its weight at the same
 // time; alone, each leaves SMs without work in its only or last wave and pays for a launch, first loads and a last drain of its
@@ -922,6 +904,34 @@ __host__ __device__ __forceinline__ PairWork pair_work(int k, int pair, int pair
   return {1, j < n1 ? j : -1};
 }
 
+// K in parts: PER_BUFFER of them side by side in one of the two accumulator buffers, the rest likewise in the other
+template <int BN>
+constexpr int PER_BUFFER = BN == 128 ? 2 : 1;
+// The parts of a tile added in their order, in place of the first (`t`: this warp's lanes, first column; `t2`: the other buffer). A pass of
+// its own before the epilogue, which then is that of a whole sum: added as each epilogue form reads its columns, the parts took a captured
+// step of four 350m layers from 2320 to 2404 us (launches without parts too: code that has to be fetched), with a kernel of their own
+// beside the one for whole sums 2420, like this 2358. A warp adds the columns that it stores: `wide`, every other 64 of them
+// (store_tile), else a half.
+template <int BN>
+__device__ __forceinline__ void add_parts(uint32_t t, uint32_t t2, int parts, int half, bool wide) {
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    if ((wide ? c >> 1 & 1 : c / (BN / 64)) != half) continue;
+    uint32_t sum[32], v[32];
+    np::tmem_ld32(t + c * 32, sum);
+#pragma unroll 1
+    for (int p = 1; p < parts; ++p) {
+      np::tmem_ld32((p / PER_BUFFER<BN> ? t2 : t) + p % PER_BUFFER<BN> * BN + c * 32, v);
+      np::tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) sum[i] = __float_as_uint(__uint_as_float(sum[i]) + __uint_as_float(v[i]));
+    }
+    np::tmem_st16(t + c * 32, sum);
+    np::tmem_st16(t + c * 32 + 16, sum + 16);
+  }
+  np::tmem_st_wait();
+}
+
 template <bool SPLIT, int BN, bool DUAL>
 __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams& p, const PairSecond* second) {
   constexpr int STAGES = pair_stages<BN>(), TM = 2 * BM, HN = BN / 2;
@@ -949,8 +959,10 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
   auto n_blocks = [&](const GemmParams& q) { return (q.N + bn_out - 1) / bn_out; };
   auto num_tiles = [&](const GemmParams& q) { return m_blocks(q) * n_blocks(q) * ((q.mode == 2) ? q.num_groups : 1); };
   const int tiles0 = num_tiles(p), tiles1 = DUAL ? num_tiles(second->p) : 0;
-  // parts that this pair sums one after the other, and columns of one of the two accumulator buffers
-  auto k_parts = [](const GemmParams& q) { return SPLIT ? 1 : q.parts; };
+  // parts that this pair sums one after the other, and columns of one of the two accumulator buffers. A product alone is summed in parts
+  // on 128 columns only: code that is not there does not have to be fetched
+  constexpr bool PARTS = DUAL || BN == 128;
+  auto k_parts = [](const GemmParams& q) { return PARTS ? q.parts : 1; };
   const int acc_cols = k_parts(p) > 1 || (DUAL && k_parts(second->p) > 1) ? PER_BUFFER<BN> * BN : BN;
   const uint32_t tmem_cols = 2 * acc_cols <= 256 ? 256 : 512;
   auto work = [&](int k) -> PairWork {
@@ -1109,9 +1121,9 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
         const int parts = k_parts(q), nkb = parts > 1 ? count_k(q, tl.g) : 0;
         // 2 or 4 parts: the first K of the next one (a division per K step made the step half as long again)
         auto part_end = [&](int part) { return (int)((long long)nkb * (part + 1) >> (parts >> 1)) * BK; };
-        int part = 0, next_k = parts > 1 ? part_end(0) : 0;
+        int part = 0, next_k = parts > 1 ? part_end(0) : -1;
         k_steps(q, tl.g, [&](int k0) -> bool {
-          if (parts > 1 && k0 == next_k) {   // the next part, in its own columns
+          if (PARTS && k0 == next_k) {   // the next part, in its own columns
             accum = 0;
             next_k = part_end(++part);
             tmem_d += BN;
@@ -1172,9 +1184,10 @@ __device__ __forceinline__ void pair_body(const PairMaps& maps, const GemmParams
         const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16), taddr = lanes + (uint32_t)(acc * acc_cols);
         const uint32_t stg = stg_base + (warp - 2) * STG_BYTES;
         const int row0 = tl.m_blk * TM + rank * BM + quarter * 32, n0 = tl.n_blk * bn_out;
-        const Acc<BN> sum{taddr, lanes + (uint32_t)((acc ^ 1) * acc_cols), have_acc ? parts : 0};
-        if (q.epilogue == 2) store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, sum, row0, lane, n0, half);
-        else store_tile<BN>(q, &tm.C, &tm.C2, stg, sum, tl.g, row0, lane, n0, half);
+        if (PARTS && parts > 1)
+          add_parts<BN>(taddr, lanes + (uint32_t)((acc ^ 1) * acc_cols), parts, half, q.epilogue == 0 && q.tma_c && !q.out_f32);
+        if (q.epilogue == 2) store_glu_bwd<BN>(q, &tm.C, &tm.C2, stg, gb, abort_flag, taddr, row0, lane, n0, half);
+        else store_tile<BN>(q, &tm.C, &tm.C2, stg, taddr, tl.g, row0, lane, n0, half, have_acc);
       }
       if (have_acc) {
         np::tc_fence_before();
@@ -1617,9 +1630,8 @@ static GemmChoice choose_gemm(const NpGemmArgs& a) {
   GemmChoice c{false, false, bn_asked == 256 ? 256 : 128, 1, 1, 1e30};
   if (f.pair && bn_asked != 128 && (a.mt == 2 || pbn_asked != 0 || (a.mt == 0 && split_asked))) {
     c.pair = true;   // asked for
-    const bool in_pair = split_asked && pbn_asked != 0 && a.split <= (pbn_asked == 128 ? 4 : 2);
-    c.bn = pbn_asked == 0 || (split_asked && !in_pair) ? 256 : pbn_asked;
-    if (split_asked) (in_pair ? c.parts : c.splits) = a.split;
+    c.bn = pbn_asked == 0 || (split_asked && pbn_asked != 128) ? 256 : pbn_asked;
+    if (split_asked) (c.bn == 128 ? c.parts : c.splits) = a.split;
   } else if (bn_asked == 0 || (bn_asked == 256 && a.mt == 0)) {
     const SumRule rule = a.mt == 0 ? sum_rule(a, f) : SumRule{false, 1};
     auto take = [&](TileCost t, int tm, int tn, int units, bool pair, int bn, int splits, int parts) {
@@ -1640,10 +1652,6 @@ static GemmChoice choose_gemm(const NpGemmArgs& a) {
       }
     } else {
       if (bn_asked == 0) take(COST_PAIR_128, 256, 128, f.sms / 2, true, 128, 1, rule.parts);
-      if (bn_asked == 0 && rule.parts == 2) {
-        take(COST_PAIR_192, 256, 192, f.sms / 2, true, 192, 1, 2);
-        take(COST_PAIR, 256, 256, f.sms / 2, true, 256, 1, 2);
-      }
       if (a.epilogue == 0) {
         if (rule.parts == 2) take(COST_SPLIT2, 256, 256, CLUSTERS4, true, 256, 2, 1);
         else take(COST_SPLIT4, 256, 256, CLUSTERS8, true, 256, 4, 1);
@@ -1667,8 +1675,8 @@ NP_API int np_gemm_bf16(const NpGemmArgs* args, void* stream) {
                             a.Cin ? a.Cin : (a.accumulate ? a.C : nullptr), a.Cin ? a.ldcin : a.ldc, (cudaStream_t)stream);
   if (c.pair)
     return c.bn == 128   ? launch_gemm<128, true>(a, (cudaStream_t)stream, 1, c.parts)
-           : c.bn == 192 ? launch_gemm<192, true>(a, (cudaStream_t)stream, 1, c.parts)
-                         : launch_gemm<256, true>(a, (cudaStream_t)stream, c.splits, c.parts);
+           : c.bn == 192 ? launch_gemm<192, true>(a, (cudaStream_t)stream)
+                         : launch_gemm<256, true>(a, (cudaStream_t)stream, c.splits);
   if (c.bn == 256) return launch_gemm<256, false>(a, (cudaStream_t)stream);
   return launch_gemm<128, false>(a, (cudaStream_t)stream);
 }
