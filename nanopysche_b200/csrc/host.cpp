@@ -37,7 +37,7 @@ int np_router_topk(const float*, const float*, float*, int*, int*, float*, float
 int np_router_aux(const int*, const float*, const float*, float, float*, float*, int, int, void*);
 int np_router_bwd(const float*, const float*, const float*, const int*, const float*, const float*, const float*, float, float, float*,
                   int, int, int, int, void*);
-int np_router_dgate_parts(int);
+long long np_router_dgate_scratch(int, int, int);
 int np_router_dgate(const float*, const void*, float*, float*, float*, int, int, int, int, void*);
 int np_router_dx(const float*, const float*, void*, int, int, int, void*);
 int np_capacity_plan(const int*, int, int, int, int, int*, int*, int*, int*, int*, int*, int, long long*, void*);
@@ -443,7 +443,7 @@ struct Router : torch::autograd::Function<Router> {
                            ptr<float>(saved[5]), ptr<float>(da), 1.f, (float)ctx->saved_data["z"].toDouble(), ptr<float>(dl), T, E,
                            (int)cfg[0], (int)cfg[1], stream()), "router_bwd");
     const auto f32 = x2.options().dtype(at::kFloat);
-    Tensor scratch = at::empty({np_router_dgate_parts(T), (int64_t)E * D + (E + 3) / 4 * 4}, f32);
+    Tensor scratch = at::empty({np_router_dgate_scratch(T, D, E)}, f32);
     Tensor dgw = empty_like_of(x2, gate_w.sizes(), gate_w.scalar_type()), dgb = at::empty({E}, f32);
     if (T <= 0) {   // no tokens: the kernels below do nothing
       dgw.zero_();

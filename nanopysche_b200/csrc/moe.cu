@@ -290,97 +290,100 @@ __global__ void __launch_bounds__(128) router_bwd_kernel(const float* logits,
     if (e < E) dlogits[(size_t)t * E + e] = dl[e];
 }
 
-// partial[c, e, d] = sum over the chunk's tokens of dl[t, e] * x[t, d], and behind them partial[c, E * D + e] = sum of dl[t, e]. CTA =
-// 64 column threads (8 columns each) x 4 token lanes; a lane walks every fourth token of the chunk with four row loads in
-// flight, the lanes are summed through shared memory.
-template <int EB>
-__global__ void __launch_bounds__(256) router_dgate_kernel(const float* dl,
-                                                           const __nv_bfloat16* x,
-                                                           float* __restrict__ partial, int T, int D, int E,
-                                                           int chunk) {
+// partial[c, e, d] = sum over a chunk of 64 tokens of dl[t, e] * x[t, d] for EB experts a CTA. CTA = CT column threads (8 columns each) x 4
+// token lanes; a lane walks every fourth token of the chunk with U row loads in flight, the lanes are summed through shared
+// memory. Beside them the first sums of the column sums of dl (the bias gradient): virtual thread (g, e) of 1024 / E groups adds rows g, g +
+// groups, ... in four sums, into bias_part[g, e]. Bound by the chain of a lane's 16 tokens: a small batch takes narrow CTAs. us with the sum
+// over the chunks, wide CTAs and the bias gradient in a launch of its own / chunks of 16 tokens (another order of the sums) / now: 64 x 2048, 8
+// experts 10.9 / 4.2 / 6.5, 512 x 768 10.6 / 5.6 / 6.7, 1000 x 1024, 16 19.6 / 11.0 / 7.8, 4096 x 2048, 8 18.0 / 13.8 / 12.1.
+constexpr int DG_TOK = 64, DG_BIAS = 1024;
+template <int EB, int CT, int U>
+__global__ void __launch_bounds__(CT * 4) router_dgate_kernel(const float* dl, const __nv_bfloat16* x, float* __restrict__ partial,
+                                                              float* __restrict__ bias_part, int T, int D, int E) {
   np::pdl_begin();
-  __shared__ float red[2][64][EB * 8 + 1];
-  const int c = blockIdx.y;
-  const int t0 = c * chunk, t1 = min(T, t0 + chunk);
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-  const long long part = (long long)E * D + (E + 3) / 4 * 4;   // floats of a partial: whole vectors
-  if (blockIdx.x == 0) {   // column sums of dl (E <= 64)
-    __shared__ float s_b[4][64];
-    float s = 0.f;
-    if (tx < E) {
-#pragma unroll 4
-      for (int t = t0 + ty; t < t1; t += 4) s += dl[(size_t)t * E + tx];
-    }
-    s_b[ty][tx] = s;
-    __syncthreads();
-    if (ty == 0 && tx < E) partial[c * part + (long long)E * D + tx] = (s_b[0][tx] + s_b[1][tx]) + (s_b[2][tx] + s_b[3][tx]);
-  }
-  const int d = (blockIdx.x * 64 + tx) * 8;
+  __shared__ float red[2][CT][EB * 8 + 1];
+  __shared__ float s_dl[DG_TOK][EB];
+  const int c = blockIdx.y, e0 = blockIdx.z * EB;
+  const int t0 = c * DG_TOK, t1 = min(T, t0 + DG_TOK);
+  const int tx = threadIdx.x % CT, ty = threadIdx.x / CT;
+  const int d = (blockIdx.x * CT + tx) * 8;
   const bool col_ok = d < D;
-  for (int e0 = 0; e0 < E; e0 += EB) {
-    float acc[EB][8];
+  uint4 q[U];
+  auto load = [&](int tb) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      q[u] = col_ok && tb + 4 * u < t1 ? *reinterpret_cast<const uint4*>(x + (size_t)(tb + 4 * u) * D + d) : make_uint4(0, 0, 0, 0);
+  };
+  load(t0 + ty);
+  for (int i = threadIdx.x; i < (t1 - t0) * EB; i += CT * 4) {
+    const int e = e0 + i % EB;
+    s_dl[i / EB][i % EB] = e < E ? dl[(size_t)(t0 + i / EB) * E + e] : 0.f;
+  }
+  const int groups = DG_BIAS / E, ctas = gridDim.x * gridDim.y * gridDim.z;
+  for (int v = ((blockIdx.z * gridDim.y + c) * gridDim.x + blockIdx.x) * CT * 4 + threadIdx.x; v < groups * E; v += ctas * CT * 4) {
+    const int e = v % E;
+    float a4[4] = {0.f, 0.f, 0.f, 0.f};
+    int r = v / E;
+    for (; r + 3 * groups < T; r += 4 * groups) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a4[u] += dl[(size_t)(r + u * groups) * E + e];
+    }
+    for (; r < T; r += groups) a4[0] += dl[(size_t)r * E + e];
+    bias_part[v] = (a4[0] + a4[1]) + (a4[2] + a4[3]);
+  }
+  __syncthreads();
+  float acc[EB][8];
+#pragma unroll
+  for (int e = 0; e < EB; ++e)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[e][j] = 0.f;
+  for (int tb = t0 + ty; tb < t1; tb += 4 * U) {   // tokens tb, tb + 4, ...
+    if (tb != t0 + ty) load(tb);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (tb + 4 * u >= t1) break;
+      float2 a = np::unpack_bf16(q[u].x), b = np::unpack_bf16(q[u].y), cc = np::unpack_bf16(q[u].z), dd = np::unpack_bf16(q[u].w);
+      const float xv[8] = {a.x, a.y, b.x, b.y, cc.x, cc.y, dd.x, dd.y};
+#pragma unroll
+      for (int e = 0; e < EB; ++e) {
+        const float g = s_dl[tb + 4 * u - t0][e];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[e][j] += g * xv[j];
+      }
+    }
+  }
+  if (ty >= 2) {   // lanes 2, 3 -> lanes 0, 1
 #pragma unroll
     for (int e = 0; e < EB; ++e)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[e][j] = 0.f;
-    if (col_ok) {
-      for (int tb = t0 + ty; tb < t1; tb += 16) {   // tokens tb, tb+4, tb+8, tb+12
-        uint4 q[4];
+      for (int j = 0; j < 8; ++j) red[ty - 2][tx][e * 8 + j] = acc[e][j];
+  }
+  __syncthreads();
+  if (ty < 2) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          q[u] = (tb + 4 * u < t1) ? *reinterpret_cast<const uint4*>(x + (size_t)(tb + 4 * u) * D + d)
-                                   : make_uint4(0, 0, 0, 0);
+    for (int e = 0; e < EB; ++e)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (tb + 4 * u >= t1) break;
-          float2 a = np::unpack_bf16(q[u].x), b = np::unpack_bf16(q[u].y), cc = np::unpack_bf16(q[u].z),
-                 dd = np::unpack_bf16(q[u].w);
-          const float xv[8] = {a.x, a.y, b.x, b.y, cc.x, cc.y, dd.x, dd.y};
+      for (int j = 0; j < 8; ++j) acc[e][j] += red[ty][tx][e * 8 + j];
+  }
+  __syncthreads();
+  if (ty == 1) {   // lane 1 -> lane 0
 #pragma unroll
-          for (int e = 0; e < EB; ++e) {
-            if (e0 + e < E) {
-              const float g = dl[(size_t)(tb + 4 * u) * E + e0 + e];
+    for (int e = 0; e < EB; ++e)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) acc[e][j] += g * xv[j];
-            }
-          }
-        }
+      for (int j = 0; j < 8; ++j) red[0][tx][e * 8 + j] = acc[e][j];
+  }
+  __syncthreads();
+  if (ty == 0 && col_ok) {
+#pragma unroll
+    for (int e = 0; e < EB; ++e) {
+      if (e0 + e < E) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[e][j] += red[0][tx][e * 8 + j];
+        float* dst = partial + ((size_t)c * E + e0 + e) * D + d;
+        *reinterpret_cast<float4*>(dst) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[e][4], acc[e][5], acc[e][6], acc[e][7]);
       }
     }
-    if (ty >= 2) {   // lanes 2, 3 -> lanes 0, 1
-#pragma unroll
-      for (int e = 0; e < EB; ++e)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) red[ty - 2][tx][e * 8 + j] = acc[e][j];
-    }
-    __syncthreads();
-    if (ty < 2) {
-#pragma unroll
-      for (int e = 0; e < EB; ++e)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[e][j] += red[ty][tx][e * 8 + j];
-    }
-    __syncthreads();
-    if (ty == 1) {   // lane 1 -> lane 0
-#pragma unroll
-      for (int e = 0; e < EB; ++e)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) red[0][tx][e * 8 + j] = acc[e][j];
-    }
-    __syncthreads();
-    if (ty == 0 && col_ok) {
-#pragma unroll
-      for (int e = 0; e < EB; ++e) {
-        if (e0 + e < E) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[e][j] += red[0][tx][e * 8 + j];
-          float* dst = partial + c * part + (size_t)(e0 + e) * D + d;
-          *reinterpret_cast<float4*>(dst) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
-          *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[e][4], acc[e][5], acc[e][6], acc[e][7]);
-        }
-      }
-    }
-    __syncthreads();
   }
 }
 
@@ -454,12 +457,26 @@ __global__ void __launch_bounds__(256, 2) router_dx_reg_kernel(const float* dl, 
   }
 }
 
-// column sums of `parts` rows (`cols` floats apart): the first n0 columns to out0, n1 behind them to out1 (added with `accumulate`)
-__global__ void colsum2_kernel(const float* partial, float* __restrict__ out0, float* __restrict__ out1, int parts, long long cols,
-                               long long n0, int n1, int accumulate) {
+// out[c] (+)= column sums of `parts` rows of `cols` floats, 64 columns a CTA; the CTA behind the last adds up the bias gradient:
+// bias_out[e] (+)= bias_part[0 .. groups, e] one after the other
+__global__ void __launch_bounds__(64) router_dgate_sum_kernel(const float* partial, float* __restrict__ out, int parts, long long cols,
+                                                              const float* bias_part, float* __restrict__ bias_out, int E, int accumulate) {
   np::pdl_begin();
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= n0 + n1) return;
+  if (blockIdx.x * 64ll >= cols) {
+    __shared__ float s_part[DG_BIAS];
+    const int groups = DG_BIAS / E;
+    for (int i = threadIdx.x; i < groups * E; i += 64) s_part[i] = bias_part[i];
+    __syncthreads();
+    if ((int)threadIdx.x < E) {
+      float s = 0.f;
+#pragma unroll 8
+      for (int g = 0; g < groups; ++g) s += s_part[g * E + threadIdx.x];
+      bias_out[threadIdx.x] = accumulate ? bias_out[threadIdx.x] + s : s;
+    }
+    return;
+  }
+  const long long c = blockIdx.x * 64ll + threadIdx.x;
+  if (c >= cols) return;
   float a8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   int p = 0;
   for (; p + 7 < parts; p += 8) {   // eight independent loads in flight
@@ -468,8 +485,7 @@ __global__ void colsum2_kernel(const float* partial, float* __restrict__ out0, f
   }
   for (; p < parts; ++p) a8[0] += partial[(size_t)p * cols + c];
   const float s = ((a8[0] + a8[1]) + (a8[2] + a8[3])) + ((a8[4] + a8[5]) + (a8[6] + a8[7]));
-  float* out = c < n0 ? out0 + c : out1 + (c - n0);
-  *out = accumulate ? *out + s : s;
+  out[c] = accumulate ? out[c] + s : s;
 }
 
 // ------------------------------------------------------------------ capacity / positions
@@ -1006,22 +1022,23 @@ NP_API int np_router_bwd(const float* logits, const float* score_bias, const flo
   CHECK_LAUNCH();
 }
 
-// Tokens of a partial sum: few enough that a small batch has CTAs for the chip (512 x 768, 8 experts, with the sum over the parts: 64 tokens 12.3 us, 16 tokens 7.5), many
-// enough that the partials of a large one stay small beside x.
-static int dgate_chunk(int T) { return T <= 1024 ? 16 : 64; }
-NP_API int np_router_dgate_parts(int T) { return (T + dgate_chunk(T) - 1) / dgate_chunk(T); }
-// scratch: fp32 [np_router_dgate_parts(T), E * D + E, the latter in whole fours]; dwg[E, D] (+)= dl^T x ; dbias[E] (+)= column sums of dl.
+// Floats of the scratch buffer of np_router_dgate
+NP_API long long np_router_dgate_scratch(int T, int D, int E) { return (long long)((T + DG_TOK - 1) / DG_TOK) * E * D + DG_BIAS; }
+// dwg[E, D] (+)= dl^T x ; dbias[E] (+)= column sums of dl.
 NP_API int np_router_dgate(const float* dl, const void* x, float* dwg, float* dbias, float* scratch, int T, int D,
                            int E, int accumulate, void* stream) {
   if (D % 8 || E > MAX_E) return 1;
   if (T <= 0) return 0;
   cudaStream_t s = (cudaStream_t)stream;
-  const int parts = np_router_dgate_parts(T);
-  dim3 grid((D / 8 + 63) / 64, parts);
-  np_launch(router_dgate_kernel<8>, grid, 256, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch, T, D, E, dgate_chunk(T));
+  const int parts = (T + DG_TOK - 1) / DG_TOK;
   const long long n = (long long)E * D;
-  np_launch(colsum2_kernel, (int)((n + E + 63) / 64), 64, 0, s, 1, scratch, dwg, dbias, parts, n + (E + 3) / 4 * 4, n,
-            dbias ? E : 0, accumulate);
+  float* bias_part = scratch + parts * n;
+  auto run = [&](auto kernel, int ct) {
+    np_launch(kernel, dim3((D / 8 + ct - 1) / ct, parts, (E + 7) / 8), ct * 4, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch, bias_part, T, D, E);
+  };
+  if (T <= 1024) run(router_dgate_kernel<8, 16, 8>, 16);
+  else run(router_dgate_kernel<8, 64, 4>, 64);
+  np_launch(router_dgate_sum_kernel, (unsigned)((n + 63) / 64 + (dbias ? 1 : 0)), 64, 0, s, 1, scratch, dwg, parts, n, bias_part, dbias, E, accumulate);
   CHECK_LAUNCH();
 }
 

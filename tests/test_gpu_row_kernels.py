@@ -531,3 +531,40 @@ def test_sum_of_squares_order(n):
     for o in (16, 8, 4, 2, 1):
         s = s + s[..., i ^ o]
     assert torch.equal(got.cpu(), s[:, 0])
+
+
+# the order of the gate's gradient: chunks of 64 tokens, of a chunk every fourth token by one lane, lanes 0 + 2 and 1 + 3, the chunks in eight
+# sums; the bias gradient in 1024 / E groups of rows. Both sizes of CTA, one and more passes over the experts, a last chunk that is short
+@pytest.mark.parametrize("T,D,E", [(1, 8, 1), (70, 136, 3), (600, 16, 8), (1025, 8, 17), (1500, 24, 5)])
+def test_router_gate_gradient_order(T, D, E):
+    from nanopysche_b200.ops import _lib
+
+    torch.manual_seed(T)
+    dl, x = torch.randn(T, E) * 2.0 ** torch.randint(-4, 5, (T, 1)), torch.randn(T, D).bfloat16()
+    w, b = torch.full((2, E, D), 0.5, device="cuda"), torch.full((2, E), 0.5, device="cuda")
+    scratch = torch.empty((T + 63) // 64 * E * D + 1024, device="cuda")
+    for acc in (0, 1):
+        _lib.call("router_dgate", dl.cuda(), x.cuda(), w[acc], b[acc], scratch, T, D, E, acc)
+    chunks = (T + 63) // 64
+    pad = lambda t: torch.nn.functional.pad(t, (0, 0, 0, chunks * 64 - T)).view(chunks, 16, 4, -1)      # noqa: E731
+    l, v = pad(dl).double(), pad(x.float()).double()
+    part = torch.zeros(chunks, 4, E, D)
+    for i in range(16):                 # one rounding for each product and its addition
+        part = (part.double() + l[:, i, :, :, None] * v[:, i, :, None, :]).float()
+    part = (part[:, 0] + part[:, 2]) + (part[:, 1] + part[:, 3])
+    a = torch.zeros(8, E, D)
+    whole = chunks // 8 * 8
+    for p in range(chunks):
+        a[p % 8 if p < whole else 0] += part[p]
+    want = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]))
+    groups = 1024 // E
+    a4 = torch.zeros(groups, 4, E)
+    for r in range(T):
+        g, i = r % groups, r // groups
+        rows = (T - g + groups - 1) // groups          # of this group
+        a4[g, i % 4 if i < rows // 4 * 4 else 0] += dl[r]
+    s = (a4[:, 0] + a4[:, 1]) + (a4[:, 2] + a4[:, 3])
+    bias = torch.zeros(E)
+    for g in range(groups):
+        bias = bias + s[g]
+    assert torch.equal(w.cpu(), torch.stack([want, want + 0.5])) and torch.equal(b.cpu(), torch.stack([bias, bias + 0.5]))
