@@ -1321,6 +1321,19 @@ NP_API int np_sumsq(const float* x, long long n, float* partial, void* stream) {
   np_launch(sumsq_kernel, np_sumsq_parts(), NT, 0, (cudaStream_t)stream, 1, x, n, partial);
   CHECK_LAUNCH();
 }
+// dst[0..2] = a, b, c by value: the numbers of the call, whatever the host does before the stream gets here
+namespace {
+__global__ void store3_kernel(float* dst, float a, float b, float c) {
+  np::pdl_begin();
+  dst[0] = a;
+  dst[1] = b;
+  dst[2] = c;
+}
+}  // namespace
+NP_API int np_store3(float* dst, float a, float b, float c, void* stream) {
+  np_launch(store3_kernel, 1, 1, 0, (cudaStream_t)stream, 1, dst, a, b, c);
+  CHECK_LAUNCH();
+}
 // Embedding backward straight into the fp32 gradient arena: grad[ids[t], :] += dy[t, :]. One thread per four
 // columns of a token row, one 16-byte vector reduction each; rows of ids outside [0, V) are skipped.
 namespace {

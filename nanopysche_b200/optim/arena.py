@@ -447,7 +447,7 @@ class ArenaAdamW(torch.optim.Optimizer):
             zp = _lib.lib().np_zero_parts()
             self._partial = torch.zeros(nreg * max(self._parts, zp), device=dev, dtype=torch.float32)
         # [lr, 1 - b1^t, 1 - b2^t]: read by the kernels from device memory so a captured step replays
-        # with the current schedule; refreshed by ``update_hyper()`` (a pinned-host -> device copy)
+        # with the current schedule; refreshed by ``update_hyper()``
         self._hyper = torch.zeros(3, device=dev, dtype=torch.float32)
         self._hyper_host = torch.zeros(3, dtype=torch.float32).pin_memory() if self._cuda else torch.zeros(3)
         self.post_step_hooks = []  # callables run at the end of every step (e.g. epoch bookkeeping)
@@ -482,7 +482,11 @@ class ArenaAdamW(torch.optim.Optimizer):
         self._hyper_host[0] = g["lr"]
         self._hyper_host[1] = 1.0 - b1 ** self.step_count
         self._hyper_host[2] = 1.0 - b2 ** self.step_count
-        self._hyper.copy_(self._hyper_host, non_blocking=True)
+        if self._cuda and not torch.cuda.is_current_stream_capturing():
+            # by value: the host may be steps ahead of the stream, and a copy from the pinned words would read a later step's
+            _lib.call("store3", self._hyper, *self._hyper_host.tolist())
+        else:   # in a capture: the replays read the words as they are then
+            self._hyper.copy_(self._hyper_host, non_blocking=True)
 
     @torch.no_grad()
     def step(self, closure=None, _hyper_ready: bool = False):

@@ -111,3 +111,48 @@ def test_graphed_step_matches_eager_and_fp32_pytorch():
         assert abs(a - c) <= tol * abs(c), (i, l_graph, l_ref)
     assert l_graph[0] < 10.6 and l_graph[-1] < l_graph[0] - 3.0, l_graph   # starts near ln(V), memorises the batch
     assert l_ref[-1] < l_ref[0] - 3.0 and l_eager[-1] < l_eager[0] - 3.0
+
+
+def _small_step(seed, vocab=512):
+    from nanopysche_b200.config import TransformerConfig
+    from nanopysche_b200.engine import prepare_training
+
+    torch.manual_seed(seed)
+    model = TransformerConfig(vocab_size=vocab, d_model=128, n_layers=1, n_heads=2, n_kv_heads=2, ffn_hidden=256, max_seq_len=64,
+                              qk_norm=False).build(dtype=torch.bfloat16, init_device="cuda")
+    opt, _ = prepare_training(model, lr=1e-3, weight_decay=0.1, max_grad_norm=1.0)
+    return model, opt, torch.randint(0, vocab, (2, 64), device="cuda")
+
+
+def test_schedule_of_a_step_is_the_one_it_was_given():
+    """The host may be many steps ahead of the stream: every step sees its own learning rate and bias corrections."""
+    _, opt, _ = _small_step(0)
+    log = torch.empty(40, 3, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda._sleep(50_000_000)      # the stream is behind
+    for i in range(len(log)):
+        opt.param_groups[0]["lr"] = float(i)
+        opt.update_hyper()
+        log[i].copy_(opt._hyper)
+    t = torch.arange(1, len(log) + 1).double()
+    want = torch.stack([t - 1, 1 - 0.9 ** t, 1 - 0.95 ** t], 1).float()
+    assert torch.equal(log.cpu(), want)
+
+
+def test_replays_without_a_wait_between_them():
+    from nanopysche_b200.engine import GraphedTrainStep
+
+    weights = []
+    for wait in (False, True):
+        model, opt, ids = _small_step(1)
+        g = GraphedTrainStep(model, opt, ids, warmup=1).capture()
+        torch.cuda.synchronize()
+        if not wait:
+            torch.cuda._sleep(50_000_000)
+        for i in range(30):
+            opt.param_groups[0]["lr"] = 1e-3 * (i % 7)
+            g.step(ids)
+            if wait:
+                torch.cuda.synchronize()
+        weights.append([p.detach().clone() for p in model.parameters()])
+    assert all(torch.equal(a, b) for a, b in zip(*weights))
