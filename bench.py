@@ -240,7 +240,7 @@ def run_ours(args, rank, local, world, dev, c):
         # the whole step (forward + backward + clip + AdamW) replayed as one CUDA graph; its two eager warm-up
         # steps run at the schedule's first learning rate (0)
         l0 = _lib.LAUNCHES
-        graphed = GraphedTrainStep(model, opt, devb[0], warmup=2).capture()
+        graphed = GraphedTrainStep(model, opt, devb[0], warmup=2).capture(count_recording=False)
         per_step = (_lib.LAUNCHES - l0) // 3  # two eager warm-up steps + the captured one
 
     def train_step(ids):

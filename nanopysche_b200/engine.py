@@ -123,7 +123,11 @@ class GraphedTrainStep:
         self.opt.zero_grad(set_to_none=True)
         return out["loss"].detach()
 
-    def capture(self):
+    def capture(self, count_recording: bool = True):
+        """Record the step. Recording takes no step, but by default it counts as one: the bias corrections of the replays are
+        those of one step later than an eager run's (updates 7 percent off in the fourth step, less in every later one), and
+        ``step_count`` is one too high. Runs that were recorded so go on as they are; ``count_recording=False`` gives the losses of
+        the eager run bit for bit."""
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -131,7 +135,7 @@ class GraphedTrainStep:
                 self._eager(False)
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
-        self.opt.update_hyper()
+        self.opt.update_hyper(advance=count_recording)
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self.static_loss = self._eager(True)

@@ -156,3 +156,28 @@ def test_replays_without_a_wait_between_them():
                 torch.cuda.synchronize()
         weights.append([p.detach().clone() for p in model.parameters()])
     assert all(torch.equal(a, b) for a, b in zip(*weights))
+
+
+def test_recording_that_does_not_count_gives_the_eager_steps():
+    from nanopysche_b200.engine import GraphedTrainStep
+
+    runs = []
+    for graphed in (False, True):
+        model, opt, ids = _small_step(2)
+        losses = []
+        if graphed:
+            g = GraphedTrainStep(model, opt, ids, warmup=2).capture(count_recording=False)
+            assert opt.step_count == 2
+            for _ in range(6):
+                losses.append(g.step(ids).item())
+        else:
+            for i in range(8):
+                loss = model(ids, labels=ids)["loss"]
+                loss.backward()
+                opt.step()
+                opt.zero_grad()
+                if i >= 2:
+                    losses.append(loss.item())
+        assert opt.step_count == 8
+        runs.append(losses)
+    assert runs[0] == runs[1] and runs[0][-1] < runs[0][0]
