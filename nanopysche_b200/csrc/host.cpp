@@ -463,7 +463,8 @@ struct Router : torch::autograd::Function<Router> {
   }
 };
 
-// What the launches of FusedMoERuntime (ops/moe.py) take from it: sizes, buffers and tables that it keeps for its whole life
+// What the launches of FusedMoERuntime (ops/moe.py) take from it: sizes, buffers and tables that it keeps for its whole life. One rank:
+// the form with peers is the Python one.
 struct MoeRuntime : torch::CustomClassHolder {
   int64_t T, D, H, E, K, N, rank, E_local, R, bpr, rows_total, blocks, capacity, max_ctas, wait_ns;
   std::vector<Tensor> recv_x, ret_y, p_recv_x, p_ret_y;
@@ -484,6 +485,7 @@ struct MoeRuntime : torch::CustomClassHolder {
     p_row_dst = ten("p_row_dst"); p_mblk_rows = ten("p_mblk_rows"); p_src_blocks = ten("p_src_blocks");
     p_dispatch_flags = ten("p_dispatch_flags"); p_done_flag = ten("p_done_flag"); mblk_group = ten("mblk_group");
     mblk_flag = ten("mblk_flag"); done_counters = ten("done_counters"); dispatch_ctr = ten("dispatch_ctr");
+    require(N == 1, "the native form of the expert layer is that of one rank");
     heap = rt.attr("heap");
     epoch_base = heap.attr("epoch_base").cast<Tensor>();
     owner = py::module_::import("weakref").attr("ref")(rt);
@@ -539,7 +541,7 @@ struct MoeRuntime : torch::CustomClassHolder {
   void push_to(NpGemmArgs& g, const Tensor& peers, int epoch) const {   // output rows go back to their sources
     g.row_dst = (const long long*)row_dst.data_ptr(); g.peer_base = (void* const*)peers.data_ptr();
     g.done_counters = ptr<int>(done_counters); g.done_expected = ptr<int>(src_blocks);
-    g.done_flag_ptr = (int* const*)p_done_flag.data_ptr(); g.epoch = epoch; g.ldc = g.N; g.local_push = N == 1;
+    g.done_flag_ptr = (int* const*)p_done_flag.data_ptr(); g.epoch = epoch; g.ldc = g.N; g.local_push = 1;
   }
   // A [rows, M (x outputs)] and B [rows, N] contracted over the rows of every expert, into the fp32 outputs of M rows per expert
   NpGemmArgs by_expert(const Tensor& A, const Tensor& B, int64_t M, int64_t n, const std::vector<Tensor>& outs, bool add) const {
@@ -551,16 +553,11 @@ struct MoeRuntime : torch::CustomClassHolder {
     g.num_groups = (int)E_local; g.blocks_per_group = (int)(N * bpr); g.group_stride_c = M * n;
     return g;
   }
-  // A product over the dispatched rows and the weight gradient beside it: together when this rank is the only one (the rows are
-  // there when the dispatch kernel has ended; rows of peers are waited for by the first product alone). The six expert GEMMs,
-  // us, apart / paired: 4096 tokens, 8 experts of 2048 x 2816 606 / 525, 512 of 768 x 2048 199 / 174, 2472, 16 of 1024 x 2816 417 / 382.
+  // A product over the dispatched rows and the weight gradient beside it, together: without peers the rows are there when the dispatch
+  // kernel has ended. The six expert GEMMs, us, apart / paired: 4096 tokens, 8 experts of 2048 x 2816 606 / 525, 512 of 768 x 2048
+  // 199 / 174, 2472, 16 of 1024 x 2816 417 / 382.
   void both(const NpGemmArgs& rows, const NpGemmArgs& experts) const {
-    if (N == 1) {
-      launched(np_gemm_bf16_two(&rows, &experts, stream()), "grouped_gemm and grouped_wgrad");
-    } else {
-      launched(np_gemm_bf16(&rows, stream()), "grouped_gemm");
-      launched(np_gemm_bf16(&experts, stream()), "grouped_wgrad");
-    }
+    launched(np_gemm_bf16_two(&rows, &experts, stream()), "grouped_gemm and grouped_wgrad");
   }
 };
 
@@ -594,7 +591,7 @@ bool same_main_grad(const Tensor& a, const Tensor& b) {
   return some(attr(a, s_main_grad)) == some(attr(b, s_main_grad)) && truthy(attr(a, s_dirty)) == truthy(attr(b, s_dirty));
 }
 
-// The bf16 form of ops.moe._FusedMoE: plan, dispatch, expert GEMMs, combine, and their mirror. Returns the output and the tokens that
+// The bf16 form of ops.moe._FusedMoE on one rank: plan, dispatch, expert GEMMs, combine, and their mirror. Returns the output and the tokens that
 // each expert dropped.
 struct FusedMoE : torch::autograd::Function<FusedMoE> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weights, const Tensor& idx, const Tensor& w1,

@@ -347,8 +347,8 @@ class FusedMoERuntime:
 
 
 # ------------------------------------------------------------------------------------------------ the layer
-class _FusedMoEFp8(torch.autograd.Function):
-    """The FP8-Flow-MoE form of the layer (the bf16 form: ``FusedMoE`` in csrc/host.cpp)."""
+class _FusedMoE(torch.autograd.Function):
+    """The layer with FP8-Flow-MoE experts or with peers (bf16 on one rank: ``FusedMoE`` in csrc/host.cpp, the same kernels)."""
 
     @staticmethod
     def forward(ctx, x, weights, indices32, w1, w3, w2, rt: FusedMoERuntime, layer: int, stats_mod, shared=None):
@@ -366,20 +366,30 @@ class _FusedMoEFp8(torch.autograd.Function):
                   rt.N, None if stats_mod is None else stats_mod._drop_stats(dev))
         e1 = rt.next_epoch()
         gu = torch.empty((rt.rows_total, 2 * H), device=dev, dtype=torch.bfloat16)
-        # FP8-Flow-MoE forward: rows travel as e4m3 with 1x128 power-of-two scales (quantised inside the dispatch
-        # kernel), the expert weights are e4m3 with 128x128 scales (made once per optimizer step), both expert
-        # GEMMs run on the block-scaled tcgen05 path with the scaling done by the tensor core: one gate|up GEMM,
-        # SwiGLU + re-quantisation in one pass, and the down GEMM pushing rows back to their sources
-        from .gemm_mxfp8 import flow_quantize_act
+        if rt.fp8:
+            # FP8-Flow-MoE forward: rows travel as e4m3 with 1x128 power-of-two scales (quantised inside the dispatch
+            # kernel), the expert weights are e4m3 with 128x128 scales (made once per optimizer step), both expert
+            # GEMMs run on the block-scaled tcgen05 path with the scaling done by the tensor core: one gate|up GEMM,
+            # SwiGLU + re-quantisation in one pass, and the down GEMM pushing rows back to their sources
+            from .gemm_mxfp8 import flow_quantize_act
 
-        w13q, s13, w2q, s2 = rt.quantised_weights(layer, w1, w3, w2)
-        rt.dispatch(x2, indices32, slot_pos, counts_kept, None, rt.p_recv_xq[layer], e1,
-                    p_scales=rt.p_recv_xs[layer])
-        xq, xs = rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer]
-        rt.grouped_gemm_fp8(xq, xs, w13q, s13, N=2 * H, out=gu, wait_epoch=e1)
-        h = torch.empty((rt.rows_total, H), device=dev, dtype=torch.bfloat16)
-        hq, hs = flow_quantize_act(gu, swiglu=True, h_out=h)
-        rt.grouped_gemm_fp8(hq, hs, w2q, s2, N=D, push_ptrs=rt.p_ret_y[layer], push_epoch=e1)
+            w13q, s13, w2q, s2 = rt.quantised_weights(layer, w1, w3, w2)
+            rt.dispatch(x2, indices32, slot_pos, counts_kept, None, rt.p_recv_xq[layer], e1,
+                        p_scales=rt.p_recv_xs[layer])
+            xq, xs = rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer]
+            rt.grouped_gemm_fp8(xq, xs, w13q, s13, N=2 * H, out=gu, wait_epoch=e1)
+            h = torch.empty((rt.rows_total, H), device=dev, dtype=torch.bfloat16)
+            hq, hs = flow_quantize_act(gu, swiglu=True, h_out=h)
+            rt.grouped_gemm_fp8(hq, hs, w2q, s2, N=D, push_ptrs=rt.p_ret_y[layer], push_epoch=e1)
+        else:
+            rt.dispatch(x2, indices32, slot_pos, counts_kept, None, rt.p_recv_x[layer], e1)
+            # experts: [gate|up] GEMM with SwiGLU epilogue, waits per block on the source's arrival flag
+            h = torch.empty((rt.rows_total, H), device=dev, dtype=torch.bfloat16)
+            rt.grouped_gemm(rt.recv_x[layer], w1, N=H, K=D, b_mn=False, group_stride_b=H, out=h, B2=w3, C2=gu,
+                            wait_epoch=e1)
+            # down projection (w2 is stored [H, D] per expert: MN-major B), rows pushed back to their sources
+            rt.grouped_gemm(h, w2, N=D, K=H, b_mn=True, group_stride_b=H, push_ptrs=rt.p_ret_y[layer],
+                            push_epoch=e1)
         out = torch.empty((T, D), device=dev, dtype=torch.bfloat16)
         add1 = None
         if shared is not None:
@@ -415,10 +425,12 @@ class _FusedMoEFp8(torch.autograd.Function):
         # dH = dY @ w2^T  (w2 [H, D] per expert is K-major for this contraction), taken to [dG | dU] in the epilogue
         dgu = rt.grouped_gemm(rt.recv_g, w2, N=H, K=D, b_mn=False, group_stride_b=H, wait_epoch=e2, glu_of=gu)
         dw2 = rt.grouped_wgrad(ctx.saved_tensors[10], rt.recv_g, w2, M=H, N=D)
-        # the rows arrived as e4m3: dequantise once for the (bf16) weight-gradient GEMMs
-        from .gemm_mxfp8 import mx_dequantize_bf16
+        if rt.fp8:  # the rows arrived as e4m3: dequantise once for the (bf16) weight-gradient GEMMs
+            from .gemm_mxfp8 import mx_dequantize_bf16
 
-        xr = mx_dequantize_bf16(rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer])
+            xr = mx_dequantize_bf16(rt.recv_xq[layer].view(torch.float8_e4m3fn), rt.recv_xs[layer])
+        else:
+            xr = rt.recv_x[layer]
         dw1, dw3 = rt.grouped_wgrad(dgu, xr, w1, M=H, N=D, w_second=w3)
         # dX = [dG | dU] @ [w1; w3], one contraction over both weights (no bf16 partial result in between), pushed back to
         # the sources. H is a multiple of 256 (MoEBase), the K steps of 64 never straddle the two.
@@ -461,6 +473,11 @@ def build_runtime(moe_modules, *, tokens: int, group=None, device=None) -> Fused
     return rt
 
 
+def _native_form(rt) -> bool:
+    """bf16 experts on one rank run in csrc/host.cpp; the forms with peers or e4m3 operands in ``_FusedMoE``."""
+    return rt.N == 1 and not rt.fp8
+
+
 def fused_moe_forward(mod, x: torch.Tensor) -> torch.Tensor:
     """Forward of ``MoEBase`` on the fused path (``x``: [B, S, D] bf16 on CUDA)."""
     rt: FusedMoERuntime = mod._fused_runtime
@@ -485,8 +502,8 @@ def fused_moe_forward(mod, x: torch.Tensor) -> torch.Tensor:
     shared = mod.shared_expert(x) if mod.shared_expert is not None else None
     with _lib.nvtx_range("fused_moe"):
         w, idx = w.reshape(B * S, -1), idx.reshape(B * S, -1)
-        if rt.fp8:
-            return _FusedMoEFp8.apply(x, w, idx, mod.w1, mod.w3, mod.w2, rt, layer, mod, shared)
+        if not _native_form(rt):
+            return _FusedMoE.apply(x, w, idx, mod.w1, mod.w3, mod.w2, rt, layer, mod, shared)
         out, mod._per_expert_drop_counts = _lib.host().fused_moe(x, w, idx, mod.w1, mod.w3, mod.w2, rt.native(), layer,
                                                                  mod._drop_stats(x.device), shared)
         return out

@@ -568,3 +568,36 @@ def test_router_gate_gradient_order(T, D, E):
     for g in range(groups):
         bias = bias + s[g]
     assert torch.equal(w.cpu(), torch.stack([want, want + 0.5])) and torch.equal(b.cpu(), torch.stack([bias, bias + 0.5]))
+
+
+# the Python form of the expert layer, which runs with peers, and the native one: the same kernels and bits on one rank. Capacity with drops,
+# gradients into main_grad and into tensors, a shared expert's output
+@pytest.mark.parametrize("T,E,K,capacity,arena,shared", [(520, 8, 2, None, True, 0), (1030, 4, 2, 1.25, True, 1), (300, 8, 1, 1.5, False, 0)])
+def test_expert_layer_forms_agree(T, E, K, capacity, arena, shared, monkeypatch):
+    from nanopysche_b200.engine import prepare_training
+    from nanopysche_b200.models.moe import MoEBase
+    from nanopysche_b200.ops import moe as ops
+
+    D, H = 256, 512
+    out = []
+    for native in (True, False):
+        monkeypatch.setattr(ops, "_native_form", lambda rt: native)
+        torch.manual_seed(T)
+        m = MoEBase(d_model=D, hidden_size=H, num_experts=E, top_k=K, capacity_factor=capacity, shared_expert=bool(shared),
+                    dtype=torch.bfloat16, device="cuda")
+        with torch.no_grad():
+            for w in m.parameters():
+                w.normal_(0, 0.05)
+        if arena:
+            _, a = prepare_training(m, tokens_per_rank=T, lr=1e-3)
+        else:
+            ops.build_runtime([m], tokens=T, device=torch.device("cuda"))
+        x = torch.randn(1, T, D, device="cuda").bfloat16().requires_grad_(True)
+        dy = torch.randn(1, T, D, device="cuda").bfloat16()
+        for _ in range(2):
+            x.grad = None
+            y = m(x)
+            y.backward(dy)
+        grads = dict(a.named_main_grads()) if arena else {n: p.grad for n, p in m.named_parameters()}
+        out.append([y, x.grad, m._per_expert_drop_counts, *(g for g in grads.values() if g is not None)])
+    assert len(out[0]) == len(out[1]) > 5 and all(torch.equal(p, q) for p, q in zip(*out))

@@ -727,3 +727,13 @@ def _cp_moe_worker(rank, world):
 
 def test_context_parallel_with_moe_matches_single_process():
     assert all(run_distributed(_cp_moe_worker, 2))
+
+
+def test_expert_layer_with_peers_runs_the_python_form():
+    """The native form of the expert layer is that of one rank with bf16 experts."""
+    from types import SimpleNamespace
+
+    from nanopysche_b200.ops.moe import _native_form
+
+    assert [_native_form(SimpleNamespace(N=n, fp8=f)) for n, f in ((1, False), (2, False), (8, False), (1, True), (2, True))] == \
+        [True, False, False, False, False]
