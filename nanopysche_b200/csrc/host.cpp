@@ -499,10 +499,11 @@ struct MoeRuntime : torch::CustomClassHolder {
     py::gil_scoped_acquire gil;
     return heap.attr("next_epoch")().cast<int>();
   }
-  void pushed() const {   // the counters of the last dispatch are used up
+  // the counters of a product that pushes its rows: once behind every dispatch, the runtime refuses more
+  int* push_counters() const {
     py::gil_scoped_acquire gil;
     py::object rt = owner();
-    if (!rt.is_none()) rt.attr("_may_push") = false;
+    return rt.is_none() ? ptr<int>(done_counters) : (int*)rt.attr("_push_counters")().cast<uintptr_t>();
   }
   void dispatch(const Tensor& x, const Tensor& idx, const Tensor& slot_pos, const Tensor& counts, const Tensor& scale, const Tensor& rows,
                 int epoch) const {
@@ -517,6 +518,9 @@ struct MoeRuntime : torch::CustomClassHolder {
     a.done_ctr = ptr<int>(dispatch_ctr); a.epoch = epoch; a.write_meta = 1; a.max_ctas = (int)max_ctas;
     a.epoch_base = ptr<int>(epoch_base); a.zero_ctr = ptr<int>(done_counters);
     launched(np_ep_dispatch(&a, stream()), "ep_dispatch");
+    py::gil_scoped_acquire gil;
+    py::object rt = owner();
+    if (!rt.is_none()) rt.attr("_may_push") = true;
   }
   void combine(const Tensor& rows, const Tensor& slot_pos, const Tensor& weights, const Tensor& add, const Tensor& out, const Tensor& sent,
                int epoch) const {
@@ -540,7 +544,7 @@ struct MoeRuntime : torch::CustomClassHolder {
   }
   void push_to(NpGemmArgs& g, const Tensor& peers, int epoch) const {   // output rows go back to their sources
     g.row_dst = (const long long*)row_dst.data_ptr(); g.peer_base = (void* const*)peers.data_ptr();
-    g.done_counters = ptr<int>(done_counters); g.done_expected = ptr<int>(src_blocks);
+    g.done_counters = push_counters(); g.done_expected = ptr<int>(src_blocks);
     g.done_flag_ptr = (int* const*)p_done_flag.data_ptr(); g.epoch = epoch; g.ldc = g.N; g.local_push = 1;
   }
   // A [rows, M (x outputs)] and B [rows, N] contracted over the rows of every expert, into the fp32 outputs of M rows per expert
@@ -591,8 +595,8 @@ bool same_main_grad(const Tensor& a, const Tensor& b) {
   return some(attr(a, s_main_grad)) == some(attr(b, s_main_grad)) && truthy(attr(a, s_dirty)) == truthy(attr(b, s_dirty));
 }
 
-// The bf16 form of ops.moe._FusedMoE on one rank: plan, dispatch, expert GEMMs, combine, and their mirror. Returns the output and the tokens that
-// each expert dropped.
+// The bf16 form of ops.moe._FusedMoE on one rank: plan, dispatch, expert GEMMs, combine, and their mirror. Returns the output and the
+// tokens that each expert dropped.
 struct FusedMoE : torch::autograd::Function<FusedMoE> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weights, const Tensor& idx, const Tensor& w1,
                                const Tensor& w3, const Tensor& w2, c10::intrusive_ptr<MoeRuntime> rt, int64_t layer,
@@ -617,7 +621,6 @@ struct FusedMoE : torch::autograd::Function<FusedMoE> {
     g = rt->by_rows(h, w2, D, H, true);
     rt->push_to(g, rt->p_ret_y[layer], epoch);
     launched(np_gemm_bf16(&g, stream()), "grouped_gemm");
-    rt->pushed();
     Tensor out = at::empty({T, D}, b16), add;
     // the shared expert's output joins in the combine pass; a token dropped by the capacity rule gets no MoE output at all,
     // shared expert included (reference: model/moe.py:1383-1390)
@@ -682,7 +685,6 @@ struct FusedMoE : torch::autograd::Function<FusedMoE> {
         (i ? dw3 : dw1) = d.grads[0];
       }
     }
-    rt->pushed();
     Tensor dx = at::empty({T, D}, b16);
     rt->combine(rt->ret_g, slot_pos, Tensor(), Tensor(), dx, sent, epoch);
     res[0] = dx.view(shape); res[1] = dweights; res[3] = dw1; res[4] = dw3; res[5] = d2.grads[0];

@@ -601,3 +601,20 @@ def test_expert_layer_forms_agree(T, E, K, capacity, arena, shared, monkeypatch)
         grads = dict(a.named_main_grads()) if arena else {n: p.grad for n, p in m.named_parameters()}
         out.append([y, x.grad, m._per_expert_drop_counts, *(g for g in grads.values() if g is not None)])
     assert len(out[0]) == len(out[1]) > 5 and all(torch.equal(p, q) for p, q in zip(*out))
+
+
+def test_native_expert_layer_asks_before_it_pushes():
+    """Every pushing product of the native layer takes its counters from the runtime, which refuses a second one behind a dispatch."""
+    from nanopysche_b200.models.moe import MoEBase
+    from nanopysche_b200.ops import _lib
+    from nanopysche_b200.ops.moe import build_runtime
+
+    m = MoEBase(d_model=256, hidden_size=256, num_experts=4, top_k=2, dtype=torch.bfloat16, device="cuda")
+    rt = build_runtime([m], tokens=300, device=torch.device("cuda"))
+    asked, ask = [], rt._push_counters
+    rt._push_counters = lambda: (asked.append(rt._may_push), ask())[1]
+    x = torch.randn(1, 300, 256, device="cuda").bfloat16().requires_grad_(True)
+    m(x).sum().backward()
+    assert asked == [True, True] and not rt._may_push                 # forward and backward, each behind a dispatch of its own
+    with pytest.raises(_lib.KernelError, match="once behind every dispatch"):
+        rt._push_counters()
