@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from pathlib import Path
 
 import torch
@@ -20,6 +21,7 @@ _LIB_ERR: str | None = None
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libnpb200.so"
 HOST_PATH = LIB_PATH.with_name("npb200_host.so")
 _HOST = None
+_LOAD = threading.RLock()   # the first call of an op may come from several threads at once
 
 c_void_p, c_int, c_ll, c_ull, c_float = C.c_void_p, C.c_int, C.c_longlong, C.c_ulonglong, C.c_float
 
@@ -191,9 +193,15 @@ def load_error() -> str | None:
 
 def lib():
     """Load (building first if the .so is missing and nvcc exists) and return the ctypes library."""
+    if _LIB is None:
+        with _LOAD:
+            if _LIB is None:
+                _load_lib()
+    return _LIB
+
+
+def _load_lib():
     global _LIB, _LIB_ERR
-    if _LIB is not None:
-        return _LIB
     if not (LIB_PATH.exists() and HOST_PATH.exists()):
         try:
             from ..build import build_extension
@@ -203,47 +211,53 @@ def lib():
             _LIB_ERR = f"build failed: {e}"
             raise KernelError(f"libnpb200.so missing and could not be built: {e}") from e
     try:
-        _LIB = C.CDLL(str(LIB_PATH))
+        dll = C.CDLL(str(LIB_PATH))
     except OSError as e:
         _LIB_ERR = str(e)
         raise KernelError(f"cannot load {LIB_PATH}: {e}") from e
-    _LIB.np_gemm_bf16.argtypes = [C.POINTER(GemmArgs), c_void_p]
-    _LIB.np_gemm_bf16_two.argtypes = [C.POINTER(GemmArgs), C.POINTER(GemmArgs), c_void_p]
-    _LIB.np_ep_dispatch.argtypes = [C.POINTER(DispatchArgs), c_void_p]
-    _LIB.np_ep_combine.argtypes = [C.POINTER(CombineArgs), c_void_p]
-    _LIB.np_gemm_fp8_block.argtypes = [C.POINTER(Fp8GemmArgs), c_void_p]
-    _LIB.np_gemm_mxfp8.argtypes = [C.POINTER(MxGemmArgs), c_void_p]
-    _LIB.np_mx_quant.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_ll, c_void_p]
-    _LIB.np_flow_quant_act.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_void_p, c_ll,
+    dll.np_gemm_bf16.argtypes = [C.POINTER(GemmArgs), c_void_p]
+    dll.np_gemm_bf16_two.argtypes = [C.POINTER(GemmArgs), C.POINTER(GemmArgs), c_void_p]
+    dll.np_ep_dispatch.argtypes = [C.POINTER(DispatchArgs), c_void_p]
+    dll.np_ep_combine.argtypes = [C.POINTER(CombineArgs), c_void_p]
+    dll.np_gemm_fp8_block.argtypes = [C.POINTER(Fp8GemmArgs), c_void_p]
+    dll.np_gemm_mxfp8.argtypes = [C.POINTER(MxGemmArgs), c_void_p]
+    dll.np_mx_quant.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_ll, c_void_p]
+    dll.np_flow_quant_act.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_void_p, c_ll,
                                         c_void_p]
-    _LIB.np_mx_dequant.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p]
-    _LIB.np_flow_quant_weight.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+    dll.np_mx_dequant.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p]
+    dll.np_flow_quant_weight.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                            c_void_p]
-    _LIB.np_attn_fwd.argtypes = [C.POINTER(AttnFwdArgs), c_void_p]
-    _LIB.np_attn_bwd.argtypes = [C.POINTER(AttnBwdArgs), c_void_p]
-    _LIB.np_decode_attn.argtypes = [C.POINTER(DecodeArgs), c_void_p]
-    _LIB.np_status_read.argtypes = [C.POINTER(c_int)]
-    return _LIB
+    dll.np_attn_fwd.argtypes = [C.POINTER(AttnFwdArgs), c_void_p]
+    dll.np_attn_bwd.argtypes = [C.POINTER(AttnBwdArgs), c_void_p]
+    dll.np_decode_attn.argtypes = [C.POINTER(DecodeArgs), c_void_p]
+    dll.np_status_read.argtypes = [C.POINTER(c_int)]
+    _LIB = dll
 
 
 def host():
     """The native host module (csrc/host.cpp): the ops of a layer with their launches and autograd nodes."""
-    global _HOST
     if _HOST is None:
-        import importlib.util
-
-        from . import gemm
-
-        lib()
-        try:
-            spec = importlib.util.spec_from_file_location("npb200_host", str(HOST_PATH))
-            mod = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(mod)
-        except (ImportError, OSError) as e:
-            raise KernelError(f"cannot load {HOST_PATH}: {e}") from e
-        mod.setup(KernelError, vars(gemm))
-        _HOST = mod
+        with _LOAD:
+            if _HOST is None:
+                _load_host()
     return _HOST
+
+
+def _load_host():
+    global _HOST
+    import importlib.util
+
+    from . import gemm
+
+    lib()
+    try:
+        spec = importlib.util.spec_from_file_location("npb200_host", str(HOST_PATH))
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except (ImportError, OSError) as e:
+        raise KernelError(f"cannot load {HOST_PATH}: {e}") from e
+    mod.setup(KernelError, vars(gemm))
+    _HOST = mod
 
 
 def available() -> bool:
