@@ -1,5 +1,5 @@
 """Build the sm_100a CUDA library (``nanopysche_b200/lib/libnpb200.so``) and the native host module that calls it from torch
-(``lib/npb200_host.so``) in-tree.
+(``lib/npb200_host.<torch>.<python>.so``: it is linked against one torch and one interpreter, and built anew for another) in-tree.
 
 Every ``csrc/*.cu`` file is compiled with nvcc for ``compute_100a/sm_100a`` (relocatable device
 code, one object per file, in parallel) and linked into one shared library that ``ops/_lib.py``
@@ -22,7 +22,16 @@ CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 OBJ_DIR = LIB_DIR / "obj"
 LIB_PATH = LIB_DIR / "libnpb200.so"
-HOST_PATH = LIB_DIR / "npb200_host.so"
+
+
+def host_path() -> Path:
+    """The native host module for the running torch and interpreter."""
+    import sysconfig
+
+    import torch
+
+    return LIB_DIR / f"npb200_host.torch-{torch.__version__}.{sysconfig.get_config_var('SOABI')}.so"
+
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -69,16 +78,16 @@ def build_host(force: bool = False) -> Path:
 
     import torch
 
-    src = CSRC / "host.cpp"
+    src, path = CSRC / "host.cpp", host_path()
     newest = max(src.stat().st_mtime, _newest_header_mtime())
-    if not force and HOST_PATH.exists() and HOST_PATH.stat().st_mtime >= newest:
-        return HOST_PATH
+    if not force and path.exists() and path.stat().st_mtime >= newest:
+        return path
     root = Path(torch.__file__).resolve().parent
     if not (root / "lib" / "libc10_cuda.so").exists():   # a CPU-only torch never calls it
-        return HOST_PATH
+        return path
     nvcc = find_nvcc()
     cuda = Path(nvcc).resolve().parent.parent if nvcc else Path("/usr/local/cuda")
-    tmp = HOST_PATH.with_suffix(".so.tmp")
+    tmp = path.with_suffix(".so.tmp")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=npb200_host",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-isystem", str(root / "include"), "-isystem", str(root / "include/torch/csrc/api/include"),
@@ -93,9 +102,9 @@ def build_host(force: bool = False) -> Path:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         sys.stderr.write(proc.stdout + proc.stderr)
-        raise RuntimeError("build of npb200_host.so failed")
-    os.replace(tmp, HOST_PATH)
-    return HOST_PATH
+        raise RuntimeError(f"build of {path.name} failed")
+    os.replace(tmp, path)
+    return path
 
 
 def build_extension(force: bool = False, verbose: bool = False) -> Path:

@@ -19,7 +19,6 @@ import torch
 _LIB = None
 _LIB_ERR: str | None = None
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libnpb200.so"
-HOST_PATH = LIB_PATH.with_name("npb200_host.so")
 _HOST = None
 _LOAD = threading.RLock()   # the first call of an op may come from several threads at once
 
@@ -202,7 +201,7 @@ def lib():
 
 def _load_lib():
     global _LIB, _LIB_ERR
-    if not (LIB_PATH.exists() and HOST_PATH.exists()):
+    if not LIB_PATH.exists():
         try:
             from ..build import build_extension
 
@@ -247,15 +246,20 @@ def _load_host():
     global _HOST
     import importlib.util
 
+    from .. import build
     from . import gemm
 
     lib()
+    path = build.host_path()
     try:
-        spec = importlib.util.spec_from_file_location("npb200_host", str(HOST_PATH))
+        if not path.exists():   # another torch or interpreter than it was built for last
+            build.build_host()
+        spec = importlib.util.spec_from_file_location("npb200_host", str(path))
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
-    except (ImportError, OSError) as e:
-        raise KernelError(f"cannot load {HOST_PATH}: {e}") from e
+    except (ImportError, OSError, RuntimeError) as e:
+        raise KernelError(f"cannot build or load {path.name}, the native host module for this torch and interpreter "
+                          f"(python -m nanopysche_b200.build): {e}") from e
     mod.setup(KernelError, vars(gemm))
     _HOST = mod
 

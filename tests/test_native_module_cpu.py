@@ -1,7 +1,8 @@
-"""Loading of the native host module (no GPU needed)."""
+"""The native host module's file and its loading: one per torch and interpreter, from several threads at once (no GPU needed)."""
 import subprocess
 import sys
 import textwrap
+import types
 
 import pytest
 import torch
@@ -9,7 +10,40 @@ import torch
 from nanopysche_b200 import build
 from nanopysche_b200.ops import _lib
 
-built = pytest.mark.skipif(not (_lib.LIB_PATH.exists() and build.HOST_PATH.exists()), reason="the library is not built here")
+built = pytest.mark.skipif(not (_lib.LIB_PATH.exists() and build.host_path().exists()), reason="the library is not built here")
+
+
+def test_the_file_belongs_to_one_torch_and_interpreter(monkeypatch):
+    import sysconfig
+
+    here = build.host_path()
+    assert torch.__version__ in here.name and sysconfig.get_config_var("SOABI") in here.name
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert build.host_path() != here
+
+
+@built
+def test_the_kernel_library_does_not_need_it(monkeypatch):
+    monkeypatch.setattr(build, "host_path", lambda: _lib.LIB_PATH.with_name("absent.so"))
+    monkeypatch.setattr(build, "build_extension", lambda *a: pytest.fail("built"))
+    monkeypatch.setattr(_lib, "_LIB", None)
+    assert _lib.lib().np_sumsq_parts() > 0
+
+
+@built
+def test_a_module_that_does_not_load_is_named_with_the_command(monkeypatch, tmp_path):
+    bad = tmp_path / "npb200_host.other.so"
+    bad.write_bytes(b"not a library")
+    monkeypatch.setattr(build, "host_path", lambda: bad)
+    monkeypatch.setattr(_lib, "_HOST", None)
+    with pytest.raises(_lib.KernelError, match="npb200_host.other.so.*python -m nanopysche_b200.build"):
+        _lib.host()
+    made = types.SimpleNamespace(done=0)
+    monkeypatch.setattr(build, "host_path", lambda: tmp_path / "absent.so")
+    monkeypatch.setattr(build, "build_host", lambda: setattr(made, "done", 1))
+    with pytest.raises(_lib.KernelError):
+        _lib.host()
+    assert made.done == 1
 
 
 @built
