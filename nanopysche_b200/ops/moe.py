@@ -207,6 +207,9 @@ class FusedMoERuntime:
             self._wq_valid.add(layer)
         return w13q, s13, w2q, s2
 
+    def __getstate__(self):
+        return {**self.__dict__, "_native": None}   # a copy has buffers of its own, and gets its own view of them
+
     def native(self):
         """The native module's view of this runtime (buffers and tables do not change once they are there)."""
         if self._native is None:

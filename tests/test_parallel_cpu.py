@@ -737,3 +737,15 @@ def test_expert_layer_with_peers_runs_the_python_form():
 
     assert [_native_form(SimpleNamespace(N=n, fp8=f)) for n, f in ((1, False), (2, False), (8, False), (1, True), (2, True))] == \
         [True, False, False, False, False]
+
+
+def test_runtime_of_an_expert_layer_can_be_copied():
+    """A model that has run can be copied: the native module's view of the runtime's buffers stays behind."""
+    import copy
+
+    from nanopysche_b200.ops.moe import FusedMoERuntime
+
+    rt = FusedMoERuntime.__new__(FusedMoERuntime)
+    rt.T, rt.recv_g, rt._native = 5, torch.ones(3), (i for i in range(3))      # a generator cannot be copied either
+    c = copy.deepcopy(rt)
+    assert c._native is None and c.T == 5 and torch.equal(c.recv_g, rt.recv_g) and c.recv_g is not rt.recv_g and rt._native is not None
