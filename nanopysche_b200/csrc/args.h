@@ -102,7 +102,7 @@ struct NpAttnBwdArgs {
   int head_dim;    // 128 (also when 0) or 64
 };
 
-// Mirrored by DecodeArgs in ops/_lib.py. All tensors bf16 with 16-byte aligned rows of HD elements (64 or 128).
+// All tensors bf16 with 16-byte aligned rows of HD elements (64 or 128).
 struct NpDecodeArgs {
   const void* q; long long q_sb, q_ss, q_sh;
   const void* kc; const void* vc; long long kc_sb, kc_ss, kc_sh, vc_sb, vc_ss, vc_sh;

@@ -131,21 +131,6 @@ class AttnBwdArgs(C.Structure):
     ]
 
 
-class DecodeArgs(C.Structure):
-    """Mirror of ``NpDecodeArgs`` in csrc/args.h."""
-
-    _fields_ = [
-        ("q", c_void_p), ("q_sb", c_ll), ("q_ss", c_ll), ("q_sh", c_ll),
-        ("kc", c_void_p), ("vc", c_void_p), ("kc_sb", c_ll), ("kc_ss", c_ll), ("kc_sh", c_ll),
-        ("vc_sb", c_ll), ("vc_ss", c_ll), ("vc_sh", c_ll),
-        ("kn", c_void_p), ("vn", c_void_p), ("kn_sb", c_ll), ("kn_ss", c_ll), ("kn_sh", c_ll),
-        ("vn_sb", c_ll), ("vn_ss", c_ll), ("vn_sh", c_ll),
-        ("ko", c_void_p), ("vo", c_void_p), ("o", c_void_p),
-        ("B", c_int), ("Sq", c_int), ("Hq", c_int), ("Hkv", c_int), ("past", c_int), ("fresh", c_int),
-        ("causal", c_int), ("head_dim", c_int), ("scale", c_float),
-    ]
-
-
 class Fp8GemmArgs(C.Structure):
     """Mirror of ``NpFp8GemmArgs`` in csrc/gemm_fp8_sm100.cu."""
 
@@ -228,7 +213,6 @@ def _load_lib():
                                            c_void_p]
     dll.np_attn_fwd.argtypes = [C.POINTER(AttnFwdArgs), c_void_p]
     dll.np_attn_bwd.argtypes = [C.POINTER(AttnBwdArgs), c_void_p]
-    dll.np_decode_attn.argtypes = [C.POINTER(DecodeArgs), c_void_p]
     dll.np_status_read.argtypes = [C.POINTER(c_int)]
     _LIB = dll
 

@@ -258,7 +258,7 @@ class FusedMoERuntime:
         _lib.check(_lib.lib().np_ep_combine(C.byref(a), C.c_void_p(_lib.stream())), "ep_combine")
 
     def grouped_gemm(self, A, B, *, N, K, b_mn, group_stride_b, out=None, B2=None, C2=None, wait_epoch=0,
-                     push_ptrs=None, push_epoch=0, out_dtype=torch.bfloat16, k_split=0, glu_of=None):
+                     push_ptrs=None, push_epoch=0, k_split=0, glu_of=None):
         """Row-grouped GEMM over the receive-buffer layout (mode 1). ``B2``: the up weight of the SwiGLU form, or with
         ``k_split`` the weight that the contraction continues with from there on. ``glu_of``: pre-activations ``[gate | up]``;
         the product is the gradient of ``silu(gate) * up`` and ``[d gate | d up]`` is what is returned."""
@@ -267,8 +267,6 @@ class FusedMoERuntime:
         if glu_of is not None:
             out = torch.empty_like(glu_of)
             g.epilogue, g.C2, g.ldc2 = 2, glu_of.data_ptr(), glu_of.stride(0)
-        if out is None and push_ptrs is None:
-            out = torch.empty((M, N), device=A.device, dtype=out_dtype)
         g.A, g.B = A.data_ptr(), B.data_ptr()
         g.lda, g.ldb = A.stride(0), B.stride(0)
         g.a_rows, g.b_rows = A.shape[0], B.shape[0]
