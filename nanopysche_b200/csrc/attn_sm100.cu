@@ -819,7 +819,6 @@ bool bind_ctx() {
 
 }  // namespace
 
-
 // a kernel of 20 us and more
 static bool busy(int B, int H, int Sq, int Sk, int hd) { return 4.0 * B * H * Sq * (double)Sk * hd > 2e10; }
 
@@ -1478,7 +1477,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 }
 
 }  // namespace
-
 
 template <int NS, int HD>
 static int launch_bwd(dim3 gq, dim3 gk, int skip, const CUtensorMap& tmQ, const CUtensorMap& tmdO, const CUtensorMap& tmK,

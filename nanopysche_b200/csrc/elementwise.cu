@@ -703,8 +703,8 @@ __device__ __forceinline__ void ld4f(const float* p, float* f) {
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
 }
 // the V heads of a block's tokens: copied by all of its threads, two tokens at a time
-__device__ __forceinline__ void copy_v_heads(const __nv_bfloat16* src, long long rs, long long hs, __nv_bfloat16* dst, long long ds, int hkv,
-                                             long long T) {
+__device__ __forceinline__ void copy_v_heads(const __nv_bfloat16* src, long long rs, long long hs, __nv_bfloat16* dst, long long ds,
+                                             int hkv, long long T) {
   for (int r = threadIdx.x; r < hkv * 16; r += blockDim.x) {
     const __nv_bfloat16* v = src + (long long)(r >> 4) * hs + (r & 15) * 8;
     __nv_bfloat16* o = dst + (r >> 4) * 128 + (r & 15) * 8;
@@ -722,16 +722,16 @@ __device__ __forceinline__ int token_pos(const int* pos_ids, long long t, long l
   return pos_ids ? pos_ids[t] : (int)(T <= 0x7fffffff ? (unsigned)t % (unsigned)S : t % S) + pos_off;
 }
 
-// Backward: inverse rotation of dq / dk, LayerNorm backward against the saved pre-norm values and statistics,
-// dv copied; the three results form one contiguous dqkv. The gamma / beta gradients are accumulated per thread
-// (a thread keeps its (head, slice) across tokens), summed over the heads of a kind through shared memory in their order and written
-// as one partial row [4 x 128] per CTA (dgamma_q, dbeta_q, dgamma_k, dbeta_k). Added up by shared-memory atomics, all heads of a
-// kind on the same words, and with one token in flight the pass took 39 us at 2331 tokens and 16 / 8 heads (14 now) and 94 at 6000
-// (55). A head is handled by 16 neighbouring threads (a 4-wide slice of the lower half and its partner in the upper half); a block
-// has a thread per slice of the rotated heads, which keeps it for all tokens of the block with TOK of them in flight. 8-wide slices
-// need twice the registers and left too few threads on an SM to cover the loads (40 to 60 bytes of these spill as it is: the forms up
-// to 24 and above 40 heads). The two means of a head are summed in the order of 8-wide slices all the same (group16_sum): dq is rounded
-// to bf16, and in another order some of its values, and the projection's gradients behind them, come out differently.
+// Backward: inverse rotation of dq / dk, LayerNorm backward against the saved pre-norm values and statistics, dv copied; the three
+// results form one contiguous dqkv. The gamma / beta gradients are accumulated per thread (a thread keeps its (head, slice) across
+// tokens), summed over the heads of a kind through shared memory in their order and written as one partial row [4 x 128] per CTA
+// (dgamma_q, dbeta_q, dgamma_k, dbeta_k). Added up by shared-memory atomics, all heads of a kind on the same words, and with one
+// token in flight the pass took 39 us at 2331 tokens and 16 / 8 heads (14 now) and 94 at 6000 (55). A head is handled by 16
+// neighbouring threads (a 4-wide slice of the lower half and its partner in the upper half); a block has a thread per slice of the
+// rotated heads, which keeps it for all tokens of the block with TOK of them in flight. 8-wide slices need twice the registers and
+// left too few threads on an SM to cover the loads (as it is 44 bytes spill in the form up to 24 heads, 20 in that above 40).
+// The two means of a head are summed in the order of 8-wide slices all the same (group16_sum): dq is rounded to bf16, and in
+// another order some of its values, and the projection's gradients behind them, come out differently.
 template <int NTH, int MINB, int TOK>
 __global__ void __launch_bounds__(NTH, MINB) qkv_norm_rope_bwd_kernel(
     HeadSrc s0, HeadSrc s1, HeadSrc s2, const __nv_bfloat16* qkv, long long row_stride, int hq, int hkv,
@@ -876,7 +876,8 @@ __global__ void __launch_bounds__(NT, 4) xent_fwd_kernel(const __nv_bfloat16* lo
   const __nv_bfloat16* lr = logits + (size_t)r * ld;
   const int nvec = V >> 3;
   auto load = [&](int c) {
-    return c < nvec ? *reinterpret_cast<const uint4*>(lr + (size_t)c * 8) : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
+    return c < nvec ? *reinterpret_cast<const uint4*>(lr + (size_t)c * 8)
+                    : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
   };
   auto pair = [](const uint32_t& w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); };
   __nv_bfloat162 m2 = __float2bfloat162_rn(-INFINITY);
@@ -1048,7 +1049,8 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const float* x, long long n,
   for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < nvec; i += U * stride) {
     float4 a[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) a[u] = i + u * stride < nvec ? reinterpret_cast<const float4*>(x)[i + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < U; ++u)
+      a[u] = i + u * stride < nvec ? reinterpret_cast<const float4*>(x)[i + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < U; ++u) s += a[u].x * a[u].x + a[u].y * a[u].y + a[u].z * a[u].z + a[u].w * a[u].w;
   }
@@ -1238,7 +1240,7 @@ NP_API int np_qkv_norm_rope_fwd(const void* qkv, long long row_stride, int hq, i
       sin_t, pos_ids, T, S, pos_off);
   CHECK_LAUNCH();
 }
-// CTAs of the backward pass: as many as are resident (two per SM up to 24 heads of q and k)
+// CTAs of the backward pass: as many as are resident up to 24 heads of q and k (two per SM), and with more heads two turns of them
 NP_API int np_qkv_norm_rope_parts(long long T) {
   const long long grid = (T + 1) / 2;
   return (int)(grid < 148 * 2 ? (grid > 0 ? grid : 1) : 148 * 2);
@@ -1261,12 +1263,15 @@ NP_API int np_qkv_norm_rope_bwd(const void* dq, long long rs0, long long hs0, co
   static NpPerDeviceOnce attr_once;
   bool& attr_set = *attr_once.slot();
   if (!attr_set) {   // more than 48 KB from 45 heads of q and k on
-    const cudaError_t e = cudaFuncSetAttribute(qkv_norm_rope_bwd_kernel<1024, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 * ROW_BYTES);
+    const cudaError_t e =
+        cudaFuncSetAttribute(qkv_norm_rope_bwd_kernel<1024, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 * ROW_BYTES);
     if (e != cudaSuccess) return 400 + (int)e;
     attr_set = true;
   }
   const int nrot = hq + hkv;   // a thread per 4-wide slice of the lower halves of the q and k heads
-  auto kern = nrot <= 24 ? qkv_norm_rope_bwd_kernel<384, 2, 2> : nrot <= 40 ? qkv_norm_rope_bwd_kernel<640, 1, 2> : qkv_norm_rope_bwd_kernel<1024, 1, 1>;
+  auto kern = nrot <= 24   ? qkv_norm_rope_bwd_kernel<384, 2, 2>
+              : nrot <= 40 ? qkv_norm_rope_bwd_kernel<640, 1, 2>
+                           : qkv_norm_rope_bwd_kernel<1024, 1, 1>;
   np_launch(kern, grid, nrot * 16, (size_t)nrot * 16 * ROW_BYTES, s, 1, s0, s1, s2, (const __nv_bfloat16*)qkv, row_stride, hq, hkv, gq, gk,
             (const float2*)stats, (__nv_bfloat16*)dqkv, scratch, cos_t, sin_t, pos_ids, T, S, pos_off);
   np_launch(colsum_tall_kernel, (4 * 128 + 31) / 32, 256, 0, s, 1, scratch, dparams, grid, 4 * 128, accumulate);

@@ -427,7 +427,6 @@ __global__ void __launch_bounds__(256) mx_quant_kernel(const __nv_bfloat16* __re
   }
 }
 
-
 // ------------------------------------------------------------------------------- 128-wide power-of-two blocks
 // The FP8-Flow-MoE recipe scales activations per 1x128 block and weights per 128x128 block. With the scale
 // restricted to a power of two (UE8M0, the form DeepSeek's own Blackwell kernels use) such a block is four

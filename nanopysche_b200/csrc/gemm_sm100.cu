@@ -792,7 +792,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // memory receives its own 128 rows of the result. Against the one-CTA 128 x 256 tile, which asks the L2 -> SM fabric for
 // 48 KB per 64-wide K step and SM, this needs 32 KB for the same FLOPs, and unlike a 256 x 256 tile on one SM the
 // 128 x 256 accumulator still fits tensor memory twice, so a tile drains under the MMAs of the next. The freed shared
-// memory deepens the pipeline to PAIR_STAGES K steps. No load is multicast.
+// memory deepens the pipeline to six K steps (eight of 128 columns). No load is multicast.
 //
 // Barriers: full[s] lives in the leader and counts the bytes of both CTAs' loads; empty[s] and tfull[a] exist in both
 // CTAs and are signalled by one multicast commit of the leader; tempty[a] lives in the leader and takes the arrivals of
@@ -868,8 +868,8 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) 
 // DUAL: two products in one launch. A backward pass asks for the gradients of a layer's input and of its weight at the same
 // time; alone, each leaves SMs without work in its only or last wave and pays for a launch, first loads and a last drain of its
 // own. A pair takes its tiles of the product with the longer contraction first, then those of the other. us, two launches /
-// one, in a graph, gradients of a layer of T tokens, N outputs, K inputs: T N K = 2048 1024 1024 22.8 / 14.9, 2048 3072 1024 34.1 /
-// 29.5, 2048 5632 1024 51.5 / 40.7, 2331 2048 2048 45.7 / 31.3, 4096 2048 5632 with the SwiGLU gradient 178.7 / 155.9.
+// one, in a graph, gradients of a layer of T tokens, N outputs, K inputs: T N K = 2048 1024 1024 23.2 / 14.9, 2048 3072 1024 34.8 /
+// 28.4, 2048 5632 1024 50.8 / 39.3, 2331 2048 2048 43.6 / 29.8, 4096 2048 5632 with the SwiGLU gradient 178.7 / 155.9.
 struct PairMaps {
   CUtensorMap A, B, B2, C, C2;
 };
@@ -1349,7 +1349,6 @@ int np_make_tmap_2d(CUtensorMap* out, const void* base, int elt_bytes, uint64_t 
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
-
 static int num_sms() {
   if (g_num_sms == 0) {
     int dev = 0;
@@ -1454,8 +1453,8 @@ static int prepare_gemm(const NpGemmArgs& a, int splits, int parts, PairMaps& m,
   // Plain outputs (dense rows, nothing added from memory, aligned) leave by TMA; peer-row tables, accumulation and other
   // alignments store from registers. The SwiGLU form needs both of its outputs aligned. So do rows whose length is no whole number
   // of 16 bytes: a tensor store rounds it up and fills with zeros, up to seven elements beside the output of a wider buffer.
-  p.tma_c = p.v16 && (a.N * (long long)es) % 16 == 0 && !a.row_dst && !a.done_counters && !p.Cin && splits == 1 && (a.epilogue != 1 || BN == 256) && a.ldc >= a.N &&
-            (a.epilogue != 1 || !a.C2 || p.v16_c2);
+  p.tma_c = p.v16 && (a.N * (long long)es) % 16 == 0 && !a.row_dst && !a.done_counters && !p.Cin && splits == 1 &&
+            (a.epilogue != 1 || BN == 256) && a.ldc >= a.N && (a.epilogue != 1 || !a.C2 || p.v16_c2);
   tmC = tmA;
   tmC2 = tmA;
   if (a.epilogue == 2) {   // [d gate | d up] out, [gate | up] in: two planes of N columns each

@@ -1,6 +1,6 @@
 // Native host path of the ops that run many times per layer: checks, output tensors, argument structures, the launch and the autograd
-// nodes. Same operands, refusals and saved tensors as the Python statements in ops/; those stay for CPU tensors and the special
-// forms. A call through ctypes from a Python autograd function took 20 us of host time forward and as much again backward (one
+// nodes. Same operands, refusals and saved tensors as the Python statements in ops/; those stay for CPU tensors and, for
+// the expert layer, the forms with peers or e4m3 operands. A call through ctypes from a Python autograd function took 20 us of host time forward and as much again backward (one
 // RMSNorm 105 us with its backward, of which the kernels are 10), more than most kernels of a small layer.
 #include <torch/extension.h>
 #include <torch/csrc/Exceptions.h>
@@ -139,7 +139,8 @@ Tensor gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const OptTen
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return o;
 }
-Tensor mm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const OptTensor& out, std::optional<at::ScalarType> dtype, bool accumulate) {
+Tensor mm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const OptTensor& out, std::optional<at::ScalarType> dtype,
+          bool accumulate) {
   return gemm(a, b, a_mn, b_mn, out, dtype, accumulate, 1.0, 0, 0, std::nullopt, std::nullopt, 0, 0, 0);
 }
 // the two gradients of a linear layer; dw goes to `out` (added with `accumulate`)
@@ -338,7 +339,8 @@ struct QkvAttention : torch::autograd::Function<QkvAttention> {
     launched(np_attn_bwd(&a, stream()), "attn_bwd");
     Tensor dqkv = empty_like_of(buf, {B, S, (hq + 2 * hkv) * hd}, at::kBFloat16);
     if (norm) {
-      Tensor dpar = empty_like_of(buf, {4, hd}, at::kFloat), scratch = empty_like_of(buf, {np_qkv_norm_rope_parts(B * S), 4 * hd}, at::kFloat);
+      Tensor dpar = empty_like_of(buf, {4, hd}, at::kFloat),
+             scratch = empty_like_of(buf, {np_qkv_norm_rope_parts(B * S), 4 * hd}, at::kFloat);
       launched(np_qkv_norm_rope_bwd(ptr(dq), dq.stride(1), dq.stride(2), ptr(dk), dk.stride(1), dk.stride(2), ptr(dv), dv.stride(1),
                                     dv.stride(2), ptr(qkv), qkv.stride(1), (int)hq, (int)hkv, ptr<float>(saved[5]), ptr<float>(saved[6]),
                                     ptr(stats), ptr(dqkv), ptr<float>(dpar), ptr<float>(scratch), ptr<float>(cos), ptr<float>(sin), ids,
@@ -357,7 +359,8 @@ struct QkvAttention : torch::autograd::Function<QkvAttention> {
 
 // Rotation of x [B, S, H, hd] (contiguous heads, rows of any stride)
 struct Rope : torch::autograd::Function<Rope> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t pos, const OptTensor& pos_ids) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t pos,
+                        const OptTensor& pos_ids) {
     const int64_t B = x.size(0), S = x.size(1), H = x.size(2), hd = x.size(3);
     require(x.stride(3) == 1 && x.stride(2) == hd && x.stride(0) == S * x.stride(1), "contiguous heads");
     Tensor out = empty_like_of(x, {B, S, H, hd}, x.scalar_type());
@@ -385,7 +388,8 @@ struct Rope : torch::autograd::Function<Rope> {
 std::tuple<Tensor, Tensor, Tensor> decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k_new, const Tensor& v_new,
                                           bool causal, double scale) {
   const int64_t B = q.size(0), Sq = q.size(1), Hq = q.size(2), hd = q.size(3), P = k.size(1), Hkv = k.size(2), n = k_new.size(1);
-  Tensor o = empty_like_of(q, {B, Sq, Hq, hd}, at::kBFloat16), ko = empty_like_of(q, {B, P + n, Hkv, hd}, at::kBFloat16), vo = at::empty_like(ko);
+  Tensor o = empty_like_of(q, {B, Sq, Hq, hd}, at::kBFloat16), ko = empty_like_of(q, {B, P + n, Hkv, hd}, at::kBFloat16),
+         vo = at::empty_like(ko);
   NpDecodeArgs a{};
   a.q = q.data_ptr(); a.q_sb = q.stride(0); a.q_ss = q.stride(1); a.q_sh = q.stride(2);
   a.kc = k.data_ptr(); a.kc_sb = k.stride(0); a.kc_ss = k.stride(1); a.kc_sh = k.stride(2);
@@ -393,7 +397,8 @@ std::tuple<Tensor, Tensor, Tensor> decode(const Tensor& q, const Tensor& k, cons
   a.kn = k_new.data_ptr(); a.kn_sb = k_new.stride(0); a.kn_ss = k_new.stride(1); a.kn_sh = k_new.stride(2);
   a.vn = v_new.data_ptr(); a.vn_sb = v_new.stride(0); a.vn_ss = v_new.stride(1); a.vn_sh = v_new.stride(2);
   a.ko = ko.data_ptr(); a.vo = vo.data_ptr(); a.o = o.data_ptr();
-  a.B = (int)B; a.Sq = (int)Sq; a.Hq = (int)Hq; a.Hkv = (int)Hkv; a.past = (int)P; a.fresh = (int)n; a.causal = causal; a.head_dim = (int)hd;
+  a.B = (int)B; a.Sq = (int)Sq; a.Hq = (int)Hq; a.Hkv = (int)Hkv; a.past = (int)P; a.fresh = (int)n; a.causal = causal;
+  a.head_dim = (int)hd;
   a.scale = (float)scale;
   launched(np_decode_attn(&a, stream()), "decode_attn");
   return {o, ko, vo};
@@ -692,8 +697,8 @@ struct FusedMoE : torch::autograd::Function<FusedMoE> {
     return res;
   }
 };
-variable_list router(const Tensor& x2, const Tensor& gate_w, const OptTensor& gate_b, const OptTensor& score_bias, int64_t K, int64_t gating,
-                     double coef_z) {
+variable_list router(const Tensor& x2, const Tensor& gate_w, const OptTensor& gate_b, const OptTensor& score_bias, int64_t K,
+                     int64_t gating, double coef_z) {
   return Router::apply(x2, gate_w, gate_b, score_bias, K, gating, coef_z);
 }
 variable_list fused_moe(const Tensor& x, const Tensor& weights, const Tensor& idx, const Tensor& w1, const Tensor& w3, const Tensor& w2,
@@ -702,8 +707,12 @@ variable_list fused_moe(const Tensor& x, const Tensor& weights, const Tensor& id
 }
 
 Tensor linear(const Tensor& x, const Tensor& w) { return Linear::apply(x, w); }
-variable_list rms_norm(const Tensor& x, const Tensor& w, const OptTensor& residual, double eps) { return RmsNorm::apply(x, w, residual, eps); }
-Tensor rope(const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t pos, const OptTensor& ids) { return Rope::apply(x, cos, sin, pos, ids); }
+variable_list rms_norm(const Tensor& x, const Tensor& w, const OptTensor& residual, double eps) {
+  return RmsNorm::apply(x, w, residual, eps);
+}
+Tensor rope(const Tensor& x, const Tensor& cos, const Tensor& sin, int64_t pos, const OptTensor& ids) {
+  return Rope::apply(x, cos, sin, pos, ids);
+}
 Tensor qkv_attention(const Tensor& qkv, const OptTensor& gq, const OptTensor& bq, const OptTensor& gk, const OptTensor& bk, double eps,
                      const Tensor& cos, const Tensor& sin, int64_t hq, int64_t hkv, int64_t hd, int64_t pos, const OptTensor& pos_ids,
                      bool causal, double scale) {

@@ -3,7 +3,7 @@
 //  router_logits / router_topk / router_bwd : fp32 gate, DeepSeek-V3 score bias, top-k with softmax-
 //      over-top-k or sigmoid+renorm gating, per-expert histogram, sum of full-softmax probabilities
 //      and sum of logsumexp^2 (aux / z loss) in one pass; analytic backward to the logits.
-//  capacity_scan : position of every token inside each expert it picked (index order), whole-token
+//  capacity_plan : position of every token inside each expert it picked (index order), whole-token
 //      drop beyond the capacity, positions among the kept tokens - no host sync.
 //  ep_dispatch   : the all-to-all dispatch as peer stores: every kept (token, k) row is written
 //      straight into the owning rank's expert-major receive buffer (region [local expert][source
@@ -36,12 +36,13 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 // ------------------------------------------------------------------ router
-// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). Four warps share TOK tokens, each over the whole rows
-// for EPW experts of a pass; MINB: CTAs per SM that the register count is held to, U: steps whose loads are in flight together. Bound by
-// L1: the gate rows are 64 KB per TOK tokens at d 2048 and 8 experts, and each warp reads the tokens again. A warp to a token had the
-// chain of its loads to wait for. 8 experts, us, before / now: 64 x 2048 7.2 / 3.5, 1024 10.8 / 5.0, 4096 20.7 / 13.3, 16384 41.4 / 40.6; 64
-// experts, 4096 x 1024 82 / 43. A quarter of the row to a warp, added over the warps, takes 11.7 at 4096 and 30.3 at 16384, but forms
-// the sums in another order; gate weights that differ in their last bits move the bf16 rows that they scale.
+// logits[t, e] = <x[t], Wg[e]> + bias[e]  (fp32 accumulate, fp32 gate weights). Four warps share TOK tokens, each over the whole
+// rows for EPW experts of a pass; MINB: CTAs per SM that the register count is held to, U: steps whose loads are in flight
+// together. Bound by L1: the gate rows are 64 KB per TOK tokens at d 2048 and 8 experts, and each warp reads the tokens again. A
+// warp to a token had the chain of its loads to wait for. 8 experts, us, before / now: 64 x 2048 7.2 / 3.5, 1024 10.8 / 5.0, 4096
+// 20.7 / 13.3, 16384 41.4 / 40.6; 64 experts, 4096 x 1024 82 / 43. A quarter of the row to a warp, added over the warps, takes 11.7
+// at 4096 and 30.3 at 16384, but forms the sums in another order; gate weights that differ in their last bits move the bf16 rows
+// that they scale.
 // Every token's sum is formed in the same order in all forms: a lane's vectors one after the other, then over the lanes.
 template <int TOK, int EPW, int MINB, int U>
 __global__ void __launch_bounds__(256, MINB) router_logits_kernel(const __nv_bfloat16* x, const float* wg, const float* bias,
@@ -290,12 +291,13 @@ __global__ void __launch_bounds__(128) router_bwd_kernel(const float* logits,
     if (e < E) dlogits[(size_t)t * E + e] = dl[e];
 }
 
-// partial[c, e, d] = sum over a chunk of 64 tokens of dl[t, e] * x[t, d] for EB experts a CTA. CTA = CT column threads (8 columns each) x 4
-// token lanes; a lane walks every fourth token of the chunk with U row loads in flight, the lanes are summed through shared
-// memory. Beside them the first sums of the column sums of dl (the bias gradient): virtual thread (g, e) of 1024 / E groups adds rows g, g +
-// groups, ... in four sums, into bias_part[g, e]. Bound by the chain of a lane's 16 tokens: a small batch takes narrow CTAs. us with the sum
-// over the chunks, wide CTAs and the bias gradient in a launch of its own / chunks of 16 tokens (another order of the sums) / now: 64 x 2048, 8
-// experts 10.9 / 4.2 / 6.5, 512 x 768 10.6 / 5.6 / 6.7, 1000 x 1024, 16 19.6 / 11.0 / 7.8, 4096 x 2048, 8 18.0 / 13.8 / 12.1.
+// partial[c, e, d] = sum over a chunk of 64 tokens of dl[t, e] * x[t, d] for EB experts a CTA. CTA = CT column threads (8 columns
+// each) x 4 token lanes; a lane walks every fourth token of the chunk with U row loads in flight, the lanes are summed through
+// shared memory. Beside them the first sums of the column sums of dl (the bias gradient): virtual thread (g, e) of 1024 / E groups
+// adds rows g, g + groups, ... in four sums, into bias_part[g, e]. Bound by the chain of a lane's 16 tokens: a small batch takes
+// narrow CTAs. us with the sum over the chunks, wide CTAs and the bias gradient in a launch of its own / chunks of 16 tokens
+// (another order of the sums) / now: 64 x 2048, 8 experts 10.9 / 4.2 / 6.5, 512 x 768 10.6 / 5.6 / 6.7, 1000 x 1024, 16 19.6 / 11.0
+// / 7.8, 4096 x 2048, 8 18.0 / 13.8 / 12.1.
 constexpr int DG_TOK = 64, DG_BIAS = 1024;
 template <int EB, int CT, int U>
 __global__ void __launch_bounds__(CT * 4) router_dgate_kernel(const float* dl, const __nv_bfloat16* x, float* __restrict__ partial,
@@ -490,15 +492,15 @@ __global__ void __launch_bounds__(64) router_dgate_sum_kernel(const float* parti
 
 // ------------------------------------------------------------------ capacity / positions
 // One CTA of 32 warps, each over a contiguous run of slots (t, k), 32 at a time, a lane per slot. One ballot per bit of the expert
-// number gives a lane the slots that picked the same expert as its own (its rank among them), and lane e those of expert e (and
-// e + 32), so that the counters of up to 64 experts stand in two registers of a warp; more experts take further passes. Two passes
-// over the slots with the warps' counts exchanged in between give the positions in token order. Phase 0 ranks every pick among all
+// number gives a lane the slots that picked the same expert as its own (its rank among them), and lane e those of expert e (and e +
+// 32), so that the counters of up to 64 experts stand in two registers of a warp; more experts take further passes. Two passes over
+// the slots with the warps' counts exchanged in between give the positions in token order. Phase 0 ranks every pick among all
 // tokens that picked the expert and clears the flag of a token any of whose picks lies at or beyond `capacity` (capacity < 0: keep
 // all); phase 1 ranks among the kept tokens. Up to 8192 slots stay in registers, more are read again (from L1). Bound by its chain
-// of barriers and shuffles, one SM. A thread per run of tokens that
-// scanned packed counters, us, before / now: 512 tokens, 8 experts, top 2 7.5 / 4.9, 4096 18.5 / 10.5, 16384, 64, top 6 977 / 246.
-// Outputs: slot_pos[t,k] (position among kept for expert idx[t,k], -1 if dropped), keep[T],
-// counts_kept[E], drops[E] (tokens beyond capacity per expert), n_dropped[1].
+// of barriers and shuffles, one SM. A thread per run of tokens that scanned packed counters, us, before / now: 512 tokens, 8
+// experts, top 2 7.5 / 4.3, 4096 18.5 / 9.3, 16384, 64, top 6 977 / 227.
+// Outputs: slot_pos[t,k] (position among kept for expert idx[t,k], -1 if dropped), keep[T], counts_kept[E], drops[E] (tokens beyond
+// capacity per expert), n_dropped[1].
 constexpr int PLAN_CHUNKS = 8;     // runs of 32 slots that a warp holds at once
 template <int EP>                  // experts per pass, 32 or 64
 __global__ void __launch_bounds__(1024) capacity_plan_kernel(const int* indices, int T, int E, int K, int capacity,
@@ -975,10 +977,10 @@ NP_API int np_router_logits(const void* x, const float* wg, const float* bias, f
     np_launch(kernel, (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream, 1, (const __nv_bfloat16*)x, wg, bias,
               logits, T, D, E, zero, n_zero);
   };
-  // Two tokens per four warps with two experts a warp and the vectors of four steps in flight as long as that is one wave of CTAs, then
-  // four, which read the gate rows half as often: an expert a warp and four steps, from nine experts on four experts a warp, which read the
-  // tokens a quarter as often. us, first / second / third: 64 x 2048, 8 experts 3.5 / 5.2 / 11.5, 1024 5.0 / 5.6 / 11.8, 2048 8.4 / 7.6 / 11.9, 4096
-  // 14.7 / 13.3 / 19.1; 2472 x 1024, 16 experts 10.8 / 11.9 / 11.1; 4096 x 1024, 64 53 / 47 / 43.
+  // Two tokens per four warps with two experts a warp and the vectors of four steps in flight as long as that is one wave of CTAs,
+  // then four, which read the gate rows half as often: an expert a warp and four steps, from nine experts on four experts a warp,
+  // which read the tokens a quarter as often. us, first / second / third: 64 x 2048, 8 experts 3.5 / 5.2 / 11.5, 1024 5.0 / 5.6 /
+  // 11.8, 2048 8.4 / 7.6 / 11.9, 4096 14.7 / 13.3 / 19.1; 2472 x 1024, 16 experts 10.8 / 11.9 / 11.1; 4096 x 1024, 64 53 / 47 / 43.
   if (T <= 148 * 2 * 4) run(router_logits_kernel<2, 2, 2, 4>, 2);
   else if (E <= 8) run(router_logits_kernel<4, 1, 2, 4>, 4);
   else run(router_logits_kernel<4, 4, 2, 1>, 4);
@@ -1034,11 +1036,13 @@ NP_API int np_router_dgate(const float* dl, const void* x, float* dwg, float* db
   const long long n = (long long)E * D;
   float* bias_part = scratch + parts * n;
   auto run = [&](auto kernel, int ct) {
-    np_launch(kernel, dim3((D / 8 + ct - 1) / ct, parts, (E + 7) / 8), ct * 4, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch, bias_part, T, D, E);
+    np_launch(kernel, dim3((D / 8 + ct - 1) / ct, parts, (E + 7) / 8), ct * 4, 0, s, 1, dl, (const __nv_bfloat16*)x, scratch,
+              bias_part, T, D, E);
   };
   if (T <= 1024) run(router_dgate_kernel<8, 16, 8>, 16);
   else run(router_dgate_kernel<8, 64, 4>, 64);
-  np_launch(router_dgate_sum_kernel, (unsigned)((n + 63) / 64 + (dbias ? 1 : 0)), 64, 0, s, 1, scratch, dwg, parts, n, bias_part, dbias, E, accumulate);
+  np_launch(router_dgate_sum_kernel, (unsigned)((n + 63) / 64 + (dbias ? 1 : 0)), 64, 0, s, 1, scratch, dwg, parts, n, bias_part,
+            dbias, E, accumulate);
   CHECK_LAUNCH();
 }
 
@@ -1056,8 +1060,7 @@ NP_API int np_router_dx(const float* dl, const float* wg, void* dx, int T, int D
   CHECK_LAUNCH();
 }
 
-// np_capacity_scan with the kept rows per rank (sent [n_ranks], may be null) and the running drop statistics (stats [3]:
-// last dropped, total dropped, total tokens; may be null) in the same launch.
+// sent [n_ranks]: kept rows per rank (may be null); stats [3]: last dropped, total dropped, total tokens (may be null).
 NP_API int np_capacity_plan(const int* indices, int T, int E, int K, int capacity, int* slot_pos, int* keep, int* counts_kept,
                             int* drops, int* n_dropped, int* sent, int n_ranks, long long* stats, void* stream) {
   if (K > MAX_K || (sent && (n_ranks <= 0 || E % n_ranks))) return 1;
@@ -1077,6 +1080,7 @@ NP_API int np_capacity_plan(const int* indices, int T, int E, int K, int capacit
   CHECK_LAUNCH();
 }
 
+// without either
 NP_API int np_capacity_scan(const int* indices, int T, int E, int K, int capacity, int* slot_pos, int* keep, int* counts_kept,
                             int* drops, int* n_dropped, void* stream) {
   return np_capacity_plan(indices, T, E, K, capacity, slot_pos, keep, counts_kept, drops, n_dropped, nullptr, 0, nullptr, stream);

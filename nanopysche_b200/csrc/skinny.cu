@@ -340,7 +340,6 @@ int np_skinny_linear(const void* x, long long ldx, const void* w, long long ldw,
   return e == cudaSuccess ? 0 : 500 + (int)e;
 }
 
-
 NP_API int np_decode_attn(const NpDecodeArgs* a, void* stream) {
   if (a->B <= 0 || a->Sq <= 0 || a->past + a->fresh <= 0) return 0;
   if (a->Hkv <= 0 || a->Hq % a->Hkv || (a->head_dim != 64 && a->head_dim != 128)) return 1;

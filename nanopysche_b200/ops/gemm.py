@@ -150,7 +150,8 @@ def gemm_dgrad_wgrad(dy: torch.Tensor, w: torch.Tensor, x: torch.Tensor, *, out:
     """``(dy @ w, dy.T @ x)`` for ``dy [M, N]``, ``w [N, K]``, ``x [M, K]``: the two gradients of a linear layer, in one launch
     where that is expected to be faster than two. The second goes to ``out`` (added with ``accumulate``), by default a new
     tensor in the dtype of ``w``. ``gu``: pre-activations ``[gate | up]`` with ``x = silu(gate) * up``; the first result is then
-    ``[d gate | d up]`` (``gemm_glu_bwd``, with ``round_dh``). ``pair_bn`` and ``mt`` ask for one launch with tiles of that many columns, two launches."""
+    ``[d gate | d up]`` (``gemm_glu_bwd``, with ``round_dh``). ``pair_bn`` and ``mt`` ask for one launch with tiles of that
+    many columns, two launches."""
     if not _use_kernel(dy):
         dx = gemm(dy, w, b_mn=True) if gu is None else gemm_glu_bwd(dy, w, gu, round_dh=round_dh)
         return dx, gemm(dy, x, a_mn=True, b_mn=True, out=out, out_dtype=w.dtype if out is None else None, accumulate=accumulate)
